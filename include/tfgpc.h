@@ -223,6 +223,72 @@ int tfgpc_grid_neighborhood_count(
     void* ws, size_t ws_bytes, int32_t* num_cells_host_out,
     int64_t* total_out);
 
+/* ---- grids with a cell table ------------------------------------------------
+ * The same grid with one int32 per cell, the place where the cell's points begin
+ * in the sorted order, which replaces the radix sort by a counting sort and the
+ * binary searches of FindNeighbors by loads.  The caller owns every array of the
+ * struct (device memory); all of them are outputs of the build.  cell_start holds
+ * tfgpc_cell_table_elems() values (0: the bounds need too large a table, use the
+ * key-based entries), packed [n,4] (D <= 3) one 16-byte row (x, y, z or 0, original
+ * index as int bits) per sorted point, ds batch_size * max_cells^2 * 2 values of
+ * which the first batch_size * C0 * C1 * 2 are the tube ranges [B,C0,C1,2]. */
+typedef struct tfgpc_cell_grid {
+  int D;
+  int max_cells;              /* bound of cells per dimension */
+  int64_t n, batch_size;
+  float *aabb_min, *aabb_max; /* [batch_size,D], widened by 1e-9 */
+  int32_t* num_cells;         /* [D], at most max_cells */
+  float* scaled_aabb_min;     /* [batch_size,D] */
+  float* inv_cell_sizes;      /* [D] */
+  int64_t* keys;              /* [n] */
+  int32_t* sorted_indices;    /* [n] */
+  int64_t* sorted_keys;       /* [n] */
+  float* sorted_points;       /* [n,D] */
+  int32_t* sorted_batch_ids;  /* [n] */
+  float* packed;              /* [n,4], D <= 3 */
+  int32_t* cell_start;
+  int32_t* ds;
+} tfgpc_cell_grid;
+
+size_t tfgpc_cell_table_elems(int D, int64_t batch_size, int max_cells);
+size_t tfgpc_cell_grid_workspace_bytes(int D, int64_t n, int64_t ns,
+                                       int64_t batch_size, int max_cells);
+
+/* Builds the grid and, with ns > 0, runs the count pass of a neighborhood on it
+ * (samples and ranges_out as in tfgpc_grid_neighborhood_count; inv_radii [D] on the
+ * device).  One blocking read: num_cells_host_out [D, host] and *total_out [host].
+ * TFGPC_ENOMEM and the counts asked for if max_cells was too small.  num_cells_in
+ * as in tfgpc_grid_neighborhood_count. */
+int tfgpc_cell_grid_neighborhood(
+    void* stream, const tfgpc_cell_grid* grid, const float* points,
+    const int32_t* batch_ids, const float* cell_sizes,
+    const int32_t* num_cells_in, const float* inv_radii, int64_t ns,
+    const float* samples, const int32_t* samples_batch_ids,
+    int samples_are_points, int max_neighs, int32_t* ranges_out, void* ws,
+    size_t ws_bytes, int32_t* num_cells_host_out, int64_t* total_out);
+
+/* Count pass (blocking, workspace of tfgpc_find_neighbors_workspace_bytes) and fill
+ * pass of FindNeighbors on a built grid; ids_out may be NULL. */
+int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid,
+                      const float* inv_radii, int64_t ns, const float* samples,
+                      const int32_t* samples_batch_ids, int samples_are_points,
+                      int max_neighs, int32_t* ranges_out, void* ws,
+                      size_t ws_bytes, int64_t* total_out);
+int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid,
+                     const float* inv_radii, int64_t ns, const float* samples,
+                     const int32_t* samples_batch_ids, int samples_are_points,
+                     int max_neighs, const int32_t* ranges, int64_t total,
+                     int32_t* neigh_out, int32_t* ids_out);
+
+/* ComputePdf at the samples over the grid's points within the radius, without a
+ * neighbor list: what tfgpc_compute_pdf_at_samples gives for the list of a
+ * neighborhood without limit. */
+int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
+                        const float* inv_radii, const float* inv_bandwidth,
+                        int mode, int64_t ns, const float* samples,
+                        const int32_t* samples_batch_ids, int samples_are_points,
+                        float* pdf_out);
+
 /* ---- FindNeighbors fill pass with original ids and densities --------------
  * tfgpc_find_neighbors_fill_ordered (sample_order may be NULL) that, in the same
  * pass, also writes what pylib computes from the neighbor list afterwards:

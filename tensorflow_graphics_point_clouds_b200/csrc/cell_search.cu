@@ -1,0 +1,509 @@
+// Radius search and density estimate on the cell table of a grid (cells.cuh).
+//
+// All samples of a cell have the same candidates, the points of its 3^(D-1) tubes.  A
+// warp takes up to 32 consecutive samples and, cell by cell among them, loads the
+// candidates into registers (kSteps per lane) and tests them against the cell's samples
+// one after the other: 32 tests per step and sample for about ten instructions (two
+// candidates per packed fp32x2 operation), against some forty-five with one sample per
+// warp and a loop over its tubes, which left a quarter of the lanes idle besides (a
+// tube of a uniform cloud with 32 neighbors per point holds 23 candidates).  The passes
+// are bound by issue slots, the fill pass by its output as well.
+#include "cell_grid.cuh"
+
+namespace tfgpc {
+namespace {
+
+constexpr int kThreads = 128;
+constexpr int kMaxSpan = 16;    // samples of one warp
+
+// What stands at the samples: mode 0 arrays of the caller; 1 the grid's own points in
+// their unsorted order, visited in the sorted one; 2 the sorted points.
+struct SampleSource {
+  int mode;
+  const float* samples;
+  const int32_t* batch_ids;
+};
+
+template <int D>
+struct Sample {
+  float p[D];
+  int cell[D];
+  int batch;
+  int key;        // of its cell, -1: no sample, or a batch id outside the batch
+  int id;         // row of its results, -1: no sample
+};
+
+template <int D>
+__device__ __forceinline__ void load_point(const CellsView& c, int64_t j, float* p, int* index) {
+  if (D <= 3) {
+    const float4 v = __ldg(c.packed + j);
+    p[0] = v.x; p[1] = v.y;
+    if (D == 3) p[D - 1] = v.z;
+    *index = __float_as_int(v.w);
+  } else {
+#pragma unroll
+    for (int d = 0; d < D; ++d) p[d] = __ldg(c.points + j * D + d);
+    *index = __ldg(c.indices + j);
+  }
+}
+
+template <int D>
+__device__ __forceinline__ Sample<D> load_sample(const CellsView& c, const SampleSource& src,
+                                                 int64_t v, bool live, const Grid<D>& g) {
+  Sample<D> s;
+  s.id = -1;
+  s.key = -1;
+  s.batch = -1;
+#pragma unroll
+  for (int d = 0; d < D; ++d) { s.p[d] = 0.0f; s.cell[d] = 0; }
+  if (!live) return s;
+  if (src.mode == 0) {
+    s.id = (int)v;
+    s.batch = __ldg(src.batch_ids + v);
+#pragma unroll
+    for (int d = 0; d < D; ++d) s.p[d] = __ldg(src.samples + v * D + d);
+  } else {
+    int index;
+    load_point<D>(c, v, s.p, &index);
+    s.id = src.mode == 1 ? index : (int)v;
+    s.batch = __ldg(c.batch_ids + v);
+  }
+  if (s.batch < 0 || s.batch >= c.batch_size) return s;
+  float smin[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) smin[d] = __ldg(c.scaled_min + (int64_t)s.batch * D + d);
+  cell_of<D>(s.p, smin, g, s.cell);
+  s.key = (int)key_of<D>(s.cell, g, s.batch);
+  return s;
+}
+
+// Two fp32 operations per instruction, each rounded like the scalar one.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+enum { kCount = 0, kFill = 1, kDensity = 2 };
+
+struct WalkArgs {
+  CellsView c;
+  SampleSource src;
+  int64_t ns;
+  int span;                     // samples per warp, 1 to kMaxSpan
+  const float* inv_radii;
+  int limit;                    // neighbors kept per sample
+  int32_t* counts;              // kCount: [ns]
+  const int32_t* ranges;        // kFill: [ns]
+  int2* neigh;                  // kFill: [M]
+  int2* ids;                    // kFill: [M] or null
+  const float* inv_bw;          // kDensity
+  int bw_mode;
+  float* density;               // kDensity: [ns]
+};
+
+// kCount: number of neighbors.  kFill: the pairs in ascending sorted index, and (ids)
+// with the neighbor's original index.  kDensity: ComputePdf (compute_pdf_kernels.cu.cc:
+// 107-128) over the points within the radius; the exponents of the D Gaussians are
+// added before the one exponential.
+// The distance test is the reference's: t_d = (s_d - p_d) * inv_r_d, the fma chain from
+// t_0 * t_0, sqrtf(d2) < 1 (count_neighbors_kernels.cu.cc:84-85), which a correctly
+// rounded square root decides like d2 < 1.
+template <int D, int MODE>
+__global__ void __launch_bounds__(kThreads)
+cells_walk_kernel(WalkArgs a) {
+  constexpr int kSteps = D <= 3 ? 8 : 4;     // candidates per lane and round
+  constexpr int kTubes = num_tubes<D>();
+  constexpr int kTop = kTubes > 16 ? 16 : kTubes > 8 ? 8 : kTubes > 4 ? 4 : 2;
+  const CellsView& c = a.c;
+  const int lane = lane_id();
+  const int64_t v0 = (((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5) * a.span;
+  if (v0 >= a.ns) return;
+  const Grid<D> g = load_grid<D>(c.num_cells, c.inv_cell);
+  const int total = total_cells<D>(g.nc, c.batch_size);
+  f32x2 inv_r[D];
+  float scale[D], norm = 1.0f;
+  bool isotropic = true;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float r = __ldg(a.inv_radii + d);
+    inv_r[d] = pack2(r, r);
+    if (MODE == kDensity) {
+      const float bw = a.bw_mode == 1 ? sqrtf((float)c.n) : __ldg(a.inv_bw + d);
+      scale[d] = bw * bw * (-0.5f * 1.44269504f);     // of a base-2 exponential
+      norm *= bw * 0.39894228f;
+      isotropic = isotropic && scale[d] == scale[0];
+    }
+  }
+  const bool live = lane < a.span && v0 + lane < a.ns;
+  const Sample<D> s = load_sample<D>(c, a.src, v0 + lane, live, g);
+  int my_count = 0, my_begin = 0;
+  float my_density = 0.0f;
+  if (MODE == kFill && s.id > 0) my_begin = __ldg(a.ranges + s.id - 1);
+  unsigned open = __ballot_sync(0xffffffffu, s.key >= 0);
+  while (open) {
+    // the samples of one cell
+    const int leader = __ffs(open) - 1;
+    const int leader_key = __shfl_sync(0xffffffffu, s.key, leader);
+    const unsigned members = __ballot_sync(0xffffffffu, s.key == leader_key);
+    open &= ~members;
+    int cell[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) cell[d] = __shfl_sync(0xffffffffu, s.cell[d], leader);
+    const int batch = __shfl_sync(0xffffffffu, s.batch, leader);
+    for (int tube0 = 0; tube0 < kTubes; tube0 += 32) {
+      // lane t: the t-th tube in ascending sorted index, and how many candidates come before
+      int2 r = make_int2(0, 0);
+      if (tube0 + lane < kTubes)
+        r = tube_points<D>(kTubes - 1 - (tube0 + lane), cell, batch, g.nc, total, c.start);
+      int before = r.y - r.x;     // inclusive running count
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += y;
+      }
+      const int candidates = __shfl_sync(0xffffffffu, before, 31);
+      const int offset = r.y - before;   // sorted index of candidate i of this tube: i + offset
+      for (int base = 0; base < candidates; base += 32 * kSteps) {
+        f32x2 np[D][kSteps / 2];         // negated coordinates of the lane's candidates
+        int at[kSteps], index[kSteps];
+#pragma unroll
+        for (int k = 0; k < kSteps; k += 2) {
+          float p[2][D];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = base + 32 * (k + u) + lane;
+            int t = 0;
+#pragma unroll
+            for (int o = kTop; o > 0; o >>= 1) {
+              const int y = __shfl_sync(0xffffffffu, before, t + o - 1);
+              if (y <= i) t += o;
+            }
+            at[k + u] = i + __shfl_sync(0xffffffffu, offset, t & 31);
+            index[k + u] = 0;
+#pragma unroll
+            for (int d = 0; d < D; ++d) p[u][d] = INFINITY;    // too far away for any sample
+            if (i < candidates) load_point<D>(c, at[k + u], p[u], &index[k + u]);
+          }
+#pragma unroll
+          for (int d = 0; d < D; ++d) np[d][k / 2] = pack2(-p[0][d], -p[1][d]);
+        }
+        const int steps = (min(candidates - base, 32 * kSteps) + 31) >> 5;
+        for (unsigned todo = members; todo; todo &= todo - 1u) {
+          const int who = __ffs(todo) - 1;
+          f32x2 sp[D];
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const float x = __shfl_sync(0xffffffffu, s.p[d], who);
+            sp[d] = pack2(x, x);
+          }
+          int n_hit = 0, id = 0, begin = 0;
+          float acc = 0.0f;
+          if (MODE == kFill) {
+            n_hit = __shfl_sync(0xffffffffu, my_count, who);
+            id = __shfl_sync(0xffffffffu, s.id, who);
+            begin = __shfl_sync(0xffffffffu, my_begin, who);
+          }
+#pragma unroll
+          for (int k = 0; k < kSteps; k += 2) {
+            if (k < steps) {
+              f32x2 t2[D], d2;
+#pragma unroll
+              for (int d = 0; d < D; ++d) {
+                t2[d] = mul2(add2(sp[d], np[d][k / 2]), inv_r[d]);
+                d2 = d == 0 ? mul2(t2[d], t2[d]) : fma2(t2[d], t2[d], d2);
+              }
+              float dist[2], e[2];
+              unpack2(d2, dist[0], dist[1]);
+              if (MODE == kDensity) {
+                if (isotropic) {
+                  e[0] = dist[0] * scale[0];
+                  e[1] = dist[1] * scale[0];
+                } else {
+                  e[0] = e[1] = 0.0f;
+#pragma unroll
+                  for (int d = 0; d < D; ++d) {
+                    float ta, tb;
+                    unpack2(t2[d], ta, tb);
+                    e[0] = fmaf(ta * ta, scale[d], e[0]);
+                    e[1] = fmaf(tb * tb, scale[d], e[1]);
+                  }
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                const bool hit = dist[u] < 1.0f;
+                if (MODE == kCount) n_hit += hit;
+                if (MODE == kFill) {
+                  const unsigned m = __ballot_sync(0xffffffffu, hit);
+                  if (hit) {
+                    const int pos = n_hit + __popc(m & ((1u << lane) - 1u));
+                    if (pos < a.limit) {
+                      a.neigh[(int64_t)begin + pos] = make_int2(at[k + u], id);
+                      if (a.ids) a.ids[(int64_t)begin + pos] = make_int2(index[k + u], id);
+                    }
+                  }
+                  n_hit += __popc(m);
+                }
+                if (MODE == kDensity) acc += hit ? exp2_approx(e[u]) : 0.0f;
+              }
+            }
+          }
+          if (MODE == kCount) {
+            n_hit = __reduce_add_sync(0xffffffffu, n_hit);
+            if (lane == who) my_count += n_hit;
+          }
+          if (MODE == kFill && lane == who) my_count = n_hit;
+          if (MODE == kDensity) {
+            acc = warp_sum(acc);
+            if (lane == who) my_density += acc;
+          }
+        }
+      }
+    }
+  }
+  if (MODE == kCount && s.id >= 0) a.counts[s.id] = min(my_count, a.limit);
+  if (MODE == kDensity && s.id >= 0) a.density[s.id] = my_density * norm;
+}
+
+// Samples per warp: more of them share the candidates of a cell (a cell of a uniform
+// cloud holds seven points), fewer spread dense regions over the SMs.  Fill pass at
+// 32 / 16 / 8 / 4: 176 / 177 / 192 / 231 us on uniform clouds with 32 neighbors, 776 /
+// 662 / 635 / 683 us on surfaces with 280; below 32 warps per SM it is the number of
+// warps that decides.
+int samples_per_warp(int64_t ns) {
+  const int64_t s = ns / ((int64_t)sm_count() * 32);
+  return (int)(s < 1 ? 1 : s > kMaxSpan ? kMaxSpan : s);
+}
+
+template <int MODE>
+int launch_walk(cudaStream_t st, const char* name, int D, WalkArgs a) {
+  a.span = samples_per_warp(a.ns);
+  const int64_t warps = (a.ns + a.span - 1) / a.span;
+  ProfScope prof(st, name);
+  TFGPC_DIM_SWITCH(D, cells_walk_kernel<kD, MODE>
+                          <<<blocks_for(warps, kThreads / 32), kThreads, 0, st>>>(a));
+  TFGPC_LAUNCH_CHECK();
+  return TFGPC_OK;
+}
+
+WalkArgs walk_args(const tfgpc_cell_grid& g, const SampleSource& src, int64_t ns,
+                   const float* inv_radii, int max_neighs) {
+  WalkArgs a{};
+  a.c = view_of(g);
+  a.src = src;
+  a.ns = ns;
+  a.inv_radii = inv_radii;
+  a.limit = max_neighs > 0 ? max_neighs : INT32_MAX;
+  return a;
+}
+
+int check_grid(const char* op, const tfgpc_cell_grid* g) {
+  TFGPC_REQUIRE(g != nullptr, "%s got a null grid", op);
+  TFGPC_REQUIRE(valid_dims(g->D), "%s expects a valid number of dimension (got %d)", op, g->D);
+  TFGPC_REQUIRE(g->n > 0 && g->n < (int64_t)INT32_MAX && g->batch_size > 0 &&
+                g->batch_size < (int64_t)INT32_MAX,
+                "%s expects 0 < n, 0 < batch size, both below 2^31", op);
+  TFGPC_REQUIRE(g->max_cells >= 1 && table_cells(g->D, g->batch_size, g->max_cells) > 0,
+                "%s expects a grid whose cell table is small enough (tfgpc_cell_table_elems)", op);
+  TFGPC_REQUIRE(g->aabb_min && g->aabb_max && g->num_cells && g->scaled_aabb_min &&
+                g->inv_cell_sizes && g->keys && g->sorted_indices && g->sorted_keys &&
+                g->sorted_points && g->sorted_batch_ids && (g->D > 3 || g->packed) &&
+                g->cell_start && g->ds, "%s got a null pointer", op);
+  TFGPC_REQUIRE((uintptr_t)g->packed % 16 == 0, "%s expects a 16-byte aligned packed table", op);
+  return TFGPC_OK;
+}
+
+int check_samples(const char* op, const tfgpc_cell_grid* g, int64_t ns, const float* samples,
+                  const int32_t* sbatch, int mode, int max_neighs) {
+  TFGPC_REQUIRE(ns >= 0 && ns < (int64_t)INT32_MAX && max_neighs >= 0,
+                "%s expects 0 <= ns < 2^31 and max_neighs >= 0", op);
+  TFGPC_REQUIRE(mode >= 0 && mode <= 2, "%s expects samples_are_points 0, 1 or 2", op);
+  TFGPC_REQUIRE(mode != 0 || ns == 0 || (samples && sbatch), "%s got a null pointer", op);
+  TFGPC_REQUIRE(mode == 0 || ns == g->n || ns == 0,
+                "%s expects as many samples as points when the samples are the points", op);
+  return TFGPC_OK;
+}
+
+// Counts and their scan; the total goes to `total` and to the report page.
+int count_and_scan(cudaStream_t st, const tfgpc_cell_grid& g, const float* inv_radii, int64_t ns,
+                   const SampleSource& src, int max_neighs, int32_t* ranges, int64_t* sums,
+                   int64_t* total, int32_t* page) {
+  WalkArgs a = walk_args(g, src, ns, inv_radii, max_neighs);
+  a.counts = ranges;
+  int rc = launch_walk<kCount>(st, "find_neighbors_count", g.D, a);
+  if (rc) return rc;
+  ScanReport rep;
+  rep.dst = page + kReportTotal;
+  return inclusive_scan_i32(st, ranges, ranges, ns, sums, total, rep);
+}
+
+// Waits for the report and turns it into the outputs of a blocking entry.
+int finish_report(cudaStream_t st, int D, int max_cells, bool with_total,
+                  int32_t* num_cells_host_out, int64_t* total_out) {
+  int32_t host[kReportWords];
+  int rc = read_report(st, sizeof(host), host);
+  if (rc) return rc;
+  for (int d = 0; num_cells_host_out && d < D; ++d) num_cells_host_out[d] = host[d];
+  if (num_cells_host_out && host[TFGPC_MAX_DIMS])
+    return fail(TFGPC_ENOMEM, "GridNeighborhood: the grid needs more than max_cells = %d cells in "
+                "a dimension; repeat the call with a larger bound", max_cells);
+  if (!with_total) return TFGPC_OK;
+  const int64_t total = (int64_t)(uint32_t)host[kReportTotal] |
+                        ((int64_t)host[kReportTotal + 1] << 32);
+  if (total > (int64_t)INT32_MAX)
+    return fail(TFGPC_EINVAL, "FindNeighbors found %lld pairs; the int32 ranges of the op "
+                "contract hold at most 2^31-1", (long long)total);
+  *total_out = total;
+  return TFGPC_OK;
+}
+
+}  // namespace
+}  // namespace tfgpc
+
+using namespace tfgpc;
+
+extern "C" size_t tfgpc_cell_table_elems(int D, int64_t batch_size, int max_cells) {
+  if (!valid_dims(D) || batch_size <= 0 || max_cells <= 0) return 0;
+  const int64_t cells = table_cells(D, batch_size, max_cells);
+  return cells > 0 ? (size_t)cells + 3 : 0;
+}
+
+extern "C" size_t tfgpc_cell_grid_workspace_bytes(int D, int64_t n, int64_t ns, int64_t batch_size,
+                                                  int max_cells) {
+  if (!valid_dims(D) || n < 0 || ns < 0 || batch_size <= 0 || max_cells <= 0) return 0;
+  return carve_cell_grid(nullptr, n, ns, D, batch_size, max_cells).bytes + 256;
+}
+
+extern "C" int tfgpc_cell_grid_neighborhood(
+    void* stream, const tfgpc_cell_grid* grid, const float* points, const int32_t* batch_ids,
+    const float* cell_sizes, const int32_t* num_cells_in, const float* inv_radii, int64_t ns,
+    const float* samples, const int32_t* samples_batch_ids, int samples_are_points,
+    int max_neighs, int32_t* ranges_out, void* ws, size_t ws_bytes, int32_t* num_cells_host_out,
+    int64_t* total_out) {
+  int rc = check_grid("GridNeighborhood", grid);
+  if (rc) return rc;
+  const tfgpc_cell_grid& g = *grid;
+  rc = check_samples("GridNeighborhood", grid, ns, samples, samples_batch_ids,
+                     samples_are_points, max_neighs);
+  if (rc) return rc;
+  TFGPC_REQUIRE(points && batch_ids && cell_sizes && ws && num_cells_host_out && total_out &&
+                (ns == 0 || (ranges_out && inv_radii)), "GridNeighborhood got a null pointer");
+  TFGPC_REQUIRE(num_cells_in != g.num_cells,
+                "GridNeighborhood expects the given cell counts outside the output array");
+  for (int d = 0; d < g.D; ++d)
+    TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "GridNeighborhood expects positive cell sizes");
+  if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, ns, g.batch_size, g.max_cells))
+    return fail(TFGPC_ENOMEM, "GridNeighborhood workspace too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  CellGridWs w = carve_cell_grid(ws, g.n, ns, g.D, g.batch_size, g.max_cells);
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  *total_out = 0;
+  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page);
+  if (rc) return rc;
+  if (ns > 0) {
+    rc = count_and_scan(st, g, inv_radii, ns,
+                        SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
+                        ranges_out, w.sums, w.total, (int32_t*)page);
+    if (rc) return rc;
+  }
+  return finish_report(st, g.D, g.max_cells, ns > 0, num_cells_host_out, total_out);
+}
+
+extern "C" int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid, const float* inv_radii,
+                                 int64_t ns, const float* samples,
+                                 const int32_t* samples_batch_ids, int samples_are_points,
+                                 int max_neighs, int32_t* ranges_out, void* ws, size_t ws_bytes,
+                                 int64_t* total_out) {
+  int rc = check_grid("FindNeighbors", grid);
+  if (rc) return rc;
+  rc = check_samples("FindNeighbors", grid, ns, samples, samples_batch_ids, samples_are_points,
+                     max_neighs);
+  if (rc) return rc;
+  TFGPC_REQUIRE(total_out, "FindNeighbors got a null pointer");
+  *total_out = 0;
+  if (ns == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(inv_radii && ranges_out && ws, "FindNeighbors got a null pointer");
+  if (ws_bytes < tfgpc_find_neighbors_workspace_bytes(ns))
+    return fail(TFGPC_ENOMEM, "FindNeighbors workspace too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  int64_t* sums = (int64_t*)ws;
+  rc = count_and_scan(st, *grid, inv_radii, ns,
+                      SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
+                      ranges_out, sums, sums + scan_block_sums_elems(ns), (int32_t*)page);
+  if (rc) return rc;
+  return finish_report(st, grid->D, grid->max_cells, true, nullptr, total_out);
+}
+
+extern "C" int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid, const float* inv_radii,
+                                int64_t ns, const float* samples,
+                                const int32_t* samples_batch_ids, int samples_are_points,
+                                int max_neighs, const int32_t* ranges, int64_t total,
+                                int32_t* neigh_out, int32_t* ids_out) {
+  int rc = check_grid("FindNeighbors", grid);
+  if (rc) return rc;
+  rc = check_samples("FindNeighbors", grid, ns, samples, samples_batch_ids, samples_are_points,
+                     max_neighs);
+  if (rc) return rc;
+  TFGPC_REQUIRE(total >= 0 && total <= (int64_t)INT32_MAX, "FindNeighbors expects 0 <= total < 2^31");
+  if (ns == 0 || total == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(inv_radii && ranges && neigh_out, "FindNeighbors got a null pointer");
+  WalkArgs a = walk_args(*grid, SampleSource{samples_are_points, samples, samples_batch_ids}, ns,
+                         inv_radii, max_neighs);
+  a.ranges = ranges;
+  a.neigh = (int2*)neigh_out;
+  a.ids = (int2*)ids_out;
+  return launch_walk<kFill>((cudaStream_t)stream,
+                            ids_out ? "find_neighbors_fill_fused" : "find_neighbors_fill",
+                            grid->D, a);
+}
+
+extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
+                                   const float* inv_radii, const float* inv_bandwidth, int mode,
+                                   int64_t ns, const float* samples,
+                                   const int32_t* samples_batch_ids, int samples_are_points,
+                                   float* pdf_out) {
+  int rc = check_grid("ComputePdf", grid);
+  if (rc) return rc;
+  rc = check_samples("ComputePdf", grid, ns, samples, samples_batch_ids, samples_are_points, 0);
+  if (rc) return rc;
+  TFGPC_REQUIRE(mode == 0 || mode == 1, "ComputePdf expects mode 0 or 1 (got %d)", mode);
+  if (ns == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(inv_radii && pdf_out && (mode == 1 || inv_bandwidth), "ComputePdf got a null pointer");
+  WalkArgs a = walk_args(*grid, SampleSource{samples_are_points, samples, samples_batch_ids}, ns,
+                         inv_radii, 0);
+  a.inv_bw = inv_bandwidth;
+  a.bw_mode = mode;
+  a.density = pdf_out;
+  return launch_walk<kDensity>((cudaStream_t)stream, "compute_pdf", grid->D, a);
+}

@@ -71,6 +71,11 @@ int sm_count();
 // not queue behind bulk transfers on other streams.
 int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_dst);
 
+// The same page for kernels that deliver their results themselves: its device address
+// and, once `st` has been synchronised, its contents on the host.
+int report_page(void** dev_page);
+int read_report(cudaStream_t st, size_t bytes, void* host_dst);
+
 inline unsigned blocks_for(int64_t work, int per_block) {
   int64_t b = (work + per_block - 1) / per_block;
   return (unsigned)(b < 1 ? 1 : b);
@@ -136,13 +141,5 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-
-// ---- device-wide inclusive scan of int32 (scan.cu) -------------------------
-// out[i] = sum_{j<=i} in[i] (int32, as the reference's ranges are), and the
-// 64-bit total is written to *total (device).  `in` may alias `out`.
-// block_sums needs scan_block_sums_elems(n) int64 elements.
-int64_t scan_block_sums_elems(int64_t n);
-int inclusive_scan_i32(cudaStream_t stream, const int32_t* in, int32_t* out,
-                       int64_t n, int64_t* block_sums, int64_t* total);
 
 }  // namespace tfgpc

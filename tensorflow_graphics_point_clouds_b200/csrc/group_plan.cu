@@ -23,12 +23,9 @@
 //   scratch of the scan
 // Groups whose pair count exceeds kMaxMerge are not merged (one row per pair).
 #include "group_plan.cuh"
+#include "scan.cuh"
 
 namespace tfgpc {
-
-int64_t scan_block_sums_elems(int64_t n);
-int inclusive_scan_i32(cudaStream_t stream, const int32_t* in, int32_t* out, int64_t n,
-                       int64_t* block_sums, int64_t* total);
 
 namespace gp {
 

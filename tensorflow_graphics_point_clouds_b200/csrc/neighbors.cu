@@ -14,6 +14,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "scan.cuh"
 
 namespace tfgpc {
 

@@ -13,6 +13,7 @@
 // The taken points are then compacted in ascending index with a scan (the
 // reference: atomicAdd, store_sampled_pts_kernels.cu.cc:42-69).
 #include "common.cuh"
+#include "scan.cuh"
 
 namespace tfgpc {
 

@@ -80,9 +80,7 @@ __global__ void mailbox_kernel(const uint32_t* __restrict__ src, uint32_t* dst, 
 
 }  // namespace
 
-int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_dst) {
-  TFGPC_REQUIRE(bytes > 0 && bytes <= 4096 && bytes % 4 == 0 && (uintptr_t)dev_src % 4 == 0,
-                "read_small expects 4 .. 4096 bytes, a multiple of 4");
+static int mailbox_of(Mailbox** out) {
   int dev = 0;
   TFGPC_CUDA(cudaGetDevice(&dev));
   TFGPC_REQUIRE(dev >= 0 && dev < 64, "read_small: device index out of range");
@@ -91,11 +89,36 @@ int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_ds
     TFGPC_CUDA(cudaHostAlloc(&m.host, 4096, cudaHostAllocMapped));
     TFGPC_CUDA(cudaHostGetDevicePointer(&m.dev, m.host, 0));
   }
-  mailbox_kernel<<<1, 32, 0, st>>>((const uint32_t*)dev_src, (uint32_t*)m.dev, (int)(bytes / 4));
-  TFGPC_LAUNCH_CHECK();
-  TFGPC_CUDA(cudaStreamSynchronize(st));
-  memcpy(host_dst, m.host, bytes);
+  *out = &m;
   return TFGPC_OK;
+}
+
+int report_page(void** dev_page) {
+  Mailbox* m = nullptr;
+  int rc = mailbox_of(&m);
+  if (rc) return rc;
+  *dev_page = m->dev;
+  return TFGPC_OK;
+}
+
+int read_report(cudaStream_t st, size_t bytes, void* host_dst) {
+  Mailbox* m = nullptr;
+  int rc = mailbox_of(&m);
+  if (rc) return rc;
+  TFGPC_CUDA(cudaStreamSynchronize(st));
+  memcpy(host_dst, m->host, bytes);
+  return TFGPC_OK;
+}
+
+int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_dst) {
+  TFGPC_REQUIRE(bytes > 0 && bytes <= 4096 && bytes % 4 == 0 && (uintptr_t)dev_src % 4 == 0,
+                "read_small expects 4 .. 4096 bytes, a multiple of 4");
+  void* page = nullptr;
+  int rc = report_page(&page);
+  if (rc) return rc;
+  mailbox_kernel<<<1, 32, 0, st>>>((const uint32_t*)dev_src, (uint32_t*)page, (int)(bytes / 4));
+  TFGPC_LAUNCH_CHECK();
+  return read_report(st, bytes, host_dst);
 }
 
 }  // namespace tfgpc

@@ -12,6 +12,7 @@ expressions of the reference one to one, and the ops themselves run through
 `custom_ops` (the C ABI).
 """
 import math
+import types
 
 import torch
 
@@ -28,22 +29,32 @@ SAMPLE_MODES = {'average': 1, 'cell average': 1, 'cell_average': 1,
 _DIMS_CACHE = {}
 
 
-def _to_dims(value, dims, device):
+def _to_dims(value, dims, device, inverse=False):
+  """value per dimension as a device tensor, or (inverse) its float32 reciprocal."""
   if not torch.is_tensor(value):
     flat = [float(v) for v in (value if hasattr(value, '__len__') else [value])]
-    key = (tuple(flat), dims, str(device))
+    key = (tuple(flat), dims, device, inverse)
     t = _DIMS_CACHE.get(key)
     if t is None:
       if len(_DIMS_CACHE) > 256:
         _DIMS_CACHE.clear()
-      t = torch.tensor(flat * dims if len(flat) == 1 else flat, dtype=torch.float32,
-                       device=device)
+      t = torch.tensor(flat * dims if len(flat) == 1 else flat, dtype=torch.float32)
+      t = (torch.reciprocal(t) if inverse else t).to(device)
       _DIMS_CACHE[key] = t
     return t
+  if inverse:
+    return torch.reciprocal(_to_dims(value, dims, device))
   t = torch.as_tensor(value, dtype=torch.float32, device=device).reshape(-1)
   if t.shape[0] == 1:
     t = t.repeat(dims)
   return t
+
+
+def _host_dims(value, dims):
+  """value per dimension as a list of floats (a device tensor costs a blocking read)."""
+  flat = (value.detach().reshape(-1).cpu().tolist() if torch.is_tensor(value) else
+          [float(v) for v in (value if hasattr(value, '__len__') else [value])])
+  return flat * dims if len(flat) == 1 else flat
 
 
 class PointCloud:
@@ -73,21 +84,80 @@ class PointCloud:
     return self._aabb
 
 
+# Upper bound of cells per dimension that a grid's cell table, tube array and sort keys
+# are sized for, per (dimension, batch size): it starts at _FIRST_BOUND and is raised to
+# what a grid asked for when one did not fit.
+_MAX_CELLS = {}
+_FIRST_BOUND = 16
+_ONE_CALL_CELLS_LIMIT = 1024
+
+
+def _raise_bound(pc, err, max_cells):
+  """The bound to repeat a call with that reported too few cells, or None if a
+  grid this fine would make the fixed-size arrays too large; other errors pass."""
+  asked = max(getattr(err, 'num_cells', [0]))
+  if err.code != 3 or asked <= max_cells:
+    raise err
+  bigger = 1 << (asked - 1).bit_length()
+  if bigger > _ONE_CALL_CELLS_LIMIT or pc._batch_size * float(bigger) ** pc._dimension >= 4e18:
+    return None
+  _MAX_CELLS[(pc._dimension, pc._batch_size)] = bigger
+  return bigger
+
+
+def _reduced_cells(pc, sizes):
+  """Boxes and cell counts of one shard of a distributed batch, the counts reduced
+  over the ranks on the device; None for a cloud that is not a shard.  (The reduced
+  counts are the same on every rank, so every rank takes the same turns after it.)"""
+  if pc._num_cells_reduce is None:
+    return None
+  cells = ops.grid_cells(pc._points, pc._batch_ids, pc._batch_size, sizes, sizes)
+  cells["num_cells"] = pc._num_cells_reduce(cells["num_cells"]).to(torch.int32)
+  return cells
+
+
+def _cell_grid(pc, sizes, cells, **neighborhood):
+  """(ops.CellGrid of a cloud, count of the neighborhood if one is given), or (None,
+  None) if its cell table would be too large."""
+  d, b = pc._dimension, pc._batch_size
+  max_cells = _MAX_CELLS.get((d, b), _FIRST_BOUND)
+  while max_cells and ops.cell_table_elems(d, b, max_cells):
+    try:
+      return ops.CellGrid.build(pc._points, pc._batch_ids, b, sizes, max_cells, cells=cells,
+                                **neighborhood)
+    except ops._lib.TfgpcError as err:
+      max_cells = _raise_bound(pc, err, max_cells)
+  return None, None
+
+
 class Grid:
-  """Grid.py:32-83: keys, descending sort, sorted copies, lazy tube ranges."""
+  """Grid.py:32-83: keys, descending sort, sorted copies, tube ranges.  Built through
+  a cell table (ops.CellGrid) unless the grid is too fine for one."""
 
   def __init__(self, point_cloud, cell_sizes):
     pc = point_cloud
     dev = pc._points.device
+    self._cell_sizes = _to_dims(cell_sizes, pc._dimension, dev)
+    cells = None
+    if pc._points.shape[0] > 0:
+      sizes = _host_dims(cell_sizes, pc._dimension)
+      cells = _reduced_cells(pc, sizes)
+      table, _ = _cell_grid(pc, sizes, cells)
+      if table is not None:
+        self._adopt(pc, table)
+        return
+    self._cells = None
     self._point_cloud = pc
     self._batch_size = pc._batch_size
-    self._cell_sizes = _to_dims(cell_sizes, pc._dimension, dev)
     self._aabb_min, self._aabb_max = pc.get_AABB()
     sizes = self._aabb_max - self._aabb_min
-    batch_num_cells = torch.ceil(sizes / self._cell_sizes).to(torch.int32)
-    self._num_cells = torch.clamp(batch_num_cells.max(dim=0).values, min=1).to(torch.int32)
-    if pc._num_cells_reduce is not None:
-      self._num_cells = pc._num_cells_reduce(self._num_cells).to(torch.int32)
+    if cells is not None:
+      self._num_cells = cells["num_cells"]
+    else:
+      batch_num_cells = torch.ceil(sizes / self._cell_sizes).to(torch.int32)
+      self._num_cells = torch.clamp(batch_num_cells.max(dim=0).values, min=1).to(torch.int32)
+      if pc._num_cells_reduce is not None:
+        self._num_cells = pc._num_cells_reduce(self._num_cells).to(torch.int32)
     self._num_cells_host = ops.read_device(self._num_cells)
     # custom_ops_wrapper.py:37-43
     self._scaled_aabb_min = self._aabb_min / self._cell_sizes
@@ -103,6 +173,21 @@ class Grid:
                                                   key_bits=min(64, key_bits))
     self._fast_DS = None
 
+  def _adopt(self, pc, built):
+    """Takes over the arrays of an ops.CellGrid."""
+    self._cells = built
+    self._point_cloud = pc
+    self._batch_size = pc._batch_size
+    self._aabb_min, self._aabb_max = built.aabb_min, built.aabb_max
+    if pc._aabb is None:
+      pc._aabb = (self._aabb_min, self._aabb_max)
+    self._num_cells, self._num_cells_host = built.num_cells, built.num_cells_host
+    self._scaled_aabb_min, self._inv_cell_sizes = built.scaled_aabb_min, built.inv_cell_sizes
+    self._cur_keys = built.keys
+    self._sorted_indices, self._sorted_keys = built.sorted_indices, built.sorted_keys
+    self._sorted_points, self._sorted_batch_ids = built.sorted_points, built.sorted_batch_ids
+    self._fast_DS = built.ds
+
   def get_DS(self):
     if self._fast_DS is None:
       self._fast_DS = ops.build_grid_ds(self._sorted_keys, self._num_cells,
@@ -116,34 +201,40 @@ class Neighborhood:
   it is first asked for, in one pass together with the list in original ids."""
 
   def __init__(self, grid, radius, point_cloud_sample=None, max_neighbors=0):
-    dev = grid._sorted_points.device
-    self._radii = _to_dims(radius, grid._point_cloud._dimension, dev)
-    if point_cloud_sample is None:
-      self._equal_samples = True
-      self._point_cloud_sampled = PointCloud(grid._sorted_points, grid._sorted_batch_ids,
-                                             grid._batch_size)
+    self._attach(grid, radius, point_cloud_sample, max_neighbors)
+    smp = self._point_cloud_sampled
+    if grid._cells is not None:
+      self._take_count(grid._cells.count_neighbors(
+          self._inv_radii, self._sample_mode, smp._points, smp._batch_ids, max_neighbors))
     else:
-      self._equal_samples = False
-      self._point_cloud_sampled = point_cloud_sample
+      self._take_count(ops.find_neighbors_count(
+          smp._points, smp._batch_ids, grid._sorted_points, grid._sorted_keys, grid.get_DS(),
+          grid._num_cells, grid._scaled_aabb_min, grid._inv_cell_sizes, self._inv_radii,
+          max_neighbors, sample_order=self._sample_order))
+
+  def _attach(self, grid, radius, point_cloud_sample, max_neighbors):
+    dev, d = grid._sorted_points.device, grid._point_cloud._dimension
+    self._radius = radius
+    self._radii = _to_dims(radius, d, dev)
+    self._inv_radii = _to_dims(radius, d, dev, inverse=True)
+    self._equal_samples = point_cloud_sample is None
+    self._point_cloud_sampled = (PointCloud(grid._sorted_points, grid._sorted_batch_ids,
+                                            grid._batch_size)
+                                 if point_cloud_sample is None else point_cloud_sample)
+    # 2: the sorted points, 1: the grid's own cloud in its unsorted order, 0: other samples
+    self._sample_mode = (2 if self._equal_samples else
+                         1 if point_cloud_sample is grid._point_cloud else 0)
     self._grid = grid
     self.max_neighbors = max_neighbors
-    smp = self._point_cloud_sampled
-    # samples that are the grid's own cloud in its unsorted order: the key sort's
-    # permutation lists them cell by cell, the sequence the search is fastest in
-    order = grid._sorted_indices if smp is grid._point_cloud else None
-    # a sequence that visits the samples cell by cell, where one is known (the
-    # samples of a self neighborhood are the sorted points: already in it)
-    self._sample_order = order
-    self._count = ops.find_neighbors_count(
-        smp._points, smp._batch_ids, grid._sorted_points, grid._sorted_keys, grid.get_DS(),
-        grid._num_cells, grid._scaled_aabb_min, grid._inv_cell_sizes,
-        torch.reciprocal(self._radii), max_neighbors, sample_order=order)
-    self._samples_neigh_ranges = self._count.ranges
-    self._nbrs = None
-    self._orig_ids = None
-    self._pdf = None
-    self._point_pdf = None
-    self._sample_pdf = None
+    # a sequence that visits the samples cell by cell, where one is known: for the
+    # grid's own cloud the key sort's permutation (the samples of a self
+    # neighborhood are the sorted points: already in it)
+    self._sample_order = grid._sorted_indices if self._sample_mode == 1 else None
+
+  def _take_count(self, count):
+    self._count = count
+    self._samples_neigh_ranges = count.ranges
+    self._nbrs = self._orig_ids = self._pdf = self._point_pdf = self._sample_pdf = None
     self._pdf_ready = False
     self._transposed = None
 
@@ -188,11 +279,16 @@ class Neighborhood:
     grid's own cloud that second search is skipped: the density at sample s is
     the density of the point it coincides with."""
     d = self._point_cloud_sampled._dimension
-    bw = _to_dims(bandwidth, d, self._radii.device)
-    inv_bw, inv_r = torch.reciprocal(bw), torch.reciprocal(self._radii)
+    inv_bw, inv_r = _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii
     g = self._grid
     self._pdf = None
-    if self._equal_samples:
+    if g._cells is not None and not (self._equal_samples and self.max_neighbors > 0):
+      # straight from the grid, without the list of a self neighborhood
+      if self._sample_mode == 1 and self.max_neighbors == 0:
+        self._sample_pdf, self._point_pdf = g._cells.density(inv_r, inv_bw, mode, 1), None
+      else:
+        self._point_pdf = g._cells.density(inv_r, inv_bw, mode, 2)
+    elif self._equal_samples:
       self._point_pdf = ops.compute_pdf_with_pt_grads(
           g._sorted_points, self._neighbors, self._samples_neigh_ranges, inv_bw, inv_r, mode)
     elif self._samples_are_grid_points():
@@ -202,7 +298,7 @@ class Neighborhood:
           self._samples_neigh_ranges, inv_bw, inv_r, mode)
       self._point_pdf = None
     else:
-      nb = Neighborhood(g, self._radii)
+      nb = Neighborhood(g, self._radius)
       self._point_pdf = ops.compute_pdf_with_pt_grads(
           g._sorted_points, nb._neighbors, nb._samples_neigh_ranges, inv_bw, inv_r, mode)
     self._pdf_ready = True
@@ -232,8 +328,8 @@ class Neighborhood:
       if self._equal_samples:
         self._transposed = self
       else:
-        grid = Grid(self._point_cloud_sampled, self._radii)
-        self._transposed = Neighborhood(grid, self._radii, self._grid._point_cloud)
+        grid = Grid(self._point_cloud_sampled, self._radius)
+        self._transposed = Neighborhood(grid, self._radius, self._grid._point_cloud)
     return self._transposed
 
   def get_pdf(self, **kwargs):
@@ -261,103 +357,59 @@ class Neighborhood:
     per_point = torch.zeros(n, dtype=torch.float32, device=g._sorted_points.device)
     per_point.index_add_(0, self._neighbors[:, 0].to(torch.int64),
                          torch.as_tensor(pdf_grads, dtype=torch.float32))
-    nb = self if self._equal_samples else Neighborhood(g, self._radii)
-    bw = _to_dims(bandwidth, d, self._radii.device)
+    nb = self if self._equal_samples else Neighborhood(g, self._radius)
     grads_sorted = ops.compute_pdf_pt_grads(
-        g._sorted_points, nb._neighbors, nb._samples_neigh_ranges, torch.reciprocal(bw),
-        torch.reciprocal(self._radii), per_point, mode)
+        g._sorted_points, nb._neighbors, nb._samples_neigh_ranges,
+        _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii, per_point, mode)
     out = torch.empty_like(grads_sorted)
     out[g._sorted_indices.to(torch.int64)] = grads_sorted
     return out
 
 
-# Upper bound of cells per dimension that grid_neighborhood sizes its tube array
-# and sort keys for, per (dimension, batch size): it starts at 64 and is raised
-# to what a grid asked for when one did not fit.
-_MAX_CELLS = {}
-_ONE_CALL_CELLS_LIMIT = 1024
-
-
 def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbors=0):
   """Grid(point_cloud, radius) and Neighborhood(grid, radius, point_cloud_sample,
-  max_neighbors) built by ONE library call with ONE blocking read
-  (tfgpc_grid_neighborhood_count) where pylib's two constructors read back twice
-  (Grid.py:44-48 cell counts, Neighborhood.py:242-245 pair count).  Same objects,
-  same contents.  For a cloud that is one shard of a distributed batch
-  (num_cells_reduce set) the cell counts are reduced over the ranks on the device,
-  between tfgpc_grid_cells and the main call: still one blocking read."""
+  max_neighbors) built by ONE library call with ONE blocking read where pylib's two
+  constructors read back twice (Grid.py:44-48 cell counts, Neighborhood.py:242-245 pair
+  count).  Same objects, same contents: on the cell table (ops.CellGrid), or by keys
+  (tfgpc_grid_neighborhood_count) for grids too fine for one.  For a cloud that is one
+  shard of a distributed batch (num_cells_reduce set) the cell counts are reduced
+  over the ranks on the device, before the main call: still one blocking read."""
   pc = point_cloud
   if pc._points.shape[0] == 0:
     return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
   dev = pc._points.device
   d = pc._dimension
-  radii = _to_dims(radius, d, dev)
-  # (a radius given as a device tensor costs a read of its own)
-  radii_host = (radius.detach().reshape(-1).cpu().tolist() if torch.is_tensor(radius) else
-                [float(v) for v in (radius if hasattr(radius, '__len__') else [radius])])
-  if len(radii_host) == 1:
-    radii_host = radii_host * d
-  if point_cloud_sample is None:
-    mode, smp = 2, None
-  elif point_cloud_sample is pc:
-    mode, smp = 1, None
-  else:
-    mode, smp = 0, point_cloud_sample
-  key = (d, pc._batch_size)
-  max_cells = _MAX_CELLS.get(key, 64)
-  cells = None
-  if pc._num_cells_reduce is not None:
-    # (the reduced counts are the same on every rank, so every rank takes the same
-    # turns through the loop below; the reduction itself happens once)
-    cells = ops.grid_cells(pc._points, pc._batch_ids, pc._batch_size, radii_host, radii_host)
-    cells["num_cells"] = pc._num_cells_reduce(cells["num_cells"]).to(torch.int32)
-  while True:
-    try:
-      g = ops.grid_neighborhood_count(
-          pc._points, pc._batch_ids, pc._batch_size, radii_host, radii_host, max_cells,
-          None if smp is None else smp._points, None if smp is None else smp._batch_ids,
-          mode, max_neighbors, cells=cells)
-      break
-    except ops._lib.TfgpcError as err:
-      asked = max(getattr(err, 'num_cells', [0]))
-      if err.code != 3 or asked <= max_cells:
-        raise
-      bigger = 1 << (asked - 1).bit_length()
-      if bigger > _ONE_CALL_CELLS_LIMIT or pc._batch_size * float(bigger) ** d >= 4e18:
-        # a grid this fine would make the call's fixed-size tube array (or its sort
-        # keys) too large: the separate constructors size both exactly
-        return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
-      max_cells = bigger
-      _MAX_CELLS[key] = max_cells
+  sizes = _host_dims(radius, d)
+  mode = 2 if point_cloud_sample is None else 1 if point_cloud_sample is pc else 0
+  smp = point_cloud_sample if mode == 0 else None
+  samples = dict(samples=None if smp is None else smp._points,
+                 samples_batch_ids=None if smp is None else smp._batch_ids,
+                 samples_are_points=mode, max_neighs=max_neighbors)
+  cells = _reduced_cells(pc, sizes)
+  table, count = _cell_grid(pc, sizes, cells, inv_radii=_to_dims(radius, d, dev, inverse=True),
+                            **samples)
   grid = object.__new__(Grid)
-  grid._point_cloud = pc
-  grid._batch_size = pc._batch_size
-  grid._cell_sizes = radii
-  grid._aabb_min, grid._aabb_max = g["aabb_min"], g["aabb_max"]
-  if pc._aabb is None:
-    pc._aabb = (grid._aabb_min, grid._aabb_max)
-  grid._num_cells = g["num_cells"]
-  grid._num_cells_host = g["num_cells_host"]
-  grid._scaled_aabb_min = g["scaled_aabb_min"]
-  grid._inv_cell_sizes = g["inv_cell_sizes"]
-  grid._cur_keys = g["keys"]
-  grid._sorted_indices, grid._sorted_keys = g["sorted_indices"], g["sorted_keys"]
-  grid._sorted_points, grid._sorted_batch_ids = g["sorted_points"], g["sorted_batch_ids"]
-  grid._fast_DS = g["ds"]
+  grid._cell_sizes = _to_dims(radius, d, dev)
+  if table is not None:
+    grid._adopt(pc, table)
+  else:
+    max_cells = _MAX_CELLS.get((d, pc._batch_size), _FIRST_BOUND)
+    while True:
+      try:
+        g = ops.grid_neighborhood_count(pc._points, pc._batch_ids, pc._batch_size, sizes, sizes,
+                                        max_cells, cells=cells, **samples)
+        break
+      except ops._lib.TfgpcError as err:
+        max_cells = _raise_bound(pc, err, max_cells)
+        if max_cells is None:
+          # the separate constructors size the tube array and the sort keys exactly
+          return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
+    grid._adopt(pc, types.SimpleNamespace(**g))
+    grid._cells = None
+    count = g["count"]
   nb = object.__new__(Neighborhood)
-  nb._radii = radii
-  nb._equal_samples = point_cloud_sample is None
-  nb._point_cloud_sampled = (PointCloud(grid._sorted_points, grid._sorted_batch_ids,
-                                        grid._batch_size)
-                             if point_cloud_sample is None else point_cloud_sample)
-  nb._grid = grid
-  nb.max_neighbors = max_neighbors
-  nb._sample_order = grid._sorted_indices if mode == 1 else None
-  nb._count = g["count"]
-  nb._samples_neigh_ranges = nb._count.ranges
-  nb._nbrs = nb._orig_ids = nb._pdf = nb._point_pdf = nb._sample_pdf = None
-  nb._pdf_ready = False
-  nb._transposed = None
+  nb._attach(grid, radius, point_cloud_sample, max_neighbors)
+  nb._take_count(count)
   return nb
 
 
