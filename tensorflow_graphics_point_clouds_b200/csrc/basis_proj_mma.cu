@@ -21,50 +21,77 @@ __global__ void split_features_kernel(const float* __restrict__ feat, int64_t n,
   *reinterpret_cast<uint2*>(fs + row * 2 * C + C + c) = m;
 }
 
-constexpr size_t kMaxBlockSmem = 227 * 1024;
+// Blocks of one SM each, and the samples a warp takes at a time: enough work items per
+// warp (four) to even out lists of unequal length, up to the 32 that one load of range
+// ends covers.  (With 32 always, 41 000 samples left 1036 warps one or two blocks each:
+// two waves, the second a quarter full.)
+struct Shape { int grid, bs; };
 
-template <typename Kern>
-int launch_persistent(Kern kern, int warp_bytes, int max_warps, int64_t ns, int* grid_out,
-                      int* threads_out, size_t* smem_out) {
-  int warps = (int)(kMaxBlockSmem / (size_t)warp_bytes);
-  if (warps > max_warps) warps = max_warps;
-  const size_t smem = (size_t)warps * warp_bytes;
-  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int64_t sample_blocks = (ns + 31) / 32;
-  int64_t grid = (sample_blocks + warps - 1) / warps;
-  if (grid > sm_count()) grid = sm_count();
-  if (grid < 1) grid = 1;
-  *grid_out = (int)grid; *threads_out = warps * 32; *smem_out = smem;
-  return TFGPC_OK;
+Shape walk_shape(int64_t items, int warps) {
+  Shape s;
+  int64_t bs = items / ((int64_t)sm_count() * warps * 4);
+  s.bs = (int)(bs < 1 ? 1 : bs > 32 ? 32 : bs);
+  int64_t grid = ((items + s.bs - 1) / s.bs + warps - 1) / warps;
+  s.grid = (int)(grid < 1 ? 1 : grid > sm_count() ? sm_count() : grid);
+  return s;
 }
 
-template <int K, int OUT>
+template <int K, int CC, int OUT>
 int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __nv_bfloat16* fs,
                const int2* neigh, const int32_t* ranges, float* out, __nv_bfloat16* hi,
                __nv_bfloat16* mid) {
-  auto kern = bpm::basis_proj_mma_kernel<K, OUT>;
-  int grid, threads; size_t smem;
-  int rc = launch_persistent(kern, bpm::Cfg<K>::kFwdWarpBytes, 11, ns, &grid, &threads, &smem);
-  if (rc) return rc;
+  typedef bpm::Cfg<K, CC> cfg;
+  auto kern = bpm::basis_proj_mma_kernel<K, CC, OUT>;
+  constexpr int smem = cfg::kFwdWarps * cfg::kFwdWarpBytes;
+  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  Shape s = walk_shape(ns, cfg::kFwdWarps);
+  // few samples: the channel passes run side by side
+  const int passes = (C + CC - 1) / CC;
+  int rows = sm_count() / s.grid;
+  rows = rows < 1 ? 1 : rows > passes ? passes : rows;
   ProfScope prof(st, OUT == 0 ? "basis_proj_mma" : "basis_proj_split_mma");
-  kern<<<grid, threads, smem, st>>>(C, ns, basis, fs, neigh, ranges, out, hi, mid);
+  kern<<<dim3(s.grid, rows), cfg::kFwdWarps * 32, smem, st>>>(s.bs, C, ns, basis, fs, neigh, ranges,
+                                                              out, hi, mid);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
-template <int K>
+template <int K, int CC>
 int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* basis,
                  const __nv_bfloat16* fs, const int2* neigh, const int32_t* ranges,
                  const float* in_grads, float* dbasis, float* dfeat) {
-  auto kern = bpm::basis_proj_grads_mma_kernel<K>;
-  int grid, threads; size_t smem;
-  int rc = launch_persistent(kern, bpm::Cfg<K>::kGradWarpBytes, 7, ns, &grid, &threads, &smem);
-  if (rc) return rc;
+  typedef bpm::Cfg<K, CC> cfg;
+  auto kern = bpm::basis_proj_grads_mma_kernel<K, CC>;
+  constexpr int smem = cfg::kGradWarps * cfg::kGradWarpBytes;
+  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // few samples with long lists: several warps share a sample's chunks
+  const int64_t warps = (int64_t)sm_count() * cfg::kGradWarps;
+  int64_t parts = ns > 0 ? 2 * warps / ns : 1;
+  const int64_t most = ns > 0 ? M / ns / (2 * bpm::kChunk) : 1;
+  if (parts > most) parts = most;
+  if (parts < 1) parts = 1;
+  Shape s = walk_shape(ns * parts, cfg::kGradWarps);
   ProfScope prof(st, "basis_proj_grads_mma");
-  kern<<<grid, threads, smem, st>>>(C, ns, M, basis, fs, neigh, ranges, in_grads, dbasis, dfeat);
+  kern<<<s.grid, cfg::kGradWarps * 32, smem, st>>>(s.bs, (int)parts, C, ns, M, basis, fs, neigh,
+                                                   ranges, in_grads, dbasis, dfeat);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
+
+// Channels per pass: the smallest that takes the layer in one, else the widest.
+#define TFGPC_CC_SWITCH(K, C, ...)                                                    \
+  if (K == 16) {                                                                      \
+    constexpr int kK = 16;                                                            \
+    if (C <= 32) { constexpr int kCC = 32; __VA_ARGS__; }                             \
+    if (C <= 64) { constexpr int kCC = 64; __VA_ARGS__; }                             \
+    { constexpr int kCC = 128; __VA_ARGS__; }                                         \
+  }                                                                                   \
+  if (K == 32) {                                                                      \
+    constexpr int kK = 32;                                                            \
+    if (C <= 32) { constexpr int kCC = 32; __VA_ARGS__; }                             \
+    { constexpr int kCC = 64; __VA_ARGS__; }                                          \
+  }                                                                                   \
+  if (K == 64) { constexpr int kK = 64; constexpr int kCC = 32; __VA_ARGS__; }
 
 }  // namespace
 
@@ -85,12 +112,8 @@ int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bf
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          __nv_bfloat16* hi, __nv_bfloat16* mid) {
-  const int2* nb = (const int2*)neigh;
-  switch (K) {
-    case 16: return launch_fwd<16, 1>(st, C, ns, basis, fs, nb, ranges, nullptr, hi, mid);
-    case 32: return launch_fwd<32, 1>(st, C, ns, basis, fs, nb, ranges, nullptr, hi, mid);
-    case 64: return launch_fwd<64, 1>(st, C, ns, basis, fs, nb, ranges, nullptr, hi, mid);
-  }
+  TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 1>(st, C, ns, basis, fs, (const int2*)neigh,
+                                                      ranges, nullptr, hi, mid))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
@@ -98,24 +121,16 @@ int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float*
 int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                        const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                        float* out) {
-  const int2* nb = (const int2*)neigh;
-  switch (K) {
-    case 16: return launch_fwd<16, 0>(st, C, ns, basis, fs, nb, ranges, out, nullptr, nullptr);
-    case 32: return launch_fwd<32, 0>(st, C, ns, basis, fs, nb, ranges, out, nullptr, nullptr);
-    case 64: return launch_fwd<64, 0>(st, C, ns, basis, fs, nb, ranges, out, nullptr, nullptr);
-  }
+  TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 0>(st, C, ns, basis, fs, (const int2*)neigh,
+                                                      ranges, out, nullptr, nullptr))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          const float* in_grads, float* dbasis, float* dfeat) {
-  const int2* nb = (const int2*)neigh;
-  switch (K) {
-    case 16: return launch_grads<16>(st, C, ns, M, basis, fs, nb, ranges, in_grads, dbasis, dfeat);
-    case 32: return launch_grads<32>(st, C, ns, M, basis, fs, nb, ranges, in_grads, dbasis, dfeat);
-    case 64: return launch_grads<64>(st, C, ns, M, basis, fs, nb, ranges, in_grads, dbasis, dfeat);
-  }
+  TFGPC_CC_SWITCH(K, C, return launch_grads<kK, kCC>(st, C, ns, M, basis, fs, (const int2*)neigh,
+                                                     ranges, in_grads, dbasis, dfeat))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 

@@ -28,10 +28,14 @@ namespace bpm {
 
 constexpr int kChunk = 16;  // pairs per MMA step (the k or m extent of m16n8k16)
 
-template <int K>
+// CC: channels per pass.  A layer narrower than the widest pass takes a smaller one:
+// shared memory and accumulators per warp shrink with it, so that more warps are
+// resident to hide the gathers (C = 64, K = 16: 16 warps per SM instead of 11).
+template <int K, int CC>
 struct Cfg {
   static_assert(K == 16 || K == 32 || K == 64, "MMA projection: K in {16, 32, 64}");
-  static constexpr int kCC = K == 16 ? 128 : (K == 32 ? 64 : 32);  // channels per pass
+  static_assert(CC % 32 == 0 && CC * K <= 2048, "at most 64 accumulators per lane");
+  static constexpr int kCC = CC;
   static constexpr int kMT = kCC / 16;   // 16-channel tiles per pass
   static constexpr int kNT = K / 8;      // 8-wide basis tiles
   static constexpr int kNTP = K / 16;    // tile pairs
@@ -44,6 +48,14 @@ struct Cfg {
   static constexpr int kFwdWarpBytes = 2 * kFeatBytes + 2 * kBasisBytes;
   static constexpr int kGradWarpBytes = kFeatBytes + kBasisBytes + kDxRawBytes + kDxBytes;
   static constexpr int kBasisVecs = K / 8;   // float4 loads per lane for a 16-row basis chunk
+  // warps per block (one block per SM): what 64 K registers and 227 KB allow
+  static constexpr int kFwdRegWarps = CC * K >= 2048 ? 12 : CC * K >= 1024 ? 16 : 24;
+  static constexpr int kGradRegWarps = K == 64 ? 8 : CC * K >= 2048 ? 8 : CC * K >= 1024 ? 12 : 16;
+  static constexpr int kMaxSmem = 227 * 1024;
+  static constexpr int kFwdWarps = kFwdRegWarps < kMaxSmem / kFwdWarpBytes
+                                       ? kFwdRegWarps : kMaxSmem / kFwdWarpBytes;
+  static constexpr int kGradWarps = kGradRegWarps < kMaxSmem / kGradWarpBytes
+                                        ? kGradRegWarps : kMaxSmem / kGradWarpBytes;
 };
 
 // ---- PTX helpers -----------------------------------------------------------------
@@ -99,35 +111,49 @@ __device__ __forceinline__ void cp_wait() {
 
 // ---- the walk over samples ---------------------------------------------------------
 //
-// A warp takes blocks of 32 consecutive samples, strided over all warps of the
-// grid.  The 32 range ends of a block are read with one coalesced load (the
-// next block's are fetched while this one is processed) and handed out by
-// shuffle, so moving from chunk to chunk and sample to sample costs no memory
-// access.  A job is one chunk of up to 16 pairs; a sample without pairs still
-// yields one empty job so that its (zero) result gets written.
+// A warp takes blocks of `bs` (1 to 32) consecutive samples, strided over all warps of
+// the grid; the launcher makes blocks small enough that every warp gets several.  The
+// range ends of a block are read with one coalesced load (the next block's are
+// fetched while this one is processed) and handed out by shuffle, so moving from chunk
+// to chunk and sample to sample costs no memory access.  A job is one chunk of up to
+// 16 pairs; a sample without pairs still yields one empty job so that its (zero) result
+// gets written.  With parts > 1 (gradients, whose pairs are independent) every sample
+// is walked as `parts` items, each a run of its chunks.
 struct Job {
-  int64_t s;     // sample, -1 once the walk is over
+  int64_t s;     // item (sample * parts + part), -1 once the walk is over
   int base;      // first pair of the chunk
   int cnt;       // pairs in the chunk (0 .. 16)
-  bool first, last;  // first / last chunk of the sample
+  bool first, last;  // first / last chunk of the item
   __device__ __forceinline__ bool valid() const { return s >= 0; }
 };
 
 struct Walker {
   const int32_t* ranges;
-  int64_t ns, blk, stride;
-  int lane, li, r_end, a0, nr_end, na0, base, e;
+  int64_t ns, blk, stride;     // ns: items
+  int lane, li, r_end, a0, nr_end, na0, base, e, bs, parts;
   bool started;
 
-  __device__ __forceinline__ void load_block(int64_t b, int& rend, int& first) const {
-    const int64_t s0 = b * 32;
-    rend = (s0 + lane < ns) ? __ldg(ranges + s0 + lane) : 0;
-    first = (s0 > 0 && s0 < ns) ? __ldg(ranges + s0 - 1) : 0;
+  // end of the pairs of item i
+  __device__ __forceinline__ int item_end(int64_t i) const {
+    if (parts == 1) return __ldg(ranges + i);
+    const int64_t s = i / parts;
+    const int p = (int)(i - s * parts) + 1;
+    const int end = __ldg(ranges + s);
+    if (p == parts) return end;
+    const int begin = s > 0 ? __ldg(ranges + s - 1) : 0;
+    const int chunks = (end - begin + kChunk - 1) / kChunk;
+    return min(end, begin + chunks * p / parts * kChunk);
   }
 
-  __device__ __forceinline__ void init(const int32_t* r, int64_t n, int64_t warp, int64_t warps,
-                                       int ln) {
-    ranges = r; ns = n; blk = warp; stride = warps; lane = ln;
+  __device__ __forceinline__ void load_block(int64_t b, int& rend, int& first) const {
+    const int64_t s0 = b * bs;
+    rend = (lane < bs && s0 + lane < ns) ? item_end(s0 + lane) : 0;
+    first = (s0 > 0 && s0 < ns) ? item_end(s0 - 1) : 0;
+  }
+
+  __device__ __forceinline__ void init(const int32_t* r, int64_t items, int64_t warp,
+                                       int64_t warps, int ln, int block, int part_count) {
+    ranges = r; ns = items; blk = warp; stride = warps; lane = ln; bs = block; parts = part_count;
     li = 0; base = 0; e = 0; started = false;
     load_block(blk, r_end, a0);
     load_block(blk + stride, nr_end, na0);
@@ -137,18 +163,18 @@ struct Walker {
     Job j;
     if (started && base + kChunk < e) {
       base += kChunk;
-      j.s = blk * 32 + li; j.base = base; j.cnt = min(kChunk, e - base);
+      j.s = blk * bs + li; j.base = base; j.cnt = min(kChunk, e - base);
       j.first = false; j.last = base + kChunk >= e;
       return j;
     }
     if (started) ++li;
     started = true;
-    if (li == 32 || blk * 32 + li >= ns) {
+    if (li == bs || blk * bs + li >= ns) {
       blk += stride; li = 0;
       r_end = nr_end; a0 = na0;
       load_block(blk + stride, nr_end, na0);
     }
-    if (blk * 32 >= ns) {
+    if (blk * bs >= ns) {
       j.s = -1; j.base = 0; j.cnt = 0; j.first = j.last = false;
       base = 0; e = 0; started = false; blk = ns;  // stay exhausted
       return j;
@@ -156,17 +182,18 @@ struct Walker {
     const int prev = __shfl_sync(0xffffffffu, r_end, (li + 31) & 31);
     e = __shfl_sync(0xffffffffu, r_end, li);
     base = li ? prev : a0;
-    j.s = blk * 32 + li; j.base = base; j.cnt = min(kChunk, e - base);
+    j.s = blk * bs + li; j.base = base; j.cnt = min(kChunk, e - base);
     j.first = true; j.last = base + kChunk >= e;
     return j;
   }
-};
 
-// Sample that follows s in the walk of its warp (>= ns when there is none).
-__device__ __forceinline__ int64_t next_sample(int64_t s, int64_t ns, int64_t stride) {
-  if ((s & 31) != 31 && s + 1 < ns) return s + 1;
-  return ((s >> 5) + stride) << 5;
-}
+  // item that follows s in the walk of this warp (>= ns when there is none)
+  __device__ __forceinline__ int64_t after(int64_t s) const {
+    const int64_t b = s / bs;
+    if (s + 1 < (b + 1) * bs && s + 1 < ns) return s + 1;
+    return (b + stride) * bs;
+  }
+};
 
 // ---- staging ---------------------------------------------------------------------------
 
@@ -178,10 +205,10 @@ __device__ __forceinline__ int load_idx(const Job& j, const int2* __restrict__ n
 // Starts the gather of a chunk's feature rows: row r of the tile receives
 // hi[c0 .. c0+w) and mid[c0 .. c0+w) of point idx(r); rows beyond the chunk are
 // zero-filled.  One commit group per call is left to the caller.
-template <int K>
+template <int K, int CC>
 __device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat16* __restrict__ fs,
                                                int C, int c0, int w, int idx, int cnt, int lane) {
-  typedef Cfg<K> cfg;
+  typedef Cfg<K, CC> cfg;
   constexpr int kLph = cfg::kCC / 8;           // 16-byte segments per half row
   constexpr int kRpi = 32 / (2 * kLph);        // rows per warp instruction
   const int sub = lane % (2 * kLph), rsub = lane / (2 * kLph);
@@ -205,7 +232,7 @@ __device__ __forceinline__ void load_basis(const float* __restrict__ basis, int 
                                            int lane, float4* v) {
   const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)base * K);
 #pragma unroll
-  for (int t = 0; t < Cfg<K>::kBasisVecs; ++t) {
+  for (int t = 0; t < K / 8; ++t) {
     const int i = lane + 32 * t;
     v[t] = (i / (K / 4) < cnt) ? __ldg(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -229,12 +256,12 @@ __device__ __forceinline__ void store_split4(uint8_t* hi_row, uint8_t* mid_row, 
 // ... and stores them split into the chunk's basis tile (hi rows, then mid rows).
 template <int K>
 __device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float4* v) {
-  typedef Cfg<K> cfg;
+  constexpr int kKStride = K * 2 + 16;
 #pragma unroll
-  for (int t = 0; t < cfg::kBasisVecs; ++t) {
+  for (int t = 0; t < K / 8; ++t) {
     const int i = lane + 32 * t;
     const int row = i / (K / 4), a4 = i % (K / 4);
-    store_split4<K>(tile + row * cfg::kKStride, tile + (kChunk + row) * cfg::kKStride, a4, v[t]);
+    store_split4<K>(tile + row * kKStride, tile + (kChunk + row) * kKStride, a4, v[t]);
   }
 }
 
@@ -246,13 +273,14 @@ __device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float
 // indices of chunk i+2 are on their way to registers, while chunk i is multiplied.
 // OUT = 0: fp32 [ns, C, K] (the op's output).  OUT = 1: the same values split
 // into two bf16 arrays [ns, C*K] (left operand of the tensor-core GEMM).
-template <int K, int OUT>
-__global__ void __launch_bounds__(352, 1)
-basis_proj_mma_kernel(int C, int64_t ns, const float* __restrict__ basis,
+// The passes over the channels are dealt to gridDim.y.
+template <int K, int CC, int OUT>
+__global__ void __launch_bounds__(Cfg<K, CC>::kFwdWarps * 32, 1)
+basis_proj_mma_kernel(int bs, int C, int64_t ns, const float* __restrict__ basis,
                       const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                       const int32_t* __restrict__ ranges, float* __restrict__ out,
                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
-  typedef Cfg<K> cfg;
+  typedef Cfg<K, CC> cfg;
   extern __shared__ __align__(128) uint8_t bpm_smem[];
   const int lane = threadIdx.x & 31;
   const int warp_in_block = threadIdx.x >> 5;
@@ -269,17 +297,17 @@ basis_proj_mma_kernel(int C, int64_t ns, const float* __restrict__ basis,
   const uint32_t a_off = (r + 8 * (mi >> 1)) * cfg::kFeatStride + 8 * (mi & 1) * 2;
   const uint32_t b_off = (r + 8 * (mi & 1)) * cfg::kKStride + 8 * (mi >> 1) * 2;
 
-  for (int c0 = 0; c0 < C; c0 += cfg::kCC) {
+  for (int c0 = blockIdx.y * cfg::kCC; c0 < C; c0 += gridDim.y * cfg::kCC) {
     const int w = min(cfg::kCC, C - c0);
     const int mt_cnt = w >> 4;
     Walker walk;
-    walk.init(ranges, ns, warp, warps, lane);
+    walk.init(ranges, ns, warp, warps, lane, bs, 1);
     Job cur = walk.next(), n1 = walk.next(), n2 = walk.next();
     int idx1 = load_idx(n1, neigh, lane);
     __syncwarp();
     if (cur.valid()) {
       const int idx0 = load_idx(cur, neigh, lane);
-      issue_features<K>(smem_addr(feat_tile(0)), fs, C, c0, w, idx0, cur.cnt, lane);
+      issue_features<K, CC>(smem_addr(feat_tile(0)), fs, C, c0, w, idx0, cur.cnt, lane);
       float4 bv[cfg::kBasisVecs];
       load_basis<K>(basis, cur.base, cur.cnt, lane, bv);
       store_basis<K>(basis_tile(0), lane, bv);
@@ -291,7 +319,7 @@ basis_proj_mma_kernel(int C, int64_t ns, const float* __restrict__ basis,
       const int idx2 = load_idx(n2, neigh, lane);
       float4 bv[cfg::kBasisVecs];
       if (n1.valid()) {
-        issue_features<K>(smem_addr(feat_tile(buf ^ 1)), fs, C, c0, w, idx1, n1.cnt, lane);
+        issue_features<K, CC>(smem_addr(feat_tile(buf ^ 1)), fs, C, c0, w, idx1, n1.cnt, lane);
         load_basis<K>(basis, n1.base, n1.cnt, lane, bv);
       }
       cp_commit();
@@ -398,14 +426,14 @@ basis_proj_mma_kernel(int C, int64_t ns, const float* __restrict__ basis,
 // The feature rows are dead after (1), so the gather of the next chunk is
 // started there and runs under (2).  dbasis is written, not accumulated (every
 // pair belongs to exactly one sample); dfeat must be zero on entry.
-template <int K>
-__global__ void __launch_bounds__(224, 1)
-basis_proj_grads_mma_kernel(int C, int64_t ns, int64_t M, const float* __restrict__ basis,
+template <int K, int CC>
+__global__ void __launch_bounds__(Cfg<K, CC>::kGradWarps * 32, 1)
+basis_proj_grads_mma_kernel(int bs, int parts, int C, int64_t ns, int64_t M, const float* __restrict__ basis,
                             const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                             const int32_t* __restrict__ ranges,
                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
                             float* __restrict__ dfeat) {
-  typedef Cfg<K> cfg;
+  typedef Cfg<K, CC> cfg;
   extern __shared__ __align__(128) uint8_t bpm_smem[];
   const int lane = threadIdx.x & 31;
   const int warp_in_block = threadIdx.x >> 5;
@@ -448,15 +476,15 @@ basis_proj_grads_mma_kernel(int C, int64_t ns, int64_t M, const float* __restric
     const int w = min(cfg::kCC, C - c0);
     const int ks_cnt = w >> 4;     // 16-channel steps of (1) = tile pairs of (2)
     Walker walk;
-    walk.init(ranges, ns, warp, warps, lane);
+    walk.init(ranges, ns * parts, warp, warps, lane, bs, parts);
     Job cur = walk.next(), n1 = walk.next(), n2 = walk.next();
     int idx0 = load_idx(cur, neigh, lane);
     int idx1 = load_idx(n1, neigh, lane);
     float4 bv[cfg::kBasisVecs];
     __syncwarp();
     if (cur.valid()) {
-      issue_dx(cur.s, c0, w);
-      issue_features<K>(smem_addr(feat_tile), fs, C, c0, w, idx0, cur.cnt, lane);
+      issue_dx(cur.s / parts, c0, w);
+      issue_features<K, CC>(smem_addr(feat_tile), fs, C, c0, w, idx0, cur.cnt, lane);
       load_basis<K>(basis, cur.base, cur.cnt, lane, bv);
     }
     cp_commit();
@@ -471,8 +499,8 @@ basis_proj_grads_mma_kernel(int C, int64_t ns, int64_t M, const float* __restric
                           raw[i]);
         }
         __syncwarp();
-        const int64_t sn = next_sample(cur.s, ns, warps);
-        if (sn < ns) issue_dx(sn, c0, w);
+        const int64_t sn = walk.after(cur.s);
+        if (sn < walk.ns) issue_dx(sn / parts, c0, w);
         cp_commit();
       }
       store_basis<K>(basis_tile, lane, bv);
@@ -543,7 +571,7 @@ basis_proj_grads_mma_kernel(int C, int64_t ns, int64_t M, const float* __restric
       // ---- prefetch for the next chunks
       const int idx2 = load_idx(n2, neigh, lane);
       if (n1.valid()) {
-        issue_features<K>(smem_addr(feat_tile), fs, C, c0, w, idx1, n1.cnt, lane);
+        issue_features<K, CC>(smem_addr(feat_tile), fs, C, c0, w, idx1, n1.cnt, lane);
         load_basis<K>(basis, n1.base, n1.cnt, lane, bv);
       }
       cp_commit();
