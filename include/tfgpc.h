@@ -289,6 +289,30 @@ int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
                         const int32_t* samples_batch_ids, int samples_are_points,
                         float* pdf_out);
 
+/* Sampling (tfgpc_sampling_count + _store) on a built grid without a neighbor list:
+ * mode 0 Poisson disk with the neighbors of a self neighborhood without limit
+ * (inv_radii [D]), mode 1 cell average.  The outputs hold n rows, the first
+ * *num_samples_out [host] are written; sample_indices_out (mode 0) are indices into
+ * the UNSORTED points.  Blocks once.  tfgpc_cell_grid_sample builds the grid in the
+ * same call (`ws` of tfgpc_cell_grid_workspace_bytes with ns = 0), with the one
+ * blocking read and the status of tfgpc_cell_grid_neighborhood. */
+size_t tfgpc_cells_sample_workspace_bytes(int64_t n);
+int tfgpc_cells_sample(void* stream, const tfgpc_cell_grid* grid, int mode,
+                       const float* inv_radii, float* sample_pts_out,
+                       int32_t* sample_batch_ids_out,
+                       int32_t* sample_indices_out, void* ws, size_t ws_bytes,
+                       int64_t* num_samples_out);
+int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
+                           const float* points, const int32_t* batch_ids,
+                           const float* cell_sizes,
+                           const int32_t* num_cells_in, int mode,
+                           const float* inv_radii, float* sample_pts_out,
+                           int32_t* sample_batch_ids_out,
+                           int32_t* sample_indices_out, void* ws,
+                           size_t ws_bytes, void* sample_ws,
+                           size_t sample_ws_bytes, int32_t* num_cells_host_out,
+                           int64_t* num_samples_out);
+
 /* ---- FindNeighbors fill pass with original ids and densities --------------
  * tfgpc_find_neighbors_fill_ordered (sample_order may be NULL) that, in the same
  * pass, also writes what pylib computes from the neighbor list afterwards:

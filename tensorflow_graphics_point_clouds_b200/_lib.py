@@ -50,6 +50,9 @@ SYMBOLS = {
     "tfgpc_cells_count": c_int,
     "tfgpc_cells_fill": c_int,
     "tfgpc_cells_density": c_int,
+    "tfgpc_cells_sample_workspace_bytes": c_sz,
+    "tfgpc_cells_sample": c_int,
+    "tfgpc_cell_grid_sample": c_int,
     "tfgpc_pack_points_density": c_int,
     "tfgpc_find_neighbors_fill_fused": c_int,
     "tfgpc_original_neighbor_ids": c_int,
@@ -110,6 +113,27 @@ def lib():
       getattr(handle, name).restype = restype
     _lib = handle
   return _lib
+
+
+_host_module = None
+
+
+def host():
+  """The native host layer (host/*.cpp): checks, allocates and enqueues for the ops
+  and layers.  Raises like lib() if it has not been built."""
+  global _host_module
+  if _host_module is None:
+    lib()
+    import torch  # noqa: F401  (the module links against torch's libraries)
+    try:
+      from . import _host
+    except ImportError as err:
+      raise RuntimeError("_host.so is missing or does not load (%s): build it with `python -m "
+                         "tensorflow_graphics_point_clouds_b200.build`; there is no CPU or eager "
+                         "fallback" % err) from err
+    _host.set_error_class(TfgpcError)
+    _host_module = _host
+  return _host_module
 
 
 def check(code):

@@ -30,4 +30,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
                     const int32_t* batch_ids, const float* cell_sizes,
                     const int32_t* num_cells_in, const CellGridWs& w, int32_t* page);
 
+// Argument check of every entry on a built grid (cell_search.cu).
+int check_cell_grid(const char* op, const tfgpc_cell_grid* g);
+
 }  // namespace tfgpc

@@ -1,0 +1,417 @@
+// Poisson-disk and cell-average sampling straight from the cell table of a grid.
+//
+// Poisson disk (count_sampling_pd_kernels.cu.cc:42-108, 157-180): 2^D passes, pass p
+// takes the cells whose coordinate d has parity bit d of p; inside a cell the points
+// are visited in sorted order and a point is taken iff none of its neighbors is.  A
+// taken point marks the points within the radius itself (the relation is symmetric),
+// so no neighbor list is needed: on 8 clouds of 100 000 Gaussian-mixture points
+// searching and writing the lists of four levels took 3.2 ms, the passes over them 0.6.
+// The passes and the compaction of the taken points in ascending index are one
+// cooperative launch with a barrier between passes; what bounds it is the chain of
+// passes on small levels and the marking on crowded ones.
+//
+// Cell average (sampling_avg_kernels.cu.cc:43-88): one thread per occupied cell,
+// sequential fp32 sum of its points / count, cells in ascending first index.
+#include "cell_grid.cuh"
+
+namespace tfgpc {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;
+constexpr int kMaxBlocks = 1024;
+constexpr unsigned long long kBarrierLimitNs = 1000000000ull;
+
+struct SampleArgs {
+  CellsView c;
+  const int64_t* keys;         // sorted
+  int mode;                    // 0 Poisson disk, 1 cell average
+  const float* inv_radii;
+  uint8_t* state;              // [n] 0 open, 1 blocked, 2 taken (zero on entry)
+  unsigned* arrived;           // barrier counter (zero on entry), then an error word
+  int32_t* block_total;        // [gridDim.x]
+  float* pts_out;
+  int32_t* batch_out;
+  int32_t* index_out;          // original indices (Poisson)
+  int32_t* page;               // number of samples (64 bits), then the error word
+};
+
+// Barrier over the blocks of a cooperative launch (all resident).  Gives up after a
+// second: the error word is set and every later barrier passes at once.
+__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    ok = true;
+    while (*(volatile unsigned*)arrived < target) {
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t - t0 > kBarrierLimitNs || *(volatile unsigned*)(arrived + 1) != 0u) {
+        *(volatile unsigned*)(arrived + 1) = 1u;
+        ok = false;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  return ok;
+}
+
+template <int D>
+__device__ void poisson_cell(const SampleArgs& a, const int* cell, int batch, int begin, int end,
+                             const int* nc, int total, const float* inv_r) {
+  constexpr int kTubes = num_tubes<D>();
+  constexpr int kRounds = (kTubes + 31) / 32;
+  const int lane = lane_id();
+  int2 r[kRounds];
+#pragma unroll
+  for (int i = 0; i < kRounds; ++i)
+    r[i] = i * 32 + lane < kTubes
+               ? tube_points<D>(i * 32 + lane, cell, batch, nc, total, a.c.start)
+               : make_int2(0, 0);
+  for (int q0 = begin; q0 < end; q0 += 32) {
+    const int q = q0 + lane;
+    unsigned open = __ballot_sync(0xffffffffu, q < end && __ldcg(a.state + q) == 0);
+    while (open) {
+      const int taken = q0 + __ffs(open) - 1;
+      open &= open - 1u;
+      float s[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) s[d] = __ldg(a.c.points + (int64_t)taken * D + d);
+      unsigned marked = 0u;
+#pragma unroll
+      for (int i = 0; i < kRounds; ++i) {
+        for (int t = 0; t < min(32, kTubes - i * 32); ++t) {
+          const int x = __shfl_sync(0xffffffffu, r[i].x, t);
+          const int y = __shfl_sync(0xffffffffu, r[i].y, t);
+          for (int j = x + lane; j < y; j += 32) {
+            float p[D];
+            if (D <= 3) {
+              const float4 v = __ldg(a.c.packed + j);
+              p[0] = v.x; p[1] = v.y;
+              if (D == 3) p[D - 1] = v.z;
+            } else {
+#pragma unroll
+              for (int d = 0; d < D; ++d) p[d] = __ldg(a.c.points + (int64_t)j * D + d);
+            }
+            // the distance test of the search (cell_search.cu)
+            float u = __fmul_rn(__fsub_rn(s[0], p[0]), inv_r[0]);
+            float d2 = __fmul_rn(u, u);
+#pragma unroll
+            for (int d = 1; d < D; ++d) {
+              u = __fmul_rn(__fsub_rn(s[d], p[d]), inv_r[d]);
+              d2 = __fmaf_rn(u, u, d2);
+            }
+            if (d2 < 1.0f && j != taken) {
+              __stcg(a.state + j, (uint8_t)1);
+              if (j >= q0 && j < q0 + 32) marked |= 1u << (j - q0);
+            }
+          }
+        }
+      }
+      if (lane == 0) __stcg(a.state + taken, (uint8_t)2);
+      open &= ~__reduce_or_sync(0xffffffffu, marked);
+    }
+    __syncwarp();   // the marks of this group are visible to the next group's reads
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kThreads, 4)
+cells_sample_kernel(SampleArgs a) {
+  __shared__ int warp_total[kWarps];
+  __shared__ int64_t before_s;
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  int nc[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) nc[d] = __ldg(a.c.num_cells + d);
+  const int total = total_cells<D>(nc, a.c.batch_size);
+  const int64_t n = a.c.n;
+  unsigned barriers = 0;
+  bool ok = true;
+  if (a.mode == 0) {
+    float inv_r[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) inv_r[d] = __ldg(a.inv_radii + d);
+    // points outside every cell have no neighbors: all of them are taken
+    const int lead = __ldg(a.c.start + 1), tail = __ldg(a.c.start + total + 1);
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < lead + (n - tail);
+         i += (int64_t)gridDim.x * kThreads)
+      a.state[i < lead ? i : tail + (i - lead)] = 2;
+    const int warps = gridDim.x * kWarps;
+    const int warp = blockIdx.x * kWarps + w;
+    for (int pass = 0; pass < (1 << D); ++pass) {
+      int half[D], cells = a.c.batch_size;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        half[d] = (nc[d] - ((pass >> d) & 1) + 1) >> 1;
+        cells *= half[d];
+      }
+      // a lane looks at every `warps`-th cell: crowded regions spread over the warps
+      for (int c0 = 0; c0 < cells; c0 += 32 * warps) {
+        const int i = c0 + lane * warps + warp;
+        int cell[D], batch = 0, begin = 0, end = 0;
+#pragma unroll
+        for (int d = 0; d < D; ++d) cell[d] = 0;
+        if (i < cells) {
+          int rem = i, key = 0, scale = 1;
+#pragma unroll
+          for (int d = D - 1; d >= 0; --d) {
+            cell[d] = 2 * (rem % half[d]) + ((pass >> d) & 1);
+            rem /= half[d];
+            key += cell[d] * scale;
+            scale *= nc[d];
+          }
+          batch = rem;
+          key += batch * scale;
+          begin = __ldg(a.c.start + (total - key));
+          end = __ldg(a.c.start + (total - key) + 1);
+        }
+        unsigned work = __ballot_sync(0xffffffffu, end > begin);
+        while (work) {
+          const int who = __ffs(work) - 1;
+          work &= work - 1u;
+          int cc[D];
+#pragma unroll
+          for (int d = 0; d < D; ++d) cc[d] = __shfl_sync(0xffffffffu, cell[d], who);
+          poisson_cell<D>(a, cc, __shfl_sync(0xffffffffu, batch, who),
+                          __shfl_sync(0xffffffffu, begin, who),
+                          __shfl_sync(0xffffffffu, end, who), nc, total, inv_r);
+        }
+      }
+      ok = grid_barrier(a.arrived, ++barriers * gridDim.x) && ok;
+    }
+  }
+  // ---- compaction: every block counts, then writes, its stretch of the points
+  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t first = min((int64_t)blockIdx.x * per, n), last = min(first + per, n);
+  auto chosen = [&](int64_t i) {
+    if (i >= last) return false;
+    return a.mode == 0 ? __ldcg(a.state + i) == 2
+                       : i == 0 || __ldg(a.keys + i) != __ldg(a.keys + i - 1);
+  };
+  int mine = 0;
+  for (int64_t i = first + threadIdx.x; i < last; i += kThreads) mine += chosen(i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  if (lane == 0) warp_total[w] = mine;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int t = 0;
+    for (int i = 0; i < kWarps; ++i) t += warp_total[i];
+    __stcg(a.block_total + blockIdx.x, t);
+  }
+  ok = grid_barrier(a.arrived, ++barriers * gridDim.x) && ok;
+  if (w == 0) {
+    int64_t t = 0, all = 0;
+    for (int i = lane; i < gridDim.x; i += 32) {
+      const int v = __ldcg(a.block_total + i);
+      all += v;
+      if (i < (int)blockIdx.x) t += v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t += __shfl_xor_sync(0xffffffffu, t, o);
+      all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    if (lane == 0) {
+      before_s = t;
+      if (blockIdx.x == 0) {
+        a.page[0] = (int32_t)(uint32_t)all;
+        a.page[1] = (int32_t)(all >> 32);
+        a.page[2] = ok ? 0 : 1;
+        __threadfence_system();
+      }
+    }
+  }
+  __syncthreads();
+  int64_t out = before_s;
+  if (!ok) return;
+  for (int64_t i0 = first; i0 < last; i0 += kThreads) {
+    const int64_t i = i0 + threadIdx.x;
+    const bool take = chosen(i);
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    __syncthreads();
+    if (lane == 0) warp_total[w] = __popc(m);
+    __syncthreads();
+    int ahead = 0, sum = 0;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) {
+      if (k < w) ahead += warp_total[k];
+      sum += warp_total[k];
+    }
+    if (take) {
+      const int64_t o = out + ahead + __popc(m & ((1u << lane) - 1u));
+      if (a.mode == 0) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) a.pts_out[o * D + d] = __ldg(a.c.points + i * D + d);
+        a.batch_out[o] = __ldg(a.c.batch_ids + i);
+        a.index_out[o] = __ldg(a.c.indices + i);
+      } else {
+        const int64_t key = __ldg(a.keys + i);
+        float acc[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) acc[d] = 0.0f;
+        int64_t end = i;
+        if (key >= 0 && key < total) {
+          end = __ldg(a.c.start + (total - (int)key) + 1);
+        } else {
+          while (end < n && __ldg(a.keys + end) == key) ++end;
+        }
+#pragma unroll 4
+        for (int64_t q = i; q < end; ++q)
+#pragma unroll
+          for (int d = 0; d < D; ++d) acc[d] += __ldg(a.c.points + q * D + d);
+        const float cnt = (float)(end - i);
+#pragma unroll
+        for (int d = 0; d < D; ++d) a.pts_out[o * D + d] = acc[d] / cnt;
+        a.batch_out[o] = (int32_t)(key / (total / a.c.batch_size));
+      }
+    }
+    out += sum;
+  }
+}
+
+template <int D>
+int launch_sample(cudaStream_t st, SampleArgs a) {
+  static int per_sm = 0;     // (the same value whoever computes it)
+  if (per_sm == 0) {
+    int v = 0;
+    TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
+    per_sm = v < 1 ? 1 : v;
+  }
+  // a warp per 64 points, at most what is resident at once and 4 blocks per SM: with
+  // more, the barriers take longer than the shorter passes give back
+  int64_t blocks = (a.c.n + 64 * kWarps - 1) / (64 * kWarps);
+  const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
+  if (blocks > most) blocks = most;
+  if (blocks > kMaxBlocks) blocks = kMaxBlocks;
+  void* args[] = {&a};
+  TFGPC_CUDA(cudaLaunchCooperativeKernel(cells_sample_kernel<D>, dim3((unsigned)blocks),
+                                         dim3(kThreads), args, 0, st));
+  return TFGPC_OK;
+}
+
+size_t sample_ws_bytes(int64_t n) {
+  return align_up((size_t)n + 16, 256) + align_up((size_t)kMaxBlocks * 4, 256);
+}
+
+// Enqueues the sampling; the number of samples goes to words kReportTotal .. of the page.
+int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const float* inv_radii,
+                 float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page) {
+  const size_t state = align_up((size_t)g.n + 16, 256);
+  SampleArgs a;
+  a.c = view_of(g);
+  a.keys = g.sorted_keys;
+  a.mode = mode;
+  a.inv_radii = inv_radii;
+  a.arrived = (unsigned*)ws;          // [0] counter, [1] error word, then the states
+  a.state = (uint8_t*)ws + 16;
+  a.block_total = (int32_t*)((char*)ws + state);
+  a.pts_out = pts_out;
+  a.batch_out = batch_out;
+  a.index_out = index_out;
+  a.page = page + kReportTotal;
+  ProfScope prof(st, mode == 0 ? "sampling_poisson" : "sampling_cell_average");
+  TFGPC_CUDA(cudaMemsetAsync(ws, 0, mode == 0 ? (size_t)g.n + 16 : 16, st));
+  switch (g.D) {
+    case 2: return launch_sample<2>(st, a);
+    case 3: return launch_sample<3>(st, a);
+    case 4: return launch_sample<4>(st, a);
+    case 5: return launch_sample<5>(st, a);
+    default: return launch_sample<6>(st, a);
+  }
+}
+
+int check_sample(const tfgpc_cell_grid* g, int mode, const float* inv_radii, const float* pts_out,
+                 const int32_t* batch_out, const int32_t* index_out, const void* ws,
+                 size_t ws_bytes, const int64_t* num_samples_out) {
+  int rc = check_cell_grid("SamplingOp", g);
+  if (rc) return rc;
+  TFGPC_REQUIRE(mode == 0 || mode == 1, "SamplingOp expects mode 0 (poisson) or 1 (average)");
+  TFGPC_REQUIRE(pts_out && batch_out && ws && num_samples_out &&
+                (mode == 1 || (index_out && inv_radii)), "SamplingOp got a null pointer");
+  if (ws_bytes < sample_ws_bytes(g->n)) return fail(TFGPC_ENOMEM, "SamplingOp workspace too small");
+  return TFGPC_OK;
+}
+
+int finish_sample(cudaStream_t st, const tfgpc_cell_grid& g, int32_t* num_cells_host_out,
+                  int64_t* num_samples_out) {
+  int32_t host[kReportWords + 1];
+  int rc = read_report(st, sizeof(host), host);
+  if (rc) return rc;
+  for (int d = 0; num_cells_host_out && d < g.D; ++d) num_cells_host_out[d] = host[d];
+  if (num_cells_host_out && host[TFGPC_MAX_DIMS])
+    return fail(TFGPC_ENOMEM, "SamplingOp: the grid needs more than max_cells = %d cells in a "
+                "dimension; repeat the call with a larger bound", g.max_cells);
+  if (host[kReportWords])
+    return fail(TFGPC_ETIMEOUT, "a bounded wait inside the sampling kernel ran out");
+  *num_samples_out = (int64_t)(uint32_t)host[kReportTotal] |
+                     ((int64_t)host[kReportTotal + 1] << 32);
+  return TFGPC_OK;
+}
+
+}  // namespace
+}  // namespace tfgpc
+
+using namespace tfgpc;
+
+extern "C" size_t tfgpc_cells_sample_workspace_bytes(int64_t n) {
+  return n > 0 ? sample_ws_bytes(n) : 256;
+}
+
+extern "C" int tfgpc_cells_sample(void* stream, const tfgpc_cell_grid* grid, int mode,
+                                  const float* inv_radii, float* sample_pts_out,
+                                  int32_t* sample_batch_ids_out, int32_t* sample_indices_out,
+                                  void* ws, size_t ws_bytes, int64_t* num_samples_out) {
+  int rc = check_sample(grid, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                        sample_indices_out, ws, ws_bytes, num_samples_out);
+  if (rc) return rc;
+  *num_samples_out = 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  rc = sample_async(st, *grid, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                    sample_indices_out, ws, (int32_t*)page);
+  if (rc) return rc;
+  return finish_sample(st, *grid, nullptr, num_samples_out);
+}
+
+extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
+                                      const float* points, const int32_t* batch_ids,
+                                      const float* cell_sizes, const int32_t* num_cells_in,
+                                      int mode, const float* inv_radii, float* sample_pts_out,
+                                      int32_t* sample_batch_ids_out, int32_t* sample_indices_out,
+                                      void* ws, size_t ws_bytes, void* sample_ws,
+                                      size_t sample_ws_bytes_given, int32_t* num_cells_host_out,
+                                      int64_t* num_samples_out) {
+  int rc = check_sample(grid, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                        sample_indices_out, sample_ws, sample_ws_bytes_given, num_samples_out);
+  if (rc) return rc;
+  const tfgpc_cell_grid& g = *grid;
+  TFGPC_REQUIRE(points && batch_ids && cell_sizes && ws && num_cells_host_out,
+                "SamplingOp got a null pointer");
+  TFGPC_REQUIRE(num_cells_in != g.num_cells,
+                "SamplingOp expects the given cell counts outside the output array");
+  for (int d = 0; d < g.D; ++d)
+    TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "SamplingOp expects positive cell sizes");
+  if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, 0, g.batch_size, g.max_cells))
+    return fail(TFGPC_ENOMEM, "SamplingOp workspace too small");
+  *num_samples_out = 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  CellGridWs w = carve_cell_grid(ws, g.n, 0, g.D, g.batch_size, g.max_cells);
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page);
+  if (rc) return rc;
+  rc = sample_async(st, g, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                    sample_indices_out, sample_ws, (int32_t*)page);
+  if (rc) return rc;
+  return finish_sample(st, g, num_cells_host_out, num_samples_out);
+}

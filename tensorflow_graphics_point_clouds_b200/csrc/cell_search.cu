@@ -323,7 +323,9 @@ WalkArgs walk_args(const tfgpc_cell_grid& g, const SampleSource& src, int64_t ns
   return a;
 }
 
-int check_grid(const char* op, const tfgpc_cell_grid* g) {
+}  // namespace
+
+int check_cell_grid(const char* op, const tfgpc_cell_grid* g) {
   TFGPC_REQUIRE(g != nullptr, "%s got a null grid", op);
   TFGPC_REQUIRE(valid_dims(g->D), "%s expects a valid number of dimension (got %d)", op, g->D);
   TFGPC_REQUIRE(g->n > 0 && g->n < (int64_t)INT32_MAX && g->batch_size > 0 &&
@@ -338,6 +340,8 @@ int check_grid(const char* op, const tfgpc_cell_grid* g) {
   TFGPC_REQUIRE((uintptr_t)g->packed % 16 == 0, "%s expects a 16-byte aligned packed table", op);
   return TFGPC_OK;
 }
+
+namespace {
 
 int check_samples(const char* op, const tfgpc_cell_grid* g, int64_t ns, const float* samples,
                   const int32_t* sbatch, int mode, int max_neighs) {
@@ -406,7 +410,7 @@ extern "C" int tfgpc_cell_grid_neighborhood(
     const float* samples, const int32_t* samples_batch_ids, int samples_are_points,
     int max_neighs, int32_t* ranges_out, void* ws, size_t ws_bytes, int32_t* num_cells_host_out,
     int64_t* total_out) {
-  int rc = check_grid("GridNeighborhood", grid);
+  int rc = check_cell_grid("GridNeighborhood", grid);
   if (rc) return rc;
   const tfgpc_cell_grid& g = *grid;
   rc = check_samples("GridNeighborhood", grid, ns, samples, samples_batch_ids,
@@ -442,7 +446,7 @@ extern "C" int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid, cons
                                  const int32_t* samples_batch_ids, int samples_are_points,
                                  int max_neighs, int32_t* ranges_out, void* ws, size_t ws_bytes,
                                  int64_t* total_out) {
-  int rc = check_grid("FindNeighbors", grid);
+  int rc = check_cell_grid("FindNeighbors", grid);
   if (rc) return rc;
   rc = check_samples("FindNeighbors", grid, ns, samples, samples_batch_ids, samples_are_points,
                      max_neighs);
@@ -470,7 +474,7 @@ extern "C" int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid, const
                                 const int32_t* samples_batch_ids, int samples_are_points,
                                 int max_neighs, const int32_t* ranges, int64_t total,
                                 int32_t* neigh_out, int32_t* ids_out) {
-  int rc = check_grid("FindNeighbors", grid);
+  int rc = check_cell_grid("FindNeighbors", grid);
   if (rc) return rc;
   rc = check_samples("FindNeighbors", grid, ns, samples, samples_batch_ids, samples_are_points,
                      max_neighs);
@@ -493,7 +497,7 @@ extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
                                    int64_t ns, const float* samples,
                                    const int32_t* samples_batch_ids, int samples_are_points,
                                    float* pdf_out) {
-  int rc = check_grid("ComputePdf", grid);
+  int rc = check_cell_grid("ComputePdf", grid);
   if (rc) return rc;
   rc = check_samples("ComputePdf", grid, ns, samples, samples_batch_ids, samples_are_points, 0);
   if (rc) return rc;

@@ -114,9 +114,10 @@ class NeighborCount:
   """Result of the count pass of FindNeighbors: the ranges [Ns], the number of
   pairs, and the checked arguments the fill pass needs again."""
 
-  def __init__(self, ranges, total, args, order, dims, cells=None):
+  cells = None             # (a count on a cell table is the host layer's own object)
+
+  def __init__(self, ranges, total, args, order, dims):
     self.ranges, self.total, self.args, self.order, self.dims = ranges, total, args, order, dims
-    self.cells = cells     # the CellGrid it was counted on; args are then those of its fill
 
 
 def find_neighbors_count(samples, samples_batch_ids, points, point_keys, grid_acc_ds, num_cells,
@@ -315,141 +316,45 @@ def grid_neighborhood_count(points, batch_ids, batch_size, cell_sizes, radii, ma
   return g
 
 
-class _CellGridStruct(ctypes.Structure):
-  """tfgpc_cell_grid of include/tfgpc.h."""
-  _fields_ = [("D", c_int), ("max_cells", c_int), ("n", c_i64), ("batch_size", c_i64)] + [
-      (name, ctypes.c_void_p) for name in
-      ("aabb_min", "aabb_max", "num_cells", "scaled_aabb_min", "inv_cell_sizes", "keys",
-       "sorted_indices", "sorted_keys", "sorted_points", "sorted_batch_ids", "packed",
-       "cell_start", "ds")]
-
+# A grid with its cell table (tfgpc_cell_grid_neighborhood) is a host-layer object with
+# the arrays of the C struct as attributes, plus num_cells_host [D] int32 on the CPU.
+# The calls below raise TfgpcError(3) with the counts asked for in its `num_cells` if a
+# dimension needs more than max_cells cells.
 
 def cell_table_elems(dims, batch_size, max_cells):
   """Values of the cell table of a grid with these bounds, 0 if it would be too large."""
-  return _lib.lib().tfgpc_cell_table_elems(c_int(dims), c_i64(batch_size), c_int(max_cells))
+  return _lib.host().cell_table_elems(dims, batch_size, max_cells)
 
 
-class CellGrid:
-  """A grid with its cell table (tfgpc_cell_grid_neighborhood): the arrays of the
-  struct as attributes and num_cells_host [D] int32 on the CPU."""
+def build_cell_grid(points, batch_ids, batch_size, cell_sizes, max_cells, cells=None,
+                    inv_radii=None, samples=None, samples_batch_ids=None, samples_are_points=-1,
+                    max_neighs=0):
+  """(grid, count of the neighborhood around the samples or None without samples).
+  cells: as in grid_neighborhood_count; samples_are_points 0: samples and their batch
+  ids, 1: the points in their own order, 2: the sorted points, -1: no samples."""
+  return _lib.host().build_grid(points, batch_ids, batch_size, cell_sizes, max_cells, cells,
+                                inv_radii, samples_are_points, samples, samples_batch_ids,
+                                max_neighs)
 
-  @classmethod
-  def build(cls, points, batch_ids, batch_size, cell_sizes, max_cells, cells=None,
-            inv_radii=None, samples=None, samples_batch_ids=None, samples_are_points=None,
-            max_neighs=0):
-    """(grid, NeighborCount of the neighborhood or None without samples).  Raises
-    TfgpcError(3) with the counts asked for in its `num_cells` if a dimension needs
-    more than max_cells cells.  cells: as in grid_neighborhood_count."""
-    self = cls()
-    points, bid = _f32(points), _i32(batch_ids)
-    _dev_check(points, bid)
-    n, d = points.shape
-    dev, b, lib = points.device, int(batch_size), _lib.lib()
-    f32 = lambda *shape: torch.empty(shape, dtype=torch.float32, device=dev)
-    i32 = lambda *shape: torch.empty(shape, dtype=torch.int32, device=dev)
-    i64 = lambda *shape: torch.empty(shape, dtype=torch.int64, device=dev)
-    self.num_cells = i32(d)
-    for name, shape in (("aabb_min", (b, d)), ("aabb_max", (b, d)), ("scaled_aabb_min", (b, d)),
-                        ("inv_cell_sizes", (d,))):
-      setattr(self, name, f32(*shape) if cells is None else cells[name])
-    self.keys, self.sorted_keys = i64(n), i64(n)
-    self.sorted_indices, self.sorted_batch_ids = i32(n), i32(n)
-    self.sorted_points = f32(n, d)
-    self.packed = f32(n, 4) if d <= 3 else None
-    self.cell_start = i32(cell_table_elems(d, b, max_cells))
-    ds_flat = i32(b * max_cells * max_cells * 2)
-    self.struct = _CellGridStruct(
-        d, max_cells, n, b, *[None if t is None else t.data_ptr() for t in (
-            self.aabb_min, self.aabb_max, self.num_cells, self.scaled_aabb_min,
-            self.inv_cell_sizes, self.keys, self.sorted_indices, self.sorted_keys,
-            self.sorted_points, self.sorted_batch_ids, self.packed, self.cell_start, ds_flat)])
-    self.source = (points, bid)
-    cells_in = None if cells is None else _i32(cells["num_cells"])
-    ns, head, ranges, keep = 0, (c_i64(0), ptr(None), ptr(None), c_int(0)), None, None
-    if samples_are_points is not None:
-      ns, head, keep = self._samples(samples, samples_batch_ids, samples_are_points)
-      ranges = i32(ns)
-    nbytes = lib.tfgpc_cell_grid_workspace_bytes(c_int(d), c_i64(n), c_i64(ns), c_i64(b),
-                                                 c_int(max_cells))
-    ws = _workspace(nbytes, dev)
-    nc_host, total = (ctypes.c_int32 * d)(), c_i64(0)
-    code = lib.tfgpc_cell_grid_neighborhood(
-        _stream(), ctypes.byref(self.struct), ptr(points), ptr(bid), _host_floats(cell_sizes, d),
-        ptr(cells_in), ptr(inv_radii), *head, c_int(int(max_neighs)), ptr(ranges), ptr(ws),
-        c_sz(nbytes), nc_host, ctypes.byref(total))
-    if code != 0:
-      err = _lib.TfgpcError(code, lib.tfgpc_last_error().decode())
-      err.num_cells = list(nc_host)
-      raise err
-    self.num_cells_host = torch.tensor(list(nc_host), dtype=torch.int32)
-    c0, c1 = int(nc_host[0]), int(nc_host[1])
-    self.ds = ds_flat[:b * c0 * c1 * 2].reshape(b, c0, c1, 2)
-    if ranges is None:
-      return self, None
-    return self, NeighborCount(ranges, int(total.value),
-                               (head, (inv_radii, int(max_neighs)), keep), None, d, self)
 
-  def _samples(self, samples, samples_batch_ids, samples_are_points):
-    """(number, C arguments, tensors to keep): samples_are_points 0 takes the two
-    arrays, 1 the grid's points in their own order, 2 the sorted points."""
-    if samples_are_points == 0:
-      samples, sbid = _f32(samples), _i32(samples_batch_ids)
-      _dev_check(samples, sbid)
-      ns = samples.shape[0]
-      if samples.shape[1] != self.struct.D:
-        raise _lib.TfgpcError(1, "FindNeighborsOp expects inputs with the dimension of the samples")
-      if sbid.shape[0] != ns:
-        raise _lib.TfgpcError(1, "FindNeighborsOp expects the same number of batch ids as samples.")
-    else:
-      samples = sbid = None
-      ns = self.struct.n
-    return ns, (c_i64(ns), ptr(samples), ptr(sbid), c_int(int(samples_are_points))), (samples, sbid)
-
-  def count_neighbors(self, inv_radii, samples_are_points, samples=None, samples_batch_ids=None,
-                      max_neighs=0):
-    """The count pass of a neighborhood on this grid (tfgpc_cells_count); blocks."""
-    ns, head, keep = self._samples(samples, samples_batch_ids, samples_are_points)
-    dev = self.cell_start.device
-    ranges = torch.empty(ns, dtype=torch.int32, device=dev)
-    nbytes = _lib.lib().tfgpc_find_neighbors_workspace_bytes(c_i64(ns))
-    ws = _workspace(nbytes, dev)
-    total = c_i64(0)
-    _lib.check(_lib.lib().tfgpc_cells_count(
-        _stream(), ctypes.byref(self.struct), ptr(inv_radii), *head, c_int(int(max_neighs)),
-        ptr(ranges), ptr(ws), c_sz(nbytes), ctypes.byref(total)))
-    return NeighborCount(ranges, int(total.value), (head, (inv_radii, int(max_neighs)), keep),
-                         None, self.struct.D, self)
-
-  def density(self, inv_radii, inv_bandwidth, mode, samples_are_points):
-    """Density at every point of the grid over all points within the radius, in the
-    unsorted (samples_are_points 1) or the sorted order (2): tfgpc_cells_density."""
-    _, head, _ = self._samples(None, None, samples_are_points)
-    pdf = torch.empty(self.struct.n, dtype=torch.float32, device=self.cell_start.device)
-    _lib.check(_lib.lib().tfgpc_cells_density(
-        _stream(), ctypes.byref(self.struct), ptr(inv_radii), ptr(inv_bandwidth), c_int(int(mode)),
-        *head, ptr(pdf)))
-    return pdf
+def build_cell_grid_and_sample(points, batch_ids, batch_size, cell_sizes, max_cells, mode,
+                               inv_radii, cells=None):
+  """(grid, sample points, sample batch ids, original indices or None): a grid and the
+  Poisson-disk (mode 0) or cell-average (1) sampling on it (tfgpc_cell_grid_sample)."""
+  return _lib.host().build_and_sample(points, batch_ids, batch_size, cell_sizes, max_cells, cells,
+                                      mode, inv_radii)
 
 
 def _cells_fill(count, with_ids, inv_bandwidth, pdf_mode):
   """find_neighbors_fill for a count taken on a cell table."""
-  head, (inv_radii, max_neighs), (samples, _) = count.args
-  dev, grid = count.ranges.device, count.cells
-  neigh = torch.empty((count.total, 2), dtype=torch.int32, device=dev)
-  ids = torch.empty((count.total, 2), dtype=torch.int32, device=dev) if with_ids else None
-  _lib.check(_lib.lib().tfgpc_cells_fill(
-      _stream(), ctypes.byref(grid.struct), ptr(inv_radii), *head, c_int(max_neighs),
-      ptr(count.ranges), c_i64(count.total), ptr(neigh), ptr(ids)))
+  neigh, ids = _lib.host().fill_neighbors(count, with_ids)
   if not with_ids:
     return neigh
   if pdf_mode is None:
     return neigh, ids
-  if samples is None:
-    samples = grid.source[0] if head[3].value == 1 else grid.sorted_points
-  if inv_bandwidth is None:
-    inv_bandwidth = inv_radii
-  return neigh, ids, compute_pdf_at_samples(samples, grid.sorted_points, neigh, count.ranges,
-                                            inv_bandwidth, inv_radii, pdf_mode)
+  return neigh, ids, compute_pdf_at_samples(
+      count.samples, count.cells.sorted_points, neigh, count.ranges,
+      count.inv_radii if inv_bandwidth is None else inv_bandwidth, count.inv_radii, pdf_mode)
 
 
 def original_neighbor_ids(neighbors, sorted_indices, pdf_by_original=None):
@@ -536,19 +441,6 @@ def compute_pdf_pt_grads(points, neighbors, sample_neigh_indices, inv_bandwidth,
   return out
 
 
-def _bp_args(basis, features, neighbors, ranges):
-  basis, features = _f32(basis), _f32(features)
-  neighbors, ranges = _i32(neighbors), _i32(ranges)
-  _dev_check(basis, features, neighbors, ranges)
-  if neighbors.dim() != 2 or neighbors.shape[1] != 2:
-    raise _lib.TfgpcError(1, "BasisProjOp expects a neighbor tensor with 2 dimensions and 2 "
-                          "indices per neighbor.")
-  if basis.shape[0] != neighbors.shape[0]:
-    raise _lib.TfgpcError(1, "BasisProjOp expects the same number of basis as the number of "
-                          "neighbors.")
-  return basis, features, neighbors, ranges
-
-
 def read_device(values):
   """Blocking read of a small device tensor (at most 4096 bytes of int32,
   int64 or float32) into a CPU tensor, through mapped host memory instead of a
@@ -565,46 +457,19 @@ def read_device(values):
   return out
 
 
-def _bp_scratch(k, c, feat):
-  """Scratch of the tensor-core BasisProj kernels (None where the shape has none)."""
-  nbytes = _lib.lib().tfgpc_basis_proj_workspace_bytes(c_int(k), c_int(c), c_i64(feat.shape[0]))
-  if nbytes == 0:
-    return None, 0
-  return torch.empty(nbytes, dtype=torch.uint8, device=feat.device), nbytes
-
-
 def basis_proj(basis_neighbors, pt_features, neighbors, sample_neigh_indices, scratch=True):
   """BasisProj (basis_proj/cc/ops/basis_proj_ops.cpp:25-39) -> [Ns, C, K].
   scratch=False keeps the call free of temporary device memory (fp32 kernels)."""
-  basis, feat, neighbors, ranges = _bp_args(basis_neighbors, pt_features, neighbors,
-                                            sample_neigh_indices)
-  k, c, ns = basis.shape[1], feat.shape[1], ranges.shape[0]
-  out = torch.empty((ns, c, k), dtype=torch.float32, device=basis.device)
-  ws, ws_bytes = _bp_scratch(k, c, feat) if scratch else (None, 0)
-  _lib.check(_lib.lib().tfgpc_basis_proj_ws(
-      _stream(), c_int(k), c_int(c), c_i64(ns), c_i64(feat.shape[0]), c_i64(basis.shape[0]),
-      ptr(basis), ptr(feat), ptr(neighbors), ptr(ranges), ptr(out), ptr(ws), c_sz(ws_bytes)))
-  return out
+  return _lib.host().basis_proj(basis_neighbors, pt_features, neighbors, sample_neigh_indices,
+                                scratch)
 
 
 def basis_proj_grads(basis_neighbors, pt_features, neighbors, sample_neigh_indices,
                      in_gradients, scratch=True):
   """BasisProjGrads (basis_proj/cc/ops/basis_proj_ops.cpp:41-53) ->
   (basis_gradients [M, K], feat_gradients [Nin, C])."""
-  basis, feat, neighbors, ranges = _bp_args(basis_neighbors, pt_features, neighbors,
-                                            sample_neigh_indices)
-  grads = _f32(in_gradients)
-  k, c, ns = basis.shape[1], feat.shape[1], ranges.shape[0]
-  if tuple(grads.shape) != (ns, c, k):
-    raise _lib.TfgpcError(1, "BasisProjGradsOp expects gradients of shape [Ns, C, K]")
-  dbasis = torch.empty_like(basis)
-  dfeat = torch.empty_like(feat)
-  ws, ws_bytes = _bp_scratch(k, c, feat) if scratch else (None, 0)
-  _lib.check(_lib.lib().tfgpc_basis_proj_grads_ws(
-      _stream(), c_int(k), c_int(c), c_i64(ns), c_i64(feat.shape[0]), c_i64(basis.shape[0]),
-      ptr(basis), ptr(feat), ptr(neighbors), ptr(ranges), ptr(grads), ptr(dbasis), ptr(dfeat),
-      ptr(ws), c_sz(ws_bytes)))
-  return dbasis, dfeat
+  return _lib.host().basis_proj_grads(basis_neighbors, pt_features, neighbors,
+                                      sample_neigh_indices, in_gradients, scratch)
 
 
 def sampling(points, batch_ids, point_keys, num_cells, neighbors, sample_neigh_indices, mode,

@@ -1,0 +1,311 @@
+// Grids with a cell table, neighborhoods, densities and sampling.
+#include "host.h"
+
+namespace tfgpc_host {
+namespace {
+
+// Arrays of a grid by name, in the order of the struct.
+struct Field { const char* name; at::ScalarType type; };
+constexpr Field kFields[] = {
+    {"aabb_min", at::kFloat}, {"aabb_max", at::kFloat}, {"num_cells", at::kInt},
+    {"scaled_aabb_min", at::kFloat}, {"inv_cell_sizes", at::kFloat}, {"keys", at::kLong},
+    {"sorted_indices", at::kInt}, {"sorted_keys", at::kLong}, {"sorted_points", at::kFloat},
+    {"sorted_batch_ids", at::kInt}, {"packed", at::kFloat}, {"cell_start", at::kInt},
+    {"ds", at::kInt}};
+constexpr int kNumFields = 13;
+
+size_t align256(size_t x) { return (x + 255) / 256 * 256; }
+
+}  // namespace
+
+// A built grid.  All its arrays lie in one allocation; tensors of them are made when
+// asked for (most are never looked at).
+class CellGrid {
+ public:
+  tfgpc_cell_grid g{};
+  Tensor arena, points, batch_ids;
+  std::vector<Tensor> given;            // the arrays a shard's grid got from its caller
+  std::vector<int32_t> num_cells_host;
+
+  CellGrid(const Tensor& pts, const Tensor& bids, int64_t batch_size, int max_cells,
+           const py::object& cells) {
+    points = f32(pts);
+    batch_ids = i32(bids);
+    on_gpu(points);
+    on_gpu(batch_ids);
+    const int64_t n = points.size(0), d = points.size(1), b = batch_size;
+    require(batch_ids.size(0) == n, "ComputeKeysOp expects the same number of points as batch ids");
+    g.D = (int)d;
+    g.max_cells = max_cells;
+    g.n = n;
+    g.batch_size = b;
+    const int64_t table = (int64_t)tfgpc_cell_table_elems((int)d, b, max_cells);
+    const int64_t elems[kNumFields] = {b * d, b * d, d, b * d, d, n, n, n, n * d, n,
+                                       d <= 3 ? 4 * n : 0, table,
+                                       2 * b * (int64_t)max_cells * max_cells};
+    size_t offset[kNumFields], total = 0;
+    for (int i = 0; i < kNumFields; ++i) {
+      offset[i] = total;
+      total += align256((size_t)elems[i] * (kFields[i].type == at::kLong ? 8 : 4));
+    }
+    arena = bytes(total, points);
+    char* base = (char*)arena.data_ptr();
+    void** slot = (void**)&g.aabb_min;
+    for (int i = 0; i < kNumFields; ++i) slot[i] = elems[i] > 0 ? base + offset[i] : nullptr;
+    if (!cells.is_none()) {
+      for (int i : {0, 1, 3, 4}) {
+        given.push_back(f32(cells[py::str(kFields[i].name)].cast<Tensor>()));
+        slot[i] = given.back().data_ptr();
+      }
+      given.push_back(i32(cells[py::str("num_cells")].cast<Tensor>()));
+    }
+  }
+
+  const int32_t* cells_in() const { return given.empty() ? nullptr : ip(given.back()); }
+
+  Tensor get(const std::string& name) const {
+    const int64_t n = g.n, d = g.D, b = g.batch_size;
+    if (name == "aabb_min") return view(0, {b, d});
+    if (name == "aabb_max") return view(1, {b, d});
+    if (name == "num_cells") return view(2, {d});
+    if (name == "scaled_aabb_min") return view(3, {b, d});
+    if (name == "inv_cell_sizes") return view(4, {d});
+    if (name == "keys") return view(5, {n});
+    if (name == "sorted_indices") return view(6, {n});
+    if (name == "sorted_keys") return view(7, {n});
+    if (name == "sorted_points") return view(8, {n, d});
+    if (name == "sorted_batch_ids") return view(9, {n});
+    if (name == "ds") return view(12, {b, num_cells_host.at(0), num_cells_host.at(1), 2});
+    if (name == "num_cells_host") return at::tensor(at::ArrayRef<int32_t>(num_cells_host), at::kInt);
+    throw py::attribute_error(name);
+  }
+
+ private:
+  Tensor view(int field, std::vector<int64_t> shape) const {
+    void* p = ((void**)&g.aabb_min)[field];
+    for (const Tensor& t : given)
+      if (t.data_ptr() == p) return t;
+    Tensor keep = arena;
+    return at::from_blob(p, shape, [keep](void*) {}, arena.options().dtype(kFields[field].type),
+                         arena.device());
+  }
+};
+
+using GridPtr = std::shared_ptr<CellGrid>;
+
+// The samples of a neighborhood: mode 0 the two tensors, 1 the grid's points in their
+// own order, 2 the sorted points.
+struct Samples {
+  int mode = 0;
+  int64_t ns = 0;
+  Tensor points, ids;
+  const float* p() const { return mode == 0 ? fp(points) : nullptr; }
+  const int32_t* b() const { return mode == 0 ? ip(ids) : nullptr; }
+};
+
+static Samples make_samples(const CellGrid& grid, int mode, const OptTensor& points,
+                            const OptTensor& ids) {
+  Samples s;
+  s.mode = mode;
+  s.ns = grid.g.n;
+  if (mode != 0) return s;
+  require(points.has_value() && ids.has_value(), "FindNeighborsOp got no samples");
+  s.points = f32(*points);
+  s.ids = i32(*ids);
+  on_gpu(s.points);
+  on_gpu(s.ids);
+  s.ns = s.points.size(0);
+  require(s.points.size(1) == grid.g.D,
+          "FindNeighborsOp expects inputs with the dimension of the samples");
+  require(s.ids.size(0) == s.ns,
+          "FindNeighborsOp expects the same number of batch ids as samples.");
+  return s;
+}
+
+// Ranges and number of pairs of a neighborhood, and what its fill pass needs again.
+struct Count {
+  GridPtr grid;
+  Samples samples;
+  Tensor ranges, inv_radii;
+  int64_t total = 0;
+  int max_neighs = 0;
+};
+
+using CountPtr = std::shared_ptr<Count>;
+
+static std::vector<float> to_floats(const std::vector<double>& v) {
+  return std::vector<float>(v.begin(), v.end());
+}
+
+// (grid, count or None)
+static py::tuple build_grid(const Tensor& points, const Tensor& batch_ids, int64_t batch_size,
+                            const std::vector<double>& cell_sizes, int max_cells,
+                            const py::object& cells, const OptTensor& inv_radii, int mode,
+                            const OptTensor& samples, const OptTensor& sample_ids,
+                            int max_neighs) {
+  GridPtr grid = std::make_shared<CellGrid>(points, batch_ids, batch_size, max_cells, cells);
+  CountPtr count;
+  if (mode >= 0) {
+    count = std::make_shared<Count>();
+    count->grid = grid;
+    count->samples = make_samples(*grid, mode, samples, sample_ids);
+    count->inv_radii = f32(*inv_radii);
+    count->max_neighs = max_neighs;
+    count->ranges = empty({count->samples.ns}, at::kInt, grid->points);
+  }
+  const int64_t ns = count ? count->samples.ns : 0;
+  const size_t need = tfgpc_cell_grid_workspace_bytes(grid->g.D, grid->g.n, ns, batch_size, max_cells);
+  Tensor ws = bytes(need, grid->points);
+  const std::vector<float> sizes = to_floats(cell_sizes);
+  require((int)sizes.size() == grid->g.D, "GridNeighborhood expects one cell size per dimension");
+  std::vector<int32_t> nc(grid->g.D);
+  int64_t total = 0;
+  void* st = stream();
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_cell_grid_neighborhood(
+        st, &grid->g, fp(grid->points), ip(grid->batch_ids), sizes.data(), grid->cells_in(),
+        count ? fp(count->inv_radii) : nullptr, ns, count ? count->samples.p() : nullptr,
+        count ? count->samples.b() : nullptr, count ? count->samples.mode : 0, max_neighs,
+        count ? ipm(count->ranges) : nullptr, ws.data_ptr(), need, nc.data(), &total);
+  }
+  if (rc) raise_error(rc, tfgpc_last_error(), &nc);
+  grid->num_cells_host = nc;
+  if (count) count->total = total;
+  return py::make_tuple(grid, count);
+}
+
+static CountPtr count_neighbors(const GridPtr& grid, const Tensor& inv_radii, int mode,
+                                const OptTensor& samples, const OptTensor& sample_ids,
+                                int max_neighs) {
+  CountPtr c = std::make_shared<Count>();
+  c->grid = grid;
+  c->samples = make_samples(*grid, mode, samples, sample_ids);
+  c->inv_radii = f32(inv_radii);
+  c->max_neighs = max_neighs;
+  const int64_t ns = c->samples.ns;
+  c->ranges = empty({ns}, at::kInt, grid->points);
+  const size_t need = tfgpc_find_neighbors_workspace_bytes(ns);
+  Tensor ws = bytes(need, grid->points);
+  void* st = stream();
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_cells_count(st, &grid->g, fp(c->inv_radii), ns, c->samples.p(), c->samples.b(),
+                           mode, max_neighs, ipm(c->ranges), ws.data_ptr(), need, &c->total);
+  }
+  check(rc);
+  return c;
+}
+
+// (pairs with sorted indices, pairs with original indices or None)
+static py::tuple fill_neighbors(const CountPtr& c, bool with_ids) {
+  const int64_t m = c->total;
+  // one allocation: the two lists are mostly used together
+  Tensor both = empty({with_ids ? 2 : 1, m, 2}, at::kInt, c->ranges);
+  int32_t* neigh = ipm(both);
+  check(tfgpc_cells_fill(stream(), &c->grid->g, fp(c->inv_radii), c->samples.ns, c->samples.p(),
+                         c->samples.b(), c->samples.mode, c->max_neighs, ip(c->ranges), m, neigh,
+                         with_ids ? neigh + 2 * m : nullptr));
+  return py::make_tuple(both.select(0, 0),
+                        with_ids ? py::cast(both.select(0, 1)) : py::object(py::none()));
+}
+
+// Density at every point of the grid, in the unsorted (mode 1) or sorted (2) order.
+static Tensor density(const GridPtr& grid, const Tensor& inv_radii, const Tensor& inv_bandwidth,
+                      int pdf_mode, int mode) {
+  Tensor r = f32(inv_radii), bw = f32(inv_bandwidth);
+  Tensor out = empty({grid->g.n}, at::kFloat, grid->points);
+  check(tfgpc_cells_density(stream(), &grid->g, fp(r), fp(bw), pdf_mode, grid->g.n, nullptr,
+                            nullptr, mode, fpm(out)));
+  return out;
+}
+
+static py::tuple cut_samples(const Tensor& pts, const Tensor& ids, const OptTensor& idx,
+                             int64_t s) {
+  return py::make_tuple(pts.narrow(0, 0, s), ids.narrow(0, 0, s),
+                        idx ? py::cast(idx->narrow(0, 0, s)) : py::object(py::none()));
+}
+
+// (points, batch ids, original indices or None) sampled on a built grid
+static py::tuple sample(const GridPtr& grid, int mode, const Tensor& inv_radii) {
+  const int64_t n = grid->g.n;
+  Tensor r = f32(inv_radii);
+  Tensor pts = empty({n, grid->g.D}, at::kFloat, grid->points);
+  Tensor ids = empty({n}, at::kInt, grid->points);
+  OptTensor idx;
+  if (mode == 0) idx = empty({n}, at::kInt, grid->points);
+  const size_t need = tfgpc_cells_sample_workspace_bytes(n);
+  Tensor ws = bytes(need, grid->points);
+  int64_t s = 0;
+  void* st = stream();
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_cells_sample(st, &grid->g, mode, fp(r), fpm(pts), ipm(ids),
+                            idx ? ipm(*idx) : nullptr, ws.data_ptr(), need, &s);
+  }
+  check(rc);
+  return cut_samples(pts, ids, idx, s);
+}
+
+// (grid, points, batch ids, original indices or None): grid and sampling in one call
+static py::tuple build_and_sample(const Tensor& points, const Tensor& batch_ids,
+                                  int64_t batch_size, const std::vector<double>& cell_sizes,
+                                  int max_cells, const py::object& cells, int mode,
+                                  const Tensor& inv_radii) {
+  GridPtr grid = std::make_shared<CellGrid>(points, batch_ids, batch_size, max_cells, cells);
+  const int64_t n = grid->g.n;
+  Tensor r = f32(inv_radii);
+  Tensor pts = empty({n, grid->g.D}, at::kFloat, grid->points);
+  Tensor ids = empty({n}, at::kInt, grid->points);
+  OptTensor idx;
+  if (mode == 0) idx = empty({n}, at::kInt, grid->points);
+  const size_t need = tfgpc_cell_grid_workspace_bytes(grid->g.D, n, 0, batch_size, max_cells);
+  const size_t need_s = tfgpc_cells_sample_workspace_bytes(n);
+  Tensor ws = bytes(align256(need) + need_s, grid->points);
+  char* p = (char*)ws.data_ptr();
+  const std::vector<float> sizes = to_floats(cell_sizes);
+  require((int)sizes.size() == grid->g.D, "SamplingOp expects one cell size per dimension");
+  std::vector<int32_t> nc(grid->g.D);
+  int64_t s = 0;
+  void* st = stream();
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_cell_grid_sample(st, &grid->g, fp(grid->points), ip(grid->batch_ids), sizes.data(),
+                                grid->cells_in(), mode, fp(r), fpm(pts), ipm(ids),
+                                idx ? ipm(*idx) : nullptr, p, need, p + align256(need), need_s,
+                                nc.data(), &s);
+  }
+  if (rc) raise_error(rc, tfgpc_last_error(), &nc);
+  grid->num_cells_host = nc;
+  py::tuple cut = cut_samples(pts, ids, idx, s);
+  return py::make_tuple(grid, cut[0], cut[1], cut[2]);
+}
+
+void bind_cells(py::module_& m) {
+  py::class_<CellGrid, GridPtr>(m, "CellGrid")
+      .def("__getattr__", [](const CellGrid& g, const std::string& name) { return g.get(name); })
+      .def_readonly("source_points", &CellGrid::points);
+  py::class_<Count, CountPtr>(m, "Count")
+      .def_readonly("ranges", &Count::ranges)
+      .def_readonly("total", &Count::total)
+      .def_readonly("cells", &Count::grid)
+      .def_readonly("inv_radii", &Count::inv_radii)
+      .def_property_readonly("mode", [](const Count& c) { return c.samples.mode; })
+      .def_property_readonly("samples", [](const Count& c) {
+        return c.samples.mode == 0 ? c.samples.points
+               : c.samples.mode == 1 ? c.grid->points : c.grid->get("sorted_points");
+      });
+  m.def("cell_table_elems", &tfgpc_cell_table_elems);
+  m.def("build_grid", &build_grid);
+  m.def("count_neighbors", &count_neighbors);
+  m.def("fill_neighbors", &fill_neighbors);
+  m.def("density", &density);
+  m.def("sample", &sample);
+  m.def("build_and_sample", &build_and_sample);
+}
+
+}  // namespace tfgpc_host

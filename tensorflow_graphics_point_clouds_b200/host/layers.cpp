@@ -1,0 +1,288 @@
+// Kernel bases, projection and weight products, pooling and the 1x1 convolution.
+#include "host.h"
+
+namespace tfgpc_host {
+namespace {
+
+const float* maybe(const OptTensor& t, Tensor* keep) {
+  if (!t) return nullptr;
+  *keep = f32(*t);
+  return fp(*keep);
+}
+
+// ---- kernel bases ------------------------------------------------------------------
+
+Tensor pack_points_density(const Tensor& points_, const Tensor& pdf_) {
+  Tensor points = f32(points_), pdf = f32(pdf_);
+  const int64_t n = points.size(0);
+  require(points.size(1) == 3 && pdf.numel() == n,
+          "PackPointsDensity expects [n, 3] points and [n] densities");
+  Tensor out = empty({n, 4}, at::kFloat, points);
+  check(tfgpc_pack_points_density(stream(), n, fp(points), fp(pdf), fpm(out)));
+  return out;
+}
+
+// (basis [M, K] float32 or None, pair [M, 2, K] bf16 or None)
+py::tuple kernel_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
+                       const OptTensor& pdf_, const Tensor& w1_, const Tensor& b1_,
+                       double radius, int act, double alpha, int pdf_mode, bool want_f32,
+                       bool want_pair) {
+  Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), w1 = f32(w1_), b1 = f32(b1_);
+  Tensor pdf_keep;
+  const float* pdf = maybe(pdf_, &pdf_keep);
+  const int64_t m = neigh.size(0), k = w1.size(1);
+  OptTensor basis, pair;
+  if (want_f32) basis = empty({m, k}, at::kFloat, p_in);
+  if (want_pair) pair = empty({m, 2, k}, at::kBFloat16, p_in);
+  const float inv = (float)(1.0 / radius);
+  if (want_pair)
+    check(tfgpc_kernel_basis_split(stream(), (int)w1.size(0), (int)k, m, fp(p_in), fp(p_out),
+                                   ip(neigh), pdf, fp(w1), fp(b1), inv, act, (float)alpha,
+                                   pdf_mode, basis ? fpm(*basis) : nullptr, pair->data_ptr()));
+  else
+    check(tfgpc_kernel_basis(stream(), (int)w1.size(0), (int)k, m, fp(p_in), fp(p_out), ip(neigh),
+                             pdf, fp(w1), fp(b1), inv, act, (float)alpha, pdf_mode, fpm(*basis)));
+  return py::make_tuple(basis, pair);
+}
+
+py::tuple kernel_basis_grads(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
+                             const OptTensor& pdf_, const Tensor& w1_, const Tensor& b1_,
+                             double radius, const Tensor& dbasis_, int act, double alpha,
+                             int pdf_mode) {
+  Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), w1 = f32(w1_), b1 = f32(b1_),
+         dbasis = f32(dbasis_);
+  Tensor pdf_keep;
+  const float* pdf = maybe(pdf_, &pdf_keep);
+  const int64_t d = w1.size(0), k = w1.size(1);
+  Tensor both = empty({d + 1, k}, at::kFloat, p_in);   // one clear for both
+  float* dw = fpm(both);
+  check(tfgpc_kernel_basis_grads(stream(), (int)d, (int)k, neigh.size(0), fp(p_in), fp(p_out),
+                                 ip(neigh), pdf, fp(w1), fp(b1), (float)(1.0 / radius), act,
+                                 (float)alpha, pdf_mode, fp(dbasis), dw, dw + d * k));
+  return py::make_tuple(both.narrow(0, 0, d), both.select(0, d));
+}
+
+Tensor kp_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
+                const Tensor& kernel_points_, double radius, double sigma, int64_t k_pad,
+                int interpolation) {
+  Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), kp = f32(kernel_points_);
+  const int64_t m = neigh.size(0);
+  Tensor basis = empty({m, k_pad}, at::kFloat, p_in);
+  check(tfgpc_kp_basis(stream(), (int)kp.size(1), (int)k_pad, (int)kp.size(0), m, fp(p_in),
+                       fp(p_out), ip(neigh), fp(kp), (float)(1.0 / radius), (float)sigma,
+                       interpolation, fpm(basis)));
+  return basis;
+}
+
+Tensor pointconv_pdf(const Tensor& pdf_, const Tensor& ranges_, const Tensor& w1_,
+                     const Tensor& b1_, const Tensor& w2_, const Tensor& b2_) {
+  Tensor pdf = f32(pdf_), ranges = i32(ranges_), w1 = f32(w1_), b1 = f32(b1_), w2 = f32(w2_),
+         b2 = f32(b2_);
+  require(w1.numel() == 16 && b1.numel() == 16 && w2.numel() == 16 && b2.numel() == 1,
+          "PointConv's density transform has 16 hidden units");
+  Tensor out = at::empty_like(pdf);
+  check(tfgpc_pointconv_pdf(stream(), ranges.size(0), pdf.numel(), ip(ranges), fp(pdf), fp(w1),
+                            fp(b1), fp(w2), fp(b2), fpm(out)));
+  return out;
+}
+
+// ---- projection + weight product ------------------------------------------------------
+
+Tensor group_plan(const Tensor& order_, const Tensor& ranges_, const Tensor& sorted_pairs_,
+                  const Tensor& original_pairs_) {
+  Tensor order = i32(order_), ranges = i32(ranges_), a = i32(sorted_pairs_),
+         b = i32(original_pairs_);
+  const int64_t ns = ranges.size(0), m = a.size(0);
+  const size_t need = tfgpc_mcconv_group_plan_bytes(ns, m);
+  Tensor plan = bytes(need, ranges);
+  check(tfgpc_mcconv_group_plan(stream(), ns, m, ip(order), ip(ranges), ip(a), ip(b),
+                                plan.data_ptr(), need));
+  return plan;
+}
+
+Tensor project_forward(int k, int c, int cout, const Tensor& ws, const Tensor& basis_,
+                       const Tensor& features_, const Tensor& neigh_, const Tensor& ranges_,
+                       const Tensor& weights_) {
+  Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
+         weights = f32(weights_);
+  const int64_t ns = ranges.size(0);
+  Tensor out = empty({ns, cout}, at::kFloat, basis);
+  check(tfgpc_mcconv_forward(stream(), k, c, cout, ns, features.size(0), basis.size(0), fp(basis),
+                             fp(features), ip(neigh), ip(ranges), fp(weights), fpm(out),
+                             ws.data_ptr(), (size_t)ws.numel()));
+  return out;
+}
+
+py::tuple project_backward(int k, int c, int cout, const Tensor& ws, const Tensor& basis_,
+                           const Tensor& features_, const Tensor& neigh_, const Tensor& ranges_,
+                           const Tensor& weights_, const Tensor& out_grads_, bool reuse) {
+  Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
+         weights = f32(weights_), g = f32(out_grads_);
+  Tensor dbasis = at::empty_like(basis), dfeat = at::empty_like(features),
+         dw = at::empty_like(weights);
+  check(tfgpc_mcconv_backward(stream(), k, c, cout, ranges.size(0), features.size(0),
+                              basis.size(0), fp(basis), fp(features), ip(neigh), ip(ranges),
+                              fp(weights), fp(g), reuse, fpm(dbasis), fpm(dfeat), fpm(dw),
+                              ws.data_ptr(), (size_t)ws.numel()));
+  return py::make_tuple(dbasis, dfeat, dw);
+}
+
+Tensor project_forward_grouped(int k, int c, int cout, int64_t ns, const Tensor& ws,
+                               const Tensor& pair, const Tensor& features_, const Tensor& weights_,
+                               const Tensor& order_, const Tensor& plan) {
+  Tensor features = f32(features_), weights = f32(weights_), order = i32(order_);
+  Tensor out = empty({ns, cout}, at::kFloat, features);
+  check(tfgpc_mcconv_forward_grouped(stream(), k, c, cout, ns, features.size(0), pair.size(0),
+                                     pair.data_ptr(), fp(features), fp(weights), ip(order),
+                                     plan.data_ptr(), fpm(out), ws.data_ptr(), (size_t)ws.numel()));
+  return out;
+}
+
+py::tuple project_backward_grouped(int k, int c, int cout, int64_t ns, const Tensor& ws,
+                                   const Tensor& pair, const Tensor& features_,
+                                   const Tensor& ranges_, const Tensor& weights_,
+                                   const Tensor& out_grads_, bool reuse, const Tensor& order_,
+                                   const Tensor& plan) {
+  Tensor features = f32(features_), ranges = i32(ranges_), weights = f32(weights_),
+         g = f32(out_grads_), order = i32(order_);
+  const int64_t m = pair.size(0);
+  Tensor dbasis = empty({m, pair.size(2)}, at::kFloat, features);
+  Tensor dfeat = at::empty_like(features), dw = at::empty_like(weights);
+  check(tfgpc_mcconv_backward_grouped(stream(), k, c, cout, ns, features.size(0), m,
+                                      pair.data_ptr(), fp(features), ip(ranges), fp(weights),
+                                      fp(g), reuse, ip(order), plan.data_ptr(), fpm(dbasis),
+                                      fpm(dfeat), fpm(dw), ws.data_ptr(), (size_t)ws.numel()));
+  return py::make_tuple(dbasis, dfeat, dw);
+}
+
+// Status word of a projection or product workspace; blocks on the stream.
+void check_status(const Tensor& ws) {
+  int status = 0, rc;
+  void* st = stream();
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_mcconv_status(st, ws.data_ptr(), &status);
+  }
+  check(rc);
+}
+
+Tensor matmul_f32(const Tensor& a_, const Tensor& b_, bool a_t, bool b_t) {
+  Tensor a = f32(a_), b = f32(b_);
+  const int64_t m = a.size(a_t ? 1 : 0), k = a.size(a_t ? 0 : 1), n = b.size(b_t ? 0 : 1);
+  require(b.size(b_t ? 1 : 0) == k, "matmul expects matching inner dimensions");
+  Tensor c = empty({m, n}, at::kFloat, a);
+  const size_t need = tfgpc_matmul_workspace_bytes(m, n, k);
+  Tensor ws = bytes(need, a);
+  check(tfgpc_matmul_f32(stream(), m, n, k, fp(a), a_t, fp(b), b_t, fpm(c), ws.data_ptr(), need));
+  check_status(ws);
+  return c;
+}
+
+// ---- the drop-in projection op ----------------------------------------------------------
+
+struct ProjArgs {
+  Tensor basis, features, neigh, ranges, ws;
+  int k, c;
+  ProjArgs(const Tensor& b, const Tensor& f, const Tensor& nb, const Tensor& r, bool scratch)
+      : basis(f32(b)), features(f32(f)), neigh(i32(nb)), ranges(i32(r)) {
+    for (const Tensor* t : {&basis, &features, &neigh, &ranges}) on_gpu(*t);
+    require(neigh.dim() == 2 && neigh.size(1) == 2,
+            "BasisProjOp expects a neighbor tensor with 2 dimensions and 2 indices per neighbor.");
+    require(basis.size(0) == neigh.size(0),
+            "BasisProjOp expects the same number of basis as the number of neighbors.");
+    k = (int)basis.size(1);
+    c = (int)features.size(1);
+    const size_t need = scratch ? tfgpc_basis_proj_workspace_bytes(k, c, features.size(0)) : 0;
+    if (need) ws = bytes(need, features);
+  }
+  void* ws_ptr() const { return ws.defined() ? ws.data_ptr() : nullptr; }
+  size_t ws_bytes() const { return ws.defined() ? (size_t)ws.numel() : 0; }
+};
+
+Tensor basis_proj(const Tensor& basis, const Tensor& features, const Tensor& neigh,
+                  const Tensor& ranges, bool scratch) {
+  ProjArgs a(basis, features, neigh, ranges, scratch);
+  const int64_t ns = a.ranges.size(0);
+  Tensor out = empty({ns, a.c, a.k}, at::kFloat, a.basis);
+  check(tfgpc_basis_proj_ws(stream(), a.k, a.c, ns, a.features.size(0), a.basis.size(0),
+                            fp(a.basis), fp(a.features), ip(a.neigh), ip(a.ranges), fpm(out),
+                            a.ws_ptr(), a.ws_bytes()));
+  return out;
+}
+
+py::tuple basis_proj_grads(const Tensor& basis, const Tensor& features, const Tensor& neigh,
+                           const Tensor& ranges, const Tensor& in_grads, bool scratch) {
+  ProjArgs a(basis, features, neigh, ranges, scratch);
+  Tensor g = f32(in_grads);
+  const int64_t ns = a.ranges.size(0);
+  require(g.dim() == 3 && g.size(0) == ns && g.size(1) == a.c && g.size(2) == a.k,
+          "BasisProjGradsOp expects gradients of shape [Ns, C, K]");
+  Tensor dbasis = at::empty_like(a.basis), dfeat = at::empty_like(a.features);
+  check(tfgpc_basis_proj_grads_ws(stream(), a.k, a.c, ns, a.features.size(0), a.basis.size(0),
+                                  fp(a.basis), fp(a.features), ip(a.neigh), ip(a.ranges), fp(g),
+                                  fpm(dbasis), fpm(dfeat), a.ws_ptr(), a.ws_bytes()));
+  return py::make_tuple(dbasis, dfeat);
+}
+
+// ---- pooling, bias, activation ------------------------------------------------------------
+
+Tensor neighborhood_pool(const Tensor& features_, const Tensor& neigh_, const Tensor& ranges_,
+                         int mode) {
+  Tensor features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_);
+  const int64_t ns = ranges.size(0), c = features.size(1);
+  Tensor out = empty({ns, c}, at::kFloat, features);
+  check(tfgpc_neighborhood_pool(stream(), mode, (int)c, ns, features.size(0), neigh.size(0),
+                                fp(features), ip(neigh), ip(ranges), fpm(out)));
+  return out;
+}
+
+Tensor global_pool(const Tensor& features_, const Tensor& ids_, int64_t batch, int mode) {
+  Tensor features = f32(features_), ids = i32(ids_);
+  const int64_t n = features.size(0), c = features.size(1);
+  Tensor out = empty({batch, c}, at::kFloat, features);
+  const size_t need = tfgpc_global_pool_workspace_bytes(batch);
+  Tensor ws = bytes(need, features);
+  check(tfgpc_global_pool(stream(), mode, (int)c, n, batch, fp(features), ip(ids), fpm(out),
+                          ws.data_ptr(), need));
+  return out;
+}
+
+void add_bias_(const Tensor& x, const Tensor& bias_) {
+  Tensor bias = f32(bias_);
+  check(tfgpc_add_bias(stream(), x.size(0), (int)x.size(1), fpm(x), fp(bias)));
+}
+
+void scale_bias_activation_(const Tensor& x, double scale, const OptTensor& bias_, bool act,
+                            double alpha) {
+  require(x.is_contiguous() && x.scalar_type() == at::kFloat,
+          "scale_bias_activation_ expects a contiguous float32 tensor");
+  Tensor keep;
+  const float* bias = maybe(bias_, &keep);
+  check(tfgpc_scale_bias_activation(stream(), x.size(0), (int)x.size(1), fpm(x), (float)scale, bias,
+                                    act, (float)alpha));
+}
+
+}  // namespace
+
+void bind_layers(py::module_& m) {
+  m.def("pack_points_density", &pack_points_density);
+  m.def("kernel_basis", &kernel_basis);
+  m.def("kernel_basis_grads", &kernel_basis_grads);
+  m.def("kp_basis", &kp_basis);
+  m.def("pointconv_pdf", &pointconv_pdf);
+  m.def("group_plan", &group_plan);
+  m.def("project_forward", &project_forward);
+  m.def("project_backward", &project_backward);
+  m.def("project_forward_grouped", &project_forward_grouped);
+  m.def("project_backward_grouped", &project_backward_grouped);
+  m.def("check_status", &check_status);
+  m.def("matmul_f32", &matmul_f32);
+  m.def("basis_proj", &basis_proj);
+  m.def("basis_proj_grads", &basis_proj_grads);
+  m.def("neighborhood_pool", &neighborhood_pool);
+  m.def("global_pool", &global_pool);
+  m.def("add_bias_", &add_bias_);
+  m.def("scale_bias_activation_", &scale_bias_activation_);
+}
+
+}  // namespace tfgpc_host

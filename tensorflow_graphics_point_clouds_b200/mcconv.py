@@ -19,21 +19,7 @@ from .custom_ops import _stream, _f32, _i32, _workspace
 
 def matmul_f32(a, b, a_transposed=False, b_transposed=False):
   """c = op(a) @ op(b) in fp32 accuracy on the tensor cores (tfgpc_matmul_f32)."""
-  a, b = _f32(a), _f32(b)
-  m, k = (a.shape[1], a.shape[0]) if a_transposed else a.shape
-  n = b.shape[0] if b_transposed else b.shape[1]
-  kb = b.shape[1] if b_transposed else b.shape[0]
-  if kb != k:
-    raise _lib.TfgpcError(1, "matmul expects matching inner dimensions")
-  c = torch.empty((m, n), dtype=torch.float32, device=a.device)
-  nbytes = _lib.lib().tfgpc_matmul_workspace_bytes(c_i64(m), c_i64(n), c_i64(k))
-  ws = _workspace(nbytes, a.device)
-  _lib.check(_lib.lib().tfgpc_matmul_f32(
-      _stream(), c_i64(m), c_i64(n), c_i64(k), ptr(a), c_int(int(a_transposed)), ptr(b),
-      c_int(int(b_transposed)), ptr(c), ptr(ws), c_sz(nbytes)))
-  status = c_int(0)
-  _lib.check(_lib.lib().tfgpc_mcconv_status(_stream(), ptr(ws), ctypes.byref(status)))
-  return c
+  return _lib.host().matmul_f32(a, b, bool(a_transposed), bool(b_transposed))
 
 
 class ProjectionGemm:
@@ -47,7 +33,7 @@ class ProjectionGemm:
     self.backward_ws = bool(backward)
     self.device = device
     self.n_in, self.nbytes, self.ws = -1, 0, None
-    self._x_valid = False
+    self._x_valid = self._x_grouped = False
     if n_in is not None:
       self._ensure_workspace(int(n_in))
 
@@ -62,14 +48,9 @@ class ProjectionGemm:
     self._x_valid = False
 
   def forward(self, basis, features, neighbors, ranges, weights):
-    basis, features, weights = _f32(basis), _f32(features), _f32(weights)
-    neighbors, ranges = _i32(neighbors), _i32(ranges)
-    out = torch.empty((self.ns, self.cout), dtype=torch.float32, device=basis.device)
     self._ensure_workspace(features.shape[0])
-    _lib.check(_lib.lib().tfgpc_mcconv_forward(
-        _stream(), c_int(self.k), c_int(self.c), c_int(self.cout), c_i64(self.ns),
-        c_i64(features.shape[0]), c_i64(basis.shape[0]), ptr(basis), ptr(features),
-        ptr(neighbors), ptr(ranges), ptr(weights), ptr(out), ptr(self.ws), c_sz(self.nbytes)))
+    out = _lib.host().project_forward(self.k, self.c, self.cout, self.ws, basis, features,
+                                      neighbors, ranges, weights)
     self._x_valid = self.backward_ws
     self._x_grouped = False
     return out
@@ -77,31 +58,18 @@ class ProjectionGemm:
   def backward(self, basis, features, neighbors, ranges, weights, out_grads, reuse_forward=True):
     if not self.backward_ws:
       raise RuntimeError("this ProjectionGemm was created without backward workspace")
-    basis, features, weights = _f32(basis), _f32(features), _f32(weights)
-    neighbors, ranges, out_grads = _i32(neighbors), _i32(ranges), _f32(out_grads)
-    dbasis = torch.empty_like(basis)
-    dfeat = torch.empty_like(features)
-    dw = torch.empty_like(weights)
     self._ensure_workspace(features.shape[0])
-    _lib.check(_lib.lib().tfgpc_mcconv_backward(
-        _stream(), c_int(self.k), c_int(self.c), c_int(self.cout), c_i64(self.ns),
-        c_i64(features.shape[0]), c_i64(basis.shape[0]), ptr(basis), ptr(features),
-        ptr(neighbors), ptr(ranges), ptr(weights), ptr(out_grads),
-        c_int(int(reuse_forward and self._x_valid and not getattr(self, '_x_grouped', False))),
-        ptr(dbasis), ptr(dfeat), ptr(dw), ptr(self.ws), c_sz(self.nbytes)))
-    return dbasis, dfeat, dw
+    reuse = bool(reuse_forward and self._x_valid and not self._x_grouped)
+    return _lib.host().project_backward(self.k, self.c, self.cout, self.ws, basis, features,
+                                        neighbors, ranges, weights, out_grads, reuse)
 
   def forward_grouped(self, basis_pair, features, weights, order, plan):
     """The forward pass through tfgpc_mcconv_forward_grouped: the projection runs
     once per distinct neighbor of a group of four samples (taken in `order`)
     instead of once per pair; basis_pair [M, 2, K] bf16."""
-    features, weights = _f32(features), _f32(weights)
-    out = torch.empty((self.ns, self.cout), dtype=torch.float32, device=features.device)
     self._ensure_workspace(features.shape[0])
-    _lib.check(_lib.lib().tfgpc_mcconv_forward_grouped(
-        _stream(), c_int(self.k), c_int(self.c), c_int(self.cout), c_i64(self.ns),
-        c_i64(features.shape[0]), c_i64(basis_pair.shape[0]), ptr(basis_pair), ptr(features),
-        ptr(weights), ptr(_i32(order)), ptr(plan), ptr(out), ptr(self.ws), c_sz(self.nbytes)))
+    out = _lib.host().project_forward_grouped(self.k, self.c, self.cout, self.ns, self.ws,
+                                              basis_pair, features, weights, order, plan)
     self._x_valid = self.backward_ws
     self._x_grouped = True
     return out
@@ -110,25 +78,15 @@ class ProjectionGemm:
                        reuse_forward=True):
     """The gradients through tfgpc_mcconv_backward_grouped (dbasis [M, K] fp32,
     dfeat, dweights)."""
-    features, weights = _f32(features), _f32(weights)
-    ranges, out_grads = _i32(ranges), _f32(out_grads)
-    m, k = basis_pair.shape[0], basis_pair.shape[2]
-    dbasis = torch.empty((m, k), dtype=torch.float32, device=features.device)
-    dfeat = torch.empty_like(features)
-    dw = torch.empty_like(weights)
     self._ensure_workspace(features.shape[0])
-    reuse = reuse_forward and self._x_valid and getattr(self, '_x_grouped', False)
-    _lib.check(_lib.lib().tfgpc_mcconv_backward_grouped(
-        _stream(), c_int(self.k), c_int(self.c), c_int(self.cout), c_i64(self.ns),
-        c_i64(features.shape[0]), c_i64(m), ptr(basis_pair), ptr(features), ptr(ranges),
-        ptr(weights), ptr(out_grads), c_int(int(reuse)), ptr(_i32(order)), ptr(plan), ptr(dbasis),
-        ptr(dfeat), ptr(dw), ptr(self.ws), c_sz(self.nbytes)))
-    return dbasis, dfeat, dw
+    reuse = bool(reuse_forward and self._x_valid and self._x_grouped)
+    return _lib.host().project_backward_grouped(self.k, self.c, self.cout, self.ns, self.ws,
+                                                basis_pair, features, ranges, weights, out_grads,
+                                                reuse, order, plan)
 
   def check_status(self):
     """Blocks on the stream; raises TfgpcError(4) if a GEMM wait timed out."""
-    status = c_int(0)
-    _lib.check(_lib.lib().tfgpc_mcconv_status(_stream(), ptr(self.ws), ctypes.byref(status)))
+    _lib.host().check_status(self.ws)
 
 
 def dense_final_weights(wf, cin, hidden):
@@ -160,14 +118,7 @@ def pack_points_density(points, pdf):
   """[n, 4] table (x, y, z, 1 / density) of a 3-D cloud and its per-point
   densities (tfgpc_pack_points_density): points_in of the kernel-basis entries
   with pdf_by_neighbor=2."""
-  points, pdf = _f32(points), _f32(pdf).reshape(-1)
-  n = points.shape[0]
-  if points.shape[1] != 3 or pdf.shape[0] != n:
-    raise _lib.TfgpcError(1, "PackPointsDensity expects [n, 3] points and [n] densities")
-  out = torch.empty((n, 4), dtype=torch.float32, device=points.device)
-  _lib.check(_lib.lib().tfgpc_pack_points_density(_stream(), c_i64(n), ptr(points), ptr(pdf),
-                                                  ptr(out)))
-  return out
+  return _lib.host().pack_points_density(points, pdf)
 
 
 def kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, radius, activation=0,
@@ -176,17 +127,8 @@ def kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, radius, activati
   w1 [D, K], b1 [K]; neighbors hold (index into points_in, index into points_out).
   pdf_by_neighbor: pdf is a table with one density per point of points_in, read
   at the pair's neighbor index, instead of the per-pair array."""
-  points_in, points_out = _f32(points_in), _f32(points_out)
-  pdf = None if pdf is None else _f32(pdf)
-  w1, b1, neighbors = _f32(w1), _f32(b1).reshape(-1), _i32(neighbors)
-  d, k = w1.shape
-  m = neighbors.shape[0]
-  basis = torch.empty((m, k), dtype=torch.float32, device=points_in.device)
-  _lib.check(_lib.lib().tfgpc_kernel_basis(
-      _stream(), c_int(d), c_int(k), c_i64(m), ptr(points_in), ptr(points_out), ptr(neighbors),
-      ptr(pdf), ptr(w1), ptr(b1), ctypes.c_float(1.0 / float(radius)), c_int(activation),
-      ctypes.c_float(alpha), c_int(int(pdf_by_neighbor)), ptr(basis)))
-  return basis
+  return _lib.host().kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, float(radius),
+                                  activation, alpha, int(pdf_by_neighbor), True, False)[0]
 
 
 def kernel_basis_split(points_in, points_out, neighbors, pdf, w1, b1, radius, activation=0,
@@ -194,19 +136,8 @@ def kernel_basis_split(points_in, points_out, neighbors, pdf, w1, b1, radius, ac
   """kernel_basis that returns every row as the bf16 (hi, mid) pair the
   tensor-core kernels multiply with: (basis [M, K] float32 or None, pair
   [M, 2, K] bf16)."""
-  points_in, points_out = _f32(points_in), _f32(points_out)
-  pdf = None if pdf is None else _f32(pdf)
-  w1, b1, neighbors = _f32(w1), _f32(b1).reshape(-1), _i32(neighbors)
-  d, k = w1.shape
-  m = neighbors.shape[0]
-  basis = (torch.empty((m, k), dtype=torch.float32, device=points_in.device) if want_fp32
-           else None)
-  pair = torch.empty((m, 2, k), dtype=torch.bfloat16, device=points_in.device)
-  _lib.check(_lib.lib().tfgpc_kernel_basis_split(
-      _stream(), c_int(d), c_int(k), c_i64(m), ptr(points_in), ptr(points_out), ptr(neighbors),
-      ptr(pdf), ptr(w1), ptr(b1), ctypes.c_float(1.0 / float(radius)), c_int(activation),
-      ctypes.c_float(alpha), c_int(int(pdf_by_neighbor)), ptr(basis), ptr(pair)))
-  return basis, pair
+  return _lib.host().kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, float(radius),
+                                  activation, alpha, int(pdf_by_neighbor), bool(want_fp32), True)
 
 
 def group_plan(neighborhood, order=None):
@@ -214,19 +145,14 @@ def group_plan(neighborhood, order=None):
   the samples four at a time in `order` (default: the neighborhood's own visiting
   order, else the sample order), every group's distinct neighbors and the pairs
   that reach them.  Returns (order [ns] int32, plan buffer)."""
-  ranges = _i32(neighborhood._samples_neigh_ranges)
-  ns, m = ranges.shape[0], neighborhood._neighbors.shape[0]
+  ranges = neighborhood._samples_neigh_ranges
   if order is None:
     order = getattr(neighborhood, '_sample_order', None)
   if order is None:
-    order = torch.arange(ns, dtype=torch.int32, device=ranges.device)
+    order = torch.arange(ranges.shape[0], dtype=torch.int32, device=ranges.device)
   order = _i32(order)
-  nbytes = _lib.lib().tfgpc_mcconv_group_plan_bytes(c_i64(ns), c_i64(m))
-  plan = _workspace(nbytes, ranges.device)
-  _lib.check(_lib.lib().tfgpc_mcconv_group_plan(
-      _stream(), c_i64(ns), c_i64(m), ptr(order), ptr(ranges), ptr(_i32(neighborhood._neighbors)),
-      ptr(_i32(neighborhood._original_neigh_ids)), ptr(plan), c_sz(nbytes)))
-  return order, plan
+  return order, _lib.host().group_plan(order, ranges, neighborhood._neighbors,
+                                       neighborhood._original_neigh_ids)
 
 
 def _mlp_blocks(weights, biases):
@@ -291,24 +217,18 @@ def kernel_mlp_grads(points_in, points_out, neighbors, pdf, weights, biases, rad
 def kernel_basis_grads(points_in, points_out, neighbors, pdf, w1, b1, radius, basis_grads,
                        activation=0, alpha=0.2, pdf_by_neighbor=False):
   """Gradients of kernel_basis with respect to w1 and b1 (tfgpc_kernel_basis_grads)."""
-  points_in, points_out = _f32(points_in), _f32(points_out)
-  pdf = None if pdf is None else _f32(pdf)
-  w1, b1, neighbors = _f32(w1), _f32(b1).reshape(-1), _i32(neighbors)
-  basis_grads = _f32(basis_grads)
-  d, k = w1.shape
-  dw1 = torch.empty_like(w1)
-  db1 = torch.empty_like(b1)
-  _lib.check(_lib.lib().tfgpc_kernel_basis_grads(
-      _stream(), c_int(d), c_int(k), c_i64(neighbors.shape[0]), ptr(points_in), ptr(points_out),
-      ptr(neighbors), ptr(pdf), ptr(w1), ptr(b1), ctypes.c_float(1.0 / float(radius)),
-      c_int(activation), ctypes.c_float(alpha), c_int(int(pdf_by_neighbor)), ptr(basis_grads),
-      ptr(dw1), ptr(db1)))
-  return dw1, db1
+  return _lib.host().kernel_basis_grads(points_in, points_out, neighbors, pdf, w1, b1,
+                                        float(radius), basis_grads, activation, alpha,
+                                        int(pdf_by_neighbor))
 
 
 # MCConv.py:27-31 / PointConv.py:27-31: name -> (activation code, slope) of the kernel-basis entries
 NON_LINEARITIES = {'relu': (0, 0.0), 'lrelu': (0, 0.2), 'leakyrelu': (0, 0.2),
                    'leaky_relu': (0, 0.2), 'elu': (1, 0.0)}
+
+
+def _grouped_supported(k, c):
+  return _lib.lib().tfgpc_mcconv_grouped_supported(c_int(k), c_int(c)) != 0
 
 
 class MCConv:
@@ -345,6 +265,8 @@ class MCConv:
 
   def _flat_kernel_weights(self):
     # [G, D, H] -> [D, G*H]: column k = g*H + h (MCConv.py:169-171)
+    if self.num_mlps == 1:
+      return self.w1[0], self.b1.reshape(self.k)
     return (self.w1.permute(1, 0, 2).reshape(self.dims, self.k).contiguous(),
             self.b1.reshape(self.k).contiguous())
 
@@ -370,7 +292,7 @@ class MCConv:
     # wide layers run on a group plan (see group_plan)
     grouped = (one_layer and self.grouped and neigh._neighbors.shape[0] > 0 and
                self.cout >= 128 and
-               _lib.lib().tfgpc_mcconv_grouped_supported(c_int(self.k), c_int(self.cin)) != 0)
+               _grouped_supported(self.k, self.cin))
     # (points, 1 / density) as one 16-byte row per point: one gather per pair
     kb_in, kb_pdf, kb_mode = p_in, pdf, int(by_nbr)
     if one_layer and by_nbr and self.dims == 3:
@@ -442,7 +364,8 @@ class MCConv:
     kb_in, kb_pdf, kb_mode = self._kb_inputs
     dw1, db1 = kernel_basis_grads(kb_in, pc_out._points, ids, kb_pdf, w1, b1, radius, dbasis,
                                   self.activation, self.alpha, pdf_by_neighbor=kb_mode)
-    dw1 = dw1.reshape(self.dims, self.num_mlps, self.hidden).permute(1, 0, 2).contiguous()
+    dw1 = (dw1.unsqueeze(0) if self.num_mlps == 1 else
+           dw1.reshape(self.dims, self.num_mlps, self.hidden).permute(1, 0, 2).contiguous())
     db1 = db1.reshape(self.num_mlps, 1, self.hidden)
     if self._list_form:
       return dfeat, [dw1], [db1], dwf
@@ -473,32 +396,14 @@ def kp_basis(points_in, points_out, neighbors, kernel_points, radius, sigma, k_p
              interpolation='linear'):
   """basis[m, k] = weighting(|diff_m - kernel_points[k]|, sigma), zero for the
   padding columns (tfgpc_kp_basis; KPConv.py:194-212)."""
-  points_in, points_out = _f32(points_in), _f32(points_out)
-  kernel_points, neighbors = _f32(kernel_points), _i32(neighbors)
-  num_kp, d = kernel_points.shape
-  m = neighbors.shape[0]
-  basis = torch.empty((m, k_pad), dtype=torch.float32, device=points_in.device)
-  _lib.check(_lib.lib().tfgpc_kp_basis(
-      _stream(), c_int(d), c_int(k_pad), c_int(num_kp), c_i64(m), ptr(points_in),
-      ptr(points_out), ptr(neighbors), ptr(kernel_points), ctypes.c_float(1.0 / float(radius)),
-      ctypes.c_float(float(sigma)), c_int({'linear': 0, 'gaussian': 1}[interpolation]),
-      ptr(basis)))
-  return basis
+  return _lib.host().kp_basis(points_in, points_out, neighbors, kernel_points, float(radius),
+                              float(sigma), int(k_pad), {'linear': 0, 'gaussian': 1}[interpolation])
 
 
 def pointconv_pdf(pdf, ranges, w1, b1, w2, b2):
   """Per pair relu(pdf / max over the sample * w1 + b1) . w2 + b2
   (tfgpc_pointconv_pdf; PointConv.py:168-183)."""
-  pdf, ranges = _f32(pdf), _i32(ranges)
-  w1, b1 = _f32(w1).reshape(-1), _f32(b1).reshape(-1)
-  w2, b2 = _f32(w2).reshape(-1), _f32(b2).reshape(-1)
-  if w1.numel() != 16 or b1.numel() != 16 or w2.numel() != 16 or b2.numel() != 1:
-    raise _lib.TfgpcError(1, "PointConv's density transform has 16 hidden units")
-  out = torch.empty_like(pdf)
-  _lib.check(_lib.lib().tfgpc_pointconv_pdf(
-      _stream(), c_i64(ranges.shape[0]), c_i64(pdf.shape[0]), ptr(ranges), ptr(pdf), ptr(w1),
-      ptr(b1), ptr(w2), ptr(b2), ptr(out)))
-  return out
+  return _lib.host().pointconv_pdf(pdf, ranges, w1, b1, w2, b2)
 
 
 class _ProjectedConv:
@@ -626,37 +531,23 @@ POOL_MODES = {'max': 0, 'avg': 1, 'average': 1, 'mean': 1}
 def neighborhood_pool(features, neighborhood, mode='max'):
   """MaxPooling / AveragePooling over a neighborhood (Pooling.py:148-162):
   [N_in, C] -> [N_out, C]."""
-  features = _f32(features)
-  nb, ranges = _i32(neighborhood._original_neigh_ids), _i32(neighborhood._samples_neigh_ranges)
-  ns, c = ranges.shape[0], features.shape[1]
-  out = torch.empty((ns, c), dtype=torch.float32, device=features.device)
-  _lib.check(_lib.lib().tfgpc_neighborhood_pool(
-      _stream(), c_int(POOL_MODES[mode]), c_int(c), c_i64(ns), c_i64(features.shape[0]),
-      c_i64(nb.shape[0]), ptr(features), ptr(nb), ptr(ranges), ptr(out)))
-  return out
+  return _lib.host().neighborhood_pool(features, neighborhood._original_neigh_ids,
+                                       neighborhood._samples_neigh_ranges, POOL_MODES[mode])
 
 
 def local_pool(features, point_cloud_in, point_cloud_out, pooling_radius, mode='max'):
   """Pooling.py:140-162: grid of the input cloud, neighborhood around the output
   points, pooled features."""
   from . import pc
-  grid = pc.Grid(point_cloud_in, pooling_radius)
-  return neighborhood_pool(features, pc.Neighborhood(grid, pooling_radius, point_cloud_out), mode)
+  return neighborhood_pool(
+      features, pc.grid_neighborhood(point_cloud_in, pooling_radius, point_cloud_out), mode)
 
 
 def global_pool(features, point_cloud, mode='max'):
   """GlobalMaxPooling / GlobalAveragePooling (Pooling.py:51-57, 90-96):
   [N, C] -> [batch_size, C]."""
-  features, bids = _f32(features), _i32(point_cloud._batch_ids)
-  n, c = features.shape
-  b = int(point_cloud._batch_size)
-  out = torch.empty((b, c), dtype=torch.float32, device=features.device)
-  nbytes = _lib.lib().tfgpc_global_pool_workspace_bytes(c_i64(b))
-  ws = _workspace(nbytes, features.device)
-  _lib.check(_lib.lib().tfgpc_global_pool(
-      _stream(), c_int(POOL_MODES[mode]), c_int(c), c_i64(n), c_i64(b), ptr(features), ptr(bids),
-      ptr(out), ptr(ws), c_sz(nbytes)))
-  return out
+  return _lib.host().global_pool(features, point_cloud._batch_ids, int(point_cloud._batch_size),
+                                 POOL_MODES[mode])
 
 
 def conv1x1(features, weights, bias):
@@ -673,19 +564,13 @@ def conv1x1(features, weights, bias):
     weights = torch.nn.functional.pad(weights, (0, cout_p - cout, 0, cin_p - cin))
     bias = torch.nn.functional.pad(bias, (0, cout_p - cout))
   out = matmul_f32(features, weights)
-  _lib.check(_lib.lib().tfgpc_add_bias(_stream(), c_i64(n), c_int(cout_p), ptr(out), ptr(bias)))
+  _lib.host().add_bias_(out, bias)
   return out[:, :cout] if cout_p != cout else out
 
 
 def scale_bias_activation_(x, scale=1.0, bias=None, leaky_alpha=None):
   """In place x = act(x * scale + bias) (tfgpc_scale_bias_activation): inference
   batch normalisation folded into scale / bias, then an optional leaky ReLU."""
-  if not x.is_contiguous() or x.dtype != torch.float32:
-    raise _lib.TfgpcError(1, "scale_bias_activation_ expects a contiguous float32 tensor")
-  n, c = x.shape
-  b = None if bias is None else _f32(bias).reshape(-1)
-  _lib.check(_lib.lib().tfgpc_scale_bias_activation(
-      _stream(), c_i64(n), c_int(c), ptr(x), ctypes.c_float(float(scale)),
-      ptr(b) if b is not None else ctypes.c_void_p(0), c_int(0 if leaky_alpha is None else 1),
-      ctypes.c_float(0.0 if leaky_alpha is None else float(leaky_alpha))))
+  _lib.host().scale_bias_activation_(x, float(scale), bias, leaky_alpha is not None,
+                                     0.0 if leaky_alpha is None else float(leaky_alpha))
   return x

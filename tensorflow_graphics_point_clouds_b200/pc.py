@@ -12,7 +12,6 @@ expressions of the reference one to one, and the ops themselves run through
 `custom_ops` (the C ABI).
 """
 import math
-import types
 
 import torch
 
@@ -116,18 +115,17 @@ def _reduced_cells(pc, sizes):
   return cells
 
 
-def _cell_grid(pc, sizes, cells, **neighborhood):
-  """(ops.CellGrid of a cloud, count of the neighborhood if one is given), or (None,
-  None) if its cell table would be too large."""
+def _cell_grid(pc, sizes, build, **args):
+  """build (ops.build_cell_grid or ops.build_cell_grid_and_sample) on a cloud with the
+  bound of cells it needs; None if the cell table would be too large."""
   d, b = pc._dimension, pc._batch_size
   max_cells = _MAX_CELLS.get((d, b), _FIRST_BOUND)
   while max_cells and ops.cell_table_elems(d, b, max_cells):
     try:
-      return ops.CellGrid.build(pc._points, pc._batch_ids, b, sizes, max_cells, cells=cells,
-                                **neighborhood)
+      return build(pc._points, pc._batch_ids, b, sizes, max_cells, **args)
     except ops._lib.TfgpcError as err:
       max_cells = _raise_bound(pc, err, max_cells)
-  return None, None
+  return None
 
 
 class Grid:
@@ -142,9 +140,9 @@ class Grid:
     if pc._points.shape[0] > 0:
       sizes = _host_dims(cell_sizes, pc._dimension)
       cells = _reduced_cells(pc, sizes)
-      table, _ = _cell_grid(pc, sizes, cells)
-      if table is not None:
-        self._adopt(pc, table)
+      built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells)
+      if built is not None:
+        self._adopt(pc, built[0])
         return
     self._cells = None
     self._point_cloud = pc
@@ -174,21 +172,26 @@ class Grid:
     self._fast_DS = None
 
   def _adopt(self, pc, built):
-    """Takes over the arrays of an ops.CellGrid."""
+    """Takes over a grid of ops.build_cell_grid."""
     self._cells = built
     self._point_cloud = pc
     self._batch_size = pc._batch_size
-    self._aabb_min, self._aabb_max = built.aabb_min, built.aabb_max
-    if pc._aabb is None:
-      pc._aabb = (self._aabb_min, self._aabb_max)
-    self._num_cells, self._num_cells_host = built.num_cells, built.num_cells_host
-    self._scaled_aabb_min, self._inv_cell_sizes = built.scaled_aabb_min, built.inv_cell_sizes
-    self._cur_keys = built.keys
-    self._sorted_indices, self._sorted_keys = built.sorted_indices, built.sorted_keys
-    self._sorted_points, self._sorted_batch_ids = built.sorted_points, built.sorted_batch_ids
-    self._fast_DS = built.ds
+    self._fast_DS = None
+
+  _FIELDS = {'_cur_keys': 'keys'}
+
+  def __getattr__(self, name):
+    # arrays of a grid built through a cell table become tensors when first asked for
+    cells = self.__dict__.get('_cells')
+    if cells is None or not name.startswith('_') or name.startswith('__'):
+      raise AttributeError(name)
+    value = getattr(cells, self._FIELDS.get(name, name[1:]))
+    self.__dict__[name] = value
+    return value
 
   def get_DS(self):
+    if self._fast_DS is None and self._cells is not None:
+      self._fast_DS = self._cells.ds
     if self._fast_DS is None:
       self._fast_DS = ops.build_grid_ds(self._sorted_keys, self._num_cells,
                                         self._num_cells_host, self._batch_size)
@@ -202,41 +205,64 @@ class Neighborhood:
 
   def __init__(self, grid, radius, point_cloud_sample=None, max_neighbors=0):
     self._attach(grid, radius, point_cloud_sample, max_neighbors)
-    smp = self._point_cloud_sampled
-    if grid._cells is not None:
-      self._take_count(grid._cells.count_neighbors(
-          self._inv_radii, self._sample_mode, smp._points, smp._batch_ids, max_neighbors))
-    else:
-      self._take_count(ops.find_neighbors_count(
-          smp._points, smp._batch_ids, grid._sorted_points, grid._sorted_keys, grid.get_DS(),
-          grid._num_cells, grid._scaled_aabb_min, grid._inv_cell_sizes, self._inv_radii,
-          max_neighbors, sample_order=self._sample_order))
+    self._counted = self._run_count()
 
-  def _attach(self, grid, radius, point_cloud_sample, max_neighbors):
-    dev, d = grid._sorted_points.device, grid._point_cloud._dimension
+  def _attach(self, grid, radius, point_cloud_sample, max_neighbors, counted=None):
+    cloud = grid._point_cloud
+    dev, d = cloud._points.device, cloud._dimension
     self._radius = radius
     self._radii = _to_dims(radius, d, dev)
     self._inv_radii = _to_dims(radius, d, dev, inverse=True)
     self._equal_samples = point_cloud_sample is None
-    self._point_cloud_sampled = (PointCloud(grid._sorted_points, grid._sorted_batch_ids,
-                                            grid._batch_size)
-                                 if point_cloud_sample is None else point_cloud_sample)
+    self._sampled = point_cloud_sample
     # 2: the sorted points, 1: the grid's own cloud in its unsorted order, 0: other samples
-    self._sample_mode = (2 if self._equal_samples else
-                         1 if point_cloud_sample is grid._point_cloud else 0)
+    self._sample_mode = (2 if point_cloud_sample is None else
+                         1 if point_cloud_sample is cloud else 0)
     self._grid = grid
     self.max_neighbors = max_neighbors
-    # a sequence that visits the samples cell by cell, where one is known: for the
-    # grid's own cloud the key sort's permutation (the samples of a self
-    # neighborhood are the sorted points: already in it)
-    self._sample_order = grid._sorted_indices if self._sample_mode == 1 else None
-
-  def _take_count(self, count):
-    self._count = count
-    self._samples_neigh_ranges = count.ranges
+    self._counted = counted
     self._nbrs = self._orig_ids = self._pdf = self._point_pdf = self._sample_pdf = None
     self._pdf_ready = False
     self._transposed = None
+    return self
+
+  def _run_count(self):
+    grid = self._grid
+    if grid._cells is not None:
+      smp = self._sampled if self._sample_mode == 0 else None
+      return ops._lib.host().count_neighbors(
+          grid._cells, self._inv_radii, self._sample_mode, None if smp is None else smp._points,
+          None if smp is None else smp._batch_ids, self.max_neighbors)
+    smp = self._point_cloud_sampled
+    return ops.find_neighbors_count(
+        smp._points, smp._batch_ids, grid._sorted_points, grid._sorted_keys, grid.get_DS(),
+        grid._num_cells, grid._scaled_aabb_min, grid._inv_cell_sizes, self._inv_radii,
+        self.max_neighbors, sample_order=self._sample_order)
+
+  @property
+  def _count(self):
+    # (a neighborhood of a PointHierarchy, whose sampling reads no lists, counts here)
+    if self._counted is None:
+      self._counted = self._run_count()
+    return self._counted
+
+  @property
+  def _samples_neigh_ranges(self):
+    return self._count.ranges
+
+  @property
+  def _point_cloud_sampled(self):
+    if self._sampled is None:
+      g = self._grid
+      self._sampled = PointCloud(g._sorted_points, g._sorted_batch_ids, g._batch_size)
+    return self._sampled
+
+  @property
+  def _sample_order(self):
+    # a sequence that visits the samples cell by cell, where one is known: for the
+    # grid's own cloud the key sort's permutation (the samples of a self
+    # neighborhood are the sorted points: already in it)
+    return self._grid._sorted_indices if self._sample_mode == 1 else None
 
   @property
   def num_pairs(self):
@@ -269,8 +295,7 @@ class Neighborhood:
     return self._orig_ids
 
   def _samples_are_grid_points(self):
-    return self._equal_samples or (self._point_cloud_sampled is self._grid._point_cloud
-                                   and self.max_neighbors == 0)
+    return self._equal_samples or (self._sample_mode == 1 and self.max_neighbors == 0)
 
   def compute_pdf(self, bandwidth=0.2, mode=0):
     """Neighborhood.py:257-311 (mode: 0 constant bandwidth, 1 by point count).
@@ -278,16 +303,17 @@ class Neighborhood:
     self neighborhood of the grid (Neighborhood.py:284); when the samples are the
     grid's own cloud that second search is skipped: the density at sample s is
     the density of the point it coincides with."""
-    d = self._point_cloud_sampled._dimension
-    inv_bw, inv_r = _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii
     g = self._grid
-    self._pdf = None
+    d = g._point_cloud._dimension
+    inv_bw, inv_r = _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii
+    self._pdf = self._point_pdf = self._sample_pdf = None
     if g._cells is not None and not (self._equal_samples and self.max_neighbors > 0):
-      # straight from the grid, without the list of a self neighborhood
-      if self._sample_mode == 1 and self.max_neighbors == 0:
-        self._sample_pdf, self._point_pdf = g._cells.density(inv_r, inv_bw, mode, 1), None
+      # straight from the grid, without the list of a self neighborhood; by original
+      # index, which the layers read the densities by, unless the samples are sorted
+      if self._equal_samples:
+        self._point_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 2)
       else:
-        self._point_pdf = g._cells.density(inv_r, inv_bw, mode, 2)
+        self._sample_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 1)
     elif self._equal_samples:
       self._point_pdf = ops.compute_pdf_with_pt_grads(
           g._sorted_points, self._neighbors, self._samples_neigh_ranges, inv_bw, inv_r, mode)
@@ -370,9 +396,9 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
   """Grid(point_cloud, radius) and Neighborhood(grid, radius, point_cloud_sample,
   max_neighbors) built by ONE library call with ONE blocking read where pylib's two
   constructors read back twice (Grid.py:44-48 cell counts, Neighborhood.py:242-245 pair
-  count).  Same objects, same contents: on the cell table (ops.CellGrid), or by keys
-  (tfgpc_grid_neighborhood_count) for grids too fine for one.  For a cloud that is one
-  shard of a distributed batch (num_cells_reduce set) the cell counts are reduced
+  count).  Same objects, same contents: on the cell table (ops.build_cell_grid), or by
+  keys (tfgpc_grid_neighborhood_count) for grids too fine for one.  For a cloud that is
+  one shard of a distributed batch (num_cells_reduce set) the cell counts are reduced
   over the ranks on the device, before the main call: still one blocking read."""
   pc = point_cloud
   if pc._points.shape[0] == 0:
@@ -386,12 +412,13 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
                  samples_batch_ids=None if smp is None else smp._batch_ids,
                  samples_are_points=mode, max_neighs=max_neighbors)
   cells = _reduced_cells(pc, sizes)
-  table, count = _cell_grid(pc, sizes, cells, inv_radii=_to_dims(radius, d, dev, inverse=True),
-                            **samples)
+  built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells,
+                     inv_radii=_to_dims(radius, d, dev, inverse=True), **samples)
   grid = object.__new__(Grid)
   grid._cell_sizes = _to_dims(radius, d, dev)
-  if table is not None:
-    grid._adopt(pc, table)
+  if built is not None:
+    grid._adopt(pc, built[0])
+    count = built[1]
   else:
     max_cells = _MAX_CELLS.get((d, pc._batch_size), _FIRST_BOUND)
     while True:
@@ -404,24 +431,26 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
         if max_cells is None:
           # the separate constructors size the tube array and the sort keys exactly
           return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
-    grid._adopt(pc, types.SimpleNamespace(**g))
-    grid._cells = None
-    count = g["count"]
-  nb = object.__new__(Neighborhood)
-  nb._attach(grid, radius, point_cloud_sample, max_neighbors)
-  nb._take_count(count)
-  return nb
+    grid._cells, count = None, g.pop("count")
+    grid._point_cloud, grid._batch_size = pc, pc._batch_size
+    grid._cur_keys, grid._fast_DS = g.pop("keys"), g.pop("ds")
+    for name, value in g.items():
+      setattr(grid, '_' + name, value)
+  return object.__new__(Neighborhood)._attach(grid, radius, point_cloud_sample, max_neighbors, count)
 
 
 def sample(neighborhood, sample_mode='poisson'):
   """sampling.py:123-150 -> (PointCloud of the samples, original indices or None)."""
   mode = SAMPLE_MODES[sample_mode.lower()]
   g = neighborhood._grid
+  symmetric = neighborhood._equal_samples and neighborhood.max_neighbors == 0
+  if g._cells is not None and (symmetric or mode == 1):
+    # (cell averages need no neighbors, symmetric ones are found from the grid)
+    pts, bids, idx = ops._lib.host().sample(g._cells, mode, neighborhood._inv_radii)
+    return PointCloud(pts, bids, g._batch_size), idx
   pts, bids, idx = ops.sampling(g._sorted_points, g._sorted_batch_ids, g._sorted_keys,
                                 g._num_cells, neighborhood._neighbors,
-                                neighborhood._samples_neigh_ranges, mode,
-                                symmetric=(neighborhood._equal_samples
-                                           and neighborhood.max_neighbors == 0))
+                                neighborhood._samples_neigh_ranges, mode, symmetric=symmetric)
   if mode == 0:
     idx = g._sorted_indices[idx.to(torch.int64)]
   else:
@@ -430,7 +459,9 @@ def sample(neighborhood, sample_mode='poisson'):
 
 
 class PointHierarchy:
-  """PointHierarchy.py:40-98: per level Grid -> self Neighborhood -> sample."""
+  """PointHierarchy.py:40-98: per level Grid -> self Neighborhood -> sample.  Grid and
+  sampling of a level are one library call with one blocking read; the neighborhoods
+  count and write their lists when they are used (the sampling needs none)."""
 
   def __init__(self, point_cloud, cell_sizes, sample_mode='poisson'):
     self._point_clouds = [point_cloud]
@@ -438,8 +469,26 @@ class PointHierarchy:
     self._sample_indices = []
     cur = point_cloud
     for cs in cell_sizes:
-      neigh = grid_neighborhood(cur, cs)
-      cur, idx = sample(neigh, sample_mode)
+      neigh, cur, idx = self._level(cur, cs, sample_mode)
       self._neighborhoods.append(neigh)
       self._point_clouds.append(cur)
       self._sample_indices.append(idx)
+
+  @staticmethod
+  def _level(pc, radius, sample_mode):
+    mode = SAMPLE_MODES[sample_mode.lower()]
+    built = None
+    if pc._points.shape[0] > 0:
+      dev, d = pc._points.device, pc._dimension
+      sizes = _host_dims(radius, d)
+      built = _cell_grid(pc, sizes, ops.build_cell_grid_and_sample, mode=mode,
+                         inv_radii=_to_dims(radius, d, dev, inverse=True),
+                         cells=_reduced_cells(pc, sizes))
+    if built is None:
+      neigh = grid_neighborhood(pc, radius)
+      return (neigh,) + sample(neigh, sample_mode)
+    grid = object.__new__(Grid)
+    grid._cell_sizes = _to_dims(radius, d, dev)
+    grid._adopt(pc, built[0])
+    neigh = object.__new__(Neighborhood)._attach(grid, radius, None, 0)
+    return neigh, PointCloud(built[1], built[2], pc._batch_size), built[3]
