@@ -61,63 +61,147 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
   return ok;
 }
 
+// The points of one cell that a warp has taken and not marked the neighbors of yet:
+// lane k holds the k-th.
 template <int D>
-__device__ void poisson_cell(const SampleArgs& a, const int* cell, int batch, int begin, int end,
-                             const int* nc, int total, const float* inv_r) {
-  constexpr int kTubes = num_tubes<D>();
-  constexpr int kRounds = (kTubes + 31) / 32;
-  const int lane = lane_id();
-  int2 r[kRounds];
+struct Taken {
+  float p[D];
+  int j;
+  int count;     // the same in every lane
+};
+
+template <int D>
+__device__ __forceinline__ void load_coords(const CellsView& c, int j, float* p) {
+  if (D <= 3) {
+    const float4 v = __ldg(c.packed + j);
+    p[0] = v.x; p[1] = v.y;
+    if (D == 3) p[D - 1] = v.z;
+  } else {
 #pragma unroll
-  for (int i = 0; i < kRounds; ++i)
-    r[i] = i * 32 + lane < kTubes
-               ? tube_points<D>(i * 32 + lane, cell, batch, nc, total, a.c.start)
-               : make_int2(0, 0);
+    for (int d = 0; d < D; ++d) p[d] = __ldg(c.points + (int64_t)j * D + d);
+  }
+}
+
+// The distance test of the search (cell_search.cu).
+template <int D>
+__device__ __forceinline__ bool within(const float* s, const float* p, const float* inv_r) {
+  float u = __fmul_rn(__fsub_rn(s[0], p[0]), inv_r[0]);
+  float d2 = __fmul_rn(u, u);
+#pragma unroll
+  for (int d = 1; d < D; ++d) {
+    u = __fmul_rn(__fsub_rn(s[d], p[d]), inv_r[d]);
+    d2 = __fmaf_rn(u, u, d2);
+  }
+  return d2 < 1.0f;
+}
+
+// Marks the neighbors of the taken points: the candidates of the cell, kSteps per lane
+// at a time in registers, against all of them.
+template <int D>
+__device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& taken,
+                                               const int* cell, int batch, const int* nc,
+                                               int total, const float* inv_r) {
+  constexpr int kSteps = 4;
+  constexpr int kTubes = num_tubes<D>();
+  constexpr int kTop = kTubes > 16 ? 16 : kTubes > 8 ? 8 : kTubes > 4 ? 4 : 2;
+  const int lane = lane_id();
+  if (lane < taken.count) __stcg(a.state + taken.j, (uint8_t)2);
+  for (int tube0 = 0; tube0 < kTubes; tube0 += 32) {
+    int2 r = make_int2(0, 0);
+    if (tube0 + lane < kTubes)
+      r = tube_points<D>(kTubes - 1 - (tube0 + lane), cell, batch, nc, total, a.c.start);
+    int before = r.y - r.x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += y;
+    }
+    const int candidates = __shfl_sync(0xffffffffu, before, 31);
+    const int offset = r.y - before;
+    for (int base = 0; base < candidates; base += 32 * kSteps) {
+      float p[kSteps][D];
+      int at[kSteps];
+      bool hit[kSteps];
+#pragma unroll
+      for (int k = 0; k < kSteps; ++k) {
+        const int i = base + 32 * k + lane;
+        int t = 0;
+#pragma unroll
+        for (int o = kTop; o > 0; o >>= 1) {
+          const int y = __shfl_sync(0xffffffffu, before, t + o - 1);
+          if (y <= i) t += o;
+        }
+        at[k] = i + __shfl_sync(0xffffffffu, offset, t & 31);
+        hit[k] = false;
+#pragma unroll
+        for (int d = 0; d < D; ++d) p[k][d] = INFINITY;
+        if (i < candidates) load_coords<D>(a.c, at[k], p[k]);
+      }
+      for (int who = 0; who < taken.count; ++who) {
+        float s[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) s[d] = __shfl_sync(0xffffffffu, taken.p[d], who);
+        const int j = __shfl_sync(0xffffffffu, taken.j, who);
+#pragma unroll
+        for (int k = 0; k < kSteps; ++k) hit[k] = hit[k] || (within<D>(s, p[k], inv_r) && at[k] != j);
+      }
+#pragma unroll
+      for (int k = 0; k < kSteps; ++k)
+        if (hit[k]) __stcg(a.state + at[k], (uint8_t)1);
+    }
+  }
+  taken.count = 0;
+}
+
+// Greedy selection in one cell.  Which of its points are taken depends on the marks of
+// earlier passes and on its own points only, so it is settled first, 32 points at a
+// time in registers; the marks of the (few) taken points follow together: the chain
+// per taken point is a ballot, not a walk over its candidates.
+template <int D>
+__device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cell, int batch,
+                                             int begin, int end, const int* nc, int total,
+                                             const float* inv_r) {
+  const int lane = lane_id();
+  Taken<D> taken;
+  taken.count = 0;
+  taken.j = -1;
+#pragma unroll
+  for (int d = 0; d < D; ++d) taken.p[d] = 0.0f;
   for (int q0 = begin; q0 < end; q0 += 32) {
     const int q = q0 + lane;
-    unsigned open = __ballot_sync(0xffffffffu, q < end && __ldcg(a.state + q) == 0);
-    while (open) {
-      const int taken = q0 + __ffs(open) - 1;
-      open &= open - 1u;
+    float p[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) p[d] = INFINITY;
+    bool free = false;
+    if (q < end) {
+      load_coords<D>(a.c, q, p);
+      free = __ldcg(a.state + q) == 0;
+    }
+    unsigned open = __ballot_sync(0xffffffffu, free);
+    for (int k = 0; k < taken.count && open; ++k) {
       float s[D];
 #pragma unroll
-      for (int d = 0; d < D; ++d) s[d] = __ldg(a.c.points + (int64_t)taken * D + d);
-      unsigned marked = 0u;
-#pragma unroll
-      for (int i = 0; i < kRounds; ++i) {
-        for (int t = 0; t < min(32, kTubes - i * 32); ++t) {
-          const int x = __shfl_sync(0xffffffffu, r[i].x, t);
-          const int y = __shfl_sync(0xffffffffu, r[i].y, t);
-          for (int j = x + lane; j < y; j += 32) {
-            float p[D];
-            if (D <= 3) {
-              const float4 v = __ldg(a.c.packed + j);
-              p[0] = v.x; p[1] = v.y;
-              if (D == 3) p[D - 1] = v.z;
-            } else {
-#pragma unroll
-              for (int d = 0; d < D; ++d) p[d] = __ldg(a.c.points + (int64_t)j * D + d);
-            }
-            // the distance test of the search (cell_search.cu)
-            float u = __fmul_rn(__fsub_rn(s[0], p[0]), inv_r[0]);
-            float d2 = __fmul_rn(u, u);
-#pragma unroll
-            for (int d = 1; d < D; ++d) {
-              u = __fmul_rn(__fsub_rn(s[d], p[d]), inv_r[d]);
-              d2 = __fmaf_rn(u, u, d2);
-            }
-            if (d2 < 1.0f && j != taken) {
-              __stcg(a.state + j, (uint8_t)1);
-              if (j >= q0 && j < q0 + 32) marked |= 1u << (j - q0);
-            }
-          }
-        }
-      }
-      if (lane == 0) __stcg(a.state + taken, (uint8_t)2);
-      open &= ~__reduce_or_sync(0xffffffffu, marked);
+      for (int d = 0; d < D; ++d) s[d] = __shfl_sync(0xffffffffu, taken.p[d], k);
+      open &= ~__ballot_sync(0xffffffffu, within<D>(s, p, inv_r));
     }
-    __syncwarp();   // the marks of this group are visible to the next group's reads
+    while (open) {
+      const int t = __ffs(open) - 1;
+      float s[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) s[d] = __shfl_sync(0xffffffffu, p[d], t);
+      open &= ~(__ballot_sync(0xffffffffu, within<D>(s, p, inv_r)) | (1u << t));
+      if (lane == taken.count) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) taken.p[d] = s[d];
+        taken.j = q0 + t;
+      }
+      if (++taken.count == 32) {
+        mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r);
+        __syncwarp();   // these marks are visible to the next group's reads
+      }
+    }
   }
+  if (taken.count > 0) mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r);
 }
 
 template <int D>
@@ -284,9 +368,8 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
     per_sm = v < 1 ? 1 : v;
   }
-  // a warp per 64 points, at most what is resident at once and 4 blocks per SM: with
-  // more, the barriers take longer than the shorter passes give back
-  int64_t blocks = (a.c.n + 64 * kWarps - 1) / (64 * kWarps);
+  // a warp per 16 points, at most 4 blocks per SM and what is resident at once
+  int64_t blocks = (a.c.n + 16 * kWarps - 1) / (16 * kWarps);
   const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
   if (blocks > most) blocks = most;
   if (blocks > kMaxBlocks) blocks = kMaxBlocks;
