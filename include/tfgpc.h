@@ -523,6 +523,30 @@ int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64_t ns,
                           float* dweights_out, void* ws, size_t ws_bytes);
 int tfgpc_mcconv_status(void* stream, const void* ws, int* status_out);
 
+/* The same two entries for weights that are not one dense [C*K, Cout] matrix.
+ * groups > 1: the blocks of that many kernel MLPs, [groups, C * K/groups,
+ * Cout/groups] as MCConv stores them (MCConv.py:123-135): output column block g is
+ * the product with basis functions g*K/groups .. of every channel, so the products
+ * run block by block (tfgpc_mcconv_blocks_supported: shapes that can).  groups == 1:
+ * [C * k_src, cout_src], taken as zero-padded to K basis functions and Cout columns
+ * (KPConv.py:199-212); out_grads is then [ns, cout_src] and out [ns, Cout].
+ * dweights_out has the layout of weights. */
+int tfgpc_mcconv_blocks_supported(int K, int C, int Cout, int groups);
+int tfgpc_mcconv_forward_blocks(void* stream, int K, int C, int Cout, int groups,
+                                int k_src, int cout_src, int64_t ns,
+                                int64_t n_in, int64_t M, const float* basis,
+                                const float* features, const int32_t* neighbors,
+                                const int32_t* ranges, const float* weights,
+                                float* out, void* ws, size_t ws_bytes);
+int tfgpc_mcconv_backward_blocks(void* stream, int K, int C, int Cout, int groups,
+                                 int k_src, int cout_src, int64_t ns,
+                                 int64_t n_in, int64_t M, const float* basis,
+                                 const float* features, const int32_t* neighbors,
+                                 const int32_t* ranges, const float* weights,
+                                 const float* out_grads, int x_in_workspace,
+                                 float* dbasis_out, float* dfeat_out,
+                                 float* dweights_out, void* ws, size_t ws_bytes);
+
 /* ---- MCConv forward and backward on a group plan -------------------------
  * No counterpart in the reference; same results as tfgpc_mcconv_forward /
  * _backward.  BasisProj and BasisProjGrads (basis_proj_kernels.cu.cc:30-127,
@@ -652,6 +676,24 @@ int tfgpc_kernel_mlp_grads(void* stream, int D, int num_mlps, int num_layers,
                            const float* basis_grads, float* dweights_out,
                            float* dbiases_out, float* dpoints_in_out,
                            float* dpoints_out_out, float* dpdf_out);
+/* The same two entries with every layer's parameters where they lie: weights and
+ * biases are [host] arrays of num_layers device pointers, [num_mlps, H_{l-1}, H_l] and
+ * [num_mlps, H_l].  (The gradients come back flat, layer after layer.) */
+int tfgpc_kernel_mlp_basis_layers(
+    void* stream, int D, int num_mlps, int num_layers,
+    const int32_t* layer_sizes, int64_t M, const float* points_in,
+    const float* points_out, const int32_t* neighbors, const float* pdf,
+    const float* const* weights, const float* const* biases, float inv_radius,
+    int activation, float alpha, int pdf_by_neighbor, float* basis_out);
+int tfgpc_kernel_mlp_grads_layers(
+    void* stream, int D, int num_mlps, int num_layers,
+    const int32_t* layer_sizes, int64_t M, int64_t n_in, int64_t ns,
+    const float* points_in, const float* points_out, const int32_t* neighbors,
+    const float* pdf, const float* const* weights, const float* const* biases,
+    float inv_radius, int activation, float alpha, int pdf_by_neighbor,
+    const float* basis_grads, float* dweights_out, float* dbiases_out,
+    float* dpoints_in_out, float* dpoints_out_out, float* dpdf_out);
+
 
 /* ---- KPConv and PointConv bases --------------------------------------------
  * The per-pair basis values of the other two convolutions of pylib/pc/layers,
@@ -720,6 +762,14 @@ size_t tfgpc_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K,
                      const float* a, int a_transposed, const float* b,
                      int b_transposed, float* c, void* ws, size_t ws_bytes);
+
+/* Conv1x1.py:97: out = x [n,cin] * weights [cin,cout] + bias [cout] (or NULL), rows of
+ * out cout rounded up to a multiple of 8 apart.  Does not block: a time-out inside the
+ * product is reported by the next call of this entry or of a blocking one. */
+size_t tfgpc_linear_workspace_bytes(int64_t n, int64_t cin, int64_t cout);
+int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t cout,
+                     const float* x, const float* weights, const float* bias,
+                     float* out, void* ws, size_t ws_bytes);
 
 /* ---- bounded-wait self test -------------------------------------------------
  * No counterpart in the reference (its kernels have no device-side waits).

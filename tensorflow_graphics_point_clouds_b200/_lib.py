@@ -73,6 +73,11 @@ SYMBOLS = {
     "tfgpc_mcconv_forward": c_int,
     "tfgpc_mcconv_backward": c_int,
     "tfgpc_mcconv_status": c_int,
+    "tfgpc_mcconv_blocks_supported": c_int,
+    "tfgpc_mcconv_forward_blocks": c_int,
+    "tfgpc_mcconv_backward_blocks": c_int,
+    "tfgpc_linear_workspace_bytes": c_sz,
+    "tfgpc_linear_f32": c_int,
     "tfgpc_mcconv_grouped_supported": c_int,
     "tfgpc_mcconv_group_plan_bytes": c_sz,
     "tfgpc_mcconv_group_plan": c_int,
@@ -83,6 +88,8 @@ SYMBOLS = {
     "tfgpc_kernel_basis_grads": c_int,
     "tfgpc_kernel_mlp_basis": c_int,
     "tfgpc_kernel_mlp_grads": c_int,
+    "tfgpc_kernel_mlp_basis_layers": c_int,
+    "tfgpc_kernel_mlp_grads_layers": c_int,
     "tfgpc_kp_basis": c_int,
     "tfgpc_pointconv_pdf": c_int,
     "tfgpc_neighborhood_pool": c_int,

@@ -48,7 +48,8 @@ __global__ void __launch_bounds__(kBpThreads)
 basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
                   const float* __restrict__ feat, const int2* __restrict__ neigh,
                   const int32_t* __restrict__ ranges, float* __restrict__ out,
-                  __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
+                  __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
+                  int shift) {
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -72,8 +73,11 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
       for (int cc = 0; cc < kCpl; ++cc)
 #pragma unroll
         for (int k = 0; k < K; ++k) acc[cc][k] = 0.0f;
+      int next = a < e ? __ldg(&neigh[a].x) : 0;
+#pragma unroll 2
       for (int m = a; m < e; ++m) {
-        const int j = __ldg(&neigh[m].x);
+        const int j = next;
+        if (m + 1 < e) next = __ldg(&neigh[m + 1].x);
         float f[kCpl], w[K];
         load_features<K, VEC>(feat + (int64_t)j * C, cbase, C, f);
         load_basis_row<K>(basis + (int64_t)m * K, w);
@@ -104,8 +108,9 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
               __nv_bfloat16 h[4], l[4];
               split_bf16(v.x, h[0], l[0]); split_bf16(v.y, h[1], l[1]);
               split_bf16(v.z, h[2], l[2]); split_bf16(v.w, h[3], l[3]);
-              *reinterpret_cast<uint2*>(out_hi + obase + f0) = *reinterpret_cast<uint2*>(h);
-              *reinterpret_cast<uint2*>(out_mid + obase + f0) = *reinterpret_cast<uint2*>(l);
+              const int64_t o = block_offset<K>(s, C, c0 + f0 / K, f0 % K, shift);
+              *reinterpret_cast<uint2*>(out_hi + o) = *reinterpret_cast<uint2*>(h);
+              *reinterpret_cast<uint2*>(out_mid + o) = *reinterpret_cast<uint2*>(l);
             }
           }
         }
@@ -113,16 +118,18 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
 #pragma unroll
         for (int cc = 0; cc < kCpl; ++cc) {
           if (cbase + cc < C) {
-            const int64_t o = s * (int64_t)C * K + (int64_t)(cbase + cc) * K;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
+            for (int k = 0; k < K; k += 4) {
+              const int64_t o = block_offset<K>(s, C, cbase + cc, k, shift);
               if (OUT == 0) {
-                out[o + k] = acc[cc][k];
+                *reinterpret_cast<float4*>(out + o) =
+                    make_float4(acc[cc][k], acc[cc][k + 1], acc[cc][k + 2], acc[cc][k + 3]);
               } else {
-                __nv_bfloat16 h, l;
-                split_bf16(acc[cc][k], h, l);
-                out_hi[o + k] = h;
-                out_mid[o + k] = l;
+                uint2 h, m;
+                split2_bf16(acc[cc][k], acc[cc][k + 1], h.x, m.x);
+                split2_bf16(acc[cc][k + 2], acc[cc][k + 3], h.y, m.y);
+                *reinterpret_cast<uint2*>(out_hi + o) = h;
+                *reinterpret_cast<uint2*>(out_mid + o) = m;
               }
             }
           }
@@ -143,7 +150,7 @@ __global__ void __launch_bounds__(kBpThreads)
 basis_proj_grads_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
                         const float* __restrict__ feat, const int2* __restrict__ neigh,
                         const int32_t* __restrict__ ranges, const float* __restrict__ in_grads,
-                        float* __restrict__ dbasis, float* __restrict__ dfeat) {
+                        float* __restrict__ dbasis, float* __restrict__ dfeat, int shift) {
   constexpr int kCpl = BpCfg<K>::kCpl;
   const int lane = lane_id();
   const int gl = lane & (G - 1);
@@ -168,10 +175,10 @@ basis_proj_grads_kernel(int C, int64_t ns, int G, const float* __restrict__ basi
 #pragma unroll
       for (int cc = 0; cc < kCpl; ++cc) {
         const bool ok = active && cbase + cc < C;
-        const float* src = in_grads + s * (int64_t)C * K + (int64_t)(cbase + cc) * K;
 #pragma unroll
         for (int q = 0; q < K / 4; ++q) {
-          float4 v = ok ? __ldg(reinterpret_cast<const float4*>(src) + q)
+          const float* src = in_grads + block_offset<K>(s, C, cbase + cc, 4 * q, shift);
+          float4 v = ok ? __ldg(reinterpret_cast<const float4*>(src))
                         : make_float4(0.f, 0.f, 0.f, 0.f);
           g[cc][4 * q] = v.x; g[cc][4 * q + 1] = v.y; g[cc][4 * q + 2] = v.z; g[cc][4 * q + 3] = v.w;
         }
@@ -272,8 +279,9 @@ basis_proj_grads_kernel(int C, int64_t ns, int G, const float* __restrict__ basi
 template <int K, int OUT>
 static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* basis,
                              const float* feat, const int2* neigh, const int32_t* ranges,
-                             float* out, __nv_bfloat16* hi, __nv_bfloat16* mid) {
+                             float* out, __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden = K) {
   constexpr int kCpl = BpCfg<K>::kCpl;
+  const int shift = hidden_shift(hidden);
   const int G = bp_group_lanes(C, kCpl);
   const bool vec = kCpl == 4 && C % 4 == 0 && ((uintptr_t)feat % 16 == 0);
   const size_t smem = G == 32 ? (size_t)(kBpThreads / 32) * 32 * BpCfg<K>::kRow * sizeof(float) : 0;
@@ -291,7 +299,7 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
     int per_sm = 1;
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, out, hi, mid);
+    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, out, hi, mid, shift);
     TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
@@ -299,12 +307,12 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
     auto kern = basis_proj_kernel<K, true, OUT>;
     if (smem > 48 * 1024)
       TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid);
+    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
   } else {
     auto kern = basis_proj_kernel<K, false, OUT>;
     if (smem > 48 * 1024)
       TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid);
+    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
   }
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
@@ -313,12 +321,12 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
 // Entry used by the fused MCConv path (mcconv.cu): split bf16 output.
 int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                      const float* feat, const int32_t* neigh, const int32_t* ranges,
-                     __nv_bfloat16* hi, __nv_bfloat16* mid) {
+                     __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden) {
   switch (K) {
-    case 8: return launch_basis_proj<8, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid);
-    case 16: return launch_basis_proj<16, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid);
-    case 32: return launch_basis_proj<32, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid);
-    case 64: return launch_basis_proj<64, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid);
+    case 8: return launch_basis_proj<8, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid, hidden);
+    case 16: return launch_basis_proj<16, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid, hidden);
+    case 32: return launch_basis_proj<32, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid, hidden);
+    case 64: return launch_basis_proj<64, 1>(st, C, ns, basis, feat, (const int2*)neigh, ranges, nullptr, hi, mid, hidden);
   }
   return fail(TFGPC_EINVAL, "BasisProj expects a valid number of basis functions.");
 }
@@ -326,8 +334,10 @@ int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* bas
 template <int K>
 static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, const float* basis,
                                    const float* feat, const int2* neigh, const int32_t* ranges,
-                                   const float* in_grads, float* dbasis, float* dfeat) {
+                                   const float* in_grads, float* dbasis, float* dfeat,
+                                   int hidden) {
   constexpr int kCpl = BpCfg<K>::kCpl;
+  const int shift = hidden_shift(hidden);
   const int G = bp_group_lanes(C, kCpl);
   const bool vec = kCpl == 4 && C % 4 == 0 && ((uintptr_t)feat % 16 == 0) &&
                    ((uintptr_t)dfeat % 16 == 0);
@@ -345,16 +355,18 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, const flo
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
     kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, in_grads, dbasis,
-                                            dfeat);
+                                            dfeat, shift);
     TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
   if (vec)
     basis_proj_grads_kernel<K, true><<<grid, kBpThreads, 0, st>>>(C, ns, G, basis, feat, neigh,
-                                                                  ranges, in_grads, dbasis, dfeat);
+                                                                  ranges, in_grads, dbasis, dfeat,
+                                                                  shift);
   else
     basis_proj_grads_kernel<K, false><<<grid, kBpThreads, 0, st>>>(C, ns, G, basis, feat, neigh,
-                                                                   ranges, in_grads, dbasis, dfeat);
+                                                                   ranges, in_grads, dbasis, dfeat,
+                                                                  shift);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -368,7 +380,7 @@ int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* b
                        float* out);
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
-                         const float* in_grads, float* dbasis, float* dfeat);
+                         const float* in_grads, float* dbasis, float* dfeat, int hidden);
 
 static int check_bp_args(const char* op, int K, int C, int64_t ns, int64_t n_in, int64_t M) {
   TFGPC_REQUIRE(valid_basis(K), "%s expects a valid number of basis functions.", op);
@@ -403,33 +415,43 @@ extern "C" int tfgpc_basis_proj(void* stream, int K, int C, int64_t ns, int64_t 
   }
 }
 
+namespace tfgpc {
+// The gradients on the SIMT kernels, in_grads with the columns of block_offset.
+int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, int64_t M,
+                            const float* basis, const float* feat, const int32_t* neigh,
+                            const int32_t* ranges, const float* in_grads, float* dbasis,
+                            float* dfeat, int hidden) {
+  if (M > 0) {
+    TFGPC_REQUIRE(dbasis, "BasisProjGradsOp got a null pointer");
+    TFGPC_CUDA(cudaMemsetAsync(dbasis, 0, sizeof(float) * (size_t)M * K, st));
+  }
+  if (n_in > 0) {
+    TFGPC_REQUIRE(dfeat, "BasisProjGradsOp got a null pointer");
+    TFGPC_CUDA(cudaMemsetAsync(dfeat, 0, sizeof(float) * (size_t)n_in * C, st));
+  }
+  if (ns == 0 || M == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(basis && feat && neigh && ranges && in_grads,
+                "BasisProjGradsOp got a null pointer");
+  TFGPC_REQUIRE((uintptr_t)basis % 16 == 0 && (uintptr_t)in_grads % 16 == 0,
+                "BasisProjGradsOp expects 16-byte aligned basis and gradient buffers");
+  const int2* nb = (const int2*)neigh;
+  switch (K) {
+    case 8: return launch_basis_proj_grads<8>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    case 16: return launch_basis_proj_grads<16>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    case 32: return launch_basis_proj_grads<32>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    default: return launch_basis_proj_grads<64>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+  }
+}
+}  // namespace tfgpc
+
 extern "C" int tfgpc_basis_proj_grads(void* stream, int K, int C, int64_t ns, int64_t n_in,
                                       int64_t M, const float* basis, const float* features,
                                       const int32_t* neighbors, const int32_t* ranges,
                                       const float* in_grads, float* dbasis_out, float* dfeat_out) {
   int rc = check_bp_args("BasisProjGradsOp", K, C, ns, n_in, M);
   if (rc) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (M > 0) {
-    TFGPC_REQUIRE(dbasis_out, "BasisProjGradsOp got a null pointer");
-    TFGPC_CUDA(cudaMemsetAsync(dbasis_out, 0, sizeof(float) * (size_t)M * K, st));
-  }
-  if (n_in > 0) {
-    TFGPC_REQUIRE(dfeat_out, "BasisProjGradsOp got a null pointer");
-    TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
-  }
-  if (ns == 0 || M == 0) return TFGPC_OK;
-  TFGPC_REQUIRE(basis && features && neighbors && ranges && in_grads,
-                "BasisProjGradsOp got a null pointer");
-  TFGPC_REQUIRE((uintptr_t)basis % 16 == 0 && (uintptr_t)in_grads % 16 == 0,
-                "BasisProjGradsOp expects 16-byte aligned basis and gradient buffers");
-  const int2* nb = (const int2*)neighbors;
-  switch (K) {
-    case 8: return launch_basis_proj_grads<8>(st, C, ns, basis, features, nb, ranges, in_grads, dbasis_out, dfeat_out);
-    case 16: return launch_basis_proj_grads<16>(st, C, ns, basis, features, nb, ranges, in_grads, dbasis_out, dfeat_out);
-    case 32: return launch_basis_proj_grads<32>(st, C, ns, basis, features, nb, ranges, in_grads, dbasis_out, dfeat_out);
-    default: return launch_basis_proj_grads<64>(st, C, ns, basis, features, nb, ranges, in_grads, dbasis_out, dfeat_out);
-  }
+  return basis_proj_grads_blocks((cudaStream_t)stream, K, C, ns, n_in, M, basis, features,
+                                 neighbors, ranges, in_grads, dbasis_out, dfeat_out, K);
 }
 
 extern "C" size_t tfgpc_basis_proj_workspace_bytes(int K, int C, int64_t n_in) {
@@ -481,5 +503,5 @@ extern "C" int tfgpc_basis_proj_grads_ws(void* stream, int K, int C, int64_t ns,
   if (rc) return rc;
   TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
   return basis_proj_grads_mma(st, K, C, ns, M, basis, fs, neighbors, ranges, in_grads, dbasis_out,
-                              dfeat_out);
+                              dfeat_out, K);
 }

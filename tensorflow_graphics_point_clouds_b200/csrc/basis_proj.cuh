@@ -20,6 +20,20 @@ inline bool valid_basis(int K) { return K == 8 || K == 16 || K == 32 || K == 64;
 // basis_proj_ops.cpp:104-108: between 1 and 8, or a multiple of 8.
 inline bool valid_features(int C) { return C > 0 && (C < 8 || C % 8 == 0); }
 
+// Where the value of channel c and basis function k of sample s lies in a projection
+// whose columns have the order (k / hidden, c, k % hidden), hidden = 2^shift; hidden = K
+// is the op's (c, k).  Four consecutive k from a multiple of four lie together.
+template <int K>
+__device__ __forceinline__ int64_t block_offset(int64_t s, int C, int c, int k, int shift) {
+  return s * (int64_t)C * K + (((int64_t)(k >> shift) * C + c) << shift) + (k & ((1 << shift) - 1));
+}
+
+inline int hidden_shift(int hidden) {
+  int s = 0;
+  while ((1 << s) < hidden) ++s;
+  return s;
+}
+
 // Lanes cooperating on one sample: the smallest power of two covering C.
 inline int bp_group_lanes(int C, int cpl) {
   int need = (C + cpl - 1) / cpl;

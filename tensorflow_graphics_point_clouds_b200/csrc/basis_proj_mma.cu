@@ -39,7 +39,7 @@ Shape walk_shape(int64_t items, int warps) {
 template <int K, int CC, int OUT>
 int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __nv_bfloat16* fs,
                const int2* neigh, const int32_t* ranges, float* out, __nv_bfloat16* hi,
-               __nv_bfloat16* mid) {
+               __nv_bfloat16* mid, int hidden) {
   typedef bpm::Cfg<K, CC> cfg;
   auto kern = bpm::basis_proj_mma_kernel<K, CC, OUT>;
   constexpr int smem = cfg::kFwdWarps * cfg::kFwdWarpBytes;
@@ -50,8 +50,8 @@ int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __n
   int rows = sm_count() / s.grid;
   rows = rows < 1 ? 1 : rows > passes ? passes : rows;
   ProfScope prof(st, OUT == 0 ? "basis_proj_mma" : "basis_proj_split_mma");
-  kern<<<dim3(s.grid, rows), cfg::kFwdWarps * 32, smem, st>>>(s.bs, C, ns, basis, fs, neigh, ranges,
-                                                              out, hi, mid);
+  kern<<<dim3(s.grid, rows), cfg::kFwdWarps * 32, smem, st>>>(s.bs, hidden_shift(hidden), C, ns, basis, fs, neigh,
+                                                              ranges, out, hi, mid);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -59,7 +59,7 @@ int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __n
 template <int K, int CC>
 int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* basis,
                  const __nv_bfloat16* fs, const int2* neigh, const int32_t* ranges,
-                 const float* in_grads, float* dbasis, float* dfeat) {
+                 const float* in_grads, float* dbasis, float* dfeat, int hidden) {
   typedef bpm::Cfg<K, CC> cfg;
   auto kern = bpm::basis_proj_grads_mma_kernel<K, CC>;
   constexpr int smem = cfg::kGradWarps * cfg::kGradWarpBytes;
@@ -72,8 +72,8 @@ int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* bas
   if (parts < 1) parts = 1;
   Shape s = walk_shape(ns * parts, cfg::kGradWarps);
   ProfScope prof(st, "basis_proj_grads_mma");
-  kern<<<s.grid, cfg::kGradWarps * 32, smem, st>>>(s.bs, (int)parts, C, ns, M, basis, fs, neigh,
-                                                   ranges, in_grads, dbasis, dfeat);
+  kern<<<s.grid, cfg::kGradWarps * 32, smem, st>>>(s.bs, (int)parts, hidden_shift(hidden), C, ns, M, basis, fs,
+                                                   neigh, ranges, in_grads, dbasis, dfeat);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -111,9 +111,9 @@ int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bf
 
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
-                         __nv_bfloat16* hi, __nv_bfloat16* mid) {
+                         __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden) {
   TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 1>(st, C, ns, basis, fs, (const int2*)neigh,
-                                                      ranges, nullptr, hi, mid))
+                                                      ranges, nullptr, hi, mid, hidden))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
@@ -122,15 +122,15 @@ int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* b
                        const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                        float* out) {
   TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 0>(st, C, ns, basis, fs, (const int2*)neigh,
-                                                      ranges, out, nullptr, nullptr))
+                                                      ranges, out, nullptr, nullptr, kK))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
-                         const float* in_grads, float* dbasis, float* dfeat) {
+                         const float* in_grads, float* dbasis, float* dfeat, int hidden) {
   TFGPC_CC_SWITCH(K, C, return launch_grads<kK, kCC>(st, C, ns, M, basis, fs, (const int2*)neigh,
-                                                     ranges, in_grads, dbasis, dfeat))
+                                                     ranges, in_grads, dbasis, dfeat, hidden))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 

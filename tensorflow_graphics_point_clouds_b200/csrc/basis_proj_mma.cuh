@@ -273,10 +273,12 @@ __device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float
 // indices of chunk i+2 are on their way to registers, while chunk i is multiplied.
 // OUT = 0: fp32 [ns, C, K] (the op's output).  OUT = 1: the same values split
 // into two bf16 arrays [ns, C*K] (left operand of the tensor-core GEMM).
-// The passes over the channels are dealt to gridDim.y.
+// The passes over the channels are dealt to gridDim.y.  The columns of a row lie in the
+// order of block_offset: 2^shift = K is the op's (c, k), less are the blocks of several
+// kernel MLPs, one after the other.
 template <int K, int CC, int OUT>
 __global__ void __launch_bounds__(Cfg<K, CC>::kFwdWarps * 32, 1)
-basis_proj_mma_kernel(int bs, int C, int64_t ns, const float* __restrict__ basis,
+basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* __restrict__ basis,
                       const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                       const int32_t* __restrict__ ranges, float* __restrict__ out,
                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
@@ -376,7 +378,7 @@ basis_proj_mma_kernel(int bs, int C, int64_t ns, const float* __restrict__ basis
       }
       if (cur.last) {
         // lane (g, q): channels c0 + 16*mt + g (+8), basis functions 16*j + 4*q .. +3
-        const int64_t obase = (cur.s * C + c0 + g) * K + 4 * q;
+        const int64_t obase = cur.s * C * K + ((c0 + g) << shift);
 #pragma unroll
         for (int mt = 0; mt < cfg::kMT; ++mt) {
           if (mt < mt_cnt) {
@@ -384,7 +386,9 @@ basis_proj_mma_kernel(int bs, int C, int64_t ns, const float* __restrict__ basis
             for (int j = 0; j < cfg::kNTP; ++j) {
 #pragma unroll
               for (int h = 0; h < 2; ++h) {   // rows g and g + 8
-                const int64_t o = obase + (int64_t)(16 * mt + 8 * h) * K + 16 * j;
+                const int k = 16 * j + 4 * q;
+                const int64_t o = obase + (((k >> shift) * C + 16 * mt + 8 * h) << shift) +
+                                  (k & ((1 << shift) - 1));
                 if (OUT == 0) {
                   *reinterpret_cast<float4*>(out + o) =
                       make_float4(acc[mt][2 * j][2 * h], acc[mt][2 * j][2 * h + 1],
@@ -428,7 +432,7 @@ basis_proj_mma_kernel(int bs, int C, int64_t ns, const float* __restrict__ basis
 // pair belongs to exactly one sample); dfeat must be zero on entry.
 template <int K, int CC>
 __global__ void __launch_bounds__(Cfg<K, CC>::kGradWarps * 32, 1)
-basis_proj_grads_mma_kernel(int bs, int parts, int C, int64_t ns, int64_t M, const float* __restrict__ basis,
+basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int64_t M, const float* __restrict__ basis,
                             const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                             const int32_t* __restrict__ ranges,
                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
@@ -466,10 +470,18 @@ basis_proj_grads_mma_kernel(int bs, int parts, int C, int64_t ns, int64_t M, con
   }
 
   auto issue_dx = [&](int64_t s, int c0, int w) {
-    // w*K floats, contiguous
-    const float* src = in_grads + (s * C + c0) * K;
+    // w*K floats, one contiguous piece per block, to rows of K per channel
+    const float* src = in_grads + s * C * K + ((int64_t)c0 << shift);
     const uint32_t dst = smem_addr(dx_raw);
-    for (int i = lane; i < w * (K / 4); i += 32) cp_async16_zfill(dst + i * 16, src + i * 4, true);
+    if ((1 << shift) == K) {
+      for (int i = lane; i < w * (K / 4); i += 32) cp_async16_zfill(dst + i * 16, src + i * 4, true);
+    } else {
+      for (int i = lane; i < w * (K / 4); i += 32) {
+        const int c = i / (K / 4), k = (i % (K / 4)) * 4;
+        cp_async16_zfill(dst + i * 16, src + (((k >> shift) * C + c) << shift) + (k & ((1 << shift) - 1)),
+                         true);
+      }
+    }
   };
 
   for (int c0 = 0; c0 < C; c0 += cfg::kCC) {

@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(kBpwThreads, 2)
 basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
                        const float* __restrict__ feat, const int2* __restrict__ neigh,
                        const int32_t* __restrict__ ranges, float* __restrict__ out,
-                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
+                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
+                       int shift) {
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -199,8 +200,9 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
           __nv_bfloat16 h[4], l[4];
           split_bf16(v.x, h[0], l[0]); split_bf16(v.y, h[1], l[1]);
           split_bf16(v.z, h[2], l[2]); split_bf16(v.w, h[3], l[3]);
-          *reinterpret_cast<uint2*>(out_hi + obase + f0) = *reinterpret_cast<uint2*>(h);
-          *reinterpret_cast<uint2*>(out_mid + obase + f0) = *reinterpret_cast<uint2*>(l);
+          const int64_t o = block_offset<K>(s, C, c0 + f0 / K, f0 % K, shift);
+          *reinterpret_cast<uint2*>(out_hi + o) = *reinterpret_cast<uint2*>(h);
+          *reinterpret_cast<uint2*>(out_mid + o) = *reinterpret_cast<uint2*>(l);
         }
       }
     }
@@ -223,7 +225,7 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
                              const float* __restrict__ feat, const int2* __restrict__ neigh,
                              const int32_t* __restrict__ ranges,
                              const float* __restrict__ in_grads, float* __restrict__ dbasis,
-                             float* __restrict__ dfeat) {
+                             float* __restrict__ dfeat, int shift) {
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kChunk = 32 * kCpl;
   constexpr int R = kBpwRing;
@@ -275,11 +277,11 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
         unsigned long long g[kCpl][K / 2];
 #pragma unroll
         for (int cc = 0; cc < kCpl; ++cc) {
-          const ulonglong2* src = reinterpret_cast<const ulonglong2*>(
-              in_grads + s * (int64_t)C * K + (int64_t)(cbase + cc) * K);
 #pragma unroll
           for (int q = 0; q < K / 4; ++q) {
-            const ulonglong2 v = c_ok ? __ldg(src + (q ^ permq)) : make_ulonglong2(0ull, 0ull);
+            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(
+                in_grads + block_offset<K>(s, C, cbase + cc, 4 * (q ^ permq), shift));
+            const ulonglong2 v = c_ok ? __ldg(src) : make_ulonglong2(0ull, 0ull);
             g[cc][2 * q] = v.x; g[cc][2 * q + 1] = v.y;
           }
         }

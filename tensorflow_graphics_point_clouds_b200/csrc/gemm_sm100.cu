@@ -25,17 +25,22 @@ namespace {
 constexpr int kBM = 128;           // rows of C per tile (TMEM lanes)
 constexpr int kBNMax = 256;        // columns of C per tile (TMEM columns per buffer)
 constexpr int kBK = 64;            // reduction elements per ring slot: 128 bytes of bf16
-constexpr int kStages = 2;
+constexpr int kMaxStages = 4;
 constexpr int kUmmaK = 16;         // reduction elements per tcgen05.mma (kind::f16)
 constexpr int kThreads = 192;
 constexpr int kTmemCols = 512;     // two accumulator buffers of 256 columns
 constexpr uint32_t kABytes = kBM * kBK * 2;        // one A tile (hi or mid)
-constexpr uint32_t kBBytes = kBNMax * kBK * 2;     // one B tile (hi or mid)
-constexpr uint32_t kStageBytes = 2 * kABytes + 2 * kBBytes;
 constexpr uint32_t kOutBoxBytes = 32 * 32 * 4;     // one 32 x 32 fp32 box of the epilogue
 constexpr uint32_t kOutStageBytes = 4 * 2 * kOutBoxBytes;  // 4 epilogue warps, double buffered
-constexpr size_t kSmemBytes = (size_t)kStages * kStageBytes + kOutStageBytes +
-                              1024 /*alignment*/ + 256 /*barriers*/;
+constexpr uint32_t kFixedBytes = kOutStageBytes + 1024 /*alignment*/ + 256 /*barriers*/;
+
+// One ring slot holds the A and B tiles (hi and mid) of 64 reduction elements; narrow
+// tiles leave room for more slots.
+inline uint32_t stage_bytes(int bn) { return 2 * kABytes + 2 * (uint32_t)bn * kBK * 2; }
+inline int stages_for(int bn) {
+  const int s = (int)((227u * 1024u - kFixedBytes) / stage_bytes(bn));
+  return s < kMaxStages ? s : kMaxStages;
+}
 
 using namespace tc;
 
@@ -79,27 +84,27 @@ __device__ __forceinline__ void store_image_row(uint8_t* image, int channels, in
 }
 
 struct TileSchedule {
-  int m_tiles, n_tiles, k_splits;
+  int m_tiles, n_tiles, batches, k_splits;
   int k_blocks;         // ring slots over the whole reduction
   int k_blocks_per_split;
   int add_slices;       // 1: every slice of the reduction is added into the one output
 };
 
 struct Barriers {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  uint64_t full[kMaxStages];
+  uint64_t empty[kMaxStages];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
 };
 
-// OUT = 0: C as fp32 through TMA stores.  OUT = 1: C is the gradient of a
-// [rows, channels, 16] projection and is written as the bf16 hi/mid operand
-// image the tensor-core gradient kernel loads with one bulk copy per group of
-// four rows (basis_proj_grads_tc.cu describes the layout).  OUT = 2: the map of C
-// describes C^T ([N, M] row-major): boxes are transposed on their way through
-// shared memory, for products whose natural left operand is the small matrix.
+// OUT = 0: C as fp32 through TMA stores.  OUT = 2: the map of C describes C^T ([N, M]
+// row-major): boxes are transposed on their way through shared memory, for products
+// whose natural left operand is the small matrix.  OUT = 3: C^T is the gradient of a
+// [rows, channels, 16] projection and is written as the bf16 hi/mid operand image the
+// tensor-core gradient kernel loads with one bulk copy per group of four rows
+// (basis_proj_grads_tc.cu describes the layout).
 // OUT = 4: like 2, but row j of C^T goes to row row_order[j] of the output
 // (`image` is then the fp32 output, image_channels its row length): the rows of a
 // product computed in another sequence than the caller's are put back in place.
@@ -110,19 +115,22 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
                    const __grid_constant__ CUtensorMap tm_b_hi,
                    const __grid_constant__ CUtensorMap tm_b_mid,
                    const __grid_constant__ CUtensorMap tm_c, int64_t m_total, int64_t n_total,
-                   int bn, uint32_t idesc, TileSchedule sch, int* err_flag, uint8_t* image,
-                   int image_channels, int image_group, const int32_t* __restrict__ row_order) {
+                   int bn, int stages, uint32_t idesc, TileSchedule sch, int* err_flag,
+                   const float* __restrict__ bias, uint8_t* image, int image_channels,
+                   int image_group, const int32_t* __restrict__ row_order) {
   extern __shared__ uint8_t smem_raw[];
   // the swizzled tiles need 1024-byte alignment
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* out_stage = smem + (size_t)kStages * kStageBytes;  // 1024-byte aligned
+  const uint32_t b_bytes = (uint32_t)bn * kBK * 2;            // one B tile (hi or mid)
+  const uint32_t slot_bytes = 2 * kABytes + 2 * b_bytes;
+  uint8_t* out_stage = smem + (size_t)stages * slot_bytes;    // 1024-byte aligned
   Barriers* bars = (Barriers*)(out_stage + kOutStageBytes);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int total_tiles = sch.m_tiles * sch.n_tiles * sch.k_splits;
+  const int total_tiles = sch.m_tiles * sch.n_tiles * sch.batches * sch.k_splits;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(smem_u32(&bars->full[s]), 1);
       mbar_init(smem_u32(&bars->empty[s]), 1);
     }
@@ -140,50 +148,51 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
   const uint32_t tmem_base = *(volatile uint32_t*)&bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
 
-  // tile -> (m, n, split); m fastest so that CTAs running together share B/k-slices
-  auto decode = [&](int t, int& m, int& n, int& sp) {
+  // tile -> (m, n, batch, split); m fastest so that CTAs running together share B/k-slices
+  auto decode = [&](int t, int& m, int& n, int& bt, int& sp) {
     m = t % sch.m_tiles;
     int r = t / sch.m_tiles;
     n = r % sch.n_tiles;
-    sp = r / sch.n_tiles;
+    r /= sch.n_tiles;
+    bt = r % sch.batches;
+    sp = r / sch.batches;
   };
-  const uint32_t b_tile_bytes = (uint32_t)bn * kBK * 2;
 
   if (warp == 0) {
     // ---------------------------------------------------------- TMA producer
     if (lane == 0) {
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t ph = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        int m, n, sp;
-        decode(t, m, n, sp);
+        int m, n, bt, sp;
+        decode(t, m, n, bt, sp);
         const int kb0 = sp * sch.k_blocks_per_split;
         const int kb1 = min(kb0 + sch.k_blocks_per_split, sch.k_blocks);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
+        for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(smem_u32(&bars->empty[s]), ph ^ 1, abort_flag, err_flag);
           const uint32_t full = smem_u32(&bars->full[s]);
-          mbar_expect_tx(full, 2 * kABytes + 2 * b_tile_bytes);
-          uint8_t* st = smem + (size_t)s * kStageBytes;
+          mbar_expect_tx(full, slot_bytes);
+          uint8_t* st = smem + (size_t)s * slot_bytes;
+          if (++s == stages) { s = 0; ph ^= 1; }
           const uint32_t a_hi = smem_u32(st), a_mid = a_hi + kABytes;
-          const uint32_t b_hi = a_mid + kABytes, b_mid = b_hi + kBBytes;
+          const uint32_t b_hi = a_mid + kABytes, b_mid = b_hi + b_bytes;
           if (!A_MN) {
-            tma_load_2d(a_hi, &tm_a_hi, kb * kBK, m * kBM, full);
-            tma_load_2d(a_mid, &tm_a_mid, kb * kBK, m * kBM, full);
+            tma_load_3d(a_hi, &tm_a_hi, kb * kBK, m * kBM, bt, full);
+            tma_load_3d(a_mid, &tm_a_mid, kb * kBK, m * kBM, bt, full);
           } else {
             // two boxes of 64 (M) x 64 (K rows): 8 KB each
             for (int j = 0; j < kBM / 64; ++j) {
-              tma_load_2d(a_hi + j * 8192, &tm_a_hi, m * kBM + j * 64, kb * kBK, full);
-              tma_load_2d(a_mid + j * 8192, &tm_a_mid, m * kBM + j * 64, kb * kBK, full);
+              tma_load_3d(a_hi + j * 8192, &tm_a_hi, m * kBM + j * 64, kb * kBK, bt, full);
+              tma_load_3d(a_mid + j * 8192, &tm_a_mid, m * kBM + j * 64, kb * kBK, bt, full);
             }
           }
           if (!B_MN) {
-            tma_load_2d(b_hi, &tm_b_hi, kb * kBK, n * bn, full);
-            tma_load_2d(b_mid, &tm_b_mid, kb * kBK, n * bn, full);
+            tma_load_3d(b_hi, &tm_b_hi, kb * kBK, n * bn, bt, full);
+            tma_load_3d(b_mid, &tm_b_mid, kb * kBK, n * bn, bt, full);
           } else {
             for (int j = 0; j < bn / 64; ++j) {
-              tma_load_2d(b_hi + j * 8192, &tm_b_hi, n * bn + j * 64, kb * kBK, full);
-              tma_load_2d(b_mid + j * 8192, &tm_b_mid, n * bn + j * 64, kb * kBK, full);
+              tma_load_3d(b_hi + j * 8192, &tm_b_hi, n * bn + j * 64, kb * kBK, bt, full);
+              tma_load_3d(b_mid + j * 8192, &tm_b_mid, n * bn + j * 64, kb * kBK, bt, full);
             }
           }
         }
@@ -192,11 +201,12 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t ph = 0;
       int tile_iter = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
-        int m, n, sp;
-        decode(t, m, n, sp);
+        int m, n, bt, sp;
+        decode(t, m, n, bt, sp);
         const int kb0 = sp * sch.k_blocks_per_split;
         const int kb1 = min(kb0 + sch.k_blocks_per_split, sch.k_blocks);
         const int buf = tile_iter & 1;
@@ -204,14 +214,12 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)buf * kBNMax;
         uint32_t accumulate = 0;
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
+        for (int kb = kb0; kb < kb1; ++kb) {
           mbar_wait(smem_u32(&bars->full[s]), ph, abort_flag, err_flag);
           tc_fence_after();
-          uint8_t* st = smem + (size_t)s * kStageBytes;
+          uint8_t* st = smem + (size_t)s * slot_bytes;
           const uint32_t a_hi = smem_u32(st), a_mid = a_hi + kABytes;
-          const uint32_t b_hi = a_mid + kABytes, b_mid = b_hi + kBBytes;
+          const uint32_t b_hi = a_mid + kABytes, b_mid = b_hi + b_bytes;
           // K-major: rows of 128 bytes, 8-row swizzle atoms 1024 bytes apart;
           // one UMMA_K step is 32 bytes inside the row.
           // MN-major: 64 (MN) x 8 (K) atoms of 1024 bytes; atoms along K are
@@ -232,6 +240,7 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
             accumulate = 1u;
           }
           umma_commit(smem_u32(&bars->empty[s]));  // slot free once these MMAs have read it
+          if (++s == stages) { s = 0; ph ^= 1; }
         }
         umma_commit(smem_u32(&bars->acc_full[buf]));
       }
@@ -248,8 +257,8 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
     uint32_t box_iter = 0;
     int tile_iter = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++tile_iter) {
-      int m, n, sp;
-      decode(t, m, n, sp);
+      int m, n, bt, sp;
+      decode(t, m, n, bt, sp);
       const int buf = tile_iter & 1;
       mbar_wait(smem_u32(&bars->acc_full[buf]), (tile_iter >> 1) & 1, abort_flag, err_flag);
       tc_fence_after();
@@ -263,13 +272,6 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) +
                                (uint32_t)(buf * kBNMax + c0);
         tmem_ld_32x32(taddr, r);
-        if (OUT == 1) {
-          // this thread holds 2 channels x 16 basis functions of row `row`
-          const int64_t row = (int64_t)row0 + lane;
-          if (row < m_total && !*abort_flag)
-            store_image_row(image, image_channels, image_group, row, (n * bn + c0) / 16, r);
-          continue;
-        }
         if (OUT == 4) {
           // as OUT == 3 below: after the transposition this thread holds columns
           // row0 .. row0 + 31 of C^T's row n * bn + c0 + lane, 128 contiguous bytes
@@ -320,6 +322,18 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
             store_image_row(image, image_channels, image_group, sample, row0 / 16, v);
           continue;
         }
+        if (OUT == 0 && bias && sp == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const int64_t col = (int64_t)n * bn + c0 + i;
+            if (col < n_total) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(bias + col));
+          }
+        }
+        if (OUT == 2 && bias && sp == 0 && row0 + lane < m_total) {
+          const float v = __ldg(bias + row0 + lane);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + v);
+        }
         uint8_t* box = my_stage + (size_t)(box_iter & 1) * kOutBoxBytes;
         if (lane == 0) tma_store_wait_read<1>();  // the store that last used this box has read it
         __syncwarp();
@@ -342,12 +356,11 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
         __syncwarp();
         const int col0 = n * bn + c0;
         if (lane == 0 && row0 < m_total && col0 < n_total && !*abort_flag) {
-          if (OUT == 2)
-            tma_store_3d(&tm_c, smem_u32(box), row0, col0, sp);
-          else if (sch.add_slices)
-            tma_reduce_add_3d(&tm_c, smem_u32(box), col0, row0, 0);
+          const int x = OUT == 2 ? row0 : col0, y = OUT == 2 ? col0 : row0;
+          if (sch.add_slices)
+            tma_reduce_add_3d(&tm_c, smem_u32(box), x, y, bt);
           else
-            tma_store_3d(&tm_c, smem_u32(box), col0, row0, sp);
+            tma_store_3d(&tm_c, smem_u32(box), x, y, bt);
         }
       }
       tc_fence_before();
@@ -383,37 +396,39 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// 2-D bf16 tensor map: dim0 (contiguous) x dim1 rows, 128-byte swizzle, zero fill.
-int make_map(CUtensorMap* map, const __nv_bfloat16* base, int64_t dim0, int64_t dim1, int64_t ld,
-             int box0, int box1) {
+// 3-D bf16 tensor map: dim0 (contiguous) x dim1 rows x batches, 128-byte swizzle, zero
+// fill beyond the edges of a batch's own matrix.
+int make_map(CUtensorMap* map, const __nv_bfloat16* base, const GemmOperand& op, int64_t dim0,
+             int64_t dim1, int batches, int box0, int box1) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(TFGPC_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  if ((uintptr_t)base % 16 != 0 || (ld * 2) % 16 != 0)
+  if ((uintptr_t)base % 16 != 0 || (op.ld * 2) % 16 != 0 || (op.batch_stride * 2) % 16 != 0)
     return fail(TFGPC_EINVAL, "tensor-core GEMM operands need 16-byte aligned rows (ld %lld)",
-                (long long)ld);
-  cuuint64_t dims[2] = {(cuuint64_t)dim0, (cuuint64_t)dim1};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {(cuuint32_t)box0, (cuuint32_t)box1};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr,
+                (long long)op.ld);
+  cuuint64_t dims[3] = {(cuuint64_t)dim0, (cuuint64_t)dim1, (cuuint64_t)batches};
+  cuuint64_t strides[2] = {(cuuint64_t)op.ld * 2,
+                           (cuuint64_t)(batches > 1 ? op.batch_stride : dim1 * op.ld) * 2};
+  cuuint32_t box[3] = {(cuuint32_t)box0, (cuuint32_t)box1, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void*)base, dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TFGPC_ECUDA, "cuTensorMapEncodeTiled failed with %d", (int)r);
   return TFGPC_OK;
 }
 
-// 3-D fp32 tensor map of C: (columns, rows, k slices), boxes of 32 x 32 x 1 with
-// the 128-byte swizzle the epilogue writes its staging boxes in.
-int make_map_c(CUtensorMap* map, float* base, int64_t n, int64_t m, int64_t slices, int64_t ldc,
-               int64_t split_stride) {
+// 3-D fp32 tensor map of C: (columns, rows, batches), boxes of 32 x 32 x 1 with the
+// 128-byte swizzle the epilogue writes its staging boxes in.
+int make_map_c(CUtensorMap* map, float* base, int64_t n, int64_t m, int batches, int64_t ldc,
+               int64_t batch_stride) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(TFGPC_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-  if ((uintptr_t)base % 16 != 0 || ldc % 4 != 0 || split_stride % 4 != 0)
+  if ((uintptr_t)base % 16 != 0 || ldc % 4 != 0 || batch_stride % 4 != 0)
     return fail(TFGPC_EINVAL, "tensor-core GEMM output needs 16-byte aligned rows (ld %lld)",
                 (long long)ldc);
-  cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)m, (cuuint64_t)slices};
+  cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)m, (cuuint64_t)batches};
   cuuint64_t strides[2] = {(cuuint64_t)ldc * 4,
-                           (cuuint64_t)(slices > 1 ? split_stride : m * ldc) * 4};
+                           (cuuint64_t)(batches > 1 ? batch_stride : m * ldc) * 4};
   cuuint32_t box[3] = {32, 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void*)base, dims, strides, box, estr,
@@ -421,6 +436,43 @@ int make_map_c(CUtensorMap* map, float* base, int64_t n, int64_t m, int64_t slic
                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(TFGPC_ECUDA, "cuTensorMapEncodeTiled (C) failed with %d", (int)r);
   return TFGPC_OK;
+}
+
+// Columns of C per tile: a multiple of 32 (epilogue chunk), of 64 for MN-major B boxes.
+int tile_columns(int64_t N, bool b_mn) {
+  const int gran = b_mn ? 64 : 32;
+  const int bn = (int)(N < kBNMax ? N : kBNMax);
+  return (bn + gran - 1) / gran * gran;
+}
+
+// The four operand maps of a product with M x N tiles of kBM x bn.
+int operand_maps(CUtensorMap* maps, const GemmOperand& a, const GemmOperand& b, int64_t M,
+                 int64_t N, int64_t K, int batches, int bn) {
+  const __nv_bfloat16* ap[2] = {a.hi, a.mid};
+  const __nv_bfloat16* bp[2] = {b.hi, b.mid};
+  for (int i = 0; i < 2; ++i) {
+    int rc = a.major == Major::MN ? make_map(&maps[i], ap[i], a, M, K, batches, 64, kBK)
+                                  : make_map(&maps[i], ap[i], a, K, M, batches, kBK, kBM);
+    if (rc) return rc;
+    rc = b.major == Major::MN ? make_map(&maps[2 + i], bp[i], b, N, K, batches, 64, kBK)
+                              : make_map(&maps[2 + i], bp[i], b, K, N, batches, kBK, bn);
+    if (rc) return rc;
+  }
+  return TFGPC_OK;
+}
+
+TileSchedule schedule(int64_t M, int64_t N, int64_t K, int batches, int bn, int k_splits) {
+  TileSchedule sch;
+  sch.m_tiles = (int)((M + kBM - 1) / kBM);
+  sch.n_tiles = (int)((N + bn - 1) / bn);
+  sch.batches = batches;
+  sch.k_blocks = (int)((K + kBK - 1) / kBK);
+  sch.k_splits = k_splits < sch.k_blocks ? k_splits : sch.k_blocks;
+  sch.k_blocks_per_split = (sch.k_blocks + sch.k_splits - 1) / sch.k_splits;
+  // drop empty trailing slices
+  sch.k_splits = (sch.k_blocks + sch.k_blocks_per_split - 1) / sch.k_blocks_per_split;
+  sch.add_slices = sch.k_splits > 1 ? 1 : 0;
+  return sch;
 }
 
 // Instruction descriptor of tcgen05.mma kind::f16: D fp32, A and B bf16.
@@ -438,21 +490,21 @@ uint32_t make_idesc(int m, int n, bool a_mn, bool b_mn) {
 
 template <bool A_MN, bool B_MN, int OUT = 0>
 int launch(cudaStream_t st, const CUtensorMap* maps, int64_t M, int64_t N, int bn,
-           TileSchedule sch, int* err_flag, uint8_t* image = nullptr, int image_channels = 0,
-           int image_group = 4, const int32_t* row_order = nullptr) {
+           TileSchedule sch, int* err_flag, const float* bias = nullptr, uint8_t* image = nullptr,
+           int image_channels = 0, int image_group = 4, const int32_t* row_order = nullptr) {
   auto kern = gemm_bf16x3_kernel<A_MN, B_MN, OUT>;
-  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)kSmemBytes));
-  const int tiles = sch.m_tiles * sch.n_tiles * sch.k_splits;
-  const int grid = tiles < sm_count() ? tiles : sm_count();
+  const int stages = stages_for(bn);
+  const size_t smem = (size_t)stages * stage_bytes(bn) + kFixedBytes;
+  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int64_t tiles = (int64_t)sch.m_tiles * sch.n_tiles * sch.batches * sch.k_splits;
+  const int grid = tiles < sm_count() ? (int)tiles : sm_count();
   ProfScope prof(st, OUT == 4 ? "gemm_bf16x3_mn_k_scatter" : OUT == 3 ? "gemm_bf16x3_mn_k_image"
                      : OUT == 2 ? "gemm_bf16x3_mn_k_t"
-                     : OUT == 1 ? (B_MN ? "gemm_bf16x3_k_mn_image" : "gemm_bf16x3_k_k_image")
-                              : A_MN ? (B_MN ? "gemm_bf16x3_mn_mn" : "gemm_bf16x3_mn_k")
-                                     : (B_MN ? "gemm_bf16x3_k_mn" : "gemm_bf16x3_k_k"));
-  kern<<<grid, kThreads, kSmemBytes, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], M, N, bn,
-                                           make_idesc(kBM, bn, A_MN, B_MN), sch, err_flag, image,
-                                           image_channels, image_group, row_order);
+                     : A_MN ? (B_MN ? "gemm_bf16x3_mn_mn" : "gemm_bf16x3_mn_k")
+                            : (B_MN ? "gemm_bf16x3_k_mn" : "gemm_bf16x3_k_k"));
+  kern<<<grid, kThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], M, N, bn, stages,
+                                     make_idesc(kBM, bn, A_MN, B_MN), sch, err_flag, bias, image,
+                                     image_channels, image_group, row_order);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -475,47 +527,65 @@ __global__ void wait_probe_kernel(int* err_flag, unsigned long long limit_ns, in
   }
 }
 
-__global__ void split_kernel(const float* __restrict__ x, int64_t n, __nv_bfloat16* __restrict__ hi,
-                             __nv_bfloat16* __restrict__ mid) {
-  int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (i + 3 < n && ((uintptr_t)x % 16 == 0) && ((uintptr_t)hi % 8 == 0) && ((uintptr_t)mid % 8 == 0)) {
-    float4 v = __ldg(reinterpret_cast<const float4*>(x + i));
-    __nv_bfloat16 h[4], l[4];
-    split_bf16(v.x, h[0], l[0]); split_bf16(v.y, h[1], l[1]);
-    split_bf16(v.z, h[2], l[2]); split_bf16(v.w, h[3], l[3]);
-    *reinterpret_cast<uint2*>(hi + i) = *reinterpret_cast<uint2*>(h);
-    *reinterpret_cast<uint2*>(mid + i) = *reinterpret_cast<uint2*>(l);
-  } else {
-    for (int64_t j = i; j < n && j < i + 4; ++j) split_bf16(__ldg(x + j), hi[j], mid[j]);
+// Row r of a job's output is the split of a row of its source, `ld` columns wide with
+// zeros from `cols` on: row order[r], or, for a weight matrix whose basis functions are
+// padded from k_src to k_dst, row (r / k_dst) * k_src + r % k_dst (none if r % k_dst
+// reaches k_src).
+struct SplitJobs {
+  SplitJob job[2];
+  int64_t first_block[2];    // of job 1; total
+};
+
+__global__ void __launch_bounds__(256) split_rows_kernel(SplitJobs jobs) {
+  const bool second = (int64_t)blockIdx.x >= jobs.first_block[0];
+  const SplitJob j = second ? jobs.job[1] : jobs.job[0];
+  const unsigned quads = (unsigned)j.ld / 4;     // four values per thread
+  const unsigned i = (unsigned)((int64_t)blockIdx.x - (second ? jobs.first_block[0] : 0)) * 256u +
+                     threadIdx.x;
+  if (i >= (unsigned)j.rows * quads) return;
+  const unsigned r = (quads & (quads - 1)) == 0 ? i >> (31 - __clz(quads)) : i / quads;
+  const int c = (int)(i - r * quads) * 4;
+  int64_t src = r;
+  if (j.order) {
+    src = __ldg(j.order + r);
+  } else if (j.k_src != j.k_dst) {
+    const unsigned ch = r / (unsigned)j.k_dst;
+    const int k = (int)(r - ch * j.k_dst);
+    src = k < j.k_src ? (int64_t)ch * j.k_src + k : -1;
   }
-}
-
-// Row v of the output is the split of row order[v] of x (cols a multiple of 4,
-// 16-byte aligned rows).
-__global__ void split_rows_gather_kernel(const float* __restrict__ x,
-                                         const int32_t* __restrict__ order, int64_t rows,
-                                         int cols4, __nv_bfloat16* __restrict__ hi,
-                                         __nv_bfloat16* __restrict__ mid) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * cols4) return;
-  const int64_t v = i / cols4;
-  const int c = (int)(i - v * cols4);
-  const float4 val = __ldg(reinterpret_cast<const float4*>(x + (int64_t)__ldg(order + v) * cols4 * 4) + c);
+  float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (src >= 0) {
+    const float* p = j.x + src * j.cols + c;
+    if (j.cols % 4 == 0 && c < j.cols && (uintptr_t)j.x % 16 == 0) {
+      const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c + e < j.cols) v[e] = __ldg(p + e);
+    }
+  }
   uint2 h, m;
-  split2_bf16(val.x, val.y, h.x, m.x);
-  split2_bf16(val.z, val.w, h.y, m.y);
-  *reinterpret_cast<uint2*>(hi + i * 4) = h;
-  *reinterpret_cast<uint2*>(mid + i * 4) = m;
+  split2_bf16(v[0], v[1], h.x, m.x);
+  split2_bf16(v[2], v[3], h.y, m.y);
+  *reinterpret_cast<uint2*>(j.hi + (int64_t)r * j.ld + c) = h;
+  *reinterpret_cast<uint2*>(j.mid + (int64_t)r * j.ld + c) = m;
 }
 
+// hi_t, mid_t [cols, rows] = the split of the transpose of x, whose rows and columns are
+// padded with zeros as in split_rows_kernel.
 __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows, int64_t cols,
+                                       int cols_src, int k_src, int k_dst,
                                        __nv_bfloat16* __restrict__ hi_t,
                                        __nv_bfloat16* __restrict__ mid_t) {
   __shared__ float tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    int64_t r = r0 + j, cc = c0 + threadIdx.x;
-    tile[j][threadIdx.x] = (r < rows && cc < cols) ? __ldg(x + r * cols + cc) : 0.0f;
+    const int64_t r = r0 + j, cc = c0 + threadIdx.x;
+    const int64_t ch = r / k_dst;
+    const int k = (int)(r - ch * k_dst);
+    tile[j][threadIdx.x] = (r < rows && cc < cols_src && k < k_src)
+                               ? __ldg(x + (ch * k_src + k) * cols_src + cc) : 0.0f;
   }
   __syncthreads();
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -529,15 +599,6 @@ __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows
   }
 }
 
-__global__ void reduce_splits_kernel(const float* __restrict__ partial, int splits, int64_t stride,
-                                     int64_t n, float* __restrict__ out) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float acc = 0.0f;
-  for (int s = 0; s < splits; ++s) acc += __ldg(partial + (int64_t)s * stride + i);
-  out[i] = acc;
-}
-
 }  // namespace
 
 // The tensor cores add into their fp32 accumulator by truncation, so the error of
@@ -549,52 +610,18 @@ __global__ void reduce_splits_kernel(const float* __restrict__ partial, int spli
 // summed in round-to-nearest fp32.
 constexpr int64_t kMaxChain = 2048;
 
-int gemm_pick_k_splits(int64_t M, int64_t N, int64_t K) {
-  const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBNMax - 1) / kBNMax);
-  const int64_t k_blocks = (K + kBK - 1) / kBK;
-  int64_t splits = sm_count() / (tiles > 0 ? tiles : 1);
-  if (splits < 1) splits = 1;
-  const int64_t for_chain = (K + kMaxChain - 1) / kMaxChain;
-  if (splits < for_chain) splits = for_chain;
-  if (splits > k_blocks) splits = k_blocks > 0 ? k_blocks : 1;
-  return (int)splits;
-}
-
-int gemm_bf16x3_grad_image(cudaStream_t stream, int64_t M, int channels, int64_t K,
-                           const GemmOperand& a, const GemmOperand& b, void* image, int group,
-                           int* err_flag) {
-  const int64_t N = (int64_t)channels * 16;
-  TFGPC_REQUIRE(M > 0 && channels > 0 && K > 0 && M < (int64_t)INT32_MAX && K < (int64_t)INT32_MAX,
-                "GEMM expects positive sizes below 2^31");
-  TFGPC_REQUIRE(a.major == Major::K && channels % 2 == 0 && (uintptr_t)image % 32 == 0 &&
-                group >= 1 && group <= 4,
-                "gradient-image GEMM expects a K-major left operand and groups of 1 to 4 rows");
-  const bool b_mn = b.major == Major::MN;
-  int bn = (int)(N < kBNMax ? N : kBNMax);
-  const int gran = b_mn ? 64 : 32;
-  bn = (bn + gran - 1) / gran * gran;
-  CUtensorMap maps[5] = {};
-  int rc;
-  if ((rc = make_map(&maps[0], a.hi, K, M, a.ld, kBK, kBM))) return rc;
-  if ((rc = make_map(&maps[1], a.mid, K, M, a.ld, kBK, kBM))) return rc;
-  const __nv_bfloat16* bp[2] = {b.hi, b.mid};
-  for (int i = 0; i < 2; ++i) {
-    rc = b_mn ? make_map(&maps[2 + i], bp[i], N, K, b.ld, 64, kBK)
-              : make_map(&maps[2 + i], bp[i], K, N, b.ld, kBK, bn);
-    if (rc) return rc;
-  }
-  TileSchedule sch;
-  sch.m_tiles = (int)((M + kBM - 1) / kBM);
-  sch.n_tiles = (int)((N + bn - 1) / bn);
-  sch.k_blocks = (int)((K + kBK - 1) / kBK);
-  sch.k_splits = 1;
-  sch.add_slices = 0;
-  sch.k_blocks_per_split = sch.k_blocks;
-  if (b_mn)
-    return launch<false, true, 1>(stream, maps, M, N, bn, sch, err_flag, (uint8_t*)image, channels,
-                                  group);
-  return launch<false, false, 1>(stream, maps, M, N, bn, sch, err_flag, (uint8_t*)image, channels,
-                                 group);
+static int pick_k_splits(int64_t tiles, int64_t K) {
+  const int64_t sms = sm_count(), k_blocks = (K + kBK - 1) / kBK;
+  const int64_t chain = (K + kMaxChain - 1) / kMaxChain;
+  // As many slices as the last wave of tiles has room for (a slice of eight slots or
+  // more pays for its share of the output): 8 tiles of a 41 000-sample weight gradient
+  // ran as 168 slices in two waves, the second of 20.
+  const int64_t waves = (tiles * chain + sms - 1) / sms;
+  int64_t splits = waves <= 4 ? waves * sms / tiles : chain;
+  const int64_t most = k_blocks / 8;
+  if (splits > most) splits = most;
+  if (splits < chain) splits = chain;
+  return (int)(splits < 1 ? 1 : splits);
 }
 
 int gemm_bf16x3_grad_image_tn(cudaStream_t stream, int channels, int64_t N, int64_t K,
@@ -607,23 +634,12 @@ int gemm_bf16x3_grad_image_tn(cudaStream_t stream, int channels, int64_t N, int6
                 (uintptr_t)image % 32 == 0 && group >= 1 && group <= 4,
                 "gradient-image GEMM (transposed form) expects an MN-major left and a K-major "
                 "right operand and groups of 1 to 4 rows");
-  int bn = (int)(N < kBNMax ? N : kBNMax);
-  bn = (bn + 31) / 32 * 32;
+  const int bn = tile_columns(N, false);
   CUtensorMap maps[5] = {};
-  int rc;
-  if ((rc = make_map(&maps[0], a.hi, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[1], a.mid, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[2], b.hi, K, N, b.ld, kBK, bn))) return rc;
-  if ((rc = make_map(&maps[3], b.mid, K, N, b.ld, kBK, bn))) return rc;
-  TileSchedule sch;
-  sch.m_tiles = (int)((M + kBM - 1) / kBM);
-  sch.n_tiles = (int)((N + bn - 1) / bn);
-  sch.k_blocks = (int)((K + kBK - 1) / kBK);
-  sch.k_splits = 1;
-  sch.add_slices = 0;
-  sch.k_blocks_per_split = sch.k_blocks;
-  return launch<true, false, 3>(stream, maps, M, N, bn, sch, err_flag, (uint8_t*)image, channels,
-                                group);
+  int rc = operand_maps(maps, a, b, M, N, K, 1, bn);
+  if (rc) return rc;
+  return launch<true, false, 3>(stream, maps, M, N, bn, schedule(M, N, K, 1, bn, 1), err_flag,
+                                nullptr, (uint8_t*)image, channels, group);
 }
 
 int gemm_bf16x3_tn_scatter(cudaStream_t stream, int64_t M, int64_t N, int64_t K,
@@ -636,139 +652,80 @@ int gemm_bf16x3_tn_scatter(cudaStream_t stream, int64_t M, int64_t N, int64_t K,
                 (uintptr_t)out % 32 == 0 && ld_out % 8 == 0,
                 "row-scattering GEMM expects an MN-major left and a K-major right operand and "
                 "32-byte aligned output rows");
-  int bn = (int)(N < kBNMax ? N : kBNMax);
-  bn = (bn + 31) / 32 * 32;
+  const int bn = tile_columns(N, false);
   CUtensorMap maps[5] = {};
-  int rc;
-  if ((rc = make_map(&maps[0], a.hi, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[1], a.mid, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[2], b.hi, K, N, b.ld, kBK, bn))) return rc;
-  if ((rc = make_map(&maps[3], b.mid, K, N, b.ld, kBK, bn))) return rc;
-  TileSchedule sch;
-  sch.m_tiles = (int)((M + kBM - 1) / kBM);
-  sch.n_tiles = (int)((N + bn - 1) / bn);
-  sch.k_blocks = (int)((K + kBK - 1) / kBK);
-  sch.k_splits = 1;
-  sch.add_slices = 0;
-  sch.k_blocks_per_split = sch.k_blocks;
-  return launch<true, false, 4>(stream, maps, M, N, bn, sch, err_flag, (uint8_t*)out, (int)ld_out, 4,
-                                row_order);
-}
-
-int gemm_bf16x3_tn(cudaStream_t stream, int64_t M, int64_t N, int64_t K, const GemmOperand& a,
-                   const GemmOperand& b, float* ct, int64_t ldct, int* err_flag) {
-  TFGPC_REQUIRE(M > 0 && N > 0 && K > 0 && M < (int64_t)INT32_MAX && N < (int64_t)INT32_MAX &&
-                K < (int64_t)INT32_MAX, "GEMM expects positive sizes below 2^31");
-  TFGPC_REQUIRE(a.major == Major::MN && b.major == Major::K,
-                "transposed-output GEMM expects an MN-major left and a K-major right operand");
-  int bn = (int)(N < kBNMax ? N : kBNMax);
-  bn = (bn + 31) / 32 * 32;
-  CUtensorMap maps[5];
-  int rc;
-  if ((rc = make_map(&maps[0], a.hi, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[1], a.mid, M, K, a.ld, 64, kBK))) return rc;
-  if ((rc = make_map(&maps[2], b.hi, K, N, b.ld, kBK, bn))) return rc;
-  if ((rc = make_map(&maps[3], b.mid, K, N, b.ld, kBK, bn))) return rc;
-  // C^T: N rows of M columns
-  if ((rc = make_map_c(&maps[4], ct, M, N, 1, ldct, 0))) return rc;
-  TileSchedule sch;
-  sch.m_tiles = (int)((M + kBM - 1) / kBM);
-  sch.n_tiles = (int)((N + bn - 1) / bn);
-  sch.k_blocks = (int)((K + kBK - 1) / kBK);
-  sch.k_splits = 1;
-  sch.add_slices = 0;
-  sch.k_blocks_per_split = sch.k_blocks;
-  return launch<true, false, 2>(stream, maps, M, N, bn, sch, err_flag);
-}
-
-int gemm_bf16x3(cudaStream_t stream, int64_t M, int64_t N, int64_t K, const GemmOperand& a,
-                const GemmOperand& b, float* c, int64_t ldc, int k_splits, int64_t split_stride,
-                int* err_flag) {
-  TFGPC_REQUIRE(M > 0 && N > 0 && K > 0, "GEMM expects positive sizes");
-  TFGPC_REQUIRE(M < (int64_t)INT32_MAX && N < (int64_t)INT32_MAX && K < (int64_t)INT32_MAX,
-                "GEMM sizes must stay below 2^31");
-  TFGPC_REQUIRE(k_splits >= 1, "GEMM expects k_splits >= 1");
-  const bool a_mn = a.major == Major::MN, b_mn = b.major == Major::MN;
-  // columns of C per tile: a multiple of 32 (epilogue chunk), of 64 for MN-major B boxes
-  int bn = (int)(N < kBNMax ? N : kBNMax);
-  const int gran = b_mn ? 64 : 32;
-  bn = (bn + gran - 1) / gran * gran;
-  CUtensorMap maps[5];
-  int rc;
-  const __nv_bfloat16* ap[2] = {a.hi, a.mid};
-  const __nv_bfloat16* bp[2] = {b.hi, b.mid};
-  for (int i = 0; i < 2; ++i) {
-    rc = a_mn ? make_map(&maps[i], ap[i], M, K, a.ld, 64, kBK)
-              : make_map(&maps[i], ap[i], K, M, a.ld, kBK, kBM);
-    if (rc) return rc;
-    rc = b_mn ? make_map(&maps[2 + i], bp[i], N, K, b.ld, 64, kBK)
-              : make_map(&maps[2 + i], bp[i], K, N, b.ld, kBK, bn);
-    if (rc) return rc;
-  }
-  TileSchedule sch;
-  sch.m_tiles = (int)((M + kBM - 1) / kBM);
-  sch.n_tiles = (int)((N + bn - 1) / bn);
-  sch.k_blocks = (int)((K + kBK - 1) / kBK);
-  sch.k_splits = k_splits < sch.k_blocks ? k_splits : sch.k_blocks;
-  sch.k_blocks_per_split = (sch.k_blocks + sch.k_splits - 1) / sch.k_splits;
-  // drop empty trailing slices
-  sch.k_splits = (sch.k_blocks + sch.k_blocks_per_split - 1) / sch.k_blocks_per_split;
-  // split_stride 0 with several slices: all of them are added into c, which
-  // starts from zero, by the store unit (the order of the additions, and with it
-  // the last bits of the sums, varies from run to run)
-  sch.add_slices = (sch.k_splits > 1 && split_stride == 0) ? 1 : 0;
-  if (sch.add_slices) {
-    TFGPC_CUDA(cudaMemset2DAsync(c, sizeof(float) * (size_t)ldc, 0, sizeof(float) * (size_t)N,
-                                 (size_t)M, stream));
-  } else if (sch.k_splits < k_splits && split_stride != 0) {
-    // the caller sums k_splits slices: the unused ones must read as zero
-    TFGPC_CUDA(cudaMemsetAsync(c + (int64_t)sch.k_splits * split_stride, 0,
-                               sizeof(float) * (size_t)(k_splits - sch.k_splits) * split_stride,
-                               stream));
-  }
-  rc = make_map_c(&maps[4], c, N, M, sch.add_slices ? 1 : sch.k_splits, ldc, split_stride);
+  int rc = operand_maps(maps, a, b, M, N, K, 1, bn);
   if (rc) return rc;
-  if (a_mn && b_mn) return launch<true, true>(stream, maps, M, N, bn, sch, err_flag);
-  if (a_mn) return launch<true, false>(stream, maps, M, N, bn, sch, err_flag);
-  if (b_mn) return launch<false, true>(stream, maps, M, N, bn, sch, err_flag);
-  return launch<false, false>(stream, maps, M, N, bn, sch, err_flag);
+  return launch<true, false, 4>(stream, maps, M, N, bn, schedule(M, N, K, 1, bn, 1), err_flag,
+                                nullptr, (uint8_t*)out, (int)ld_out, 4, row_order);
 }
 
-int split_to_bf16(cudaStream_t stream, const float* x, int64_t n, __nv_bfloat16* hi,
-                  __nv_bfloat16* mid) {
-  if (n <= 0) return TFGPC_OK;
-  ProfScope prof(stream, "split_bf16");
-  split_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, stream>>>(x, n, hi, mid);
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
+int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
+  TFGPC_REQUIRE(p.M > 0 && p.N > 0 && p.K > 0 && p.batches > 0, "GEMM expects positive sizes");
+  TFGPC_REQUIRE(p.M < (int64_t)INT32_MAX && p.N < (int64_t)INT32_MAX && p.K < (int64_t)INT32_MAX,
+                "GEMM sizes must stay below 2^31");
+  const bool a_mn = p.a.major == Major::MN, b_mn = p.b.major == Major::MN;
+  TFGPC_REQUIRE(!p.transposed || (a_mn && !b_mn),
+                "transposed-output GEMM expects an MN-major left and a K-major right operand");
+  const int bn = tile_columns(p.N, b_mn);
+  CUtensorMap maps[5] = {};
+  int rc = operand_maps(maps, p.a, p.b, p.M, p.N, p.K, p.batches, bn);
+  if (rc) return rc;
+  const int64_t tiles = ((p.M + kBM - 1) / kBM) * ((p.N + bn - 1) / bn) * p.batches;
+  const TileSchedule sch = schedule(p.M, p.N, p.K, p.batches, bn, pick_k_splits(tiles, p.K));
+  const int64_t rows = p.transposed ? p.N : p.M, cols = p.transposed ? p.M : p.N;
+  if (sch.add_slices) {
+    // the slices are added into c, which starts from zero, by the store unit (the order
+    // of the additions, and with it the last bits of the sums, varies from run to run)
+    const bool dense = p.batches == 1 ? p.ldc == cols
+                                      : (p.c_batch_stride == cols && p.ldc == cols * p.batches) ||
+                                            (p.ldc == cols && p.c_batch_stride == cols * rows);
+    if (dense) {
+      TFGPC_CUDA(cudaMemsetAsync(p.c, 0, sizeof(float) * (size_t)rows * cols * p.batches, stream));
+    } else {
+      for (int b = 0; b < p.batches; ++b)
+        TFGPC_CUDA(cudaMemset2DAsync(p.c + b * p.c_batch_stride, sizeof(float) * (size_t)p.ldc, 0,
+                                     sizeof(float) * (size_t)cols, (size_t)rows, stream));
+    }
+  }
+  rc = make_map_c(&maps[4], p.c, cols, rows, p.batches, p.ldc, p.c_batch_stride);
+  if (rc) return rc;
+  if (p.transposed)
+    return launch<true, false, 2>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
+  if (a_mn && b_mn) return launch<true, true>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
+  if (a_mn) return launch<true, false>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
+  if (b_mn) return launch<false, true>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
+  return launch<false, false>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
 }
 
-int split_rows_gather_to_bf16(cudaStream_t stream, const float* x, const int32_t* order,
-                              int64_t rows, int64_t cols, __nv_bfloat16* hi, __nv_bfloat16* mid) {
-  if (rows <= 0 || cols <= 0) return TFGPC_OK;
-  TFGPC_REQUIRE(cols % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)hi % 8 == 0 &&
-                (uintptr_t)mid % 8 == 0, "split_rows_gather expects 16-byte aligned rows");
+int split_rows(cudaStream_t stream, const SplitJob& first, const SplitJob* second) {
+  SplitJobs jobs{};
+  int64_t blocks = 0;
+  for (int i = 0; i < (second ? 2 : 1); ++i) {
+    const SplitJob& j = i ? *second : first;
+    TFGPC_REQUIRE(j.ld % 4 == 0 && (uintptr_t)j.hi % 8 == 0 && (uintptr_t)j.mid % 8 == 0,
+                  "split_rows expects rows of a multiple of 4 values");
+    TFGPC_REQUIRE(j.rows * (j.ld / 4) < (int64_t)UINT32_MAX, "split_rows: too many values");
+    jobs.job[i] = j;
+    blocks += j.rows > 0 && j.ld > 0 ? (j.rows * (j.ld / 4) + 255) / 256 : 0;
+    jobs.first_block[i] = blocks;
+  }
+  if (!second) jobs.first_block[0] = blocks + 1;   // every block works on job 0
+  if (blocks == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(blocks < (int64_t)INT32_MAX, "split_rows: too many values");
   ProfScope prof(stream, "split_bf16");
-  split_rows_gather_kernel<<<blocks_for(rows * (cols / 4), 256), 256, 0, stream>>>(
-      x, order, rows, (int)(cols / 4), hi, mid);
+  split_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(jobs);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
 int split_transpose_to_bf16(cudaStream_t stream, const float* x, int64_t rows, int64_t cols,
-                            __nv_bfloat16* hi_t, __nv_bfloat16* mid_t) {
+                            int cols_src, int k_src, int k_dst, __nv_bfloat16* hi_t,
+                            __nv_bfloat16* mid_t) {
   if (rows <= 0 || cols <= 0) return TFGPC_OK;
   dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-  split_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(x, rows, cols, hi_t, mid_t);
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
-}
-
-int reduce_splits(cudaStream_t stream, const float* partial, int splits, int64_t stride, int64_t n,
-                  float* out) {
-  if (n <= 0) return TFGPC_OK;
-  ProfScope prof(stream, "reduce_splits");
-  reduce_splits_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(partial, splits, stride, n, out);
+  split_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(x, rows, cols, cols_src, k_src, k_dst,
+                                                           hi_t, mid_t);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }

@@ -7,12 +7,18 @@
 // concatenated (column g * H_last + h) and divided by the pair's density:
 //   diff = (p_in[j] - p_out[s]) * inv_radius                      (MCConv.py:264-269)
 //   a_0 = diff, a_l = act(a_{l-1} W_l[g] + b_l[g]), basis[m, g H + h] = a_L[h] / pdf[m]
-// kernel_basis.cu holds the fast path for one hidden layer and the weight
-// gradients only; this file is the general path: one thread per pair walks the
-// MLPs with its activations in local arrays.  The backward pass recomputes the
+// kernel_basis.cu holds the fast path for one hidden layer and the weight gradients
+// only; this file is the general path.  A block takes a tile of pairs, one per thread,
+// whose activations stand in shared memory as [unit][pair]: a layer is eight outputs at
+// a time in registers (one load of the pair's input and two broadcast loads of weights
+// per eight FMAs), for any width.  (Activations in per-thread arrays indexed at run time
+// lived in local memory: 83 us forward and 286 us backward on 360 000 pairs of an 8-16
+// MLP, against a few us of arithmetic.)  The backward pass recomputes the
 // activations, back-propagates dbasis, and adds
-//   * the weight and bias gradients: reduced over the warp by shuffles, then over
-//     the block in shared memory, one global atomic per value and block;
+//   * the weight and bias gradients: every value belongs to one thread of the block, which
+//     sums it over the tile's pairs, four per load, and over its tiles in shared memory
+//     (a shuffle reduction per value and warp before); one global atomic per value and
+//     block;
 //   * the gradient of the point coordinates (MCConv's inputs are the positions:
 //     monte_carlo_conv_test.py:182-219 checks this jacobian): +d_diff / radius to
 //     the neighbor's row of points_in, -d_diff / radius to the sample's row of
@@ -24,17 +30,22 @@
 namespace tfgpc {
 namespace {
 
-constexpr int kMlpThreads = 128;
 constexpr int kMaxLayers = 4;
 constexpr int kMaxWidth = 64;
-constexpr int kMaxParams = 8192;     // floats of all weights and biases (32 KB of shared memory)
+constexpr int kMaxParams = 8192;     // floats of all weights and biases
+constexpr size_t kMaxMlpSmem = 227 * 1024;
 
 struct MlpShape {
   int D, G, L;
   int h[kMaxLayers + 1];       // h[0] = D, h[l] = width of layer l
-  int w_off[kMaxLayers];       // offset of layer l's weights [G][h[l-1]][h[l]] in the parameter block
-  int b_off[kMaxLayers];       // offset of layer l's biases [G][h[l]]
-  int params;                  // floats in the parameter block (weights of all layers, then biases)
+  int hp[kMaxLayers + 1];      // the same rounded up to 8 (l > 0)
+  int w_off[kMaxLayers];       // layer l's weights [G][h[l-1]][hp[l]] in the padded parameter block
+  int b_off[kMaxLayers];       // layer l's biases [G][hp[l]]
+  int params;                  // floats in the padded block
+  int rows;                    // h[0] + ... + h[L]
+  int widest;                  // max h[l]
+  const float* w[kMaxLayers];  // [G][h[l-1]][h[l]]
+  const float* b[kMaxLayers];  // [G][h[l]]
 };
 
 __device__ __forceinline__ float act_fwd(float x, int act, float alpha) {
@@ -42,180 +53,327 @@ __device__ __forceinline__ float act_fwd(float x, int act, float alpha) {
   return x > 0.0f ? x : x * alpha;
 }
 
-__device__ __forceinline__ float act_bwd(float x, int act, float alpha) {
-  if (act == 1) return x > 0.0f ? 1.0f : expf(x);
-  return x > 0.0f ? 1.0f : alpha;
+// Slope from the activation's value (ELU: exp(x) = value + 1 below zero).
+__device__ __forceinline__ float act_slope(float value, int act, float alpha) {
+  if (value > 0.0f) return 1.0f;
+  return act == 1 ? value + 1.0f : alpha;
 }
 
-__device__ __forceinline__ void load_params(const MlpShape& s, const float* __restrict__ weights,
-                                            const float* __restrict__ biases, float* par) {
-  const int nw = s.b_off[0];   // biases follow the weights
-  for (int i = threadIdx.x; i < s.params; i += kMlpThreads)
-    par[i] = i < nw ? __ldg(weights + i) : __ldg(biases + i - nw);
-}
-
-__global__ void __launch_bounds__(kMlpThreads)
-kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
-                        const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                        const float* __restrict__ pdf, const float* __restrict__ weights,
-                        const float* __restrict__ biases, float inv_radius, int act, float alpha,
-                        int pdf_by_nbr, float* __restrict__ basis) {
-  extern __shared__ float par[];
-  load_params(s, weights, biases, par);
-  __syncthreads();
-  const int k_total = s.G * s.h[s.L];
-  for (int64_t m = (int64_t)blockIdx.x * kMlpThreads + threadIdx.x; m < M;
-       m += (int64_t)gridDim.x * kMlpThreads) {
-    const int2 nb = __ldg(neigh + m);
-    float diff[TFGPC_MAX_DIMS];
-    for (int d = 0; d < s.D; ++d)
-      diff[d] = (__ldg(p_in + (int64_t)nb.x * s.D + d) - __ldg(p_out + (int64_t)nb.y * s.D + d)) *
-                inv_radius;
-    const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
-    for (int g = 0; g < s.G; ++g) {
-      float a[kMaxWidth], b[kMaxWidth];
-      for (int d = 0; d < s.D; ++d) a[d] = diff[d];
-      for (int l = 1; l <= s.L; ++l) {
-        const int hi = s.h[l - 1], ho = s.h[l];
-        const float* w = par + s.w_off[l - 1] + g * hi * ho;
-        const float* bb = par + s.b_off[l - 1] + g * ho;
-        for (int j = 0; j < ho; ++j) {
-          float pre = bb[j];
-          for (int i = 0; i < hi; ++i) pre = fmaf(a[i], w[i * ho + j], pre);
-          b[j] = act_fwd(pre, act, alpha);
-        }
-        for (int j = 0; j < ho; ++j) a[j] = b[j];
-      }
-      float* dst = basis + m * k_total + g * s.h[s.L];
-      for (int j = 0; j < s.h[s.L]; ++j) dst[j] = a[j] * inv_pdf;
+__device__ __forceinline__ void load_params(const MlpShape& s, float* par) {
+  for (int l = 0; l < s.L; ++l) {
+    const int ho = s.h[l + 1], hp = s.hp[l + 1];
+    for (int i = threadIdx.x; i < s.G * s.h[l] * hp; i += blockDim.x) {
+      const int r = i / hp, c = i - r * hp;
+      par[s.w_off[l] + i] = c < ho ? __ldg(s.w[l] + r * ho + c) : 0.0f;
+    }
+    for (int i = threadIdx.x; i < s.G * hp; i += blockDim.x) {
+      const int r = i / hp, c = i - r * hp;
+      par[s.b_off[l] + i] = c < ho ? __ldg(s.b[l] + r * ho + c) : 0.0f;
     }
   }
 }
 
-__global__ void __launch_bounds__(kMlpThreads)
+// Outputs 8q .. 8q+7 (before the activation) of layer l + 1 of MLP g for this thread's
+// pair, whose inputs are the column `in` (`stride` floats apart).
+__device__ __forceinline__ void layer8(const MlpShape& s, const float* par, int l, int g, int q,
+                                       const float* in, int stride, float* acc) {
+  const int hi = s.h[l], hp = s.hp[l + 1];
+  const float4* bb = reinterpret_cast<const float4*>(par + s.b_off[l] + g * hp) + 2 * q;
+  const float4* ww = reinterpret_cast<const float4*>(par + s.w_off[l] + g * hi * hp) + 2 * q;
+  float4 b0 = bb[0], b1 = bb[1];
+  acc[0] = b0.x; acc[1] = b0.y; acc[2] = b0.z; acc[3] = b0.w;
+  acc[4] = b1.x; acc[5] = b1.y; acc[6] = b1.z; acc[7] = b1.w;
+#pragma unroll 4
+  for (int i = 0; i < hi; ++i) {
+    const float a = in[i * stride];
+    const float4 w0 = ww[i * (hp / 4)], w1 = ww[i * (hp / 4) + 1];
+    acc[0] = fmaf(a, w0.x, acc[0]); acc[1] = fmaf(a, w0.y, acc[1]);
+    acc[2] = fmaf(a, w0.z, acc[2]); acc[3] = fmaf(a, w0.w, acc[3]);
+    acc[4] = fmaf(a, w1.x, acc[4]); acc[5] = fmaf(a, w1.y, acc[5]);
+    acc[6] = fmaf(a, w1.z, acc[6]); acc[7] = fmaf(a, w1.w, acc[7]);
+  }
+}
+
+__device__ __forceinline__ void load_diff(const MlpShape& s, int2 nb, const float* __restrict__ p_in,
+                                          const float* __restrict__ p_out, float inv_radius,
+                                          float* col, int stride) {
+  for (int d = 0; d < s.D; ++d)
+    col[d * stride] = (__ldg(p_in + (int64_t)nb.x * s.D + d) - __ldg(p_out + (int64_t)nb.y * s.D + d)) *
+                      inv_radius;
+}
+
+__global__ void __launch_bounds__(128)
+kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
+                        const float* __restrict__ p_out, const int2* __restrict__ neigh,
+                        const float* __restrict__ pdf, float inv_radius, int act, float alpha,
+                        int pdf_by_nbr, float* __restrict__ basis) {
+  extern __shared__ __align__(16) float par[];
+  const int stride = blockDim.x;
+  float* diff = par + s.params + threadIdx.x;        // [D][pair]
+  float* buf0 = diff + s.D * stride;                 // [widest][pair], twice
+  float* buf1 = buf0 + s.widest * stride;
+  load_params(s, par);
+  __syncthreads();
+  const int hl = s.h[s.L], k_total = s.G * hl;
+  for (int64_t m = (int64_t)blockIdx.x * stride + threadIdx.x; m < M;
+       m += (int64_t)gridDim.x * stride) {
+    const int2 nb = __ldg(neigh + m);
+    load_diff(s, nb, p_in, p_out, inv_radius, diff, stride);
+    const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+    for (int g = 0; g < s.G; ++g) {
+      const float* in = diff;
+      for (int l = 0; l < s.L; ++l) {
+        const bool last = l == s.L - 1;
+        float* out = (l & 1) ? buf1 : buf0;
+        float* dst = basis + m * k_total + g * hl;
+        for (int q = 0; q * 8 < s.h[l + 1]; ++q) {
+          float acc[8];
+          layer8(s, par, l, g, q, in, stride, acc);
+          const int cnt = min(8, s.h[l + 1] - 8 * q);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[e] = act_fwd(acc[e], act, alpha);
+          if (!last) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (e < cnt) out[(8 * q + e) * stride] = acc[e];
+          } else if (hl % 4 == 0) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 4)
+              if (e < cnt)
+                *reinterpret_cast<float4*>(dst + 8 * q + e) =
+                    make_float4(acc[e] * inv_pdf, acc[e + 1] * inv_pdf, acc[e + 2] * inv_pdf,
+                                acc[e + 3] * inv_pdf);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (e < cnt) dst[8 * q + e] = acc[e] * inv_pdf;
+          }
+        }
+        in = out;
+      }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(128)
 kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
                         const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                        const float* __restrict__ pdf, const float* __restrict__ weights,
-                        const float* __restrict__ biases, float inv_radius, int act, float alpha,
+                        const float* __restrict__ pdf, float inv_radius, int act, float alpha,
                         int pdf_by_nbr, const float* __restrict__ dbasis,
-                        float* __restrict__ dweights,
-                        float* __restrict__ dbiases, float* __restrict__ dp_in,
-                        float* __restrict__ dp_out, float* __restrict__ dpdf) {
-  extern __shared__ float smem[];
-  float* par = smem;                 // parameters
-  float* acc = smem + s.params;      // their gradients, summed over the block
-  load_params(s, weights, biases, par);
-  for (int i = threadIdx.x; i < s.params; i += kMlpThreads) acc[i] = 0.0f;
+                        float* __restrict__ dweights, float* __restrict__ dbiases,
+                        float* __restrict__ dp_in, float* __restrict__ dp_out,
+                        float* __restrict__ dpdf) {
+  extern __shared__ __align__(16) float par[];       // parameters
+  const int tile = blockDim.x;
+  const int stride = tile + 4;                       // rows of [unit][pair], banks shifted by 4
+  float* acc = par + s.params;                       // their gradients, summed over the tiles
+  float* units = acc + s.params;                     // activations of every layer
+  float* grads = units + s.rows * stride;            // [2][widest][pair]
+  load_params(s, par);
+  for (int i = threadIdx.x; i < s.params; i += tile) acc[i] = 0.0f;
   __syncthreads();
-  const int k_total = s.G * s.h[s.L];
-  const int lane = threadIdx.x & 31;
-  // whole warps iterate together (the shuffles below need all lanes): the loop
-  // bound is rounded up to the warp, lanes beyond M contribute zeros
-  const int64_t stride = (int64_t)gridDim.x * kMlpThreads;
-  for (int64_t m0 = (int64_t)blockIdx.x * kMlpThreads + (threadIdx.x & ~31); m0 < M; m0 += stride) {
-    const int64_t m = m0 + lane;
-    const bool live = m < M;
+  const int hl = s.h[s.L], k_total = s.G * hl;
+  float* my_units = units + threadIdx.x;
+  for (int64_t m0 = (int64_t)blockIdx.x * tile; m0 < M; m0 += (int64_t)gridDim.x * tile) {
+    const int64_t m = m0 + threadIdx.x;
+    const bool live = m < M;     // other threads' pairs contribute zeros
     int2 nb = make_int2(0, 0);
-    float diff[TFGPC_MAX_DIMS], ddiff[TFGPC_MAX_DIMS];
     float inv_pdf = 0.0f, dpdf_m = 0.0f;
+    float ddiff[TFGPC_MAX_DIMS];
+#pragma unroll
+    for (int d = 0; d < TFGPC_MAX_DIMS; ++d) ddiff[d] = 0.0f;
     if (live) {
       nb = __ldg(neigh + m);
       inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
-    }
-    for (int d = 0; d < s.D; ++d) {
-      diff[d] = live ? (__ldg(p_in + (int64_t)nb.x * s.D + d) - __ldg(p_out + (int64_t)nb.y * s.D + d)) *
-                           inv_radius : 0.0f;
-      ddiff[d] = 0.0f;
+      load_diff(s, nb, p_in, p_out, inv_radius, my_units, stride);
+    } else {
+      for (int d = 0; d < s.D; ++d) my_units[d * stride] = 0.0f;
     }
     for (int g = 0; g < s.G; ++g) {
-      // forward with every layer's input and pre-activation kept
-      float a[kMaxLayers + 1][kMaxWidth], pre[kMaxLayers][kMaxWidth];
-      for (int d = 0; d < s.D; ++d) a[0][d] = diff[d];
-      for (int l = 1; l <= s.L; ++l) {
-        const int hi = s.h[l - 1], ho = s.h[l];
-        const float* w = par + s.w_off[l - 1] + g * hi * ho;
-        const float* bb = par + s.b_off[l - 1] + g * ho;
-        for (int j = 0; j < ho; ++j) {
-          float p = bb[j];
-          for (int i = 0; i < hi; ++i) p = fmaf(a[l - 1][i], w[i * ho + j], p);
-          pre[l - 1][j] = p;
-          a[l][j] = act_fwd(p, act, alpha);
+      int row = 0;
+      for (int l = 0; l < s.L; ++l) {
+        const int next = row + s.h[l];
+        for (int q = 0; q * 8 < s.h[l + 1]; ++q) {
+          float v[8];
+          layer8(s, par, l, g, q, my_units + row * stride, stride, v);
+          const int cnt = min(8, s.h[l + 1] - 8 * q);
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (e < cnt) my_units[(next + 8 * q + e) * stride] = act_fwd(v[e], act, alpha);
         }
+        row = next;
       }
-      // gradient of the last layer's output: dbasis / pdf; the density's own
-      // gradient: basis = a_L / pdf  ->  d/dpdf = -a_L / pdf^2
-      float grad[kMaxWidth], gprev[kMaxWidth];
-      const int hl = s.h[s.L];
+      // gradient of the last layer's pre-activations: dbasis / pdf * slope; the density's
+      // own gradient: basis = a_L / pdf  ->  d/dpdf = -a_L / pdf^2
+      int cur = 0;
       for (int j = 0; j < hl; ++j) {
         const float gb = live ? __ldg(dbasis + m * k_total + g * hl + j) : 0.0f;
-        grad[j] = gb * inv_pdf;
-        dpdf_m -= gb * a[s.L][j] * inv_pdf * inv_pdf;
+        const float a = my_units[(row + j) * stride];
+        grads[j * stride + threadIdx.x] = gb * inv_pdf * act_slope(a, act, alpha);
+        dpdf_m -= gb * a * inv_pdf * inv_pdf;
       }
-      for (int l = s.L; l >= 1; --l) {
-        const int hi = s.h[l - 1], ho = s.h[l];
-        const float* w = par + s.w_off[l - 1] + g * hi * ho;
-        float* dw = acc + s.w_off[l - 1] + g * hi * ho;
-        float* db = acc + s.b_off[l - 1] + g * ho;
-        for (int j = 0; j < ho; ++j) {
-          grad[j] *= act_bwd(pre[l - 1][j], act, alpha);      // now d(pre-activation)
-          const float t = warp_sum(grad[j]);
-          if (lane == 0) atomicAdd(db + j, t);
+      for (int l = s.L - 1; l >= 0; --l) {
+        const int hi = s.h[l], ho = s.h[l + 1], hp = s.hp[l + 1];
+        row -= hi;                                        // first row of the layer's inputs
+        const float* gl = grads + cur * s.widest * stride;
+        float* gp = grads + (cur ^ 1) * s.widest * stride;
+        __syncthreads();      // the tile's gradients of this layer are complete
+        // weights and biases: thread o owns the o-th value
+        for (int o = threadIdx.x; o < (hi + 1) * hp; o += tile) {
+          const int i = o / hp, j = o - i * hp;
+          if (j >= ho) continue;
+          const float4* gq = reinterpret_cast<const float4*>(gl + j * stride);
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (i < hi) {
+            const float4* aq = reinterpret_cast<const float4*>(units + (row + i) * stride);
+#pragma unroll 4
+            for (int p = 0; p < tile / 4; ++p) {
+              const float4 a = aq[p], b = gq[p];
+              sum.x = fmaf(a.x, b.x, sum.x); sum.y = fmaf(a.y, b.y, sum.y);
+              sum.z = fmaf(a.z, b.z, sum.z); sum.w = fmaf(a.w, b.w, sum.w);
+            }
+            acc[s.w_off[l] + (g * hi + i) * hp + j] += (sum.x + sum.y) + (sum.z + sum.w);
+          } else {
+#pragma unroll 4
+            for (int p = 0; p < tile / 4; ++p) {
+              const float4 b = gq[p];
+              sum.x += b.x; sum.y += b.y; sum.z += b.z; sum.w += b.w;
+            }
+            acc[s.b_off[l] + g * hp + j] += (sum.x + sum.y) + (sum.z + sum.w);
+          }
         }
+        // back to the layer's inputs
+        const float* w = par + s.w_off[l] + g * hi * hp;
         for (int i = 0; i < hi; ++i) {
           float back = 0.0f;
-          for (int j = 0; j < ho; ++j) {
-            const float t = warp_sum(a[l - 1][i] * grad[j]);
-            if (lane == 0) atomicAdd(dw + i * ho + j, t);
-            back = fmaf(grad[j], w[i * ho + j], back);
+          for (int j = 0; j < ho; j += 8) {
+            const float4 w0 = *reinterpret_cast<const float4*>(w + i * hp + j);
+            const float4 w1 = *reinterpret_cast<const float4*>(w + i * hp + j + 4);
+            const float* c = gl + j * stride + threadIdx.x;
+            const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (j + e < ho) back = fmaf(c[e * stride], wj[e], back);
           }
-          gprev[i] = back;
+          if (l > 0) {
+            gp[i * stride + threadIdx.x] = back * act_slope(my_units[(row + i) * stride], act, alpha);
+          } else {
+#pragma unroll
+            for (int d = 0; d < TFGPC_MAX_DIMS; ++d)
+              if (d == i) ddiff[d] += back;
+          }
         }
-        for (int i = 0; i < hi; ++i) grad[i] = gprev[i];
+        cur ^= 1;
       }
-      for (int d = 0; d < s.D; ++d) ddiff[d] += grad[d];
+      __syncthreads();        // before the next MLP or tile overwrites the activations
     }
-    if (live) {
-      if (dpdf) dpdf[m] = dpdf_m;
-      for (int d = 0; d < s.D; ++d) {
-        const float v = ddiff[d] * inv_radius;
-        if (dp_in) atomicAdd(dp_in + (int64_t)nb.x * s.D + d, v);
-        if (dp_out) atomicAdd(dp_out + (int64_t)nb.y * s.D + d, -v);
+    if (live && dpdf) dpdf[m] = dpdf_m;
+    if (dp_in || dp_out) {
+      // a sample's pairs follow one another: its first lane in the warp adds them up
+      const int lane = threadIdx.x & 31;
+      const int who = live ? nb.y : -1;
+      const int prev = __shfl_up_sync(0xffffffffu, who, 1);
+      const bool head = lane == 0 || prev != who;
+#pragma unroll
+      for (int d = 0; d < TFGPC_MAX_DIMS; ++d) {
+        if (d < s.D) {
+          float v = ddiff[d] * inv_radius;
+          if (live && dp_in) atomicAdd(dp_in + (int64_t)nb.x * s.D + d, v);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_down_sync(0xffffffffu, v, o);
+            const int id = __shfl_down_sync(0xffffffffu, who, o);
+            if (lane + o < 32 && id == who) v += y;
+          }
+          if (live && head && dp_out) atomicAdd(dp_out + (int64_t)nb.y * s.D + d, -v);
+        }
       }
     }
   }
   __syncthreads();
-  const int nw = s.b_off[0];
-  for (int i = threadIdx.x; i < s.params; i += kMlpThreads) {
-    if (i < nw) atomicAdd(dweights + i, acc[i]);
-    else atomicAdd(dbiases + i - nw, acc[i]);
+  int w_base = 0, b_base = 0;
+  for (int l = 0; l < s.L; ++l) {
+    const int ho = s.h[l + 1], hp = s.hp[l + 1], wr = s.G * s.h[l];
+    for (int i = threadIdx.x; i < wr * ho; i += tile) {
+      const int r = i / ho;
+      atomicAdd(dweights + w_base + i, acc[s.w_off[l] + r * hp + (i - r * ho)]);
+    }
+    for (int i = threadIdx.x; i < s.G * ho; i += tile) {
+      const int r = i / ho;
+      atomicAdd(dbiases + b_base + i, acc[s.b_off[l] + r * hp + (i - r * ho)]);
+    }
+    w_base += wr * ho;
+    b_base += s.G * ho;
   }
 }
 
-int make_shape(const char* op, int D, int G, int L, const int32_t* layer_sizes, MlpShape* out) {
+int make_shape(const char* op, int D, int G, int L, const int32_t* layer_sizes,
+               const float* const* weights, const float* const* biases, MlpShape* out,
+               int* num_weights, int* num_biases) {
   TFGPC_REQUIRE(valid_dims(D), "%s expects a valid number of dimension (got %d)", op, D);
   TFGPC_REQUIRE(G >= 1 && L >= 1 && L <= kMaxLayers && layer_sizes,
                 "%s expects 1 to %d hidden layers and at least one MLP", op, kMaxLayers);
-  MlpShape s;
-  s.D = D; s.G = G; s.L = L; s.h[0] = D;
-  int off = 0;
+  MlpShape s{};
+  s.D = D; s.G = G; s.L = L; s.h[0] = s.hp[0] = D;
+  s.rows = s.widest = D;
+  int off = 0, nw = 0, nb = 0;
   for (int l = 0; l < L; ++l) {
     TFGPC_REQUIRE(layer_sizes[l] >= 1 && layer_sizes[l] <= kMaxWidth,
                   "%s expects hidden layers of 1 to %d units", op, kMaxWidth);
     s.h[l + 1] = layer_sizes[l];
+    s.hp[l + 1] = (layer_sizes[l] + 7) / 8 * 8;
+    s.rows += layer_sizes[l];
+    if (layer_sizes[l] > s.widest) s.widest = layer_sizes[l];
     s.w_off[l] = off;
-    off += G * s.h[l] * s.h[l + 1];
+    off += G * s.h[l] * s.hp[l + 1];
+    nw += G * s.h[l] * s.h[l + 1];
+    nb += G * s.h[l + 1];
+    s.w[l] = weights ? weights[l] : nullptr;
+    s.b[l] = biases ? biases[l] : nullptr;
   }
   for (int l = 0; l < L; ++l) {
     s.b_off[l] = off;
-    off += G * s.h[l + 1];
+    off += G * s.hp[l + 1];
   }
-  for (int l = L + 1; l <= kMaxLayers; ++l) s.h[l] = 0;
-  for (int l = L; l < kMaxLayers; ++l) { s.w_off[l] = 0; s.b_off[l] = 0; }
   s.params = off;
-  TFGPC_REQUIRE(off <= kMaxParams, "%s: the kernel MLPs hold %d parameters, at most %d are supported",
-                op, off, kMaxParams);
+  TFGPC_REQUIRE(nw + nb <= kMaxParams, "%s: the kernel MLPs hold %d parameters, at most %d are supported",
+                op, nw + nb, kMaxParams);
   *out = s;
+  *num_weights = nw;
+  *num_biases = nb;
   return TFGPC_OK;
+}
+
+// Shared memory of a tile of `pairs` pairs.
+size_t mlp_smem(const MlpShape& s, int pairs, bool backward) {
+  const size_t f = backward ? 2 * (size_t)s.params + (size_t)(s.rows + 2 * s.widest) * (pairs + 4)
+                            : (size_t)s.params + (size_t)(s.D + 2 * s.widest) * pairs;
+  return f * sizeof(float);
+}
+
+// Pairs per tile: 128, fewer for MLPs so wide that they would not fit.
+int mlp_tile(const MlpShape& s, bool backward) {
+  int pairs = 128;
+  while (pairs > 32 && mlp_smem(s, pairs, backward) > kMaxMlpSmem) pairs /= 2;
+  return pairs;
+}
+
+// Per-layer pointers into flat parameter arrays.
+struct LayerPointers {
+  const float *w[kMaxLayers], *b[kMaxLayers];
+};
+LayerPointers layer_pointers(int D, int G, int L, const int32_t* sizes, const float* w,
+                             const float* b) {
+  LayerPointers p{};
+  int prev = D;
+  for (int l = 0; l < L && l < kMaxLayers && sizes; ++l) {
+    p.w[l] = w;
+    p.b[l] = b;
+    w += (int64_t)G * prev * sizes[l];
+    b += (int64_t)G * sizes[l];
+    prev = sizes[l];
+  }
+  return p;
 }
 
 }  // namespace
@@ -230,8 +388,22 @@ extern "C" int tfgpc_kernel_mlp_basis(void* stream, int D, int num_mlps, int num
                                       const float* weights, const float* biases, float inv_radius,
                                       int activation, float alpha, int pdf_by_neighbor,
                                       float* basis_out) {
+  TFGPC_REQUIRE(M == 0 || (weights && biases), "KernelMlpBasis got a null pointer");
+  const LayerPointers p = layer_pointers(D, num_mlps, num_layers, layer_sizes, weights, biases);
+  return tfgpc_kernel_mlp_basis_layers(stream, D, num_mlps, num_layers, layer_sizes, M, points_in,
+                                       points_out, neighbors, pdf, p.w, p.b, inv_radius, activation,
+                                       alpha, pdf_by_neighbor, basis_out);
+}
+
+extern "C" int tfgpc_kernel_mlp_basis_layers(
+    void* stream, int D, int num_mlps, int num_layers, const int32_t* layer_sizes, int64_t M,
+    const float* points_in, const float* points_out, const int32_t* neighbors, const float* pdf,
+    const float* const* weights, const float* const* biases, float inv_radius, int activation,
+    float alpha, int pdf_by_neighbor, float* basis_out) {
   MlpShape s;
-  int rc = make_shape("KernelMlpBasis", D, num_mlps, num_layers, layer_sizes, &s);
+  int nw, nb;
+  int rc = make_shape("KernelMlpBasis", D, num_mlps, num_layers, layer_sizes, weights, biases, &s,
+                      &nw, &nb);
   if (rc) return rc;
   TFGPC_REQUIRE(M >= 0 && M <= (int64_t)INT32_MAX, "KernelMlpBasis expects 0 <= M < 2^31");
   TFGPC_REQUIRE(activation == 0 || activation == 1,
@@ -239,12 +411,17 @@ extern "C" int tfgpc_kernel_mlp_basis(void* stream, int D, int num_mlps, int num
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_out,
                 "KernelMlpBasis got a null pointer");
+  TFGPC_REQUIRE((uintptr_t)basis_out % 16 == 0, "KernelMlpBasis expects a 16-byte aligned output");
   cudaStream_t st = (cudaStream_t)stream;
-  unsigned grid = min(blocks_for(M, kMlpThreads), (unsigned)(sm_count() * 16));
+  const int tile = mlp_tile(s, false);
+  const size_t smem = mlp_smem(s, tile, false);
+  TFGPC_CUDA(cudaFuncSetAttribute(kernel_mlp_basis_kernel,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  unsigned grid = min(blocks_for(M, tile), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "kernel_mlp_basis");
-  kernel_mlp_basis_kernel<<<grid, kMlpThreads, sizeof(float) * (size_t)s.params, st>>>(
-      s, M, points_in, points_out, (const int2*)neighbors, pdf, weights, biases, inv_radius,
-      activation, alpha, pdf_by_neighbor, basis_out);
+  kernel_mlp_basis_kernel<<<grid, tile, smem, st>>>(s, M, points_in, points_out,
+                                                    (const int2*)neighbors, pdf, inv_radius,
+                                                    activation, alpha, pdf_by_neighbor, basis_out);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -259,8 +436,26 @@ extern "C" int tfgpc_kernel_mlp_grads(void* stream, int D, int num_mlps, int num
                                       float* dbiases_out,
                                       float* dpoints_in_out, float* dpoints_out_out,
                                       float* dpdf_out) {
+  TFGPC_REQUIRE(M == 0 || (weights && biases), "KernelMlpGrads got a null pointer");
+  const LayerPointers p = layer_pointers(D, num_mlps, num_layers, layer_sizes, weights, biases);
+  return tfgpc_kernel_mlp_grads_layers(stream, D, num_mlps, num_layers, layer_sizes, M, n_in, ns,
+                                       points_in, points_out, neighbors, pdf, p.w, p.b, inv_radius,
+                                       activation, alpha, pdf_by_neighbor, basis_grads,
+                                       dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out,
+                                       dpdf_out);
+}
+
+extern "C" int tfgpc_kernel_mlp_grads_layers(
+    void* stream, int D, int num_mlps, int num_layers, const int32_t* layer_sizes, int64_t M,
+    int64_t n_in, int64_t ns, const float* points_in, const float* points_out,
+    const int32_t* neighbors, const float* pdf, const float* const* weights,
+    const float* const* biases, float inv_radius, int activation, float alpha,
+    int pdf_by_neighbor, const float* basis_grads, float* dweights_out, float* dbiases_out,
+    float* dpoints_in_out, float* dpoints_out_out, float* dpdf_out) {
   MlpShape s;
-  int rc = make_shape("KernelMlpGrads", D, num_mlps, num_layers, layer_sizes, &s);
+  int nw, nb;
+  int rc = make_shape("KernelMlpGrads", D, num_mlps, num_layers, layer_sizes, weights, biases, &s,
+                      &nw, &nb);
   if (rc) return rc;
   TFGPC_REQUIRE(M >= 0 && M <= (int64_t)INT32_MAX && n_in >= 0 && ns >= 0,
                 "KernelMlpGrads expects 0 <= M < 2^31 and non-negative point counts");
@@ -268,9 +463,8 @@ extern "C" int tfgpc_kernel_mlp_grads(void* stream, int D, int num_mlps, int num
                 "KernelMlpGrads expects activation 0 (leaky ReLU) or 1 (ELU)");
   TFGPC_REQUIRE(dweights_out && dbiases_out, "KernelMlpGrads got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  const int nw = s.b_off[0];
   TFGPC_CUDA(cudaMemsetAsync(dweights_out, 0, sizeof(float) * (size_t)nw, st));
-  TFGPC_CUDA(cudaMemsetAsync(dbiases_out, 0, sizeof(float) * (size_t)(s.params - nw), st));
+  TFGPC_CUDA(cudaMemsetAsync(dbiases_out, 0, sizeof(float) * (size_t)nb, st));
   // points_in and points_out may be one cloud: its gradient is then one array
   // that both roles add into
   if (dpoints_in_out)
@@ -280,15 +474,16 @@ extern "C" int tfgpc_kernel_mlp_grads(void* stream, int D, int num_mlps, int num
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_grads,
                 "KernelMlpGrads got a null pointer");
-  const size_t smem = sizeof(float) * 2 * (size_t)s.params;
+  const int tile = mlp_tile(s, true);
+  const size_t smem = mlp_smem(s, tile, true);
   TFGPC_CUDA(cudaFuncSetAttribute(kernel_mlp_grads_kernel,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  unsigned grid = min(blocks_for(M, kMlpThreads), (unsigned)(sm_count() * 8));
+  unsigned grid = min(blocks_for(M, tile), (unsigned)(sm_count() * 8));
   ProfScope prof(st, "kernel_mlp_grads");
-  kernel_mlp_grads_kernel<<<grid, kMlpThreads, smem, st>>>(
-      s, M, points_in, points_out, (const int2*)neighbors, pdf, weights, biases, inv_radius,
-      activation, alpha, pdf_by_neighbor, basis_grads, dweights_out, dbiases_out, dpoints_in_out,
-      dpoints_out_out, dpdf_out);
+  kernel_mlp_grads_kernel<<<grid, tile, smem, st>>>(
+      s, M, points_in, points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha,
+      pdf_by_neighbor, basis_grads, dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out,
+      dpdf_out);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }

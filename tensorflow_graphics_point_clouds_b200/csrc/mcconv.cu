@@ -15,16 +15,20 @@ namespace tfgpc {
 
 int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                      const float* feat, const int32_t* neigh, const int32_t* ranges,
-                     __nv_bfloat16* hi, __nv_bfloat16* mid);
+                     __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
+int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, int64_t M,
+                            const float* basis, const float* feat, const int32_t* neigh,
+                            const int32_t* ranges, const float* in_grads, float* dbasis,
+                            float* dfeat, int hidden);
 // basis_proj_mma.cu: the projection on warp-level tensor-core MMAs
 bool basis_proj_mma_supported(int K, int C);
 int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bfloat16* fs);
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
-                         __nv_bfloat16* hi, __nv_bfloat16* mid);
+                         __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
-                         const float* in_grads, float* dbasis, float* dfeat);
+                         const float* in_grads, float* dbasis, float* dfeat, int hidden);
 
 // basis_proj_grads_tc.cu: the gradients on tcgen05 tensor cores
 bool basis_proj_grads_tc_supported(int K, int C);
@@ -54,7 +58,7 @@ struct McWs {
   float* dx;                        // [ns, C*K]    (backward)
   __nv_bfloat16* fs;                // [n_in, 2, C] split features (tensor-core projection)
   __nv_bfloat16 *wt_hi, *wt_mid;    // [Cout, C*K]: W transposed (backward)
-  int dw_splits;
+  float* dw_pad;                    // [C*K, Cout]: gradient of padded weights (backward)
   size_t bytes;
 };
 
@@ -72,8 +76,7 @@ McWs carve(void* ws, int K, int C, int Cout, int64_t ns, int64_t n_in, bool back
   // of the same workspace agree on where it lies
   w.fs = nullptr;
   if (basis_proj_mma_supported(K, C)) w.fs = (__nv_bfloat16*)take((size_t)n_in * C * 4);
-  w.dw_splits = 1;
-  w.g_hi = w.g_mid = nullptr; w.dx = nullptr; w.wt_hi = w.wt_mid = nullptr;
+  w.g_hi = w.g_mid = nullptr; w.dx = nullptr; w.wt_hi = w.wt_mid = nullptr; w.dw_pad = nullptr;
   if (backward) {
     w.g_hi = (__nv_bfloat16*)take((size_t)ns * Cout * 2);
     w.g_mid = (__nv_bfloat16*)take((size_t)ns * Cout * 2);
@@ -82,7 +85,7 @@ McWs carve(void* ws, int K, int C, int Cout, int64_t ns, int64_t n_in, bool back
     w.dx = (float*)take((size_t)((ns + 2) / 3) * 4 * ck * 4);
     w.wt_hi = (__nv_bfloat16*)take(ck * Cout * 2);
     w.wt_mid = (__nv_bfloat16*)take(ck * Cout * 2);
-    w.dw_splits = gemm_pick_k_splits((int64_t)ck, Cout, ns);
+    w.dw_pad = (float*)take(ck * Cout * 4);
   }
   w.bytes = (size_t)(p - (char*)ws);
   return w;
@@ -99,10 +102,61 @@ int check_mc_args(const char* op, int K, int C, int Cout, int64_t ns, int64_t n_
   return TFGPC_OK;
 }
 
+// How the weights lie in memory.  groups > 1: `groups` kernel MLPs with K / groups
+// outputs each, whose blocks [C * K/groups, Cout/groups] lie one after the other: the
+// products run block by block (a dense matrix would be zero but for its diagonal
+// blocks), X and dX with their columns in the order (group, channel, output).
+// groups == 1: [C * k_src, cout_src], zero-padded to K basis functions and Cout columns.
+struct Blocks {
+  int groups, k_src, cout_src;
+};
+
+// out[(c * k_src + k), o] = padded[(c * k_dst + k), o]
+__global__ void crop_weights_kernel(int64_t n, int cols, int ld, int k_src, int k_dst,
+                                    const float* __restrict__ padded, float* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t r = i / cols, c = r / k_src;
+  out[i] = __ldg(padded + (c * k_dst + (r - c * k_src)) * ld + (i - r * cols));
+}
+
+int check_blocks(const char* op, int K, int C, int Cout, const Blocks& b) {
+  TFGPC_REQUIRE(b.groups >= 1 && K % b.groups == 0 && Cout % b.groups == 0 &&
+                b.k_src >= 1 && b.k_src <= K && b.cout_src >= 1 && b.cout_src <= Cout &&
+                (b.groups == 1 || (b.k_src == K && b.cout_src == Cout &&
+                                   tfgpc_mcconv_blocks_supported(K, C, Cout, b.groups))),
+                "%s: weight blocks of this shape are not supported", op);
+  return TFGPC_OK;
+}
+
+SplitJob weight_job(const McWs& w, const float* weights, int64_t ck, int K, int Cout,
+                    const Blocks& b) {
+  SplitJob j;
+  j.x = weights;
+  j.rows = ck;
+  j.ld = Cout / b.groups;
+  j.cols = b.groups > 1 ? j.ld : b.cout_src;
+  j.k_src = b.k_src;
+  j.k_dst = K;
+  j.hi = w.w_hi;
+  j.mid = w.w_mid;
+  return j;
+}
+
 }  // namespace
 }  // namespace tfgpc
 
 using namespace tfgpc;
+
+// Block-diagonal products need 16-byte aligned block columns, and the projection hands
+// over four basis functions of one block at a time.
+extern "C" int tfgpc_mcconv_blocks_supported(int K, int C, int Cout, int groups) {
+  if (K <= 0 || C <= 0 || Cout <= 0 || groups < 1) return 0;
+  if (groups == 1) return 1;
+  if (K % groups || Cout % groups) return 0;
+  const int h = K / groups, co = Cout / groups;
+  return h % 4 == 0 && ((int64_t)C * h) % 8 == 0 && co % 8 == 0;
+}
 
 extern "C" size_t tfgpc_mcconv_workspace_bytes(int K, int C, int Cout, int64_t ns, int64_t n_in,
                                                int backward) {
@@ -114,20 +168,34 @@ extern "C" size_t tfgpc_mcconv_workspace_bytes(int K, int C, int Cout, int64_t n
 // where the shape allows it, else on the SIMT kernels.
 static int project(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, const float* basis,
                    const float* features, const int32_t* neighbors, const int32_t* ranges,
-                   const McWs& w) {
+                   const McWs& w, int hidden) {
   if (w.fs && (uintptr_t)features % 16 == 0) {
     int rc = split_features(st, features, n_in, C, w.fs);
     if (rc) return rc;
-    return basis_proj_mma_split(st, K, C, ns, basis, w.fs, neighbors, ranges, w.x_hi, w.x_mid);
+    return basis_proj_mma_split(st, K, C, ns, basis, w.fs, neighbors, ranges, w.x_hi, w.x_mid,
+                                hidden);
   }
-  return basis_proj_split(st, K, C, ns, basis, features, neighbors, ranges, w.x_hi, w.x_mid);
+  return basis_proj_split(st, K, C, ns, basis, features, neighbors, ranges, w.x_hi, w.x_mid, hidden);
 }
 
 extern "C" int tfgpc_mcconv_forward(void* stream, int K, int C, int Cout, int64_t ns, int64_t n_in,
                                     int64_t M, const float* basis, const float* features,
                                     const int32_t* neighbors, const int32_t* ranges,
                                     const float* weights, float* out, void* ws, size_t ws_bytes) {
+  return tfgpc_mcconv_forward_blocks(stream, K, C, Cout, 1, K, Cout, ns, n_in, M, basis, features,
+                                     neighbors, ranges, weights, out, ws, ws_bytes);
+}
+
+extern "C" int tfgpc_mcconv_forward_blocks(void* stream, int K, int C, int Cout, int groups,
+                                           int k_src, int cout_src, int64_t ns, int64_t n_in,
+                                           int64_t M, const float* basis, const float* features,
+                                           const int32_t* neighbors, const int32_t* ranges,
+                                           const float* weights, float* out, void* ws,
+                                           size_t ws_bytes) {
   int rc = check_mc_args("MCConvForward", K, C, Cout, ns, n_in, M);
+  if (rc) return rc;
+  const Blocks blocks{groups, k_src, cout_src};
+  rc = check_blocks("MCConvForward", K, C, Cout, blocks);
   if (rc) return rc;
   if (ns == 0) return TFGPC_OK;
   TFGPC_REQUIRE(ranges && weights && out && ws && (M == 0 || (basis && features && neighbors)),
@@ -139,19 +207,29 @@ extern "C" int tfgpc_mcconv_forward(void* stream, int K, int C, int Cout, int64_
                 tfgpc_mcconv_workspace_bytes(K, C, Cout, ns, n_in, 0));
   cudaStream_t st = (cudaStream_t)stream;
   McWs w = carve(ws, K, C, Cout, ns, n_in, false);
-  const int64_t ck = (int64_t)C * K;
+  const int64_t ck = (int64_t)C * K, ch = ck / groups, co = Cout / groups;
   TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-  rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w);
+  rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w, K / groups);
   if (rc) return rc;
-  rc = split_to_bf16(st, weights, ck * Cout, w.w_hi, w.w_mid);
+  rc = split_rows(st, weight_job(w, weights, ck, K, Cout, blocks));
   if (rc) return rc;
-  GemmOperand a{w.x_hi, w.x_mid, ck, Major::K};
-  GemmOperand b{w.w_hi, w.w_mid, (int64_t)Cout, Major::MN};  // W is [C*K, Cout]: N contiguous
+  GemmProblem p{};
+  const GemmOperand x{w.x_hi, w.x_mid, ck, Major::K, ch};
+  const GemmOperand wt{w.w_hi, w.w_mid, co, Major::MN, ch * co};  // [C*K, Cout]: N contiguous
+  p.K = ch;
+  p.c = out;
+  p.ldc = Cout;
+  p.batches = groups;
+  p.c_batch_stride = co;
   // With at least one full tile of output features the roles are swapped,
   // out^T = W^T * X^T with W as the (MN-major) left operand, and the tiles are
   // transposed on their way out.
-  if (Cout >= 128) return gemm_bf16x3_tn(st, Cout, ns, ck, b, a, out, Cout, w.err);
-  return gemm_bf16x3(st, ns, Cout, ck, a, b, out, Cout, 1, 0, w.err);
+  p.transposed = co >= 128;
+  p.M = p.transposed ? co : ns;
+  p.N = p.transposed ? ns : co;
+  p.a = p.transposed ? wt : x;
+  p.b = p.transposed ? x : wt;
+  return gemm_bf16x3(st, p, w.err);
 }
 
 extern "C" int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64_t ns,
@@ -161,13 +239,28 @@ extern "C" int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64
                                      const float* out_grads, int x_in_workspace, float* dbasis_out,
                                      float* dfeat_out, float* dweights_out, void* ws,
                                      size_t ws_bytes) {
+  return tfgpc_mcconv_backward_blocks(stream, K, C, Cout, 1, K, Cout, ns, n_in, M, basis, features,
+                                      neighbors, ranges, weights, out_grads, x_in_workspace,
+                                      dbasis_out, dfeat_out, dweights_out, ws, ws_bytes);
+}
+
+extern "C" int tfgpc_mcconv_backward_blocks(
+    void* stream, int K, int C, int Cout, int groups, int k_src, int cout_src, int64_t ns,
+    int64_t n_in, int64_t M, const float* basis, const float* features, const int32_t* neighbors,
+    const int32_t* ranges, const float* weights, const float* out_grads, int x_in_workspace,
+    float* dbasis_out, float* dfeat_out, float* dweights_out, void* ws, size_t ws_bytes) {
   int rc = check_mc_args("MCConvBackward", K, C, Cout, ns, n_in, M);
   if (rc) return rc;
+  const Blocks blocks{groups, k_src, cout_src};
+  rc = check_blocks("MCConvBackward", K, C, Cout, blocks);
+  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t ck = (int64_t)C * K;
+  const int64_t ck = (int64_t)C * K, ch = ck / groups, co = Cout / groups;
+  const bool padded = k_src != K || cout_src != Cout;
+  const int64_t weight_elems = groups > 1 ? ck * co : (int64_t)C * k_src * cout_src;
   TFGPC_REQUIRE(dweights_out && weights, "MCConvBackward got a null pointer");
   if (ns == 0 || M == 0) {
-    TFGPC_CUDA(cudaMemsetAsync(dweights_out, 0, sizeof(float) * (size_t)ck * Cout, st));
+    TFGPC_CUDA(cudaMemsetAsync(dweights_out, 0, sizeof(float) * (size_t)weight_elems, st));
     if (M > 0 && dbasis_out) TFGPC_CUDA(cudaMemsetAsync(dbasis_out, 0, sizeof(float) * (size_t)M * K, st));
     if (n_in > 0 && dfeat_out) TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
     return TFGPC_OK;
@@ -181,25 +274,31 @@ extern "C" int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64
     return fail(TFGPC_ENOMEM, "MCConvBackward workspace too small: %zu < %zu", ws_bytes,
                 tfgpc_mcconv_workspace_bytes(K, C, Cout, ns, n_in, 1));
   McWs w = carve(ws, K, C, Cout, ns, n_in, true);
+  const int hidden = K / groups;
   if (!x_in_workspace) {
     // (with x_in_workspace the word keeps what the forward call left: a timeout
     // there means that the projection this call is about to read is incomplete)
     TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-    rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w);
+    rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w, hidden);
     if (rc) return rc;
   }
-  // The weights are split again on every call (2 MB): every branch below then
-  // works on the values of this call's `weights`, whatever the forward call saw.
-  rc = split_to_bf16(st, weights, ck * Cout, w.w_hi, w.w_mid);
-  if (rc) return rc;
-  rc = split_to_bf16(st, out_grads, ns * Cout, w.g_hi, w.g_mid);
-  if (rc) return rc;
-  // dX[ns, C*K] = dOut[ns, Cout] * W^T: B rows are W's rows, reduction over Cout
-  GemmOperand g_k{w.g_hi, w.g_mid, (int64_t)Cout, Major::K};
-  GemmOperand w_k{w.w_hi, w.w_mid, (int64_t)Cout, Major::K};
   const bool fs_ok = w.fs && (uintptr_t)features % 16 == 0 && (uintptr_t)dbasis_out % 32 == 0 &&
                      (uintptr_t)dfeat_out % 16 == 0;
-  if (fs_ok && basis_proj_grads_tc_supported(K, C)) {
+  const bool image = fs_ok && groups == 1 && basis_proj_grads_tc_supported(K, C);
+  SplitJob gj;
+  gj.x = out_grads;
+  gj.rows = ns;
+  gj.cols = cout_src;
+  gj.ld = Cout;
+  gj.hi = w.g_hi;
+  gj.mid = w.g_mid;
+  // The weights are split again on every call (2 MB): the products below then work on
+  // the values of this call's `weights`, whatever the forward call saw.
+  const SplitJob wj = weight_job(w, weights, ck, K, Cout, blocks);
+  rc = split_rows(st, gj, image ? nullptr : &wj);
+  if (rc) return rc;
+  TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
+  if (image) {
     // dX goes straight into the operand image of the tcgen05 gradient kernel
     const int group = basis_proj_grads_tc_group(ns, M);
     if (ns % group != 0) {
@@ -210,34 +309,54 @@ extern "C" int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64
     // dX^T = W * dOut^T with W^T [Cout, C*K] as the MN-major left operand (the
     // tensor pipe reads it faster than a K-major one; transposing 2 MB is free),
     // tiles transposed back on their way into the image
-    rc = split_transpose_to_bf16(st, weights, ck, Cout, w.wt_hi, w.wt_mid);
+    rc = split_transpose_to_bf16(st, weights, ck, Cout, cout_src, k_src, K, w.wt_hi, w.wt_mid);
     if (rc) return rc;
-    GemmOperand wt_mn{w.wt_hi, w.wt_mid, ck, Major::MN};
+    const GemmOperand wt_mn{w.wt_hi, w.wt_mid, ck, Major::MN};
+    const GemmOperand g_k{w.g_hi, w.g_mid, (int64_t)Cout, Major::K};
     rc = gemm_bf16x3_grad_image_tn(st, C, ns, Cout, wt_mn, g_k, w.dx, group, w.err);
     if (rc) return rc;
-    TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
     rc = basis_proj_grads_tc(st, group, ns, M, basis, w.fs, neighbors, ranges, w.dx, dbasis_out,
                              dfeat_out, w.err);
   } else {
-    rc = gemm_bf16x3(st, ns, ck, Cout, g_k, w_k, w.dx, ck, 1, 0, w.err);
+    // dX[ns, C*K] = dOut[ns, Cout] * W^T: B rows are W's rows, reduction over Cout
+    GemmProblem p{};
+    p.M = ns;
+    p.N = ch;
+    p.K = co;
+    p.a = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::K, co};
+    p.b = GemmOperand{w.w_hi, w.w_mid, co, Major::K, ch * co};
+    p.c = w.dx;
+    p.ldc = ck;
+    p.batches = groups;
+    p.c_batch_stride = ch;
+    rc = gemm_bf16x3(st, p, w.err);
     if (rc) return rc;
-    if (fs_ok) {
-      TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
+    if (fs_ok)
       rc = basis_proj_grads_mma(st, K, C, ns, M, basis, w.fs, neighbors, ranges, w.dx, dbasis_out,
-                                dfeat_out);
-    } else {
-      rc = tfgpc_basis_proj_grads(stream, K, C, ns, n_in, M, basis, features, neighbors, ranges,
-                                  w.dx, dbasis_out, dfeat_out);
-    }
+                                dfeat_out, hidden);
+    else
+      rc = basis_proj_grads_blocks(st, K, C, ns, n_in, M, basis, features, neighbors, ranges, w.dx,
+                                   dbasis_out, dfeat_out, hidden);
   }
   if (rc) return rc;
   // dW[C*K, Cout] = X^T * dOut: both operands have the reduction (sample) index
   // as their row index, i.e. they are MN-major
-  GemmOperand x_mn{w.x_hi, w.x_mid, ck, Major::MN};
-  GemmOperand g_mn{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN};
-  // the reduction over the samples is cut into slices (see gemm_pick_k_splits)
-  // that the GEMM adds into dweights_out
-  return gemm_bf16x3(st, ck, Cout, ns, x_mn, g_mn, dweights_out, Cout, w.dw_splits, 0, w.err);
+  GemmProblem p{};
+  p.M = ch;
+  p.N = co;
+  p.K = ns;
+  p.a = GemmOperand{w.x_hi, w.x_mid, ck, Major::MN, ch};
+  p.b = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN, co};
+  p.c = padded ? w.dw_pad : dweights_out;
+  p.ldc = co;
+  p.batches = groups;
+  p.c_batch_stride = ch * co;
+  rc = gemm_bf16x3(st, p, w.err);
+  if (rc || !padded) return rc;
+  crop_weights_kernel<<<blocks_for(weight_elems, 256), 256, 0, st>>>(weight_elems, cout_src, Cout,
+                                                                     k_src, K, w.dw_pad, dweights_out);
+  TFGPC_LAUNCH_CHECK();
+  return TFGPC_OK;
 }
 
 extern "C" int tfgpc_mcconv_grouped_supported(int K, int C) {
@@ -294,7 +413,7 @@ extern "C" int tfgpc_mcconv_forward_grouped(
   TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
   rc = project_grouped(st, C, ns, n_in, M, basis_pair, features, plan, w);
   if (rc) return rc;
-  rc = split_to_bf16(st, weights, ck * Cout, w.w_hi, w.w_mid);
+  rc = split_rows(st, weight_job(w, weights, ck, K, Cout, Blocks{1, K, Cout}));
   if (rc) return rc;
   GemmOperand a{w.x_hi, w.x_mid, ck, Major::K};
   GemmOperand b{w.w_hi, w.w_mid, (int64_t)Cout, Major::MN};
@@ -341,14 +460,21 @@ extern "C" int tfgpc_mcconv_backward_grouped(
   // X lies in the visiting order (tfgpc_mcconv_forward_grouped wrote it so): the
   // rows of out_grads are brought into the same order while they are split, for
   // both products
-  rc = split_rows_gather_to_bf16(st, out_grads, order, ns, Cout, w.g_hi, w.g_mid);
+  SplitJob gj;
+  gj.x = out_grads;
+  gj.rows = ns;
+  gj.cols = gj.ld = Cout;
+  gj.order = order;
+  gj.hi = w.g_hi;
+  gj.mid = w.g_mid;
+  rc = split_rows(st, gj);
   if (rc) return rc;
   constexpr int group = 4;
   if (ns % group != 0) {
     char* last = (char*)w.dx + (size_t)(ns / group) * 4 * ck * 4;
     TFGPC_CUDA(cudaMemsetAsync(last, 0, (size_t)4 * ck * 4, st));
   }
-  rc = split_transpose_to_bf16(st, weights, ck, Cout, w.wt_hi, w.wt_mid);
+  rc = split_transpose_to_bf16(st, weights, ck, Cout, Cout, K, K, w.wt_hi, w.wt_mid);
   if (rc) return rc;
   GemmOperand wt_mn{w.wt_hi, w.wt_mid, ck, Major::MN};
   GemmOperand gv_k{w.g_hi, w.g_mid, (int64_t)Cout, Major::K};
@@ -358,9 +484,15 @@ extern "C" int tfgpc_mcconv_backward_grouped(
   rc = basis_proj_grads_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, ranges, w.dx,
                             dbasis_out, dfeat_out, w.err);
   if (rc) return rc;
-  GemmOperand x_mn{w.x_hi, w.x_mid, ck, Major::MN};
-  GemmOperand g_mn{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN};
-  return gemm_bf16x3(st, ck, Cout, ns, x_mn, g_mn, dweights_out, Cout, w.dw_splits, 0, w.err);
+  GemmProblem p{};
+  p.M = ck;
+  p.N = Cout;
+  p.K = ns;
+  p.a = GemmOperand{w.x_hi, w.x_mid, ck, Major::MN};
+  p.b = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN};
+  p.c = dweights_out;
+  p.ldc = Cout;
+  return gemm_bf16x3(st, p, w.err);
 }
 
 extern "C" int tfgpc_mcconv_status(void* stream, const void* ws, int* status_out) {
@@ -400,14 +532,88 @@ extern "C" int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K, c
   __nv_bfloat16* b_hi = (__nv_bfloat16*)p; p += align_up((size_t)N * K * 2, 1024);
   __nv_bfloat16* b_mid = (__nv_bfloat16*)p; p += align_up((size_t)N * K * 2, 1024);
   TFGPC_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
-  int rc = split_to_bf16(st, a, M * K, a_hi, a_mid);
-  if (rc) return rc;
-  rc = split_to_bf16(st, b, N * K, b_hi, b_mid);
+  SplitJob ja, jb;
+  ja.x = a;
+  ja.rows = a_transposed ? K : M;
+  ja.cols = ja.ld = (int)(a_transposed ? M : K);
+  ja.hi = a_hi;
+  ja.mid = a_mid;
+  jb.x = b;
+  jb.rows = b_transposed ? N : K;
+  jb.cols = jb.ld = (int)(b_transposed ? K : N);
+  jb.hi = b_hi;
+  jb.mid = b_mid;
+  int rc = split_rows(st, ja, &jb);
   if (rc) return rc;
   // a is [M,K] (K-major) or, transposed, [K,M] (MN-major); b is [K,N] (MN-major)
   // or, transposed, [N,K] (K-major)
-  GemmOperand ao{a_hi, a_mid, a_transposed ? M : K, a_transposed ? Major::MN : Major::K};
-  GemmOperand bo{b_hi, b_mid, b_transposed ? K : N, b_transposed ? Major::K : Major::MN};
-  // several slices of the reduction are added into c by the GEMM itself
-  return gemm_bf16x3(st, M, N, K, ao, bo, c, N, gemm_pick_k_splits(M, N, K), 0, err);
+  GemmProblem g{};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.a = GemmOperand{a_hi, a_mid, a_transposed ? M : K, a_transposed ? Major::MN : Major::K};
+  g.b = GemmOperand{b_hi, b_mid, b_transposed ? K : N, b_transposed ? Major::K : Major::MN};
+  g.c = c;
+  g.ldc = N;
+  return gemm_bf16x3(st, g, err);
+}
+
+// ---- Conv1x1 ------------------------------------------------------------------------
+
+namespace {
+inline int64_t up8(int64_t v) { return (v + 7) / 8 * 8; }
+}  // namespace
+
+extern "C" size_t tfgpc_linear_workspace_bytes(int64_t n, int64_t cin, int64_t cout) {
+  if (n <= 0 || cin <= 0 || cout <= 0) return 1024;
+  return 1024 + 2 * align_up((size_t)n * up8(cin) * 2, 1024) +
+         2 * align_up((size_t)cin * up8(cout) * 2, 1024);
+}
+
+extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t cout, const float* x,
+                                const float* weights, const float* bias, float* out, void* ws,
+                                size_t ws_bytes) {
+  TFGPC_REQUIRE(n >= 0 && cin > 0 && cout > 0 && cin < (1 << 30) && cout < (1 << 30),
+                "Conv1x1 expects positive sizes");
+  int rc = take_deferred_error();
+  if (rc) return rc;
+  if (n == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(x && weights && out && ws, "Conv1x1 got a null pointer");
+  TFGPC_REQUIRE((uintptr_t)ws % 256 == 0 && (uintptr_t)out % 16 == 0,
+                "Conv1x1 expects a 256-byte aligned workspace and a 16-byte aligned output");
+  if (ws_bytes < tfgpc_linear_workspace_bytes(n, cin, cout))
+    return fail(TFGPC_ENOMEM, "Conv1x1 workspace too small");
+  int* err = nullptr;
+  rc = deferred_error_word(&err);
+  if (rc) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  char* p = (char*)ws + 1024;
+  auto take = [&](size_t b) { char* r = p; p += align_up(b, 1024); return (__nv_bfloat16*)r; };
+  SplitJob jx, jw;
+  jx.x = x;
+  jx.rows = n;
+  jx.cols = (int)cin;
+  jx.ld = (int)up8(cin);
+  jx.hi = take((size_t)n * jx.ld * 2);
+  jx.mid = take((size_t)n * jx.ld * 2);
+  jw.x = weights;
+  jw.rows = cin;
+  jw.cols = (int)cout;
+  jw.ld = (int)up8(cout);
+  jw.hi = take((size_t)cin * jw.ld * 2);
+  jw.mid = take((size_t)cin * jw.ld * 2);
+  rc = split_rows(st, jx, &jw);
+  if (rc) return rc;
+  const GemmOperand xo{jx.hi, jx.mid, jx.ld, Major::K}, wo{jw.hi, jw.mid, jw.ld, Major::MN};
+  GemmProblem g{};
+  g.K = cin;
+  g.transposed = cout >= 128;    // (see gemm_bf16x3)
+  g.M = g.transposed ? cout : n;
+  g.N = g.transposed ? n : cout;
+  g.a = g.transposed ? wo : xo;
+  g.b = g.transposed ? xo : wo;
+  g.c = out;
+  g.ldc = up8(cout);
+  g.bias = bias;
+  return gemm_bf16x3(st, g, err);
 }

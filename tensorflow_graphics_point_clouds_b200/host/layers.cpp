@@ -62,6 +62,85 @@ py::tuple kernel_basis_grads(const Tensor& p_in_, const Tensor& p_out_, const Te
   return py::make_tuple(both.narrow(0, 0, d), both.select(0, d));
 }
 
+// Parameters of a kernel MLP, one tensor per layer: weights [G, H_{l-1}, H_l], biases
+// [G, 1, H_l].
+struct Mlp {
+  std::vector<Tensor> w, b;
+  std::vector<const float*> wp, bp;
+  std::vector<int32_t> sizes;
+  int d, g;
+  Mlp(const std::vector<Tensor>& weights, const std::vector<Tensor>& biases) {
+    require(!weights.empty() && weights.size() == biases.size(),
+            "KernelMlp expects one bias per layer");
+    for (size_t l = 0; l < weights.size(); ++l) {
+      w.push_back(f32(weights[l]));
+      b.push_back(f32(biases[l]));
+      wp.push_back(fp(w[l]));
+      bp.push_back(fp(b[l]));
+      sizes.push_back((int32_t)w[l].size(2));
+    }
+    g = (int)w[0].size(0);
+    d = (int)w[0].size(1);
+  }
+  int layers() const { return (int)sizes.size(); }
+};
+
+Tensor kernel_mlp_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
+                        const Tensor& pdf_, const std::vector<Tensor>& weights,
+                        const std::vector<Tensor>& biases, double radius, int act, double alpha,
+                        bool pdf_by_nbr) {
+  Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), pdf = f32(pdf_);
+  Mlp mlp(weights, biases);
+  const int64_t m = neigh.size(0);
+  Tensor basis = empty({m, (int64_t)mlp.g * mlp.sizes.back()}, at::kFloat, p_in);
+  check(tfgpc_kernel_mlp_basis_layers(stream(), mlp.d, mlp.g, mlp.layers(), mlp.sizes.data(), m,
+                                      fp(p_in), fp(p_out), ip(neigh), fp(pdf), mlp.wp.data(),
+                                      mlp.bp.data(), (float)(1.0 / radius), act, (float)alpha,
+                                      pdf_by_nbr, fpm(basis)));
+  return basis;
+}
+
+// (d_weights, d_biases[, d_points_in, d_points_out, d_pdf])
+py::tuple kernel_mlp_grads(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
+                           const Tensor& pdf_, const std::vector<Tensor>& weights,
+                           const std::vector<Tensor>& biases, double radius,
+                           const Tensor& dbasis_, int act, double alpha, bool point_grads,
+                           bool pdf_by_nbr) {
+  Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), pdf = f32(pdf_),
+         dbasis = f32(dbasis_);
+  Mlp mlp(weights, biases);
+  int64_t nw = 0, nb = 0;
+  for (int l = 0; l < mlp.layers(); ++l) {
+    nw += mlp.w[l].numel();
+    nb += mlp.b[l].numel();
+  }
+  Tensor flat = empty({nw + nb}, at::kFloat, p_in);
+  const int64_t m = neigh.size(0);
+  OptTensor dpin, dpout, dpdf;
+  if (point_grads) {
+    dpin = at::empty_like(p_in);
+    dpout = p_out.data_ptr() == p_in.data_ptr() ? *dpin : at::empty_like(p_out);
+    dpdf = empty({m}, at::kFloat, pdf);
+  }
+  check(tfgpc_kernel_mlp_grads_layers(
+      stream(), mlp.d, mlp.g, mlp.layers(), mlp.sizes.data(), m, p_in.size(0), p_out.size(0),
+      fp(p_in), fp(p_out), ip(neigh), fp(pdf), mlp.wp.data(), mlp.bp.data(),
+      (float)(1.0 / radius), act, (float)alpha, pdf_by_nbr, fp(dbasis), fpm(flat), fpm(flat) + nw,
+      dpin ? fpm(*dpin) : nullptr, dpout ? fpm(*dpout) : nullptr, dpdf ? fpm(*dpdf) : nullptr));
+  py::list dw, db;
+  int64_t ow = 0, ob = nw;
+  for (int l = 0; l < mlp.layers(); ++l) {
+    dw.append(flat.narrow(0, ow, mlp.w[l].numel()).view(mlp.w[l].sizes()));
+    db.append(flat.narrow(0, ob, mlp.b[l].numel()).view(mlp.b[l].sizes()));
+    ow += mlp.w[l].numel();
+    ob += mlp.b[l].numel();
+  }
+  if (!point_grads) return py::make_tuple(dw, db);
+  py::object a = py::cast(*dpin);      // one cloud: one gradient, the same object twice
+  py::object b = dpout->data_ptr() == dpin->data_ptr() ? a : py::cast(*dpout);
+  return py::make_tuple(dw, db, a, b, *dpdf);
+}
+
 Tensor kp_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
                 const Tensor& kernel_points_, double radius, double sigma, int64_t k_pad,
                 int interpolation) {
@@ -100,30 +179,34 @@ Tensor group_plan(const Tensor& order_, const Tensor& ranges_, const Tensor& sor
   return plan;
 }
 
-Tensor project_forward(int k, int c, int cout, const Tensor& ws, const Tensor& basis_,
-                       const Tensor& features_, const Tensor& neigh_, const Tensor& ranges_,
-                       const Tensor& weights_) {
+// groups, k_src, cout_src: how the weights lie (tfgpc_mcconv_forward_blocks)
+Tensor project_forward(int k, int c, int cout, int groups, int k_src, int cout_src,
+                       const Tensor& ws, const Tensor& basis_, const Tensor& features_,
+                       const Tensor& neigh_, const Tensor& ranges_, const Tensor& weights_) {
   Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
          weights = f32(weights_);
   const int64_t ns = ranges.size(0);
   Tensor out = empty({ns, cout}, at::kFloat, basis);
-  check(tfgpc_mcconv_forward(stream(), k, c, cout, ns, features.size(0), basis.size(0), fp(basis),
-                             fp(features), ip(neigh), ip(ranges), fp(weights), fpm(out),
-                             ws.data_ptr(), (size_t)ws.numel()));
+  check(tfgpc_mcconv_forward_blocks(stream(), k, c, cout, groups, k_src, cout_src, ns,
+                                    features.size(0), basis.size(0), fp(basis), fp(features),
+                                    ip(neigh), ip(ranges), fp(weights), fpm(out), ws.data_ptr(),
+                                    (size_t)ws.numel()));
   return out;
 }
 
-py::tuple project_backward(int k, int c, int cout, const Tensor& ws, const Tensor& basis_,
-                           const Tensor& features_, const Tensor& neigh_, const Tensor& ranges_,
-                           const Tensor& weights_, const Tensor& out_grads_, bool reuse) {
+py::tuple project_backward(int k, int c, int cout, int groups, int k_src, int cout_src,
+                           const Tensor& ws, const Tensor& basis_, const Tensor& features_,
+                           const Tensor& neigh_, const Tensor& ranges_, const Tensor& weights_,
+                           const Tensor& out_grads_, bool reuse) {
   Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
          weights = f32(weights_), g = f32(out_grads_);
   Tensor dbasis = at::empty_like(basis), dfeat = at::empty_like(features),
          dw = at::empty_like(weights);
-  check(tfgpc_mcconv_backward(stream(), k, c, cout, ranges.size(0), features.size(0),
-                              basis.size(0), fp(basis), fp(features), ip(neigh), ip(ranges),
-                              fp(weights), fp(g), reuse, fpm(dbasis), fpm(dfeat), fpm(dw),
-                              ws.data_ptr(), (size_t)ws.numel()));
+  check(tfgpc_mcconv_backward_blocks(stream(), k, c, cout, groups, k_src, cout_src,
+                                     ranges.size(0), features.size(0), basis.size(0), fp(basis),
+                                     fp(features), ip(neigh), ip(ranges), fp(weights), fp(g), reuse,
+                                     fpm(dbasis), fpm(dfeat), fpm(dw), ws.data_ptr(),
+                                     (size_t)ws.numel()));
   return py::make_tuple(dbasis, dfeat, dw);
 }
 
@@ -247,9 +330,19 @@ Tensor global_pool(const Tensor& features_, const Tensor& ids_, int64_t batch, i
   return out;
 }
 
-void add_bias_(const Tensor& x, const Tensor& bias_) {
-  Tensor bias = f32(bias_);
-  check(tfgpc_add_bias(stream(), x.size(0), (int)x.size(1), fpm(x), fp(bias)));
+// x [N, C_in] @ weights [C_in, C_out] + bias; C_out that is not a multiple of 8 comes
+// back as the front columns of a wider array
+Tensor linear(const Tensor& x_, const Tensor& weights_, const Tensor& bias_) {
+  Tensor x = f32(x_), weights = f32(weights_), bias = f32(bias_);
+  const int64_t n = x.size(0), cin = x.size(1), cout = weights.size(1);
+  require(weights.size(0) == cin, "matmul expects matching inner dimensions");
+  require(bias.numel() == cout, "Conv1x1 expects one bias per output feature");
+  Tensor out = empty({n, (cout + 7) / 8 * 8}, at::kFloat, x);
+  const size_t need = tfgpc_linear_workspace_bytes(n, cin, cout);
+  Tensor ws = bytes(need, x);
+  check(tfgpc_linear_f32(stream(), n, cin, cout, fp(x), fp(weights), fp(bias), fpm(out),
+                         ws.data_ptr(), need));
+  return out.size(1) == cout ? out : out.narrow(1, 0, cout);
 }
 
 void scale_bias_activation_(const Tensor& x, double scale, const OptTensor& bias_, bool act,
@@ -268,6 +361,8 @@ void bind_layers(py::module_& m) {
   m.def("pack_points_density", &pack_points_density);
   m.def("kernel_basis", &kernel_basis);
   m.def("kernel_basis_grads", &kernel_basis_grads);
+  m.def("kernel_mlp_basis", &kernel_mlp_basis);
+  m.def("kernel_mlp_grads", &kernel_mlp_grads);
   m.def("kp_basis", &kp_basis);
   m.def("pointconv_pdf", &pointconv_pdf);
   m.def("group_plan", &group_plan);
@@ -281,7 +376,8 @@ void bind_layers(py::module_& m) {
   m.def("basis_proj_grads", &basis_proj_grads);
   m.def("neighborhood_pool", &neighborhood_pool);
   m.def("global_pool", &global_pool);
-  m.def("add_bias_", &add_bias_);
+  m.def("linear", &linear);
+  m.def("blocks_supported", &tfgpc_mcconv_blocks_supported);
   m.def("scale_bias_activation_", &scale_bias_activation_);
 }
 

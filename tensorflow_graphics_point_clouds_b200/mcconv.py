@@ -47,21 +47,27 @@ class ProjectionGemm:
     self.ws = _workspace(self.nbytes, self.device)
     self._x_valid = False
 
-  def forward(self, basis, features, neighbors, ranges, weights):
+  def forward(self, basis, features, neighbors, ranges, weights, blocks=None):
+    """blocks: (groups, k_src, cout_src) of weights that are not one dense [C*K, Cout]
+    matrix (tfgpc_mcconv_forward_blocks)."""
     self._ensure_workspace(features.shape[0])
-    out = _lib.host().project_forward(self.k, self.c, self.cout, self.ws, basis, features,
-                                      neighbors, ranges, weights)
+    groups, k_src, cout_src = blocks or (1, self.k, self.cout)
+    out = _lib.host().project_forward(self.k, self.c, self.cout, groups, k_src, cout_src, self.ws,
+                                      basis, features, neighbors, ranges, weights)
     self._x_valid = self.backward_ws
     self._x_grouped = False
     return out
 
-  def backward(self, basis, features, neighbors, ranges, weights, out_grads, reuse_forward=True):
+  def backward(self, basis, features, neighbors, ranges, weights, out_grads, reuse_forward=True,
+               blocks=None):
     if not self.backward_ws:
       raise RuntimeError("this ProjectionGemm was created without backward workspace")
     self._ensure_workspace(features.shape[0])
     reuse = bool(reuse_forward and self._x_valid and not self._x_grouped)
-    return _lib.host().project_backward(self.k, self.c, self.cout, self.ws, basis, features,
-                                        neighbors, ranges, weights, out_grads, reuse)
+    groups, k_src, cout_src = blocks or (1, self.k, self.cout)
+    return _lib.host().project_backward(self.k, self.c, self.cout, groups, k_src, cout_src, self.ws,
+                                        basis, features, neighbors, ranges, weights, out_grads,
+                                        reuse)
 
   def forward_grouped(self, basis_pair, features, weights, order, plan):
     """The forward pass through tfgpc_mcconv_forward_grouped: the projection runs
@@ -155,63 +161,24 @@ def group_plan(neighborhood, order=None):
                                        neighborhood._original_neigh_ids)
 
 
-def _mlp_blocks(weights, biases):
-  """Per-layer tensors [G, H_{l-1}, H_l] / [G, 1, H_l] -> (flat weights, flat
-  biases, layer sizes as a host int32 array, D, G)."""
-  weights = [_f32(w) for w in weights]
-  biases = [_f32(b) for b in biases]
-  g, d, _ = weights[0].shape
-  sizes = (ctypes.c_int32 * len(weights))(*[int(w.shape[2]) for w in weights])
-  flat_w = torch.cat([w.reshape(-1) for w in weights]).contiguous()
-  flat_b = torch.cat([b.reshape(-1) for b in biases]).contiguous()
-  return flat_w, flat_b, sizes, int(d), int(g)
-
-
 def kernel_mlp_basis(points_in, points_out, neighbors, pdf, weights, biases, radius,
                      activation=0, alpha=0.2, pdf_by_neighbor=False):
-  """The kernel MLP with any number of hidden layers (tfgpc_kernel_mlp_basis):
+  """The kernel MLP with any number of hidden layers (tfgpc_kernel_mlp_basis_layers):
   weights[l] [G, H_{l-1}, H_l], biases[l] [G, 1, H_l] -> basis [M, G * H_last]."""
-  points_in, points_out, pdf, neighbors = _f32(points_in), _f32(points_out), _f32(pdf), _i32(neighbors)
-  flat_w, flat_b, sizes, d, g = _mlp_blocks(weights, biases)
-  m = neighbors.shape[0]
-  basis = torch.empty((m, g * int(sizes[len(sizes) - 1])), dtype=torch.float32,
-                      device=points_in.device)
-  _lib.check(_lib.lib().tfgpc_kernel_mlp_basis(
-      _stream(), c_int(d), c_int(g), c_int(len(sizes)), sizes, c_i64(m), ptr(points_in),
-      ptr(points_out), ptr(neighbors), ptr(pdf), ptr(flat_w), ptr(flat_b),
-      ctypes.c_float(1.0 / float(radius)), c_int(activation), ctypes.c_float(alpha),
-      c_int(int(pdf_by_neighbor)), ptr(basis)))
-  return basis
+  return _lib.host().kernel_mlp_basis(points_in, points_out, neighbors, pdf, list(weights),
+                                      list(biases), float(radius), activation, alpha,
+                                      bool(pdf_by_neighbor))
 
 
 def kernel_mlp_grads(points_in, points_out, neighbors, pdf, weights, biases, radius, basis_grads,
                      activation=0, alpha=0.2, point_grads=False, pdf_by_neighbor=False):
-  """All gradients of kernel_mlp_basis (tfgpc_kernel_mlp_grads): ([d_weights],
+  """All gradients of kernel_mlp_basis (tfgpc_kernel_mlp_grads_layers): ([d_weights],
   [d_biases]) in the layouts of the inputs and, with point_grads, also
   (d_points_in, d_points_out, d_pdf [M]); when points_in and points_out are the
   same tensor, d_points_in and d_points_out are one tensor holding the sum."""
-  points_in, points_out, pdf, neighbors = _f32(points_in), _f32(points_out), _f32(pdf), _i32(neighbors)
-  basis_grads = _f32(basis_grads)
-  flat_w, flat_b, sizes, d, g = _mlp_blocks(weights, biases)
-  dw, db = torch.empty_like(flat_w), torch.empty_like(flat_b)
-  dpin = dpout = dpdf = None
-  if point_grads:
-    dpin = torch.empty_like(points_in)
-    dpout = dpin if points_out.data_ptr() == points_in.data_ptr() else torch.empty_like(points_out)
-    dpdf = torch.empty(neighbors.shape[0], dtype=torch.float32, device=pdf.device)
-  _lib.check(_lib.lib().tfgpc_kernel_mlp_grads(
-      _stream(), c_int(d), c_int(g), c_int(len(sizes)), sizes, c_i64(neighbors.shape[0]),
-      c_i64(points_in.shape[0]), c_i64(points_out.shape[0]), ptr(points_in), ptr(points_out),
-      ptr(neighbors), ptr(pdf), ptr(flat_w), ptr(flat_b), ctypes.c_float(1.0 / float(radius)),
-      c_int(activation), ctypes.c_float(alpha), c_int(int(pdf_by_neighbor)), ptr(basis_grads),
-      ptr(dw), ptr(db), ptr(dpin), ptr(dpout), ptr(dpdf)))
-  d_weights, d_biases, ow, ob = [], [], 0, 0
-  for w, b in zip(weights, biases):
-    d_weights.append(dw[ow:ow + w.numel()].reshape(w.shape)); ow += w.numel()
-    d_biases.append(db[ob:ob + b.numel()].reshape(b.shape)); ob += b.numel()
-  if point_grads:
-    return d_weights, d_biases, dpin, dpout, dpdf
-  return d_weights, d_biases
+  return _lib.host().kernel_mlp_grads(points_in, points_out, neighbors, pdf, list(weights),
+                                      list(biases), float(radius), basis_grads, activation, alpha,
+                                      bool(point_grads), bool(pdf_by_neighbor))
 
 
 def kernel_basis_grads(points_in, points_out, neighbors, pdf, w1, b1, radius, basis_grads,
@@ -313,12 +280,18 @@ class MCConv:
     if (self._op is None or self._op.ns != ns or self._op.backward_ws != keep_for_backward):
       self._op = ProjectionGemm(self.k, self.cin, self.cout, ns, features.device,
                                 backward=keep_for_backward)
-    wd = self._dense_weights()
+    # several kernel MLPs: their weight blocks as they are, or one dense matrix
+    self._blocks = None
+    if (self.num_mlps > 1 and not grouped and
+        _lib.host().blocks_supported(self.k, self.cin, self.cout, self.num_mlps)):
+      self._blocks, wd = (self.num_mlps, self.k, self.cout), self.wf
+    else:
+      wd = self._dense_weights()
     if grouped:
       out = self._op.forward_grouped(self._grouped[0], features, wd, self._grouped[1],
                                      self._grouped[2])
     else:
-      out = self._op.forward(basis, features, ids, neigh._samples_neigh_ranges, wd)
+      out = self._op.forward(basis, features, ids, neigh._samples_neigh_ranges, wd, self._blocks)
     if keep_for_backward:
       self._saved = (neigh, point_cloud_in, point_cloud_out, radius, pdf, basis,
                      _f32(features), wd, w1, b1)
@@ -351,8 +324,8 @@ class MCConv:
           pair, features, neigh._samples_neigh_ranges, wd, out_grads, order, plan)
     else:
       dbasis, dfeat, dwd = self._op.backward(basis, features, ids, neigh._samples_neigh_ranges,
-                                             wd, out_grads)
-    dwf = (dwd.unsqueeze(0) if self.num_mlps == 1
+                                             wd, out_grads, blocks=self._blocks)
+    dwf = (dwd.unsqueeze(0) if self.num_mlps == 1 else dwd if self._blocks
            else blocks_of_dense_grad(dwd, self.num_mlps, self.cin, self.hidden))
     if point_grads or len(self.kernel_weights) > 1:
       res = kernel_mlp_grads(pc_in._points, pc_out._points, ids, pdf, self.kernel_weights,
@@ -381,15 +354,6 @@ def _basis_count(k):
     if k <= cand:
       return cand
   raise _lib.TfgpcError(1, "at most 64 basis functions are supported")
-
-
-def _pad_weights(w, cin, k, k_pad, cout_pad):
-  """[cin*k, cout] -> [cin*k_pad, cout_pad] with zero rows for the padding
-  basis functions and zero columns up to a multiple of 8."""
-  cout = w.shape[1]
-  wp = torch.zeros((cin, k_pad, cout_pad), dtype=torch.float32, device=w.device)
-  wp[:, :k, :cout] = w.reshape(cin, k, cout)
-  return wp.reshape(cin * k_pad, cout_pad)
 
 
 def kp_basis(points_in, points_out, neighbors, kernel_points, radius, sigma, k_pad,
@@ -428,22 +392,19 @@ class _ProjectedConv:
     if self._op is None or self._op.ns != ns or self._op.backward_ws != keep_for_backward:
       self._op = ProjectionGemm(self.k_pad, self.cin, self.cout_pad, ns, features.device,
                                 backward=keep_for_backward)
-    wp = _pad_weights(_f32(weights), self.cin, self.k, self.k_pad, self.cout_pad)
-    out = self._op.forward(basis, _f32(features), neigh._original_neigh_ids,
-                           neigh._samples_neigh_ranges, wp)
+    weights, blocks = _f32(weights), (1, self.k, self.cout)
+    features = _f32(features)
+    out = self._op.forward(basis, features, neigh._original_neigh_ids, neigh._samples_neigh_ranges,
+                           weights, blocks)
     if keep_for_backward:
-      self._saved = (neigh, basis, _f32(features), wp)
+      self._saved = (neigh, basis, features, weights)
     return out[:, :self.cout] if self.cout_pad != self.cout else out
 
   def _backward(self, out_grads):
-    neigh, basis, features, wp = self._saved
-    g = _f32(out_grads)
-    if self.cout_pad != self.cout:
-      g = torch.nn.functional.pad(g, (0, self.cout_pad - self.cout))
-    dbasis, dfeat, dwp = self._op.backward(basis, features, neigh._original_neigh_ids,
-                                           neigh._samples_neigh_ranges, wp, g)
-    dw = dwp.reshape(self.cin, self.k_pad, self.cout_pad)[:, :self.k, :self.cout]
-    return dbasis, dfeat, dw.reshape(self.cin * self.k, self.cout).contiguous()
+    neigh, basis, features, weights = self._saved
+    return self._op.backward(basis, features, neigh._original_neigh_ids,
+                             neigh._samples_neigh_ranges, weights, out_grads,
+                             blocks=(1, self.k, self.cout))
 
 
 class KPConv(_ProjectedConv):
@@ -552,20 +513,9 @@ def global_pool(features, point_cloud, mode='max'):
 
 def conv1x1(features, weights, bias):
   """Conv1x1.py:97: features [N, C_in] @ weights [C_in, C_out] + bias [1, C_out].
-  The product runs on the tensor cores; channel counts that are not multiples
-  of 8 are zero padded for it."""
-  features, weights, bias = _f32(features), _f32(weights), _f32(bias).reshape(-1)
-  n, cin = features.shape
-  cout = weights.shape[1]
-  cin_p, cout_p = (cin + 7) // 8 * 8, (cout + 7) // 8 * 8
-  if cin_p != cin:
-    features = torch.nn.functional.pad(features, (0, cin_p - cin))
-  if cin_p != cin or cout_p != cout:
-    weights = torch.nn.functional.pad(weights, (0, cout_p - cout, 0, cin_p - cin))
-    bias = torch.nn.functional.pad(bias, (0, cout_p - cout))
-  out = matmul_f32(features, weights)
-  _lib.host().add_bias_(out, bias)
-  return out[:, :cout] if cout_p != cout else out
+  The product and the bias run on the tensor cores as one call
+  (tfgpc_linear_f32)."""
+  return _lib.host().linear(features, weights, bias)
 
 
 def scale_bias_activation_(x, scale=1.0, bias=None, leaky_alpha=None):
