@@ -7,8 +7,10 @@
 // so no neighbor list is needed: on 8 clouds of 100 000 Gaussian-mixture points
 // searching and writing the lists of four levels took 3.2 ms, the passes over them 0.6.
 // The passes and the compaction of the taken points in ascending index are one
-// cooperative launch with a barrier between passes; what bounds it is the chain of
-// passes on small levels and the marking on crowded ones.
+// cooperative launch; what bounds it is the chain of passes on small levels and the
+// marking on crowded ones.  Only cells of later passes are marked (13 of 26 neighbors
+// on average).  Clouds do not meet, so each has a team of blocks, in proportion to its
+// points, with barriers of its own.
 //
 // Cell average (sampling_avg_kernels.cu.cc:43-88): one thread per occupied cell,
 // sequential fp32 sum of its points / count, cells in ascending first index.
@@ -20,6 +22,8 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxBlocks = 1024;
+constexpr int kMaxTeams = kMaxBlocks / 2;
+constexpr size_t kHeadBytes = (size_t)(kMaxTeams + 4) * 4;   // barrier words before the states
 constexpr unsigned long long kBarrierLimitNs = 1000000000ull;
 
 struct SampleArgs {
@@ -28,7 +32,8 @@ struct SampleArgs {
   int mode;                    // 0 Poisson disk, 1 cell average
   const float* inv_radii;
   uint8_t* state;              // [n] 0 open, 1 blocked, 2 taken (zero on entry)
-  unsigned* arrived;           // barrier counter (zero on entry), then an error word
+  unsigned* arrived;           // barrier counter of the grid, an error word, two words unused,
+                               // then the teams' counters; all zero on entry
   int32_t* block_total;        // [gridDim.x]
   float* pts_out;
   int32_t* batch_out;
@@ -36,9 +41,9 @@ struct SampleArgs {
   int32_t* page;               // number of samples (64 bits), then the error word
 };
 
-// Barrier over the blocks of a cooperative launch (all resident).  Gives up after a
-// second: the error word is set and every later barrier passes at once.
-__device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target) {
+// Barrier over blocks of a cooperative launch (all resident) that share a counter.
+// Gives up after a second: the error word is set and every later barrier passes at once.
+__device__ __forceinline__ bool barrier(unsigned* arrived, unsigned target, unsigned* error) {
   __shared__ bool ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -49,8 +54,8 @@ __device__ __forceinline__ bool grid_barrier(unsigned* arrived, unsigned target)
     ok = true;
     while (*(volatile unsigned*)arrived < target) {
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (t - t0 > kBarrierLimitNs || *(volatile unsigned*)(arrived + 1) != 0u) {
-        *(volatile unsigned*)(arrived + 1) = 1u;
+      if (t - t0 > kBarrierLimitNs || *(volatile unsigned*)error != 0u) {
+        *(volatile unsigned*)error = 1u;
         ok = false;
         break;
       }
@@ -95,21 +100,59 @@ __device__ __forceinline__ bool within(const float* s, const float* p, const flo
   return d2 < 1.0f;
 }
 
+// Sorted points [x, y) to be marked in one half of a tube around `cell`.  The pass of
+// a cell is the number whose bit d is the parity of its coordinate d, so the last
+// coordinate decides first: from an even one both ends of a tube are later, from an odd
+// one none is; the middle is later if the leading coordinates' bits are.  A tube that
+// is later as a whole is its first half alone.  own: the cell itself counts as later.
+template <int D>
+__device__ __forceinline__ int2 later_points(int code, const int* cell, int batch, const int* nc,
+                                             int total, bool own,
+                                             const int32_t* __restrict__ start) {
+  int base = 0, scale = 1, rem = code >> 1, mine = 0, theirs = 0;
+  bool ok = true;
+#pragma unroll
+  for (int d = D - 2; d >= 0; --d) {
+    const int c = cell[d] + rem % 3 - 1;
+    rem /= 3;
+    ok = ok && c >= 0 && c < nc[d];
+    base += c * scale;
+    scale *= nc[d];
+    mine |= (cell[d] & 1) << d;
+    theirs |= (c & 1) << d;
+  }
+  const int z = cell[D - 1];
+  const bool second = code & 1, even = (z & 1) == 0;
+  const bool later = theirs > mine || (own && code >> 1 == num_tubes<D>() / 2);
+  int lo, hi;
+  if (later) {
+    lo = even ? max(z - 1, 0) : z;
+    hi = even ? min(z + 1, nc[D - 1] - 1) : z;
+    ok = ok && !second;
+  } else {
+    lo = hi = second ? z + 1 : z - 1;
+    ok = ok && even && lo >= 0 && lo < nc[D - 1];
+  }
+  if (!ok) return make_int2(0, 0);
+  base = (batch * scale + base) * nc[D - 1];
+  return make_int2(__ldg(start + (total - (base + hi))), __ldg(start + (total - (base + lo)) + 1));
+}
+
 // Marks the neighbors of the taken points: the candidates of the cell, kSteps per lane
-// at a time in registers, against all of them.
+// at a time in registers, against all of them.  own: in the cell itself too.
 template <int D>
 __device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& taken,
                                                const int* cell, int batch, const int* nc,
-                                               int total, const float* inv_r) {
+                                               int total, const float* inv_r, bool own) {
   constexpr int kSteps = 4;
-  constexpr int kTubes = num_tubes<D>();
-  constexpr int kTop = kTubes > 16 ? 16 : kTubes > 8 ? 8 : kTubes > 4 ? 4 : 2;
+  constexpr int kHalves = 2 * num_tubes<D>();
+  constexpr int kTop = kHalves > 16 ? 16 : kHalves > 8 ? 8 : 4;
   const int lane = lane_id();
   if (lane < taken.count) __stcg(a.state + taken.j, (uint8_t)2);
-  for (int tube0 = 0; tube0 < kTubes; tube0 += 32) {
+  for (int half0 = 0; half0 < kHalves; half0 += 32) {
     int2 r = make_int2(0, 0);
-    if (tube0 + lane < kTubes)
-      r = tube_points<D>(kTubes - 1 - (tube0 + lane), cell, batch, nc, total, a.c.start);
+    if (half0 + lane < kHalves)
+      r = later_points<D>(half0 + lane, cell, batch, nc, total, own, a.c.start);
     int before = r.y - r.x;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -196,12 +239,50 @@ __device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cel
         taken.j = q0 + t;
       }
       if (++taken.count == 32) {
-        mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r);
+        mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, true);
         __syncwarp();   // these marks are visible to the next group's reads
       }
     }
   }
-  if (taken.count > 0) mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r);
+  if (taken.count > 0) mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, false);
+}
+
+// The team of a block: blocks [begin, begin + size) work on `cloud`; with too many clouds
+// for teams, all blocks on all of them (cloud -1).  size 0: a block left over.
+struct Team { int cloud, begin, size; };
+
+// One block per cloud and the others in proportion to the clouds' points.
+__device__ __forceinline__ Team team_of(const CellsView& c, int total) {
+  const int lane = lane_id();
+  if (c.batch_size > kMaxTeams || c.batch_size * 2 > (int)gridDim.x)
+    return Team{-1, 0, (int)gridDim.x};
+  const int cells = total / c.batch_size;
+  const long long spare = (int)gridDim.x - c.batch_size;
+  int before = 0;
+  for (int b0 = 0; b0 < c.batch_size; b0 += 32) {
+    const int b = b0 + lane;
+    int share = 0;
+    if (b < c.batch_size) {
+      const int points = __ldg(c.start + (total - b * cells) + 1) -
+                         __ldg(c.start + (total - (b + 1) * cells) + 1);
+      share = 1 + (int)(spare * points / c.n);
+    }
+    int upto = share;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    upto += before;
+    const unsigned m = __ballot_sync(0xffffffffu, upto > (int)blockIdx.x);
+    if (m) {
+      const int who = __ffs(m) - 1;
+      const int size = __shfl_sync(0xffffffffu, share, who);
+      return Team{b0 + who, __shfl_sync(0xffffffffu, upto, who) - size, size};
+    }
+    before = __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return Team{0, 0, 0};
 }
 
 template <int D>
@@ -226,10 +307,12 @@ cells_sample_kernel(SampleArgs a) {
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < lead + (n - tail);
          i += (int64_t)gridDim.x * kThreads)
       a.state[i < lead ? i : tail + (i - lead)] = 2;
-    const int warps = gridDim.x * kWarps;
-    const int warp = blockIdx.x * kWarps + w;
-    for (int pass = 0; pass < (1 << D); ++pass) {
-      int half[D], cells = a.c.batch_size;
+    const Team team = team_of(a.c, total);
+    const int warps = team.size * kWarps;
+    const int warp = ((int)blockIdx.x - team.begin) * kWarps + w;
+    unsigned* const counter = team.cloud < 0 ? a.arrived : a.arrived + 4 + team.cloud;
+    for (int pass = 0; pass < (1 << D) && team.size > 0; ++pass) {
+      int half[D], cells = team.cloud < 0 ? a.c.batch_size : 1;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
         half[d] = (nc[d] - ((pass >> d) & 1) + 1) >> 1;
@@ -250,7 +333,7 @@ cells_sample_kernel(SampleArgs a) {
             key += cell[d] * scale;
             scale *= nc[d];
           }
-          batch = rem;
+          batch = team.cloud < 0 ? rem : team.cloud;
           key += batch * scale;
           begin = __ldg(a.c.start + (total - key));
           end = __ldg(a.c.start + (total - key) + 1);
@@ -267,8 +350,12 @@ cells_sample_kernel(SampleArgs a) {
                           __shfl_sync(0xffffffffu, end, who), nc, total, inv_r);
         }
       }
-      ok = grid_barrier(a.arrived, ++barriers * gridDim.x) && ok;
+      // (the barrier after the last pass is the one of the compaction)
+      if (pass + 1 < (1 << D))
+        ok = barrier(counter, (pass + 1) * team.size, a.arrived + 1) && ok;
     }
+    if (team.cloud < 0) barriers = (1 << D) - 1;
+    ok = barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1) && ok;
   }
   // ---- compaction: every block counts, then writes, its stretch of the points
   const int64_t per = (n + gridDim.x - 1) / gridDim.x;
@@ -289,7 +376,7 @@ cells_sample_kernel(SampleArgs a) {
     for (int i = 0; i < kWarps; ++i) t += warp_total[i];
     __stcg(a.block_total + blockIdx.x, t);
   }
-  ok = grid_barrier(a.arrived, ++barriers * gridDim.x) && ok;
+  ok = barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1) && ok;
   if (w == 0) {
     int64_t t = 0, all = 0;
     for (int i = lane; i < gridDim.x; i += 32) {
@@ -380,27 +467,27 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
 }
 
 size_t sample_ws_bytes(int64_t n) {
-  return align_up((size_t)n + 16, 256) + align_up((size_t)kMaxBlocks * 4, 256);
+  return align_up((size_t)n + kHeadBytes, 256) + align_up((size_t)kMaxBlocks * 4, 256);
 }
 
 // Enqueues the sampling; the number of samples goes to words kReportTotal .. of the page.
 int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const float* inv_radii,
                  float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page) {
-  const size_t state = align_up((size_t)g.n + 16, 256);
+  const size_t state = align_up((size_t)g.n + kHeadBytes, 256);
   SampleArgs a;
   a.c = view_of(g);
   a.keys = g.sorted_keys;
   a.mode = mode;
   a.inv_radii = inv_radii;
-  a.arrived = (unsigned*)ws;          // [0] counter, [1] error word, then the states
-  a.state = (uint8_t*)ws + 16;
+  a.arrived = (unsigned*)ws;
+  a.state = (uint8_t*)ws + kHeadBytes;
   a.block_total = (int32_t*)((char*)ws + state);
   a.pts_out = pts_out;
   a.batch_out = batch_out;
   a.index_out = index_out;
   a.page = page + kReportTotal;
   ProfScope prof(st, mode == 0 ? "sampling_poisson" : "sampling_cell_average");
-  TFGPC_CUDA(cudaMemsetAsync(ws, 0, mode == 0 ? (size_t)g.n + 16 : 16, st));
+  TFGPC_CUDA(cudaMemsetAsync(ws, 0, mode == 0 ? (size_t)g.n + kHeadBytes : kHeadBytes, st));
   switch (g.D) {
     case 2: return launch_sample<2>(st, a);
     case 3: return launch_sample<3>(st, a);
