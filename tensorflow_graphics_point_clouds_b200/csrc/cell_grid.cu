@@ -11,10 +11,19 @@
 // start plus the number of points of the cell with a smaller index, counted over the
 // cell's members; that is quadratic in the cell size like the neighbor search
 // that follows, and a 27th of its work.
+//
+// Up to kClusterPoints points the whole chain is ONE kernel of one thread-block cluster
+// (grid_cluster_kernel): its phases meet at the cluster's hardware barrier, boxes and
+// table sums are exchanged through distributed shared memory, and there is nothing to
+// initialise before it.
+#include <cooperative_groups.h>
+
 #include "cell_grid.cuh"
 
 namespace tfgpc {
 namespace {
+
+namespace cg = cooperative_groups;
 
 constexpr int kThreads = 256;
 constexpr int kBoxPer = 4;     // points per lane of the bounding-box pass
@@ -39,8 +48,7 @@ __device__ __forceinline__ void clip_and_report(int D, int max_cells, const int*
     page[d] = c;
     used[d] = min(c, max_cells);
   }
-  page[TFGPC_MAX_DIMS] = over;
-  __threadfence_system();
+  page[TFGPC_MAX_DIMS] = over;     // (read after the stream is synchronised: no fence)
 }
 
 // Per-cloud boxes (PointCloud.py:38-43) folded per lane, then per warp where a warp
@@ -187,6 +195,18 @@ scatter_kernel(int64_t n, const int64_t* __restrict__ keys, const int32_t* __res
   members[__ldg(start + r) + __ldg(arrival + i)] = (int32_t)i;
 }
 
+// Number of the members [a, e) of a bucket with an index below idx.
+__device__ __forceinline__ int rank_in_bucket(const int32_t* members, int a, int e, int idx) {
+  int rank = 0, q = a;
+  for (; q < e && (q & 3); ++q) rank += members[q] < idx;
+  for (; q + 4 <= e; q += 4) {
+    const int4 m = *(const int4*)(members + q);
+    rank += (m.x < idx) + (m.y < idx) + (m.z < idx) + (m.w < idx);
+  }
+  for (; q < e; ++q) rank += members[q] < idx;
+  return rank;
+}
+
 // One thread per slot of `members`: the rank of its point inside the bucket, and the
 // point's row of every sorted array; then the tube ranges, read off the table.
 template <int D>
@@ -207,10 +227,7 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
     const int64_t key = __ldg(keys + idx);
     const int r = bucket_of(key, total);
     const int a = __ldg(start + r), e = __ldg(start + r + 1);
-    int rank = 0;
-#pragma unroll 4
-    for (int q = a; q < e; ++q) rank += __ldg(members + q) < idx;
-    const int64_t o = a + rank;
+    const int64_t o = a + rank_in_bucket(members, a, e, idx);
     perm[o] = idx;
     skeys[o] = key;
     sbid[o] = __ldg(batch_ids + idx);
@@ -233,12 +250,265 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
   }
 }
 
+// ---- the chain in one cluster -------------------------------------------------------
+
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterBoxes = 1024;        // batch size x D at most
+// Where the cluster stops: its 16 SMs build a grid of 41 000 points in 20 us and the
+// separate kernels in 25, and the host launches one kernel or two in place of eight
+// (layer step on 4 x 1024 points 191 -> 173 us, 3-level cell averages of 5 x 9000 points
+// 243 -> 197, three-level classifier 884 -> 834); the table is zeroed and scanned by
+// them alone, so a large one goes to the whole GPU.  The sorted copies scatter 44 bytes
+// a point: from 8192 points on they are a launch of their own (41 000 points: 13 us of
+// the cluster's 33, 4.4 by themselves).
+constexpr int kMaxRanks = 16;
+constexpr int64_t kClusterPoints = 65536;
+constexpr int64_t kClusterCells = int64_t(1) << 21;
+constexpr int64_t kClusterPlacePoints = 8192;
+
+struct ClusterBuild {
+  int64_t n;
+  const float* pts;
+  const int32_t* batch_ids;
+  int batch_size, max_cells;
+  DimValues cell_sizes;
+  tfgpc_cell_grid g;
+  int32_t *arrival, *members, *page;
+  bool place;
+};
+
+template <int D>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+grid_cluster_kernel(ClusterBuild a) {
+  // [0] ordered keys of the lower corners, [1] complements of those of the upper ones
+  __shared__ unsigned box[2][kClusterBoxes];
+  __shared__ float smin_s[kClusterBoxes];
+  __shared__ int asked[D], nc_s[D];
+  __shared__ int warp_sum_s[32], block_sum_s;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+  const int n = (int)a.n, boxes = a.batch_size * D;
+  const int stride = ranks * kClusterThreads, first = rank * kClusterThreads + tid;
+  // ---- boxes of this block's points
+  for (int i = tid; i < boxes; i += kClusterThreads) box[0][i] = box[1][i] = 0xffffffffu;
+  if (tid < D) asked[tid] = 1;
+  __syncthreads();
+  for (int i0 = first - lane; i0 < n; i0 += stride) {
+    const int i = i0 + lane;
+    const bool live = i < n;
+    const int b = live ? __ldg(a.batch_ids + i) : -1;
+    float lo[D], hi[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const float v = live ? __ldg(a.pts + (int64_t)i * D + d) : 0.0f;
+      // (a coordinate that is no number counts for no box)
+      lo[d] = live ? fminf(INFINITY, v) : INFINITY;
+      hi[d] = live ? fmaxf(-INFINITY, v) : -INFINITY;
+    }
+    const int b0 = __shfl_sync(0xffffffffu, b, 0);
+    const bool uniform = __all_sync(0xffffffffu, b == b0 || !live);
+    if (uniform) {
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+          hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+    }
+    if (b >= 0 && b < a.batch_size && (!uniform || lane == 0)) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        atomicMin(&box[0][b * D + d], ordered(lo[d]));
+        atomicMin(&box[1][b * D + d], ~ordered(hi[d]));
+      }
+    }
+  }
+  cluster.sync();
+  // ---- parameters, by every block for itself (see boxes_kernel)
+  for (int i = tid; i < boxes; i += kClusterThreads) {
+    unsigned kl = 0xffffffffu, kh = 0xffffffffu;
+#pragma unroll
+    for (int r = 0; r < kMaxRanks; ++r) {      // (all loads in flight together)
+      const unsigned* other = cluster.map_shared_rank(&box[0][0], min(r, ranks - 1));
+      kl = min(kl, other[i]);
+      kh = min(kh, other[kClusterBoxes + i]);
+    }
+    const int d = i % D;
+    const float cs = a.cell_sizes.v[d];
+    const float mn = __fsub_rn(kl == 0xffffffffu ? INFINITY : unordered(kl), 1e-9f);
+    const float mx = __fadd_rn(kh == 0xffffffffu ? -INFINITY : unordered(~kh), 1e-9f);
+    const float sm = __fdiv_rn(mn, cs);
+    smin_s[i] = sm;
+    if (rank == 0) {
+      a.g.aabb_min[i] = mn;
+      a.g.aabb_max[i] = mx;
+      a.g.scaled_aabb_min[i] = sm;
+    }
+    const float c = ceilf(__fdiv_rn(__fsub_rn(mx, mn), cs));
+    if (c > 0.0f && c < 2147483000.0f) atomicMax(&asked[d], (int)c);
+  }
+  __syncthreads();
+  if (tid < D) nc_s[tid] = min(asked[tid], a.max_cells);
+  __syncthreads();
+  Grid<D> g;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    g.nc[d] = nc_s[d];
+    g.inv[d] = __fdiv_rn(1.0f, a.cell_sizes.v[d]);
+    if (rank == 0 && tid == 0) a.g.inv_cell_sizes[d] = g.inv[d];
+  }
+  const int total = total_cells<D>(g.nc, a.batch_size);
+  int32_t* const table = a.g.cell_start;
+  for (int i = first; i < total + 3; i += stride) __stcg(table + i, 0);
+  cluster.sync();
+  // ---- keys and the number of points per bucket (see keys_histogram_kernel)
+  for (int i = first; i < n; i += stride) {
+    const int b = __ldg(a.batch_ids + i);
+    const int bs = min(max(b, 0), a.batch_size - 1);
+    float p[D];
+    int cell[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) p[d] = __ldg(a.pts + (int64_t)i * D + d);
+    cell_of<D>(p, smin_s + bs * D, g, cell);
+    const int64_t key = key_of<D>(cell, g, b);
+    __stcg((long long*)a.g.keys + i, (long long)key);
+    __stcg(a.arrival + i, atomicAdd(table + bucket_of(key, total), 1));
+  }
+  cluster.sync();
+  // ---- exclusive scan of the table: a stretch per block, its sum first
+  const int per = (((total + 3) + ranks - 1) / ranks + 3) / 4 * 4;
+  const int begin = min(rank * per, total + 3), end = min(begin + per, total + 3);
+  int sum = 0;
+  for (int i = begin + tid; i < end; i += kClusterThreads) sum += __ldcg(table + i);
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) warp_sum_s[w] = sum;
+  __syncthreads();
+  if (w == 0) {
+    sum = __reduce_add_sync(0xffffffffu, warp_sum_s[lane]);
+    if (lane == 0) block_sum_s = sum;
+  }
+  cluster.sync();
+  int run = 0;
+  if (lane < rank) run = *cluster.map_shared_rank(&block_sum_s, lane);
+  run = __reduce_add_sync(0xffffffffu, run);
+  for (int t0 = begin; t0 < end; t0 += 4 * kClusterThreads) {
+    const int i = t0 + 4 * tid;
+    int v[4], x = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = i + k < end ? __ldcg(table + i + k) : 0;
+      x += v[k];
+    }
+    const int own = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    __syncthreads();
+    if (lane == 31) warp_sum_s[w] = x;
+    __syncthreads();
+    const int s = warp_sum_s[lane];
+    int at = run + x - own + __reduce_add_sync(0xffffffffu, lane < w ? s : 0);
+    run += __reduce_add_sync(0xffffffffu, s);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i + k < end) __stcg(table + i + k, at);
+      at += v[k];
+    }
+  }
+  cluster.sync();
+  // ---- members of the buckets, then every point's place (see place_kernel)
+  for (int i = first; i < n; i += stride) {
+    const int r = bucket_of(__ldcg((const long long*)a.g.keys + i), total);
+    __stcg(a.members + __ldcg(table + r) + __ldcg(a.arrival + i), i);
+  }
+  cluster.sync();   // (also: no block leaves while others read its shared memory)
+  if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
+  if (!a.place) return;
+  for (int i = first; i < n; i += stride) {
+    const int idx = __ldcg(a.members + i);
+    const int64_t key = __ldcg((const long long*)a.g.keys + idx);
+    const int r = bucket_of(key, total);
+    const int o = __ldcg(table + r) + rank_in_bucket(a.members, __ldcg(table + r),
+                                                     __ldcg(table + r + 1), idx);
+    a.g.sorted_indices[o] = idx;
+    a.g.sorted_keys[o] = key;
+    a.g.sorted_batch_ids[o] = __ldg(a.batch_ids + idx);
+    float p[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      p[d] = __ldg(a.pts + (int64_t)idx * D + d);
+      a.g.sorted_points[(int64_t)o * D + d] = p[d];
+    }
+    if (D <= 3)
+      ((float4*)a.g.packed)[o] = make_float4(p[0], p[1], D == 3 ? p[D - 1] : 0.0f,
+                                             __int_as_float(idx));
+  }
+  int span = 1;
+#pragma unroll
+  for (int d = 2; d < D; ++d) span *= g.nc[d];
+  const int tubes = total / span;
+  for (int t = first; t < tubes; t += stride) {
+    const int x = __ldcg(table + (total - (t * span + span - 1)));
+    const int y = __ldcg(table + (total - t * span) + 1);
+    ((int2*)a.g.ds)[t] = y > x ? make_int2(x, y) : make_int2(0, 0);
+  }
+}
+
+template <int D>
+int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
+  static int ranks_of[64] = {0};     // per device (the same value whoever computes it)
+  int dev = 0;
+  TFGPC_CUDA(cudaGetDevice(&dev));
+  int ranks = dev < 64 ? ranks_of[dev] : 0;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {kMaxRanks, 1, 1};
+  cfg.gridDim = dim3(kMaxRanks);
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (ranks == 0) {
+    int fit = 0;
+    if (cudaFuncSetAttribute(grid_cluster_kernel<D>,
+                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&fit, grid_cluster_kernel<D>, &cfg) != cudaSuccess)
+      fit = 0;
+    cudaGetLastError();
+    ranks = fit > 0 ? kMaxRanks : 8;
+    if (dev < 64) ranks_of[dev] = ranks;
+  }
+  // a thread per point, and per 16 cells the table has room for
+  const int64_t room = table_cells(D, a.batch_size, a.max_cells) / 16;
+  const int64_t threads = a.n > room ? a.n : room;
+  while (ranks > 1 && threads <= (int64_t)(ranks / 2) * kClusterThreads) ranks /= 2;
+  cfg.gridDim = dim3(ranks);
+  at[0].val.clusterDim = {(unsigned)ranks, 1, 1};
+  TFGPC_CUDA(cudaLaunchKernelEx(&cfg, grid_cluster_kernel<D>, a));
+  return TFGPC_OK;
+}
+
+int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const int32_t* batch_ids,
+          const CellGridWs& w) {
+  TFGPC_DIM_SWITCH(g.D, place_kernel<kD><<<blocks_for(g.n, kThreads), kThreads, 0, st>>>(
+      g.n, w.members, g.keys, g.num_cells, (int)g.batch_size, g.cell_start, points, batch_ids,
+      g.sorted_indices, g.sorted_keys, g.sorted_points, g.sorted_batch_ids, (float4*)g.packed,
+      (int2*)g.ds));
+  TFGPC_LAUNCH_CHECK();
+  return TFGPC_OK;
+}
+
 }  // namespace
 
 CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch_size,
                            int max_cells) {
   CellGridWs w;
-  char* p = (char*)ws;
+  char* p = (char*)align_up((size_t)ws, 256);
   auto take = [&](size_t b) { char* r = p; p += align_up(b, 256); return r; };
   const int64_t cells = table_cells(D, batch_size, max_cells) + 3;
   w.box_bytes = ((size_t)batch_size * D * 2 + 1) * 4;
@@ -248,7 +518,7 @@ CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch
   const int64_t a = scan_block_sums_elems(cells), b = scan_block_sums_elems(ns);
   w.sums = (int64_t*)take((size_t)(a > b ? a : b) * 8);
   w.total = (int64_t*)take(8);
-  w.bytes = (size_t)(p - (char*)ws);
+  w.bytes = (size_t)(p - (char*)align_up((size_t)ws, 256));
   return w;
 }
 
@@ -260,6 +530,17 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   const int64_t cells = table_cells(D, B, g.max_cells);
   DimValues cs{};
   for (int d = 0; d < D; ++d) cs.v[d] = cell_sizes[d];
+  const unsigned blocks = blocks_for(n, kThreads);
+  if (!num_cells_in && n <= kClusterPoints && cells <= kClusterCells &&
+      (int64_t)B * D <= kClusterBoxes) {
+    ProfScope prof(st, "grid_cluster");
+    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.arrival, w.members, page,
+                         n <= kClusterPlacePoints};
+    int rc = TFGPC_OK;
+    TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a));
+    if (rc) return rc;
+    return a.place ? TFGPC_OK : place(st, g, points, batch_ids, w);
+  }
   if (num_cells_in) {
     ProfScope prof(st, "grid_params");
     given_cells_kernel<<<1, 32, 0, st>>>(D, num_cells_in, g.max_cells, g.num_cells, page);
@@ -273,7 +554,6 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
         g.aabb_max, g.num_cells, g.scaled_aabb_min, g.inv_cell_sizes, page));
   }
   TFGPC_LAUNCH_CHECK();
-  const unsigned blocks = blocks_for(n, kThreads);
   {
     ProfScope prof(st, "compute_keys");
     TFGPC_CUDA(cudaMemsetAsync(g.cell_start, 0, (size_t)(cells + 3) * 4, st));
@@ -288,11 +568,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   TFGPC_DIM_SWITCH(D, scatter_kernel<kD><<<blocks, kThreads, 0, st>>>(
       n, g.keys, g.num_cells, B, g.cell_start, w.arrival, w.members));
   TFGPC_LAUNCH_CHECK();
-  TFGPC_DIM_SWITCH(D, place_kernel<kD><<<blocks, kThreads, 0, st>>>(
-      n, w.members, g.keys, g.num_cells, B, g.cell_start, points, batch_ids, g.sorted_indices,
-      g.sorted_keys, g.sorted_points, g.sorted_batch_ids, (float4*)g.packed, (int2*)g.ds));
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
+  return place(st, g, points, batch_ids, w);
 }
 
 }  // namespace tfgpc

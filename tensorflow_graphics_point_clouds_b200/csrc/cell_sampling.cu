@@ -395,7 +395,6 @@ cells_sample_kernel(SampleArgs a) {
         a.page[0] = (int32_t)(uint32_t)all;
         a.page[1] = (int32_t)(all >> 32);
         a.page[2] = ok ? 0 : 1;
-        __threadfence_system();
       }
     }
   }
@@ -455,8 +454,8 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
     per_sm = v < 1 ? 1 : v;
   }
-  // a warp per 16 points, at most 4 blocks per SM and what is resident at once
-  int64_t blocks = (a.c.n + 16 * kWarps - 1) / (16 * kWarps);
+  // a warp per 8 points, at most 4 blocks per SM and what is resident at once
+  int64_t blocks = (a.c.n + 8 * kWarps - 1) / (8 * kWarps);
   const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
   if (blocks > most) blocks = most;
   if (blocks > kMaxBlocks) blocks = kMaxBlocks;

@@ -130,7 +130,6 @@ scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, Sca
       for (int i = 0; i < rep.words; ++i) rep.dst[i] = __ldcg(rep.src + i);
       rep.dst[rep.words] = (int32_t)(uint32_t)run;
       rep.dst[rep.words + 1] = (int32_t)(run >> 32);
-      __threadfence_system();
     }
   }
 }

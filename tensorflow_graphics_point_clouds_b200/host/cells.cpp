@@ -85,9 +85,12 @@ class CellGrid {
     void* p = ((void**)&g.aabb_min)[field];
     for (const Tensor& t : given)
       if (t.data_ptr() == p) return t;
-    Tensor keep = arena;
-    return at::from_blob(p, shape, [keep](void*) {}, arena.options().dtype(kFields[field].type),
-                         arena.device());
+    // (a view of the arena's storage: record_stream on it reaches the allocator)
+    int64_t elems = 1;
+    for (int64_t x : shape) elems *= x;
+    const at::ScalarType type = kFields[field].type;
+    return arena.narrow(0, (char*)p - (char*)arena.data_ptr(), elems * (int64_t)c10::elementSize(type))
+        .view(type).view(shape);
   }
 };
 

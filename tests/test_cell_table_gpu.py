@@ -1,0 +1,172 @@
+"""Grids, searches, densities and sampling on the cell table, and layers of several
+kernel MLPs, at the sizes where their kernels change form: whole numbers bit for bit
+against the CPU oracle, float results within 1e-4 of the value or the result's rms."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import pylib_ref as pr
+from tensorflow_graphics_point_clouds_b200 import mcconv, pc
+
+pytestmark = pytest.mark.gpu
+F32 = np.float32
+DEV = "cuda"
+
+
+def t(a):
+  return torch.as_tensor(np.ascontiguousarray(a)).to(DEV)
+
+
+def close(x, y, rel=1e-4):
+  x = np.asarray(x, np.float64); y = np.asarray(y, np.float64)
+  scale = np.maximum(np.abs(y), np.sqrt(np.mean(y * y)))
+  assert (np.abs(x - y) <= rel * scale + 1e-30).all()
+
+
+def same(a, b):
+  assert np.array_equal(a.cpu().numpy(), b)
+
+
+def clouds(seed, sizes, d, shuffled=True):
+  rng = np.random.default_rng(seed)
+  bid = np.repeat(np.arange(len(sizes)), sizes).astype(np.int32)
+  if shuffled:
+    rng.shuffle(bid)
+  return rng.uniform(-1, 1, (len(bid), d)).astype(F32), bid, len(sizes)
+
+
+# one cluster of 1, 2, .. 16 blocks, with the sorted copies in it (to 8192 points) and
+# without (to 65536), and the separate kernels: above that, with more than 1024 box edges
+# or a table of more than 2^21 cells
+@pytest.mark.parametrize("sizes,d,cell", [
+    ([1], 3, 0.5), ([31], 2, 0.01), ([1024], 3, 0.2), ([1000, 0, 25], 3, 0.1),
+    ([2049, 6143], 3, 0.3), ([8193], 4, 0.4), ([20000, 1, 12000], 3, 0.07), ([65536], 3, 0.1),
+    ([65537], 3, 0.1), ([7] * 341, 3, 0.9), ([7] * 342, 3, 0.9), ([300] * 40, 4, 0.6),
+    ([900] * 10, 4, 0.6)])
+@pytest.mark.parametrize("shuffled", [True, False])
+def test_grid(sizes, d, cell, shuffled):
+  pts, bid, b = clouds(11, sizes, d, shuffled)
+  ref = pr.Grid(pts, bid, b, cell)
+  g = pc.Grid(pc.PointCloud(t(pts), t(bid), b), cell)
+  assert g._cells is not None
+  same(g._num_cells, ref.num_cells)
+  same(g._aabb_min, ref.aabb_min)
+  same(g._aabb_max, ref.aabb_max)
+  same(g._scaled_aabb_min, ref.scaled_aabb_min)
+  same(g._cur_keys, ref.keys)
+  same(g._sorted_indices, ref.sorted_indices)
+  same(g._sorted_keys, ref.sorted_keys)
+  same(g._sorted_points, ref.sorted_points)
+  same(g._sorted_batch_ids, ref.sorted_batch_ids)
+  same(g.get_DS(), ref.get_ds())
+
+
+def test_grid_arrays_share_one_allocation():
+  """Arrays of a grid outlive it, and are views of storage the allocator knows."""
+  pts, bid, b = clouds(12, [500, 700], 3)
+  g = pc.Grid(pc.PointCloud(t(pts), t(bid), b), 0.2)
+  order, keys = g._sorted_indices, g._sorted_keys
+  assert order.untyped_storage().data_ptr() == keys.untyped_storage().data_ptr()
+  ref = pr.Grid(pts, bid, b, 0.2)
+  order.record_stream(torch.cuda.Stream())
+  del g
+  torch.empty(1 << 20, device=DEV).fill_(1.0)
+  same(order, ref.sorted_indices)
+  same(keys, ref.sorted_keys)
+
+
+# teams of blocks per cloud of equal, uneven and no points; more clouds than teams; every
+# dimension; cells far wider than the radius, which hold more samples than a warp keeps
+@pytest.mark.parametrize("sizes,d,cell,radius", [
+    ([1], 3, 0.5, 0.5), ([3000], 2, 0.05, 0.05), ([5000, 17, 0, 900], 3, 0.12, 0.12),
+    ([40] * 130, 3, 0.4, 0.4), ([9] * 600, 3, 0.5, 0.5), ([1500, 700], 4, 0.5, 0.5),
+    ([900, 300], 5, 0.8, 0.8), ([500, 300], 6, 1.0, 1.0), ([4000, 100], 3, 0.9, 0.15),
+    ([3000], 2, 0.7, 0.06)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_sampling(sizes, d, cell, radius, mode):
+  pts, bid, b = clouds(13, sizes, d)
+  nb_ref = pr.Neighborhood(pr.Grid(pts, bid, b, cell), radius)
+  rp, rb, ri = pr.sample(nb_ref, mode)
+  nb = pc.Neighborhood(pc.Grid(pc.PointCloud(t(pts), t(bid), b), cell), radius)
+  cloud, idx = pc.sample(nb, 'poisson' if mode == 0 else 'average')
+  same(cloud._batch_ids, rb)
+  if mode == 0:
+    same(idx, ri)
+    same(cloud._points, rp)
+  else:
+    close(cloud._points.cpu().numpy(), rp)
+
+
+# lists shorter and longer than a round of candidates, samples in and outside the boxes
+@pytest.mark.parametrize("sizes,d,radius,limit", [
+    ([2000, 1], 2, 0.3, 0), ([1500, 800], 3, 0.9, 0), ([1500, 800], 3, 0.2, 5),
+    ([33, 2000], 4, 0.6, 0), ([800], 6, 1.2, 0)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_search_and_density(sizes, d, radius, limit, mode):
+  pts, bid, b = clouds(14, sizes, d)
+  smp, sbid, _ = clouds(15, [257] * b, d)
+  smp = (1.5 * smp).astype(F32)
+  g_ref = pr.Grid(pts, bid, b, radius)
+  cloud = pc.PointCloud(t(pts), t(bid), b)
+  for own in (True, False):
+    s, sb = (pts, bid) if own else (smp, sbid)
+    ref = pr.Neighborhood(g_ref, radius, s, sb, limit)
+    nb = pc.grid_neighborhood(cloud, radius, cloud if own else pc.PointCloud(t(smp), t(sbid), b),
+                              limit)
+    same(nb._samples_neigh_ranges, ref.ranges)
+    same(nb._neighbors, ref.neighbors)
+    same(nb._original_neigh_ids, ref.original_neigh_ids)
+    close(nb.get_pdf(bandwidth=0.3, mode=mode).cpu().numpy(), ref.get_pdf(0.3, mode))
+
+
+# blocks of the weight product, channel passes side by side, few samples with long lists,
+# one pair more or less than a block of the gradient kernel
+@pytest.mark.parametrize("n_smp,cin,g,h,cout,radius,act", [
+    (1, 16, 2, 8, 16, 3.0, 'elu'), (33, 48, 4, 8, 32, 0.9, 'leaky_relu'),
+    (257, 64, 4, 16, 128, 0.4, 'elu'), (1200, 128, 1, 32, 40, 0.25, 'relu'),
+    (1200, 3, 2, 8, 16, 0.3, 'leaky_relu')])
+def test_layer_of_several_mlps(n_smp, cin, g, h, cout, radius, act):
+  pts, bid, b = clouds(16, [900, 400], 3)
+  smp, sbid, _ = clouds(17, [n_smp - n_smp // 2, n_smp // 2], 3)
+  rng = np.random.default_rng(18)
+  feat = rng.normal(size=(len(pts), cin)).astype(F32)
+  ws = [rng.normal(size=(g, 3, h)).astype(F32)]
+  bs = [(rng.normal(size=(g, 1, h)) * 0.1).astype(F32)]
+  wf = (rng.normal(size=(g, cin * h, cout // g)) * 0.05).astype(F32)
+  d_out = rng.normal(size=(n_smp, cout)).astype(F32)
+  nb_ref = pr.Neighborhood(pr.Grid(pts, bid, b, radius), radius, smp, sbid)
+  pdf = nb_ref.get_pdf(bandwidth=0.2, mode=0)
+  ref_out = pr.mcconv_layer(pts, smp, feat, nb_ref, pdf, ws, bs, wf, radius, act)
+  ref = pr.mcconv_layer_grads(pts, smp, feat, nb_ref, pdf, ws, bs, wf, radius, d_out, act)
+  layer = mcconv.MCConv(t(ws[0]), t(bs[0]), t(wf), cin, non_linearity_type=act)
+  out = layer.forward(t(feat), pc.PointCloud(t(pts), t(bid), b),
+                      pc.PointCloud(t(smp), t(sbid), b), radius)
+  dfeat, dw1, db1, dwf = layer.backward(t(d_out))
+  layer._op.check_status()
+  close(out.cpu().numpy(), ref_out)
+  close(dfeat.cpu().numpy(), ref["d_features"])
+  close(dwf.cpu().numpy(), ref["d_wf"])
+  close(dw1.cpu().numpy(), ref["d_weights"][0])
+  close(db1.cpu().numpy(), ref["d_biases"][0])
+
+
+@pytest.mark.parametrize("m", [1, 255, 257, 75777])
+@pytest.mark.parametrize("d,k", [(2, 8), (3, 16), (3, 64), (5, 32)])
+def test_kernel_basis_grads(m, d, k):
+  """Around one pair per thread, and the wave of blocks that loads ahead."""
+  rng = np.random.default_rng(m + k)
+  p_in = rng.uniform(0, 1, (50, d)).astype(F32)
+  p_out = rng.uniform(0, 1, (20, d)).astype(F32)
+  nb = np.stack([rng.integers(0, 50, m), rng.integers(0, 20, m)], 1).astype(np.int32)
+  pdf = rng.uniform(0.5, 2, m).astype(F32)
+  w, bias = rng.normal(size=(d, k)).astype(F32), rng.normal(size=k).astype(F32)
+  grads = rng.normal(size=(m, k)).astype(F32)
+  dw, db = mcconv.kernel_basis_grads(t(p_in), t(p_out), t(nb), t(pdf), t(w), t(bias), 0.5,
+                                     t(grads))
+  diff = (p_in[nb[:, 0]].astype(np.float64) - p_out[nb[:, 1]]) / 0.5
+  pre = diff @ w + bias
+  dpre = grads / pdf[:, None].astype(np.float64) * np.where(pre > 0, 1.0, 0.2)
+  # (a pair whose pre-activation rounds to the other side of 0 changes one term of the
+  # sum by 0.8 of it: of m * k terms of random sign about 1e-7 do)
+  close(dw.cpu().numpy(), diff.T @ dpre, 2e-4)
+  close(db.cpu().numpy(), dpre.sum(0), 2e-4)
