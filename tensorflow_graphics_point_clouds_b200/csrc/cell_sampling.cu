@@ -23,6 +23,12 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxBlocks = 1024;
 constexpr int kMaxTeams = kMaxBlocks / 2;
+// Cells of more points than this are left to the end of a block's pass, for all its
+// warps together: one warp with a cell of a thousand points, and a few thousand to
+// mark, keeps its whole team waiting (8 x 100 000 Gaussian-mixture points, four levels:
+// 427 -> 385 us in this kernel).
+constexpr int kCrowded = 96;
+constexpr int kMaxCrowded = 128;
 constexpr size_t kHeadBytes = (size_t)(kMaxTeams + 4) * 4;   // barrier words before the states
 constexpr unsigned long long kBarrierLimitNs = 1000000000ull;
 
@@ -139,16 +145,18 @@ __device__ __forceinline__ int2 later_points(int code, const int* cell, int batc
 }
 
 // Marks the neighbors of the taken points: the candidates of the cell, kSteps per lane
-// at a time in registers, against all of them.  own: in the cell itself too.
+// at a time in registers, against all of them.  own: in the cell itself too.  Warp
+// `part` of `parts` takes its share of the candidates.
 template <int D>
 __device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& taken,
                                                const int* cell, int batch, const int* nc,
-                                               int total, const float* inv_r, bool own) {
+                                               int total, const float* inv_r, bool own,
+                                               int part, int parts) {
   constexpr int kSteps = 4;
   constexpr int kHalves = 2 * num_tubes<D>();
   constexpr int kTop = kHalves > 16 ? 16 : kHalves > 8 ? 8 : 4;
   const int lane = lane_id();
-  if (lane < taken.count) __stcg(a.state + taken.j, (uint8_t)2);
+  if (part == 0 && lane < taken.count) __stcg(a.state + taken.j, (uint8_t)2);
   for (int half0 = 0; half0 < kHalves; half0 += 32) {
     int2 r = make_int2(0, 0);
     if (half0 + lane < kHalves)
@@ -161,7 +169,7 @@ __device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& ta
     }
     const int candidates = __shfl_sync(0xffffffffu, before, 31);
     const int offset = r.y - before;
-    for (int base = 0; base < candidates; base += 32 * kSteps) {
+    for (int base = part * 32 * kSteps; base < candidates; base += parts * 32 * kSteps) {
       float p[kSteps][D];
       int at[kSteps];
       bool hit[kSteps];
@@ -199,27 +207,37 @@ __device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& ta
 // Greedy selection in one cell.  Which of its points are taken depends on the marks of
 // earlier passes and on its own points only, so it is settled first, 32 points at a
 // time in registers; the marks of the (few) taken points follow together: the chain
-// per taken point is a ballot, not a walk over its candidates.
+// per taken point is a ballot, not a walk over its candidates.  parts > 1: all warps of
+// the block are here, every one of them selects the same points (nobody writes a state
+// meanwhile) and marks a share of their neighbors.
 template <int D>
 __device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cell, int batch,
                                              int begin, int end, const int* nc, int total,
-                                             const float* inv_r) {
+                                             const float* inv_r, int part, int parts) {
   const int lane = lane_id();
   Taken<D> taken;
   taken.count = 0;
   taken.j = -1;
 #pragma unroll
   for (int d = 0; d < D; ++d) taken.p[d] = 0.0f;
+  float p_next[D];
+  bool free_next;
+  auto load = [&](int q) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) p_next[d] = INFINITY;
+    free_next = false;
+    if (q < end) {
+      load_coords<D>(a.c, q, p_next);
+      free_next = __ldcg(a.state + q) == 0;
+    }
+  };
+  load(begin + lane);
   for (int q0 = begin; q0 < end; q0 += 32) {
-    const int q = q0 + lane;
     float p[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = INFINITY;
-    bool free = false;
-    if (q < end) {
-      load_coords<D>(a.c, q, p);
-      free = __ldcg(a.state + q) == 0;
-    }
+    for (int d = 0; d < D; ++d) p[d] = p_next[d];
+    const bool free = free_next;
+    load(q0 + 32 + lane);      // (again below if marks come in between)
     unsigned open = __ballot_sync(0xffffffffu, free);
     for (int k = 0; k < taken.count && open; ++k) {
       float s[D];
@@ -239,12 +257,17 @@ __device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cel
         taken.j = q0 + t;
       }
       if (++taken.count == 32) {
-        mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, true);
-        __syncwarp();   // these marks are visible to the next group's reads
+        if (parts > 1) __syncthreads();
+        mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, true, part, parts);
+        // these marks are visible to the next group's reads
+        if (parts > 1) __syncthreads(); else __syncwarp();
+        load(q0 + 32 + lane);
       }
     }
   }
-  if (taken.count > 0) mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, false);
+  if (parts > 1) __syncthreads();
+  if (taken.count > 0)
+    mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, false, part, parts);
 }
 
 // The team of a block: blocks [begin, begin + size) work on `cloud`; with too many clouds
@@ -290,6 +313,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 cells_sample_kernel(SampleArgs a) {
   __shared__ int warp_total[kWarps];
   __shared__ int64_t before_s;
+  __shared__ int crowded[kMaxCrowded], num_crowded[2];     // (counters of this pass and the next)
   const int lane = lane_id(), w = threadIdx.x >> 5;
   int nc[D];
 #pragma unroll
@@ -307,9 +331,12 @@ cells_sample_kernel(SampleArgs a) {
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < lead + (n - tail);
          i += (int64_t)gridDim.x * kThreads)
       a.state[i < lead ? i : tail + (i - lead)] = 2;
+    if (threadIdx.x == 0) num_crowded[0] = 0;
+    __syncthreads();
     const Team team = team_of(a.c, total);
     const int warps = team.size * kWarps;
-    const int warp = ((int)blockIdx.x - team.begin) * kWarps + w;
+    // neighboring cells go to different blocks: crowded ones come side by side
+    const int warp = w * team.size + (int)blockIdx.x - team.begin;
     unsigned* const counter = team.cloud < 0 ? a.arrived : a.arrived + 4 + team.cloud;
     for (int pass = 0; pass < (1 << D) && team.size > 0; ++pass) {
       int half[D], cells = team.cloud < 0 ? a.c.batch_size : 1;
@@ -318,25 +345,35 @@ cells_sample_kernel(SampleArgs a) {
         half[d] = (nc[d] - ((pass >> d) & 1) + 1) >> 1;
         cells *= half[d];
       }
+      int* const queued = num_crowded + (pass & 1);
+      // the i-th cell of this pass
+      auto cell_at = [&](int i, int* cell, int* batch, int* begin, int* end) {
+        int rem = i, key = 0, scale = 1;
+#pragma unroll
+        for (int d = D - 1; d >= 0; --d) {
+          cell[d] = 2 * (rem % half[d]) + ((pass >> d) & 1);
+          rem /= half[d];
+          key += cell[d] * scale;
+          scale *= nc[d];
+        }
+        *batch = team.cloud < 0 ? rem : team.cloud;
+        key += *batch * scale;
+        *begin = __ldg(a.c.start + (total - key));
+        *end = __ldg(a.c.start + (total - key) + 1);
+      };
       // a lane looks at every `warps`-th cell: crowded regions spread over the warps
       for (int c0 = 0; c0 < cells; c0 += 32 * warps) {
         const int i = c0 + lane * warps + warp;
         int cell[D], batch = 0, begin = 0, end = 0;
 #pragma unroll
         for (int d = 0; d < D; ++d) cell[d] = 0;
-        if (i < cells) {
-          int rem = i, key = 0, scale = 1;
-#pragma unroll
-          for (int d = D - 1; d >= 0; --d) {
-            cell[d] = 2 * (rem % half[d]) + ((pass >> d) & 1);
-            rem /= half[d];
-            key += cell[d] * scale;
-            scale *= nc[d];
+        if (i < cells) cell_at(i, cell, &batch, &begin, &end);
+        if (end - begin > kCrowded) {
+          const int slot = atomicAdd(queued, 1);
+          if (slot < kMaxCrowded) {
+            crowded[slot] = i;
+            end = begin;
           }
-          batch = team.cloud < 0 ? rem : team.cloud;
-          key += batch * scale;
-          begin = __ldg(a.c.start + (total - key));
-          end = __ldg(a.c.start + (total - key) + 1);
         }
         unsigned work = __ballot_sync(0xffffffffu, end > begin);
         while (work) {
@@ -347,12 +384,19 @@ cells_sample_kernel(SampleArgs a) {
           for (int d = 0; d < D; ++d) cc[d] = __shfl_sync(0xffffffffu, cell[d], who);
           poisson_cell<D>(a, cc, __shfl_sync(0xffffffffu, batch, who),
                           __shfl_sync(0xffffffffu, begin, who),
-                          __shfl_sync(0xffffffffu, end, who), nc, total, inv_r);
+                          __shfl_sync(0xffffffffu, end, who), nc, total, inv_r, 0, 1);
         }
       }
-      // (the barrier after the last pass is the one of the compaction)
-      if (pass + 1 < (1 << D))
-        ok = barrier(counter, (pass + 1) * team.size, a.arrived + 1) && ok;
+      __syncthreads();
+      const int shared_cells = min(*queued, kMaxCrowded);
+      if (threadIdx.x == 0) num_crowded[(pass + 1) & 1] = 0;
+      for (int k = 0; k < shared_cells; ++k) {
+        int cell[D], batch, begin, end;
+        cell_at(crowded[k], cell, &batch, &begin, &end);
+        poisson_cell<D>(a, cell, batch, begin, end, nc, total, inv_r, w, kWarps);
+      }
+      if (pass + 1 == (1 << D)) break;     // (the compaction begins with a barrier)
+      ok = barrier(counter, (pass + 1) * team.size, a.arrived + 1) && ok;
     }
     if (team.cloud < 0) barriers = (1 << D) - 1;
     ok = barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1) && ok;
@@ -454,7 +498,7 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
     per_sm = v < 1 ? 1 : v;
   }
-  // a warp per 8 points, at most 4 blocks per SM and what is resident at once
+  // a warp per 8 points (16: 158 against 140 us in the three-level classifier), at most 4 blocks per SM and what is resident at once
   int64_t blocks = (a.c.n + 8 * kWarps - 1) / (8 * kWarps);
   const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
   if (blocks > most) blocks = most;
