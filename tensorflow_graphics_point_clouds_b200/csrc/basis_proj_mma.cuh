@@ -22,6 +22,7 @@
 #pragma once
 
 #include "basis_proj.cuh"
+#include "list_parts.h"
 
 namespace tfgpc {
 namespace bpm {
@@ -139,10 +140,8 @@ struct Walker {
     const int64_t s = i / parts;
     const int p = (int)(i - s * parts) + 1;
     const int end = __ldg(ranges + s);
-    if (p == parts) return end;
     const int begin = s > 0 ? __ldg(ranges + s - 1) : 0;
-    const int chunks = (end - begin + kChunk - 1) / kChunk;
-    return min(end, begin + chunks * p / parts * kChunk);
+    return part_end(begin, end, p, parts, kChunk);
   }
 
   __device__ __forceinline__ void load_block(int64_t b, int& rend, int& first) const {

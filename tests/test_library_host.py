@@ -4,6 +4,7 @@ touches the device."""
 import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -91,3 +92,30 @@ def test_layer_entries_reject_bad_arguments(lib):
   rc = lib.tfgpc_mcconv_workspace_bytes(16, 128, 256, i64(100), i64(100), 1)
   assert rc > 0
   assert lib.tfgpc_global_pool_workspace_bytes(i64(32)) >= 128
+
+
+@pytest.fixture(scope="module")
+def part_end(tmp_path_factory):
+  """part_end of csrc/list_parts.h, compiled for the host."""
+  folder = tmp_path_factory.mktemp("list_parts")
+  src, so = folder / "parts.cpp", folder / "parts.so"
+  src.write_text('#include "list_parts.h"\nextern "C" int part_end(int b, int e, int p, int n, '
+                 'int c) { return tfgpc::part_end(b, e, p, n, c); }\n')
+  subprocess.run(["g++", "-O1", "-shared", "-fPIC", "-I", build.CSRC, str(src), "-o", str(so)],
+                 check=True)
+  return ctypes.CDLL(str(so)).part_end
+
+
+# lists around and far beyond the length at which chunks x parts passes 2^31, up to the
+# most pairs an entry accepts
+@pytest.mark.parametrize("begin,pairs,parts", [
+    (0, 5, 1), (7, 40, 3), (0, 7_250_000, 4736), (0, 7_300_000, 4736), (16, 9_700_000, 4736),
+    (1 << 30, (1 << 30) - 1, 4736), (0, (1 << 31) - 32, 2368), (0, (1 << 31) - 1, 4736)])
+def test_list_parts_cover_the_list(part_end, begin, pairs, parts):
+  end, chunk = begin + pairs, 16
+  ends = [begin] + [part_end(begin, end, p, parts, chunk) for p in range(1, parts + 1)]
+  assert ends[-1] == end
+  share = -(-pairs // chunk) // parts
+  for a, b in zip(ends, ends[1:]):
+    assert begin <= a <= b <= end
+    assert b == end or share * chunk <= b - a <= (share + 1) * chunk
