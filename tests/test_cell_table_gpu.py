@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from oracle import pylib_ref as pr
+from tensorflow_graphics_point_clouds_b200 import custom_ops as ops
 from tensorflow_graphics_point_clouds_b200 import mcconv, pc
 
 pytestmark = pytest.mark.gpu
@@ -186,3 +187,26 @@ def test_global_pool(n, c, mode):
     assert np.array_equal(out, ref)
   else:
     close(out, ref)
+
+
+# the density's error against 64 bits: no larger than that of the walk over the list,
+# which takes one expf per dimension
+@pytest.mark.parametrize("d,n,radius,bandwidth,mode", [
+    (3, 16384, 0.15, 0.2, 0), (4, 16384, 0.28, 0.2, 0), (3, 16384, 0.15, 0.1, 0),
+    (2, 4096, 0.1, 0.2, 0), (3, 2048, 0.3, 0.2, 1)])
+def test_density_error(d, n, radius, bandwidth, mode):
+  pts, bid, b = clouds(61, [n] * 4, d, False)
+  g = pc.Grid(pc.PointCloud(t(pts), t(bid), b), radius)
+  nb = pc.Neighborhood(g, radius)
+  inv_bw = pc._to_dims(bandwidth, d, nb._radii.device, inverse=True)
+  nb.compute_pdf(bandwidth=bandwidth, mode=mode)
+  by_list = ops.compute_pdf_with_pt_grads(g._sorted_points, nb._neighbors,
+                                          nb._samples_neigh_ranges, inv_bw, nb._inv_radii, mode)
+  bw = inv_bw.double() if mode == 0 else torch.full_like(inv_bw, np.sqrt(F32(b * n))).double()
+  p = g._sorted_points.double()
+  i, j = nb._neighbors[:, 0].long(), nb._neighbors[:, 1].long()
+  u = (p[i] - p[j]) * nb._inv_radii.double() * bw
+  terms = torch.exp(-0.5 * (u * u).sum(1)) * (bw / np.sqrt(2 * np.pi)).prod()
+  exact = torch.zeros(b * n, dtype=torch.float64, device=DEV).index_add_(0, j, terms)
+  error = lambda x: float((x.double() - exact).norm() / exact.norm())
+  assert error(nb.point_pdf()) <= 1.01 * error(by_list)
