@@ -179,6 +179,26 @@ Tensor group_plan(const Tensor& order_, const Tensor& ranges_, const Tensor& sor
   return plan;
 }
 
+// The kernels index with the layer's sizes: what they are given has to match them.
+// (weights and gradients by their number of values: they come in several shapes)
+void check_projection(int k, int c, int64_t rows, int64_t pairs, int64_t weight_elems,
+                      int64_t weight_expected, const Tensor& features) {
+  require(k > 0 && c > 0 && rows == pairs, "MCConv expects one basis row per neighbor pair");
+  require(features.dim() == 2 && features.size(1) == c,
+          "MCConv expects features with the layer's number of channels");
+  require(weight_elems == weight_expected,
+          "MCConv expects weights of the layer's basis functions, input and output features");
+}
+
+int64_t weight_elems(int k, int c, int cout, int groups, int k_src, int cout_src) {
+  return groups > 1 ? (int64_t)k * c * (cout / groups) : (int64_t)c * k_src * cout_src;
+}
+
+void check_pairs(int k, const Tensor& basis, const Tensor& neigh) {
+  require(basis.dim() == 2 && basis.size(1) == k, "MCConv expects a basis row of the layer's width");
+  require(neigh.dim() == 2 && neigh.size(1) == 2, "MCConv expects two indices per neighbor pair");
+}
+
 // groups, k_src, cout_src: how the weights lie (tfgpc_mcconv_forward_blocks)
 Tensor project_forward(int k, int c, int cout, int groups, int k_src, int cout_src,
                        const Tensor& ws, const Tensor& basis_, const Tensor& features_,
@@ -186,6 +206,9 @@ Tensor project_forward(int k, int c, int cout, int groups, int k_src, int cout_s
   Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
          weights = f32(weights_);
   const int64_t ns = ranges.size(0);
+  check_pairs(k, basis, neigh);
+  check_projection(k, c, basis.size(0), neigh.size(0), weights.numel(),
+                   weight_elems(k, c, cout, groups, k_src, cout_src), features);
   Tensor out = empty({ns, cout}, at::kFloat, basis);
   check(tfgpc_mcconv_forward_blocks(stream(), k, c, cout, groups, k_src, cout_src, ns,
                                     features.size(0), basis.size(0), fp(basis), fp(features),
@@ -200,6 +223,11 @@ py::tuple project_backward(int k, int c, int cout, int groups, int k_src, int co
                            const Tensor& out_grads_, bool reuse) {
   Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
          weights = f32(weights_), g = f32(out_grads_);
+  check_pairs(k, basis, neigh);
+  check_projection(k, c, basis.size(0), neigh.size(0), weights.numel(),
+                   weight_elems(k, c, cout, groups, k_src, cout_src), features);
+  require(g.numel() == ranges.size(0) * (groups > 1 ? cout : cout_src),
+          "MCConv expects one gradient per output feature of every sample");
   Tensor dbasis = at::empty_like(basis), dfeat = at::empty_like(features),
          dw = at::empty_like(weights);
   check(tfgpc_mcconv_backward_blocks(stream(), k, c, cout, groups, k_src, cout_src,
@@ -210,10 +238,24 @@ py::tuple project_backward(int k, int c, int cout, int groups, int k_src, int co
   return py::make_tuple(dbasis, dfeat, dw);
 }
 
+void check_group_plan(int k, int c, int cout, int64_t ns, const Tensor& pair,
+                      const Tensor& features, const Tensor& weights, const Tensor& order,
+                      const Tensor& plan) {
+  require(pair.dim() == 3 && pair.size(1) == 2 && pair.size(2) == k && pair.is_contiguous() &&
+              pair.scalar_type() == at::kBFloat16,
+          "MCConv expects the basis as bf16 pairs of the layer's width");
+  check_projection(k, c, pair.size(0), pair.size(0), weights.numel(), (int64_t)k * c * cout,
+                   features);
+  require(order.numel() == ns &&
+              (size_t)plan.numel() >= tfgpc_mcconv_group_plan_bytes(ns, pair.size(0)),
+          "MCConv expects the group plan of these samples and pairs");
+}
+
 Tensor project_forward_grouped(int k, int c, int cout, int64_t ns, const Tensor& ws,
                                const Tensor& pair, const Tensor& features_, const Tensor& weights_,
                                const Tensor& order_, const Tensor& plan) {
   Tensor features = f32(features_), weights = f32(weights_), order = i32(order_);
+  check_group_plan(k, c, cout, ns, pair, features, weights, order, plan);
   Tensor out = empty({ns, cout}, at::kFloat, features);
   check(tfgpc_mcconv_forward_grouped(stream(), k, c, cout, ns, features.size(0), pair.size(0),
                                      pair.data_ptr(), fp(features), fp(weights), ip(order),
@@ -229,6 +271,9 @@ py::tuple project_backward_grouped(int k, int c, int cout, int64_t ns, const Ten
   Tensor features = f32(features_), ranges = i32(ranges_), weights = f32(weights_),
          g = f32(out_grads_), order = i32(order_);
   const int64_t m = pair.size(0);
+  check_group_plan(k, c, cout, ns, pair, features, weights, order, plan);
+  require(g.numel() == ns * cout && ranges.size(0) == ns,
+          "MCConv expects one gradient per output feature of every sample");
   Tensor dbasis = empty({m, pair.size(2)}, at::kFloat, features);
   Tensor dfeat = at::empty_like(features), dw = at::empty_like(weights);
   check(tfgpc_mcconv_backward_grouped(stream(), k, c, cout, ns, features.size(0), m,

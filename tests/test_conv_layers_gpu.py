@@ -2,10 +2,11 @@
 NumPy restatements of pylib/pc/layers/KPConv.py and PointConv.py."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import pylib_ref as pr
-from tensorflow_graphics_point_clouds_b200 import mcconv, pc
-from test_ops_gpu import close, t, grid_pair, neigh_pair, random_cloud
+from tensorflow_graphics_point_clouds_b200 import _lib, mcconv, pc
+from test_ops_gpu import DEV, close, t, grid_pair, neigh_pair, random_cloud
 
 pytestmark = pytest.mark.gpu
 F32 = np.float32
@@ -163,3 +164,39 @@ def test_three_level_classifier_forward():
   out = net.forward(t(pts), t(bid), b, t(feat))
   assert out.shape == (b, 40)
   close(out.cpu().numpy(), ref)
+
+
+def small_layers():
+  """A layer of every form of final weights, by name: (layer, attribute of the weights)."""
+  g = torch.Generator(device=DEV).manual_seed(3)
+  rnd = lambda *s: torch.randn(s, generator=g, device=DEV)
+  one = mcconv.MCConv(rnd(1, 3, 16), rnd(1, 1, 16), rnd(1, 8 * 16, 16), 8)
+  grouped = mcconv.MCConv(rnd(1, 3, 16), rnd(1, 1, 16), rnd(1, 128 * 16, 128), 128)
+  blocks = mcconv.MCConv(rnd(2, 3, 8), rnd(2, 1, 8), rnd(2, 8 * 8, 8), 8)
+  kp = mcconv.KPConv(rnd(15, 3), rnd(8 * 15, 12), 8)
+  pconv = mcconv.PointConv(rnd(3, 16), rnd(1, 16), rnd(8 * 16, 12), [rnd(1, 16), rnd(16, 1)],
+                           [rnd(1, 16), rnd(1, 1)], 8)
+  return dict(one=one, grouped=grouped, blocks=blocks, kp=kp, pconv=pconv)
+
+
+# the kernels index with the layer's sizes: arrays of other sizes are refused
+@pytest.mark.parametrize("name", ["one", "grouped", "blocks", "kp", "pconv"])
+def test_wrong_sizes_are_refused(name):
+  layer = small_layers()[name]
+  g = torch.Generator(device=DEV).manual_seed(4)
+  pts = torch.rand((600, 3), generator=g, device=DEV)
+  cloud = pc.PointCloud(pts, torch.zeros(600, dtype=torch.int32, device=DEV), 1)
+  feat = torch.randn((600, layer.cin), generator=g, device=DEV)
+  out = layer.forward(feat, cloud, cloud, 0.2)
+  good = torch.randn(out.shape, generator=g, device=DEV)
+  layer.backward(good)
+  for bad in (good[:-1], good[:, :-1].contiguous()):
+    with pytest.raises(_lib.TfgpcError, match="gradient per output feature"):
+      layer.backward(bad)
+  with pytest.raises(_lib.TfgpcError, match="number of channels"):
+    layer.forward(feat[:, :-1].contiguous(), cloud, cloud, 0.2)
+  where = "wf" if name in ("one", "grouped", "blocks") else "weights"
+  w = getattr(layer, where)
+  setattr(layer, where, w[..., :-8, :].contiguous())
+  with pytest.raises(_lib.TfgpcError, match="expects weights"):
+    layer.forward(feat, cloud, cloud, 0.2)
