@@ -133,17 +133,21 @@ class Grid:
   a cell table (ops.CellGrid) unless the grid is too fine for one."""
 
   def __init__(self, point_cloud, cell_sizes):
-    pc = point_cloud
-    dev = pc._points.device
-    self._cell_sizes = _to_dims(cell_sizes, pc._dimension, dev)
-    cells = None
+    cells, pc = None, point_cloud
     if pc._points.shape[0] > 0:
       sizes = _host_dims(cell_sizes, pc._dimension)
       cells = _reduced_cells(pc, sizes)
       built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells)
       if built is not None:
+        self._cell_sizes = _to_dims(cell_sizes, pc._dimension, pc._points.device)
         self._adopt(pc, built[0])
         return
+    self._build_by_keys(pc, cell_sizes, cells)
+
+  def _build_by_keys(self, pc, cell_sizes, cells):
+    """Boxes, keys and radix sort one by one.  cells: see _reduced_cells."""
+    dev = pc._points.device
+    self._cell_sizes = _to_dims(cell_sizes, pc._dimension, dev)
     self._cells = None
     self._point_cloud = pc
     self._batch_size = pc._batch_size
@@ -400,18 +404,24 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
   keys (tfgpc_grid_neighborhood_count) for grids too fine for one.  For a cloud that is
   one shard of a distributed batch (num_cells_reduce set) the cell counts are reduced
   over the ranks on the device, before the main call: still one blocking read."""
-  pc = point_cloud
-  if pc._points.shape[0] == 0:
-    return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
+  if point_cloud._points.shape[0] == 0:
+    return Neighborhood(Grid(point_cloud, radius), radius, point_cloud_sample, max_neighbors)
+  sizes = _host_dims(radius, point_cloud._dimension)
+  return _grid_neighborhood(point_cloud, radius, sizes, point_cloud_sample, max_neighbors,
+                            _reduced_cells(point_cloud, sizes))
+
+
+def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cells):
+  """grid_neighborhood of a cloud with points whose counts have been reduced: whether
+  a rank's grid fits a table depends on its own share of the batch, and a second
+  reduction on some ranks only would meet another one of theirs."""
   dev = pc._points.device
   d = pc._dimension
-  sizes = _host_dims(radius, d)
   mode = 2 if point_cloud_sample is None else 1 if point_cloud_sample is pc else 0
   smp = point_cloud_sample if mode == 0 else None
   samples = dict(samples=None if smp is None else smp._points,
                  samples_batch_ids=None if smp is None else smp._batch_ids,
                  samples_are_points=mode, max_neighs=max_neighbors)
-  cells = _reduced_cells(pc, sizes)
   built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells,
                      inv_radii=_to_dims(radius, d, dev, inverse=True), **samples)
   grid = object.__new__(Grid)
@@ -430,7 +440,8 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
         max_cells = _raise_bound(pc, err, max_cells)
         if max_cells is None:
           # the separate constructors size the tube array and the sort keys exactly
-          return Neighborhood(Grid(pc, radius), radius, point_cloud_sample, max_neighbors)
+          grid._build_by_keys(pc, radius, cells)
+          return Neighborhood(grid, radius, point_cloud_sample, max_neighbors)
     grid._cells, count = None, g.pop("count")
     grid._point_cloud, grid._batch_size = pc, pc._batch_size
     grid._cur_keys, grid._fast_DS = g.pop("keys"), g.pop("ds")
@@ -477,15 +488,16 @@ class PointHierarchy:
   @staticmethod
   def _level(pc, radius, sample_mode):
     mode = SAMPLE_MODES[sample_mode.lower()]
-    built = None
-    if pc._points.shape[0] > 0:
-      dev, d = pc._points.device, pc._dimension
-      sizes = _host_dims(radius, d)
-      built = _cell_grid(pc, sizes, ops.build_cell_grid_and_sample, mode=mode,
-                         inv_radii=_to_dims(radius, d, dev, inverse=True),
-                         cells=_reduced_cells(pc, sizes))
-    if built is None:
+    if pc._points.shape[0] == 0:
       neigh = grid_neighborhood(pc, radius)
+      return (neigh,) + sample(neigh, sample_mode)
+    dev, d = pc._points.device, pc._dimension
+    sizes = _host_dims(radius, d)
+    cells = _reduced_cells(pc, sizes)
+    built = _cell_grid(pc, sizes, ops.build_cell_grid_and_sample, mode=mode,
+                       inv_radii=_to_dims(radius, d, dev, inverse=True), cells=cells)
+    if built is None:
+      neigh = _grid_neighborhood(pc, radius, sizes, None, 0, cells)
       return (neigh,) + sample(neigh, sample_mode)
     grid = object.__new__(Grid)
     grid._cell_sizes = _to_dims(radius, d, dev)

@@ -118,3 +118,86 @@ def test_bench_shards_concatenate_to_the_batch():
       assert lo == first
       assert inp[1].min() == 0 and inp[1].max() == clouds - 1
       first += len(inp[0])
+
+
+def _hierarchy_worker(rank, world, port, cells, last_empty, result_dir):
+  """One rank's PointHierarchy with the library calls replaced by stand-ins on the CPU:
+  what is under test is which reductions the rank takes part in."""
+  import datetime
+  from tensorflow_graphics_point_clouds_b200 import pc
+  os.environ["MASTER_ADDR"] = "127.0.0.1"
+  os.environ["MASTER_PORT"] = str(port)
+  dist.init_process_group("gloo", rank=rank, world_size=world,
+                          timeout=datetime.timedelta(seconds=20))
+  try:
+    begin, end = tdist.shard_clouds(17, world, rank)
+    per = 0 if last_empty and rank == world - 1 else 4
+    n = per * (end - begin)
+    calls = []
+
+    def reduce(counts):
+      calls.append(1)
+      return tdist.allreduce_max_(counts)
+
+    def built(max_cells, given):
+      asked = given["num_cells"].tolist()
+      if max(asked) > max_cells:
+        err = pc.ops._lib.TfgpcError(3, "too few cells")
+        err.num_cells = asked
+        raise err
+
+    def table_elems(d, b, max_cells):
+      return b * max_cells ** d if b * max_cells ** d <= 2 ** 24 else 0
+
+    class Count:
+      ranges, total, cells = torch.zeros(n, dtype=torch.int32), 0, None
+
+    def grid_cells(points, batch_ids, batch_size, sizes, radii):
+      return dict(num_cells=torch.full((3,), cells + rank, dtype=torch.int32),
+                  aabb_min=torch.zeros(batch_size, 3), aabb_max=torch.ones(batch_size, 3),
+                  scaled_aabb_min=torch.zeros(batch_size, 3), inv_cell_sizes=torch.ones(3))
+
+    def by_keys(points, batch_ids, batch_size, sizes, radii, max_cells, cells=None, **samples):
+      built(max_cells, cells)
+      return dict(count=Count(), keys=None, ds=None, sorted_points=points,
+                  sorted_batch_ids=batch_ids, num_cells=cells["num_cells"])
+
+    def on_table(points, batch_ids, batch_size, sizes, max_cells, cells=None, **args):
+      built(max_cells, cells)
+      return None, points[:1], batch_ids[:1], None
+
+    pc.ops.grid_cells = grid_cells
+    pc.ops.cell_table_elems = table_elems
+    pc.ops.build_cell_grid_and_sample = on_table
+    pc.ops.build_cell_grid = lambda *a, **k: on_table(*a, **k)[:2]
+    pc.ops.grid_neighborhood_count = by_keys
+    pc.ops.compute_aabb = lambda p, i, b: (torch.zeros(b, 3), torch.ones(b, 3))
+    pc.ops.compute_keys = lambda p, *rest: torch.zeros(len(p), dtype=torch.int64)
+    pc.ops.sort_keys_desc = lambda k, p, i, key_bits: (k, k, p, i)
+    pc.ops.build_grid_ds = lambda *a: None
+    pc.ops.find_neighbors_count = lambda *a, **k: Count()
+    pc.ops.read_device = lambda v: v.cpu()
+    pc.sample = lambda neigh, mode: (pc.PointCloud(torch.zeros(1, 3), torch.zeros(1), 1), None)
+
+    ids = torch.arange(end - begin, dtype=torch.int32).repeat_interleave(per)
+    cloud = pc.PointCloud(torch.rand(n, 3), ids, end - begin, num_cells_reduce=reduce)
+    hier = pc.PointHierarchy(cloud, [0.01])
+    assert len(hier._point_clouds) == 2
+    total = tdist.allreduce_sum_([torch.ones(1)])[0]
+    np.savez(os.path.join(result_dir, "rank%d.npz" % rank), calls=len(calls), total=total.numpy())
+  finally:
+    dist.destroy_process_group()
+
+
+# shards that differ by one cloud: 100 cells per dimension fit the cell table of 8 clouds
+# and not that of 9; more than 1024 cells take the constructors that size their arrays
+# exactly; a rank without points
+@pytest.mark.parametrize("cells,last_empty", [(100, False), (1500, False), (30, True)])
+def test_sharded_hierarchy_reduces_once_on_every_rank(tmp_path, cells, last_empty):
+  world, port = 2, 31000 + (os.getpid() + cells) % 2000
+  mp.start_processes(_hierarchy_worker, args=(world, port, cells, last_empty, str(tmp_path)),
+                     nprocs=world, join=True, start_method="spawn")
+  for r in range(world):
+    got = np.load(os.path.join(str(tmp_path), "rank%d.npz" % r))
+    assert int(got["calls"]) == 1
+    assert got["total"][0] == world
