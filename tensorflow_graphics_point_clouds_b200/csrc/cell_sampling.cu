@@ -15,6 +15,7 @@
 // Cell average (sampling_avg_kernels.cu.cc:43-88): one thread per occupied cell,
 // sequential fp32 sum of its points / count, cells in ascending first index.
 #include "cell_grid.cuh"
+#include "grid_barrier.cuh"
 
 namespace tfgpc {
 namespace {
@@ -46,31 +47,6 @@ struct SampleArgs {
   int32_t* index_out;          // original indices (Poisson)
   int32_t* page;               // number of samples (64 bits), then the error word
 };
-
-// Barrier over blocks of a cooperative launch (all resident) that share a counter.
-// Gives up after a second: the error word is set and every later barrier passes at once.
-__device__ __forceinline__ bool barrier(unsigned* arrived, unsigned target, unsigned* error) {
-  __shared__ bool ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(arrived, 1u);
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    ok = true;
-    while (*(volatile unsigned*)arrived < target) {
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (t - t0 > kBarrierLimitNs || *(volatile unsigned*)error != 0u) {
-        *(volatile unsigned*)error = 1u;
-        ok = false;
-        break;
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok;
-}
 
 // The points of one cell that a warp has taken and not marked the neighbors of yet:
 // lane k holds the k-th.
@@ -396,10 +372,10 @@ cells_sample_kernel(SampleArgs a) {
         poisson_cell<D>(a, cell, batch, begin, end, nc, total, inv_r, w, kWarps);
       }
       if (pass + 1 == (1 << D)) break;     // (the compaction begins with a barrier)
-      ok = barrier(counter, (pass + 1) * team.size, a.arrived + 1) && ok;
+      ok = grid_barrier(counter, (pass + 1) * team.size, a.arrived + 1, kBarrierLimitNs) && ok;
     }
     if (team.cloud < 0) barriers = (1 << D) - 1;
-    ok = barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1) && ok;
+    ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, kBarrierLimitNs) && ok;
   }
   // ---- compaction: every block counts, then writes, its stretch of the points
   const int64_t per = (n + gridDim.x - 1) / gridDim.x;
@@ -420,7 +396,8 @@ cells_sample_kernel(SampleArgs a) {
     for (int i = 0; i < kWarps; ++i) t += warp_total[i];
     __stcg(a.block_total + blockIdx.x, t);
   }
-  ok = barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1) && ok;
+  ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, kBarrierLimitNs) && ok;
+  ok = ok && !any_gave_up(a.arrived + 1);
   if (w == 0) {
     int64_t t = 0, all = 0;
     for (int i = lane; i < gridDim.x; i += 32) {
@@ -507,6 +484,29 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
   TFGPC_CUDA(cudaLaunchCooperativeKernel(cells_sample_kernel<D>, dim3((unsigned)blocks),
                                          dim3(kThreads), args, 0, st));
   return TFGPC_OK;
+}
+
+// The sampling's sequence of barriers without its work: two at the counter of a block's
+// team (even and odd blocks), two of the grid.  Block late_block comes to barrier late_at
+// after four times the limit.  words: error, barrier counters, what block 0 would report,
+// number of blocks that would return without writing.
+__global__ void barrier_probe_kernel(unsigned* words, int late_block, int late_at,
+                                     unsigned long long limit_ns) {
+  bool ok = true;
+  for (int k = 0; k < 4; ++k) {
+    if ((int)blockIdx.x == late_block && k == late_at && threadIdx.x == 0) {
+      unsigned long long t0, t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+      do { asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); } while (t - t0 < 4 * limit_ns);
+    }
+    unsigned* const counter = words + 1 + (k < 2 ? 1 + (blockIdx.x & 1) : 0);
+    const unsigned blocks = k < 2 ? gridDim.x / 2 : gridDim.x;
+    ok = grid_barrier(counter, (k % 2 + 1) * blocks, words, limit_ns) && ok;
+  }
+  ok = ok && !any_gave_up(words);
+  if (threadIdx.x != 0) return;
+  if (blockIdx.x == 0) words[4] = ok ? 0u : 1u;
+  if (!ok) atomicAdd(words + 5, 1u);
 }
 
 size_t sample_ws_bytes(int64_t n) {
@@ -627,4 +627,25 @@ extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
                     sample_indices_out, sample_ws, (int32_t*)page);
   if (rc) return rc;
   return finish_sample(st, g, num_cells_host_out, num_samples_out);
+}
+
+extern "C" int tfgpc_debug_sampling_barrier(void* stream, void* ws, size_t ws_bytes,
+                                            unsigned limit_us, int late_block, int late_at,
+                                            int* reported_out, int* gave_up_out) {
+  TFGPC_REQUIRE(ws && reported_out && gave_up_out && ws_bytes >= 256 && (uintptr_t)ws % 256 == 0,
+                "debug_sampling_barrier expects a 256-byte aligned workspace of 256 bytes");
+  TFGPC_REQUIRE(limit_us >= 1 && limit_us <= 100000,
+                "debug_sampling_barrier expects a limit between 1 us and 100 ms");
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned* words = (unsigned*)ws;
+  TFGPC_CUDA(cudaMemsetAsync(words, 0, 6 * sizeof(unsigned), st));
+  unsigned long long limit_ns = (unsigned long long)limit_us * 1000ull;
+  void* args[] = {&words, &late_block, &late_at, &limit_ns};
+  TFGPC_CUDA(cudaLaunchCooperativeKernel(barrier_probe_kernel, dim3(16), dim3(32), args, 0, st));
+  int back[6];
+  int rc = read_small(st, words, sizeof(back), back);
+  if (rc) return rc;
+  *reported_out = back[4];
+  *gave_up_out = back[5];
+  return TFGPC_OK;
 }

@@ -1,13 +1,15 @@
 """Grids, searches, densities and sampling on the cell table, and layers of several
 kernel MLPs, at the sizes where their kernels change form: whole numbers bit for bit
 against the CPU oracle, float results within 1e-4 of the value or the result's rms."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import pylib_ref as pr
 from tensorflow_graphics_point_clouds_b200 import custom_ops as ops
-from tensorflow_graphics_point_clouds_b200 import mcconv, pc
+from tensorflow_graphics_point_clouds_b200 import _lib, mcconv, pc
 
 pytestmark = pytest.mark.gpu
 F32 = np.float32
@@ -210,3 +212,17 @@ def test_density_error(d, n, radius, bandwidth, mode):
   exact = torch.zeros(b * n, dtype=torch.float64, device=DEV).index_add_(0, j, terms)
   error = lambda x: float((x.double() - exact).norm() / exact.norm())
   assert error(nb.point_pdf()) <= 1.01 * error(by_list)
+
+
+# a wait of the sampling that runs out is reported if any block left its samples
+# unwritten, whichever block was late and at whichever barrier
+@pytest.mark.parametrize("late_block,late_at", [(-1, 0), (0, 0), (0, 1), (0, 2), (0, 3), (7, 0),
+                                                (7, 3), (15, 2)])
+def test_sampling_barrier_reports(late_block, late_at):
+  ws = torch.empty(256, dtype=torch.uint8, device=DEV)
+  reported, gave_up = _lib.c_int(-1), _lib.c_int(-1)
+  _lib.check(_lib.lib().tfgpc_debug_sampling_barrier(
+      None, _lib.ptr(ws), _lib.c_sz(256), _lib.c_int(20000), _lib.c_int(late_block),
+      _lib.c_int(late_at), ctypes.byref(reported), ctypes.byref(gave_up)))
+  assert (gave_up.value > 0) == (late_block >= 0)
+  assert reported.value == (1 if gave_up.value else 0)
