@@ -788,12 +788,14 @@ int tfgpc_debug_bounded_wait(void* stream, void* ws, size_t ws_bytes,
 
 /* Exercises the barriers of the sampling kernel (tfgpc_cells_sample): 16 blocks meet
  * at four of them, block late_block (-1: none) reaches the one numbered late_at after
- * four times limit_us.  *reported_out [host]: 1 if the sampling would have returned
+ * four times limit_us, the longest wait without a sign of progress; working: it shows
+ * progress meanwhile.  *reported_out [host]: 1 if the sampling would have returned
  * TFGPC_ETIMEOUT; *gave_up_out: the number of blocks that would have left their
  * samples unwritten.  ws: 256 bytes, 256-byte aligned.  Blocks on the stream. */
 int tfgpc_debug_sampling_barrier(void* stream, void* ws, size_t ws_bytes,
                                  unsigned limit_us, int late_block, int late_at,
-                                 int* reported_out, int* gave_up_out);
+                                 int working, int* reported_out,
+                                 int* gave_up_out);
 
 /* ---- small blocking reads -------------------------------------------------
  * No counterpart in the reference (it reads its counts with cudaMemcpy behind

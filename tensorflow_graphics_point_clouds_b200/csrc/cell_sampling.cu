@@ -31,7 +31,12 @@ constexpr int kMaxTeams = kMaxBlocks / 2;
 constexpr int kCrowded = 96;
 constexpr int kMaxCrowded = 128;
 constexpr size_t kHeadBytes = (size_t)(kMaxTeams + 4) * 4;   // barrier words before the states
-constexpr unsigned long long kBarrierLimitNs = 1000000000ull;
+// Candidates of a mark loop between two signs of progress: well under a millisecond, and
+// none at all in cells of ordinary size.  A selection shows none (its loop has no register
+// left for it: spills, 1 % of a hierarchy); one over all points of a call takes some 30 ns
+// a point, which the period of the barriers allows for.
+constexpr int kProgressMarks = 65536;
+inline unsigned long long barrier_period_ns(int64_t n) { return 500000000ull + 100ull * n; }
 
 struct SampleArgs {
   CellsView c;
@@ -39,13 +44,14 @@ struct SampleArgs {
   int mode;                    // 0 Poisson disk, 1 cell average
   const float* inv_radii;
   uint8_t* state;              // [n] 0 open, 1 blocked, 2 taken (zero on entry)
-  unsigned* arrived;           // barrier counter of the grid, an error word, two words unused,
+  unsigned* arrived;           // barrier counter of the grid, error word, progress, a word unused,
                                // then the teams' counters; all zero on entry
   int32_t* block_total;        // [gridDim.x]
   float* pts_out;
   int32_t* batch_out;
   int32_t* index_out;          // original indices (Poisson)
   int32_t* page;               // number of samples (64 bits), then the error word
+  unsigned long long period_ns;
 };
 
 // The points of one cell that a warp has taken and not marked the neighbors of yet:
@@ -146,6 +152,8 @@ __device__ __forceinline__ void mark_neighbors(const SampleArgs& a, Taken<D>& ta
     const int candidates = __shfl_sync(0xffffffffu, before, 31);
     const int offset = r.y - before;
     for (int base = part * 32 * kSteps; base < candidates; base += parts * 32 * kSteps) {
+      if (base >= kProgressMarks && base % kProgressMarks < parts * 32 * kSteps && lane == 0)
+        show_progress(a.arrived + 2);
       float p[kSteps][D];
       int at[kSteps];
       bool hit[kSteps];
@@ -339,6 +347,7 @@ cells_sample_kernel(SampleArgs a) {
       };
       // a lane looks at every `warps`-th cell: crowded regions spread over the warps
       for (int c0 = 0; c0 < cells; c0 += 32 * warps) {
+        if (c0 >= 64 * 32 * warps && lane == 0) show_progress(a.arrived + 2);
         const int i = c0 + lane * warps + warp;
         int cell[D], batch = 0, begin = 0, end = 0;
 #pragma unroll
@@ -372,10 +381,12 @@ cells_sample_kernel(SampleArgs a) {
         poisson_cell<D>(a, cell, batch, begin, end, nc, total, inv_r, w, kWarps);
       }
       if (pass + 1 == (1 << D)) break;     // (the compaction begins with a barrier)
-      ok = grid_barrier(counter, (pass + 1) * team.size, a.arrived + 1, kBarrierLimitNs) && ok;
+      ok = grid_barrier(counter, (pass + 1) * team.size, a.arrived + 1, a.arrived + 2,
+                        a.period_ns) && ok;
     }
     if (team.cloud < 0) barriers = (1 << D) - 1;
-    ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, kBarrierLimitNs) && ok;
+    ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, a.arrived + 2,
+                      a.period_ns) && ok;
   }
   // ---- compaction: every block counts, then writes, its stretch of the points
   const int64_t per = (n + gridDim.x - 1) / gridDim.x;
@@ -396,7 +407,8 @@ cells_sample_kernel(SampleArgs a) {
     for (int i = 0; i < kWarps; ++i) t += warp_total[i];
     __stcg(a.block_total + blockIdx.x, t);
   }
-  ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, kBarrierLimitNs) && ok;
+  ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, a.arrived + 2,
+                    a.period_ns) && ok;
   ok = ok && !any_gave_up(a.arrived + 1);
   if (w == 0) {
     int64_t t = 0, all = 0;
@@ -488,20 +500,23 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
 
 // The sampling's sequence of barriers without its work: two at the counter of a block's
 // team (even and odd blocks), two of the grid.  Block late_block comes to barrier late_at
-// after four times the limit.  words: error, barrier counters, what block 0 would report,
-// number of blocks that would return without writing.
-__global__ void barrier_probe_kernel(unsigned* words, int late_block, int late_at,
-                                     unsigned long long limit_ns) {
+// after eight periods.  words: error, barrier counters, what block 0 would report, number
+// of blocks that would return without writing, progress.
+__global__ void barrier_probe_kernel(unsigned* words, int late_block, int late_at, int working,
+                                     unsigned long long period_ns) {
   bool ok = true;
   for (int k = 0; k < 4; ++k) {
     if ((int)blockIdx.x == late_block && k == late_at && threadIdx.x == 0) {
       unsigned long long t0, t;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-      do { asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); } while (t - t0 < 4 * limit_ns);
+      do {
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (working) show_progress(words + 6);
+      } while (t - t0 < 8 * period_ns);
     }
     unsigned* const counter = words + 1 + (k < 2 ? 1 + (blockIdx.x & 1) : 0);
     const unsigned blocks = k < 2 ? gridDim.x / 2 : gridDim.x;
-    ok = grid_barrier(counter, (k % 2 + 1) * blocks, words, limit_ns) && ok;
+    ok = grid_barrier(counter, (k % 2 + 1) * blocks, words, words + 6, period_ns) && ok;
   }
   ok = ok && !any_gave_up(words);
   if (threadIdx.x != 0) return;
@@ -529,6 +544,7 @@ int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const floa
   a.batch_out = batch_out;
   a.index_out = index_out;
   a.page = page + kReportTotal;
+  a.period_ns = barrier_period_ns(g.n);
   ProfScope prof(st, mode == 0 ? "sampling_poisson" : "sampling_cell_average");
   TFGPC_CUDA(cudaMemsetAsync(ws, 0, mode == 0 ? (size_t)g.n + kHeadBytes : kHeadBytes, st));
   switch (g.D) {
@@ -631,16 +647,16 @@ extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
 
 extern "C" int tfgpc_debug_sampling_barrier(void* stream, void* ws, size_t ws_bytes,
                                             unsigned limit_us, int late_block, int late_at,
-                                            int* reported_out, int* gave_up_out) {
+                                            int working, int* reported_out, int* gave_up_out) {
   TFGPC_REQUIRE(ws && reported_out && gave_up_out && ws_bytes >= 256 && (uintptr_t)ws % 256 == 0,
                 "debug_sampling_barrier expects a 256-byte aligned workspace of 256 bytes");
   TFGPC_REQUIRE(limit_us >= 1 && limit_us <= 100000,
                 "debug_sampling_barrier expects a limit between 1 us and 100 ms");
   cudaStream_t st = (cudaStream_t)stream;
   unsigned* words = (unsigned*)ws;
-  TFGPC_CUDA(cudaMemsetAsync(words, 0, 6 * sizeof(unsigned), st));
-  unsigned long long limit_ns = (unsigned long long)limit_us * 1000ull;
-  void* args[] = {&words, &late_block, &late_at, &limit_ns};
+  TFGPC_CUDA(cudaMemsetAsync(words, 0, 7 * sizeof(unsigned), st));
+  unsigned long long period_ns = (unsigned long long)limit_us * 500ull;
+  void* args[] = {&words, &late_block, &late_at, &working, &period_ns};
   TFGPC_CUDA(cudaLaunchCooperativeKernel(barrier_probe_kernel, dim3(16), dim3(32), args, 0, st));
   int back[6];
   int rc = read_small(st, words, sizeof(back), back);

@@ -215,14 +215,16 @@ def test_density_error(d, n, radius, bandwidth, mode):
 
 
 # a wait of the sampling that runs out is reported if any block left its samples
-# unwritten, whichever block was late and at whichever barrier
-@pytest.mark.parametrize("late_block,late_at", [(-1, 0), (0, 0), (0, 1), (0, 2), (0, 3), (7, 0),
-                                                (7, 3), (15, 2)])
-def test_sampling_barrier_reports(late_block, late_at):
+# unwritten, whichever block was late and at whichever barrier; a block that is late
+# because it works (shows progress) is waited for
+@pytest.mark.parametrize("late_block,late_at,working", [
+    (-1, 0, 0), (0, 0, 0), (0, 1, 0), (0, 2, 0), (0, 3, 0), (7, 0, 0), (7, 3, 0), (15, 2, 0),
+    (0, 1, 1), (9, 0, 1), (3, 3, 1)])
+def test_sampling_barrier_reports(late_block, late_at, working):
   ws = torch.empty(256, dtype=torch.uint8, device=DEV)
   reported, gave_up = _lib.c_int(-1), _lib.c_int(-1)
   _lib.check(_lib.lib().tfgpc_debug_sampling_barrier(
       None, _lib.ptr(ws), _lib.c_sz(256), _lib.c_int(20000), _lib.c_int(late_block),
-      _lib.c_int(late_at), ctypes.byref(reported), ctypes.byref(gave_up)))
-  assert (gave_up.value > 0) == (late_block >= 0)
+      _lib.c_int(late_at), _lib.c_int(working), ctypes.byref(reported), ctypes.byref(gave_up)))
+  assert (gave_up.value > 0) == (late_block >= 0 and not working)
   assert reported.value == (1 if gave_up.value else 0)
