@@ -140,7 +140,7 @@ class Grid:
       built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells)
       if built is not None:
         self._cell_sizes = _to_dims(cell_sizes, pc._dimension, pc._points.device)
-        self._adopt(pc, built[0])
+        self._adopt(pc, built[0], sizes)
         return
     self._build_by_keys(pc, cell_sizes, cells)
 
@@ -175,9 +175,10 @@ class Grid:
                                                   key_bits=min(64, key_bits))
     self._fast_DS = None
 
-  def _adopt(self, pc, built):
-    """Takes over a grid of ops.build_cell_grid."""
+  def _adopt(self, pc, built, sizes):
+    """Takes over a grid of ops.build_cell_grid with cells of these sizes."""
     self._cells = built
+    self._sizes = sizes
     self._point_cloud = pc
     self._batch_size = pc._batch_size
     self._fast_DS = None
@@ -427,7 +428,7 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   grid = object.__new__(Grid)
   grid._cell_sizes = _to_dims(radius, d, dev)
   if built is not None:
-    grid._adopt(pc, built[0])
+    grid._adopt(pc, built[0], sizes)
     count = built[1]
   else:
     max_cells = _MAX_CELLS.get((d, pc._batch_size), _FIRST_BOUND)
@@ -450,12 +451,27 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   return object.__new__(Neighborhood)._attach(grid, radius, point_cloud_sample, max_neighbors, count)
 
 
+# Cells up to this many radii wide are sampled from the grid, wider ones from a neighbor
+# list: a cell's taken points are marked around by one block, (taken) x (candidates) tests,
+# and a wide cell holds many of both.  From the grid / by lists, us, at 1, 3, 4, 6 and 8 radii:
+# 100 000 points 89/247, 363/1121, 1295/2134, 6364/5647, 16914/9854 (40 neighbors a point),
+# 106/286, 228/403, 717/622, 1453/1489, 5846/2980 (6); 20 000 points 79/204, 211/251,
+# 640/346, 1107/705, 2397/1340 (6).
+_SAMPLED_CELLS = 3.0
+
+
+def _cells_near_radius(neighborhood):
+  g = neighborhood._grid
+  radii = _host_dims(neighborhood._radius, g._point_cloud._dimension)
+  return all(c <= _SAMPLED_CELLS * abs(r) for c, r in zip(g._sizes, radii))
+
+
 def sample(neighborhood, sample_mode='poisson'):
   """sampling.py:123-150 -> (PointCloud of the samples, original indices or None)."""
   mode = SAMPLE_MODES[sample_mode.lower()]
   g = neighborhood._grid
   symmetric = neighborhood._equal_samples and neighborhood.max_neighbors == 0
-  if g._cells is not None and (symmetric or mode == 1):
+  if g._cells is not None and (mode == 1 or symmetric and _cells_near_radius(neighborhood)):
     # (cell averages need no neighbors, symmetric ones are found from the grid)
     pts, bids, idx = ops._lib.host().sample(g._cells, mode, neighborhood._inv_radii)
     return PointCloud(pts, bids, g._batch_size), idx
@@ -501,6 +517,6 @@ class PointHierarchy:
       return (neigh,) + sample(neigh, sample_mode)
     grid = object.__new__(Grid)
     grid._cell_sizes = _to_dims(radius, d, dev)
-    grid._adopt(pc, built[0])
+    grid._adopt(pc, built[0], sizes)
     neigh = object.__new__(Neighborhood)._attach(grid, radius, None, 0)
     return neigh, PointCloud(built[1], built[2], pc._batch_size), built[3]

@@ -228,3 +228,20 @@ def test_sampling_barrier_reports(late_block, late_at, working):
       _lib.c_int(late_at), _lib.c_int(working), ctypes.byref(reported), ctypes.byref(gave_up)))
   assert (gave_up.value > 0) == (late_block >= 0 and not working)
   assert reported.value == (1 if gave_up.value else 0)
+
+
+# a cell much wider than the radius, with many of its points taken, is sampled from the
+# neighbor list: from the grid one block marks around all of them
+@pytest.mark.parametrize("cell,radius,by_list", [(0.5, 0.03, True), (0.13, 0.04, True),
+                                                 (0.12, 0.04, False), (0.04, 0.04, False)])
+def test_sampling_of_wide_cells(cell, radius, by_list, monkeypatch):
+  pts, bid, b = clouds(71, [20000], 3)
+  calls = []
+  real = ops.sampling
+  monkeypatch.setattr(ops, "sampling", lambda *a, **k: calls.append(1) or real(*a, **k))
+  nb = pc.Neighborhood(pc.Grid(pc.PointCloud(t(pts), t(bid), b), cell), radius)
+  cloud, idx = pc.sample(nb)
+  assert bool(calls) == by_list
+  rp, rb, ri = pr.sample(pr.Neighborhood(pr.Grid(pts, bid, b, cell), radius), 0)
+  same(idx, ri)
+  same(cloud._points, rp)
