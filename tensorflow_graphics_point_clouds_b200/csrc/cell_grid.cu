@@ -37,8 +37,11 @@ __device__ __forceinline__ float unordered(unsigned k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// The cell counts asked for go to the report; the kernels index with the counts cut
-// to max_cells, which the table and the tube array were sized for.
+// The cell counts asked for go to the report.  A grid that asks for more than max_cells,
+// which the table and the tube array were sized for, gets no cells at all: the call fails
+// with the counts, and the kernels behind this one return at once (total_cells is 0).  Cut
+// to max_cells, its border cells took all points beyond them, and ranks, counts and
+// samples were worked out there (quadratic in the cell) to be thrown away.
 __device__ __forceinline__ void clip_and_report(int D, int max_cells, const int* asked,
                                                 int32_t* __restrict__ used, int32_t* page) {
   int over = 0;
@@ -46,8 +49,9 @@ __device__ __forceinline__ void clip_and_report(int D, int max_cells, const int*
     const int c = max(asked[d], 1);
     over |= c > max_cells;
     page[d] = c;
-    used[d] = min(c, max_cells);
+    used[d] = c;
   }
+  for (int d = 0; over && d < D; ++d) used[d] = 0;
   page[TFGPC_MAX_DIMS] = over;     // (read after the stream is synchronised: no fence)
 }
 
@@ -165,7 +169,7 @@ keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
   const Grid<D> g = load_grid<D>(num_cells, inv_cell);
   const int total = total_cells<D>(g.nc, batch_size);
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || total == 0) return;
   const int b = __ldg(batch_ids + i);
   const int bs = min(max(b, 0), batch_size - 1);   // (the key keeps the id that was passed in)
   float p[D], smin[D];
@@ -191,7 +195,9 @@ scatter_kernel(int64_t n, const int64_t* __restrict__ keys, const int32_t* __res
   int nc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
-  const int r = bucket_of(__ldg(keys + i), total_cells<D>(nc, batch_size));
+  const int total = total_cells<D>(nc, batch_size);
+  if (total == 0) return;
+  const int r = bucket_of(__ldg(keys + i), total);
   members[__ldg(start + r) + __ldg(arrival + i)] = (int32_t)i;
 }
 
@@ -221,6 +227,7 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
   const int total = total_cells<D>(nc, batch_size);
+  if (total == 0) return;
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (i < n) {
     const int idx = __ldg(members + i);
@@ -350,7 +357,15 @@ grid_cluster_kernel(ClusterBuild a) {
     if (c > 0.0f && c < 2147483000.0f) atomicMax(&asked[d], (int)c);
   }
   __syncthreads();
-  if (tid < D) nc_s[tid] = min(asked[tid], a.max_cells);
+  bool over = false;
+#pragma unroll
+  for (int d = 0; d < D; ++d) over = over || asked[d] > a.max_cells;
+  if (over) {                // (the same in every block)
+    if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
+    cluster.sync();          // no block leaves while others read its shared memory
+    return;
+  }
+  if (tid < D) nc_s[tid] = asked[tid];
   __syncthreads();
   Grid<D> g;
 #pragma unroll

@@ -303,6 +303,7 @@ cells_sample_kernel(SampleArgs a) {
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(a.c.num_cells + d);
   const int total = total_cells<D>(nc, a.c.batch_size);
+  if (total == 0) return;        // (a grid that got no cells: the call fails)
   const int64_t n = a.c.n;
   unsigned barriers = 0;
   bool ok = true;

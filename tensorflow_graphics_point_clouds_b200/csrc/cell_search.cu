@@ -151,6 +151,7 @@ cells_walk_kernel(WalkArgs a) {
   if (v0 >= a.ns) return;
   const Grid<D> g = load_grid<D>(c.num_cells, c.inv_cell);
   const int total = total_cells<D>(g.nc, c.batch_size);
+  if (total == 0) return;        // (a grid that got no cells: the call fails)
   f32x2 inv_r[D], scale[D], scale_lo[D];
   double norm_exact = 1.0;
   bool isotropic = true;

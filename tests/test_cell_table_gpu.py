@@ -245,3 +245,59 @@ def test_sampling_of_wide_cells(cell, radius, by_list, monkeypatch):
   rp, rb, ri = pr.sample(pr.Neighborhood(pr.Grid(pts, bid, b, cell), radius), 0)
   same(idx, ri)
   same(cloud._points, rp)
+
+
+class CellGridArrays(ctypes.Structure):
+  """tfgpc_cell_grid with arrays of its own, filled with -7."""
+  _fields_ = [("D", ctypes.c_int), ("max_cells", ctypes.c_int), ("n", ctypes.c_int64),
+              ("batch_size", ctypes.c_int64)] + [(name, ctypes.c_void_p) for name in (
+                  "aabb_min", "aabb_max", "num_cells", "scaled_aabb_min", "inv_cell_sizes", "keys",
+                  "sorted_indices", "sorted_keys", "sorted_points", "sorted_batch_ids", "packed",
+                  "cell_start", "ds")]
+
+  def __init__(self, d, max_cells, n, b):
+    table = _lib.lib().tfgpc_cell_table_elems(d, _lib.c_i64(b), max_cells)
+    f, i, l = torch.float32, torch.int32, torch.int64
+    self.arrays = dict(
+        aabb_min=(b * d, f), aabb_max=(b * d, f), num_cells=(d, i), scaled_aabb_min=(b * d, f),
+        inv_cell_sizes=(d, f), keys=(n, l), sorted_indices=(n, i), sorted_keys=(n, l),
+        sorted_points=(n * d, f), sorted_batch_ids=(n, i), packed=(4 * n, f), cell_start=(table, i),
+        ds=(2 * b * max_cells ** 2, i))
+    self.arrays = {k: torch.full((s,), -7, dtype=ty, device=DEV)
+                   for k, (s, ty) in self.arrays.items()}
+    super().__init__(d, max_cells, n, b, *[v.data_ptr() for v in self.arrays.values()])
+
+
+# a grid that asks for more cells than its arrays were sized for is not sorted, searched
+# or sampled: in one cluster (with and without the sorted copies), and in separate kernels
+@pytest.mark.parametrize("n", [3000, 20000, 70000])
+@pytest.mark.parametrize("sample", [True, False])
+def test_too_few_cells(n, sample):
+  lib, d, b, max_cells = _lib.lib(), 3, 1, 8
+  pts, bid, _ = clouds(81, [n], d)
+  pts, bid = t(pts), t(bid)
+  g = CellGridArrays(d, max_cells, n, b)
+  sizes = (ctypes.c_float * d)(0.1, 0.5, 0.5)
+  asked, total = (ctypes.c_int32 * d)(), _lib.c_i64(-1)
+  inv = torch.full((d,), 10.0, device=DEV)
+  out = [torch.full((s,), -7, dtype=ty, device=DEV)
+         for s, ty in ((3 * n, torch.float32), (n, torch.int32), (n, torch.int32))]
+  lib.tfgpc_cell_grid_workspace_bytes.restype = ctypes.c_size_t
+  need = lib.tfgpc_cell_grid_workspace_bytes(d, _lib.c_i64(n), _lib.c_i64(n), _lib.c_i64(b), max_cells)
+  need_s = lib.tfgpc_cells_sample_workspace_bytes(_lib.c_i64(n))
+  ws, ws_s = (torch.empty(k, dtype=torch.uint8, device=DEV) for k in (need, need_s))
+  stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+  head = (stream, ctypes.byref(g), _lib.ptr(pts), _lib.ptr(bid), sizes, None)
+  if sample:
+    rc = lib.tfgpc_cell_grid_sample(*head, 0, _lib.ptr(inv), *[_lib.ptr(o) for o in out],
+                                    _lib.ptr(ws), _lib.c_sz(need), _lib.ptr(ws_s),
+                                    _lib.c_sz(need_s), asked, ctypes.byref(total))
+  else:
+    rc = lib.tfgpc_cell_grid_neighborhood(*head, _lib.ptr(inv), _lib.c_i64(n), None, None, 2, 0,
+                                          _lib.ptr(out[1]), _lib.ptr(ws), _lib.c_sz(need), asked,
+                                          ctypes.byref(total))
+  assert rc == 3
+  ext = (pts.max(0).values - pts.min(0).values).cpu().numpy()
+  assert list(asked) == [int(c) for c in np.ceil(ext / np.array([0.1, 0.5, 0.5], F32))]
+  for x in [g.arrays[k] for k in ("keys", "sorted_indices", "sorted_points", "packed")] + out[::2]:
+    assert bool((x == -7).all())
