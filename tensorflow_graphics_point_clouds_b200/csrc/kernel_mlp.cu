@@ -42,7 +42,8 @@ struct MlpShape {
   int w_off[kMaxLayers];       // layer l's weights [G][h[l-1]][hp[l]] in the padded parameter block
   int b_off[kMaxLayers];       // layer l's biases [G][hp[l]]
   int params;                  // floats in the padded block
-  int rows;                    // h[0] + ... + h[L]
+  int rows;                    // of [pair] that the backward pass keeps: the inputs, and the
+                               // activations and their slopes of every layer but the last
   int widest;                  // max h[l]
   const float* w[kMaxLayers];  // [G][h[l-1]][h[l]]
   const float* b[kMaxLayers];  // [G][h[l]]
@@ -53,10 +54,11 @@ __device__ __forceinline__ float act_fwd(float x, int act, float alpha) {
   return x > 0.0f ? x : x * alpha;
 }
 
-// Slope from the activation's value (ELU: exp(x) = value + 1 below zero).
-__device__ __forceinline__ float act_slope(float value, int act, float alpha) {
-  if (value > 0.0f) return 1.0f;
-  return act == 1 ? value + 1.0f : alpha;
+// Slope at x.  (From the activation's value it would be wrong for a negative alpha, whose
+// values below zero are positive, and value + 1 loses the digits of ELU's exp(x).)
+__device__ __forceinline__ float act_slope(float x, int act, float alpha) {
+  if (x > 0.0f) return 1.0f;
+  return act == 1 ? expf(x) : alpha;
 }
 
 __device__ __forceinline__ void load_params(const MlpShape& s, float* par) {
@@ -167,7 +169,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   const int tile = blockDim.x;
   const int stride = tile + 4;                       // rows of [unit][pair], banks shifted by 4
   float* acc = par + s.params;                       // their gradients, summed over the tiles
-  float* units = acc + s.params;                     // activations of every layer
+  float* units = acc + s.params;                     // inputs, then activations and slopes
   float* grads = units + s.rows * stride;            // [2][widest][pair]
   load_params(s, par);
   for (int i = threadIdx.x; i < s.params; i += tile) acc[i] = 0.0f;
@@ -190,31 +192,40 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
       for (int d = 0; d < s.D; ++d) my_units[d * stride] = 0.0f;
     }
     for (int g = 0; g < s.G; ++g) {
+      // rows of a layer's inputs: D coordinates, else its activations and then their slopes
       int row = 0;
       for (int l = 0; l < s.L; ++l) {
-        const int next = row + s.h[l];
-        for (int q = 0; q * 8 < s.h[l + 1]; ++q) {
+        const bool last = l == s.L - 1;
+        const int ho = s.h[l + 1], next = row + (l == 0 ? s.D : 2 * s.h[l]);
+        for (int q = 0; q * 8 < ho; ++q) {
           float v[8];
           layer8(s, par, l, g, q, my_units + row * stride, stride, v);
-          const int cnt = min(8, s.h[l + 1] - 8 * q);
+          const int cnt = min(8, ho - 8 * q);
+          if (!last) {
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (e < cnt) my_units[(next + 8 * q + e) * stride] = act_fwd(v[e], act, alpha);
+            for (int e = 0; e < 8; ++e)
+              if (e < cnt) {
+                my_units[(next + 8 * q + e) * stride] = act_fwd(v[e], act, alpha);
+                my_units[(next + ho + 8 * q + e) * stride] = act_slope(v[e], act, alpha);
+              }
+          } else {
+            // gradient of the last layer's pre-activations: dbasis / pdf * slope; the
+            // density's own gradient: basis = a_L / pdf  ->  d/dpdf = -a_L / pdf^2
+            const float* gb = dbasis + m * k_total + g * hl + 8 * q;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (e < cnt) {
+                const float b = live ? __ldg(gb + e) : 0.0f;
+                grads[(8 * q + e) * stride + threadIdx.x] = b * inv_pdf * act_slope(v[e], act, alpha);
+                if (dpdf) dpdf_m -= b * act_fwd(v[e], act, alpha) * inv_pdf * inv_pdf;
+              }
+          }
         }
-        row = next;
+        if (!last) row = next;
       }
-      // gradient of the last layer's pre-activations: dbasis / pdf * slope; the density's
-      // own gradient: basis = a_L / pdf  ->  d/dpdf = -a_L / pdf^2
       int cur = 0;
-      for (int j = 0; j < hl; ++j) {
-        const float gb = live ? __ldg(dbasis + m * k_total + g * hl + j) : 0.0f;
-        const float a = my_units[(row + j) * stride];
-        grads[j * stride + threadIdx.x] = gb * inv_pdf * act_slope(a, act, alpha);
-        dpdf_m -= gb * a * inv_pdf * inv_pdf;
-      }
       for (int l = s.L - 1; l >= 0; --l) {
         const int hi = s.h[l], ho = s.h[l + 1], hp = s.hp[l + 1];
-        row -= hi;                                        // first row of the layer's inputs
         const float* gl = grads + cur * s.widest * stride;
         float* gp = grads + (cur ^ 1) * s.widest * stride;
         __syncthreads();      // the tile's gradients of this layer are complete
@@ -256,7 +267,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
               if (j + e < ho) back = fmaf(c[e * stride], wj[e], back);
           }
           if (l > 0) {
-            gp[i * stride + threadIdx.x] = back * act_slope(my_units[(row + i) * stride], act, alpha);
+            gp[i * stride + threadIdx.x] = back * my_units[(row + hi + i) * stride];
           } else {
 #pragma unroll
             for (int d = 0; d < TFGPC_MAX_DIMS; ++d)
@@ -264,6 +275,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
           }
         }
         cur ^= 1;
+        if (l > 0) row -= l == 1 ? s.D : 2 * s.h[l - 1];
       }
       __syncthreads();        // before the next MLP or tile overwrites the activations
     }
@@ -322,7 +334,7 @@ int make_shape(const char* op, int D, int G, int L, const int32_t* layer_sizes,
                   "%s expects hidden layers of 1 to %d units", op, kMaxWidth);
     s.h[l + 1] = layer_sizes[l];
     s.hp[l + 1] = (layer_sizes[l] + 7) / 8 * 8;
-    s.rows += layer_sizes[l];
+    if (l + 1 < L) s.rows += 2 * layer_sizes[l];
     if (layer_sizes[l] > s.widest) s.widest = layer_sizes[l];
     s.w_off[l] = off;
     off += G * s.h[l] * s.hp[l + 1];

@@ -305,3 +305,39 @@ def test_kernel_basis_packed_point_table(act, alpha):
   with pytest.raises(mcconv._lib.TfgpcError):
     mcconv.kernel_basis(packed[:, :2].contiguous(), p_out[:, :2].contiguous(), nbrs, None,
                         w1[:2].contiguous(), b1, 0.3, act, alpha, pdf_by_neighbor=2)
+
+
+# slopes are those at the pre-activation: for a leaky ReLU whose slope below zero is
+# negative, and for ELU far below zero, where the value has lost the digits of exp(x)
+# (layer: the one whose units lie at -8 to -14; exp there, and the sums of 2000 terms of
+# one sign, are good to 1e-6 in float32)
+@pytest.mark.parametrize("act,alpha,layer,sizes", [
+    (0, -0.3, None, [8, 16]), (0, -0.3, None, [16]), (1, 0.0, 0, [8, 16]), (1, 0.0, 1, [8, 16]),
+    (1, 0.0, 2, [5, 6, 7]), (1, 0.0, 0, [9])])
+def test_kernel_mlp_slopes(act, alpha, layer, sizes):
+  g = torch.Generator(device="cuda").manual_seed(17)
+  rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+  groups, n, m = 2, 300, 2000
+  widths = [3] + sizes
+  ws = [rnd(groups, a, b) for a, b in zip(widths, widths[1:])]
+  bs = [0.1 * rnd(groups, 1, b) for b in sizes]
+  if layer is not None:
+    ws[layer] = 0.1 * ws[layer]
+    bs[layer] = -11.0 + bs[layer]
+  p_in, p_out = rnd(n, 3), rnd(n, 3)
+  nb = torch.randint(0, n, (m, 2), generator=g, device="cuda", dtype=torch.int32)
+  nb[:, 1] = nb[:, 1].sort().values      # a sample's pairs follow one another
+  pdf = 1.0 + torch.rand(m, generator=g, device="cuda")
+  d_basis = torch.rand((m, groups * sizes[-1]), generator=g, device="cuda")
+  dws, dbs, dpin, dpout, dpdf = mcconv.kernel_mlp_grads(
+      p_in, p_out, nb, pdf, ws, bs, 1.5, d_basis, activation=act, alpha=alpha, point_grads=True)
+  leaf = [x.double().requires_grad_() for x in ws + bs + [p_in, p_out, pdf]]
+  w64, b64, (pi, po, pd) = leaf[:len(ws)], leaf[len(ws):2 * len(ws)], leaf[-3:]
+  x = ((pi[nb[:, 0].long()] - po[nb[:, 1].long()]) / 1.5).expand(groups, m, 3)
+  for w, b in zip(w64, b64):
+    x = x @ w + b
+    x = torch.where(x > 0, x, torch.expm1(x) if act == 1 else alpha * x)
+  basis = x.permute(1, 0, 2).reshape(m, -1) / pd[:, None]
+  exact = torch.autograd.grad((basis * d_basis.double()).sum(), leaf)
+  for got, ref in zip(dws + dbs + [dpin, dpout, dpdf], exact):
+    assert float((got.double() - ref).norm() / ref.norm()) < 1e-5
