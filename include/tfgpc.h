@@ -765,11 +765,12 @@ int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K,
 
 /* Conv1x1.py:97: out = x [n,cin] * weights [cin,cout] + bias [cout] (or NULL), rows of
  * out cout rounded up to a multiple of 8 apart.  Does not block: a time-out inside the
- * product is reported by the next call of this entry or of a blocking one. */
+ * product sets *status (a device int that the caller has cleared, and reads with
+ * tfgpc_mcconv_status before it uses the result); several products may share one. */
 size_t tfgpc_linear_workspace_bytes(int64_t n, int64_t cin, int64_t cout);
 int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t cout,
                      const float* x, const float* weights, const float* bias,
-                     float* out, void* ws, size_t ws_bytes);
+                     float* out, int* status, void* ws, size_t ws_bytes);
 
 /* ---- bounded-wait self test -------------------------------------------------
  * No counterpart in the reference (its kernels have no device-side waits).

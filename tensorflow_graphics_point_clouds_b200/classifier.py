@@ -52,12 +52,13 @@ class SmallClassifier:
     hier = pc.PointHierarchy(cloud, self.radii, 'poisson')
     clouds = hier._point_clouds
     x = features
+    status = mcconv.product_status(x.device)
     last = len(self.convs) - 1
     for i, conv in enumerate(self.convs):
       x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], keep_for_backward=False)
       if i < last:
         x = self._bn_act(x)
-        x = mcconv.conv1x1(x, *self.conv1x1[i])
+        x = mcconv.conv1x1(x, *self.conv1x1[i], status=status)
         x = self._bn_act(x)
     # return_sorted=True of the last convolution (modelnet40_small.py:249-254):
     # rows in ascending batch id; the last radius leaves one point per cloud
@@ -68,5 +69,7 @@ class SmallClassifier:
       x = x[order].contiguous()
     x = self._bn_act(x)
     for w, b in self.dense[:-1]:
-      x = self._bn_act(mcconv.conv1x1(x, w, b))
-    return mcconv.conv1x1(x, *self.dense[-1])
+      x = self._bn_act(mcconv.conv1x1(x, w, b, status))
+    x = mcconv.conv1x1(x, *self.dense[-1], status=status)
+    mcconv.check_product_status(status)
+    return x

@@ -76,12 +76,6 @@ int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_ds
 int report_page(void** dev_page);
 int read_report(cudaStream_t st, size_t bytes, void* host_dst);
 
-// A status word in that page for entries that do not block: a kernel whose bounded wait
-// runs out sets it, and the next entry of this thread that looks at it fails with
-// TFGPC_ETIMEOUT.
-int deferred_error_word(int** dev_word);
-int take_deferred_error();
-
 inline unsigned blocks_for(int64_t work, int per_block) {
   int64_t b = (work + per_block - 1) / per_block;
   return (unsigned)(b < 1 ? 1 : b);

@@ -566,28 +566,22 @@ inline int64_t up8(int64_t v) { return (v + 7) / 8 * 8; }
 
 extern "C" size_t tfgpc_linear_workspace_bytes(int64_t n, int64_t cin, int64_t cout) {
   if (n <= 0 || cin <= 0 || cout <= 0) return 1024;
-  return 1024 + 2 * align_up((size_t)n * up8(cin) * 2, 1024) +
+  return 2 * align_up((size_t)n * up8(cin) * 2, 1024) +
          2 * align_up((size_t)cin * up8(cout) * 2, 1024);
 }
 
 extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t cout, const float* x,
-                                const float* weights, const float* bias, float* out, void* ws,
-                                size_t ws_bytes) {
-  TFGPC_REQUIRE(n >= 0 && cin > 0 && cout > 0 && cin < (1 << 30) && cout < (1 << 30),
+                                const float* weights, const float* bias, float* out, int* status,
+                                void* ws, size_t ws_bytes) {
+  TFGPC_REQUIRE(n > 0 && cin > 0 && cout > 0 && cin < (1 << 30) && cout < (1 << 30),
                 "Conv1x1 expects positive sizes");
-  int rc = take_deferred_error();
-  if (rc) return rc;
-  if (n == 0) return TFGPC_OK;
-  TFGPC_REQUIRE(x && weights && out && ws, "Conv1x1 got a null pointer");
+  TFGPC_REQUIRE(x && weights && out && status && ws, "Conv1x1 got a null pointer");
   TFGPC_REQUIRE((uintptr_t)ws % 256 == 0 && (uintptr_t)out % 16 == 0,
                 "Conv1x1 expects a 256-byte aligned workspace and a 16-byte aligned output");
   if (ws_bytes < tfgpc_linear_workspace_bytes(n, cin, cout))
     return fail(TFGPC_ENOMEM, "Conv1x1 workspace too small");
-  int* err = nullptr;
-  rc = deferred_error_word(&err);
-  if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  char* p = (char*)ws + 1024;
+  char* p = (char*)ws;
   auto take = [&](size_t b) { char* r = p; p += align_up(b, 1024); return (__nv_bfloat16*)r; };
   SplitJob jx, jw;
   jx.x = x;
@@ -602,7 +596,7 @@ extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t co
   jw.ld = (int)up8(cout);
   jw.hi = take((size_t)cin * jw.ld * 2);
   jw.mid = take((size_t)cin * jw.ld * 2);
-  rc = split_rows(st, jx, &jw);
+  int rc = split_rows(st, jx, &jw);
   if (rc) return rc;
   const GemmOperand xo{jx.hi, jx.mid, jx.ld, Major::K}, wo{jw.hi, jw.mid, jw.ld, Major::MN};
   GemmProblem g{};
@@ -615,5 +609,5 @@ extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t co
   g.c = out;
   g.ldc = up8(cout);
   g.bias = bias;
-  return gemm_bf16x3(st, g, err);
+  return gemm_bf16x3(st, g, status);
 }

@@ -70,7 +70,7 @@ int sm_count() {
 // first use and kept.
 namespace {
 
-constexpr size_t kPageBytes = 4096 + 64;    // the values read, then the deferred error word
+constexpr size_t kPageBytes = 4096;
 struct Mailbox { void* host; void* dev; };
 thread_local Mailbox g_mail[64] = {};
 
@@ -89,7 +89,6 @@ static int mailbox_of(Mailbox** out) {
   if (!m.host) {
     TFGPC_CUDA(cudaHostAlloc(&m.host, kPageBytes, cudaHostAllocMapped));
     TFGPC_CUDA(cudaHostGetDevicePointer(&m.dev, m.host, 0));
-    memset(m.host, 0, kPageBytes);
   }
   *out = &m;
   return TFGPC_OK;
@@ -109,25 +108,7 @@ int read_report(cudaStream_t st, size_t bytes, void* host_dst) {
   if (rc) return rc;
   TFGPC_CUDA(cudaStreamSynchronize(st));
   memcpy(host_dst, m->host, bytes);
-  return take_deferred_error();
-}
-
-int deferred_error_word(int** dev_word) {
-  Mailbox* m = nullptr;
-  int rc = mailbox_of(&m);
-  if (rc) return rc;
-  *dev_word = (int*)((char*)m->dev + 4096);
   return TFGPC_OK;
-}
-
-int take_deferred_error() {
-  Mailbox* m = nullptr;
-  int rc = mailbox_of(&m);
-  if (rc) return rc;
-  volatile int* word = (volatile int*)((char*)m->host + 4096);
-  if (*word == 0) return TFGPC_OK;
-  *word = 0;
-  return fail(TFGPC_ETIMEOUT, "a bounded wait inside an earlier tensor-core product ran out");
 }
 
 int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_dst) {
@@ -151,7 +132,8 @@ extern "C" int tfgpc_read_device(void* stream, const void* device_src, size_t by
 }
 
 extern "C" const char* tfgpc_last_error(void) { return tfgpc::g_err; }
-extern "C" int tfgpc_version(void) { return 2; }   // 2: pdf_by_neighbor on the kernel-basis entries
+// 2: pdf_by_neighbor on the kernel-basis entries; 3: status word of tfgpc_linear_f32
+extern "C" int tfgpc_version(void) { return 3; }
 
 extern "C" int tfgpc_profile_enable(int on) {
   tfgpc::g_prof_on = on != 0;

@@ -283,7 +283,7 @@ py::tuple project_backward_grouped(int k, int c, int cout, int64_t ns, const Ten
   return py::make_tuple(dbasis, dfeat, dw);
 }
 
-// Status word of a projection or product workspace; blocks on the stream.
+// Status word of a product, or of the workspace that begins with it; blocks on the stream.
 void check_status(const Tensor& ws) {
   int status = 0, rc;
   void* st = stream();
@@ -376,17 +376,21 @@ Tensor global_pool(const Tensor& features_, const Tensor& ids_, int64_t batch, i
 }
 
 // x [N, C_in] @ weights [C_in, C_out] + bias; C_out that is not a multiple of 8 comes
-// back as the front columns of a wider array
-Tensor linear(const Tensor& x_, const Tensor& weights_, const Tensor& bias_) {
+// back as the front columns of a wider array.  status: an int32 that check_status reads
+// before the result is used.
+Tensor linear(const Tensor& x_, const Tensor& weights_, const Tensor& bias_,
+              const Tensor& status) {
   Tensor x = f32(x_), weights = f32(weights_), bias = f32(bias_);
   const int64_t n = x.size(0), cin = x.size(1), cout = weights.size(1);
   require(weights.size(0) == cin, "matmul expects matching inner dimensions");
   require(bias.numel() == cout, "Conv1x1 expects one bias per output feature");
+  require(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1,
+          "Conv1x1 expects an int32 status word on the GPU");
   Tensor out = empty({n, (cout + 7) / 8 * 8}, at::kFloat, x);
   const size_t need = tfgpc_linear_workspace_bytes(n, cin, cout);
   Tensor ws = bytes(need, x);
   check(tfgpc_linear_f32(stream(), n, cin, cout, fp(x), fp(weights), fp(bias), fpm(out),
-                         ws.data_ptr(), need));
+                         ipm(status), ws.data_ptr(), need));
   return out.size(1) == cout ? out : out.narrow(1, 0, cout);
 }
 

@@ -511,11 +511,27 @@ def global_pool(features, point_cloud, mode='max'):
                                  POOL_MODES[mode])
 
 
-def conv1x1(features, weights, bias):
+def conv1x1(features, weights, bias, status=None):
   """Conv1x1.py:97: features [N, C_in] @ weights [C_in, C_out] + bias [1, C_out].
-  The product and the bias run on the tensor cores as one call
-  (tfgpc_linear_f32)."""
-  return _lib.host().linear(features, weights, bias)
+  The product and the bias run on the tensor cores as one call (tfgpc_linear_f32).
+  Blocks, and raises TfgpcError(4) if a wait inside the product ran out; with status
+  (product_status(), shared by several products) that is left to one
+  check_product_status at their end."""
+  own = product_status(features.device) if status is None else status
+  out = _lib.host().linear(features, weights, bias, own)
+  if status is None:
+    check_product_status(own)
+  return out
+
+
+def product_status(device):
+  """A cleared status word for conv1x1."""
+  return torch.zeros(1, dtype=torch.int32, device=device)
+
+
+def check_product_status(status):
+  """Blocks on the stream; raises TfgpcError(4) if a wait of a product ran out."""
+  _lib.host().check_status(status)
 
 
 def scale_bias_activation_(x, scale=1.0, bias=None, leaky_alpha=None):

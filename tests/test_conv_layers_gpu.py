@@ -1,5 +1,7 @@
 """KPConv and PointConv on the projection + weight-product path against the
 NumPy restatements of pylib/pc/layers/KPConv.py and PointConv.py."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -200,3 +202,48 @@ def test_wrong_sizes_are_refused(name):
   setattr(layer, where, w[..., :-8, :].contiguous())
   with pytest.raises(_lib.TfgpcError, match="expects weights"):
     layer.forward(feat, cloud, cloud, 0.2)
+
+
+def test_product_that_ran_out_is_reported(monkeypatch):
+  """A wait of a product that runs out is raised by the call whose result it spoils, and
+  by no other: by conv1x1 itself, by the classifier for any of its products."""
+  from tensorflow_graphics_point_clouds_b200 import classifier, synthetic
+  host = _lib.host()
+  real, spoil, seen = host.linear, [], []
+
+  def linear(x, weights, bias, status):
+    out = real(x, weights, bias, status)
+    if len(seen) in spoil:
+      # what the bounded wait of a product does when it runs out (after 1 ms)
+      ws = torch.zeros(1024, dtype=torch.uint8, device=DEV)
+      returned = _lib.c_int(0)
+      stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+      _lib.check(_lib.lib().tfgpc_debug_bounded_wait(stream, _lib.ptr(ws), _lib.c_sz(1024), 1000,
+                                                     ctypes.byref(returned)))
+      status.copy_(ws[:4].view(torch.int32))
+    seen.append(1)
+    return out
+
+  monkeypatch.setattr(host, "linear", linear)
+  x, w, b = torch.randn(100, 16, device=DEV), torch.randn(16, 24, device=DEV), torch.randn(24, device=DEV)
+  good = mcconv.conv1x1(x, w, b)
+  del seen[:]
+  spoil[:] = [0]
+  with pytest.raises(_lib.TfgpcError, match="ran out"):
+    mcconv.conv1x1(x, w, b)
+  assert torch.equal(mcconv.conv1x1(x, w, b), good)
+  preset = classifier.PRESETS["script"]
+  pts, ids = synthetic.unit_sphere_shapes(2, 256, 5)
+  weights = synthetic.small_classifier_weights(5, preset["feature_sizes"],
+                                               head_layers=preset["head_layers"])
+  net = classifier.SmallClassifier(weights, preset["radii"], torch.device(DEV),
+                                   preset["pool_before_head"])
+  run = lambda: net.forward(t(pts), t(ids), 2, torch.ones((len(pts), 1), device=DEV))
+  spoil[:] = []
+  del seen[:]
+  run()
+  for at in range(len(seen)):
+    del seen[:]
+    spoil[:] = [at]
+    with pytest.raises(_lib.TfgpcError, match="ran out"):
+      run()
