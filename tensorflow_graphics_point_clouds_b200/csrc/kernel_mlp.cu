@@ -38,7 +38,8 @@ constexpr size_t kMaxMlpSmem = 227 * 1024;
 struct MlpShape {
   int D, G, L;
   int h[kMaxLayers + 1];       // h[0] = D, h[l] = width of layer l
-  int hp[kMaxLayers + 1];      // the same rounded up to 8 (l > 0)
+  int hp[kMaxLayers + 1];      // the same rounded up to 8 (l > 0) if wide, else as they are
+  bool wide;                   // parameters are read eight at a time
   int w_off[kMaxLayers];       // layer l's weights [G][h[l-1]][hp[l]] in the padded parameter block
   int b_off[kMaxLayers];       // layer l's biases [G][hp[l]]
   int params;                  // floats in the padded block
@@ -80,6 +81,16 @@ __device__ __forceinline__ void load_params(const MlpShape& s, float* par) {
 __device__ __forceinline__ void layer8(const MlpShape& s, const float* par, int l, int g, int q,
                                        const float* in, int stride, float* acc) {
   const int hi = s.h[l], hp = s.hp[l + 1];
+  if (!s.wide) {
+    const float* w = par + s.w_off[l] + g * hi * hp + 8 * q;
+    const float* b = par + s.b_off[l] + g * hp + 8 * q;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      acc[e] = 8 * q + e < hp ? b[e] : 0.0f;
+      for (int i = 0; i < hi && 8 * q + e < hp; ++i) acc[e] = fmaf(in[i * stride], w[i * hp + e], acc[e]);
+    }
+    return;
+  }
   const float4* bb = reinterpret_cast<const float4*>(par + s.b_off[l] + g * hp) + 2 * q;
   const float4* ww = reinterpret_cast<const float4*>(par + s.w_off[l] + g * hi * hp) + 2 * q;
   float4 b0 = bb[0], b1 = bb[1];
@@ -117,6 +128,7 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   load_params(s, par);
   __syncthreads();
   const int hl = s.h[s.L], k_total = s.G * hl;
+  const bool quads = hl % 4 == 0 && (uintptr_t)basis % 16 == 0;
   for (int64_t m = (int64_t)blockIdx.x * stride + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * stride) {
     const int2 nb = __ldg(neigh + m);
@@ -138,7 +150,7 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               if (e < cnt) out[(8 * q + e) * stride] = acc[e];
-          } else if (hl % 4 == 0) {
+          } else if (quads) {
 #pragma unroll
             for (int e = 0; e < 8; e += 4)
               if (e < cnt)
@@ -257,10 +269,12 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
         const float* w = par + s.w_off[l] + g * hi * hp;
         for (int i = 0; i < hi; ++i) {
           float back = 0.0f;
-          for (int j = 0; j < ho; j += 8) {
+          const float* col = gl + threadIdx.x;
+          for (int j = 0; j < ho && !s.wide; ++j) back = fmaf(col[j * stride], w[i * hp + j], back);
+          for (int j = 0; j < ho && s.wide; j += 8) {
             const float4 w0 = *reinterpret_cast<const float4*>(w + i * hp + j);
             const float4 w1 = *reinterpret_cast<const float4*>(w + i * hp + j + 4);
-            const float* c = gl + j * stride + threadIdx.x;
+            const float* c = col + j * stride;
             const float wj[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e)
@@ -319,6 +333,29 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   }
 }
 
+// Shared memory of a tile of `pairs` pairs.
+size_t mlp_smem(const MlpShape& s, int pairs, bool backward) {
+  const size_t f = backward ? 2 * (size_t)s.params + (size_t)(s.rows + 2 * s.widest) * (pairs + 4)
+                            : (size_t)s.params + (size_t)(s.D + 2 * s.widest) * pairs;
+  return f * sizeof(float);
+}
+
+// Where the parameters of the layers lie in shared memory.
+void place_params(MlpShape* s, bool wide) {
+  s->wide = wide;
+  int off = 0;
+  for (int l = 0; l < s->L; ++l) {
+    s->hp[l + 1] = wide ? (s->h[l + 1] + 7) / 8 * 8 : s->h[l + 1];
+    s->w_off[l] = off;
+    off += s->G * s->h[l] * s->hp[l + 1];
+  }
+  for (int l = 0; l < s->L; ++l) {
+    s->b_off[l] = off;
+    off += s->G * s->hp[l + 1];
+  }
+  s->params = wide ? off : (off + 3) / 4 * 4;   // (what follows is read in quads)
+}
+
 int make_shape(const char* op, int D, int G, int L, const int32_t* layer_sizes,
                const float* const* weights, const float* const* biases, MlpShape* out,
                int* num_weights, int* num_biases) {
@@ -328,39 +365,27 @@ int make_shape(const char* op, int D, int G, int L, const int32_t* layer_sizes,
   MlpShape s{};
   s.D = D; s.G = G; s.L = L; s.h[0] = s.hp[0] = D;
   s.rows = s.widest = D;
-  int off = 0, nw = 0, nb = 0;
+  int nw = 0, nb = 0;
   for (int l = 0; l < L; ++l) {
     TFGPC_REQUIRE(layer_sizes[l] >= 1 && layer_sizes[l] <= kMaxWidth,
                   "%s expects hidden layers of 1 to %d units", op, kMaxWidth);
     s.h[l + 1] = layer_sizes[l];
-    s.hp[l + 1] = (layer_sizes[l] + 7) / 8 * 8;
     if (l + 1 < L) s.rows += 2 * layer_sizes[l];
     if (layer_sizes[l] > s.widest) s.widest = layer_sizes[l];
-    s.w_off[l] = off;
-    off += G * s.h[l] * s.hp[l + 1];
     nw += G * s.h[l] * s.h[l + 1];
     nb += G * s.h[l + 1];
     s.w[l] = weights ? weights[l] : nullptr;
     s.b[l] = biases ? biases[l] : nullptr;
   }
-  for (int l = 0; l < L; ++l) {
-    s.b_off[l] = off;
-    off += G * s.hp[l + 1];
-  }
-  s.params = off;
   TFGPC_REQUIRE(nw + nb <= kMaxParams, "%s: the kernel MLPs hold %d parameters, at most %d are supported",
                 op, nw + nb, kMaxParams);
+  // a thousand MLPs of a unit or two do not fit with their rows padded to eight
+  place_params(&s, true);
+  if (mlp_smem(s, 32, true) > kMaxMlpSmem) place_params(&s, false);
   *out = s;
   *num_weights = nw;
   *num_biases = nb;
   return TFGPC_OK;
-}
-
-// Shared memory of a tile of `pairs` pairs.
-size_t mlp_smem(const MlpShape& s, int pairs, bool backward) {
-  const size_t f = backward ? 2 * (size_t)s.params + (size_t)(s.rows + 2 * s.widest) * (pairs + 4)
-                            : (size_t)s.params + (size_t)(s.D + 2 * s.widest) * pairs;
-  return f * sizeof(float);
 }
 
 // Pairs per tile: 128, fewer for MLPs so wide that they would not fit.
@@ -423,7 +448,6 @@ extern "C" int tfgpc_kernel_mlp_basis_layers(
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_out,
                 "KernelMlpBasis got a null pointer");
-  TFGPC_REQUIRE((uintptr_t)basis_out % 16 == 0, "KernelMlpBasis expects a 16-byte aligned output");
   cudaStream_t st = (cudaStream_t)stream;
   const int tile = mlp_tile(s, false);
   const size_t smem = mlp_smem(s, tile, false);

@@ -315,9 +315,20 @@ def test_kernel_basis_packed_point_table(act, alpha):
     (0, -0.3, None, [8, 16]), (0, -0.3, None, [16]), (1, 0.0, 0, [8, 16]), (1, 0.0, 1, [8, 16]),
     (1, 0.0, 2, [5, 6, 7]), (1, 0.0, 0, [9])])
 def test_kernel_mlp_slopes(act, alpha, layer, sizes):
+  check_kernel_mlp(2, 2000, act, alpha, layer, sizes)
+
+
+# parameters that fit shared memory only as they are, not with rows of eight
+@pytest.mark.parametrize("groups,sizes", [(2000, [1]), (640, [1, 1]), (300, [3, 3])])
+def test_many_small_kernel_mlps(groups, sizes):
+  check_kernel_mlp(groups, 300, 1, 0.0, None, sizes)
+
+
+def check_kernel_mlp(groups, m, act, alpha, layer, sizes):
+  """Basis and all gradients of a kernel MLP against float64 autograd."""
   g = torch.Generator(device="cuda").manual_seed(17)
   rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
-  groups, n, m = 2, 300, 2000
+  n = 300
   widths = [3] + sizes
   ws = [rnd(groups, a, b) for a, b in zip(widths, widths[1:])]
   bs = [0.1 * rnd(groups, 1, b) for b in sizes]
@@ -339,5 +350,8 @@ def test_kernel_mlp_slopes(act, alpha, layer, sizes):
     x = torch.where(x > 0, x, torch.expm1(x) if act == 1 else alpha * x)
   basis = x.permute(1, 0, 2).reshape(m, -1) / pd[:, None]
   exact = torch.autograd.grad((basis * d_basis.double()).sum(), leaf)
+  got = mcconv.kernel_mlp_basis(p_in, p_out, nb, pdf, ws, bs, 1.5, activation=act, alpha=alpha)
+  basis = basis.detach()
+  assert float((got.double() - basis).norm() / basis.norm()) < 1e-5
   for got, ref in zip(dws + dbs + [dpin, dpout, dpdf], exact):
     assert float((got.double() - ref).norm() / ref.norm()) < 1e-5
