@@ -88,6 +88,7 @@ struct TileSchedule {
   int k_blocks;         // ring slots over the whole reduction
   int k_blocks_per_split;
   int add_slices;       // 1: every slice of the reduction is added into the one output
+  int slice_batches;    // > 0: slice s of batch b goes to matrix s * slice_batches + b of C
 };
 
 struct Barriers {
@@ -360,7 +361,7 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
           if (sch.add_slices)
             tma_reduce_add_3d(&tm_c, smem_u32(box), x, y, bt);
           else
-            tma_store_3d(&tm_c, smem_u32(box), x, y, bt);
+            tma_store_3d(&tm_c, smem_u32(box), x, y, bt + sp * sch.slice_batches);
         }
       }
       tc_fence_before();
@@ -472,6 +473,7 @@ TileSchedule schedule(int64_t M, int64_t N, int64_t K, int batches, int bn, int 
   // drop empty trailing slices
   sch.k_splits = (sch.k_blocks + sch.k_blocks_per_split - 1) / sch.k_blocks_per_split;
   sch.add_slices = sch.k_splits > 1 ? 1 : 0;
+  sch.slice_batches = 0;
   return sch;
 }
 
@@ -572,6 +574,33 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitJobs jobs) {
   *reinterpret_cast<uint2*>(j.mid + (int64_t)r * j.ld + c) = m;
 }
 
+// out = the sum of `slices` slices, one after the other (and the bias, [cols] or
+// null), four values per thread.
+__global__ void __launch_bounds__(256)
+sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, int64_t rows,
+                  int cols, const float* __restrict__ bias, float* __restrict__ out, int64_t ldc,
+                  int64_t c_batch_stride) {
+  const int quads = cols / 4;
+  const int64_t per_slice = (int64_t)batches * rows * quads;
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= per_slice) return;
+  const float4* src = reinterpret_cast<const float4*>(partials) + i;
+  float4 v = __ldg(src);
+#pragma unroll 4
+  for (int s = 1; s < slices; ++s) {
+    const float4 t = __ldg(src + (int64_t)s * per_slice);
+    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+  }
+  const int64_t r = i / quads;
+  const int c = (int)(i - r * quads) * 4;
+  if (bias) {
+    v.x += __ldg(bias + c); v.y += __ldg(bias + c + 1);
+    v.z += __ldg(bias + c + 2); v.w += __ldg(bias + c + 3);
+  }
+  const int64_t b = r / rows;
+  *reinterpret_cast<float4*>(out + b * c_batch_stride + (r - b * rows) * ldc + c) = v;
+}
+
 // hi_t, mid_t [cols, rows] = the split of the transpose of x, whose rows and columns are
 // padded with zeros as in split_rows_kernel.
 __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows, int64_t cols,
@@ -624,6 +653,14 @@ static int pick_k_splits(int64_t tiles, int64_t K) {
   return (int)(splits < 1 ? 1 : splits);
 }
 
+int64_t gemm_partial_elems(int64_t M, int64_t N, int64_t K, bool b_mn) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int bn = tile_columns(N, b_mn);
+  const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
+  const int splits = schedule(M, N, K, 1, bn, pick_k_splits(tiles, K)).k_splits;
+  return splits > 2 ? splits * M * N : 0;
+}
+
 int gemm_bf16x3_grad_image_tn(cudaStream_t stream, int channels, int64_t N, int64_t K,
                               const GemmOperand& a, const GemmOperand& b, void* image, int group,
                               int* err_flag) {
@@ -672,8 +709,18 @@ int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
   int rc = operand_maps(maps, p.a, p.b, p.M, p.N, p.K, p.batches, bn);
   if (rc) return rc;
   const int64_t tiles = ((p.M + kBM - 1) / kBM) * ((p.N + bn - 1) / bn) * p.batches;
-  const TileSchedule sch = schedule(p.M, p.N, p.K, p.batches, bn, pick_k_splits(tiles, p.K));
   const int64_t rows = p.transposed ? p.N : p.M, cols = p.transposed ? p.M : p.N;
+  int splits = pick_k_splits(tiles, p.K);
+  if (p.ordered && splits > 2) {
+    const int64_t room = cols % 4 == 0 ? p.partial_elems / (rows * cols * p.batches) : 0;
+    splits = (int)(room > 2 ? (room < splits ? room : splits) : 2);
+  }
+  TileSchedule sch = schedule(p.M, p.N, p.K, p.batches, bn, splits);
+  const bool apart = p.ordered && sch.k_splits > 2;
+  if (apart) {
+    sch.add_slices = 0;
+    sch.slice_batches = p.batches;
+  }
   if (sch.add_slices) {
     // the slices are added into c, which starts from zero, by the store unit (the order
     // of the additions, and with it the last bits of the sums, varies from run to run)
@@ -688,14 +735,27 @@ int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
                                      sizeof(float) * (size_t)cols, (size_t)rows, stream));
     }
   }
-  rc = make_map_c(&maps[4], p.c, cols, rows, p.batches, p.ldc, p.c_batch_stride);
+  rc = apart ? make_map_c(&maps[4], p.partials, cols, rows, sch.k_splits * p.batches, cols,
+                          rows * cols)
+             : make_map_c(&maps[4], p.c, cols, rows, p.batches, p.ldc, p.c_batch_stride);
   if (rc) return rc;
+  const float* bias = apart ? nullptr : p.bias;
   if (p.transposed)
-    return launch<true, false, 2>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
-  if (a_mn && b_mn) return launch<true, true>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
-  if (a_mn) return launch<true, false>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
-  if (b_mn) return launch<false, true>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
-  return launch<false, false>(stream, maps, p.M, p.N, bn, sch, err_flag, p.bias);
+    rc = launch<true, false, 2>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
+  else if (a_mn && b_mn)
+    rc = launch<true, true>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
+  else if (a_mn)
+    rc = launch<true, false>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
+  else if (b_mn)
+    rc = launch<false, true>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
+  else
+    rc = launch<false, false>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
+  if (rc || !apart) return rc;
+  ProfScope prof(stream, "sum_slices");
+  sum_slices_kernel<<<blocks_for(p.batches * rows * (cols / 4), 256), 256, 0, stream>>>(
+      p.partials, sch.k_splits, p.batches, rows, (int)cols, p.bias, p.c, p.ldc, p.c_batch_stride);
+  TFGPC_LAUNCH_CHECK();
+  return TFGPC_OK;
 }
 
 int split_rows(cudaStream_t stream, const SplitJob& first, const SplitJob* second) {

@@ -42,7 +42,16 @@ struct GemmProblem {
   int batches = 1;
   int64_t c_batch_stride = 0;
   const float* bias = nullptr;
+  // The sums have a fixed order: more than two slices of the reduction go to `partials`
+  // (partial_elems values, see gemm_partial_elems) and are added one after the other; two
+  // are added into zeros, in either order the same.
+  bool ordered = false;
+  float* partials = nullptr;
+  int64_t partial_elems = 0;
 };
+
+// Values that an ordered product needs for the slices of its reduction (0: none).
+int64_t gemm_partial_elems(int64_t M, int64_t N, int64_t K, bool b_mn);
 
 // err_flag (device int, zero-initialised by the caller) is set to 1 if a bounded wait
 // inside the kernel ran out.

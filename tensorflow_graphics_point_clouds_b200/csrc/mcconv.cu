@@ -57,10 +57,17 @@ struct McWs {
   __nv_bfloat16 *g_hi, *g_mid;      // [ns, Cout]   (backward)
   float* dx;                        // [ns, C*K]    (backward)
   __nv_bfloat16* fs;                // [n_in, 2, C] split features (tensor-core projection)
+  float* partials;                  // slices of the forward product, where it has several
+  int64_t partial_elems;
   __nv_bfloat16 *wt_hi, *wt_mid;    // [Cout, C*K]: W transposed (backward)
   float* dw_pad;                    // [C*K, Cout]: gradient of padded weights (backward)
   size_t bytes;
 };
+
+// With at least one full tile of output features the roles of the forward product are
+// swapped, out^T = W^T * X^T with W as the (MN-major) left operand, and the tiles are
+// transposed on their way out.
+inline bool forward_swapped(int64_t cout) { return cout >= 128; }
 
 McWs carve(void* ws, int K, int C, int Cout, int64_t ns, int64_t n_in, bool backward) {
   McWs w;
@@ -76,6 +83,9 @@ McWs carve(void* ws, int K, int C, int Cout, int64_t ns, int64_t n_in, bool back
   // of the same workspace agree on where it lies
   w.fs = nullptr;
   if (basis_proj_mma_supported(K, C)) w.fs = (__nv_bfloat16*)take((size_t)n_in * C * 4);
+  w.partial_elems = forward_swapped(Cout) ? gemm_partial_elems(Cout, ns, ck, false)
+                                          : gemm_partial_elems(ns, Cout, ck, true);
+  w.partials = (float*)take((size_t)w.partial_elems * 4);
   w.g_hi = w.g_mid = nullptr; w.dx = nullptr; w.wt_hi = w.wt_mid = nullptr; w.dw_pad = nullptr;
   if (backward) {
     w.g_hi = (__nv_bfloat16*)take((size_t)ns * Cout * 2);
@@ -221,14 +231,14 @@ extern "C" int tfgpc_mcconv_forward_blocks(void* stream, int K, int C, int Cout,
   p.ldc = Cout;
   p.batches = groups;
   p.c_batch_stride = co;
-  // With at least one full tile of output features the roles are swapped,
-  // out^T = W^T * X^T with W as the (MN-major) left operand, and the tiles are
-  // transposed on their way out.
-  p.transposed = co >= 128;
+  p.transposed = forward_swapped(co);
   p.M = p.transposed ? co : ns;
   p.N = p.transposed ? ns : co;
   p.a = p.transposed ? wt : x;
   p.b = p.transposed ? x : wt;
+  p.ordered = true;
+  p.partials = w.partials;
+  p.partial_elems = w.partial_elems;
   return gemm_bf16x3(st, p, w.err);
 }
 
@@ -329,6 +339,7 @@ extern "C" int tfgpc_mcconv_backward_blocks(
     p.ldc = ck;
     p.batches = groups;
     p.c_batch_stride = ch;
+    p.ordered = true;
     rc = gemm_bf16x3(st, p, w.err);
     if (rc) return rc;
     if (fs_ok)

@@ -355,3 +355,30 @@ def check_kernel_mlp(groups, m, act, alpha, layer, sizes):
   assert float((got.double() - basis).norm() / basis.norm()) < 1e-5
   for got, ref in zip(dws + dbs + [dpin, dpout, dpdf], exact):
     assert float((got.double() - ref).norm() / ref.norm()) < 1e-5
+
+
+# forward products of one, two and more slices of their reduction (tall and swapped forms,
+# blocks of several kernel MLPs, a remainder in the last slice): the same bits every time
+@pytest.mark.parametrize("ns,c,k,cout,groups", [
+    (1024, 64, 32, 64, 1), (1000, 64, 32, 256, 1), (70, 128, 64, 128, 1), (33, 128, 64, 40, 1),
+    (300, 96, 32, 64, 1), (700, 48, 16, 32, 1), (257, 128, 64, 128, 2), (20000, 128, 64, 8, 1),
+    (300, 128, 32, 16, 1)])
+def test_forward_is_the_same_every_time(ns, c, k, cout, groups):
+  g = torch.Generator(device="cuda").manual_seed(23)
+  rnd = lambda *s: torch.randn(s, generator=g, device="cuda")
+  per = 3
+  basis, feat = rnd(ns * per, k), rnd(200, c)
+  w = rnd(groups, c * k // groups, cout // groups)
+  nb = torch.randint(0, 200, (ns * per, 2), generator=g, device="cuda", dtype=torch.int32)
+  nb[:, 1] = torch.arange(ns, device="cuda").repeat_interleave(per)
+  ranges = torch.arange(per, ns * per + 1, per, device="cuda", dtype=torch.int32)
+  op = mcconv.ProjectionGemm(k, c, cout, ns, "cuda", backward=False)
+  run = lambda: op.forward(basis, feat, nb, ranges, w, (groups, k, cout))
+  out = run()
+  x = torch.einsum("spk,spc->sck", basis.double().view(ns, per, k),
+                   feat.double()[nb[:, 0].long()].view(ns, per, c))
+  exact = torch.cat([x[:, :, i * k // groups:(i + 1) * k // groups].reshape(ns, -1) @ w[i].double()
+                     for i in range(groups)], dim=1)
+  assert float((out.double() - exact).norm() / exact.norm()) < 2e-5
+  for _ in range(12):
+    assert torch.equal(run(), out)
