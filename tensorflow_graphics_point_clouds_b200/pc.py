@@ -83,25 +83,57 @@ class PointCloud:
     return self._aabb
 
 
-# Upper bound of cells per dimension that a grid's cell table, tube array and sort keys
-# are sized for, per (dimension, batch size): it starts at _FIRST_BOUND and is raised to
-# what a grid asked for when one did not fit.
+# Cells per dimension that arrays are sized for, a power of two.  Of a cell table: per
+# (dimension, batch size, cell sizes, bits of the number of points) what such a grid asked
+# for; for sizes not met before what the last grid of about as many points asked for (the
+# same level of a scene in another unit of length), else _first_bound.  Of the key-based
+# call's tube array and sort keys: per (dimension, batch size), raised when one did not fit.
+# (One bound for both kept every later grid of a batch size on the tables, or off them, that
+# its finest one had needed.)
 _MAX_CELLS = {}
 _FIRST_BOUND = 16
+_FIRST_KEY_BOUND = 64
 _ONE_CALL_CELLS_LIMIT = 1024
+# Grids whose table would be too large: [calls that do not try one again, the bound asked
+# for].  Finding that out costs a call its bounding boxes and a blocking read.
+_TOO_FINE = {}
+_TOO_FINE_CALLS = 16
 
 
-def _raise_bound(pc, err, max_cells):
-  """The bound to repeat a call with that reported too few cells, or None if a
-  grid this fine would make the fixed-size arrays too large; other errors pass."""
+def _remember(table, key, value):
+  if len(table) > 256:
+    table.clear()
+  table[key] = value
+
+
+def _asked_bound(err, max_cells):
+  """The bound to repeat a call with that reported too few cells; other errors pass."""
   asked = max(getattr(err, 'num_cells', [0]))
   if err.code != 3 or asked <= max_cells:
     raise err
-  bigger = 1 << (asked - 1).bit_length()
+  return 1 << (asked - 1).bit_length()
+
+
+def _raise_bound(pc, err, max_cells):
+  """_asked_bound of the key-based call, or None if a grid this fine would make its
+  fixed-size arrays too large."""
+  bigger = _asked_bound(err, max_cells)
   if bigger > _ONE_CALL_CELLS_LIMIT or pc._batch_size * float(bigger) ** pc._dimension >= 4e18:
     return None
-  _MAX_CELLS[(pc._dimension, pc._batch_size)] = bigger
+  _remember(_MAX_CELLS, (pc._dimension, pc._batch_size), bigger)
   return bigger
+
+
+def _bound_key(pc, sizes):
+  return pc._dimension, pc._batch_size, pc._points.shape[0].bit_length(), tuple(sizes)
+
+
+def _first_bound(pc):
+  """Bound where nothing is known: a cell per two points, as far as a table goes."""
+  d, b, bound = pc._dimension, pc._batch_size, _FIRST_BOUND
+  while 2 * b * bound ** d < pc._points.shape[0] and ops.cell_table_elems(d, b, 2 * bound):
+    bound *= 2
+  return bound
 
 
 def _reduced_cells(pc, sizes):
@@ -119,12 +151,32 @@ def _cell_grid(pc, sizes, build, **args):
   """build (ops.build_cell_grid or ops.build_cell_grid_and_sample) on a cloud with the
   bound of cells it needs; None if the cell table would be too large."""
   d, b = pc._dimension, pc._batch_size
-  max_cells = _MAX_CELLS.get((d, b), _FIRST_BOUND)
-  while max_cells and ops.cell_table_elems(d, b, max_cells):
+  key = _bound_key(pc, sizes)
+  fine = _TOO_FINE.get(key)
+  if fine is not None and fine[0] > 0:
+    fine[0] -= 1
+    return None
+  found = known = _MAX_CELLS.get(key)
+  like = None if known else key[:3]
+  max_cells = known or _MAX_CELLS.get(like) or _first_bound(pc)
+  while max_cells <= _ONE_CALL_CELLS_LIMIT and ops.cell_table_elems(d, b, max_cells):
     try:
-      return build(pc._points, pc._batch_ids, b, sizes, max_cells, **args)
+      built = build(pc._points, pc._batch_ids, b, sizes, max_cells, **args)
     except ops._lib.TfgpcError as err:
-      max_cells = _raise_bound(pc, err, max_cells)
+      max_cells = known = _asked_bound(err, max_cells)
+      if max_cells <= _ONE_CALL_CELLS_LIMIT:       # (where the key-based call starts)
+        _remember(_MAX_CELLS, (d, b), max(max_cells, _MAX_CELLS.get((d, b), 0)))
+      continue
+    if known is None:
+      known = max(_FIRST_BOUND, 1 << (max(built[0].num_cells_host.tolist()) - 1).bit_length())
+    if found != known:
+      _remember(_MAX_CELLS, key, known)
+      if like is not None:
+        _remember(_MAX_CELLS, like, known)
+    if fine is not None:
+      _TOO_FINE.pop(key, None)
+    return built
+  _remember(_TOO_FINE, key, [_TOO_FINE_CALLS, max_cells])
   return None
 
 
@@ -431,18 +483,21 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
     grid._adopt(pc, built[0], sizes)
     count = built[1]
   else:
-    max_cells = _MAX_CELLS.get((d, pc._batch_size), _FIRST_BOUND)
+    max_cells = _MAX_CELLS.get((d, pc._batch_size), _FIRST_KEY_BOUND)
+    asked = _TOO_FINE.get(_bound_key(pc, sizes), [0, 0])[1]
+    if asked > _ONE_CALL_CELLS_LIMIT:
+      max_cells = None
     while True:
+      if max_cells is None:
+        # the separate constructors size the tube array and the sort keys exactly
+        grid._build_by_keys(pc, radius, cells)
+        return Neighborhood(grid, radius, point_cloud_sample, max_neighbors)
       try:
         g = ops.grid_neighborhood_count(pc._points, pc._batch_ids, pc._batch_size, sizes, sizes,
                                         max_cells, cells=cells, **samples)
         break
       except ops._lib.TfgpcError as err:
         max_cells = _raise_bound(pc, err, max_cells)
-        if max_cells is None:
-          # the separate constructors size the tube array and the sort keys exactly
-          grid._build_by_keys(pc, radius, cells)
-          return Neighborhood(grid, radius, point_cloud_sample, max_neighbors)
     grid._cells, count = None, g.pop("count")
     grid._point_cloud, grid._batch_size = pc, pc._batch_size
     grid._cur_keys, grid._fast_DS = g.pop("keys"), g.pop("ds")

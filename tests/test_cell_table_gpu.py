@@ -301,3 +301,43 @@ def test_too_few_cells(n, sample):
   assert list(asked) == [int(c) for c in np.ceil(ext / np.array([0.1, 0.5, 0.5], F32))]
   for x in [g.arrays[k] for k in ("keys", "sorted_indices", "sorted_points", "packed")] + out[::2]:
     assert bool((x == -7).all())
+
+
+def test_a_fine_grid_leaves_later_grids_as_they_are():
+  """Whether a grid gets a table, and of what size, does not depend on the grids of the
+  same batch size before it."""
+  pts, bid, b = clouds(91, [300] * 16, 3)
+  cloud = pc.PointCloud(t(pts), t(bid), b)
+  def size_of(cell):
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    grid = pc.Grid(cloud, cell)
+    grown = torch.cuda.memory_allocated() - before
+    return grid._cells is not None, grown
+  pc.Grid(cloud, 0.25)
+  pc.Grid(cloud, 0.25)
+  alone = size_of(0.25)
+  assert alone[0]
+  # 40 cells: a larger table; [100, 1, 1]: 16 x 128^3 cells have none; 0.0015: over 1024 cells
+  for cell in (0.05, [0.02, 3.0, 3.0], 0.0015):
+    fine = pc.Grid(cloud, cell)
+    assert (fine._cells is not None) == (cell == 0.05)
+    ref = pr.Grid(pts, bid, b, cell)
+    same(fine._sorted_keys, ref.sorted_keys)
+    same(fine._sorted_indices, ref.sorted_indices)
+    assert size_of(0.25) == alone
+
+
+def test_an_outlier_costs_the_table_for_a_while_only():
+  pts, bid, b = clouds(92, [500] * 3, 3)
+  far = pts.copy()
+  far[7] = 1000.0
+  cloud, outlier = (pc.PointCloud(t(p), t(bid), b) for p in (pts, far))
+  assert pc.Grid(cloud, 0.21)._cells is not None
+  nb = pc.grid_neighborhood(outlier, 0.21)
+  assert nb._grid._cells is None
+  ref = pr.Neighborhood(pr.Grid(far, bid, b, 0.21), 0.21)
+  same(nb._samples_neigh_ranges, ref.ranges)
+  same(nb._neighbors, ref.neighbors)
+  assert any(pc.Grid(cloud, 0.21)._cells is not None for _ in range(20))
+  assert pc.Grid(cloud, 0.21)._cells is not None
