@@ -10,7 +10,10 @@
 // tubes.  The sort is stable without comparing keys: a point's place is its cell's
 // start plus the number of points of the cell with a smaller index, counted over the
 // cell's members; that is quadratic in the cell size like the neighbor search
-// that follows, and a 27th of its work.
+// that follows, and a 27th of its work.  No search need follow, though, so that above
+// kCrowdedBucket members they are read once per tile of slots and not once per slot:
+// n points in one cell, before -> after: 65 000 1325 -> 98 us, 200 000 5430 -> 357, 500 000
+// 39400 -> 1110, a million in 8 cells 16500 -> 810 (by sorted keys: 180 to 190 us for all).
 //
 // Up to kClusterPoints points the whole chain is ONE kernel of one thread-block cluster
 // (grid_cluster_kernel): its phases meet at the cluster's hardware barrier, boxes and
@@ -27,6 +30,9 @@ namespace cg = cooperative_groups;
 
 constexpr int kThreads = 256;
 constexpr int kBoxPer = 4;     // points per lane of the bounding-box pass
+// Members of a bucket above which the ranks of a tile of its slots are worked out by the
+// block together (rank_in_tile).  At least a tile, so that one meets two such buckets at most.
+constexpr int kCrowdedBucket = 1024;
 
 // Order-preserving map from floats to unsigned integers (-0.0 counts as 0.0).
 __device__ __forceinline__ unsigned ordered(float v) {
@@ -68,7 +74,8 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
              int batch_size, unsigned* lo_keys, unsigned* hi_keys, unsigned* ticket,
              DimValues cell_sizes, int max_cells, float* __restrict__ aabb_min,
              float* __restrict__ aabb_max, int32_t* __restrict__ num_cells,
-             float* __restrict__ scaled_min, float* __restrict__ inv_cell, int32_t* page) {
+             float* __restrict__ scaled_min, float* __restrict__ inv_cell, int32_t* crowded,
+             int32_t* page) {
   __shared__ int cells[D];
   __shared__ bool last;
   const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
@@ -141,13 +148,18 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
   }
   __syncthreads();
   if (threadIdx.x < D) inv_cell[threadIdx.x] = __fdiv_rn(1.0f, cell_sizes.v[threadIdx.x]);
-  if (threadIdx.x == 0) clip_and_report(D, max_cells, cells, num_cells, page);
+  if (threadIdx.x == 0) {
+    *crowded = 0;
+    clip_and_report(D, max_cells, cells, num_cells, page);
+  }
 }
 
 // Cell counts given by the caller (reduced over the shards of a batch).
 __global__ void given_cells_kernel(int D, const int32_t* __restrict__ given, int max_cells,
-                                   int32_t* __restrict__ used, int32_t* page) {
+                                   int32_t* __restrict__ used, int32_t* crowded,
+                                   int32_t* page) {
   if (threadIdx.x != 0) return;
+  *crowded = 0;
   int asked[TFGPC_MAX_DIMS];
   for (int d = 0; d < D; ++d) asked[d] = given[d];
   clip_and_report(D, max_cells, asked, used, page);
@@ -157,18 +169,42 @@ __device__ __forceinline__ int bucket_of(int64_t key, int total) {
   return key >= total ? 0 : key < 0 ? total + 1 : total - (int)key;
 }
 
-// Keys, and the number of points per bucket; `arrival` is a point's number among
-// those of its bucket, in no particular order.
+// A point's number among those of its bucket, in no particular order; a bucket of more
+// than kCrowdedBucket points raises the flag.  Where more than a few lanes of a warp (`live`:
+// those that are here) share a bucket it is one atomic per bucket: a million points in one
+// cell would otherwise queue up at one address.
+__device__ __forceinline__ int arrive(int32_t* counts, int bucket, unsigned live,
+                                      int32_t* crowded) {
+  const int lane = lane_id();
+  const unsigned like_first =
+      __ballot_sync(live, bucket == __shfl_sync(live, bucket, __ffs(live) - 1));
+  if (__popc(like_first) <= 4) {
+    const int at = atomicAdd(counts + bucket, 1);
+    if (at >= kCrowdedBucket) __stcg(crowded, 1);
+    return at;
+  }
+  const unsigned peers = __match_any_sync(live, bucket);
+  const int leader = __ffs(peers) - 1;
+  int first = 0;
+  if (lane == leader) {
+    first = atomicAdd(counts + bucket, __popc(peers));
+    if (first + __popc(peers) > kCrowdedBucket) __stcg(crowded, 1);
+  }
+  return __shfl_sync(peers, first, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
+// Keys, and the number of points per bucket.
 template <int D>
 __global__ void __launch_bounds__(kThreads)
 keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
                       const int32_t* __restrict__ batch_ids, int batch_size,
                       const float* __restrict__ smin_all, const int32_t* __restrict__ num_cells,
                       const float* __restrict__ inv_cell, int64_t* __restrict__ keys_out,
-                      int32_t* counts, int32_t* __restrict__ arrival) {
+                      int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded) {
   const Grid<D> g = load_grid<D>(num_cells, inv_cell);
   const int total = total_cells<D>(g.nc, batch_size);
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const unsigned live = __ballot_sync(0xffffffffu, i < n);
   if (i >= n || total == 0) return;
   const int b = __ldg(batch_ids + i);
   const int bs = min(max(b, 0), batch_size - 1);   // (the key keeps the id that was passed in)
@@ -182,7 +218,7 @@ keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
   cell_of<D>(p, smin, g, cell);
   const int64_t key = key_of<D>(cell, g, b);
   keys_out[i] = key;
-  arrival[i] = atomicAdd(counts + bucket_of(key, total), 1);
+  arrival[i] = arrive(counts, bucket_of(key, total), live, crowded);
 }
 
 template <int D>
@@ -213,28 +249,132 @@ __device__ __forceinline__ int rank_in_bucket(const int32_t* members, int a, int
   return rank;
 }
 
+template <int THREADS>
+struct RankScratch {
+  int idx[THREADS], sorted[THREADS], upto[THREADS], warp_sum[32];
+  int below, first[2], last[2];
+};
+
+// rank_in_bucket for the slots of the crowded bucket [a, e) among those of the tile
+// [tile0, tile0 + THREADS): the block sorts the tile's own members, reads the bucket once
+// and counts, by binary search, before how many of the sorted ones each member comes.
+// One read of the bucket per tile in place of one per warp.
+template <int THREADS>
+__device__ __forceinline__ int rank_in_crowded(RankScratch<THREADS>& s, const int32_t* members,
+                                               int a, int e, int tile0, int idx) {
+  const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+  const int lo = max(a, tile0) - tile0;
+  const int count = min(e, tile0 + THREADS) - tile0 - lo;
+  const bool mine = tid >= lo && tid < lo + count;
+  if (mine) s.idx[tid - lo] = idx;
+  s.upto[tid] = 0;
+  if (tid == 0) s.below = 0;
+  __syncthreads();
+  int r = 0;
+  if (mine) {
+#pragma unroll 8
+    for (int j = 0; j < count; ++j) r += s.idx[j] < idx;
+    s.sorted[r] = idx;
+  }
+  __syncthreads();
+  const int least = s.sorted[0], most = s.sorted[count - 1];
+  int below = 0;
+  for (int q = (a & ~3) + 4 * tid; q < e; q += 4 * THREADS) {
+    const int4 m = *(const int4*)(members + q);
+    const int x[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (q + k < a || q + k >= e) continue;
+      if (x[k] < least) {
+        ++below;
+      } else if (x[k] < most) {      // it comes before the members from `from` on
+        int from = 0, to = count - 1;
+        while (from < to) {
+          const int mid = (from + to) >> 1;
+          if (s.sorted[mid] <= x[k]) from = mid + 1; else to = mid;
+        }
+        atomicAdd(&s.upto[from], 1);
+      }
+    }
+  }
+  below = __reduce_add_sync(0xffffffffu, below);
+  if (lane == 0) atomicAdd(&s.below, below);
+  __syncthreads();
+  int x = s.upto[tid];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s.warp_sum[w] = x;
+  __syncthreads();
+  const int before = lane < w ? s.warp_sum[lane] : 0;
+  s.upto[tid] = x + __reduce_add_sync(0xffffffffu, before);
+  __syncthreads();
+  const int rank = s.below + s.upto[mine ? r : 0];
+  __syncthreads();
+  return rank;
+}
+
+// Rank inside its bucket [a, e) of the member idx in slot tile0 + threadIdx.x (live: there
+// is one); the whole block calls.  any: a bucket of the grid is crowded.
+template <int THREADS>
+__device__ __forceinline__ int rank_in_tile(RankScratch<THREADS>& s, const int32_t* members, int a,
+                                            int e, int tile0, int idx, bool live, bool last,
+                                            bool any) {
+  static_assert(THREADS <= kCrowdedBucket, "more than two crowded buckets in a tile");
+  if (!any) return live ? rank_in_bucket(members, a, e, idx) : 0;
+  const bool crowded = live && e - a > kCrowdedBucket;
+  int rank = live && !crowded ? rank_in_bucket(members, a, e, idx) : 0;
+  if (!__syncthreads_or(crowded)) return rank;
+  if (threadIdx.x == 0) { s.first[0] = a; s.first[1] = e; }
+  if (last) { s.last[0] = a; s.last[1] = e; }
+  __syncthreads();
+  const int fa = s.first[0], fe = s.first[1], la = s.last[0], le = s.last[1];
+  if (fe - fa > kCrowdedBucket) {
+    const int r = rank_in_crowded<THREADS>(s, members, fa, fe, tile0, idx);
+    if (crowded && a == fa) rank = r;
+  }
+  if (la != fa && le - la > kCrowdedBucket) {
+    const int r = rank_in_crowded<THREADS>(s, members, la, le, tile0, idx);
+    if (crowded && a == la) rank = r;
+  }
+  return rank;
+}
+
 // One thread per slot of `members`: the rank of its point inside the bucket, and the
 // point's row of every sorted array; then the tube ranges, read off the table.
-template <int D>
-__global__ void __launch_bounds__(kThreads)
+template <int D, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __restrict__ keys,
              const int32_t* __restrict__ num_cells, int batch_size,
              const int32_t* __restrict__ start, const float* __restrict__ pts,
              const int32_t* __restrict__ batch_ids, int32_t* __restrict__ perm,
              int64_t* __restrict__ skeys, float* __restrict__ spts, int32_t* __restrict__ sbid,
-             float4* __restrict__ packed, int2* __restrict__ ds) {
+             float4* __restrict__ packed, int2* __restrict__ ds,
+             const int32_t* __restrict__ crowded) {
   int nc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
   const int total = total_cells<D>(nc, batch_size);
   if (total == 0) return;
-  const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (i < n) {
-    const int idx = __ldg(members + i);
-    const int64_t key = __ldg(keys + idx);
+  __shared__ RankScratch<THREADS> scratch;
+  const int64_t i = (int64_t)blockIdx.x * THREADS + threadIdx.x;
+  const bool live = i < n;
+  int idx = 0, a = 0, e = 0;
+  int64_t key = 0;
+  if (live) {
+    idx = __ldg(members + i);
+    key = __ldg(keys + idx);
     const int r = bucket_of(key, total);
-    const int a = __ldg(start + r), e = __ldg(start + r + 1);
-    const int64_t o = a + rank_in_bucket(members, a, e, idx);
+    a = __ldg(start + r);
+    e = __ldg(start + r + 1);
+  }
+  const int rank = rank_in_tile<THREADS>(
+      scratch, members, a, e, (int)(i - threadIdx.x), idx, live,
+      live && (threadIdx.x == THREADS - 1 || i == n - 1), __ldg(crowded) != 0);
+  if (live) {
+    const int64_t o = a + rank;
     perm[o] = idx;
     skeys[o] = key;
     sbid[o] = __ldg(batch_ids + idx);
@@ -250,7 +390,7 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
 #pragma unroll
   for (int d = 2; d < D; ++d) span *= nc[d];
   const int tubes = total / span;
-  for (int64_t t = i; t < tubes; t += (int64_t)gridDim.x * kThreads) {
+  for (int64_t t = i; t < tubes; t += (int64_t)gridDim.x * THREADS) {
     const int a = __ldg(start + (total - ((int)t * span + span - 1)));
     const int e = __ldg(start + (total - (int)t * span) + 1);
     ds[t] = e > a ? make_int2(a, e) : make_int2(0, 0);
@@ -280,7 +420,7 @@ struct ClusterBuild {
   int batch_size, max_cells;
   DimValues cell_sizes;
   tfgpc_cell_grid g;
-  int32_t *arrival, *members, *page;
+  int32_t *arrival, *members, *crowded, *page;
   bool place;
 };
 
@@ -292,6 +432,7 @@ grid_cluster_kernel(ClusterBuild a) {
   __shared__ float smin_s[kClusterBoxes];
   __shared__ int asked[D], nc_s[D];
   __shared__ int warp_sum_s[32], block_sum_s;
+  __shared__ RankScratch<kClusterThreads> scratch;
   cg::cluster_group cluster = cg::this_cluster();
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
@@ -377,9 +518,13 @@ grid_cluster_kernel(ClusterBuild a) {
   const int total = total_cells<D>(g.nc, a.batch_size);
   int32_t* const table = a.g.cell_start;
   for (int i = first; i < total + 3; i += stride) __stcg(table + i, 0);
+  if (first == 0) __stcg(a.crowded, 0);
   cluster.sync();
   // ---- keys and the number of points per bucket (see keys_histogram_kernel)
-  for (int i = first; i < n; i += stride) {
+  for (int i0 = first - lane; i0 < n; i0 += stride) {
+    const int i = i0 + lane;
+    const unsigned live = __ballot_sync(0xffffffffu, i < n);
+    if (i >= n) break;
     const int b = __ldg(a.batch_ids + i);
     const int bs = min(max(b, 0), a.batch_size - 1);
     float p[D];
@@ -389,7 +534,7 @@ grid_cluster_kernel(ClusterBuild a) {
     cell_of<D>(p, smin_s + bs * D, g, cell);
     const int64_t key = key_of<D>(cell, g, b);
     __stcg((long long*)a.g.keys + i, (long long)key);
-    __stcg(a.arrival + i, atomicAdd(table + bucket_of(key, total), 1));
+    __stcg(a.arrival + i, arrive(table, bucket_of(key, total), live, a.crowded));
   }
   cluster.sync();
   // ---- exclusive scan of the table: a stretch per block, its sum first
@@ -443,12 +588,23 @@ grid_cluster_kernel(ClusterBuild a) {
   cluster.sync();   // (also: no block leaves while others read its shared memory)
   if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
   if (!a.place) return;
-  for (int i = first; i < n; i += stride) {
-    const int idx = __ldcg(a.members + i);
-    const int64_t key = __ldcg((const long long*)a.g.keys + idx);
-    const int r = bucket_of(key, total);
-    const int o = __ldcg(table + r) + rank_in_bucket(a.members, __ldcg(table + r),
-                                                     __ldcg(table + r + 1), idx);
+  const bool any = __ldcg(a.crowded) != 0;
+  for (int tile0 = rank * kClusterThreads; tile0 < n; tile0 += stride) {
+    const int i = tile0 + tid;
+    const bool live = i < n;
+    int idx = 0, from = 0, to = 0;
+    int64_t key = 0;
+    if (live) {
+      idx = __ldcg(a.members + i);
+      key = __ldcg((const long long*)a.g.keys + idx);
+      const int r = bucket_of(key, total);
+      from = __ldcg(table + r);
+      to = __ldcg(table + r + 1);
+    }
+    const bool last = live && (tid == kClusterThreads - 1 || i == n - 1);
+    const int o = from + rank_in_tile<kClusterThreads>(scratch, a.members, from, to, tile0, idx,
+                                                       live, last, any);
+    if (!live) break;
     a.g.sorted_indices[o] = idx;
     a.g.sorted_keys[o] = key;
     a.g.sorted_batch_ids[o] = __ldg(a.batch_ids + idx);
@@ -508,12 +664,25 @@ int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
   return TFGPC_OK;
 }
 
-int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const int32_t* batch_ids,
-          const CellGridWs& w) {
-  TFGPC_DIM_SWITCH(g.D, place_kernel<kD><<<blocks_for(g.n, kThreads), kThreads, 0, st>>>(
+// A tile (a block) reads a crowded bucket once: large ones for clouds that can have cells
+// of hundreds of thousands of points, small ones spread a small cloud over the SMs.
+constexpr int64_t kLargeTilePoints = 131072;
+
+template <int THREADS>
+void launch_place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
+                  const int32_t* batch_ids, const CellGridWs& w) {
+  TFGPC_DIM_SWITCH(g.D, place_kernel<kD, THREADS><<<blocks_for(g.n, THREADS), THREADS, 0, st>>>(
       g.n, w.members, g.keys, g.num_cells, (int)g.batch_size, g.cell_start, points, batch_ids,
       g.sorted_indices, g.sorted_keys, g.sorted_points, g.sorted_batch_ids, (float4*)g.packed,
-      (int2*)g.ds));
+      (int2*)g.ds, w.crowded));
+}
+
+int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const int32_t* batch_ids,
+          const CellGridWs& w) {
+  if (g.n >= kLargeTilePoints)
+    launch_place<512>(st, g, points, batch_ids, w);
+  else
+    launch_place<256>(st, g, points, batch_ids, w);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
@@ -533,6 +702,7 @@ CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch
   const int64_t a = scan_block_sums_elems(cells), b = scan_block_sums_elems(ns);
   w.sums = (int64_t*)take((size_t)(a > b ? a : b) * 8);
   w.total = (int64_t*)take(8);
+  w.crowded = (int32_t*)take(4);
   w.bytes = (size_t)(p - (char*)align_up((size_t)ws, 256));
   return w;
 }
@@ -549,8 +719,8 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   if (!num_cells_in && n <= kClusterPoints && cells <= kClusterCells &&
       (int64_t)B * D <= kClusterBoxes) {
     ProfScope prof(st, "grid_cluster");
-    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.arrival, w.members, page,
-                         n <= kClusterPlacePoints};
+    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.arrival, w.members,
+                         w.crowded, page, n <= kClusterPlacePoints};
     int rc = TFGPC_OK;
     TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a));
     if (rc) return rc;
@@ -558,7 +728,8 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   }
   if (num_cells_in) {
     ProfScope prof(st, "grid_params");
-    given_cells_kernel<<<1, 32, 0, st>>>(D, num_cells_in, g.max_cells, g.num_cells, page);
+    given_cells_kernel<<<1, 32, 0, st>>>(D, num_cells_in, g.max_cells, g.num_cells, w.crowded,
+                                         page);
   } else {
     ProfScope prof(st, "grid_params");
     TFGPC_CUDA(cudaMemsetAsync(w.box_keys, 0xff, w.box_bytes, st));
@@ -566,7 +737,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
     unsigned* hi = lo + (size_t)B * D;
     TFGPC_DIM_SWITCH(D, boxes_kernel<kD><<<blocks_for(n, kThreads * kBoxPer), kThreads, 0, st>>>(
         n, points, batch_ids, B, lo, hi, hi + (size_t)B * D, cs, g.max_cells, g.aabb_min,
-        g.aabb_max, g.num_cells, g.scaled_aabb_min, g.inv_cell_sizes, page));
+        g.aabb_max, g.num_cells, g.scaled_aabb_min, g.inv_cell_sizes, w.crowded, page));
   }
   TFGPC_LAUNCH_CHECK();
   {
@@ -574,7 +745,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
     TFGPC_CUDA(cudaMemsetAsync(g.cell_start, 0, (size_t)(cells + 3) * 4, st));
     TFGPC_DIM_SWITCH(D, keys_histogram_kernel<kD><<<blocks, kThreads, 0, st>>>(
         n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells, g.inv_cell_sizes, g.keys,
-        g.cell_start, w.arrival));
+        g.cell_start, w.arrival, w.crowded));
   }
   TFGPC_LAUNCH_CHECK();
   int rc = exclusive_scan_cells(st, g.cell_start, g.num_cells, D, B, cells + 3, w.sums);

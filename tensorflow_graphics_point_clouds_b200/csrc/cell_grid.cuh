@@ -19,6 +19,7 @@ struct CellGridWs {
   int32_t *arrival, *members;   // [n]
   int64_t* sums;           // tile sums of the scans
   int64_t* total;          // [1]
+  int32_t* crowded;        // [1] set if a bucket holds more than a sort tile
   size_t bytes;
 };
 

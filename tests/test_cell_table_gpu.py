@@ -341,3 +341,31 @@ def test_an_outlier_costs_the_table_for_a_while_only():
   same(nb._neighbors, ref.neighbors)
   assert any(pc.Grid(cloud, 0.21)._cells is not None for _ in range(20))
   assert pc.Grid(cloud, 0.21)._cells is not None
+
+
+# cells of more points than a tile of the sort (512 slots, 1024 in the cluster), around the
+# line where the block ranks them together, at tile edges, several side by side, with and
+# without points that belong to no cell
+@pytest.mark.parametrize("cells", [
+    [1024], [1025], [8192], [1, 1025, 3], [511, 1500, 1500, 2], [1026] * 7, [40000], [3000, 60000],
+    [70001], [1025, 1, 90000, 700], [100000, 100000]])
+@pytest.mark.parametrize("strays", [0, 1500])
+def test_crowded_cells(cells, strays):
+  rng = np.random.default_rng(101)
+  pts = np.concatenate([np.full((m, 3), k) for k, m in enumerate(cells)]).astype(F32)
+  pts += rng.uniform(0.1, 0.9, pts.shape).astype(F32)
+  bid = np.zeros(len(pts), np.int32)
+  if strays:
+    pts = np.concatenate([pts, rng.uniform(0, 1, (2 * strays, 3)).astype(F32)])
+    bid = np.concatenate([bid, np.repeat(np.array([-1, 2], np.int32), strays)])
+  order = rng.permutation(len(pts))
+  pts, bid = pts[order], bid[order]
+  g = pc.Grid(pc.PointCloud(t(pts), t(bid), 1), 1.0)
+  assert g._cells is not None
+  keys = g._cur_keys.cpu().numpy()
+  assert len(np.unique(keys)) >= len(cells)
+  perm = np.argsort(-keys, kind="stable")
+  same(g._sorted_indices, perm.astype(np.int32))
+  same(g._sorted_keys, keys[perm])
+  same(g._sorted_points, pts[perm])
+  same(g._sorted_batch_ids, bid[perm])
