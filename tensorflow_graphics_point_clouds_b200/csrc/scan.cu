@@ -2,10 +2,10 @@
 // Takes the place of the reference's recursive Blelloch scan with its host
 // loop (find_neighbors/cc/kernels/scan_alg_kernels.cu.cc:41-266): one launch for
 // inputs that one block can take (kOneBlock elements), else two -- tile sums, then a
-// pass in which every block first adds up the sums of the tiles before its own (at
-// most a few thousand values out of L2, cheaper than a third launch) --, no host
-// synchronisation, 64-bit tile sums so that totals beyond 2^31 are detected by the
-// caller instead of wrapping silently.
+// pass in which every block first adds up the sums of the tiles before its own (up to
+// kDirectTiles values out of L2, cheaper than a third launch) --, and above that three,
+// the tile sums scanned by one block in between; no host synchronisation, 64-bit tile
+// sums so that totals beyond 2^31 are detected by the caller instead of wrapping silently.
 #include "scan.cuh"
 
 namespace tfgpc {
@@ -55,13 +55,43 @@ scan_reduce_kernel(const int32_t* __restrict__ in, ScanSize size, int64_t* __res
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = v;
 }
 
+// Tile sums to the sums of the tiles before each, by one block.
+__global__ void __launch_bounds__(1024)
+scan_sums_kernel(ScanSize size, int64_t* tile_sums) {
+  __shared__ int64_t smem[32];
+  const int64_t n = elems_of(size);
+  const int64_t tiles = (n + kScanTile - 1) / kScanTile;
+  const int w = threadIdx.x >> 5;
+  int64_t run = 0;
+  for (int64_t t0 = 0; t0 < tiles; t0 += 1024) {
+    const int64_t t = t0 + threadIdx.x;
+    const int64_t own = t < tiles ? tile_sums[t] : 0;
+    int64_t x = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane_id() >= o) x += y;
+    }
+    if (lane_id() == 31) smem[w] = x;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+    for (int i = 0; i < 32; ++i) {
+      if (i < w) before += smem[i];
+      all += smem[i];
+    }
+    if (t < tiles) tile_sums[t] = run + before + x - own;
+    run += all;
+    __syncthreads();
+  }
+}
+
 // One tile per block.  EXCLUSIVE: out[i] = sum of in[0..i), else of in[0..i].  The
 // last tile's block also delivers the report.
 template <int THREADS, int ITEMS, bool EXCLUSIVE>
 __global__ void __launch_bounds__(THREADS)
 scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, ScanSize size,
-                  const int64_t* __restrict__ tile_sums, int64_t* __restrict__ total,
-                  ScanReport rep) {
+                  const int64_t* __restrict__ tile_sums, bool sums_scanned,
+                  int64_t* __restrict__ total, ScanReport rep) {
   constexpr int kTile = THREADS * ITEMS;
   __shared__ int64_t smem[32];
   __shared__ int32_t stage[kTile];
@@ -69,7 +99,9 @@ scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, Sca
   const int64_t tile0 = (int64_t)blockIdx.x * kTile;
   if (tile0 >= n) return;
   int64_t before = 0;
-  if (blockIdx.x > 0) {
+  if (sums_scanned) {
+    before = __ldg(tile_sums + blockIdx.x);
+  } else if (blockIdx.x > 0) {
     for (int64_t t = threadIdx.x; t < blockIdx.x; t += THREADS) before += __ldg(tile_sums + t);
     before = block_sum<THREADS>(before, smem);
   }
@@ -137,6 +169,8 @@ scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, Sca
 constexpr int kOneThreads = 1024;
 constexpr int kOneItems = 8;
 constexpr int64_t kOneBlock = (int64_t)kOneThreads * kOneItems;   // 8192
+// Tiles up to which every block adds up the sums before its own: 33 million elements.
+constexpr unsigned kDirectTiles = 8192;
 
 template <bool EXCLUSIVE>
 int scan_impl(cudaStream_t st, const int32_t* in, int32_t* out, const ScanSize& size,
@@ -144,15 +178,20 @@ int scan_impl(cudaStream_t st, const int32_t* in, int32_t* out, const ScanSize& 
   ProfScope prof(st, "scan_i32");
   if (capacity <= kOneBlock) {
     scan_tiles_kernel<kOneThreads, kOneItems, EXCLUSIVE><<<1, kOneThreads, 0, st>>>(
-        in, out, size, nullptr, total, rep);
+        in, out, size, nullptr, false, total, rep);
     TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
   const unsigned tiles = (unsigned)((capacity + kScanTile - 1) / kScanTile);
   scan_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(in, size, block_sums);
   TFGPC_LAUNCH_CHECK();
+  const bool scanned = tiles > kDirectTiles;
+  if (scanned) {
+    scan_sums_kernel<<<1, 1024, 0, st>>>(size, block_sums);
+    TFGPC_LAUNCH_CHECK();
+  }
   scan_tiles_kernel<kScanThreads, kScanItems, EXCLUSIVE><<<tiles, kScanThreads, 0, st>>>(
-      in, out, size, block_sums, total, rep);
+      in, out, size, block_sums, scanned, total, rep);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }

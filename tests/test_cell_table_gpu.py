@@ -369,3 +369,20 @@ def test_crowded_cells(cells, strays):
   same(g._sorted_keys, keys[perm])
   same(g._sorted_points, pts[perm])
   same(g._sorted_batch_ids, bid[perm])
+
+
+@pytest.mark.parametrize("n", [8192 * 4096, 8192 * 4096 + 1, 9000 * 4096 + 77])
+def test_ranges_of_millions_of_samples(n):
+  """Scans above and below the line where the sums of their tiles are scanned by themselves."""
+  pts, bid, b = clouds(111, [100], 3)
+  grid = pc.Grid(pc.PointCloud(t(pts), t(bid), b), 0.6)
+  at = torch.cat([torch.arange(0, n, 1_000_003), torch.tensor([n - 1])]).to(DEV)
+  samples = torch.zeros(n, 3, device=DEV)
+  samples[at] = t(pts)[torch.arange(len(at), device=DEV) % 100]
+  ids = torch.full((n,), -1, device=DEV, dtype=torch.int32)
+  ids[at] = 0
+  few = pc.Neighborhood(grid, 0.6, pc.PointCloud(samples[at].contiguous(), ids[at], b))
+  counts = torch.zeros(n, device=DEV, dtype=torch.int64)
+  counts[at] = few._samples_neigh_ranges.long().diff(prepend=torch.zeros(1, device=DEV).long())
+  many = pc.Neighborhood(grid, 0.6, pc.PointCloud(samples, ids, b))
+  assert torch.equal(many._samples_neigh_ranges.long(), counts.cumsum(0))
