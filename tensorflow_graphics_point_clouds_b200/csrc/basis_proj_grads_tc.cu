@@ -25,7 +25,7 @@
 //   F      gathered from the pre-split features ([n, 2, C] bf16) by 16-byte
 //          cp.async, one 64-channel block (hi 16 KB + mid 16 KB) per ring slot;
 //   Bx     built by the producer warps from the fp32 basis rows;
-//   dXcat  produced in exactly this image by the dX GEMM (gemm_bf16x3_grad_image)
+//   dXcat  produced in exactly this image by the dX GEMM (gemm_bf16x3_grad_image_tn)
 //          and fetched with one 32 KB bulk copy per group.  The same bytes serve
 //          as the MN-major B operand of (1) and the K-major A operand of (2).
 // Roles: warps 0-7 gather and build; warps 8 and 9 issue the MMAs of (1) and (2)
@@ -467,7 +467,7 @@ static int launch_grads_tc(cudaStream_t st, int64_t ns, int64_t M, const float* 
   return TFGPC_OK;
 }
 
-// `image`: the dX operand image written by gemm_bf16x3_grad_image for these ns
+// `image`: the dX operand image written by gemm_bf16x3_grad_image_tn for these ns
 // samples in groups of `group` (ceil(ns / group) groups of 32 KB; the columns of
 // the samples beyond ns in the last group must be finite).  dfeat must be zero
 // on entry; dbasis is overwritten.

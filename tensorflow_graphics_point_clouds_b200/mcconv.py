@@ -5,16 +5,15 @@ kernel MLP on the relative neighbor positions gives the per-neighbor basis
 (divided by the density estimate), the basis projection aggregates it with the
 input features, and the final weights map [C_in * K] to C_out.  The projection
 and the final matrix product run as one C-ABI call (tfgpc_mcconv_forward) and
-their gradients as another (tfgpc_mcconv_backward); the small kernel MLP
-([M, D] x [D, K]) stays in torch, like it stays in TensorFlow in the reference.
+their gradients as another (tfgpc_mcconv_backward); the kernel MLP runs as one
+kernel per direction (tfgpc_kernel_basis*, or tfgpc_kernel_mlp_* for more hidden
+layers and point gradients).
 """
-import ctypes
-
 import torch
 
 from . import _lib
-from ._lib import c_i64, c_int, c_sz, ptr
-from .custom_ops import _stream, _f32, _i32, _workspace
+from ._lib import c_i64, c_int
+from .custom_ops import _f32, _i32, _workspace
 
 
 def matmul_f32(a, b, a_transposed=False, b_transposed=False):
