@@ -10,6 +10,7 @@
 // basis_proj_kernels.cu.cc:30-127.)
 #include "basis_proj.cuh"
 #include "basis_proj_wide.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 
@@ -147,7 +148,7 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
 // fit one pass, else accumulated with atomics.
 template <int K, bool VEC>
 __global__ void __launch_bounds__(kBpThreads)
-basis_proj_grads_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
+basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __restrict__ basis,
                         const float* __restrict__ feat, const int2* __restrict__ neigh,
                         const int32_t* __restrict__ ranges, const float* __restrict__ in_grads,
                         float* __restrict__ dbasis, float* __restrict__ dfeat, int shift) {
@@ -159,6 +160,11 @@ basis_proj_grads_kernel(int C, int64_t ns, int G, const float* __restrict__ basi
   const int64_t warps = ((int64_t)gridDim.x * kBpThreads) >> 5;
   const int chunk = G * kCpl;
   const bool single_pass = C <= chunk;
+  // pairs beyond the last range belong to no sample: their gradient is zero
+  if (single_pass)
+    for (int64_t i = (int64_t)__ldg(ranges + ns - 1) * K + warp0 * 32 + lane; i < M * K;
+         i += warps * 32)
+      dbasis[i] = 0.0f;
   for (int64_t s0 = warp0 * groups_per_warp; s0 < ns; s0 += warps * groups_per_warp) {
     const int64_t s = s0 + lane / G;
     const bool active = s < ns;
@@ -332,7 +338,7 @@ int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* bas
 }
 
 template <int K>
-static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, const float* basis,
+static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* basis,
                                    const float* feat, const int2* neigh, const int32_t* ranges,
                                    const float* in_grads, float* dbasis, float* dfeat,
                                    int hidden) {
@@ -360,11 +366,11 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, const flo
     return TFGPC_OK;
   }
   if (vec)
-    basis_proj_grads_kernel<K, true><<<grid, kBpThreads, 0, st>>>(C, ns, G, basis, feat, neigh,
+    basis_proj_grads_kernel<K, true><<<grid, kBpThreads, 0, st>>>(C, ns, M, G, basis, feat, neigh,
                                                                   ranges, in_grads, dbasis, dfeat,
                                                                   shift);
   else
-    basis_proj_grads_kernel<K, false><<<grid, kBpThreads, 0, st>>>(C, ns, G, basis, feat, neigh,
+    basis_proj_grads_kernel<K, false><<<grid, kBpThreads, 0, st>>>(C, ns, M, G, basis, feat, neigh,
                                                                    ranges, in_grads, dbasis, dfeat,
                                                                   shift);
   TFGPC_LAUNCH_CHECK();
@@ -374,7 +380,6 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, const flo
 // basis_proj_mma.cu: the same contractions on warp-level tensor-core MMAs, over a
 // bf16 hi/mid copy of the features kept in caller scratch
 bool basis_proj_mma_supported(int K, int C);
-int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bfloat16* fs);
 int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                        const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                        float* out);
@@ -416,19 +421,16 @@ extern "C" int tfgpc_basis_proj(void* stream, int K, int C, int64_t ns, int64_t 
 }
 
 namespace tfgpc {
+// Layers of fewer than 32 lanes write a pair's gradient row once; the others add into it.
+bool basis_proj_grads_adds_dbasis(int K, int C) {
+  return bp_group_lanes(C, K >= 64 ? 1 : K == 32 ? 2 : 4) == 32;
+}
+
 // The gradients on the SIMT kernels, in_grads with the columns of block_offset.
-int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, int64_t M,
+int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t M,
                             const float* basis, const float* feat, const int32_t* neigh,
                             const int32_t* ranges, const float* in_grads, float* dbasis,
                             float* dfeat, int hidden) {
-  if (M > 0) {
-    TFGPC_REQUIRE(dbasis, "BasisProjGradsOp got a null pointer");
-    TFGPC_CUDA(cudaMemsetAsync(dbasis, 0, sizeof(float) * (size_t)M * K, st));
-  }
-  if (n_in > 0) {
-    TFGPC_REQUIRE(dfeat, "BasisProjGradsOp got a null pointer");
-    TFGPC_CUDA(cudaMemsetAsync(dfeat, 0, sizeof(float) * (size_t)n_in * C, st));
-  }
   if (ns == 0 || M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(basis && feat && neigh && ranges && in_grads,
                 "BasisProjGradsOp got a null pointer");
@@ -436,10 +438,10 @@ int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t n
                 "BasisProjGradsOp expects 16-byte aligned basis and gradient buffers");
   const int2* nb = (const int2*)neigh;
   switch (K) {
-    case 8: return launch_basis_proj_grads<8>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
-    case 16: return launch_basis_proj_grads<16>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
-    case 32: return launch_basis_proj_grads<32>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
-    default: return launch_basis_proj_grads<64>(st, C, ns, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    case 8: return launch_basis_proj_grads<8>(st, C, ns, M, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    case 16: return launch_basis_proj_grads<16>(st, C, ns, M, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    case 32: return launch_basis_proj_grads<32>(st, C, ns, M, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
+    default: return launch_basis_proj_grads<64>(st, C, ns, M, basis, feat, nb, ranges, in_grads, dbasis, dfeat, hidden);
   }
 }
 }  // namespace tfgpc
@@ -450,8 +452,16 @@ extern "C" int tfgpc_basis_proj_grads(void* stream, int K, int C, int64_t ns, in
                                       const float* in_grads, float* dbasis_out, float* dfeat_out) {
   int rc = check_bp_args("BasisProjGradsOp", K, C, ns, n_in, M);
   if (rc) return rc;
-  return basis_proj_grads_blocks((cudaStream_t)stream, K, C, ns, n_in, M, basis, features,
-                                 neighbors, ranges, in_grads, dbasis_out, dfeat_out, K);
+  TFGPC_REQUIRE((M == 0 || dbasis_out) && (n_in == 0 || dfeat_out),
+                "BasisProjGradsOp got a null pointer");
+  Prepare jobs;
+  if (ns == 0 || basis_proj_grads_adds_dbasis(K, C))
+    jobs.zero(dbasis_out, (size_t)M * K * sizeof(float));
+  jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
+  rc = prepare((cudaStream_t)stream, jobs);
+  if (rc) return rc;
+  return basis_proj_grads_blocks((cudaStream_t)stream, K, C, ns, M, basis, features, neighbors,
+                                 ranges, in_grads, dbasis_out, dfeat_out, K);
 }
 
 extern "C" size_t tfgpc_basis_proj_workspace_bytes(int K, int C, int64_t n_in) {
@@ -479,7 +489,9 @@ extern "C" int tfgpc_basis_proj_ws(void* stream, int K, int C, int64_t ns, int64
   TFGPC_REQUIRE(ranges && out && basis && features && neighbors, "BasisProjOp got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   __nv_bfloat16* fs = (__nv_bfloat16*)ws;
-  rc = split_features(st, features, n_in, C, fs);
+  Prepare jobs;
+  jobs.add(feature_job(features, n_in, C, fs));
+  rc = prepare(st, jobs);
   if (rc) return rc;
   return basis_proj_mma_f32(st, K, C, ns, basis, fs, neighbors, ranges, out);
 }
@@ -499,9 +511,11 @@ extern "C" int tfgpc_basis_proj_grads_ws(void* stream, int K, int C, int64_t ns,
                 "BasisProjGradsOp got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   __nv_bfloat16* fs = (__nv_bfloat16*)ws;
-  rc = split_features(st, features, n_in, C, fs);
+  Prepare jobs;
+  jobs.add(feature_job(features, n_in, C, fs));
+  jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
+  rc = prepare(st, jobs);
   if (rc) return rc;
-  TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
   return basis_proj_grads_mma(st, K, C, ns, M, basis, fs, neighbors, ranges, in_grads, dbasis_out,
                               dfeat_out, K);
 }

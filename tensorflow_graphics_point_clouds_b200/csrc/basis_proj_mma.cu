@@ -1,25 +1,9 @@
-// Host side of the tensor-core basis projection (basis_proj_mma.cuh): the
-// one-off split of the feature matrix and the two launchers.
+// Host side of the tensor-core basis projection (basis_proj_mma.cuh).
 #include "basis_proj_mma.cuh"
 
 namespace tfgpc {
 
 namespace {
-
-// feat [n, C] fp32 -> fs [n, 2, C] bf16: row 0 the hi terms, row 1 the mid terms.
-__global__ void split_features_kernel(const float* __restrict__ feat, int64_t n, int C,
-                                      __nv_bfloat16* __restrict__ fs) {
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (i >= n * C) return;
-  const int64_t row = i / C;
-  const int c = (int)(i - row * C);
-  const float4 v = __ldg(reinterpret_cast<const float4*>(feat + i));
-  uint2 h, m;
-  bpm::split2(v.x, v.y, h.x, m.x);
-  bpm::split2(v.z, v.w, h.y, m.y);
-  *reinterpret_cast<uint2*>(fs + row * 2 * C + c) = h;
-  *reinterpret_cast<uint2*>(fs + row * 2 * C + C + c) = m;
-}
 
 // Blocks of one SM each, and the samples a warp takes at a time: enough work items per
 // warp (four) to even out lists of unequal length, up to the 32 that one load of range
@@ -97,16 +81,6 @@ int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* bas
 
 bool basis_proj_mma_supported(int K, int C) {
   return (K == 16 || K == 32 || K == 64) && C >= 16 && C % 16 == 0;
-}
-
-int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bfloat16* fs) {
-  if (n <= 0) return TFGPC_OK;
-  TFGPC_REQUIRE(C % 4 == 0 && (uintptr_t)feat % 16 == 0 && (uintptr_t)fs % 16 == 0,
-                "split_features expects 16-byte aligned rows");
-  ProfScope prof(st, "split_features");
-  split_features_kernel<<<blocks_for(n * C / 4, 256), 256, 0, st>>>(feat, n, C, fs);
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
 }
 
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,

@@ -529,51 +529,6 @@ __global__ void wait_probe_kernel(int* err_flag, unsigned long long limit_ns, in
   }
 }
 
-// Row r of a job's output is the split of a row of its source, `ld` columns wide with
-// zeros from `cols` on: row order[r], or, for a weight matrix whose basis functions are
-// padded from k_src to k_dst, row (r / k_dst) * k_src + r % k_dst (none if r % k_dst
-// reaches k_src).
-struct SplitJobs {
-  SplitJob job[2];
-  int64_t first_block[2];    // of job 1; total
-};
-
-__global__ void __launch_bounds__(256) split_rows_kernel(SplitJobs jobs) {
-  const bool second = (int64_t)blockIdx.x >= jobs.first_block[0];
-  const SplitJob j = second ? jobs.job[1] : jobs.job[0];
-  const unsigned quads = (unsigned)j.ld / 4;     // four values per thread
-  const unsigned i = (unsigned)((int64_t)blockIdx.x - (second ? jobs.first_block[0] : 0)) * 256u +
-                     threadIdx.x;
-  if (i >= (unsigned)j.rows * quads) return;
-  const unsigned r = (quads & (quads - 1)) == 0 ? i >> (31 - __clz(quads)) : i / quads;
-  const int c = (int)(i - r * quads) * 4;
-  int64_t src = r;
-  if (j.order) {
-    src = __ldg(j.order + r);
-  } else if (j.k_src != j.k_dst) {
-    const unsigned ch = r / (unsigned)j.k_dst;
-    const int k = (int)(r - ch * j.k_dst);
-    src = k < j.k_src ? (int64_t)ch * j.k_src + k : -1;
-  }
-  float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  if (src >= 0) {
-    const float* p = j.x + src * j.cols + c;
-    if (j.cols % 4 == 0 && c < j.cols && (uintptr_t)j.x % 16 == 0) {
-      const float4 q = __ldg(reinterpret_cast<const float4*>(p));
-      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (c + e < j.cols) v[e] = __ldg(p + e);
-    }
-  }
-  uint2 h, m;
-  split2_bf16(v[0], v[1], h.x, m.x);
-  split2_bf16(v[2], v[3], h.y, m.y);
-  *reinterpret_cast<uint2*>(j.hi + (int64_t)r * j.ld + c) = h;
-  *reinterpret_cast<uint2*>(j.mid + (int64_t)r * j.ld + c) = m;
-}
-
 // out = the sum of `slices` slices, one after the other (and the bias, [cols] or
 // null), four values per thread.
 __global__ void __launch_bounds__(256)
@@ -602,7 +557,7 @@ sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, i
 }
 
 // hi_t, mid_t [cols, rows] = the split of the transpose of x, whose rows and columns are
-// padded with zeros as in split_rows_kernel.
+// padded with zeros as in split_block (prepare.cu).
 __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows, int64_t cols,
                                        int cols_src, int k_src, int k_dst,
                                        __nv_bfloat16* __restrict__ hi_t,
@@ -697,6 +652,26 @@ int gemm_bf16x3_tn_scatter(cudaStream_t stream, int64_t M, int64_t N, int64_t K,
                                 nullptr, (uint8_t*)out, (int)ld_out, 4, row_order);
 }
 
+// Tiles and slices of a product; slice_batches > 0: its slices are kept apart.
+static TileSchedule schedule_of(const GemmProblem& p) {
+  const int bn = tile_columns(p.N, p.b.major == Major::MN);
+  const int64_t tiles = ((p.M + kBM - 1) / kBM) * ((p.N + bn - 1) / bn) * p.batches;
+  const int64_t cols = p.transposed ? p.M : p.N;
+  int splits = pick_k_splits(tiles, p.K);
+  if (p.ordered && splits > 2) {
+    const int64_t room = cols % 4 == 0 ? p.partial_elems / (p.M * p.N * p.batches) : 0;
+    splits = (int)(room > 2 ? (room < splits ? room : splits) : 2);
+  }
+  TileSchedule sch = schedule(p.M, p.N, p.K, p.batches, bn, splits);
+  if (p.ordered && sch.k_splits > 2) {
+    sch.add_slices = 0;
+    sch.slice_batches = p.batches;
+  }
+  return sch;
+}
+
+bool gemm_adds_slices(const GemmProblem& p) { return schedule_of(p).add_slices != 0; }
+
 int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
   TFGPC_REQUIRE(p.M > 0 && p.N > 0 && p.K > 0 && p.batches > 0, "GEMM expects positive sizes");
   TFGPC_REQUIRE(p.M < (int64_t)INT32_MAX && p.N < (int64_t)INT32_MAX && p.K < (int64_t)INT32_MAX,
@@ -708,20 +683,10 @@ int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
   CUtensorMap maps[5] = {};
   int rc = operand_maps(maps, p.a, p.b, p.M, p.N, p.K, p.batches, bn);
   if (rc) return rc;
-  const int64_t tiles = ((p.M + kBM - 1) / kBM) * ((p.N + bn - 1) / bn) * p.batches;
   const int64_t rows = p.transposed ? p.N : p.M, cols = p.transposed ? p.M : p.N;
-  int splits = pick_k_splits(tiles, p.K);
-  if (p.ordered && splits > 2) {
-    const int64_t room = cols % 4 == 0 ? p.partial_elems / (rows * cols * p.batches) : 0;
-    splits = (int)(room > 2 ? (room < splits ? room : splits) : 2);
-  }
-  TileSchedule sch = schedule(p.M, p.N, p.K, p.batches, bn, splits);
-  const bool apart = p.ordered && sch.k_splits > 2;
-  if (apart) {
-    sch.add_slices = 0;
-    sch.slice_batches = p.batches;
-  }
-  if (sch.add_slices) {
+  const TileSchedule sch = schedule_of(p);
+  const bool apart = sch.slice_batches > 0;
+  if (sch.add_slices && !p.cleared) {
     // the slices are added into c, which starts from zero, by the store unit (the order
     // of the additions, and with it the last bits of the sums, varies from run to run)
     const bool dense = p.batches == 1 ? p.ldc == cols
@@ -754,27 +719,6 @@ int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
   ProfScope prof(stream, "sum_slices");
   sum_slices_kernel<<<blocks_for(p.batches * rows * (cols / 4), 256), 256, 0, stream>>>(
       p.partials, sch.k_splits, p.batches, rows, (int)cols, p.bias, p.c, p.ldc, p.c_batch_stride);
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
-}
-
-int split_rows(cudaStream_t stream, const SplitJob& first, const SplitJob* second) {
-  SplitJobs jobs{};
-  int64_t blocks = 0;
-  for (int i = 0; i < (second ? 2 : 1); ++i) {
-    const SplitJob& j = i ? *second : first;
-    TFGPC_REQUIRE(j.ld % 4 == 0 && (uintptr_t)j.hi % 8 == 0 && (uintptr_t)j.mid % 8 == 0,
-                  "split_rows expects rows of a multiple of 4 values");
-    TFGPC_REQUIRE(j.rows * (j.ld / 4) < (int64_t)UINT32_MAX, "split_rows: too many values");
-    jobs.job[i] = j;
-    blocks += j.rows > 0 && j.ld > 0 ? (j.rows * (j.ld / 4) + 255) / 256 : 0;
-    jobs.first_block[i] = blocks;
-  }
-  if (!second) jobs.first_block[0] = blocks + 1;   // every block works on job 0
-  if (blocks == 0) return TFGPC_OK;
-  TFGPC_REQUIRE(blocks < (int64_t)INT32_MAX, "split_rows: too many values");
-  ProfScope prof(stream, "split_bf16");
-  split_rows_kernel<<<(unsigned)blocks, 256, 0, stream>>>(jobs);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }

@@ -9,7 +9,7 @@
 
 #include <cuda_bf16.h>
 
-#include "common.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 
@@ -48,10 +48,16 @@ struct GemmProblem {
   bool ordered = false;
   float* partials = nullptr;
   int64_t partial_elems = 0;
+  bool cleared = false;      // c holds zeros already (see gemm_adds_slices)
 };
 
 // Values that an ordered product needs for the slices of its reduction (0: none).
 int64_t gemm_partial_elems(int64_t M, int64_t N, int64_t K, bool b_mn);
+
+// Whether the product adds the slices of its reduction into c, which then has to start
+// from zero: a caller that clears all of c beforehand says so (cleared), else gemm_bf16x3
+// does it with a launch of its own.
+bool gemm_adds_slices(const GemmProblem& p);
 
 // err_flag (device int, zero-initialised by the caller) is set to 1 if a bounded wait
 // inside the kernel ran out.
@@ -72,18 +78,6 @@ int gemm_bf16x3_grad_image_tn(cudaStream_t stream, int channels, int64_t N, int6
 int gemm_bf16x3_tn_scatter(cudaStream_t stream, int64_t M, int64_t N, int64_t K,
                            const GemmOperand& a, const GemmOperand& b, float* out, int64_t ld_out,
                            const int32_t* row_order, int* err_flag);
-
-// x [*, cols] fp32 -> hi, mid [rows, ld] bf16 (see split_rows_kernel); two jobs share a
-// launch.
-struct SplitJob {
-  const float* x = nullptr;
-  int64_t rows = 0;
-  int cols = 0, ld = 0;
-  const int32_t* order = nullptr;
-  int k_src = 1, k_dst = 1;
-  __nv_bfloat16 *hi = nullptr, *mid = nullptr;
-};
-int split_rows(cudaStream_t stream, const SplitJob& first, const SplitJob* second = nullptr);
 
 // x padded to [rows, cols] (see split_transpose_kernel) -> transposed bf16 pair.
 int split_transpose_to_bf16(cudaStream_t stream, const float* x, int64_t rows, int64_t cols,

@@ -12,6 +12,7 @@
 // db1[k] = sum_m dpre_k, accumulated in registers over a grid-stride loop,
 // reduced through shuffles and shared memory, one atomic per block and value.
 #include "basis_proj.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 namespace {
@@ -463,8 +464,11 @@ extern "C" int tfgpc_kernel_basis_grads(void* stream, int D, int K, int64_t M,
   if (rc) return rc;
   TFGPC_REQUIRE(dw1_out && db1_out, "KernelBasisGrads got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  TFGPC_CUDA(cudaMemsetAsync(dw1_out, 0, sizeof(float) * (size_t)D * K, st));
-  TFGPC_CUDA(cudaMemsetAsync(db1_out, 0, sizeof(float) * (size_t)K, st));
+  Prepare jobs;
+  jobs.zero(dw1_out, sizeof(float) * (size_t)D * K);
+  jobs.zero(db1_out, sizeof(float) * (size_t)K);
+  rc = prepare(st, jobs);
+  if (rc) return rc;
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && (pdf || pdf_by_neighbor == 2) && w1 &&
                 b1 && basis_grads, "KernelBasisGrads got a null pointer");

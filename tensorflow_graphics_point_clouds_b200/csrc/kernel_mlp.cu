@@ -25,7 +25,7 @@
 //     points_out, by atomics;
 //   * the gradient of the density, d_pdf[m] = -sum_k dbasis[m,k] basis[m,k] / pdf[m],
 //     which the caller carries on through ComputePdfPtGrads.
-#include "common.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 namespace {
@@ -499,14 +499,16 @@ extern "C" int tfgpc_kernel_mlp_grads_layers(
                 "KernelMlpGrads expects activation 0 (leaky ReLU) or 1 (ELU)");
   TFGPC_REQUIRE(dweights_out && dbiases_out, "KernelMlpGrads got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  TFGPC_CUDA(cudaMemsetAsync(dweights_out, 0, sizeof(float) * (size_t)nw, st));
-  TFGPC_CUDA(cudaMemsetAsync(dbiases_out, 0, sizeof(float) * (size_t)nb, st));
+  Prepare jobs;
+  jobs.zero(dweights_out, sizeof(float) * (size_t)nw);
+  jobs.zero(dbiases_out, sizeof(float) * (size_t)nb);
   // points_in and points_out may be one cloud: its gradient is then one array
   // that both roles add into
-  if (dpoints_in_out)
-    TFGPC_CUDA(cudaMemsetAsync(dpoints_in_out, 0, sizeof(float) * (size_t)n_in * D, st));
+  if (dpoints_in_out) jobs.zero(dpoints_in_out, sizeof(float) * (size_t)n_in * D);
   if (dpoints_out_out && dpoints_out_out != dpoints_in_out)
-    TFGPC_CUDA(cudaMemsetAsync(dpoints_out_out, 0, sizeof(float) * (size_t)ns * D, st));
+    jobs.zero(dpoints_out_out, sizeof(float) * (size_t)ns * D);
+  rc = prepare(st, jobs);
+  if (rc) return rc;
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_grads,
                 "KernelMlpGrads got a null pointer");

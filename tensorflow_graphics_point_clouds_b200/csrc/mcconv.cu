@@ -16,13 +16,15 @@ namespace tfgpc {
 int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                      const float* feat, const int32_t* neigh, const int32_t* ranges,
                      __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
-int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, int64_t M,
+// (adds into dfeat, and into dbasis where basis_proj_grads_adds_dbasis says so: the caller
+// clears them)
+bool basis_proj_grads_adds_dbasis(int K, int C);
+int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t M,
                             const float* basis, const float* feat, const int32_t* neigh,
                             const int32_t* ranges, const float* in_grads, float* dbasis,
                             float* dfeat, int hidden);
 // basis_proj_mma.cu: the projection on warp-level tensor-core MMAs
 bool basis_proj_mma_supported(int K, int C);
-int split_features(cudaStream_t st, const float* feat, int64_t n, int C, __nv_bfloat16* fs);
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
@@ -175,16 +177,24 @@ extern "C" size_t tfgpc_mcconv_workspace_bytes(int K, int C, int Cout, int64_t n
 }
 
 // The projection, written as the GEMM's bf16 operand pair: on tensor-core MMAs
-// where the shape allows it, else on the SIMT kernels.
-static int project(cudaStream_t st, int K, int C, int64_t ns, int64_t n_in, const float* basis,
+// where the shape allows it (prepare_projection then splits the features), else on the
+// SIMT kernels.
+static bool on_mma(const McWs& w, const float* features) {
+  return w.fs && (uintptr_t)features % 16 == 0;
+}
+
+static void prepare_projection(Prepare* jobs, const McWs& w, const float* features, int64_t n_in,
+                               int C) {
+  jobs->zero(w.err, sizeof(int));
+  if (on_mma(w, features)) jobs->add(feature_job(features, n_in, C, w.fs));
+}
+
+static int project(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                    const float* features, const int32_t* neighbors, const int32_t* ranges,
                    const McWs& w, int hidden) {
-  if (w.fs && (uintptr_t)features % 16 == 0) {
-    int rc = split_features(st, features, n_in, C, w.fs);
-    if (rc) return rc;
+  if (on_mma(w, features))
     return basis_proj_mma_split(st, K, C, ns, basis, w.fs, neighbors, ranges, w.x_hi, w.x_mid,
                                 hidden);
-  }
   return basis_proj_split(st, K, C, ns, basis, features, neighbors, ranges, w.x_hi, w.x_mid, hidden);
 }
 
@@ -218,11 +228,6 @@ extern "C" int tfgpc_mcconv_forward_blocks(void* stream, int K, int C, int Cout,
   cudaStream_t st = (cudaStream_t)stream;
   McWs w = carve(ws, K, C, Cout, ns, n_in, false);
   const int64_t ck = (int64_t)C * K, ch = ck / groups, co = Cout / groups;
-  TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-  rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w, K / groups);
-  if (rc) return rc;
-  rc = split_rows(st, weight_job(w, weights, ck, K, Cout, blocks));
-  if (rc) return rc;
   GemmProblem p{};
   const GemmOperand x{w.x_hi, w.x_mid, ck, Major::K, ch};
   const GemmOperand wt{w.w_hi, w.w_mid, co, Major::MN, ch * co};  // [C*K, Cout]: N contiguous
@@ -239,6 +244,15 @@ extern "C" int tfgpc_mcconv_forward_blocks(void* stream, int K, int C, int Cout,
   p.ordered = true;
   p.partials = w.partials;
   p.partial_elems = w.partial_elems;
+  Prepare jobs;
+  prepare_projection(&jobs, w, features, n_in, C);
+  jobs.add(weight_job(w, weights, ck, K, Cout, blocks));
+  p.cleared = gemm_adds_slices(p);
+  if (p.cleared) jobs.zero(out, (size_t)ns * Cout * sizeof(float));
+  rc = prepare(st, jobs);
+  if (rc) return rc;
+  rc = project(st, K, C, ns, basis, features, neighbors, ranges, w, K / groups);
+  if (rc) return rc;
   return gemm_bf16x3(st, p, w.err);
 }
 
@@ -285,16 +299,37 @@ extern "C" int tfgpc_mcconv_backward_blocks(
                 tfgpc_mcconv_workspace_bytes(K, C, Cout, ns, n_in, 1));
   McWs w = carve(ws, K, C, Cout, ns, n_in, true);
   const int hidden = K / groups;
-  if (!x_in_workspace) {
-    // (with x_in_workspace the word keeps what the forward call left: a timeout
-    // there means that the projection this call is about to read is incomplete)
-    TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-    rc = project(st, K, C, ns, n_in, basis, features, neighbors, ranges, w, hidden);
-    if (rc) return rc;
-  }
-  const bool fs_ok = w.fs && (uintptr_t)features % 16 == 0 && (uintptr_t)dbasis_out % 32 == 0 &&
+  const bool fs_ok = on_mma(w, features) && (uintptr_t)dbasis_out % 32 == 0 &&
                      (uintptr_t)dfeat_out % 16 == 0;
   const bool image = fs_ok && groups == 1 && basis_proj_grads_tc_supported(K, C);
+  // dX[ns, C*K] = dOut[ns, Cout] * W^T: B rows are W's rows, reduction over Cout
+  GemmProblem px{};
+  px.M = ns;
+  px.N = ch;
+  px.K = co;
+  px.a = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::K, co};
+  px.b = GemmOperand{w.w_hi, w.w_mid, co, Major::K, ch * co};
+  px.c = w.dx;
+  px.ldc = ck;
+  px.batches = groups;
+  px.c_batch_stride = ch;
+  px.ordered = true;
+  // dW[C*K, Cout] = X^T * dOut: both operands have the reduction (sample) index
+  // as their row index, i.e. they are MN-major
+  GemmProblem pw{};
+  pw.M = ch;
+  pw.N = co;
+  pw.K = ns;
+  pw.a = GemmOperand{w.x_hi, w.x_mid, ck, Major::MN, ch};
+  pw.b = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN, co};
+  pw.c = padded ? w.dw_pad : dweights_out;
+  pw.ldc = co;
+  pw.batches = groups;
+  pw.c_batch_stride = ch * co;
+  Prepare jobs;
+  // (with x_in_workspace the word keeps what the forward call left: a timeout
+  // there means that the projection this call is about to read is incomplete)
+  if (!x_in_workspace) prepare_projection(&jobs, w, features, n_in, C);
   SplitJob gj;
   gj.x = out_grads;
   gj.rows = ns;
@@ -302,12 +337,25 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   gj.ld = Cout;
   gj.hi = w.g_hi;
   gj.mid = w.g_mid;
+  jobs.add(gj);
   // The weights are split again on every call (2 MB): the products below then work on
   // the values of this call's `weights`, whatever the forward call saw.
-  const SplitJob wj = weight_job(w, weights, ck, K, Cout, blocks);
-  rc = split_rows(st, gj, image ? nullptr : &wj);
+  if (!image) {
+    jobs.add(weight_job(w, weights, ck, K, Cout, blocks));
+    px.cleared = gemm_adds_slices(px);
+    if (px.cleared) jobs.zero(w.dx, (size_t)ns * ck * sizeof(float));
+  }
+  pw.cleared = gemm_adds_slices(pw);
+  if (pw.cleared) jobs.zero(pw.c, (size_t)ck * co * sizeof(float));
+  jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
+  if (!fs_ok && basis_proj_grads_adds_dbasis(K, C))
+    jobs.zero(dbasis_out, (size_t)M * K * sizeof(float));
+  rc = prepare(st, jobs);
   if (rc) return rc;
-  TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
+  if (!x_in_workspace) {
+    rc = project(st, K, C, ns, basis, features, neighbors, ranges, w, hidden);
+    if (rc) return rc;
+  }
   if (image) {
     // dX goes straight into the operand image of the tcgen05 gradient kernel
     const int group = basis_proj_grads_tc_group(ns, M);
@@ -328,41 +376,17 @@ extern "C" int tfgpc_mcconv_backward_blocks(
     rc = basis_proj_grads_tc(st, group, ns, M, basis, w.fs, neighbors, ranges, w.dx, dbasis_out,
                              dfeat_out, w.err);
   } else {
-    // dX[ns, C*K] = dOut[ns, Cout] * W^T: B rows are W's rows, reduction over Cout
-    GemmProblem p{};
-    p.M = ns;
-    p.N = ch;
-    p.K = co;
-    p.a = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::K, co};
-    p.b = GemmOperand{w.w_hi, w.w_mid, co, Major::K, ch * co};
-    p.c = w.dx;
-    p.ldc = ck;
-    p.batches = groups;
-    p.c_batch_stride = ch;
-    p.ordered = true;
-    rc = gemm_bf16x3(st, p, w.err);
+    rc = gemm_bf16x3(st, px, w.err);
     if (rc) return rc;
     if (fs_ok)
       rc = basis_proj_grads_mma(st, K, C, ns, M, basis, w.fs, neighbors, ranges, w.dx, dbasis_out,
                                 dfeat_out, hidden);
     else
-      rc = basis_proj_grads_blocks(st, K, C, ns, n_in, M, basis, features, neighbors, ranges, w.dx,
+      rc = basis_proj_grads_blocks(st, K, C, ns, M, basis, features, neighbors, ranges, w.dx,
                                    dbasis_out, dfeat_out, hidden);
   }
   if (rc) return rc;
-  // dW[C*K, Cout] = X^T * dOut: both operands have the reduction (sample) index
-  // as their row index, i.e. they are MN-major
-  GemmProblem p{};
-  p.M = ch;
-  p.N = co;
-  p.K = ns;
-  p.a = GemmOperand{w.x_hi, w.x_mid, ck, Major::MN, ch};
-  p.b = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN, co};
-  p.c = padded ? w.dw_pad : dweights_out;
-  p.ldc = co;
-  p.batches = groups;
-  p.c_batch_stride = ch * co;
-  rc = gemm_bf16x3(st, p, w.err);
+  rc = gemm_bf16x3(st, pw, w.err);
   if (rc || !padded) return rc;
   crop_weights_kernel<<<blocks_for(weight_elems, 256), 256, 0, st>>>(weight_elems, cout_src, Cout,
                                                                      k_src, K, w.dw_pad, dweights_out);
@@ -388,16 +412,6 @@ int check_grouped_args(const char* op, int K, int C, int Cout, const void* featu
   return TFGPC_OK;
 }
 
-// The projection in the plan's visiting order, into the workspace.
-int project_grouped(cudaStream_t st, int C, int64_t ns, int64_t n_in, int64_t M,
-                    const void* basis_pair, const float* features, const void* plan,
-                    const McWs& w) {
-  int rc = split_features(st, features, n_in, C, w.fs);
-  if (rc) return rc;
-  return basis_proj_fwd_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, w.x_hi,
-                            w.x_mid, w.err);
-}
-
 }  // namespace
 
 // Forward pass on the rows of a group plan: the projection is computed once per
@@ -421,10 +435,14 @@ extern "C" int tfgpc_mcconv_forward_grouped(
   cudaStream_t st = (cudaStream_t)stream;
   McWs w = carve(ws, K, C, Cout, ns, n_in, false);
   const int64_t ck = (int64_t)C * K;
-  TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-  rc = project_grouped(st, C, ns, n_in, M, basis_pair, features, plan, w);
+  Prepare jobs;
+  jobs.zero(w.err, sizeof(int));
+  jobs.add(feature_job(features, n_in, C, w.fs));
+  jobs.add(weight_job(w, weights, ck, K, Cout, Blocks{1, K, Cout}));
+  rc = prepare(st, jobs);
   if (rc) return rc;
-  rc = split_rows(st, weight_job(w, weights, ck, K, Cout, Blocks{1, K, Cout}));
+  rc = basis_proj_fwd_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, w.x_hi, w.x_mid,
+                          w.err);
   if (rc) return rc;
   GemmOperand a{w.x_hi, w.x_mid, ck, Major::K};
   GemmOperand b{w.w_hi, w.w_mid, (int64_t)Cout, Major::MN};
@@ -463,10 +481,10 @@ extern "C" int tfgpc_mcconv_backward_grouped(
     return fail(TFGPC_ENOMEM, "MCConvBackward workspace too small: %zu < %zu", ws_bytes,
                 tfgpc_mcconv_workspace_bytes(K, C, Cout, ns, n_in, 1));
   McWs w = carve(ws, K, C, Cout, ns, n_in, true);
+  Prepare jobs;
   if (!x_in_workspace) {
-    TFGPC_CUDA(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-    rc = project_grouped(st, C, ns, n_in, M, basis_pair, features, plan, w);
-    if (rc) return rc;
+    jobs.zero(w.err, sizeof(int));
+    jobs.add(feature_job(features, n_in, C, w.fs));
   }
   // X lies in the visiting order (tfgpc_mcconv_forward_grouped wrote it so): the
   // rows of out_grads are brought into the same order while they are split, for
@@ -478,23 +496,10 @@ extern "C" int tfgpc_mcconv_backward_grouped(
   gj.order = order;
   gj.hi = w.g_hi;
   gj.mid = w.g_mid;
-  rc = split_rows(st, gj);
-  if (rc) return rc;
+  jobs.add(gj);
   constexpr int group = 4;
-  if (ns % group != 0) {
-    char* last = (char*)w.dx + (size_t)(ns / group) * 4 * ck * 4;
-    TFGPC_CUDA(cudaMemsetAsync(last, 0, (size_t)4 * ck * 4, st));
-  }
-  rc = split_transpose_to_bf16(st, weights, ck, Cout, Cout, K, K, w.wt_hi, w.wt_mid);
-  if (rc) return rc;
-  GemmOperand wt_mn{w.wt_hi, w.wt_mid, ck, Major::MN};
-  GemmOperand gv_k{w.g_hi, w.g_mid, (int64_t)Cout, Major::K};
-  rc = gemm_bf16x3_grad_image_tn(st, C, ns, Cout, wt_mn, gv_k, w.dx, group, w.err);
-  if (rc) return rc;
-  TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
-  rc = basis_proj_grads_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, ranges, w.dx,
-                            dbasis_out, dfeat_out, w.err);
-  if (rc) return rc;
+  if (ns % group != 0)
+    jobs.zero((char*)w.dx + (size_t)(ns / group) * 4 * ck * 4, (size_t)4 * ck * 4);
   GemmProblem p{};
   p.M = ck;
   p.N = Cout;
@@ -503,6 +508,25 @@ extern "C" int tfgpc_mcconv_backward_grouped(
   p.b = GemmOperand{w.g_hi, w.g_mid, (int64_t)Cout, Major::MN};
   p.c = dweights_out;
   p.ldc = Cout;
+  p.cleared = gemm_adds_slices(p);
+  if (p.cleared) jobs.zero(dweights_out, (size_t)ck * Cout * sizeof(float));
+  jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
+  rc = prepare(st, jobs);
+  if (rc) return rc;
+  if (!x_in_workspace) {
+    rc = basis_proj_fwd_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, w.x_hi,
+                            w.x_mid, w.err);
+    if (rc) return rc;
+  }
+  rc = split_transpose_to_bf16(st, weights, ck, Cout, Cout, K, K, w.wt_hi, w.wt_mid);
+  if (rc) return rc;
+  GemmOperand wt_mn{w.wt_hi, w.wt_mid, ck, Major::MN};
+  GemmOperand gv_k{w.g_hi, w.g_mid, (int64_t)Cout, Major::K};
+  rc = gemm_bf16x3_grad_image_tn(st, C, ns, Cout, wt_mn, gv_k, w.dx, group, w.err);
+  if (rc) return rc;
+  rc = basis_proj_grads_tcu(st, ns, M, plan, (const __nv_bfloat16*)basis_pair, w.fs, ranges, w.dx,
+                            dbasis_out, dfeat_out, w.err);
+  if (rc) return rc;
   return gemm_bf16x3(st, p, w.err);
 }
 
@@ -542,7 +566,6 @@ extern "C" int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K, c
   __nv_bfloat16* a_mid = (__nv_bfloat16*)p; p += align_up((size_t)M * K * 2, 1024);
   __nv_bfloat16* b_hi = (__nv_bfloat16*)p; p += align_up((size_t)N * K * 2, 1024);
   __nv_bfloat16* b_mid = (__nv_bfloat16*)p; p += align_up((size_t)N * K * 2, 1024);
-  TFGPC_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
   SplitJob ja, jb;
   ja.x = a;
   ja.rows = a_transposed ? K : M;
@@ -554,8 +577,6 @@ extern "C" int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K, c
   jb.cols = jb.ld = (int)(b_transposed ? K : N);
   jb.hi = b_hi;
   jb.mid = b_mid;
-  int rc = split_rows(st, ja, &jb);
-  if (rc) return rc;
   // a is [M,K] (K-major) or, transposed, [K,M] (MN-major); b is [K,N] (MN-major)
   // or, transposed, [N,K] (K-major)
   GemmProblem g{};
@@ -566,6 +587,14 @@ extern "C" int tfgpc_matmul_f32(void* stream, int64_t M, int64_t N, int64_t K, c
   g.b = GemmOperand{b_hi, b_mid, b_transposed ? K : N, b_transposed ? Major::K : Major::MN};
   g.c = c;
   g.ldc = N;
+  Prepare jobs;
+  jobs.zero(err, sizeof(int));
+  jobs.add(ja);
+  jobs.add(jb);
+  g.cleared = gemm_adds_slices(g);
+  if (g.cleared) jobs.zero(c, (size_t)M * N * sizeof(float));
+  int rc = prepare(st, jobs);
+  if (rc) return rc;
   return gemm_bf16x3(st, g, err);
 }
 
@@ -607,8 +636,6 @@ extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t co
   jw.ld = (int)up8(cout);
   jw.hi = take((size_t)cin * jw.ld * 2);
   jw.mid = take((size_t)cin * jw.ld * 2);
-  int rc = split_rows(st, jx, &jw);
-  if (rc) return rc;
   const GemmOperand xo{jx.hi, jx.mid, jx.ld, Major::K}, wo{jw.hi, jw.mid, jw.ld, Major::MN};
   GemmProblem g{};
   g.K = cin;
@@ -620,5 +647,12 @@ extern "C" int tfgpc_linear_f32(void* stream, int64_t n, int64_t cin, int64_t co
   g.c = out;
   g.ldc = up8(cout);
   g.bias = bias;
+  Prepare jobs;
+  jobs.add(jx);
+  jobs.add(jw);
+  g.cleared = g.ldc == cout && gemm_adds_slices(g);
+  if (g.cleared) jobs.zero(out, (size_t)n * cout * sizeof(float));
+  int rc = prepare(st, jobs);
+  if (rc) return rc;
   return gemm_bf16x3(st, g, status);
 }
