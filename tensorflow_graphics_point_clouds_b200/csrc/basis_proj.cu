@@ -51,6 +51,7 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
                   const int32_t* __restrict__ ranges, float* __restrict__ out,
                   __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
                   int shift) {
+  chain_enter(ns * G, (int64_t)gridDim.x * kBpThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -152,6 +153,7 @@ basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __rest
                         const float* __restrict__ feat, const int2* __restrict__ neigh,
                         const int32_t* __restrict__ ranges, const float* __restrict__ in_grads,
                         float* __restrict__ dbasis, float* __restrict__ dfeat, int shift) {
+  chain_enter(ns * G, (int64_t)gridDim.x * kBpThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   const int lane = lane_id();
   const int gl = lane & (G - 1);
@@ -305,22 +307,23 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
     int per_sm = 1;
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, out, hi, mid, shift);
-    TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
+        ranges, out, hi, mid, shift));
     return TFGPC_OK;
   }
   if (vec) {
     auto kern = basis_proj_kernel<K, true, OUT>;
     if (smem > 48 * 1024)
       TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
+    TFGPC_CUDA(launch_chained(st, grid, kBpThreads, smem, kern, C, ns, G, basis, feat, neigh,
+        ranges, out, hi, mid, shift));
   } else {
     auto kern = basis_proj_kernel<K, false, OUT>;
     if (smem > 48 * 1024)
       TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
+    TFGPC_CUDA(launch_chained(st, grid, kBpThreads, smem, kern, C, ns, G, basis, feat, neigh,
+        ranges, out, hi, mid, shift));
   }
-  TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
@@ -360,20 +363,16 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M
     int per_sm = 1;
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, in_grads, dbasis,
-                                            dfeat, shift);
-    TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
+        ranges, in_grads, dbasis, dfeat, shift));
     return TFGPC_OK;
   }
   if (vec)
-    basis_proj_grads_kernel<K, true><<<grid, kBpThreads, 0, st>>>(C, ns, M, G, basis, feat, neigh,
-                                                                  ranges, in_grads, dbasis, dfeat,
-                                                                  shift);
+    TFGPC_CUDA(launch_chained(st, grid, kBpThreads, 0, basis_proj_grads_kernel<K, true>, C, ns, M,
+        G, basis, feat, neigh, ranges, in_grads, dbasis, dfeat, shift));
   else
-    basis_proj_grads_kernel<K, false><<<grid, kBpThreads, 0, st>>>(C, ns, M, G, basis, feat, neigh,
-                                                                   ranges, in_grads, dbasis, dfeat,
-                                                                  shift);
-  TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, grid, kBpThreads, 0, basis_proj_grads_kernel<K, false>, C, ns, M,
+        G, basis, feat, neigh, ranges, in_grads, dbasis, dfeat, shift));
   return TFGPC_OK;
 }
 

@@ -146,6 +146,7 @@ basis_proj_fwd_tcu_kernel(int64_t ns, int64_t groups, const int32_t* __restrict_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
+  chain_enter(groups, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -381,10 +382,9 @@ int basis_proj_fwd_tcu(cudaStream_t st, int64_t ns, int64_t M, const void* plan,
   const int grid = (int)(v.groups < sm_count() ? v.groups : sm_count());
   if (grid == 0) return TFGPC_OK;
   ProfScope prof(st, "basis_proj_fwd_tcu");
-  kern<<<grid, kThreads, kSmemBytes, st>>>(ns, v.groups, v.group_begin, v.group_rows, v.rows_id,
-                                           v.rows_pair, basis_pair, fs, x_hi, x_mid,
-                                           make_idesc(kC, 16 * kG, true, true), err_flag);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kThreads, kSmemBytes, kern, ns, v.groups, v.group_begin,
+      v.group_rows, v.rows_id, v.rows_pair, basis_pair, fs, x_hi, x_mid,
+      make_idesc(kC, 16 * kG, true, true), err_flag));
   return TFGPC_OK;
 }
 

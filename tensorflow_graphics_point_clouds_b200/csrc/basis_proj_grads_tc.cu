@@ -105,6 +105,7 @@ basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basi
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
+  chain_enter(groups, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -459,11 +460,9 @@ static int launch_grads_tc(cudaStream_t st, int64_t ns, int64_t M, const float* 
   const int64_t groups = (ns + G - 1) / G;
   const int grid = (int)(groups < sm_count() ? groups : sm_count());
   ProfScope prof(st, "basis_proj_grads_tc");
-  kern<<<grid, kThreads, kSmemBytes, st>>>(ns, M, basis, fs, (const int2*)neigh, ranges,
-                                           (const uint8_t*)image, dbasis, dfeat,
-                                           make_idesc(kRows, 16 * G, false, true),
-                                           make_idesc(kRows, kC, false, false), err_flag);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kThreads, kSmemBytes, kern, ns, M, basis, fs,
+      (const int2*)neigh, ranges, (const uint8_t*)image, dbasis, dfeat,
+      make_idesc(kRows, 16 * G, false, true), make_idesc(kRows, kC, false, false), err_flag));
   return TFGPC_OK;
 }
 

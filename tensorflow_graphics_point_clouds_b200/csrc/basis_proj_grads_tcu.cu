@@ -158,6 +158,7 @@ basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
+  chain_enter(groups, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -446,12 +447,9 @@ int basis_proj_grads_tcu(cudaStream_t st, int64_t ns, int64_t M, const void* pla
   const int grid = (int)(v.groups < sm_count() ? v.groups : sm_count());
   if (grid == 0) return TFGPC_OK;
   ProfScope prof(st, "basis_proj_grads_tcu");
-  kern<<<grid, kThreads, kSmemBytes, st>>>(ns, M, v.groups, v.group_begin, v.group_rows, v.rows_id,
-                                           v.rows_pair, basis_pair, fs, ranges,
-                                           (const uint8_t*)image, dbasis, dfeat,
-                                           make_idesc(128, 16 * kG, false, true),
-                                           make_idesc(kC, 128, false, false), err_flag);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kThreads, kSmemBytes, kern, ns, M, v.groups, v.group_begin,
+      v.group_rows, v.rows_id, v.rows_pair, basis_pair, fs, ranges, (const uint8_t*)image, dbasis,
+      dfeat, make_idesc(128, 16 * kG, false, true), make_idesc(kC, 128, false, false), err_flag));
   return TFGPC_OK;
 }
 

@@ -34,9 +34,8 @@ int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __n
   int rows = sm_count() / s.grid;
   rows = rows < 1 ? 1 : rows > passes ? passes : rows;
   ProfScope prof(st, OUT == 0 ? "basis_proj_mma" : "basis_proj_split_mma");
-  kern<<<dim3(s.grid, rows), cfg::kFwdWarps * 32, smem, st>>>(s.bs, hidden_shift(hidden), C, ns, basis, fs, neigh,
-                                                              ranges, out, hi, mid);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, dim3(s.grid, rows), cfg::kFwdWarps * 32, smem, kern, s.bs,
+      hidden_shift(hidden), C, ns, basis, fs, neigh, ranges, out, hi, mid));
   return TFGPC_OK;
 }
 
@@ -56,9 +55,8 @@ int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* bas
   if (parts < 1) parts = 1;
   Shape s = walk_shape(ns * parts, cfg::kGradWarps);
   ProfScope prof(st, "basis_proj_grads_mma");
-  kern<<<s.grid, cfg::kGradWarps * 32, smem, st>>>(s.bs, (int)parts, hidden_shift(hidden), C, ns, M, basis, fs,
-                                                   neigh, ranges, in_grads, dbasis, dfeat);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, s.grid, cfg::kGradWarps * 32, smem, kern, s.bs, (int)parts,
+      hidden_shift(hidden), C, ns, M, basis, fs, neigh, ranges, in_grads, dbasis, dfeat));
   return TFGPC_OK;
 }
 

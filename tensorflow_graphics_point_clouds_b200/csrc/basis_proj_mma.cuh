@@ -281,6 +281,7 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* __restr
                       const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                       const int32_t* __restrict__ ranges, float* __restrict__ out,
                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
+  chain_enter(ns * 32, (int64_t)gridDim.x * blockDim.x);
   typedef Cfg<K, CC> cfg;
   extern __shared__ __align__(128) uint8_t bpm_smem[];
   const int lane = threadIdx.x & 31;
@@ -436,6 +437,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
                             const int32_t* __restrict__ ranges,
                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
                             float* __restrict__ dfeat) {
+  chain_enter(ns * parts * 32, (int64_t)gridDim.x * blockDim.x);
   typedef Cfg<K, CC> cfg;
   extern __shared__ __align__(128) uint8_t bpm_smem[];
   const int lane = threadIdx.x & 31;

@@ -109,6 +109,7 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
                        const int32_t* __restrict__ ranges, float* __restrict__ out,
                        __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
                        int shift) {
+  chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -226,6 +227,7 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
                              const int32_t* __restrict__ ranges,
                              const float* __restrict__ in_grads, float* __restrict__ dbasis,
                              float* __restrict__ dfeat, int shift) {
+  chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kChunk = 32 * kCpl;
   constexpr int R = kBpwRing;

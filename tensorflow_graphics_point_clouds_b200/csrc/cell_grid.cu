@@ -76,6 +76,7 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
              float* __restrict__ aabb_max, int32_t* __restrict__ num_cells,
              float* __restrict__ scaled_min, float* __restrict__ inv_cell, int32_t* crowded,
              int32_t* page) {
+  chain_enter();
   __shared__ int cells[D];
   __shared__ bool last;
   const int64_t warp = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
@@ -158,6 +159,7 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
 __global__ void given_cells_kernel(int D, const int32_t* __restrict__ given, int max_cells,
                                    int32_t* __restrict__ used, int32_t* crowded,
                                    int32_t* page) {
+  chain_enter();
   if (threadIdx.x != 0) return;
   *crowded = 0;
   int asked[TFGPC_MAX_DIMS];
@@ -201,6 +203,7 @@ keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
                       const float* __restrict__ smin_all, const int32_t* __restrict__ num_cells,
                       const float* __restrict__ inv_cell, int64_t* __restrict__ keys_out,
                       int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded) {
+  chain_enter();
   const Grid<D> g = load_grid<D>(num_cells, inv_cell);
   const int total = total_cells<D>(g.nc, batch_size);
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -226,6 +229,7 @@ __global__ void __launch_bounds__(kThreads)
 scatter_kernel(int64_t n, const int64_t* __restrict__ keys, const int32_t* __restrict__ num_cells,
                int batch_size, const int32_t* __restrict__ start,
                const int32_t* __restrict__ arrival, int32_t* __restrict__ members) {
+  chain_enter();
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
   int nc[D];
@@ -353,6 +357,7 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
              int64_t* __restrict__ skeys, float* __restrict__ spts, int32_t* __restrict__ sbid,
              float4* __restrict__ packed, int2* __restrict__ ds,
              const int32_t* __restrict__ crowded) {
+  chain_enter();
   int nc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
@@ -427,6 +432,7 @@ struct ClusterBuild {
 template <int D>
 __global__ void __launch_bounds__(kClusterThreads, 1)
 grid_cluster_kernel(ClusterBuild a) {
+  chain_enter();
   // [0] ordered keys of the lower corners, [1] complements of those of the upper ones
   __shared__ unsigned box[2][kClusterBoxes];
   __shared__ float smin_s[kClusterBoxes];
@@ -638,7 +644,7 @@ int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
   cudaLaunchConfig_t cfg{};
   cfg.blockDim = dim3(kClusterThreads);
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim = {kMaxRanks, 1, 1};
   cfg.gridDim = dim3(kMaxRanks);
@@ -658,6 +664,9 @@ int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
   const int64_t room = table_cells(D, a.batch_size, a.max_cells) / 16;
   const int64_t threads = a.n > room ? a.n : room;
   while (ranks > 1 && threads <= (int64_t)(ranks / 2) * kClusterThreads) ranks /= 2;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;    // (see launch_chained)
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   cfg.gridDim = dim3(ranks);
   at[0].val.clusterDim = {(unsigned)ranks, 1, 1};
   TFGPC_CUDA(cudaLaunchKernelEx(&cfg, grid_cluster_kernel<D>, a));
@@ -669,22 +678,19 @@ int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
 constexpr int64_t kLargeTilePoints = 131072;
 
 template <int THREADS>
-void launch_place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
+int launch_place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                   const int32_t* batch_ids, const CellGridWs& w) {
-  TFGPC_DIM_SWITCH(g.D, place_kernel<kD, THREADS><<<blocks_for(g.n, THREADS), THREADS, 0, st>>>(
-      g.n, w.members, g.keys, g.num_cells, (int)g.batch_size, g.cell_start, points, batch_ids,
-      g.sorted_indices, g.sorted_keys, g.sorted_points, g.sorted_batch_ids, (float4*)g.packed,
-      (int2*)g.ds, w.crowded));
+  TFGPC_DIM_SWITCH(g.D, TFGPC_CUDA(launch_chained(st, blocks_for(g.n, THREADS), THREADS, 0,
+      place_kernel<kD, THREADS>, g.n, w.members, g.keys, g.num_cells, (int)g.batch_size,
+      g.cell_start, points, batch_ids, g.sorted_indices, g.sorted_keys, g.sorted_points,
+      g.sorted_batch_ids, (float4*)g.packed, (int2*)g.ds, w.crowded)));
+  return TFGPC_OK;
 }
 
 int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const int32_t* batch_ids,
           const CellGridWs& w) {
-  if (g.n >= kLargeTilePoints)
-    launch_place<512>(st, g, points, batch_ids, w);
-  else
-    launch_place<256>(st, g, points, batch_ids, w);
-  TFGPC_LAUNCH_CHECK();
-  return TFGPC_OK;
+  return g.n >= kLargeTilePoints ? launch_place<512>(st, g, points, batch_ids, w)
+                                 : launch_place<256>(st, g, points, batch_ids, w);
 }
 
 }  // namespace
@@ -728,32 +734,30 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   }
   if (num_cells_in) {
     ProfScope prof(st, "grid_params");
-    given_cells_kernel<<<1, 32, 0, st>>>(D, num_cells_in, g.max_cells, g.num_cells, w.crowded,
-                                         page);
+    TFGPC_CUDA(launch_chained(st, 1, 32, 0, given_cells_kernel, D, num_cells_in, g.max_cells,
+        g.num_cells, w.crowded, page));
   } else {
     ProfScope prof(st, "grid_params");
     TFGPC_CUDA(cudaMemsetAsync(w.box_keys, 0xff, w.box_bytes, st));
     unsigned* lo = w.box_keys;
     unsigned* hi = lo + (size_t)B * D;
-    TFGPC_DIM_SWITCH(D, boxes_kernel<kD><<<blocks_for(n, kThreads * kBoxPer), kThreads, 0, st>>>(
-        n, points, batch_ids, B, lo, hi, hi + (size_t)B * D, cs, g.max_cells, g.aabb_min,
-        g.aabb_max, g.num_cells, g.scaled_aabb_min, g.inv_cell_sizes, w.crowded, page));
+    TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks_for(n, kThreads * kBoxPer), kThreads,
+        0, boxes_kernel<kD>, n, points, batch_ids, B, lo, hi, hi + (size_t)B * D, cs, g.max_cells,
+        g.aabb_min, g.aabb_max, g.num_cells, g.scaled_aabb_min, g.inv_cell_sizes, w.crowded,
+        page)));
   }
-  TFGPC_LAUNCH_CHECK();
   {
     ProfScope prof(st, "compute_keys");
     TFGPC_CUDA(cudaMemsetAsync(g.cell_start, 0, (size_t)(cells + 3) * 4, st));
-    TFGPC_DIM_SWITCH(D, keys_histogram_kernel<kD><<<blocks, kThreads, 0, st>>>(
-        n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells, g.inv_cell_sizes, g.keys,
-        g.cell_start, w.arrival, w.crowded));
+    TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0,
+        keys_histogram_kernel<kD>, n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells,
+        g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded)));
   }
-  TFGPC_LAUNCH_CHECK();
   int rc = exclusive_scan_cells(st, g.cell_start, g.num_cells, D, B, cells + 3, w.sums);
   if (rc) return rc;
   ProfScope prof(st, "sort_cells");
-  TFGPC_DIM_SWITCH(D, scatter_kernel<kD><<<blocks, kThreads, 0, st>>>(
-      n, g.keys, g.num_cells, B, g.cell_start, w.arrival, w.members));
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0, scatter_kernel<kD>, n,
+      g.keys, g.num_cells, B, g.cell_start, w.arrival, w.members)));
   return place(st, g, points, batch_ids, w);
 }
 

@@ -295,6 +295,7 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int total) {
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 cells_sample_kernel(SampleArgs a) {
+  chain_enter();
   __shared__ int warp_total[kWarps];
   __shared__ int64_t before_s;
   __shared__ int crowded[kMaxCrowded], num_crowded[2];     // (counters of this pass and the next)

@@ -142,6 +142,7 @@ struct WalkArgs {
 template <int D, int MODE>
 __global__ void __launch_bounds__(kThreads)
 cells_walk_kernel(WalkArgs a) {
+  chain_enter();
   constexpr int kSteps = D <= 3 ? 8 : 4;     // candidates per lane and round
   constexpr int kTubes = num_tubes<D>();
   constexpr int kTop = kTubes > 16 ? 16 : kTubes > 8 ? 8 : kTubes > 4 ? 4 : 2;
@@ -317,9 +318,8 @@ int launch_walk(cudaStream_t st, const char* name, int D, WalkArgs a) {
   a.span = samples_per_warp(a.ns);
   const int64_t warps = (a.ns + a.span - 1) / a.span;
   ProfScope prof(st, name);
-  TFGPC_DIM_SWITCH(D, cells_walk_kernel<kD, MODE>
-                          <<<blocks_for(warps, kThreads / 32), kThreads, 0, st>>>(a));
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks_for(warps, kThreads / 32), kThreads, 0,
+      cells_walk_kernel<kD, MODE>, a)));
   return TFGPC_OK;
 }
 

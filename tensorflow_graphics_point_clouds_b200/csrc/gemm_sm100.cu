@@ -143,6 +143,7 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
+  chain_enter((int64_t)total_tiles * 4, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -504,10 +505,9 @@ int launch(cudaStream_t st, const CUtensorMap* maps, int64_t M, int64_t N, int b
                      : OUT == 2 ? "gemm_bf16x3_mn_k_t"
                      : A_MN ? (B_MN ? "gemm_bf16x3_mn_mn" : "gemm_bf16x3_mn_k")
                             : (B_MN ? "gemm_bf16x3_k_mn" : "gemm_bf16x3_k_k"));
-  kern<<<grid, kThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], M, N, bn, stages,
-                                     make_idesc(kBM, bn, A_MN, B_MN), sch, err_flag, bias, image,
-                                     image_channels, image_group, row_order);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kThreads, smem, kern, maps[0], maps[1], maps[2], maps[3],
+      maps[4], M, N, bn, stages, make_idesc(kBM, bn, A_MN, B_MN), sch, err_flag, bias, image,
+      image_channels, image_group, row_order));
   return TFGPC_OK;
 }
 
@@ -535,6 +535,7 @@ __global__ void __launch_bounds__(256)
 sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, int64_t rows,
                   int cols, const float* __restrict__ bias, float* __restrict__ out, int64_t ldc,
                   int64_t c_batch_stride) {
+  chain_enter();
   const int quads = cols / 4;
   const int64_t per_slice = (int64_t)batches * rows * quads;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -562,6 +563,7 @@ __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows
                                        int cols_src, int k_src, int k_dst,
                                        __nv_bfloat16* __restrict__ hi_t,
                                        __nv_bfloat16* __restrict__ mid_t) {
+  chain_enter();
   __shared__ float tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {
@@ -717,9 +719,9 @@ int gemm_bf16x3(cudaStream_t stream, const GemmProblem& p, int* err_flag) {
     rc = launch<false, false>(stream, maps, p.M, p.N, bn, sch, err_flag, bias);
   if (rc || !apart) return rc;
   ProfScope prof(stream, "sum_slices");
-  sum_slices_kernel<<<blocks_for(p.batches * rows * (cols / 4), 256), 256, 0, stream>>>(
-      p.partials, sch.k_splits, p.batches, rows, (int)cols, p.bias, p.c, p.ldc, p.c_batch_stride);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(stream, blocks_for(p.batches * rows * (cols / 4), 256), 256, 0,
+      sum_slices_kernel, p.partials, sch.k_splits, p.batches, rows, (int)cols, p.bias, p.c, p.ldc,
+      p.c_batch_stride));
   return TFGPC_OK;
 }
 
@@ -728,9 +730,8 @@ int split_transpose_to_bf16(cudaStream_t stream, const float* x, int64_t rows, i
                             __nv_bfloat16* mid_t) {
   if (rows <= 0 || cols <= 0) return TFGPC_OK;
   dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
-  split_transpose_kernel<<<grid, dim3(32, 8), 0, stream>>>(x, rows, cols, cols_src, k_src, k_dst,
-                                                           hi_t, mid_t);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(stream, grid, dim3(32, 8), 0, split_transpose_kernel, x, rows, cols,
+      cols_src, k_src, k_dst, hi_t, mid_t));
   return TFGPC_OK;
 }
 

@@ -59,6 +59,7 @@ __device__ __forceinline__ void sample_range(const int32_t* __restrict__ ranges,
 __global__ void __launch_bounds__(kPlanThreads)
 group_pairs_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order,
                    const int32_t* __restrict__ ranges, int32_t* __restrict__ pairs_out) {
+  chain_enter();
   const int64_t g = (int64_t)blockIdx.x * kPlanThreads + threadIdx.x;
   if (g >= groups) return;
   int total = 0;
@@ -100,6 +101,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
                    const int2* __restrict__ nb_ids, const int32_t* __restrict__ group_begin,
                    int32_t* __restrict__ group_rows, int32_t* __restrict__ rows_id,
                    int4* __restrict__ rows_pair) {
+  chain_enter(groups, (int64_t)gridDim.x * kPlanWarps);
   __shared__ int32_t s_val[kPlanWarps][kMaxMerge];
   __shared__ int16_t s_pre[kPlanWarps][kMaxMerge + 2];
   __shared__ uint32_t s_bits[kPlanWarps][kBitmapBits / 32];
@@ -276,16 +278,14 @@ extern "C" int tfgpc_mcconv_group_plan(void* stream, int64_t ns, int64_t M, cons
   TFGPC_REQUIRE(ranges && (M == 0 || (neighbors_sorted && neighbor_ids)),
                 "group plan got a null pointer");
   ProfScope prof(st, "group_plan");
-  gp::group_pairs_kernel<<<blocks_for(v.groups, gp::kPlanThreads), gp::kPlanThreads, 0, st>>>(
-      ns, v.groups, order, ranges, v.group_begin + 1);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(v.groups, gp::kPlanThreads), gp::kPlanThreads, 0,
+      gp::group_pairs_kernel, ns, v.groups, order, ranges, v.group_begin + 1));
   int rc = inclusive_scan_i32(st, v.group_begin + 1, v.group_begin + 1, v.groups, v.scan_sums,
                               v.scan_sums + scan_block_sums_elems(v.groups));
   if (rc) return rc;
   unsigned grid = min(blocks_for(v.groups, gp::kPlanWarps), (unsigned)(sm_count() * 8));
-  gp::group_merge_kernel<<<grid, gp::kPlanThreads, 0, st>>>(
-      ns, v.groups, order, ranges, (const int2*)neighbors_sorted, (const int2*)neighbor_ids,
-      v.group_begin, v.group_rows, v.rows_id, v.rows_pair);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, gp::kPlanThreads, 0, gp::group_merge_kernel, ns, v.groups,
+      order, ranges, (const int2*)neighbors_sorted, (const int2*)neighbor_ids, v.group_begin,
+      v.group_rows, v.rows_id, v.rows_pair));
   return TFGPC_OK;
 }

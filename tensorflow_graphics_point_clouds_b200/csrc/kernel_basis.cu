@@ -82,6 +82,7 @@ __device__ __forceinline__ float pair_inputs(const float* __restrict__ p_in,
 __global__ void pack_points_density_kernel(int64_t n, const float* __restrict__ pts,
                                            const float* __restrict__ pdf,
                                            float4* __restrict__ out) {
+  chain_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   out[i] = make_float4(__ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
@@ -96,6 +97,7 @@ kernel_basis_kernel(int64_t M, const float* __restrict__ p_in, const float* __re
                     const float* __restrict__ w1, const float* __restrict__ b1, float inv_radius,
                     int act, float alpha, float* __restrict__ basis,
                     __nv_bfloat16* __restrict__ pair, int pdf_by_nbr) {
+  chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   __shared__ float w_s[D * K + K];
   for (int i = threadIdx.x; i < D * K + K; i += kKbThreads)
     w_s[i] = i < D * K ? __ldg(w1 + i) : __ldg(b1 + i - D * K);
@@ -183,6 +185,7 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
                           const float* __restrict__ b1, float inv_radius, int act, float alpha,
                           const float* __restrict__ dbasis, float* __restrict__ dw1,
                           float* __restrict__ db1, int pdf_by_nbr) {
+  chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   constexpr int KT = k_tile(D, K);
   __shared__ float w_s[D * K + K];
   __shared__ float red[(D + 1) * KT];
@@ -277,6 +280,7 @@ kp_basis_kernel(int64_t M, int num_kp, const float* __restrict__ p_in,
                 const float* __restrict__ p_out, const int2* __restrict__ neigh,
                 const float* __restrict__ kernel_points, float inv_radius, float sigma,
                 int interpolation, float* __restrict__ basis) {
+  chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   __shared__ float kp_s[kMaxKernelPoints * D];
   for (int i = threadIdx.x; i < num_kp * D; i += kKbThreads) kp_s[i] = __ldg(kernel_points + i);
   __syncthreads();
@@ -332,6 +336,7 @@ pointconv_pdf_kernel(int64_t ns, const int32_t* __restrict__ ranges,
                      const float* __restrict__ pdf, const float* __restrict__ w1,
                      const float* __restrict__ b1, const float* __restrict__ w2,
                      const float* __restrict__ b2, float* __restrict__ out) {
+  chain_enter(ns * 32, (int64_t)gridDim.x * kKbThreads);
   __shared__ float par[3 * kPdfHidden + 1];
   for (int i = threadIdx.x; i < 3 * kPdfHidden + 1; i += kKbThreads)
     par[i] = i < kPdfHidden ? __ldg(w1 + i)
@@ -396,9 +401,8 @@ extern "C" int tfgpc_pack_points_density(void* stream, int64_t n, const float* p
   TFGPC_REQUIRE((uintptr_t)packed_out % 16 == 0, "PackPointsDensity expects a 16-byte aligned output");
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope prof(st, "pack_points_density");
-  pack_points_density_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, points, pdf,
-                                                               (float4*)packed_out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(n, 256), 256, 0, pack_points_density_kernel, n, points,
+      pdf, (float4*)packed_out));
   return TFGPC_OK;
 }
 
@@ -420,15 +424,14 @@ static int kernel_basis_impl(void* stream, int D, int K, int64_t M, const float*
   unsigned grid = min(blocks_for(M, kKbThreads), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "kernel_basis");
   if ((uintptr_t)basis_out % 32 == 0) {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kernel_basis_kernel<kD, kK, true><<<grid, kKbThreads, 0, st>>>(
-        M, points_in, points_out, (const int2*)neighbors, pdf, w1, b1, inv_radius, activation,
-        alpha, basis_out, pair_out, pdf_by_nbr)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kernel_basis_kernel<kD, kK, true>, M, points_in, points_out, (const int2*)neighbors, pdf,
+        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr))));
   } else {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kernel_basis_kernel<kD, kK, false><<<grid, kKbThreads, 0, st>>>(
-        M, points_in, points_out, (const int2*)neighbors, pdf, w1, b1, inv_radius, activation,
-        alpha, basis_out, pair_out, pdf_by_nbr)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kernel_basis_kernel<kD, kK, false>, M, points_in, points_out, (const int2*)neighbors, pdf,
+        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr))));
   }
-  TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
@@ -480,15 +483,16 @@ extern "C" int tfgpc_kernel_basis_grads(void* stream, int D, int K, int64_t M,
   dim3 grid(min(blocks_for(M, kKbThreads), max(2u * sm_count() / tiles, 1u)), tiles);
   ProfScope prof(st, "kernel_basis_grads");
   if ((uintptr_t)basis_grads % 32 == 0) {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kernel_basis_grads_kernel<kD, kK, true><<<grid, kKbThreads, 0, st>>>(
-        M, points_in, points_out, (const int2*)neighbors, pdf, w1, b1, inv_radius, activation,
-        alpha, basis_grads, dw1_out, db1_out, pdf_by_neighbor)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kernel_basis_grads_kernel<kD, kK, true>, M, points_in, points_out, (const int2*)neighbors,
+        pdf, w1, b1, inv_radius, activation, alpha, basis_grads, dw1_out, db1_out,
+        pdf_by_neighbor))));
   } else {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kernel_basis_grads_kernel<kD, kK, false><<<grid, kKbThreads, 0, st>>>(
-        M, points_in, points_out, (const int2*)neighbors, pdf, w1, b1, inv_radius, activation,
-        alpha, basis_grads, dw1_out, db1_out, pdf_by_neighbor)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kernel_basis_grads_kernel<kD, kK, false>, M, points_in, points_out, (const int2*)neighbors,
+        pdf, w1, b1, inv_radius, activation, alpha, basis_grads, dw1_out, db1_out,
+        pdf_by_neighbor))));
   }
-  TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
@@ -512,15 +516,14 @@ extern "C" int tfgpc_kp_basis(void* stream, int D, int K, int num_kernel_points,
   unsigned grid = min(blocks_for(M, kKbThreads), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "kp_basis");
   if ((uintptr_t)basis_out % 32 == 0) {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kp_basis_kernel<kD, kK, true><<<grid, kKbThreads, 0, st>>>(
-        M, num_kernel_points, points_in, points_out, (const int2*)neighbors, kernel_points,
-        inv_radius, sigma, interpolation, basis_out)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kp_basis_kernel<kD, kK, true>, M, num_kernel_points, points_in, points_out,
+        (const int2*)neighbors, kernel_points, inv_radius, sigma, interpolation, basis_out))));
   } else {
-    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, kp_basis_kernel<kD, kK, false><<<grid, kKbThreads, 0, st>>>(
-        M, num_kernel_points, points_in, points_out, (const int2*)neighbors, kernel_points,
-        inv_radius, sigma, interpolation, basis_out)));
+    TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
+        kp_basis_kernel<kD, kK, false>, M, num_kernel_points, points_in, points_out,
+        (const int2*)neighbors, kernel_points, inv_radius, sigma, interpolation, basis_out))));
   }
-  TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
@@ -535,7 +538,7 @@ extern "C" int tfgpc_pointconv_pdf(void* stream, int64_t ns, int64_t M, const in
   cudaStream_t st = (cudaStream_t)stream;
   unsigned grid = min(blocks_for(ns, kKbThreads / 32), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "pointconv_pdf");
-  pointconv_pdf_kernel<<<grid, kKbThreads, 0, st>>>(ns, ranges, pdf, w1, b1, w2, b2, pdf_out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0, pointconv_pdf_kernel, ns, ranges, pdf, w1, b1,
+      w2, b2, pdf_out));
   return TFGPC_OK;
 }

@@ -120,6 +120,7 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
                         const float* __restrict__ p_out, const int2* __restrict__ neigh,
                         const float* __restrict__ pdf, float inv_radius, int act, float alpha,
                         int pdf_by_nbr, float* __restrict__ basis) {
+  chain_enter(M, (int64_t)gridDim.x * blockDim.x);
   extern __shared__ __align__(16) float par[];
   const int stride = blockDim.x;
   float* diff = par + s.params + threadIdx.x;        // [D][pair]
@@ -177,6 +178,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
                         float* __restrict__ dweights, float* __restrict__ dbiases,
                         float* __restrict__ dp_in, float* __restrict__ dp_out,
                         float* __restrict__ dpdf) {
+  chain_enter(M, (int64_t)gridDim.x * blockDim.x);
   extern __shared__ __align__(16) float par[];       // parameters
   const int tile = blockDim.x;
   const int stride = tile + 4;                       // rows of [unit][pair], banks shifted by 4
@@ -455,10 +457,9 @@ extern "C" int tfgpc_kernel_mlp_basis_layers(
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   unsigned grid = min(blocks_for(M, tile), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "kernel_mlp_basis");
-  kernel_mlp_basis_kernel<<<grid, tile, smem, st>>>(s, M, points_in, points_out,
-                                                    (const int2*)neighbors, pdf, inv_radius,
-                                                    activation, alpha, pdf_by_neighbor, basis_out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, tile, smem, kernel_mlp_basis_kernel, s, M, points_in,
+      points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
+      basis_out));
   return TFGPC_OK;
 }
 
@@ -518,10 +519,8 @@ extern "C" int tfgpc_kernel_mlp_grads_layers(
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   unsigned grid = min(blocks_for(M, tile), (unsigned)(sm_count() * 8));
   ProfScope prof(st, "kernel_mlp_grads");
-  kernel_mlp_grads_kernel<<<grid, tile, smem, st>>>(
-      s, M, points_in, points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha,
-      pdf_by_neighbor, basis_grads, dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out,
-      dpdf_out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, tile, smem, kernel_mlp_grads_kernel, s, M, points_in,
+      points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
+      basis_grads, dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out, dpdf_out));
   return TFGPC_OK;
 }

@@ -126,6 +126,7 @@ struct Blocks {
 // out[(c * k_src + k), o] = padded[(c * k_dst + k), o]
 __global__ void crop_weights_kernel(int64_t n, int cols, int ld, int k_src, int k_dst,
                                     const float* __restrict__ padded, float* __restrict__ out) {
+  chain_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t r = i / cols, c = r / k_src;
@@ -388,9 +389,8 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   if (rc) return rc;
   rc = gemm_bf16x3(st, pw, w.err);
   if (rc || !padded) return rc;
-  crop_weights_kernel<<<blocks_for(weight_elems, 256), 256, 0, st>>>(weight_elems, cout_src, Cout,
-                                                                     k_src, K, w.dw_pad, dweights_out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(weight_elems, 256), 256, 0, crop_weights_kernel,
+      weight_elems, cout_src, Cout, k_src, K, w.dw_pad, dweights_out));
   return TFGPC_OK;
 }
 

@@ -30,6 +30,7 @@ neighborhood_pool_kernel(int mode, int C, int64_t ns, const float* __restrict__ 
                          float* __restrict__ out) {
   const int groups = C / VEC;
   const int64_t total = ns * groups;
+  chain_enter(total, (int64_t)gridDim.x * kPoolThreads);
   for (int64_t i = (int64_t)blockIdx.x * kPoolThreads + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * kPoolThreads) {
     const int64_t s = i / groups;
@@ -74,6 +75,7 @@ __device__ __forceinline__ float key_float(unsigned k) {
 }
 
 __global__ void pool_init_kernel(int mode, int64_t n, float* out, float* counts, int64_t b) {
+  chain_enter();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = mode == 0 ? __uint_as_float(float_key(-FLT_MAX)) : 0.0f;
   if (i < b) counts[i] = 0.0f;
@@ -90,6 +92,7 @@ global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
                    const float* __restrict__ features, const int32_t* __restrict__ batch_ids,
                    float* out, float* counts) {
   const int64_t total = (n + kPoolRun - 1) / kPoolRun * C;
+  chain_enter(total, (int64_t)gridDim.x * kPoolThreads);
   for (int64_t i = (int64_t)blockIdx.x * kPoolThreads + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * kPoolThreads) {
     const int64_t run = i / C;
@@ -126,6 +129,7 @@ global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
 
 __global__ void pool_finish_kernel(int mode, int C, int64_t n, float* out,
                                    const float* __restrict__ counts) {
+  chain_enter();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (mode == 0) {
@@ -137,6 +141,7 @@ __global__ void pool_finish_kernel(int mode, int C, int64_t n, float* out,
 }
 
 __global__ void add_bias_kernel(int64_t n, int C, float* x, const float* __restrict__ bias) {
+  chain_enter();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n * C) x[i] += __ldg(bias + (i % C));
 }
@@ -146,6 +151,7 @@ __global__ void add_bias_kernel(int64_t n, int C, float* x, const float* __restr
 // (modelnet40_small.py:236-243).  act 0: none, 1: leaky ReLU with slope alpha.
 __global__ void scale_bias_act_kernel(int64_t total, int C, float* x, float scale,
                                       const float* __restrict__ bias, int act, float alpha) {
+  chain_enter(total, (int64_t)gridDim.x * blockDim.x);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     float v = x[i] * scale;
@@ -176,8 +182,8 @@ extern "C" int tfgpc_neighborhood_pool(void* stream, int mode, int C, int64_t ns
   const unsigned grid = min(blocks_for(ns * (wide ? C / 4 : C), kPoolThreads),
                             (unsigned)(sm_count() * 32));
   auto kernel = wide ? neighborhood_pool_kernel<4> : neighborhood_pool_kernel<1>;
-  kernel<<<grid, kPoolThreads, 0, st>>>(mode, C, ns, features, (const int2*)neighbors, ranges, out);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, kPoolThreads, 0, kernel, mode, C, ns, features,
+      (const int2*)neighbors, ranges, out));
   return TFGPC_OK;
 }
 
@@ -199,17 +205,16 @@ extern "C" int tfgpc_global_pool(void* stream, int mode, int C, int64_t n, int64
   float* counts = (float*)ws;
   const int64_t cells = batch_size * C;
   const int64_t init = cells > batch_size ? cells : batch_size;
-  pool_init_kernel<<<blocks_for(init, 256), 256, 0, st>>>(mode, cells, out, counts, batch_size);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(init, 256), 256, 0, pool_init_kernel, mode, cells, out,
+      counts, batch_size));
   if (n > 0) {
     const unsigned grid = min(blocks_for((n + kPoolRun - 1) / kPoolRun * C, kPoolThreads),
                               (unsigned)(sm_count() * 32));
-    global_pool_kernel<<<grid, kPoolThreads, 0, st>>>(mode, C, n, batch_size, features, batch_ids,
-                                                      out, counts);
-    TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, grid, kPoolThreads, 0, global_pool_kernel, mode, C, n,
+        batch_size, features, batch_ids, out, counts));
   }
-  pool_finish_kernel<<<blocks_for(cells, 256), 256, 0, st>>>(mode, C, cells, out, counts);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(cells, 256), 256, 0, pool_finish_kernel, mode, C, cells,
+      out, counts));
   return TFGPC_OK;
 }
 
@@ -219,8 +224,7 @@ extern "C" int tfgpc_add_bias(void* stream, int64_t n, int C, float* x, const fl
   TFGPC_REQUIRE(x && bias, "AddBias got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope prof(st, "add_bias");
-  add_bias_kernel<<<blocks_for(n * C, 256), 256, 0, st>>>(n, C, x, bias);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, blocks_for(n * C, 256), 256, 0, add_bias_kernel, n, C, x, bias));
   return TFGPC_OK;
 }
 
@@ -234,7 +238,7 @@ extern "C" int tfgpc_scale_bias_activation(void* stream, int64_t n, int C, float
   cudaStream_t st = (cudaStream_t)stream;
   ProfScope prof(st, "scale_bias_activation");
   unsigned grid = min(blocks_for(n * C, 256), (unsigned)(sm_count() * 16));
-  scale_bias_act_kernel<<<grid, 256, 0, st>>>(n * C, C, x, scale, bias, activation, alpha);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, grid, 256, 0, scale_bias_act_kernel, n * C, C, x, scale, bias,
+      activation, alpha));
   return TFGPC_OK;
 }

@@ -83,6 +83,7 @@ __device__ __forceinline__ void clear_block(const Prepare::Clear& j, int64_t blo
 }
 
 __global__ void __launch_bounds__(256) prepare_kernel(const __grid_constant__ PrepareJobs a) {
+  chain_enter();
   const int block = (int)blockIdx.x;
 #pragma unroll
   for (int i = 0; i < Prepare::kSplits; ++i)
@@ -122,8 +123,7 @@ int prepare(cudaStream_t stream, const Prepare& jobs) {
   a.first_block[Prepare::kSplits + Prepare::kClears] = (int)blocks;
   if (blocks == 0) return TFGPC_OK;
   ProfScope prof(stream, "prepare");
-  prepare_kernel<<<(unsigned)blocks, 256, 0, stream>>>(a);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(stream, (unsigned)blocks, 256, 0, prepare_kernel, a));
   return TFGPC_OK;
 }
 

@@ -41,6 +41,7 @@ __device__ __forceinline__ int64_t elems_of(const ScanSize& s) {
 
 __global__ void __launch_bounds__(kScanThreads)
 scan_reduce_kernel(const int32_t* __restrict__ in, ScanSize size, int64_t* __restrict__ tile_sums) {
+  chain_enter();
   __shared__ int64_t smem[32];
   const int64_t n = elems_of(size);
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
@@ -58,6 +59,7 @@ scan_reduce_kernel(const int32_t* __restrict__ in, ScanSize size, int64_t* __res
 // Tile sums to the sums of the tiles before each, by one block.
 __global__ void __launch_bounds__(1024)
 scan_sums_kernel(ScanSize size, int64_t* tile_sums) {
+  chain_enter();
   __shared__ int64_t smem[32];
   const int64_t n = elems_of(size);
   const int64_t tiles = (n + kScanTile - 1) / kScanTile;
@@ -92,6 +94,7 @@ __global__ void __launch_bounds__(THREADS)
 scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, ScanSize size,
                   const int64_t* __restrict__ tile_sums, bool sums_scanned,
                   int64_t* __restrict__ total, ScanReport rep) {
+  chain_enter();
   constexpr int kTile = THREADS * ITEMS;
   __shared__ int64_t smem[32];
   __shared__ int32_t stage[kTile];
@@ -177,22 +180,20 @@ int scan_impl(cudaStream_t st, const int32_t* in, int32_t* out, const ScanSize& 
               int64_t capacity, int64_t* block_sums, int64_t* total, const ScanReport& rep) {
   ProfScope prof(st, "scan_i32");
   if (capacity <= kOneBlock) {
-    scan_tiles_kernel<kOneThreads, kOneItems, EXCLUSIVE><<<1, kOneThreads, 0, st>>>(
-        in, out, size, nullptr, false, total, rep);
-    TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, 1, kOneThreads, 0,
+        scan_tiles_kernel<kOneThreads, kOneItems, EXCLUSIVE>, in, out, size, nullptr, false, total,
+        rep));
     return TFGPC_OK;
   }
   const unsigned tiles = (unsigned)((capacity + kScanTile - 1) / kScanTile);
-  scan_reduce_kernel<<<tiles, kScanThreads, 0, st>>>(in, size, block_sums);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, tiles, kScanThreads, 0, scan_reduce_kernel, in, size, block_sums));
   const bool scanned = tiles > kDirectTiles;
   if (scanned) {
-    scan_sums_kernel<<<1, 1024, 0, st>>>(size, block_sums);
-    TFGPC_LAUNCH_CHECK();
+    TFGPC_CUDA(launch_chained(st, 1, 1024, 0, scan_sums_kernel, size, block_sums));
   }
-  scan_tiles_kernel<kScanThreads, kScanItems, EXCLUSIVE><<<tiles, kScanThreads, 0, st>>>(
-      in, out, size, block_sums, scanned, total, rep);
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, tiles, kScanThreads, 0,
+      scan_tiles_kernel<kScanThreads, kScanItems, EXCLUSIVE>, in, out, size, block_sums, scanned,
+      total, rep));
   return TFGPC_OK;
 }
 

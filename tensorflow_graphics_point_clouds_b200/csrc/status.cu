@@ -75,6 +75,7 @@ struct Mailbox { void* host; void* dev; };
 thread_local Mailbox g_mail[64] = {};
 
 __global__ void mailbox_kernel(const uint32_t* __restrict__ src, uint32_t* dst, int words) {
+  chain_enter();
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
   __threadfence_system();
 }
@@ -117,8 +118,8 @@ int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_ds
   void* page = nullptr;
   int rc = report_page(&page);
   if (rc) return rc;
-  mailbox_kernel<<<1, 32, 0, st>>>((const uint32_t*)dev_src, (uint32_t*)page, (int)(bytes / 4));
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_CUDA(launch_chained(st, 1, 32, 0, mailbox_kernel, (const uint32_t*)dev_src,
+      (uint32_t*)page, (int)(bytes / 4)));
   return read_report(st, bytes, host_dst);
 }
 
