@@ -216,13 +216,10 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
     w_s[i] = i < D * K ? __ldg(w1 + i) : __ldg(b1 + i - D * K);
   for (int i = threadIdx.x; i < (D + 1) * KT; i += kKbThreads) red[i] = 0.0f;
   __syncthreads();
-  float acc_w[D][KT], acc_b[KT];
+  constexpr int kValues = ((D + 1) * KT + 31) / 32 * 32;
+  float acc[kValues];                     // [D][KT] of the weights, [KT] of the biases
 #pragma unroll
-  for (int k = 0; k < KT; ++k) {
-    acc_b[k] = 0.0f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) acc_w[d][k] = 0.0f;
-  }
+  for (int i = 0; i < kValues; ++i) acc[i] = 0.0f;
   for (; m < M; m += stride) {
     const int64_t next = min(m + stride, M - 1);
     const PairLoads<D> ahead = load_pair<D>(p_in, p_out, pdf, nb_next, next, pdf_by_nbr);
@@ -239,25 +236,36 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
 #pragma unroll
       for (int d = 0; d < D; ++d) pre = fmaf(diff[d], w_s[d * K + k0 + k], pre);
       const float dpre = g[k] * inv_pdf * act_bwd(pre, act, alpha);
-      acc_b[k] += dpre;
+      acc[D * KT + k] += dpre;
 #pragma unroll
-      for (int d = 0; d < D; ++d) acc_w[d][k] = fmaf(diff[d], dpre, acc_w[d][k]);
+      for (int d = 0; d < D; ++d) acc[d * KT + k] = fmaf(diff[d], dpre, acc[d * KT + k]);
     }
     cur = ahead;
 #pragma unroll
     for (int k = 0; k < KT; ++k) g[k] = g_next[k];
   }
-  // warp reduction, then one shared-memory atomic per warp and value
+  // Sums over the warp by halving: at every step a lane hands half of its values to its
+  // partner and keeps the other half, (D + 1) * KT shuffles in all in place of five per
+  // value; then one shared-memory atomic per warp and value.  (20 000 pairs, K 16: 13.0 ->
+  // 4.3 us; 250 000, K 32: 22.8 -> 18.7.)
+  int first = 0;
 #pragma unroll
-  for (int k = 0; k < KT; ++k) {
-    float v = warp_sum(acc_b[k]);
-    if (lane_id() == 0) atomicAdd(&red[D * KT + k], v);
+  for (int step = 0; step < 5; ++step) {
+    const int o = 16 >> step, width = kValues >> (step + 1);
+    const bool upper = (lane_id() & o) != 0;
+    if (upper) first += width;
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      v = warp_sum(acc_w[d][k]);
-      if (lane_id() == 0) atomicAdd(&red[d * KT + k], v);
+    for (int i = 0; i < kValues / 2; ++i) {
+      if (i < width) {
+        const float send = upper ? acc[i] : acc[i + width];
+        const float keep = upper ? acc[i + width] : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
     }
   }
+#pragma unroll
+  for (int i = 0; i < kValues / 32; ++i)
+    if (first + i < (D + 1) * KT) atomicAdd(&red[first + i], acc[i]);
   __syncthreads();
   for (int i = threadIdx.x; i < (D + 1) * KT; i += kKbThreads) {
     const int d = i / KT, k = i % KT;
