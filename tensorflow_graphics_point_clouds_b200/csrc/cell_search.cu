@@ -365,16 +365,19 @@ int check_samples(const char* op, const tfgpc_cell_grid* g, int64_t ns, const fl
   return TFGPC_OK;
 }
 
-// Counts and their scan; the total goes to `total` and to the report page.
+// Counts and their scan; the total goes to `total` and to the report page.  room: where the
+// counts may stand before they are scanned, [ns], or null.
 int count_and_scan(cudaStream_t st, const tfgpc_cell_grid& g, const float* inv_radii, int64_t ns,
                    const SampleSource& src, int max_neighs, int32_t* ranges, int64_t* sums,
-                   int64_t* total, int32_t* page) {
+                   int64_t* total, int32_t* page, int32_t* room) {
   WalkArgs a = walk_args(g, src, ns, inv_radii, max_neighs);
-  a.counts = ranges;
+  const bool apart = room && ns <= kDirectScan;
+  a.counts = apart ? room : ranges;
   int rc = launch_walk<kCount>(st, "find_neighbors_count", g.D, a);
   if (rc) return rc;
   ScanReport rep;
   rep.dst = page + kReportTotal;
+  if (apart) return inclusive_scan_apart(st, room, ranges, ns, total, rep);
   return inclusive_scan_i32(st, ranges, ranges, ns, sums, total, rep);
 }
 
@@ -446,7 +449,8 @@ extern "C" int tfgpc_cell_grid_neighborhood(
   if (ns > 0) {
     rc = count_and_scan(st, g, inv_radii, ns,
                         SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
-                        ranges_out, w.sums, w.total, (int32_t*)page);
+                        ranges_out, w.sums, w.total, (int32_t*)page,
+                        ns <= g.n ? w.arrival : nullptr);     // (free once the grid is built)
     if (rc) return rc;
   }
   return finish_report(st, g.D, g.max_cells, ns > 0, num_cells_host_out, total_out);
@@ -475,7 +479,8 @@ extern "C" int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid, cons
   int64_t* sums = (int64_t*)ws;
   rc = count_and_scan(st, *grid, inv_radii, ns,
                       SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
-                      ranges_out, sums, sums + scan_block_sums_elems(ns), (int32_t*)page);
+                      ranges_out, sums, sums + scan_block_sums_elems(ns), (int32_t*)page,
+                      nullptr);
   if (rc) return rc;
   return finish_report(st, grid->D, grid->max_cells, true, nullptr, total_out);
 }

@@ -169,6 +169,76 @@ scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, Sca
   }
 }
 
+// Up to kDirectScan elements that do not lie where the result goes: every block adds up all
+// elements before its tile itself, at most 32 loads a thread out of L2, in place of a launch
+// for the tile sums (41 000 elements, from the end of the kernel before: 9.9 us with that
+// launch, 6.5 so), and 4096 are two blocks' work, not one's (7.6 -> 3.5).
+constexpr int kDirectThreads = 512;
+constexpr int kDirectTile = 4 * kDirectThreads;
+
+__global__ void __launch_bounds__(kDirectThreads)
+scan_direct_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n,
+                   int64_t* __restrict__ total, ScanReport rep) {
+  chain_enter();
+  constexpr int kWarps = kDirectThreads / 32;
+  __shared__ int64_t tile_s[kWarps], before_s[kWarps];
+  const int4* in4 = reinterpret_cast<const int4*>(in);
+  const int64_t tile0 = (int64_t)blockIdx.x * kDirectTile;
+  int64_t before = 0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < (int)(tile0 / 4); i += kDirectThreads) {
+    const int4 v = __ldg(in4 + i);
+    before += ((int64_t)v.x + v.y) + ((int64_t)v.z + v.w);
+  }
+  const int64_t at = tile0 + 4 * threadIdx.x;
+  int v[4];
+  if (at + 4 <= n) {
+    const int4 q = __ldg(in4 + at / 4);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = at + e < n ? __ldg(in + at + e) : 0;
+  }
+  const int64_t own = ((int64_t)v[0] + v[1]) + ((int64_t)v[2] + v[3]);
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  int64_t x = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+    before += __shfl_xor_sync(0xffffffffu, before, o);
+  }
+  if (lane == 31) {
+    tile_s[w] = x;
+    before_s[w] = before;
+  }
+  __syncthreads();
+  int64_t run = 0;
+#pragma unroll
+  for (int k = 0; k < kWarps; ++k) run += before_s[k] + (k < w ? tile_s[k] : 0);
+  run += x - own;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    run += v[e];
+    v[e] = (int)run;
+  }
+  if (at + 4 <= n && (uintptr_t)out % 16 == 0) {
+    *reinterpret_cast<int4*>(out + at) = make_int4(v[0], v[1], v[2], v[3]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (at + e < n) out[at + e] = v[e];
+  }
+  if (tile0 + kDirectTile >= n && threadIdx.x == kDirectThreads - 1) {
+    if (total) *total = run;
+    if (rep.dst) {
+      for (int i = 0; i < rep.words; ++i) rep.dst[i] = __ldcg(rep.src + i);
+      rep.dst[rep.words] = (int32_t)(uint32_t)run;
+      rep.dst[rep.words + 1] = (int32_t)(run >> 32);
+    }
+  }
+}
+
 constexpr int kOneThreads = 1024;
 constexpr int kOneItems = 8;
 constexpr int64_t kOneBlock = (int64_t)kOneThreads * kOneItems;   // 8192
@@ -206,6 +276,16 @@ int inclusive_scan_i32(cudaStream_t stream, const int32_t* in, int32_t* out, int
     return TFGPC_OK;
   }
   return scan_impl<false>(stream, in, out, ScanSize{n, nullptr, 0, 0}, n, block_sums, total, rep);
+}
+
+int inclusive_scan_apart(cudaStream_t stream, const int32_t* in, int32_t* out, int64_t n,
+                         int64_t* total, ScanReport rep) {
+  TFGPC_REQUIRE(n > 0 && n <= kDirectScan && in != out && (uintptr_t)in % 16 == 0,
+                "scan of too many elements for one launch");
+  ProfScope prof(stream, "scan_i32");
+  TFGPC_CUDA(launch_chained(stream, blocks_for(n, kDirectTile), kDirectThreads, 0,
+      scan_direct_kernel, in, out, n, total, rep));
+  return TFGPC_OK;
 }
 
 int exclusive_scan_cells(cudaStream_t stream, int32_t* table, const int32_t* num_cells, int dims,

@@ -33,6 +33,11 @@ int64_t scan_block_sums_elems(int64_t n);
 int inclusive_scan_i32(cudaStream_t stream, const int32_t* in, int32_t* out, int64_t n,
                        int64_t* block_sums, int64_t* total, ScanReport rep = ScanReport());
 
+// The same of at most kDirectScan counts in one launch; `in` (16-byte aligned) is not `out`.
+constexpr int64_t kDirectScan = 65536;
+int inclusive_scan_apart(cudaStream_t stream, const int32_t* in, int32_t* out, int64_t n,
+                         int64_t* total, ScanReport rep = ScanReport());
+
 // table[i] = sum_{j<i} table[j], in place, over the cells of a grid + 3 (at most
 // `capacity` elements).
 int exclusive_scan_cells(cudaStream_t stream, int32_t* table, const int32_t* num_cells, int dims,
