@@ -267,6 +267,20 @@ int tfgpc_cell_grid_neighborhood(
     int samples_are_points, int max_neighs, int32_t* ranges_out, void* ws,
     size_t ws_bytes, int32_t* num_cells_host_out, int64_t* total_out);
 
+/* The same, followed by the density at every point in the points' own order (pdf_out
+ * [n]; as tfgpc_cells_density with samples_are_points 1) and, with D == 3 and
+ * packed_out, by the table of tfgpc_pack_points_density.  The call returns when its
+ * first part is done, like tfgpc_cell_grid_neighborhood; the densities, which need
+ * nothing from the host, are worked out while it reads the counts and goes on. */
+int tfgpc_cell_grid_neighborhood_pdf(
+    void* stream, const tfgpc_cell_grid* grid, const float* points,
+    const int32_t* batch_ids, const float* cell_sizes,
+    const int32_t* num_cells_in, const float* inv_radii, int64_t ns,
+    const float* samples, const int32_t* samples_batch_ids,
+    int samples_are_points, int max_neighs, int32_t* ranges_out,
+    const float* inv_bandwidth, int pdf_mode, float* pdf_out, float* packed_out,
+    void* ws, size_t ws_bytes, int32_t* num_cells_host_out, int64_t* total_out);
+
 /* Count pass (blocking, workspace of tfgpc_find_neighbors_workspace_bytes) and fill
  * pass of FindNeighbors on a built grid; ids_out may be NULL. */
 int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid,
@@ -710,6 +724,8 @@ int tfgpc_kernel_mlp_grads_layers(
  * tfgpc_pointconv_pdf replaces PointConv.py:168-183: per sample the largest
  * density among its pairs (pairs of sample s end at ranges[s]), then per pair
  * out[m] = relu(pdf[m] / max * w1 + b1) . w2 + b2 with w1, b1, w2 [16], b2 [1].
+ * tfgpc_pointconv_pdf_by_neighbor reads the densities from a table with one value
+ * per point, at the pair's first index (neighbors [M,2] in original ids).
  * The PointConv basis is then tfgpc_kernel_basis with inv_radius 1, pdf_out as
  * its density and the layer's non-linearity (PointConv.py:160-166, 186). */
 int tfgpc_kp_basis(void* stream, int D, int K, int num_kernel_points, int64_t M,
@@ -721,6 +737,12 @@ int tfgpc_pointconv_pdf(void* stream, int64_t ns, int64_t M,
                         const int32_t* ranges, const float* pdf,
                         const float* w1, const float* b1, const float* w2,
                         const float* b2, float* pdf_out);
+int tfgpc_pointconv_pdf_by_neighbor(void* stream, int64_t ns, int64_t M,
+                                    const int32_t* ranges,
+                                    const int32_t* neighbors, const float* pdf,
+                                    const float* w1, const float* b1,
+                                    const float* w2, const float* b2,
+                                    float* pdf_out);
 
 /* ---- pooling and the bias of Conv1x1 ----------------------------------------
  * tfgpc_neighborhood_pool replaces the gather + unsorted_segment_max / _mean

@@ -47,6 +47,7 @@ SYMBOLS = {
     "tfgpc_cell_table_elems": c_sz,
     "tfgpc_cell_grid_workspace_bytes": c_sz,
     "tfgpc_cell_grid_neighborhood": c_int,
+    "tfgpc_cell_grid_neighborhood_pdf": c_int,
     "tfgpc_cells_count": c_int,
     "tfgpc_cells_fill": c_int,
     "tfgpc_cells_density": c_int,
@@ -92,6 +93,7 @@ SYMBOLS = {
     "tfgpc_kernel_mlp_grads_layers": c_int,
     "tfgpc_kp_basis": c_int,
     "tfgpc_pointconv_pdf": c_int,
+    "tfgpc_pointconv_pdf_by_neighbor": c_int,
     "tfgpc_neighborhood_pool": c_int,
     "tfgpc_global_pool_workspace_bytes": c_sz,
     "tfgpc_global_pool": c_int,

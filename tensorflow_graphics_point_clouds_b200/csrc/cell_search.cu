@@ -125,6 +125,7 @@ struct WalkArgs {
   const float* inv_bw;          // kDensity
   int bw_mode;
   float* density;               // kDensity: [ns]
+  float4* packed;               // kDensity, D == 3: [ns] (point, 1 / density), or null
 };
 
 // kCount: number of neighbors.  kFill: the pairs in ascending sorted index, and (ids)
@@ -300,7 +301,12 @@ cells_walk_kernel(WalkArgs a) {
     }
   }
   if (MODE == kCount && s.id >= 0) a.counts[s.id] = min(my_count, a.limit);
-  if (MODE == kDensity && s.id >= 0) a.density[s.id] = (float)(my_density * (norm_exact / norm));
+  if (MODE == kDensity && s.id >= 0) {
+    const float density = (float)(my_density * (norm_exact / norm));
+    a.density[s.id] = density;
+    if (D == 3 && a.packed)
+      a.packed[s.id] = make_float4(s.p[0], s.p[1], s.p[D - 1], 1.0f / density);
+  }
 }
 
 // Samples per warp: more of them share the candidates of a cell (a cell of a uniform
@@ -381,11 +387,12 @@ int count_and_scan(cudaStream_t st, const tfgpc_cell_grid& g, const float* inv_r
   return inclusive_scan_i32(st, ranges, ranges, ns, sums, total, rep);
 }
 
-// Waits for the report and turns it into the outputs of a blocking entry.
+// Waits for the report (marked: see mark_report) and turns it into the outputs of a
+// blocking entry.
 int finish_report(cudaStream_t st, int D, int max_cells, bool with_total,
-                  int32_t* num_cells_host_out, int64_t* total_out) {
+                  int32_t* num_cells_host_out, int64_t* total_out, bool marked = false) {
   int32_t host[kReportWords];
-  int rc = read_report(st, sizeof(host), host);
+  int rc = marked ? read_marked_report(sizeof(host), host) : read_report(st, sizeof(host), host);
   if (rc) return rc;
   for (int d = 0; num_cells_host_out && d < D; ++d) num_cells_host_out[d] = host[d];
   if (num_cells_host_out && host[TFGPC_MAX_DIMS])
@@ -399,6 +406,73 @@ int finish_report(cudaStream_t st, int D, int max_cells, bool with_total,
                 "contract hold at most 2^31-1", (long long)total);
   *total_out = total;
   return TFGPC_OK;
+}
+
+// The density at every point in its own order, and the table of tfgpc_pack_points_density
+// (or null).
+struct DensityRequest {
+  const float* inv_bandwidth;
+  int mode;
+  float* pdf;
+  float4* packed;
+};
+
+int enqueue_density(cudaStream_t st, const tfgpc_cell_grid& g, const SampleSource& src, int64_t ns,
+                    const float* inv_radii, const DensityRequest& d) {
+  WalkArgs a = walk_args(g, src, ns, inv_radii, 0);
+  a.inv_bw = d.inv_bandwidth;
+  a.bw_mode = d.mode;
+  a.density = d.pdf;
+  a.packed = d.packed;
+  return launch_walk<kDensity>(st, "compute_pdf", g.D, a);
+}
+
+int grid_neighborhood(cudaStream_t st, const tfgpc_cell_grid* grid, const float* points,
+                      const int32_t* batch_ids, const float* cell_sizes,
+                      const int32_t* num_cells_in, const float* inv_radii, int64_t ns,
+                      const float* samples, const int32_t* samples_batch_ids,
+                      int samples_are_points, int max_neighs, int32_t* ranges_out,
+                      const DensityRequest* density, void* ws, size_t ws_bytes,
+                      int32_t* num_cells_host_out, int64_t* total_out) {
+  int rc = check_cell_grid("GridNeighborhood", grid);
+  if (rc) return rc;
+  const tfgpc_cell_grid& g = *grid;
+  rc = check_samples("GridNeighborhood", grid, ns, samples, samples_batch_ids,
+                     samples_are_points, max_neighs);
+  if (rc) return rc;
+  TFGPC_REQUIRE(points && batch_ids && cell_sizes && ws && num_cells_host_out && total_out &&
+                (ns == 0 || (ranges_out && inv_radii)), "GridNeighborhood got a null pointer");
+  TFGPC_REQUIRE(!density || ((density->mode == 0 || density->mode == 1) && density->pdf &&
+                             inv_radii && (density->mode == 1 || density->inv_bandwidth) &&
+                             (!density->packed || g.D == 3) && (uintptr_t)density->packed % 16 == 0),
+                "GridNeighborhood: densities need mode 0 or 1, radii, a bandwidth and an output "
+                "(packed: 16-byte aligned, three dimensions)");
+  TFGPC_REQUIRE(num_cells_in != g.num_cells,
+                "GridNeighborhood expects the given cell counts outside the output array");
+  for (int d = 0; d < g.D; ++d)
+    TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "GridNeighborhood expects positive cell sizes");
+  if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, ns, g.batch_size, g.max_cells))
+    return fail(TFGPC_ENOMEM, "GridNeighborhood workspace too small");
+  CellGridWs w = carve_cell_grid(ws, g.n, ns, g.D, g.batch_size, g.max_cells);
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  *total_out = 0;
+  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page);
+  if (rc) return rc;
+  if (ns > 0) {
+    rc = count_and_scan(st, g, inv_radii, ns,
+                        SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
+                        ranges_out, w.sums, w.total, (int32_t*)page,
+                        ns <= g.n ? w.arrival : nullptr);     // (free once the grid is built)
+    if (rc) return rc;
+  }
+  if (density) {
+    rc = mark_report(st);
+    if (!rc) rc = enqueue_density(st, g, SampleSource{1, nullptr, nullptr}, g.n, inv_radii, *density);
+    if (rc) return rc;
+  }
+  return finish_report(st, g.D, g.max_cells, ns > 0, num_cells_host_out, total_out, density != nullptr);
 }
 
 }  // namespace
@@ -424,36 +498,24 @@ extern "C" int tfgpc_cell_grid_neighborhood(
     const float* samples, const int32_t* samples_batch_ids, int samples_are_points,
     int max_neighs, int32_t* ranges_out, void* ws, size_t ws_bytes, int32_t* num_cells_host_out,
     int64_t* total_out) {
-  int rc = check_cell_grid("GridNeighborhood", grid);
-  if (rc) return rc;
-  const tfgpc_cell_grid& g = *grid;
-  rc = check_samples("GridNeighborhood", grid, ns, samples, samples_batch_ids,
-                     samples_are_points, max_neighs);
-  if (rc) return rc;
-  TFGPC_REQUIRE(points && batch_ids && cell_sizes && ws && num_cells_host_out && total_out &&
-                (ns == 0 || (ranges_out && inv_radii)), "GridNeighborhood got a null pointer");
-  TFGPC_REQUIRE(num_cells_in != g.num_cells,
-                "GridNeighborhood expects the given cell counts outside the output array");
-  for (int d = 0; d < g.D; ++d)
-    TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "GridNeighborhood expects positive cell sizes");
-  if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, ns, g.batch_size, g.max_cells))
-    return fail(TFGPC_ENOMEM, "GridNeighborhood workspace too small");
-  cudaStream_t st = (cudaStream_t)stream;
-  CellGridWs w = carve_cell_grid(ws, g.n, ns, g.D, g.batch_size, g.max_cells);
-  void* page = nullptr;
-  rc = report_page(&page);
-  if (rc) return rc;
-  *total_out = 0;
-  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page);
-  if (rc) return rc;
-  if (ns > 0) {
-    rc = count_and_scan(st, g, inv_radii, ns,
-                        SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
-                        ranges_out, w.sums, w.total, (int32_t*)page,
-                        ns <= g.n ? w.arrival : nullptr);     // (free once the grid is built)
-    if (rc) return rc;
-  }
-  return finish_report(st, g.D, g.max_cells, ns > 0, num_cells_host_out, total_out);
+  return grid_neighborhood((cudaStream_t)stream, grid, points, batch_ids, cell_sizes, num_cells_in,
+                           inv_radii, ns, samples, samples_batch_ids, samples_are_points,
+                           max_neighs, ranges_out, nullptr, ws, ws_bytes, num_cells_host_out,
+                           total_out);
+}
+
+extern "C" int tfgpc_cell_grid_neighborhood_pdf(
+    void* stream, const tfgpc_cell_grid* grid, const float* points, const int32_t* batch_ids,
+    const float* cell_sizes, const int32_t* num_cells_in, const float* inv_radii, int64_t ns,
+    const float* samples, const int32_t* samples_batch_ids, int samples_are_points,
+    int max_neighs, int32_t* ranges_out, const float* inv_bandwidth, int pdf_mode, float* pdf_out,
+    float* packed_out, void* ws, size_t ws_bytes, int32_t* num_cells_host_out,
+    int64_t* total_out) {
+  const DensityRequest density{inv_bandwidth, pdf_mode, pdf_out, (float4*)packed_out};
+  return grid_neighborhood((cudaStream_t)stream, grid, points, batch_ids, cell_sizes, num_cells_in,
+                           inv_radii, ns, samples, samples_batch_ids, samples_are_points,
+                           max_neighs, ranges_out, &density, ws, ws_bytes, num_cells_host_out,
+                           total_out);
 }
 
 extern "C" int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid, const float* inv_radii,
@@ -520,10 +582,7 @@ extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
   TFGPC_REQUIRE(mode == 0 || mode == 1, "ComputePdf expects mode 0 or 1 (got %d)", mode);
   if (ns == 0) return TFGPC_OK;
   TFGPC_REQUIRE(inv_radii && pdf_out && (mode == 1 || inv_bandwidth), "ComputePdf got a null pointer");
-  WalkArgs a = walk_args(*grid, SampleSource{samples_are_points, samples, samples_batch_ids}, ns,
-                         inv_radii, 0);
-  a.inv_bw = inv_bandwidth;
-  a.bw_mode = mode;
-  a.density = pdf_out;
-  return launch_walk<kDensity>((cudaStream_t)stream, "compute_pdf", grid->D, a);
+  return enqueue_density((cudaStream_t)stream, *grid,
+                         SampleSource{samples_are_points, samples, samples_batch_ids}, ns,
+                         inv_radii, DensityRequest{inv_bandwidth, mode, pdf_out, nullptr});
 }

@@ -76,6 +76,11 @@ int read_small(cudaStream_t st, const void* dev_src, size_t bytes, void* host_ds
 int report_page(void** dev_page);
 int read_report(cudaStream_t st, size_t bytes, void* host_dst);
 
+// For what is enqueued between a report and its reading, and need not be waited for:
+// mark_report behind the report, read_marked_report in place of read_report.
+int mark_report(cudaStream_t st);
+int read_marked_report(size_t bytes, void* host_dst);
+
 // ---- launches ----------------------------------------------------------------
 //
 // A layer is a chain of some twenty kernels of a few microseconds each, every one reading

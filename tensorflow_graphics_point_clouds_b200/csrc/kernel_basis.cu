@@ -336,12 +336,13 @@ kp_basis_kernel(int64_t M, int num_kp, const float* __restrict__ p_in,
 // Density transform of PointConv (PointConv.py:168-183): per sample the largest
 // density among its neighbor pairs, then per pair
 //   out[m] = sum_j relu(pdf[m] / max * w1[j] + b1[j]) * w2[j] + b2      (j < 16)
-// One warp owns one sample; its pairs are contiguous (ranges holds their end).
+// One warp owns one sample; its pairs are contiguous (ranges holds their end).  neigh null:
+// pdf holds a density per pair, else one per point, read at the pair's neighbor index.
 constexpr int kPdfHidden = 16;
 
 __global__ void __launch_bounds__(kKbThreads)
 pointconv_pdf_kernel(int64_t ns, const int32_t* __restrict__ ranges,
-                     const float* __restrict__ pdf, const float* __restrict__ w1,
+                     const int2* __restrict__ neigh, const float* __restrict__ pdf, const float* __restrict__ w1,
                      const float* __restrict__ b1, const float* __restrict__ w2,
                      const float* __restrict__ b2, float* __restrict__ out) {
   chain_enter(ns * 32, (int64_t)gridDim.x * kKbThreads);
@@ -357,11 +358,12 @@ pointconv_pdf_kernel(int64_t ns, const int32_t* __restrict__ ranges,
     const int a = s ? __ldg(ranges + s - 1) : 0;
     const int e = __ldg(ranges + s);
     float mx = -INFINITY;
-    for (int m = a + lane; m < e; m += 32) mx = fmaxf(mx, __ldg(pdf + m));
+    auto density = [&](int m) { return __ldg(pdf + (neigh ? __ldg(&neigh[m].x) : m)); };
+    for (int m = a + lane; m < e; m += 32) mx = fmaxf(mx, density(m));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     for (int m = a + lane; m < e; m += 32) {
-      const float x = __ldg(pdf + m) / mx;
+      const float x = density(m) / mx;
       float acc = 0.0f;
 #pragma unroll
       for (int j = 0; j < kPdfHidden; ++j)
@@ -535,9 +537,9 @@ extern "C" int tfgpc_kp_basis(void* stream, int D, int K, int num_kernel_points,
   return TFGPC_OK;
 }
 
-extern "C" int tfgpc_pointconv_pdf(void* stream, int64_t ns, int64_t M, const int32_t* ranges,
-                                   const float* pdf, const float* w1, const float* b1,
-                                   const float* w2, const float* b2, float* pdf_out) {
+static int pointconv_pdf(void* stream, int64_t ns, int64_t M, const int32_t* ranges,
+                         const int32_t* neighbors, const float* pdf, const float* w1,
+                         const float* b1, const float* w2, const float* b2, float* pdf_out) {
   TFGPC_REQUIRE(ns >= 0 && ns < (int64_t)INT32_MAX && M >= 0 && M <= (int64_t)INT32_MAX,
                 "PointConvPdf expects 0 <= ns, M < 2^31");
   if (ns == 0 || M == 0) return TFGPC_OK;
@@ -546,7 +548,21 @@ extern "C" int tfgpc_pointconv_pdf(void* stream, int64_t ns, int64_t M, const in
   cudaStream_t st = (cudaStream_t)stream;
   unsigned grid = min(blocks_for(ns, kKbThreads / 32), (unsigned)(sm_count() * 16));
   ProfScope prof(st, "pointconv_pdf");
-  TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0, pointconv_pdf_kernel, ns, ranges, pdf, w1, b1,
-      w2, b2, pdf_out));
+  TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0, pointconv_pdf_kernel, ns, ranges,
+      (const int2*)neighbors, pdf, w1, b1, w2, b2, pdf_out));
   return TFGPC_OK;
+}
+
+extern "C" int tfgpc_pointconv_pdf(void* stream, int64_t ns, int64_t M, const int32_t* ranges,
+                                   const float* pdf, const float* w1, const float* b1,
+                                   const float* w2, const float* b2, float* pdf_out) {
+  return pointconv_pdf(stream, ns, M, ranges, nullptr, pdf, w1, b1, w2, b2, pdf_out);
+}
+
+extern "C" int tfgpc_pointconv_pdf_by_neighbor(void* stream, int64_t ns, int64_t M,
+                                               const int32_t* ranges, const int32_t* neighbors,
+                                               const float* pdf, const float* w1, const float* b1,
+                                               const float* w2, const float* b2, float* pdf_out) {
+  TFGPC_REQUIRE(ns == 0 || M == 0 || neighbors, "PointConvPdf got a null pointer");
+  return pointconv_pdf(stream, ns, M, ranges, neighbors, pdf, w1, b1, w2, b2, pdf_out);
 }

@@ -67,11 +67,11 @@ int sm_count() {
 // 16 ms behind an 800 MB download).  Instead a one-warp kernel writes the values
 // into a page of mapped pinned host memory and the host reads them after
 // synchronising the stream.  One page per host thread and device, allocated on
-// first use and kept.
+// first use and kept, and with it an event (mark_report).
 namespace {
 
 constexpr size_t kPageBytes = 4096;
-struct Mailbox { void* host; void* dev; };
+struct Mailbox { void* host; void* dev; cudaEvent_t mark; };
 thread_local Mailbox g_mail[64] = {};
 
 __global__ void mailbox_kernel(const uint32_t* __restrict__ src, uint32_t* dst, int words) {
@@ -88,6 +88,7 @@ static int mailbox_of(Mailbox** out) {
   TFGPC_REQUIRE(dev >= 0 && dev < 64, "read_small: device index out of range");
   Mailbox& m = g_mail[dev];
   if (!m.host) {
+    if (!m.mark) TFGPC_CUDA(cudaEventCreateWithFlags(&m.mark, cudaEventDisableTiming));
     TFGPC_CUDA(cudaHostAlloc(&m.host, kPageBytes, cudaHostAllocMapped));
     TFGPC_CUDA(cudaHostGetDevicePointer(&m.dev, m.host, 0));
   }
@@ -108,6 +109,23 @@ int read_report(cudaStream_t st, size_t bytes, void* host_dst) {
   int rc = mailbox_of(&m);
   if (rc) return rc;
   TFGPC_CUDA(cudaStreamSynchronize(st));
+  memcpy(host_dst, m->host, bytes);
+  return TFGPC_OK;
+}
+
+int mark_report(cudaStream_t st) {
+  Mailbox* m = nullptr;
+  int rc = mailbox_of(&m);
+  if (rc) return rc;
+  TFGPC_CUDA(cudaEventRecord(m->mark, st));
+  return TFGPC_OK;
+}
+
+int read_marked_report(size_t bytes, void* host_dst) {
+  Mailbox* m = nullptr;
+  int rc = mailbox_of(&m);
+  if (rc) return rc;
+  TFGPC_CUDA(cudaEventSynchronize(m->mark));
   memcpy(host_dst, m->host, bytes);
   return TFGPC_OK;
 }

@@ -140,12 +140,13 @@ static std::vector<float> to_floats(const std::vector<double>& v) {
   return std::vector<float>(v.begin(), v.end());
 }
 
-// (grid, count or None)
+// (grid, count or None, density at the points in their own order or None, table of
+// tfgpc_pack_points_density or None); the last two with inv_bandwidth
 static py::tuple build_grid(const Tensor& points, const Tensor& batch_ids, int64_t batch_size,
                             const std::vector<double>& cell_sizes, int max_cells,
                             const py::object& cells, const OptTensor& inv_radii, int mode,
                             const OptTensor& samples, const OptTensor& sample_ids,
-                            int max_neighs) {
+                            int max_neighs, const OptTensor& inv_bandwidth, int pdf_mode) {
   GridPtr grid = std::make_shared<CellGrid>(points, batch_ids, batch_size, max_cells, cells);
   CountPtr count;
   if (mode >= 0) {
@@ -161,22 +162,39 @@ static py::tuple build_grid(const Tensor& points, const Tensor& batch_ids, int64
   Tensor ws = bytes(need, grid->points);
   const std::vector<float> sizes = to_floats(cell_sizes);
   require((int)sizes.size() == grid->g.D, "GridNeighborhood expects one cell size per dimension");
+  OptTensor pdf, packed;
+  Tensor inv_bw;
+  if (inv_bandwidth) {
+    require(inv_radii.has_value(), "GridNeighborhood: densities need radii");
+    inv_bw = f32(*inv_bandwidth);
+    pdf = empty({grid->g.n}, at::kFloat, grid->points);
+    if (grid->g.D == 3) packed = empty({grid->g.n, 4}, at::kFloat, grid->points);
+  }
   std::vector<int32_t> nc(grid->g.D);
   int64_t total = 0;
   void* st = stream();
   int rc;
   {
     py::gil_scoped_release release;
-    rc = tfgpc_cell_grid_neighborhood(
-        st, &grid->g, fp(grid->points), ip(grid->batch_ids), sizes.data(), grid->cells_in(),
-        count ? fp(count->inv_radii) : nullptr, ns, count ? count->samples.p() : nullptr,
-        count ? count->samples.b() : nullptr, count ? count->samples.mode : 0, max_neighs,
-        count ? ipm(count->ranges) : nullptr, ws.data_ptr(), need, nc.data(), &total);
+    const float* radii = count ? fp(count->inv_radii) : nullptr;
+    const float* smp = count ? count->samples.p() : nullptr;
+    const int32_t* smp_ids = count ? count->samples.b() : nullptr;
+    const int smp_mode = count ? count->samples.mode : 0;
+    int32_t* ranges = count ? ipm(count->ranges) : nullptr;
+    rc = pdf ? tfgpc_cell_grid_neighborhood_pdf(
+                   st, &grid->g, fp(grid->points), ip(grid->batch_ids), sizes.data(),
+                   grid->cells_in(), radii, ns, smp, smp_ids, smp_mode, max_neighs, ranges,
+                   fp(inv_bw), pdf_mode, fpm(*pdf), packed ? fpm(*packed) : nullptr,
+                   ws.data_ptr(), need, nc.data(), &total)
+             : tfgpc_cell_grid_neighborhood(
+                   st, &grid->g, fp(grid->points), ip(grid->batch_ids), sizes.data(),
+                   grid->cells_in(), radii, ns, smp, smp_ids, smp_mode, max_neighs, ranges,
+                   ws.data_ptr(), need, nc.data(), &total);
   }
   if (rc) raise_error(rc, tfgpc_last_error(), &nc);
   grid->num_cells_host = nc;
   if (count) count->total = total;
-  return py::make_tuple(grid, count);
+  return py::make_tuple(grid, count, pdf, packed);
 }
 
 static CountPtr count_neighbors(const GridPtr& grid, const Tensor& inv_radii, int mode,

@@ -154,11 +154,21 @@ Tensor kp_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
 }
 
 Tensor pointconv_pdf(const Tensor& pdf_, const Tensor& ranges_, const Tensor& w1_,
-                     const Tensor& b1_, const Tensor& w2_, const Tensor& b2_) {
+                     const Tensor& b1_, const Tensor& w2_, const Tensor& b2_,
+                     const OptTensor& neigh_) {
   Tensor pdf = f32(pdf_), ranges = i32(ranges_), w1 = f32(w1_), b1 = f32(b1_), w2 = f32(w2_),
          b2 = f32(b2_);
   require(w1.numel() == 16 && b1.numel() == 16 && w2.numel() == 16 && b2.numel() == 1,
           "PointConv's density transform has 16 hidden units");
+  if (neigh_) {
+    Tensor neigh = i32(*neigh_);
+    require(neigh.dim() == 2 && neigh.size(1) == 2, "PointConvPdf expects two indices per pair");
+    Tensor out = empty({neigh.size(0)}, at::kFloat, pdf);
+    check(tfgpc_pointconv_pdf_by_neighbor(stream(), ranges.size(0), neigh.size(0), ip(ranges),
+                                          ip(neigh), fp(pdf), fp(w1), fp(b1), fp(w2), fp(b2),
+                                          fpm(out)));
+    return out;
+  }
   Tensor out = at::empty_like(pdf);
   check(tfgpc_pointconv_pdf(stream(), ranges.size(0), pdf.numel(), ip(ranges), fp(pdf), fp(w1),
                             fp(b1), fp(w2), fp(b2), fpm(out)));

@@ -197,6 +197,12 @@ def _grouped_supported(k, c):
   return _lib.lib().tfgpc_mcconv_grouped_supported(c_int(k), c_int(c)) != 0
 
 
+def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
+  from . import pc
+  return pc.grid_neighborhood_with_pdf(point_cloud_in, radius, point_cloud_out,
+                                       bandwidth=bandwidth)
+
+
 class MCConv:
   """Monte-Carlo convolution layer (MCConv.py:36-278) with explicit backward.
 
@@ -244,7 +250,11 @@ class MCConv:
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    neigh = neighborhood or self.build_neighborhood(point_cloud_in, point_cloud_out, radius)
+    neigh = neighborhood
+    if neigh is None:
+      own = getattr(self.build_neighborhood, '__func__', None) is MCConv.build_neighborhood
+      neigh = (_neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth) if own
+               else self.build_neighborhood(point_cloud_in, point_cloud_out, radius))
     # the densities as a per-point table where the neighborhood has them so (it
     # then never forms the per-pair array), else per pair
     pdf = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0)
@@ -262,7 +272,8 @@ class MCConv:
     # (points, 1 / density) as one 16-byte row per point: one gather per pair
     kb_in, kb_pdf, kb_mode = p_in, pdf, int(by_nbr)
     if one_layer and by_nbr and self.dims == 3:
-      kb_in, kb_pdf, kb_mode = pack_points_density(p_in, pdf), None, 2
+      packed = neigh._packed
+      kb_in, kb_pdf, kb_mode = pack_points_density(p_in, pdf) if packed is None else packed, None, 2
     if grouped:
       # the basis only as the bf16 pair the tensor-core kernels read
       basis, pair = kernel_basis_split(kb_in, p_out, ids, kb_pdf, w1, b1, radius, self.activation,
@@ -363,10 +374,11 @@ def kp_basis(points_in, points_out, neighbors, kernel_points, radius, sigma, k_p
                               float(sigma), int(k_pad), {'linear': 0, 'gaussian': 1}[interpolation])
 
 
-def pointconv_pdf(pdf, ranges, w1, b1, w2, b2):
+def pointconv_pdf(pdf, ranges, w1, b1, w2, b2, neighbors=None):
   """Per pair relu(pdf / max over the sample * w1 + b1) . w2 + b2
-  (tfgpc_pointconv_pdf; PointConv.py:168-183)."""
-  return _lib.host().pointconv_pdf(pdf, ranges, w1, b1, w2, b2)
+  (tfgpc_pointconv_pdf; PointConv.py:168-183).  With neighbors [M, 2] pdf is a table
+  with one density per point, read at the pair's first index, in place of one per pair."""
+  return _lib.host().pointconv_pdf(pdf, ranges, w1, b1, w2, b2, neighbors)
 
 
 class _ProjectedConv:
@@ -457,10 +469,16 @@ class PointConv(_ProjectedConv):
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    neigh = self._neighborhood(point_cloud_in, point_cloud_out, radius, neighborhood)
-    pdf = neigh.get_pdf(bandwidth=bandwidth, mode=0)
+    neigh = neighborhood
+    if neigh is None:
+      neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
+    pdf, table_ids = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0), None
+    if pdf is None:
+      pdf = neigh.get_pdf(bandwidth=bandwidth, mode=0)
+    else:
+      table_ids = neigh._original_neigh_ids
     scale = pointconv_pdf(pdf, neigh._samples_neigh_ranges, self.pdf_weights[0],
-                          self.pdf_biases[0], self.pdf_weights[1], self.pdf_biases[1])
+                          self.pdf_biases[0], self.pdf_weights[1], self.pdf_biases[1], table_ids)
     # PointConv.py:272: the kernel input is the point difference itself (radius 1)
     basis = kernel_basis(point_cloud_in._points, point_cloud_out._points,
                          neigh._original_neigh_ids, scale, self.hidden_w, self.hidden_b, 1.0,

@@ -279,6 +279,7 @@ class Neighborhood:
     self.max_neighbors = max_neighbors
     self._counted = counted
     self._nbrs = self._orig_ids = self._pdf = self._point_pdf = self._sample_pdf = None
+    self._packed = None       # (points, 1 / density) as one row per point, where known
     self._pdf_ready = False
     self._transposed = None
     return self
@@ -363,7 +364,7 @@ class Neighborhood:
     g = self._grid
     d = g._point_cloud._dimension
     inv_bw, inv_r = _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii
-    self._pdf = self._point_pdf = self._sample_pdf = None
+    self._pdf = self._point_pdf = self._sample_pdf = self._packed = None
     if g._cells is not None and not (self._equal_samples and self.max_neighbors > 0):
       # straight from the grid, without the list of a self neighborhood; by original
       # index, which the layers read the densities by, unless the samples are sorted
@@ -457,26 +458,39 @@ def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbor
   keys (tfgpc_grid_neighborhood_count) for grids too fine for one.  For a cloud that is
   one shard of a distributed batch (num_cells_reduce set) the cell counts are reduced
   over the ranks on the device, before the main call: still one blocking read."""
+  return grid_neighborhood_with_pdf(point_cloud, radius, point_cloud_sample, max_neighbors, None)
+
+
+def grid_neighborhood_with_pdf(point_cloud, radius, point_cloud_sample=None, max_neighbors=0,
+                               bandwidth=0.2, mode=0):
+  """grid_neighborhood followed by compute_pdf(bandwidth, mode) (None: without it).  The
+  densities need the grid only, so they are worked out while the host reads the number
+  of pairs and goes on."""
   if point_cloud._points.shape[0] == 0:
     return Neighborhood(Grid(point_cloud, radius), radius, point_cloud_sample, max_neighbors)
   sizes = _host_dims(radius, point_cloud._dimension)
   return _grid_neighborhood(point_cloud, radius, sizes, point_cloud_sample, max_neighbors,
-                            _reduced_cells(point_cloud, sizes))
+                            _reduced_cells(point_cloud, sizes), bandwidth, mode)
 
 
-def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cells):
+def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cells,
+                       bandwidth=None, pdf_mode=0):
   """grid_neighborhood of a cloud with points whose counts have been reduced: whether
   a rank's grid fits a table depends on its own share of the batch, and a second
   reduction on some ranks only would meet another one of theirs."""
   dev = pc._points.device
   d = pc._dimension
+  # (the sorted points' densities come in the sorted order: compute_pdf's)
+  with_pdf = bandwidth is not None and point_cloud_sample is not None
   mode = 2 if point_cloud_sample is None else 1 if point_cloud_sample is pc else 0
   smp = point_cloud_sample if mode == 0 else None
   samples = dict(samples=None if smp is None else smp._points,
                  samples_batch_ids=None if smp is None else smp._batch_ids,
                  samples_are_points=mode, max_neighs=max_neighbors)
+  inv_bw = _to_dims(bandwidth, d, dev, inverse=True) if with_pdf else None
   built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells,
-                     inv_radii=_to_dims(radius, d, dev, inverse=True), **samples)
+                     inv_radii=_to_dims(radius, d, dev, inverse=True), inv_bandwidth=inv_bw,
+                     pdf_mode=pdf_mode, **samples)
   grid = object.__new__(Grid)
   grid._cell_sizes = _to_dims(radius, d, dev)
   if built is not None:
@@ -503,7 +517,11 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
     grid._cur_keys, grid._fast_DS = g.pop("keys"), g.pop("ds")
     for name, value in g.items():
       setattr(grid, '_' + name, value)
-  return object.__new__(Neighborhood)._attach(grid, radius, point_cloud_sample, max_neighbors, count)
+  neigh = object.__new__(Neighborhood)._attach(grid, radius, point_cloud_sample, max_neighbors,
+                                               count)
+  if with_pdf and built is not None:
+    neigh._sample_pdf, neigh._packed, neigh._pdf_ready = built[2], built[3], True
+  return neigh
 
 
 # Cells up to this many radii wide are sampled from the grid, wider ones from a neighbor
