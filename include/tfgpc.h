@@ -656,6 +656,22 @@ int tfgpc_kernel_basis_split(void* stream, int D, int K, int64_t M,
                              int pdf_by_neighbor, float* basis_out,
                              void* basis_pair_out);
 
+/* The same (basis_out or basis_pair_out may be NULL) and tfgpc_kernel_basis_grads
+ * with w1 and dw1_out as num_mlps kernel MLPs hold them one after the other,
+ * [num_mlps,D,K / num_mlps] (MCConv.py:92-110); b1 [K] lies the same either way. */
+int tfgpc_kernel_basis_mlps(void* stream, int D, int K, int num_mlps, int64_t M,
+                            const float* points_in, const float* points_out,
+                            const int32_t* neighbors, const float* pdf,
+                            const float* w1, const float* b1, float inv_radius,
+                            int activation, float alpha, int pdf_by_neighbor,
+                            float* basis_out, void* basis_pair_out);
+int tfgpc_kernel_basis_mlps_grads(
+    void* stream, int D, int K, int num_mlps, int64_t M, const float* points_in,
+    const float* points_out, const int32_t* neighbors, const float* pdf,
+    const float* w1, const float* b1, float inv_radius, int activation,
+    float alpha, int pdf_by_neighbor, const float* basis_grads, float* dw1_out,
+    float* db1_out);
+
 /* ---- MCConv kernel MLP, general form ---------------------------------------
  * Replaces the TensorFlow ops of pylib/pc/layers/MCConv.py:163-171 and :264-269
  * and what autodiff makes of them, for kernel MLPs with any number of hidden

@@ -87,6 +87,8 @@ SYMBOLS = {
     "tfgpc_kernel_basis_split": c_int,
     "tfgpc_kernel_basis": c_int,
     "tfgpc_kernel_basis_grads": c_int,
+    "tfgpc_kernel_basis_mlps": c_int,
+    "tfgpc_kernel_basis_mlps_grads": c_int,
     "tfgpc_kernel_mlp_basis": c_int,
     "tfgpc_kernel_mlp_grads": c_int,
     "tfgpc_kernel_mlp_basis_layers": c_int,

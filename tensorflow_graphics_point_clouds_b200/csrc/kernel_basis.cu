@@ -89,6 +89,14 @@ __global__ void pack_points_density_kernel(int64_t n, const float* __restrict__ 
                        1.0f / __ldg(pdf + i));
 }
 
+// Where the weight of dimension d and basis function k lies in [K / hidden, D, hidden]: the
+// kernel MLPs one after the other, as a layer stores them; hidden = K is [D, K].
+template <int D>
+__device__ __forceinline__ int weight_at(int d, int k, int hidden) {
+  const int g = k / hidden;
+  return (g * D + d) * hidden + (k - g * hidden);
+}
+
 // WIDE: rows are 32-byte aligned, 256-bit accesses are allowed.
 template <int D, int K, bool WIDE>
 __global__ void __launch_bounds__(kKbThreads)
@@ -96,11 +104,11 @@ kernel_basis_kernel(int64_t M, const float* __restrict__ p_in, const float* __re
                     const int2* __restrict__ neigh, const float* __restrict__ pdf,
                     const float* __restrict__ w1, const float* __restrict__ b1, float inv_radius,
                     int act, float alpha, float* __restrict__ basis,
-                    __nv_bfloat16* __restrict__ pair, int pdf_by_nbr) {
+                    __nv_bfloat16* __restrict__ pair, int pdf_by_nbr, int hidden) {
   chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   __shared__ float w_s[D * K + K];
   for (int i = threadIdx.x; i < D * K + K; i += kKbThreads)
-    w_s[i] = i < D * K ? __ldg(w1 + i) : __ldg(b1 + i - D * K);
+    w_s[i] = i < D * K ? __ldg(w1 + weight_at<D>(i / K, i % K, hidden)) : __ldg(b1 + i - D * K);
   __syncthreads();
   for (int64_t m = (int64_t)blockIdx.x * kKbThreads + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * kKbThreads) {
@@ -184,7 +192,7 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
                           const float* __restrict__ pdf, const float* __restrict__ w1,
                           const float* __restrict__ b1, float inv_radius, int act, float alpha,
                           const float* __restrict__ dbasis, float* __restrict__ dw1,
-                          float* __restrict__ db1, int pdf_by_nbr) {
+                          float* __restrict__ db1, int pdf_by_nbr, int hidden) {
   chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   constexpr int KT = k_tile(D, K);
   __shared__ float w_s[D * K + K];
@@ -213,7 +221,7 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
   load_row(min(m, M - 1), g);
   PairLoads<D> cur = load_pair<D>(p_in, p_out, pdf, nb, min(m, M - 1), pdf_by_nbr);
   for (int i = threadIdx.x; i < D * K + K; i += kKbThreads)
-    w_s[i] = i < D * K ? __ldg(w1 + i) : __ldg(b1 + i - D * K);
+    w_s[i] = i < D * K ? __ldg(w1 + weight_at<D>(i / K, i % K, hidden)) : __ldg(b1 + i - D * K);
   for (int i = threadIdx.x; i < (D + 1) * KT; i += kKbThreads) red[i] = 0.0f;
   __syncthreads();
   constexpr int kValues = ((D + 1) * KT + 31) / 32 * 32;
@@ -269,7 +277,7 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
   __syncthreads();
   for (int i = threadIdx.x; i < (D + 1) * KT; i += kKbThreads) {
     const int d = i / KT, k = i % KT;
-    if (d < D) atomicAdd(dw1 + d * K + k0 + k, red[i]);
+    if (d < D) atomicAdd(dw1 + weight_at<D>(d, k0 + k, hidden), red[i]);
     else atomicAdd(db1 + k0 + k, red[i]);
   }
 }
@@ -420,9 +428,11 @@ static int kernel_basis_impl(void* stream, int D, int K, int64_t M, const float*
                              const float* points_out, const int32_t* neighbors, const float* pdf,
                              const float* w1, const float* b1, float inv_radius, int activation,
                              float alpha, float* basis_out, __nv_bfloat16* pair_out,
-                             int pdf_by_nbr) {
+                             int pdf_by_nbr, int num_mlps = 1) {
   int rc = check_kb_args("KernelBasis", D, K, M, activation);
   if (rc) return rc;
+  TFGPC_REQUIRE(num_mlps >= 1 && K % num_mlps == 0,
+                "KernelBasis expects as many basis functions from every kernel MLP");
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && (pdf || pdf_by_nbr == 2) && w1 && b1 &&
                 (basis_out || pair_out), "KernelBasis got a null pointer");
@@ -436,11 +446,13 @@ static int kernel_basis_impl(void* stream, int D, int K, int64_t M, const float*
   if ((uintptr_t)basis_out % 32 == 0) {
     TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
         kernel_basis_kernel<kD, kK, true>, M, points_in, points_out, (const int2*)neighbors, pdf,
-        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr))));
+        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr,
+        K / num_mlps))));
   } else {
     TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
         kernel_basis_kernel<kD, kK, false>, M, points_in, points_out, (const int2*)neighbors, pdf,
-        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr))));
+        w1, b1, inv_radius, activation, alpha, basis_out, pair_out, pdf_by_nbr,
+        K / num_mlps))));
   }
   return TFGPC_OK;
 }
@@ -466,15 +478,27 @@ extern "C" int tfgpc_kernel_basis_split(void* stream, int D, int K, int64_t M,
                            (__nv_bfloat16*)basis_pair_out, pdf_by_neighbor);
 }
 
-extern "C" int tfgpc_kernel_basis_grads(void* stream, int D, int K, int64_t M,
-                                        const float* points_in, const float* points_out,
-                                        const int32_t* neighbors, const float* pdf,
-                                        const float* w1, const float* b1, float inv_radius,
-                                        int activation, float alpha, int pdf_by_neighbor,
-                                        const float* basis_grads, float* dw1_out,
-                                        float* db1_out) {
+extern "C" int tfgpc_kernel_basis_mlps(void* stream, int D, int K, int num_mlps, int64_t M,
+                                       const float* points_in, const float* points_out,
+                                       const int32_t* neighbors, const float* pdf,
+                                       const float* w1, const float* b1, float inv_radius,
+                                       int activation, float alpha, int pdf_by_neighbor,
+                                       float* basis_out, void* basis_pair_out) {
+  return kernel_basis_impl(stream, D, K, M, points_in, points_out, neighbors, pdf, w1, b1,
+                           inv_radius, activation, alpha, basis_out,
+                           (__nv_bfloat16*)basis_pair_out, pdf_by_neighbor, num_mlps);
+}
+
+static int kernel_basis_grads_impl(void* stream, int D, int K, int num_mlps, int64_t M,
+                                   const float* points_in, const float* points_out,
+                                   const int32_t* neighbors, const float* pdf, const float* w1,
+                                   const float* b1, float inv_radius, int activation, float alpha,
+                                   int pdf_by_neighbor, const float* basis_grads, float* dw1_out,
+                                   float* db1_out) {
   int rc = check_kb_args("KernelBasisGrads", D, K, M, activation);
   if (rc) return rc;
+  TFGPC_REQUIRE(num_mlps >= 1 && K % num_mlps == 0,
+                "KernelBasisGrads expects as many basis functions from every kernel MLP");
   TFGPC_REQUIRE(dw1_out && db1_out, "KernelBasisGrads got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
   Prepare jobs;
@@ -496,14 +520,36 @@ extern "C" int tfgpc_kernel_basis_grads(void* stream, int D, int K, int64_t M,
     TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
         kernel_basis_grads_kernel<kD, kK, true>, M, points_in, points_out, (const int2*)neighbors,
         pdf, w1, b1, inv_radius, activation, alpha, basis_grads, dw1_out, db1_out,
-        pdf_by_neighbor))));
+        pdf_by_neighbor, K / num_mlps))));
   } else {
     TFGPC_DIM_SWITCH(D, TFGPC_K_SWITCH(K, TFGPC_CUDA(launch_chained(st, grid, kKbThreads, 0,
         kernel_basis_grads_kernel<kD, kK, false>, M, points_in, points_out, (const int2*)neighbors,
         pdf, w1, b1, inv_radius, activation, alpha, basis_grads, dw1_out, db1_out,
-        pdf_by_neighbor))));
+        pdf_by_neighbor, K / num_mlps))));
   }
   return TFGPC_OK;
+}
+
+extern "C" int tfgpc_kernel_basis_grads(void* stream, int D, int K, int64_t M,
+                                        const float* points_in, const float* points_out,
+                                        const int32_t* neighbors, const float* pdf,
+                                        const float* w1, const float* b1, float inv_radius,
+                                        int activation, float alpha, int pdf_by_neighbor,
+                                        const float* basis_grads, float* dw1_out,
+                                        float* db1_out) {
+  return kernel_basis_grads_impl(stream, D, K, 1, M, points_in, points_out, neighbors, pdf, w1, b1,
+                                 inv_radius, activation, alpha, pdf_by_neighbor, basis_grads,
+                                 dw1_out, db1_out);
+}
+
+extern "C" int tfgpc_kernel_basis_mlps_grads(
+    void* stream, int D, int K, int num_mlps, int64_t M, const float* points_in,
+    const float* points_out, const int32_t* neighbors, const float* pdf, const float* w1,
+    const float* b1, float inv_radius, int activation, float alpha, int pdf_by_neighbor,
+    const float* basis_grads, float* dw1_out, float* db1_out) {
+  return kernel_basis_grads_impl(stream, D, K, num_mlps, M, points_in, points_out, neighbors, pdf,
+                                 w1, b1, inv_radius, activation, alpha, pdf_by_neighbor,
+                                 basis_grads, dw1_out, db1_out);
 }
 
 extern "C" int tfgpc_kp_basis(void* stream, int D, int K, int num_kernel_points, int64_t M,

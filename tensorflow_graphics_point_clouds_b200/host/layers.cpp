@@ -22,6 +22,17 @@ Tensor pack_points_density(const Tensor& points_, const Tensor& pdf_) {
   return out;
 }
 
+// Weights of one-layer kernel MLPs: [D, K], or [G, D, K / G] as a layer holds G of them.
+struct OneLayer {
+  int d, k, g;
+  explicit OneLayer(const Tensor& w1) {
+    require(w1.dim() == 2 || w1.dim() == 3, "KernelBasis expects weights [D, K] or [G, D, K / G]");
+    g = w1.dim() == 3 ? (int)w1.size(0) : 1;
+    d = (int)w1.size(-2);
+    k = g * (int)w1.size(-1);
+  }
+};
+
 // (basis [M, K] float32 or None, pair [M, 2, K] bf16 or None)
 py::tuple kernel_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
                        const OptTensor& pdf_, const Tensor& w1_, const Tensor& b1_,
@@ -30,21 +41,19 @@ py::tuple kernel_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& 
   Tensor p_in = f32(p_in_), p_out = f32(p_out_), neigh = i32(neigh_), w1 = f32(w1_), b1 = f32(b1_);
   Tensor pdf_keep;
   const float* pdf = maybe(pdf_, &pdf_keep);
-  const int64_t m = neigh.size(0), k = w1.size(1);
+  const OneLayer mlp(w1);
+  const int64_t m = neigh.size(0);
   OptTensor basis, pair;
-  if (want_f32) basis = empty({m, k}, at::kFloat, p_in);
-  if (want_pair) pair = empty({m, 2, k}, at::kBFloat16, p_in);
-  const float inv = (float)(1.0 / radius);
-  if (want_pair)
-    check(tfgpc_kernel_basis_split(stream(), (int)w1.size(0), (int)k, m, fp(p_in), fp(p_out),
-                                   ip(neigh), pdf, fp(w1), fp(b1), inv, act, (float)alpha,
-                                   pdf_mode, basis ? fpm(*basis) : nullptr, pair->data_ptr()));
-  else
-    check(tfgpc_kernel_basis(stream(), (int)w1.size(0), (int)k, m, fp(p_in), fp(p_out), ip(neigh),
-                             pdf, fp(w1), fp(b1), inv, act, (float)alpha, pdf_mode, fpm(*basis)));
+  if (want_f32) basis = empty({m, mlp.k}, at::kFloat, p_in);
+  if (want_pair) pair = empty({m, 2, mlp.k}, at::kBFloat16, p_in);
+  check(tfgpc_kernel_basis_mlps(stream(), mlp.d, mlp.k, mlp.g, m, fp(p_in), fp(p_out), ip(neigh),
+                                pdf, fp(w1), fp(b1), (float)(1.0 / radius), act, (float)alpha,
+                                pdf_mode, basis ? fpm(*basis) : nullptr,
+                                pair ? pair->data_ptr() : nullptr));
   return py::make_tuple(basis, pair);
 }
 
+// (gradient of the weights in their layout, of the biases [K])
 py::tuple kernel_basis_grads(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
                              const OptTensor& pdf_, const Tensor& w1_, const Tensor& b1_,
                              double radius, const Tensor& dbasis_, int act, double alpha,
@@ -53,13 +62,14 @@ py::tuple kernel_basis_grads(const Tensor& p_in_, const Tensor& p_out_, const Te
          dbasis = f32(dbasis_);
   Tensor pdf_keep;
   const float* pdf = maybe(pdf_, &pdf_keep);
-  const int64_t d = w1.size(0), k = w1.size(1);
-  Tensor both = empty({d + 1, k}, at::kFloat, p_in);   // one clear for both
+  const OneLayer mlp(w1);
+  Tensor both = empty({mlp.d + 1, mlp.k}, at::kFloat, p_in);
   float* dw = fpm(both);
-  check(tfgpc_kernel_basis_grads(stream(), (int)d, (int)k, neigh.size(0), fp(p_in), fp(p_out),
-                                 ip(neigh), pdf, fp(w1), fp(b1), (float)(1.0 / radius), act,
-                                 (float)alpha, pdf_mode, fp(dbasis), dw, dw + d * k));
-  return py::make_tuple(both.narrow(0, 0, d), both.select(0, d));
+  check(tfgpc_kernel_basis_mlps_grads(stream(), mlp.d, mlp.k, mlp.g, neigh.size(0), fp(p_in),
+                                      fp(p_out), ip(neigh), pdf, fp(w1), fp(b1),
+                                      (float)(1.0 / radius), act, (float)alpha, pdf_mode,
+                                      fp(dbasis), dw, dw + (int64_t)mlp.d * mlp.k));
+  return py::make_tuple(both.narrow(0, 0, mlp.d).view(w1.sizes()), both.select(0, mlp.d));
 }
 
 // Parameters of a kernel MLP, one tensor per layer: weights [G, H_{l-1}, H_l], biases

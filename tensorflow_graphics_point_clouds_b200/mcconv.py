@@ -129,7 +129,7 @@ def pack_points_density(points, pdf):
 def kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, radius, activation=0,
                  alpha=0.2, pdf_by_neighbor=False):
   """basis[m, k] = act(diff_m . w1[:, k] + b1[k]) / pdf[m] (tfgpc_kernel_basis).
-  w1 [D, K], b1 [K]; neighbors hold (index into points_in, index into points_out).
+  w1 [D, K] (or [G, D, K / G], G kernel MLPs), b1 [K]; neighbors hold (index into points_in, index into points_out).
   pdf_by_neighbor: pdf is a table with one density per point of points_in, read
   at the pair's neighbor index, instead of the per-pair array."""
   return _lib.host().kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, float(radius),
@@ -235,13 +235,6 @@ class MCConv:
       return self.wf[0]
     return dense_final_weights(self.wf, self.cin, self.hidden)
 
-  def _flat_kernel_weights(self):
-    # [G, D, H] -> [D, G*H]: column k = g*H + h (MCConv.py:169-171)
-    if self.num_mlps == 1:
-      return self.w1[0], self.b1.reshape(self.k)
-    return (self.w1.permute(1, 0, 2).reshape(self.dims, self.k).contiguous(),
-            self.b1.reshape(self.k).contiguous())
-
   def build_neighborhood(self, point_cloud_in, point_cloud_out, radius):
     """MCConv.py:254-261: grid of the input cloud, neighborhood around the
     output points."""
@@ -264,7 +257,8 @@ class MCConv:
     ns = point_cloud_out._points.shape[0]
     p_in, p_out, ids = point_cloud_in._points, point_cloud_out._points, neigh._original_neigh_ids
     one_layer = len(self.kernel_weights) == 1
-    w1, b1 = self._flat_kernel_weights() if one_layer else (None, None)
+    # (column k = g*H + h of the basis belongs to MLP g: MCConv.py:169-171)
+    w1, b1 = (self.w1, self.b1) if one_layer else (None, None)
     # wide layers run on a group plan (see group_plan)
     grouped = (one_layer and self.grouped and neigh._neighbors.shape[0] > 0 and
                self.cout >= 128 and
@@ -347,8 +341,6 @@ class MCConv:
     kb_in, kb_pdf, kb_mode = self._kb_inputs
     dw1, db1 = kernel_basis_grads(kb_in, pc_out._points, ids, kb_pdf, w1, b1, radius, dbasis,
                                   self.activation, self.alpha, pdf_by_neighbor=kb_mode)
-    dw1 = (dw1.unsqueeze(0) if self.num_mlps == 1 else
-           dw1.reshape(self.dims, self.num_mlps, self.hidden).permute(1, 0, 2).contiguous())
     db1 = db1.reshape(self.num_mlps, 1, self.hidden)
     if self._list_form:
       return dfeat, [dw1], [db1], dwf
