@@ -5,15 +5,16 @@ namespace tfgpc {
 
 namespace {
 
-// Blocks of one SM each, and the samples a warp takes at a time: enough work items per
-// warp (four) to even out lists of unequal length, up to the 32 that one load of range
-// ends covers.  (With 32 always, 41 000 samples left 1036 warps one or two blocks each:
-// two waves, the second a quarter full.)
+// Blocks of one SM each, and the samples a warp (or team) takes at a time: enough work
+// items per warp (eight) to even out lists of unequal length, up to the 32 that one load of
+// range ends covers.  (With 32 always, 41 000 samples left 1036 warps one or two blocks
+// each; with four items, gradients of 33 000 ragged samples at C = 64, K = 32 took 183 us,
+// with eight 165, with sixteen 167.)
 struct Shape { int grid, bs; };
 
 Shape walk_shape(int64_t items, int warps) {
   Shape s;
-  int64_t bs = items / ((int64_t)sm_count() * warps * 4);
+  int64_t bs = items / ((int64_t)sm_count() * warps * 8);
   s.bs = (int)(bs < 1 ? 1 : bs > 32 ? 32 : bs);
   int64_t grid = ((items + s.bs - 1) / s.bs + warps - 1) / warps;
   s.grid = (int)(grid < 1 ? 1 : grid > sm_count() ? sm_count() : grid);
@@ -43,19 +44,19 @@ template <int K, int CC>
 int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* basis,
                  const __nv_bfloat16* fs, const int2* neigh, const int32_t* ranges,
                  const float* in_grads, float* dbasis, float* dfeat, int hidden) {
-  typedef bpm::Cfg<K, CC> cfg;
+  typedef bpm::GradCfg<K, CC> cfg;
   auto kern = bpm::basis_proj_grads_mma_kernel<K, CC>;
-  constexpr int smem = cfg::kGradWarps * cfg::kGradWarpBytes;
+  constexpr int smem = cfg::kTeams * cfg::kTeamBytes;
   TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  // few samples with long lists: several warps share a sample's chunks
-  const int64_t warps = (int64_t)sm_count() * cfg::kGradWarps;
-  int64_t parts = ns > 0 ? 2 * warps / ns : 1;
+  // few samples with long lists: several teams share a sample's chunks
+  const int64_t teams = (int64_t)sm_count() * cfg::kTeams;
+  int64_t parts = ns > 0 ? 2 * teams / ns : 1;
   const int64_t most = ns > 0 ? M / ns / (2 * bpm::kChunk) : 1;
   if (parts > most) parts = most;
   if (parts < 1) parts = 1;
-  Shape s = walk_shape(ns * parts, cfg::kGradWarps);
+  Shape s = walk_shape(ns * parts, cfg::kTeams);
   ProfScope prof(st, "basis_proj_grads_mma");
-  TFGPC_CUDA(launch_chained(st, s.grid, cfg::kGradWarps * 32, smem, kern, s.bs, (int)parts,
+  TFGPC_CUDA(launch_chained(st, s.grid, cfg::kThreads, smem, kern, s.bs, (int)parts,
       hidden_shift(hidden), C, ns, M, basis, fs, neigh, ranges, in_grads, dbasis, dfeat));
   return TFGPC_OK;
 }
@@ -101,8 +102,10 @@ int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* b
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          const float* in_grads, float* dbasis, float* dfeat, int hidden) {
-  TFGPC_CC_SWITCH(K, C, return launch_grads<kK, kCC>(st, C, ns, M, basis, fs, (const int2*)neigh,
-                                                     ranges, in_grads, dbasis, dfeat, hidden))
+  // (at K = 16 wide layers take two passes: a team could not share their fragments)
+  TFGPC_CC_SWITCH(K, C, return launch_grads<kK, (kK * kCC > 1024 && kK == 16 ? 64 : kCC)>(
+                            st, C, ns, M, basis, fs, (const int2*)neigh, ranges, in_grads, dbasis,
+                            dfeat, hidden))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 

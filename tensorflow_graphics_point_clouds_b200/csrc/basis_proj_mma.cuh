@@ -44,19 +44,13 @@ struct Cfg {
   static constexpr int kKStride = K * 2 + 16;       // bytes of one bf16 row over k (+ pad)
   static constexpr int kFeatBytes = kChunk * kFeatStride;
   static constexpr int kBasisBytes = 2 * kChunk * kKStride;   // hi rows, then mid rows
-  static constexpr int kDxRawBytes = kCC * K * 4;
-  static constexpr int kDxBytes = 2 * kCC * kKStride;         // hi rows, then mid rows
   static constexpr int kFwdWarpBytes = 2 * kFeatBytes + 2 * kBasisBytes;
-  static constexpr int kGradWarpBytes = kFeatBytes + kBasisBytes + kDxRawBytes + kDxBytes;
   static constexpr int kBasisVecs = K / 8;   // float4 loads per lane for a 16-row basis chunk
   // warps per block (one block per SM): what 64 K registers and 227 KB allow
   static constexpr int kFwdRegWarps = CC * K >= 2048 ? 12 : CC * K >= 1024 ? 16 : 24;
-  static constexpr int kGradRegWarps = K == 64 ? 8 : CC * K >= 2048 ? 8 : CC * K >= 1024 ? 12 : 16;
   static constexpr int kMaxSmem = 227 * 1024;
   static constexpr int kFwdWarps = kFwdRegWarps < kMaxSmem / kFwdWarpBytes
                                        ? kFwdRegWarps : kMaxSmem / kFwdWarpBytes;
-  static constexpr int kGradWarps = kGradRegWarps < kMaxSmem / kGradWarpBytes
-                                        ? kGradRegWarps : kMaxSmem / kGradWarpBytes;
 };
 
 // ---- PTX helpers -----------------------------------------------------------------
@@ -94,6 +88,10 @@ __device__ __forceinline__ void mma3(float* d, const uint32_t* a_hi, const uint3
 
 __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid) {
   split2_bf16(x, y, hi, mid);
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
 // 16-byte asynchronous copy; copies nothing and writes zeros when !valid
@@ -418,237 +416,400 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* __restr
 
 // ---- gradients ---------------------------------------------------------------------------
 //
-// Per sample the incoming gradient dX[s] (C x K floats) is copied raw into
-// shared memory while the previous sample is still being processed, then split
-// once into bf16 hi/mid rows [c][k].  Per chunk of 16 pairs:
-//   (1) dbasis[pair, k] = A[pair, c] * B[c, k]: A straight out of the gathered
-//       feature rows, B transposed out of the dX rows; 128-bit stores;
-//   (2) dfeat[pair, c]  = A[pair, k] * B[k, c]: A out of the staged basis rows,
-//       B out of the dX rows (whose order inside a tile is chosen so that a lane
-//       ends up with four consecutive channels); one 128-bit reduction per lane
-//       and 4 channels into dfeat[nbr(pair)].
-// The feature rows are dead after (1), so the gather of the next chunk is
-// started there and runs under (2).  dbasis is written, not accumulated (every
-// pair belongs to exactly one sample); dfeat must be zero on entry.
+// The incoming gradient dX[s] (C x K floats) takes part in every chunk of a sample, so it
+// is the LEFT operand of both products and stays in registers, split into bf16 hi / mid
+// fragments once per sample, while the pairs stand in the columns, eight at a time:
+//   (1) dbasis^T[k, pair] = A[k, c] * B[c, pair]: B straight out of the gathered feature rows;
+//   (2) dfeat^T[c, pair]  = A[c, k] * B[k, pair]: B out of the staged basis rows; one 128-bit
+//       reduction per lane and 4 channels into dfeat[nbr(pair)], 128 bytes in a row per pair.
+// Both fragment sets together are C * K / 16 registers; where one warp cannot hold them a
+// team of two shares a sample: both warps see all pairs, (1) is split by basis functions and
+// (2) by channels, so that no sum crosses warps.
+// While a chunk is multiplied the next one's feature rows are on their way to the team's
+// other stage and its basis rows to registers, and dX of the next sample to the place that
+// this one's has left for registers.
+// What bounds it: the SM's L1 data path (62 % of its wavefronts, 75 % on the busiest SM:
+// copies into shared memory, operand reads, reductions at ~24 B/clk) and the instructions
+// around the MMAs (issue 50 %).  65 536 samples of 28 pairs at C = 64, K = 32: 345 -> 290 us
+// (1.07 GB: 3.7 TB/s); 41 000 at C = 64, K = 16: 166 -> 139.  (One warp per sample with dX as
+// bf16 rows in shared memory, read by ldmatrix again for every chunk, took 25 KB at C = 64,
+// K = 32 -- 8 warps per SM -- and a chunk of nine pairs cost as much as one of sixteen.
+// Everything straight from global memory to registers, without shared memory, read each
+// piece of dX twice through L1: 228 against 185 us on 33 000 samples.)
+// dbasis is written, not accumulated (every pair belongs to exactly one sample; layers
+// wider than a pass add to it pass by pass); dfeat must be zero on entry.
 template <int K, int CC>
-__global__ void __launch_bounds__(Cfg<K, CC>::kGradWarps * 32, 1)
-basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int64_t M, const float* __restrict__ basis,
+struct GradCfg {
+  static_assert(K * CC <= 2048 && CC % 32 == 0 && (K * CC <= 1024 || K >= 32), "fragments");
+  static constexpr int kTeam = K * CC > 1024 ? 2 : 1;       // warps per sample
+  static constexpr int kMt1 = K / 16 / kTeam;               // 16-row tiles of (1) per warp
+  static constexpr int kKs1 = CC / 16;                      // its reduction steps
+  static constexpr int kMt2 = CC / 16 / kTeam;              // tiles of (2)
+  static constexpr int kKs2 = K / 16;
+  static constexpr int kFeatStride = CC * 4 + 16;           // bytes: hi[CC] | mid[CC] | pad
+  static constexpr int kKStride = K * 2 + 16;               // a bf16 row over k
+  static constexpr int kRawStride = K + 4;                  // floats, a row of dX over k
+  static constexpr int kFeatBytes = kChunk * kFeatStride;
+  static constexpr int kStageBytes = kFeatBytes + 2 * kChunk * kKStride;
+  static constexpr int kRawBytes = CC * kRawStride * 4;
+  static constexpr int kTeamBytes = kRawBytes + 2 * kStageBytes;
+  static constexpr int kFit = 227 * 1024 / kTeamBytes * kTeam;      // warps: 16 of 128 registers
+  static constexpr int kTeams = (kFit >= 16 && kMt1 == 1 ? 16 : 12) / kTeam;     // or 12 of 168
+  static constexpr int kThreads = kTeams * kTeam * 32;
+  static constexpr int kBasisVecs = kChunk * K / 4 / (32 * kTeam);   // float4 per lane and chunk
+  static_assert(kTeams * kTeamBytes <= 227 * 1024 && (kTeam == 1 || kTeams <= 15),
+                "shared memory, and a named barrier per team");
+};
+
+// d = a * b
+__device__ __forceinline__ void mma16816_first(float* d, const uint32_t* a, uint32_t b0,
+                                               uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+}
+
+template <int N>
+__device__ __forceinline__ void red_add(float* dst, const float* v) {
+  if (N == 4)
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]),
+                 "f"(v[2]), "f"(v[N - 1]) : "memory");
+  else
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(v[0]), "f"(v[1])
+                 : "memory");
+}
+
+// The chunks of a team, one after the other (see Walker; an item without pairs is left out).
+struct Chunk {
+  int item, base, end;     // item -1: no more
+  bool first;
+  __device__ __forceinline__ bool valid() const { return item >= 0; }
+  __device__ __forceinline__ int cnt() const { return min(end - base, kChunk); }
+};
+
+struct ChunkWalk {
+  const int32_t* ranges;
+  int items, parts, bs, stride, lane;
+  int blk, li, upto, begin, upto_next, begin_next;   // upto: end of the lane's item of the block
+
+  __device__ __forceinline__ int item_end(int i) const {
+    if (parts == 1) return __ldg(ranges + i);
+    const int s = i / parts;
+    return part_end(s > 0 ? __ldg(ranges + s - 1) : 0, __ldg(ranges + s), i - s * parts + 1, parts,
+                    kChunk);
+  }
+  __device__ __forceinline__ void load(int64_t b, int* upto_b, int* begin_b) const {
+    const int64_t s0 = b * bs;
+    *upto_b = lane < bs && s0 + lane < items ? item_end((int)s0 + lane) : 0;
+    *begin_b = s0 > 0 && s0 < items ? item_end((int)s0 - 1) : 0;
+  }
+  __device__ __forceinline__ Chunk start(const int32_t* r, int item_count, int team, int teams,
+                                         int ln, int block, int part_count) {
+    ranges = r; items = item_count; blk = team; stride = teams; lane = ln; bs = block;
+    parts = part_count; li = -1;
+    load(blk, &upto, &begin);
+    load((int64_t)blk + stride, &upto_next, &begin_next);
+    Chunk c;
+    c.item = 0; c.base = c.end = 0; c.first = false;
+    return next(c);
+  }
+  __device__ __forceinline__ Chunk next(Chunk c) {
+    c.first = false;
+    if (c.end - c.base > kChunk) {
+      c.base += kChunk;
+      return c;
+    }
+    do {
+      ++li;
+      if (li == bs || (int64_t)blk * bs + li >= items) {
+        if ((int64_t)blk * bs >= items || ((int64_t)blk + stride) * bs >= items) {
+          c.item = -1;
+          c.base = c.end = 0;
+          c.first = false;
+          blk = items;        // (stays at the end)
+          bs = 1;
+          return c;
+        }
+        blk += stride;
+        li = 0;
+        upto = upto_next; begin = begin_next;
+        load((int64_t)blk + stride, &upto_next, &begin_next);
+      }
+      c.end = __shfl_sync(0xffffffffu, upto, li);
+      const int before = __shfl_sync(0xffffffffu, upto, (li + 31) & 31);
+      c.base = li ? before : begin;
+      c.item = blk * bs + li;
+      c.first = true;
+    } while (c.base >= c.end);
+    return c;
+  }
+};
+
+template <int K, int CC>
+__global__ void __launch_bounds__(GradCfg<K, CC>::kThreads, 1)
+basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int64_t M,
+                            const float* __restrict__ basis,
                             const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
                             const int32_t* __restrict__ ranges,
                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
                             float* __restrict__ dfeat) {
-  chain_enter(ns * parts * 32, (int64_t)gridDim.x * blockDim.x);
-  typedef Cfg<K, CC> cfg;
+  typedef GradCfg<K, CC> cfg;
+  constexpr int W = cfg::kTeam;
+  chain_enter(ns * parts * 32 * W, (int64_t)gridDim.x * blockDim.x);
   extern __shared__ __align__(128) uint8_t bpm_smem[];
   const int lane = threadIdx.x & 31;
-  const int warp_in_block = threadIdx.x >> 5;
-  const int warps_per_block = blockDim.x >> 5;
-  uint8_t* wsm = bpm_smem + (size_t)warp_in_block * cfg::kGradWarpBytes;
-  uint8_t* feat_tile = wsm;
-  uint8_t* basis_tile = feat_tile + cfg::kFeatBytes;
-  uint8_t* dx_raw = basis_tile + cfg::kBasisBytes;
-  uint8_t* dx_tile = dx_raw + cfg::kDxRawBytes;   // hi rows [c], then mid rows [c]
-  const int64_t warp = (int64_t)blockIdx.x * warps_per_block + warp_in_block;
-  const int64_t warps = (int64_t)gridDim.x * warps_per_block;
+  const int team = (threadIdx.x >> 5) / W, sub = (threadIdx.x >> 5) % W;
+  const int tid = threadIdx.x % (32 * W);
+  uint8_t* const mem = bpm_smem + (size_t)team * cfg::kTeamBytes;
+  float* const raw = reinterpret_cast<float*>(mem);
+  auto team_sync = [&]() {
+    if (W == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(32 * W) : "memory");
+  };
   const int g = lane >> 2, q = lane & 3;
-  const int mi = lane >> 3, r = lane & 7;
-  // (1) A: matrices (pairs 0-7 | 8-15) x (c 0-7 | 8-15) of a 16-channel step
-  const uint32_t a1_off = (r + 8 * (mi & 1)) * cfg::kFeatStride + 8 * (mi >> 1) * 2;
-  // (1) B, transposed: matrices (c 0-7 | 8-15) x (positions 0-7 | 8-15)
-  const uint32_t b1_off = (r + 8 * (mi & 1)) * cfg::kKStride + 8 * (mi >> 1) * 2;
-  // (2) A: matrices (pairs 0-7 | 8-15) x (positions 0-7 | 8-15) of a 16-k step
-  const uint32_t a2_off = (r + 8 * (mi & 1)) * cfg::kKStride + 8 * (mi >> 1) * 2;
-  // (2) B: matrices (tile 2j | 2j+1) x (positions 0-7 | 8-15); row n of tile 2j+t
-  // is channel 4*(n/2) + 2*t + (n%2) of the 16-channel group
-  const uint32_t b2_off = (4 * (r >> 1) + 2 * (mi >> 1) + (r & 1)) * cfg::kKStride + 8 * (mi & 1) * 2;
-  constexpr int kDxMid = cfg::kCC * cfg::kKStride;
-  constexpr int kBasisMid = kChunk * cfg::kKStride;
+  // ldmatrix rows of this lane: pair lane % 8 of a group; matrices 0 and 1 are the hi terms of
+  // columns 0-7 and 8-15 of a 16-column step, 2 and 3 the mid terms
+  const uint32_t f_off = (lane & 7) * cfg::kFeatStride + ((lane >> 3) & 1) * 16 + (lane >> 4) * (CC * 2);
+  const uint32_t b_off = cfg::kFeatBytes + ((lane & 7) + (lane >> 4) * kChunk) * cfg::kKStride +
+                         ((lane >> 3) & 1) * 16;
+  // The row order inside a tile gives a lane consecutive outputs: row g + 8h of a lone tile
+  // is output 2g + h, of tile t of a pair output 4g + 2t + h of the pair's 32.
+  constexpr int kVec1 = cfg::kMt1 % 2 == 0 ? 4 : 2, kVec2 = cfg::kMt2 % 2 == 0 ? 4 : 2;
+  auto out_row = [&](int mt, int vec) {
+    return vec == 4 ? 32 * (mt >> 1) + 4 * g + 2 * (mt & 1) : 16 * mt + 2 * g;
+  };
+  const int row1 = 16 * cfg::kMt1 * sub, row2 = 16 * cfg::kMt2 * sub;   // this warp's rows
 
   // pairs beyond the last range belong to no sample: their gradient is zero
-  if (blockIdx.x == 0 && warp_in_block == 0) {
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
     const int64_t covered = ns > 0 ? __ldg(ranges + ns - 1) : 0;
     for (int64_t i = covered * K + lane; i < M * K; i += 32) dbasis[i] = 0.0f;
   }
 
-  auto issue_dx = [&](int64_t s, int c0, int w) {
-    // w*K floats, one contiguous piece per block, to rows of K per channel
-    const float* src = in_grads + s * C * K + ((int64_t)c0 << shift);
-    const uint32_t dst = smem_addr(dx_raw);
-    if ((1 << shift) == K) {
-      for (int i = lane; i < w * (K / 4); i += 32) cp_async16_zfill(dst + i * 16, src + i * 4, true);
-    } else {
-      for (int i = lane; i < w * (K / 4); i += 32) {
-        const int c = i / (K / 4), k = (i % (K / 4)) * 4;
-        cp_async16_zfill(dst + i * 16, src + (((k >> shift) * C + c) << shift) + (k & ((1 << shift) - 1)),
-                         true);
+  for (int c0 = 0; c0 < C; c0 += CC) {
+    const int w = min(CC, C - c0);
+    // ---- copies
+    // dX: rows of K floats per channel, out of one piece of w * K floats per block of columns
+    // 16-byte pieces of rows 8-15 of every 16 change places with those two further on: the
+    // rows 4g that (2) reads then lie in different banks
+    constexpr int kRowStep = 32 * W / (K / 4);      // rows of dX that a copy per lane covers
+    static_assert(kRowStep == 8 || kRowStep == 4, "rows of one copy lie in half of 16");
+    const uint32_t dx_row = smem_addr(raw) + tid / (K / 4) * cfg::kRawStride * 4;
+    const uint32_t dx_dst[2] = {dx_row + tid % (K / 4) * 16, dx_row + (tid % (K / 4) ^ 2) * 16};
+    auto issue_dx = [&](int item) {
+      const float* src = in_grads + (int64_t)(parts == 1 ? item : item / parts) * C * K +
+                         ((int64_t)c0 << shift);
+      if ((1 << shift) == K && w == CC) {
+        src += tid * 4;
+#pragma unroll
+        for (int i = 0; i < CC * K / 4 / (32 * W); ++i)
+          cp_async16(dx_dst[i * kRowStep / 8 & 1] + i * kRowStep * cfg::kRawStride * 4,
+                     src + i * 32 * W * 4);
+      } else {
+#pragma unroll 1
+        for (int i = tid; i < w * (K / 4); i += 32 * W) {
+          const int c = i / (K / 4), k = (i % (K / 4)) * 4;
+          cp_async16(smem_addr(raw) + (c * cfg::kRawStride + (k ^ (c & 8))) * 4,
+                     src + (((k >> shift) * C + c) << shift) + (k & ((1 << shift) - 1)));
+        }
+      }
+    };
+    // feature rows: hi[c0 .. c0 + w) and mid[c0 .. c0 + w) of the chunk's neighbors (a row
+    // beyond them keeps what it held: it is a column of the products, and nobody takes it)
+    constexpr int kSeg = CC / 8;             // 16-byte segments per half row
+    constexpr int kRpi = 32 / (2 * kSeg);    // rows per warp instruction
+    const int seg = lane % kSeg, half_row = lane / kSeg % 2, row0 = sub * kRpi + lane / (2 * kSeg);
+    const uint32_t f_dst = smem_addr(mem) + cfg::kRawBytes + row0 * cfg::kFeatStride +
+                           half_row * (CC * 2) + seg * 16;
+    const __nv_bfloat16* const f_src = fs + (int64_t)half_row * C + c0 + seg * 8;
+    const int row_limit = seg * 8 < w ? row0 : kChunk;      // a lane without channels: no row
+    auto issue_rows = [&](int st, const Chunk& j, int idx) {
+      const uint32_t dst = f_dst + st * cfg::kStageBytes;
+      const int cnt = j.cnt();
+#pragma unroll
+      for (int it = 0; it < kChunk / kRpi / W; ++it) {
+        const int p = __shfl_sync(0xffffffffu, idx, it * W * kRpi + row0);
+        if (row_limit + it * W * kRpi < cnt)
+          cp_async16(dst + it * W * kRpi * cfg::kFeatStride, f_src + (int64_t)p * (2 * C));
+      }
+    };
+    // basis rows: float4 number tid + 32 W t of the chunk
+    auto load_rows = [&](const Chunk& j, float4* v) {
+      const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)j.base * K) + tid;
+      const int have = j.cnt() * (K / 4) - tid;
+#pragma unroll
+      for (int t = 0; t < cfg::kBasisVecs; ++t)
+        if (32 * W * t < have) v[t] = __ldg(src + 32 * W * t);
+    };
+    uint8_t* const b_dst = mem + cfg::kRawBytes + cfg::kFeatBytes + tid / (K / 4) * cfg::kKStride +
+                           tid % (K / 4) * 8;
+    auto store_rows = [&](int st, const float4* v) {
+#pragma unroll
+      for (int t = 0; t < cfg::kBasisVecs; ++t) {
+        uint2 h, m;
+        split2(v[t].x, v[t].y, h.x, m.x);
+        split2(v[t].z, v[t].w, h.y, m.y);
+        uint8_t* dst = b_dst + st * cfg::kStageBytes + t * (32 * W / (K / 4)) * cfg::kKStride;
+        *reinterpret_cast<uint2*>(dst) = h;
+        *reinterpret_cast<uint2*>(dst + kChunk * cfg::kKStride) = m;
+      }
+    };
+
+    if (c0 > 0) team_sync();       // (the pass before has read its stages and dX)
+    if (w < CC) {
+      // channels that do not exist, on either side of (1)
+      for (int i = tid; i < (CC - w) * cfg::kRawStride; i += 32 * W) raw[w * cfg::kRawStride + i] = 0.0f;
+      for (int i = tid; i < 2 * kChunk * 2 * (CC - w) / 8; i += 32 * W) {
+        const int r = i / (2 * (CC - w) / 8), e = i % (2 * (CC - w) / 8), h = e / ((CC - w) / 8);
+        uint8_t* row = mem + cfg::kRawBytes + (r / kChunk) * cfg::kStageBytes + (r % kChunk) * cfg::kFeatStride;
+        *reinterpret_cast<uint4*>(row + h * (CC * 2) + (w + e % ((CC - w) / 8) * 8) * 2) =
+            make_uint4(0, 0, 0, 0);
       }
     }
-  };
-
-  for (int c0 = 0; c0 < C; c0 += cfg::kCC) {
-    const int w = min(cfg::kCC, C - c0);
-    const int ks_cnt = w >> 4;     // 16-channel steps of (1) = tile pairs of (2)
-    Walker walk;
-    walk.init(ranges, ns * parts, warp, warps, lane, bs, parts);
-    Job cur = walk.next(), n1 = walk.next(), n2 = walk.next();
-    int idx0 = load_idx(cur, neigh, lane);
-    int idx1 = load_idx(n1, neigh, lane);
-    float4 bv[cfg::kBasisVecs];
-    __syncwarp();
+    ChunkWalk walk;
+    Chunk cur = walk.start(ranges, (int)(ns * parts), (int)blockIdx.x * cfg::kTeams + team,
+                           (int)gridDim.x * cfg::kTeams, lane, bs, parts);
+    Chunk n1 = walk.next(cur), n2 = walk.next(n1);
+    auto load_idx = [&](const Chunk& j) {
+      return j.valid() && lane < j.cnt() ? __ldg(&neigh[j.base + lane].x) : 0;
+    };
+    int idx0 = load_idx(cur), idx1 = load_idx(n1);
+    float4 rows[cfg::kBasisVecs];
+#pragma unroll
+    for (int t = 0; t < cfg::kBasisVecs; ++t) rows[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (cur.valid()) {
-      issue_dx(cur.s / parts, c0, w);
-      issue_features<K, CC>(smem_addr(feat_tile), fs, C, c0, w, idx0, cur.cnt, lane);
-      load_basis<K>(basis, cur.base, cur.cnt, lane, bv);
+      issue_dx(cur.item);
+      issue_rows(0, cur, idx0);
+      load_rows(cur, rows);
+      store_rows(0, rows);
     }
     cp_commit();
+    uint32_t a1h[cfg::kMt1][cfg::kKs1][4], a1m[cfg::kMt1][cfg::kKs1][4];
+    uint32_t a2h[cfg::kMt2][cfg::kKs2][4], a2m[cfg::kMt2][cfg::kKs2][4];
+    float* const db_lane = dbasis + row1 + out_row(0, kVec1) + 2 * q * K;
+    float* const df_lane = dfeat + c0 + row2 + out_row(0, kVec2);
+    int st = 0;
     while (cur.valid()) {
-      cp_wait<0>();   // features of `cur`, and dX of its sample if this is its first chunk
-      __syncwarp();
+      // the rows of this chunk have landed, and dX if it is the item's first; the other
+      // stage has been read
+      cp_wait<0>();
+      team_sync();
       if (cur.first) {
-        const float4* raw = reinterpret_cast<const float4*>(dx_raw);
-        for (int i = lane; i < w * (K / 4); i += 32) {
-          const int row = i / (K / 4), a4 = i % (K / 4);
-          store_split4<K>(dx_tile + row * cfg::kKStride, dx_tile + kDxMid + row * cfg::kKStride, a4,
-                          raw[i]);
-        }
-        __syncwarp();
-        const int64_t sn = walk.after(cur.s);
-        if (sn < walk.ns) issue_dx(sn / parts, c0, w);
-        cp_commit();
-      }
-      store_basis<K>(basis_tile, lane, bv);
-      __syncwarp();
-      const uint32_t ft = smem_addr(feat_tile), bt = smem_addr(basis_tile), dt = smem_addr(dx_tile);
-      // ---- (1) dbasis
-      if (cur.cnt > 0) {
-        // one accumulator set per pass and per parity of the channel step: the
-        // MMAs of a step are independent of each other and of the previous step
-        constexpr int kPar = K == 64 ? 1 : 2;   // register budget
-        float dbp[kPar][3][cfg::kNT][4];
 #pragma unroll
-        for (int e = 0; e < kPar; ++e)
+        for (int mt = 0; mt < cfg::kMt1; ++mt) {
+          const int k = row1 + out_row(mt, kVec1);
 #pragma unroll
-          for (int p = 0; p < 3; ++p)
+          for (int ks = 0; ks < cfg::kKs1; ++ks) {
 #pragma unroll
-            for (int nt = 0; nt < cfg::kNT; ++nt)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) dbp[e][p][nt][i] = 0.0f;
-#pragma unroll
-        for (int ks = 0; ks < cfg::kMT; ++ks) {
-          if (ks < ks_cnt) {
-            uint32_t ah[4], am[4];
-            ldsm_x4(ft + a1_off + ks * 32, ah);
-            ldsm_x4(ft + a1_off + cfg::kCC * 2 + ks * 32, am);
-#pragma unroll
-            for (int j = 0; j < cfg::kNTP; ++j) {
-              uint32_t bh[4], bm[4];
-              ldsm_x4_t(dt + b1_off + ks * 16 * cfg::kKStride + j * 32, bh);
-              ldsm_x4_t(dt + kDxMid + b1_off + ks * 16 * cfg::kKStride + j * 32, bm);
-              mma16816(dbp[ks & (kPar - 1)][0][2 * j], ah, bm[0], bm[1]);
-              mma16816(dbp[ks & (kPar - 1)][0][2 * j + 1], ah, bm[2], bm[3]);
-              mma16816(dbp[ks & (kPar - 1)][1][2 * j], am, bh[0], bh[1]);
-              mma16816(dbp[ks & (kPar - 1)][1][2 * j + 1], am, bh[2], bh[3]);
-              mma16816(dbp[ks & (kPar - 1)][2][2 * j], ah, bh[0], bh[1]);
-              mma16816(dbp[ks & (kPar - 1)][2][2 * j + 1], ah, bh[2], bh[3]);
+            for (int half = 0; half < 2; ++half) {
+              const float* r = raw + (16 * ks + 8 * half + 2 * q) * cfg::kRawStride + (k ^ (8 * half));
+              const float2 x = *reinterpret_cast<const float2*>(r);
+              const float2 y = *reinterpret_cast<const float2*>(r + cfg::kRawStride);
+              split2(x.x, y.x, a1h[mt][ks][2 * half], a1m[mt][ks][2 * half]);
+              split2(x.y, y.y, a1h[mt][ks][2 * half + 1], a1m[mt][ks][2 * half + 1]);
             }
           }
         }
-        float db[cfg::kNT][4];
 #pragma unroll
-        for (int nt = 0; nt < cfg::kNT; ++nt)
+        for (int mt = 0; mt < cfg::kMt2; ++mt) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            db[nt][i] = ((dbp[0][0][nt][i] + dbp[kPar - 1][0][nt][i] * (kPar - 1)) +
-                         (dbp[0][1][nt][i] + dbp[kPar - 1][1][nt][i] * (kPar - 1))) +
-                        (dbp[0][2][nt][i] + dbp[kPar - 1][2][nt][i] * (kPar - 1));
-        // lane (g, q): pairs g and g + 8, basis functions 16*j + 4*q .. +3
+          for (int h = 0; h < 2; ++h) {
+            const int c = row2 + out_row(mt, kVec2) + h;
+            const float* r = raw + c * cfg::kRawStride + 2 * q;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = g + 8 * h;
-          if (row < cur.cnt) {
-            float4* dst = reinterpret_cast<float4*>(dbasis + (int64_t)(cur.base + row) * K + 4 * q);
+            for (int ks = 0; ks < cfg::kKs2; ++ks) {
 #pragma unroll
-            for (int j = 0; j < cfg::kNTP; ++j) {
-              float4 v = make_float4(db[2 * j][2 * h], db[2 * j][2 * h + 1], db[2 * j + 1][2 * h],
-                                     db[2 * j + 1][2 * h + 1]);
-              if (c0 > 0) {
-                const float4 o = dst[4 * j];
-                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+              for (int half = 0; half < 2; ++half) {
+                const float2 x = *reinterpret_cast<const float2*>(r + 16 * ks + ((8 * half) ^ (c & 8)));
+                split2(x.x, x.y, a2h[mt][ks][2 * half + h], a2m[mt][ks][2 * half + h]);
               }
-              dst[4 * j] = v;
             }
           }
         }
+        team_sync();     // dX has been read: the next item's may come
+        const Chunk& following = n1.first ? n1 : n2;      // (further ahead: at the next chunk)
+        if (following.valid() && following.first) issue_dx(following.item);
+      } else if (!n1.first && n2.valid() && n2.first) {
+        issue_dx(n2.item);
       }
-      __syncwarp();   // every lane is done with the feature tile
-      // ---- prefetch for the next chunks
-      const int idx2 = load_idx(n2, neigh, lane);
       if (n1.valid()) {
-        issue_features<K, CC>(smem_addr(feat_tile), fs, C, c0, w, idx1, n1.cnt, lane);
-        load_basis<K>(basis, n1.base, n1.cnt, lane, bv);
+        issue_rows(st ^ 1, n1, idx1);
+        load_rows(n1, rows);
       }
       cp_commit();
-      // ---- (2) dfeat
-      if (cur.cnt > 0) {
-        float df[cfg::kMT * 2][4];
+      const int idx2 = load_idx(n2);
+      // ---- the products, eight pairs at a time
+      const uint32_t tile = smem_addr(mem) + cfg::kRawBytes + st * cfg::kStageBytes;
+      const int cnt = cur.cnt();
+      float* const db = db_lane + (int64_t)cur.base * K;
 #pragma unroll
-        for (int nt = 0; nt < cfg::kMT * 2; ++nt)
+      for (int p = 0; p < kChunk; p += 8) {
+        if (p >= cnt) break;
+        float d1[cfg::kMt1][4], d2[cfg::kMt2][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) df[nt][i] = 0.0f;
+        for (int ks = 0; ks < cfg::kKs1; ++ks) {
+          uint32_t b[4];
+          ldsm_x4(tile + f_off + p * cfg::kFeatStride + ks * 32, b);
 #pragma unroll
-        for (int kk = 0; kk < cfg::kNTP; ++kk) {
-          uint32_t ah[4], am[4];
-          ldsm_x4(bt + a2_off + kk * 32, ah);
-          ldsm_x4(bt + kBasisMid + a2_off + kk * 32, am);
-#pragma unroll
-          for (int j = 0; j < cfg::kMT; j += 2) {
-            if (j < ks_cnt) {
-              const bool two = j + 1 < ks_cnt;
-              uint32_t bh[2][4], bm[2][4];
-              ldsm_x4(dt + b2_off + j * 16 * cfg::kKStride + kk * 32, bh[0]);
-              ldsm_x4(dt + kDxMid + b2_off + j * 16 * cfg::kKStride + kk * 32, bm[0]);
-              if (two) {
-                ldsm_x4(dt + b2_off + (j + 1) * 16 * cfg::kKStride + kk * 32, bh[1]);
-                ldsm_x4(dt + kDxMid + b2_off + (j + 1) * 16 * cfg::kKStride + kk * 32, bm[1]);
-              }
-#pragma unroll
-              for (int pass = 0; pass < 3; ++pass) {
-                const uint32_t* a = pass == 1 ? am : ah;
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                  if (u == 0 || two) {
-                    const uint32_t* b = pass == 0 ? bm[u] : bh[u];
-                    mma16816(df[2 * (j + u)], a, b[0], b[1]);
-                    mma16816(df[2 * (j + u) + 1], a, b[2], b[3]);
-                  }
-                }
-              }
-            }
+          for (int mt = 0; mt < cfg::kMt1; ++mt) {
+            if (ks == 0) mma16816_first(d1[mt], a1h[mt][ks], b[2], b[3]);
+            else mma16816(d1[mt], a1h[mt][ks], b[2], b[3]);
+            mma16816(d1[mt], a1m[mt][ks], b[0], b[1]);
+            mma16816(d1[mt], a1h[mt][ks], b[0], b[1]);
           }
         }
-        // lane (g, q): pairs g and g + 8, channels c0 + 16*j + 4*q .. +3
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int row = g + 8 * h;
-          const int pt = __shfl_sync(0xffffffffu, idx0, row);
-          if (row < cur.cnt) {
-            float* dst = dfeat + (int64_t)pt * C + c0 + 4 * q;
+        for (int ks = 0; ks < cfg::kKs2; ++ks) {
+          uint32_t b[4];
+          ldsm_x4(tile + b_off + p * cfg::kKStride + ks * 32, b);
 #pragma unroll
-            for (int j = 0; j < cfg::kMT; ++j) {
-              if (j < ks_cnt)
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 16 * j),
-                             "f"(df[2 * j][2 * h]), "f"(df[2 * j][2 * h + 1]),
-                             "f"(df[2 * j + 1][2 * h]), "f"(df[2 * j + 1][2 * h + 1])
-                             : "memory");
+          for (int pass = 0; pass < 3; ++pass)
+#pragma unroll
+            for (int mt = 0; mt < cfg::kMt2; ++mt) {
+              const uint32_t* a = pass == 1 ? a2m[mt][ks] : a2h[mt][ks];
+              const uint32_t b0 = pass == 0 ? b[2] : b[0], b1 = pass == 0 ? b[3] : b[1];
+              if (ks == 0 && pass == 0) mma16816_first(d2[mt], a, b0, b1);
+              else mma16816(d2[mt], a, b0, b1);
+            }
+        }
+        // lane (g, q): pairs 2q and 2q + 1 of the eight
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int pt = __shfl_sync(0xffffffffu, idx0, p + 2 * q + e);
+          if (p + 2 * q + e < cnt) {
+            float* const df = df_lane + (int64_t)pt * C;
+#pragma unroll
+            for (int mt = 0; mt < cfg::kMt2; mt += kVec2 / 2) {
+              float v[kVec2];
+#pragma unroll
+              for (int i = 0; i < kVec2; ++i) v[i] = d2[mt + i / 2][2 * (i % 2) + e];
+              const int c = out_row(mt, kVec2) - out_row(0, kVec2);
+              if (w == CC || row2 + out_row(mt, kVec2) < w) red_add<kVec2>(df + c, v);
+            }
+#pragma unroll
+            for (int mt = 0; mt < cfg::kMt1; mt += kVec1 / 2) {
+              float v[kVec1];
+#pragma unroll
+              for (int i = 0; i < kVec1; ++i) v[i] = d1[mt + i / 2][2 * (i % 2) + e];
+              float* dst = db + (p + e) * K + (out_row(mt, kVec1) - out_row(0, kVec1));
+              if (c0 > 0)      // (a load of the pass before's sum would stall the warp)
+                red_add<kVec1>(dst, v);
+              else if (kVec1 == 4)
+                *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[kVec1 - 1]);
+              else
+                *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
             }
           }
         }
       }
-      cur = n1; n1 = n2; n2 = walk.next();
+      st ^= 1;
+      if (n1.valid()) store_rows(st, rows);
+      cur = n1; n1 = n2; n2 = walk.next(n1);
       idx0 = idx1; idx1 = idx2;
     }
     cp_wait<0>();
-    __syncwarp();
   }
 }
 
