@@ -335,6 +335,263 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   }
 }
 
+// ---- two hidden layers of at most 8 and 16 units, three dimensions --------------------------
+//
+// The layers' usual sizes fit registers: no activation passes through shared memory, which
+// bounded the general kernels (355 000 pairs, ELU, 8-16: forward 34 us and 78 warp
+// instructions per pair, gradients 131 and 224; now 25 and 95 us).  Units are padded to H1 = 8 and H2 = 8 or
+// 16 with zero weights: a padded unit is zero, and nothing comes back through it.
+constexpr int kH1 = 8;
+
+bool small_mlp(const MlpShape& s) {
+  return s.D == 3 && s.L == 2 && s.h[1] <= kH1 && s.h[2] <= 16;
+}
+
+// Parameters of MLP g in shared memory: [3][8] and [8], then [8][H2] and [H2].
+template <int H2>
+struct SmallParams {
+  float4 w1[3][kH1 / 4], b1[kH1 / 4], w2[kH1][H2 / 4], b2[H2 / 4];
+  __device__ __forceinline__ void load(const MlpShape& s, int g, int threads) {
+    float* p = reinterpret_cast<float*>(this);
+    constexpr int kFirst = 4 * kH1, kAll = kFirst + (kH1 + 1) * H2;
+    for (int i = threadIdx.x; i < kAll; i += threads) {
+      const bool second = i >= kFirst;
+      const int h = second ? H2 : kH1, l = second;
+      const int r = (second ? i - kFirst : i) / h, c = (second ? i - kFirst : i) % h;
+      const int rows = second ? kH1 : 3, in = s.h[l], out = s.h[l + 1];
+      float v = 0.0f;
+      if (c < out) {
+        if (r == rows) v = __ldg(s.b[l] + g * out + c);
+        else if (r < in) v = __ldg(s.w[l] + (g * in + r) * out + c);
+      }
+      p[i] = v;
+    }
+  }
+};
+
+__device__ __forceinline__ void fma4(float* acc, float a, float4 w) {
+  acc[0] = fmaf(a, w.x, acc[0]); acc[1] = fmaf(a, w.y, acc[1]);
+  acc[2] = fmaf(a, w.z, acc[2]); acc[3] = fmaf(a, w.w, acc[3]);
+}
+__device__ __forceinline__ void set4(float* acc, float4 b) {
+  acc[0] = b.x; acc[1] = b.y; acc[2] = b.z; acc[3] = b.w;
+}
+
+// One pair per thread.
+template <int H2>
+__global__ void __launch_bounds__(256)
+small_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
+                       const float* __restrict__ p_out, const int2* __restrict__ neigh,
+                       const float* __restrict__ pdf, float inv_radius, int act, float alpha,
+                       int pdf_by_nbr, float* __restrict__ basis) {
+  chain_enter(M, (int64_t)gridDim.x * 256);
+  __shared__ SmallParams<H2> par;
+  const int hl = s.h[2], k_total = s.G * hl;
+  const bool quads = hl % 4 == 0 && (uintptr_t)basis % 16 == 0;
+  for (int g = 0; g < s.G; ++g) {
+    if (g > 0) __syncthreads();
+    par.load(s, g, 256);
+    __syncthreads();
+    for (int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x; m < M; m += (int64_t)gridDim.x * 256) {
+      const int2 nb = __ldg(neigh + m);
+      const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+      float h[kH1];
+#pragma unroll
+      for (int q = 0; q < kH1 / 4; ++q) set4(h + 4 * q, par.b1[q]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float x = (__ldg(p_in + (int64_t)nb.x * 3 + d) - __ldg(p_out + (int64_t)nb.y * 3 + d)) *
+                        inv_radius;
+#pragma unroll
+        for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, x, par.w1[d][q]);
+      }
+#pragma unroll
+      for (int i = 0; i < kH1; ++i) h[i] = act_fwd(h[i], act, alpha);
+      float* dst = basis + m * k_total + g * hl;
+#pragma unroll
+      for (int q = 0; q < H2 / 4; ++q) {
+        float v[4];
+        set4(v, par.b2[q]);
+#pragma unroll
+        for (int i = 0; i < kH1; ++i) fma4(v, h[i], par.w2[i][q]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = act_fwd(v[e], act, alpha) * inv_pdf;
+        if (quads) {
+          if (4 * q < hl) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (4 * q + e < hl) dst[4 * q + e] = v[e];
+        }
+      }
+    }
+  }
+}
+
+// Two lanes per pair, each with half of the last layer's units and, of what comes before
+// them, half of the hidden ones: the gradients of all parameters are sums over pairs in
+// (9 H2 + 32) / 2 registers per lane, 88 at H2 = 16, folded over the warp once at the end.
+// blockIdx.y: the MLP.
+template <int H2>
+__global__ void __launch_bounds__(128, 3)
+small_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
+                       const float* __restrict__ p_out, const int2* __restrict__ neigh,
+                       const float* __restrict__ pdf, float inv_radius, int act, float alpha,
+                       int pdf_by_nbr, const float* __restrict__ dbasis,
+                       float* __restrict__ dweights, float* __restrict__ dbiases,
+                       float* __restrict__ dp_in, float* __restrict__ dp_out,
+                       float* __restrict__ dpdf) {
+  constexpr int HJ = H2 / 2, HI = kH1 / 2;             // units of a lane
+  constexpr int kB2 = kH1 * HJ, kW1 = kB2 + HJ, kB1 = kW1 + 3 * HI;
+  constexpr int kValues = kB1 + HI, kPadded = (kValues + 15) / 16 * 16;
+  chain_enter(M * 2, (int64_t)gridDim.x * 128);
+  __shared__ SmallParams<H2> par;
+  __shared__ float red[2][kPadded];
+  const int g = blockIdx.y;
+  par.load(s, g, 128);
+  for (int i = threadIdx.x; i < 2 * kPadded; i += 128) red[0][i] = 0.0f;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, half = lane & 1;
+  const int h1 = s.h[1], hl = s.h[2], k_total = s.G * hl;
+  const bool quads = hl == H2 && k_total % 4 == 0 && (uintptr_t)dbasis % 16 == 0;
+  // acc: [8][HJ] and [HJ] of the second layer, [3][HI] and [HI] of the first
+  float acc[kPadded];
+#pragma unroll
+  for (int i = 0; i < kPadded; ++i) acc[i] = 0.0f;
+  const int64_t stride = (int64_t)gridDim.x * 64;
+  // (the whole warp goes on until its first pair is beyond the end)
+  for (int64_t m0 = (int64_t)blockIdx.x * 64 + (threadIdx.x >> 5) * 16; m0 < M; m0 += stride) {
+    const int64_t m = m0 + (lane >> 1);
+    const bool live = m < M;
+    const int2 nb = __ldg(neigh + (live ? m : M - 1));
+    float diff[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      diff[d] = (__ldg(p_in + (int64_t)nb.x * 3 + d) - __ldg(p_out + (int64_t)nb.y * 3 + d)) * inv_radius;
+    const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : live ? m : M - 1));
+    float up[HJ];
+    const float* gb = dbasis + m * k_total + g * hl + half * HJ;
+#pragma unroll
+    for (int j = 0; j < HJ; j += 4) {
+      if (quads) {
+        const float4 q = live ? __ldg(reinterpret_cast<const float4*>(gb + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        set4(up + j, q);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) up[j + e] = live && half * HJ + j + e < hl ? __ldg(gb + j + e) : 0.0f;
+      }
+    }
+    // own hidden units, the partner's by a shuffle
+    float own[HI], slope1[HI], a1[kH1];
+    set4(own, par.b1[half]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) fma4(own, diff[d], par.w1[d][half]);
+#pragma unroll
+    for (int i = 0; i < HI; ++i) {
+      slope1[i] = act_slope(own[i], act, alpha);
+      own[i] = act_fwd(own[i], act, alpha);
+      const float other = __shfl_xor_sync(0xffffffffu, own[i], 1);
+      a1[i] = half ? other : own[i];
+      a1[HI + i] = half ? own[i] : other;
+    }
+    float back[kH1], dpdf_m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kH1; ++i) back[i] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < HJ / 4; ++q) {
+      float v[4];
+      set4(v, par.b2[half * (HJ / 4) + q]);
+#pragma unroll
+      for (int i = 0; i < kH1; ++i) fma4(v, a1[i], par.w2[i][half * (HJ / 4) + q]);
+      // d/dpre of the last layer; the density's own gradient: basis = a / pdf -> -a / pdf^2
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float b = up[4 * q + e];
+        if (dpdf) dpdf_m -= b * act_fwd(v[e], act, alpha) * inv_pdf * inv_pdf;
+        v[e] = b * inv_pdf * act_slope(v[e], act, alpha);
+        acc[kB2 + 4 * q + e] += v[e];
+      }
+#pragma unroll
+      for (int i = 0; i < kH1; ++i) {
+        const float4 w = par.w2[i][half * (HJ / 4) + q];
+        back[i] = fmaf(v[3], w.w, fmaf(v[2], w.z, fmaf(v[1], w.y, fmaf(v[0], w.x, back[i]))));
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          acc[i * HJ + 4 * q + e] = fmaf(a1[i], v[e], acc[i * HJ + 4 * q + e]);
+      }
+    }
+    // both halves' sums for the own hidden units
+    float g1[HI];
+#pragma unroll
+    for (int i = 0; i < HI; ++i) {
+      const float send = half ? back[i] : back[HI + i], keep = half ? back[HI + i] : back[i];
+      g1[i] = (keep + __shfl_xor_sync(0xffffffffu, send, 1)) * slope1[i];
+      acc[kB1 + i] += g1[i];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) acc[kW1 + d * HI + i] = fmaf(diff[d], g1[i], acc[kW1 + d * HI + i]);
+    }
+    if (dpdf) {
+      dpdf_m += __shfl_xor_sync(0xffffffffu, dpdf_m, 1);
+      if (live && half == 0) dpdf[m] = dpdf_m;
+    }
+    if (dp_in || dp_out) {
+      // a sample's pairs follow one another: its first lane in the warp adds them up
+      const int who = live ? nb.y : -1;
+      const int prev = __shfl_up_sync(0xffffffffu, who, 2);
+      const bool head = lane < 2 || prev != who;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float4 w = par.w1[d][half];
+        const float mine = g1[0] * w.x + g1[1] * w.y + g1[2] * w.z + g1[3] * w.w;
+        float v = (mine + __shfl_xor_sync(0xffffffffu, mine, 1)) * inv_radius;
+        if (live && half == 0 && dp_in) atomicAdd(dp_in + (int64_t)nb.x * 3 + d, v);
+#pragma unroll
+        for (int o = 2; o < 32; o <<= 1) {
+          const float y = __shfl_down_sync(0xffffffffu, v, o);
+          const int id = __shfl_down_sync(0xffffffffu, who, o);
+          if (lane + o < 32 && id == who) v += y;
+        }
+        if (live && half == 1 && head && dp_out) atomicAdd(dp_out + (int64_t)nb.y * 3 + d, -v);
+      }
+    }
+  }
+  // ---- sums over the lanes of the same half by halving (see kernel_basis_grads_kernel)
+  int first = 0;
+#pragma unroll
+  for (int step = 0; step < 4; ++step) {
+    const int o = 16 >> step, width = kPadded >> (step + 1);
+    const bool upper = (lane & o) != 0;
+    if (upper) first += width;
+#pragma unroll
+    for (int i = 0; i < kPadded / 2; ++i) {
+      if (i < width) {
+        const float send = upper ? acc[i] : acc[i + width];
+        const float keep = upper ? acc[i + width] : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kPadded / 16; ++i) atomicAdd(&red[half][first + i], acc[i]);
+  __syncthreads();
+  float* const dw1 = dweights + g * 3 * h1;
+  float* const dw2 = dweights + s.G * 3 * h1 + g * h1 * hl;
+  float* const db1 = dbiases + g * h1;
+  float* const db2 = dbiases + s.G * h1 + g * hl;
+  for (int i = threadIdx.x; i < 2 * kValues; i += 128) {
+    const int side = i >= kValues, v = side ? i - kValues : i;
+    const float x = red[side][v];
+    if (v < kW1) {
+      const int r = v / HJ, c = side * HJ + v % HJ;       // r = 8: the bias
+      if (c < hl && r < h1) atomicAdd(dw2 + r * hl + c, x);
+      else if (c < hl && r == kH1) atomicAdd(db2 + c, x);
+    } else {
+      const int d = (v - kW1) / HI, c = side * HI + (v - kW1) % HI;
+      if (c < h1) atomicAdd(d < 3 ? dw1 + d * h1 + c : db1 + c, x);
+    }
+  }
+}
+
 // Shared memory of a tile of `pairs` pairs.
 size_t mlp_smem(const MlpShape& s, int pairs, bool backward) {
   const size_t f = backward ? 2 * (size_t)s.params + (size_t)(s.rows + 2 * s.widest) * (pairs + 4)
@@ -451,6 +708,15 @@ extern "C" int tfgpc_kernel_mlp_basis_layers(
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_out,
                 "KernelMlpBasis got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  if (small_mlp(s)) {
+    const unsigned blocks = min(blocks_for(M, 256), (unsigned)(sm_count() * 8));
+    ProfScope prof(st, "kernel_mlp_basis");
+    TFGPC_CUDA(launch_chained(st, blocks, 256, 0,
+        s.h[2] <= 8 ? small_mlp_basis_kernel<8> : small_mlp_basis_kernel<16>, s, M, points_in,
+        points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
+        basis_out));
+    return TFGPC_OK;
+  }
   const int tile = mlp_tile(s, false);
   const size_t smem = mlp_smem(s, tile, false);
   TFGPC_CUDA(cudaFuncSetAttribute(kernel_mlp_basis_kernel,
@@ -513,6 +779,17 @@ extern "C" int tfgpc_kernel_mlp_grads_layers(
   if (M == 0) return TFGPC_OK;
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_grads,
                 "KernelMlpGrads got a null pointer");
+  // (the gradient of a density is the sum over its MLPs: written by one block row only)
+  if (small_mlp(s) && (s.G == 1 || !dpdf_out)) {
+    const unsigned most = max(3u * sm_count() / (unsigned)s.G, 1u);
+    dim3 blocks(min(blocks_for(M, 64), most), (unsigned)s.G);
+    ProfScope prof(st, "kernel_mlp_grads");
+    TFGPC_CUDA(launch_chained(st, blocks, 128, 0,
+        s.h[2] <= 8 ? small_mlp_grads_kernel<8> : small_mlp_grads_kernel<16>, s, M, points_in,
+        points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
+        basis_grads, dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out, dpdf_out));
+    return TFGPC_OK;
+  }
   const int tile = mlp_tile(s, true);
   const size_t smem = mlp_smem(s, tile, true);
   TFGPC_CUDA(cudaFuncSetAttribute(kernel_mlp_grads_kernel,
