@@ -399,6 +399,11 @@ int tfgpc_compute_pdf(void* stream, int D, int mode, int64_t n,
                       const float* points, const int32_t* neighbors, int64_t M,
                       const int32_t* ranges, const float* inv_bandwidth,
                       const float* inv_radii, float* pdf_out);
+/* out[j] = sum of values[m] over the pairs whose first index is j (neighbors [M,2],
+ * out [n], overwritten): per-pair gradients brought to the points, the transpose of
+ * the gather of Neighborhood.py:287. */
+int tfgpc_add_by_neighbor(void* stream, int64_t M, const int32_t* neighbors,
+                          const float* values, int64_t n, float* out);
 int tfgpc_compute_pdf_pt_grads(void* stream, int D, int mode, int64_t n,
                                const float* points, const int32_t* neighbors,
                                int64_t M, const int32_t* ranges,

@@ -6,7 +6,7 @@
 // ascending in point index, so mostly from the same cache lines), and the
 // partial sums are combined with shuffles.  The reference walks each list with
 // a single thread (compute_pdf_kernels.cu.cc:73-130).
-#include "common.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 
@@ -69,6 +69,7 @@ compute_pdf_grads_kernel(int mode, int64_t n, const float* __restrict__ pts,
                          const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
                          const float* __restrict__ inv_bw, const float* __restrict__ inv_r,
                          const float* __restrict__ pdf_grads, float* __restrict__ grads_out) {
+  chain_enter(n * 32, (int64_t)gridDim.x * kPdfThreads);
   float bw[D], ir[D];
   load_bandwidth<D>(mode, n, inv_bw, inv_r, bw, ir);
   const int lane = lane_id();
@@ -103,6 +104,18 @@ compute_pdf_grads_kernel(int mode, int64_t n, const float* __restrict__ pts,
       float v = warp_sum(own[d]);
       if (lane == 0 && v != 0.0f) atomicAdd(grads_out + i * D + d, v);
     }
+  }
+}
+
+// out[neighbor of pair m] += values[m]
+__global__ void __launch_bounds__(kPdfThreads)
+add_by_neighbor_kernel(int64_t M, int64_t n, const int2* __restrict__ neigh,
+                       const float* __restrict__ values, float* __restrict__ out) {
+  chain_enter(M, (int64_t)gridDim.x * kPdfThreads);
+  for (int64_t m = (int64_t)blockIdx.x * kPdfThreads + threadIdx.x; m < M;
+       m += (int64_t)gridDim.x * kPdfThreads) {
+    const int j = __ldg(&neigh[m].x);
+    if (j >= 0 && j < n) atomicAdd(out + j, __ldg(values + m));
   }
 }
 
@@ -169,12 +182,31 @@ extern "C" int tfgpc_compute_pdf_pt_grads(void* stream, int D, int mode, int64_t
   TFGPC_REQUIRE(points && ranges && inv_bandwidth && inv_radii && pdf_grads && pt_grads_out &&
                 (M == 0 || neighbors), "ComputePdfPtGrads got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  TFGPC_CUDA(cudaMemsetAsync(pt_grads_out, 0, sizeof(float) * (size_t)n * D, st));
+  Prepare jobs;
+  jobs.zero(pt_grads_out, sizeof(float) * (size_t)n * D);
+  rc = prepare(st, jobs);
+  if (rc) return rc;
   unsigned grid = min(blocks_for(n, kPdfThreads / 32), (unsigned)(sm_count() * 32));
   ProfScope prof(st, "compute_pdf_grads");
-  TFGPC_DIM_SWITCH(D, compute_pdf_grads_kernel<kD><<<grid, kPdfThreads, 0, st>>>(
-      mode, n, points, (const int2*)neighbors, ranges, inv_bandwidth, inv_radii, pdf_grads,
-      pt_grads_out));
-  TFGPC_LAUNCH_CHECK();
+  TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, grid, kPdfThreads, 0,
+      compute_pdf_grads_kernel<kD>, mode, n, points, (const int2*)neighbors, ranges,
+      inv_bandwidth, inv_radii, pdf_grads, pt_grads_out)));
+  return TFGPC_OK;
+}
+
+extern "C" int tfgpc_add_by_neighbor(void* stream, int64_t M, const int32_t* neighbors,
+                                     const float* values, int64_t n, float* out) {
+  TFGPC_REQUIRE(n >= 0 && n < (int64_t)INT32_MAX && M >= 0 && M <= (int64_t)INT32_MAX,
+                "AddByNeighbor expects 0 <= n, M < 2^31");
+  if (n == 0) return TFGPC_OK;
+  TFGPC_REQUIRE(out && (M == 0 || (neighbors && values)), "AddByNeighbor got a null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  Prepare jobs;
+  jobs.zero(out, sizeof(float) * (size_t)n);
+  int rc = prepare(st, jobs);
+  if (rc || M == 0) return rc;
+  ProfScope prof(st, "add_by_neighbor");
+  TFGPC_CUDA(launch_chained(st, min(blocks_for(M, kPdfThreads), (unsigned)(sm_count() * 16)),
+      kPdfThreads, 0, add_by_neighbor_kernel, M, n, (const int2*)neighbors, values, out));
   return TFGPC_OK;
 }

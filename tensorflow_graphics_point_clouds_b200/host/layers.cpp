@@ -151,6 +151,16 @@ py::tuple kernel_mlp_grads(const Tensor& p_in_, const Tensor& p_out_, const Tens
   return py::make_tuple(dw, db, a, b, *dpdf);
 }
 
+// [n] sums of values [M] over the pairs of every point (first index)
+Tensor add_by_neighbor(const Tensor& neigh_, const Tensor& values_, int64_t n) {
+  Tensor neigh = i32(neigh_), values = f32(values_);
+  require(neigh.dim() == 2 && neigh.size(1) == 2 && values.numel() == neigh.size(0),
+          "AddByNeighbor expects one value and two indices per pair");
+  Tensor out = empty({n}, at::kFloat, values);
+  check(tfgpc_add_by_neighbor(stream(), neigh.size(0), ip(neigh), fp(values), n, fpm(out)));
+  return out;
+}
+
 Tensor kp_basis(const Tensor& p_in_, const Tensor& p_out_, const Tensor& neigh_,
                 const Tensor& kernel_points_, double radius, double sigma, int64_t k_pad,
                 int interpolation) {
@@ -432,6 +442,7 @@ void bind_layers(py::module_& m) {
   m.def("kernel_basis_grads", &kernel_basis_grads);
   m.def("kernel_mlp_basis", &kernel_mlp_basis);
   m.def("kernel_mlp_grads", &kernel_mlp_grads);
+  m.def("add_by_neighbor", &add_by_neighbor);
   m.def("kp_basis", &kp_basis);
   m.def("pointconv_pdf", &pointconv_pdf);
   m.def("group_plan", &group_plan);

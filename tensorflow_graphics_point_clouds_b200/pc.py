@@ -437,14 +437,21 @@ class Neighborhood:
     sorted points = gather(points, sorted indices) (Grid.py:60-62)."""
     g = self._grid
     d = g._point_cloud._dimension
-    n = g._sorted_points.shape[0]
-    per_point = torch.zeros(n, dtype=torch.float32, device=g._sorted_points.device)
-    per_point.index_add_(0, self._neighbors[:, 0].to(torch.int64),
-                         torch.as_tensor(pdf_grads, dtype=torch.float32))
+    inv_bw = _to_dims(bandwidth, d, self._radii.device, inverse=True)
+    n = g._point_cloud._points.shape[0]
+    pdf_grads = torch.as_tensor(pdf_grads, dtype=torch.float32)
+    if not self._equal_samples and self._samples_are_grid_points():
+      # the grid's own cloud as samples: these lists are the self neighborhood's, in the
+      # points' own order
+      ids = self._original_neigh_ids
+      per_point = ops._lib.host().add_by_neighbor(ids, pdf_grads, n)
+      return ops.compute_pdf_pt_grads(g._point_cloud._points, ids, self._samples_neigh_ranges,
+                                      inv_bw, self._inv_radii, per_point, mode)
+    per_point = ops._lib.host().add_by_neighbor(self._neighbors, pdf_grads, n)
     nb = self if self._equal_samples else Neighborhood(g, self._radius)
     grads_sorted = ops.compute_pdf_pt_grads(
-        g._sorted_points, nb._neighbors, nb._samples_neigh_ranges,
-        _to_dims(bandwidth, d, self._radii.device, inverse=True), self._inv_radii, per_point, mode)
+        g._sorted_points, nb._neighbors, nb._samples_neigh_ranges, inv_bw, self._inv_radii,
+        per_point, mode)
     out = torch.empty_like(grads_sorted)
     out[g._sorted_indices.to(torch.int64)] = grads_sorted
     return out
