@@ -72,13 +72,13 @@ struct UTile {
   __device__ __forceinline__ int blocks() const { return (rows + kBlk - 1) / kBlk; }
 };
 
-__device__ __forceinline__ UTile load_utile(const int32_t* __restrict__ group_begin,
-                                            const int32_t* __restrict__ group_rows, int64_t groups,
+__device__ __forceinline__ UTile load_utile(const int32_t* group_begin,
+                                            const int32_t* group_rows, int64_t groups,
                                             int64_t g) {
   UTile t;
   if (g >= groups) { t.ra = 0; t.rows = 0; return t; }
-  t.ra = __ldg(group_begin + g);
-  t.rows = __ldg(group_rows + g);
+  t.ra = ld_global(group_begin + g);
+  t.rows = ld_global(group_rows + g);
   return t;
 }
 
@@ -119,11 +119,11 @@ __device__ __forceinline__ void st_global_256(void* p, const uint32_t* v) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
-basis_proj_fwd_tcu_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ group_begin,
-                          const int32_t* __restrict__ group_rows,
-                          const int32_t* __restrict__ rows_id, const int4* __restrict__ rows_pair,
-                          const __nv_bfloat16* __restrict__ basis_pair,
-                          const __nv_bfloat16* __restrict__ fs, __nv_bfloat16* __restrict__ x_hi,
+basis_proj_fwd_tcu_kernel(int64_t ns, int64_t groups, const int32_t* group_begin,
+                          const int32_t* group_rows,
+                          const int32_t* rows_id, const int4* rows_pair,
+                          const __nv_bfloat16* basis_pair,
+                          const __nv_bfloat16* fs, __nv_bfloat16* __restrict__ x_hi,
                           __nv_bfloat16* __restrict__ x_mid, uint32_t idesc, int* err_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -184,8 +184,8 @@ basis_proj_fwd_tcu_kernel(int64_t ns, int64_t groups, const int32_t* __restrict_
 #pragma unroll
       for (int it = 0; it < kSteps; ++it) {
         const bool have = 16 * it + frow < rows_n;
-        ids_n[it] = have ? __ldg(rows_id + r0 + 16 * it + frow) : 0;
-        pr_n[it] = have ? __ldg(reinterpret_cast<const int32_t*>(rows_pair + r0 + 16 * it + frow) + bq)
+        ids_n[it] = have ? ld_global(rows_id + r0 + 16 * it + frow) : 0;
+        pr_n[it] = have ? ld_global(reinterpret_cast<const int32_t*>(rows_pair + r0 + 16 * it + frow) + bq)
                         : -1;
       }
     };

@@ -73,9 +73,9 @@ struct Barriers {
 
 template <int G>
 __global__ void __launch_bounds__(kThreads, 1)
-basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basis,
-                           const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
-                           const int32_t* __restrict__ ranges, const uint8_t* __restrict__ image,
+basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* basis,
+                           const __nv_bfloat16* fs, const int2* neigh,
+                           const int32_t* ranges, const uint8_t* image,
                            float* __restrict__ dbasis, float* __restrict__ dfeat, uint32_t idesc1,
                            uint32_t idesc2, int* err_flag) {
   extern __shared__ uint8_t smem_raw[];
@@ -114,7 +114,7 @@ basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basi
 
   // pairs beyond the last range belong to no sample: their gradient is zero
   if (blockIdx.x == 0 && warp == kDxWarp) {
-    const int64_t covered = ns > 0 ? __ldg(ranges + ns - 1) : 0;
+    const int64_t covered = ns > 0 ? ld_global(ranges + ns - 1) : 0;
     for (int64_t i = covered * kK + lane; i < M * kK; i += 32) dbasis[i] = 0.0f;
   }
 
@@ -145,13 +145,13 @@ basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basi
       m0_n = walk.t.pa + walk.b * kRows + row_base;
       // ids of rows 0-7 in lanes 0-7, of rows 8-15 in lanes 16-23: a shuffle within
       // half warps then hands row it + 8 * (lane / 16) to every lane
-      idx_n = ((lane & 8) == 0 && m0_n + idx_row < t_n.pe) ? __ldg(&neigh[m0_n + idx_row].x) : 0;
+      idx_n = ((lane & 8) == 0 && m0_n + idx_row < t_n.pe) ? ld_global(&neigh[m0_n + idx_row].x) : 0;
       b0_n = b1_n = make_float4(0.f, 0.f, 0.f, 0.f);
       if (m0_n + brow < t_n.pe) {
         const float4* src =
             reinterpret_cast<const float4*>(basis + (int64_t)(m0_n + brow) * kK + 8 * bh);
-        b0_n = __ldg(src);
-        b1_n = __ldg(src + 1);
+        b0_n = ld_global(src);
+        b1_n = ld_global(src + 1);
       }
     };
     if (walk.valid) prefetch();
@@ -348,7 +348,7 @@ basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basi
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int mp = m_first + 32 * (half + 2 * u) + lane;
-        pts[u] = mp < t.pe ? __ldg(&neigh[mp].x) : 0;
+        pts[u] = mp < t.pe ? ld_global(&neigh[mp].x) : 0;
       }
       const uint32_t abuf = item & 1;
       TT_WAIT(0, smem_u32(&bars->acc_full[abuf]), (item >> 1) & 1);
@@ -397,7 +397,7 @@ basis_proj_grads_tc_kernel(int64_t ns, int64_t M, const float* __restrict__ basi
             const int2* idp = neigh + m_first + col0;
             int p[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) p[i] = __ldg(&idp[i].x);
+            for (int i = 0; i < 32; ++i) p[i] = ld_global(&idp[i].x);
 #pragma unroll
             for (int i = 0; i < 32; ++i)
               atomicAdd(dcol + (int64_t)p[i] * kC, __uint_as_float(v[i]));

@@ -78,13 +78,13 @@ struct UTile {
   __device__ __forceinline__ int blocks() const { return (rows + kBlk - 1) / kBlk; }
 };
 
-__device__ __forceinline__ UTile load_utile(const int32_t* __restrict__ group_begin,
-                                            const int32_t* __restrict__ group_rows, int64_t groups,
+__device__ __forceinline__ UTile load_utile(const int32_t* group_begin,
+                                            const int32_t* group_rows, int64_t groups,
                                             int64_t g) {
   UTile t;
   if (g >= groups) { t.ra = 0; t.rows = 0; return t; }
-  t.ra = __ldg(group_begin + g);
-  t.rows = __ldg(group_rows + g);
+  t.ra = ld_global(group_begin + g);
+  t.rows = ld_global(group_rows + g);
   return t;
 }
 
@@ -122,12 +122,12 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 
 __global__ void __launch_bounds__(kThreads, 1)
 basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
-                            const int32_t* __restrict__ group_begin,
-                            const int32_t* __restrict__ group_rows,
-                            const int32_t* __restrict__ rows_id, const int4* __restrict__ rows_pair,
-                            const __nv_bfloat16* __restrict__ basis_pair,
-                            const __nv_bfloat16* __restrict__ fs, const int32_t* __restrict__ ranges,
-                            const uint8_t* __restrict__ image, float* __restrict__ dbasis,
+                            const int32_t* group_begin,
+                            const int32_t* group_rows,
+                            const int32_t* rows_id, const int4* rows_pair,
+                            const __nv_bfloat16* basis_pair,
+                            const __nv_bfloat16* fs, const int32_t* ranges,
+                            const uint8_t* image, float* __restrict__ dbasis,
                             float* __restrict__ dfeat, uint32_t idesc1, uint32_t idesc2,
                             int* err_flag) {
   extern __shared__ uint8_t smem_raw[];
@@ -167,7 +167,7 @@ basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
 
   // pairs beyond the last range belong to no sample: their gradient is zero
   if (blockIdx.x == 0 && warp == kDxWarp) {
-    const int64_t covered = ns > 0 ? __ldg(ranges + ns - 1) : 0;
+    const int64_t covered = ns > 0 ? ld_global(ranges + ns - 1) : 0;
     for (int64_t i = covered * kK + lane; i < M * kK; i += 32) dbasis[i] = 0.0f;
   }
 
@@ -199,8 +199,8 @@ basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
 #pragma unroll
       for (int it = 0; it < kSteps; ++it) {
         const bool have = 16 * it + frow < rows_n;
-        ids_n[it] = have ? __ldg(rows_id + r0 + 16 * it + frow) : 0;
-        pr_n[it] = have ? __ldg(reinterpret_cast<const int32_t*>(rows_pair + r0 + 16 * it + frow) + bq)
+        ids_n[it] = have ? ld_global(rows_id + r0 + 16 * it + frow) : 0;
+        pr_n[it] = have ? ld_global(reinterpret_cast<const int32_t*>(rows_pair + r0 + 16 * it + frow) + bq)
                         : -1;
       }
     };
@@ -361,10 +361,10 @@ basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int c = 32 * (half + 2 * u) + lane;
-        pts[u] = c < rows ? __ldg(rows_id + r_first + c) : 0;
+        pts[u] = c < rows ? ld_global(rows_id + r_first + c) : 0;
       }
       int4 pr = make_int4(-1, -1, -1, -1);
-      if (half == 1 && r < rows) pr = __ldg(rows_pair + r_first + r);
+      if (half == 1 && r < rows) pr = ld_global(rows_pair + r_first + r);
       const uint32_t abuf = item % kAccBufs;
       mbar_wait(smem_u32(&bars->acc_full[abuf]), (item / kAccBufs) & 1, abort_flag, err_flag);
       tc_fence_after();

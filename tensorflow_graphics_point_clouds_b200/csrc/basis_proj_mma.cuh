@@ -134,11 +134,11 @@ struct Walker {
 
   // end of the pairs of item i
   __device__ __forceinline__ int item_end(int64_t i) const {
-    if (parts == 1) return __ldg(ranges + i);
+    if (parts == 1) return ld_global(ranges + i);
     const int64_t s = i / parts;
     const int p = (int)(i - s * parts) + 1;
-    const int end = __ldg(ranges + s);
-    const int begin = s > 0 ? __ldg(ranges + s - 1) : 0;
+    const int end = ld_global(ranges + s);
+    const int begin = s > 0 ? ld_global(ranges + s - 1) : 0;
     return part_end(begin, end, p, parts, kChunk);
   }
 
@@ -195,15 +195,15 @@ struct Walker {
 // ---- staging ---------------------------------------------------------------------------
 
 // Neighbor (point) index of pair base + lane of a job, 0 beyond the chunk.
-__device__ __forceinline__ int load_idx(const Job& j, const int2* __restrict__ neigh, int lane) {
-  return (j.valid() && lane < j.cnt) ? __ldg(&neigh[j.base + lane].x) : 0;
+__device__ __forceinline__ int load_idx(const Job& j, const int2* neigh, int lane) {
+  return (j.valid() && lane < j.cnt) ? ld_global(&neigh[j.base + lane].x) : 0;
 }
 
 // Starts the gather of a chunk's feature rows: row r of the tile receives
 // hi[c0 .. c0+w) and mid[c0 .. c0+w) of point idx(r); rows beyond the chunk are
 // zero-filled.  One commit group per call is left to the caller.
 template <int K, int CC>
-__device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat16* __restrict__ fs,
+__device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat16* fs,
                                                int C, int c0, int w, int idx, int cnt, int lane) {
   typedef Cfg<K, CC> cfg;
   constexpr int kLph = cfg::kCC / 8;           // 16-byte segments per half row
@@ -225,13 +225,13 @@ __device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat1
 // Basis rows of a chunk, 16 x K floats contiguous in memory: each lane loads
 // K/8 float4 (zeros beyond the chunk) ...
 template <int K>
-__device__ __forceinline__ void load_basis(const float* __restrict__ basis, int base, int cnt,
+__device__ __forceinline__ void load_basis(const float* basis, int base, int cnt,
                                            int lane, float4* v) {
   const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)base * K);
 #pragma unroll
   for (int t = 0; t < K / 8; ++t) {
     const int i = lane + 32 * t;
-    v[t] = (i / (K / 4) < cnt) ? __ldg(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[t] = (i / (K / 4) < cnt) ? ld_global(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 }
 
@@ -275,9 +275,9 @@ __device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float
 // kernel MLPs, one after the other.
 template <int K, int CC, int OUT>
 __global__ void __launch_bounds__(Cfg<K, CC>::kFwdWarps * 32, 1)
-basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* __restrict__ basis,
-                      const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
-                      const int32_t* __restrict__ ranges, float* __restrict__ out,
+basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
+                      const __nv_bfloat16* fs, const int2* neigh,
+                      const int32_t* ranges, float* __restrict__ out,
                       __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid) {
   chain_enter(ns * 32, (int64_t)gridDim.x * blockDim.x);
   typedef Cfg<K, CC> cfg;
@@ -507,9 +507,9 @@ struct ChunkWalk {
   int blk, li, upto, begin, upto_next, begin_next;   // upto: end of the lane's item of the block
 
   __device__ __forceinline__ int item_end(int i) const {
-    if (parts == 1) return __ldg(ranges + i);
+    if (parts == 1) return ld_global(ranges + i);
     const int s = i / parts;
-    return part_end(s > 0 ? __ldg(ranges + s - 1) : 0, __ldg(ranges + s), i - s * parts + 1, parts,
+    return part_end(s > 0 ? ld_global(ranges + s - 1) : 0, ld_global(ranges + s), i - s * parts + 1, parts,
                     kChunk);
   }
   __device__ __forceinline__ void load(int64_t b, int* upto_b, int* begin_b) const {
@@ -562,10 +562,10 @@ struct ChunkWalk {
 template <int K, int CC>
 __global__ void __launch_bounds__(GradCfg<K, CC>::kThreads, 1)
 basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int64_t M,
-                            const float* __restrict__ basis,
-                            const __nv_bfloat16* __restrict__ fs, const int2* __restrict__ neigh,
-                            const int32_t* __restrict__ ranges,
-                            const float* __restrict__ in_grads, float* __restrict__ dbasis,
+                            const float* basis,
+                            const __nv_bfloat16* fs, const int2* neigh,
+                            const int32_t* ranges,
+                            const float* in_grads, float* __restrict__ dbasis,
                             float* __restrict__ dfeat) {
   typedef GradCfg<K, CC> cfg;
   constexpr int W = cfg::kTeam;
@@ -596,7 +596,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
 
   // pairs beyond the last range belong to no sample: their gradient is zero
   if (blockIdx.x == 0 && threadIdx.x < 32) {
-    const int64_t covered = ns > 0 ? __ldg(ranges + ns - 1) : 0;
+    const int64_t covered = ns > 0 ? ld_global(ranges + ns - 1) : 0;
     for (int64_t i = covered * K + lane; i < M * K; i += 32) dbasis[i] = 0.0f;
   }
 
@@ -653,7 +653,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
       const int have = j.cnt() * (K / 4) - tid;
 #pragma unroll
       for (int t = 0; t < cfg::kBasisVecs; ++t)
-        if (32 * W * t < have) v[t] = __ldg(src + 32 * W * t);
+        if (32 * W * t < have) v[t] = ld_global(src + 32 * W * t);
     };
     uint8_t* const b_dst = mem + cfg::kRawBytes + cfg::kFeatBytes + tid / (K / 4) * cfg::kKStride +
                            tid % (K / 4) * 8;
@@ -685,7 +685,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
                            (int)gridDim.x * cfg::kTeams, lane, bs, parts);
     Chunk n1 = walk.next(cur), n2 = walk.next(n1);
     auto load_idx = [&](const Chunk& j) {
-      return j.valid() && lane < j.cnt() ? __ldg(&neigh[j.base + lane].x) : 0;
+      return j.valid() && lane < j.cnt() ? ld_global(&neigh[j.base + lane].x) : 0;
     };
     int idx0 = load_idx(cur), idx1 = load_idx(n1);
     float4 rows[cfg::kBasisVecs];

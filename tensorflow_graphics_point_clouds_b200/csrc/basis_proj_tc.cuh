@@ -27,15 +27,15 @@ struct Tile {
 };
 
 template <int G>
-__device__ __forceinline__ Tile load_tile(const int32_t* __restrict__ ranges, int64_t ns, int64_t g) {
+__device__ __forceinline__ Tile load_tile(const int32_t* ranges, int64_t ns, int64_t g) {
   Tile t;
   const int64_t s0 = g * G;
   if (s0 >= ns) { t.pa = t.e0 = t.e1 = t.e2 = t.pe = 0; return t; }
-  t.pa = s0 > 0 ? __ldg(ranges + s0 - 1) : 0;
-  t.e0 = __ldg(ranges + s0);
-  t.e1 = __ldg(ranges + min(s0 + 1, ns - 1));
-  t.e2 = __ldg(ranges + min(s0 + 2, ns - 1));
-  t.pe = G == 4 ? __ldg(ranges + min(s0 + 3, ns - 1)) : t.e2;
+  t.pa = s0 > 0 ? ld_global(ranges + s0 - 1) : 0;
+  t.e0 = ld_global(ranges + s0);
+  t.e1 = ld_global(ranges + min(s0 + 1, ns - 1));
+  t.e2 = ld_global(ranges + min(s0 + 2, ns - 1));
+  t.pe = G == 4 ? ld_global(ranges + min(s0 + 3, ns - 1)) : t.e2;
   return t;
 }
 

@@ -70,7 +70,7 @@ __device__ __forceinline__ void clip_and_report(int D, int max_cells, const int*
 // (custom_ops_wrapper.py:37-43); every division is the IEEE one.
 template <int D>
 __global__ void __launch_bounds__(kThreads)
-boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict__ batch_ids,
+boxes_kernel(int64_t n, const float* pts, const int32_t* batch_ids,
              int batch_size, unsigned* lo_keys, unsigned* hi_keys, unsigned* ticket,
              DimValues cell_sizes, int max_cells, float* __restrict__ aabb_min,
              float* __restrict__ aabb_max, int32_t* __restrict__ num_cells,
@@ -98,7 +98,7 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
   for (int i = 0; i < kBoxPer; ++i) {
     const int64_t p = begin + i * 32;
     if (p >= n) break;
-    const int b = __ldg(batch_ids + p);
+    const int b = ld_global(batch_ids + p);
     if (b != cur) {
       flush();
       cur = b;
@@ -107,7 +107,7 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
     }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const float v = __ldg(pts + p * D + d);
+      const float v = ld_global(pts + p * D + d);
       lo[d] = fminf(lo[d], v);
       hi[d] = fmaxf(hi[d], v);
     }
@@ -156,7 +156,7 @@ boxes_kernel(int64_t n, const float* __restrict__ pts, const int32_t* __restrict
 }
 
 // Cell counts given by the caller (reduced over the shards of a batch).
-__global__ void given_cells_kernel(int D, const int32_t* __restrict__ given, int max_cells,
+__global__ void given_cells_kernel(int D, const int32_t* given, int max_cells,
                                    int32_t* __restrict__ used, int32_t* crowded,
                                    int32_t* page) {
   chain_enter();
@@ -198,25 +198,26 @@ __device__ __forceinline__ int arrive(int32_t* counts, int bucket, unsigned live
 // Keys, and the number of points per bucket.
 template <int D>
 __global__ void __launch_bounds__(kThreads)
-keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
-                      const int32_t* __restrict__ batch_ids, int batch_size,
-                      const float* __restrict__ smin_all, const int32_t* __restrict__ num_cells,
-                      const float* __restrict__ inv_cell, int64_t* __restrict__ keys_out,
-                      int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded) {
+keys_histogram_kernel(int64_t n, const float* pts,
+                      const int32_t* batch_ids, int batch_size,
+                      const float* smin_all, const int32_t* num_cells,
+                      const float* inv_cell, int64_t* __restrict__ keys_out,
+                      int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded,
+                      int64_t capacity) {
   chain_enter();
   const Grid<D> g = load_grid<D>(num_cells, inv_cell);
   const int total = total_cells<D>(g.nc, batch_size);
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   const unsigned live = __ballot_sync(0xffffffffu, i < n);
-  if (i >= n || total == 0) return;
-  const int b = __ldg(batch_ids + i);
+  if (i >= n || total <= 0 || total > capacity) return;     // (what the table holds)
+  const int b = ld_global(batch_ids + i);
   const int bs = min(max(b, 0), batch_size - 1);   // (the key keeps the id that was passed in)
   float p[D], smin[D];
   int cell[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    p[d] = __ldg(pts + i * D + d);
-    smin[d] = __ldg(smin_all + (int64_t)bs * D + d);
+    p[d] = ld_global(pts + i * D + d);
+    smin[d] = ld_global(smin_all + (int64_t)bs * D + d);
   }
   cell_of<D>(p, smin, g, cell);
   const int64_t key = key_of<D>(cell, g, b);
@@ -226,19 +227,19 @@ keys_histogram_kernel(int64_t n, const float* __restrict__ pts,
 
 template <int D>
 __global__ void __launch_bounds__(kThreads)
-scatter_kernel(int64_t n, const int64_t* __restrict__ keys, const int32_t* __restrict__ num_cells,
-               int batch_size, const int32_t* __restrict__ start,
-               const int32_t* __restrict__ arrival, int32_t* __restrict__ members) {
+scatter_kernel(int64_t n, const int64_t* keys, const int32_t* num_cells,
+               int batch_size, const int32_t* start,
+               const int32_t* arrival, int32_t* __restrict__ members) {
   chain_enter();
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   if (i >= n) return;
   int nc[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
+  for (int d = 0; d < D; ++d) nc[d] = ld_global(num_cells + d);
   const int total = total_cells<D>(nc, batch_size);
   if (total == 0) return;
-  const int r = bucket_of(__ldg(keys + i), total);
-  members[__ldg(start + r) + __ldg(arrival + i)] = (int32_t)i;
+  const int r = bucket_of(ld_global(keys + i), total);
+  members[ld_global(start + r) + ld_global(arrival + i)] = (int32_t)i;
 }
 
 // Number of the members [a, e) of a bucket with an index below idx.
@@ -350,17 +351,17 @@ __device__ __forceinline__ int rank_in_tile(RankScratch<THREADS>& s, const int32
 // point's row of every sorted array; then the tube ranges, read off the table.
 template <int D, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __restrict__ keys,
-             const int32_t* __restrict__ num_cells, int batch_size,
-             const int32_t* __restrict__ start, const float* __restrict__ pts,
-             const int32_t* __restrict__ batch_ids, int32_t* __restrict__ perm,
+place_kernel(int64_t n, const int32_t* members, const int64_t* keys,
+             const int32_t* num_cells, int batch_size,
+             const int32_t* start, const float* pts,
+             const int32_t* batch_ids, int32_t* __restrict__ perm,
              int64_t* __restrict__ skeys, float* __restrict__ spts, int32_t* __restrict__ sbid,
              float4* __restrict__ packed, int2* __restrict__ ds,
-             const int32_t* __restrict__ crowded) {
+             const int32_t* crowded) {
   chain_enter();
   int nc[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) nc[d] = __ldg(num_cells + d);
+  for (int d = 0; d < D; ++d) nc[d] = ld_global(num_cells + d);
   const int total = total_cells<D>(nc, batch_size);
   if (total == 0) return;
   __shared__ RankScratch<THREADS> scratch;
@@ -369,24 +370,24 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
   int idx = 0, a = 0, e = 0;
   int64_t key = 0;
   if (live) {
-    idx = __ldg(members + i);
-    key = __ldg(keys + idx);
+    idx = ld_global(members + i);
+    key = ld_global(keys + idx);
     const int r = bucket_of(key, total);
-    a = __ldg(start + r);
-    e = __ldg(start + r + 1);
+    a = ld_global(start + r);
+    e = ld_global(start + r + 1);
   }
   const int rank = rank_in_tile<THREADS>(
       scratch, members, a, e, (int)(i - threadIdx.x), idx, live,
-      live && (threadIdx.x == THREADS - 1 || i == n - 1), __ldg(crowded) != 0);
+      live && (threadIdx.x == THREADS - 1 || i == n - 1), ld_global(crowded) != 0);
   if (live) {
     const int64_t o = a + rank;
     perm[o] = idx;
     skeys[o] = key;
-    sbid[o] = __ldg(batch_ids + idx);
+    sbid[o] = ld_global(batch_ids + idx);
     float p[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      p[d] = __ldg(pts + (int64_t)idx * D + d);
+      p[d] = ld_global(pts + (int64_t)idx * D + d);
       spts[o * D + d] = p[d];
     }
     if (D <= 3) packed[o] = make_float4(p[0], p[1], D == 3 ? p[D - 1] : 0.0f, __int_as_float(idx));
@@ -396,8 +397,8 @@ place_kernel(int64_t n, const int32_t* __restrict__ members, const int64_t* __re
   for (int d = 2; d < D; ++d) span *= nc[d];
   const int tubes = total / span;
   for (int64_t t = i; t < tubes; t += (int64_t)gridDim.x * THREADS) {
-    const int a = __ldg(start + (total - ((int)t * span + span - 1)));
-    const int e = __ldg(start + (total - (int)t * span) + 1);
+    const int a = ld_global(start + (total - ((int)t * span + span - 1)));
+    const int e = ld_global(start + (total - (int)t * span) + 1);
     ds[t] = e > a ? make_int2(a, e) : make_int2(0, 0);
   }
 }
@@ -451,11 +452,11 @@ grid_cluster_kernel(ClusterBuild a) {
   for (int i0 = first - lane; i0 < n; i0 += stride) {
     const int i = i0 + lane;
     const bool live = i < n;
-    const int b = live ? __ldg(a.batch_ids + i) : -1;
+    const int b = live ? ld_global(a.batch_ids + i) : -1;
     float lo[D], hi[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const float v = live ? __ldg(a.pts + (int64_t)i * D + d) : 0.0f;
+      const float v = live ? ld_global(a.pts + (int64_t)i * D + d) : 0.0f;
       // (a coordinate that is no number counts for no box)
       lo[d] = live ? fminf(INFINITY, v) : INFINITY;
       hi[d] = live ? fmaxf(-INFINITY, v) : -INFINITY;
@@ -531,12 +532,12 @@ grid_cluster_kernel(ClusterBuild a) {
     const int i = i0 + lane;
     const unsigned live = __ballot_sync(0xffffffffu, i < n);
     if (i >= n) break;
-    const int b = __ldg(a.batch_ids + i);
+    const int b = ld_global(a.batch_ids + i);
     const int bs = min(max(b, 0), a.batch_size - 1);
     float p[D];
     int cell[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = __ldg(a.pts + (int64_t)i * D + d);
+    for (int d = 0; d < D; ++d) p[d] = ld_global(a.pts + (int64_t)i * D + d);
     cell_of<D>(p, smin_s + bs * D, g, cell);
     const int64_t key = key_of<D>(cell, g, b);
     __stcg((long long*)a.g.keys + i, (long long)key);
@@ -613,11 +614,11 @@ grid_cluster_kernel(ClusterBuild a) {
     if (!live) break;
     a.g.sorted_indices[o] = idx;
     a.g.sorted_keys[o] = key;
-    a.g.sorted_batch_ids[o] = __ldg(a.batch_ids + idx);
+    a.g.sorted_batch_ids[o] = ld_global(a.batch_ids + idx);
     float p[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      p[d] = __ldg(a.pts + (int64_t)idx * D + d);
+      p[d] = ld_global(a.pts + (int64_t)idx * D + d);
       a.g.sorted_points[(int64_t)o * D + d] = p[d];
     }
     if (D <= 3)
@@ -751,7 +752,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
     TFGPC_CUDA(cudaMemsetAsync(g.cell_start, 0, (size_t)(cells + 3) * 4, st));
     TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0,
         keys_histogram_kernel<kD>, n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells,
-        g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded)));
+        g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded, cells)));
   }
   int rc = exclusive_scan_cells(st, g.cell_start, g.num_cells, D, B, cells + 3, w.sums);
   if (rc) return rc;

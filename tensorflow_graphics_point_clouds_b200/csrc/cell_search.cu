@@ -36,14 +36,14 @@ struct Sample {
 template <int D>
 __device__ __forceinline__ void load_point(const CellsView& c, int64_t j, float* p, int* index) {
   if (D <= 3) {
-    const float4 v = __ldg(c.packed + j);
+    const float4 v = ld_global(c.packed + j);
     p[0] = v.x; p[1] = v.y;
     if (D == 3) p[D - 1] = v.z;
     *index = __float_as_int(v.w);
   } else {
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = __ldg(c.points + j * D + d);
-    *index = __ldg(c.indices + j);
+    for (int d = 0; d < D; ++d) p[d] = ld_global(c.points + j * D + d);
+    *index = ld_global(c.indices + j);
   }
 }
 
@@ -59,19 +59,19 @@ __device__ __forceinline__ Sample<D> load_sample(const CellsView& c, const Sampl
   if (!live) return s;
   if (src.mode == 0) {
     s.id = (int)v;
-    s.batch = __ldg(src.batch_ids + v);
+    s.batch = ld_global(src.batch_ids + v);
 #pragma unroll
-    for (int d = 0; d < D; ++d) s.p[d] = __ldg(src.samples + v * D + d);
+    for (int d = 0; d < D; ++d) s.p[d] = ld_global(src.samples + v * D + d);
   } else {
     int index;
     load_point<D>(c, v, s.p, &index);
     s.id = src.mode == 1 ? index : (int)v;
-    s.batch = __ldg(c.batch_ids + v);
+    s.batch = ld_global(c.batch_ids + v);
   }
   if (s.batch < 0 || s.batch >= c.batch_size) return s;
   float smin[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) smin[d] = __ldg(c.scaled_min + (int64_t)s.batch * D + d);
+  for (int d = 0; d < D; ++d) smin[d] = ld_global(c.scaled_min + (int64_t)s.batch * D + d);
   cell_of<D>(s.p, smin, g, s.cell);
   s.key = (int)key_of<D>(s.cell, g, s.batch);
   return s;
@@ -159,10 +159,10 @@ cells_walk_kernel(WalkArgs a) {
   bool isotropic = true;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    const float r = __ldg(a.inv_radii + d);
+    const float r = ld_global(a.inv_radii + d);
     inv_r[d] = pack2(r, r);
     if (MODE == kDensity) {
-      const float bw = a.bw_mode == 1 ? sqrtf((float)c.n) : __ldg(a.inv_bw + d);
+      const float bw = a.bw_mode == 1 ? sqrtf((float)c.n) : ld_global(a.inv_bw + d);
       // of a base-2 exponential, in two parts: rounded once it would shift all
       // exponents of a sample the same way
       const double factor = (double)bw * bw * (-0.5 * 1.4426950408889634);
@@ -178,7 +178,7 @@ cells_walk_kernel(WalkArgs a) {
   const Sample<D> s = load_sample<D>(c, a.src, v0 + lane, live, g);
   int my_count = 0, my_begin = 0;
   float my_density = 0.0f;
-  if (MODE == kFill && s.id > 0) my_begin = __ldg(a.ranges + s.id - 1);
+  if (MODE == kFill && s.id > 0) my_begin = ld_global(a.ranges + s.id - 1);
   unsigned open = __ballot_sync(0xffffffffu, s.key >= 0);
   while (open) {
     // the samples of one cell

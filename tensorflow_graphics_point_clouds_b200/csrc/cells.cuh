@@ -65,7 +65,7 @@ __host__ __device__ constexpr int num_tubes() {
 // descending code and points ascending inside a tube is ascending sorted index.
 template <int D>
 __device__ __forceinline__ int2 tube_points(int code, const int* cell, int batch, const int* nc,
-                                            int total, const int32_t* __restrict__ start) {
+                                            int total, const int32_t* start) {
   int base = 0, scale = 1, rem = code;
   bool ok = true;
 #pragma unroll
@@ -80,7 +80,7 @@ __device__ __forceinline__ int2 tube_points(int code, const int* cell, int batch
   base = (batch * scale + base) * nc[D - 1];
   const int hi = base + min(cell[D - 1] + 1, nc[D - 1] - 1);
   const int lo = base + max(cell[D - 1] - 1, 0);
-  return make_int2(__ldg(start + (total - hi)), __ldg(start + (total - lo) + 1));
+  return make_int2(ld_global(start + (total - hi)), ld_global(start + (total - lo) + 1));
 }
 
 }  // namespace tfgpc

@@ -108,6 +108,12 @@ cudaError_t launch_chained(cudaStream_t st, dim3 grid, dim3 block, size_t smem, 
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+// Every load of a chained kernel is a plain one: the kernel begins before its inputs are
+// written, so that a load on the read-only path (__ldg, or a const __restrict__ parameter,
+// which gets it by itself) may be made before the wait.
+template <typename T>
+__device__ __forceinline__ T ld_global(const T* p) { return *p; }
+
 // Waits for the kernel before this one and, in a short kernel, lets the next one be set up
 // at once (else that happens as the blocks end).  Nothing but the kernel's own parameters,
 // shared memory and tensor memory is touched before it.  Short: the grid makes at most
@@ -140,13 +146,13 @@ struct Grid {
 // Loads the D cell counts / inverse cell sizes that the reference keeps in
 // device tensors (they are op inputs, so the host never reads them).
 template <int D>
-__device__ __forceinline__ Grid<D> load_grid(const int32_t* __restrict__ num_cells,
-                                             const float* __restrict__ inv_cell) {
+__device__ __forceinline__ Grid<D> load_grid(const int32_t* num_cells,
+                                             const float* inv_cell) {
   Grid<D> g;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    g.nc[d] = __ldg(num_cells + d);
-    g.inv[d] = __ldg(inv_cell + d);
+    g.nc[d] = ld_global(num_cells + d);
+    g.inv[d] = ld_global(inv_cell + d);
   }
   return g;
 }

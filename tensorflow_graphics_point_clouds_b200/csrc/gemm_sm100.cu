@@ -117,8 +117,8 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
                    const __grid_constant__ CUtensorMap tm_b_mid,
                    const __grid_constant__ CUtensorMap tm_c, int64_t m_total, int64_t n_total,
                    int bn, int stages, uint32_t idesc, TileSchedule sch, int* err_flag,
-                   const float* __restrict__ bias, uint8_t* image, int image_channels,
-                   int image_group, const int32_t* __restrict__ row_order) {
+                   const float* bias, uint8_t* image, int image_channels,
+                   int image_group, const int32_t* row_order) {
   extern __shared__ uint8_t smem_raw[];
   // the swizzled tiles need 1024-byte alignment
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -287,7 +287,7 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
           const int64_t j = (int64_t)n * bn + c0 + lane;
           if (j < n_total && !*abort_flag) {
             float* dst = reinterpret_cast<float*>(image) +
-                         (int64_t)__ldg(row_order + j) * image_channels + row0;
+                         (int64_t)ld_global(row_order + j) * image_channels + row0;
             if (row0 + 32 <= m_total) {
 #pragma unroll
               for (int q = 0; q < 8; q += 2)   // whole 32-byte sectors per store
@@ -328,11 +328,11 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
             const int64_t col = (int64_t)n * bn + c0 + i;
-            if (col < n_total) r[i] = __float_as_uint(__uint_as_float(r[i]) + __ldg(bias + col));
+            if (col < n_total) r[i] = __float_as_uint(__uint_as_float(r[i]) + ld_global(bias + col));
           }
         }
         if (OUT == 2 && bias && sp == 0 && row0 + lane < m_total) {
-          const float v = __ldg(bias + row0 + lane);
+          const float v = ld_global(bias + row0 + lane);
 #pragma unroll
           for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + v);
         }
@@ -532,8 +532,8 @@ __global__ void wait_probe_kernel(int* err_flag, unsigned long long limit_ns, in
 // out = the sum of `slices` slices, one after the other (and the bias, [cols] or
 // null), four values per thread.
 __global__ void __launch_bounds__(256)
-sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, int64_t rows,
-                  int cols, const float* __restrict__ bias, float* __restrict__ out, int64_t ldc,
+sum_slices_kernel(const float* partials, int slices, int batches, int64_t rows,
+                  int cols, const float* bias, float* __restrict__ out, int64_t ldc,
                   int64_t c_batch_stride) {
   chain_enter();
   const int quads = cols / 4;
@@ -541,17 +541,17 @@ sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, i
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= per_slice) return;
   const float4* src = reinterpret_cast<const float4*>(partials) + i;
-  float4 v = __ldg(src);
+  float4 v = ld_global(src);
 #pragma unroll 4
   for (int s = 1; s < slices; ++s) {
-    const float4 t = __ldg(src + (int64_t)s * per_slice);
+    const float4 t = ld_global(src + (int64_t)s * per_slice);
     v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
   }
   const int64_t r = i / quads;
   const int c = (int)(i - r * quads) * 4;
   if (bias) {
-    v.x += __ldg(bias + c); v.y += __ldg(bias + c + 1);
-    v.z += __ldg(bias + c + 2); v.w += __ldg(bias + c + 3);
+    v.x += ld_global(bias + c); v.y += ld_global(bias + c + 1);
+    v.z += ld_global(bias + c + 2); v.w += ld_global(bias + c + 3);
   }
   const int64_t b = r / rows;
   *reinterpret_cast<float4*>(out + b * c_batch_stride + (r - b * rows) * ldc + c) = v;
@@ -559,7 +559,7 @@ sum_slices_kernel(const float* __restrict__ partials, int slices, int batches, i
 
 // hi_t, mid_t [cols, rows] = the split of the transpose of x, whose rows and columns are
 // padded with zeros as in split_block (prepare.cu).
-__global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows, int64_t cols,
+__global__ void split_transpose_kernel(const float* x, int64_t rows, int64_t cols,
                                        int cols_src, int k_src, int k_dst,
                                        __nv_bfloat16* __restrict__ hi_t,
                                        __nv_bfloat16* __restrict__ mid_t) {
@@ -571,7 +571,7 @@ __global__ void split_transpose_kernel(const float* __restrict__ x, int64_t rows
     const int64_t ch = r / k_dst;
     const int k = (int)(r - ch * k_dst);
     tile[j][threadIdx.x] = (r < rows && cc < cols_src && k < k_src)
-                               ? __ldg(x + (ch * k_src + k) * cols_src + cc) : 0.0f;
+                               ? ld_global(x + (ch * k_src + k) * cols_src + cc) : 0.0f;
   }
   __syncthreads();
   for (int j = threadIdx.y; j < 32; j += blockDim.y) {

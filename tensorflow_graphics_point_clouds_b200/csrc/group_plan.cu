@@ -50,15 +50,15 @@ constexpr int kPlanThreads = 256;
 constexpr int kPlanWarps = kPlanThreads / 32;
 
 // Pairs of sample s: [a, a + n).
-__device__ __forceinline__ void sample_range(const int32_t* __restrict__ ranges, int64_t s, int& a,
+__device__ __forceinline__ void sample_range(const int32_t* ranges, int64_t s, int& a,
                                              int& n) {
-  a = s > 0 ? __ldg(ranges + s - 1) : 0;
-  n = __ldg(ranges + s) - a;
+  a = s > 0 ? ld_global(ranges + s - 1) : 0;
+  n = ld_global(ranges + s) - a;
 }
 
 __global__ void __launch_bounds__(kPlanThreads)
-group_pairs_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order,
-                   const int32_t* __restrict__ ranges, int32_t* __restrict__ pairs_out) {
+group_pairs_kernel(int64_t ns, int64_t groups, const int32_t* order,
+                   const int32_t* ranges, int32_t* __restrict__ pairs_out) {
   chain_enter();
   const int64_t g = (int64_t)blockIdx.x * kPlanThreads + threadIdx.x;
   if (g >= groups) return;
@@ -68,7 +68,7 @@ group_pairs_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
     const int64_t v = g * kG + q;
     if (v < ns) {
       int a, n;
-      sample_range(ranges, order ? __ldg(order + v) : v, a, n);
+      sample_range(ranges, order ? ld_global(order + v) : v, a, n);
       total += n;
     }
   }
@@ -96,9 +96,9 @@ __device__ __forceinline__ int lower_bound(const int32_t* l, int n, int x) {
 // the number of first elements with a smaller id, counted list by list with one
 // binary search each and a running count of the first flags.
 __global__ void __launch_bounds__(kPlanThreads)
-group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order,
-                   const int32_t* __restrict__ ranges, const int2* __restrict__ nb_sorted,
-                   const int2* __restrict__ nb_ids, const int32_t* __restrict__ group_begin,
+group_merge_kernel(int64_t ns, int64_t groups, const int32_t* order,
+                   const int32_t* ranges, const int2* nb_sorted,
+                   const int2* nb_ids, const int32_t* group_begin,
                    int32_t* __restrict__ group_rows, int32_t* __restrict__ rows_id,
                    int4* __restrict__ rows_pair) {
   chain_enter(groups, (int64_t)gridDim.x * kPlanWarps);
@@ -114,13 +114,13 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
     int a0 = 0, a1 = 0, a2 = 0, a3 = 0, n0 = 0, n1 = 0, n2 = 0, n3 = 0;
     {
       const int64_t v = g * kG;
-      if (v < ns) sample_range(ranges, order ? __ldg(order + v) : v, a0, n0);
-      if (v + 1 < ns) sample_range(ranges, order ? __ldg(order + v + 1) : v + 1, a1, n1);
-      if (v + 2 < ns) sample_range(ranges, order ? __ldg(order + v + 2) : v + 2, a2, n2);
-      if (v + 3 < ns) sample_range(ranges, order ? __ldg(order + v + 3) : v + 3, a3, n3);
+      if (v < ns) sample_range(ranges, order ? ld_global(order + v) : v, a0, n0);
+      if (v + 1 < ns) sample_range(ranges, order ? ld_global(order + v + 1) : v + 1, a1, n1);
+      if (v + 2 < ns) sample_range(ranges, order ? ld_global(order + v + 2) : v + 2, a2, n2);
+      if (v + 3 < ns) sample_range(ranges, order ? ld_global(order + v + 3) : v + 3, a3, n3);
     }
     const int o1 = n0, o2 = o1 + n1, o3 = o2 + n2, total = o3 + n3;
-    const int base = __ldg(group_begin + g);
+    const int base = ld_global(group_begin + g);
     // element e of the concatenation -> (slot q, position i, pair index m)
     auto locate = [&](int e, int& q, int& i, int& m) {
       q = (e >= o1) + (e >= o2) + (e >= o3);
@@ -137,7 +137,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
       const int a = q == 0 ? a0 : q == 1 ? a1 : q == 2 ? a2 : a3;
       const int n = q == 0 ? n0 : q == 1 ? n1 : q == 2 ? n2 : n3;
       if (n > 0) {
-        const int x = __ldg(&nb_sorted[lane < 4 ? a : a + n - 1].x);
+        const int x = ld_global(&nb_sorted[lane < 4 ? a : a + n - 1].x);
         lo = x; hi = x;
       }
     }
@@ -157,7 +157,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
       for (int e = lane; e < total; e += 32) {
         int q, i, m;
         locate(e, q, i, m);
-        const int x = __ldg(&nb_sorted[m].x) - lo;
+        const int x = ld_global(&nb_sorted[m].x) - lo;
         atomicOr(&bits[x >> 5], 1u << (x & 31));
       }
       __syncwarp();
@@ -182,9 +182,9 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
       for (int e = lane; e < total; e += 32) {
         int q, i, m;
         locate(e, q, i, m);
-        const int x = __ldg(&nb_sorted[m].x) - lo;
+        const int x = ld_global(&nb_sorted[m].x) - lo;
         const int rank = wpre[x >> 5] + __popc(bits[x >> 5] & ((1u << (x & 31)) - 1u));
-        rows_id[base + rank] = __ldg(&nb_ids[m].x);   // every pair of a row holds the same id
+        rows_id[base + rank] = ld_global(&nb_ids[m].x);   // every pair of a row holds the same id
         reinterpret_cast<int32_t*>(rows_pair + base + rank)[q] = m;
       }
       if (lane == 0) group_rows[g] = rows;
@@ -196,7 +196,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
       for (int e = lane; e < total; e += 32) {
         int q, i, m;
         locate(e, q, i, m);
-        rows_id[base + e] = __ldg(&nb_ids[m].x);
+        rows_id[base + e] = ld_global(&nb_ids[m].x);
         rows_pair[base + e] = make_int4(q == 0 ? m : -1, q == 1 ? m : -1, q == 2 ? m : -1,
                                         q == 3 ? m : -1);
       }
@@ -206,7 +206,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
     for (int e = lane; e < total; e += 32) {
       int q, i, m;
       locate(e, q, i, m);
-      val[e] = __ldg(&nb_sorted[m].x);
+      val[e] = ld_global(&nb_sorted[m].x);
     }
     __syncwarp();
     // first flags and their running count
@@ -241,7 +241,7 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* __restrict__ order
       { const int p = q == 1 ? i : lower_bound(val + o1, n1, x); rank += pre[o1 + p] - pre[o1]; }
       { const int p = q == 2 ? i : lower_bound(val + o2, n2, x); rank += pre[o2 + p] - pre[o2]; }
       { const int p = q == 3 ? i : lower_bound(val + o3, n3, x); rank += pre[o3 + p] - pre[o3]; }
-      if (pre[e + 1] != pre[e]) rows_id[base + rank] = __ldg(&nb_ids[m].x);
+      if (pre[e + 1] != pre[e]) rows_id[base + rank] = ld_global(&nb_ids[m].x);
       reinterpret_cast<int32_t*>(rows_pair + base + rank)[q] = m;
     }
     if (lane == 0) group_rows[g] = rows;

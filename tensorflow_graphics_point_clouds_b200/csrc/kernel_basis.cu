@@ -48,12 +48,12 @@ __device__ __forceinline__ void ld_global_256(const float* p, float* v) {
 }
 
 template <int D>
-__device__ __forceinline__ void pair_diff(const float* __restrict__ p_in,
-                                          const float* __restrict__ p_out, int2 nb,
+__device__ __forceinline__ void pair_diff(const float* p_in,
+                                          const float* p_out, int2 nb,
                                           float inv_radius, float* diff) {
 #pragma unroll
   for (int d = 0; d < D; ++d)
-    diff[d] = (__ldg(p_in + (int64_t)nb.x * D + d) - __ldg(p_out + (int64_t)nb.y * D + d)) * inv_radius;
+    diff[d] = (ld_global(p_in + (int64_t)nb.x * D + d) - ld_global(p_out + (int64_t)nb.y * D + d)) * inv_radius;
 }
 
 // diff and 1 / density of pair m.  pdf_mode 0: density per pair, 1: a table with
@@ -63,30 +63,30 @@ __device__ __forceinline__ void pair_diff(const float* __restrict__ p_in,
 // matters because these kernels are bound by the number of scattered loads a warp
 // issues, not by bytes.
 template <int D>
-__device__ __forceinline__ float pair_inputs(const float* __restrict__ p_in,
-                                             const float* __restrict__ p_out,
-                                             const float* __restrict__ pdf, int2 nb, int64_t m,
+__device__ __forceinline__ float pair_inputs(const float* p_in,
+                                             const float* p_out,
+                                             const float* pdf, int2 nb, int64_t m,
                                              float inv_radius, int pdf_mode, float* diff) {
   if (D == 3 && pdf_mode == 2) {
-    const float4 pp = __ldg(reinterpret_cast<const float4*>(p_in) + nb.x);
+    const float4 pp = ld_global(reinterpret_cast<const float4*>(p_in) + nb.x);
     const float* q = p_out + (int64_t)nb.y * 3;
-    diff[0] = (pp.x - __ldg(q)) * inv_radius;
-    diff[1] = (pp.y - __ldg(q + 1)) * inv_radius;
-    diff[2] = (pp.z - __ldg(q + 2)) * inv_radius;
+    diff[0] = (pp.x - ld_global(q)) * inv_radius;
+    diff[1] = (pp.y - ld_global(q + 1)) * inv_radius;
+    diff[2] = (pp.z - ld_global(q + 2)) * inv_radius;
     return pp.w;
   }
   pair_diff<D>(p_in, p_out, nb, inv_radius, diff);
-  return 1.0f / __ldg(pdf + (pdf_mode ? (int64_t)nb.x : m));
+  return 1.0f / ld_global(pdf + (pdf_mode ? (int64_t)nb.x : m));
 }
 
-__global__ void pack_points_density_kernel(int64_t n, const float* __restrict__ pts,
-                                           const float* __restrict__ pdf,
+__global__ void pack_points_density_kernel(int64_t n, const float* pts,
+                                           const float* pdf,
                                            float4* __restrict__ out) {
   chain_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = make_float4(__ldg(pts + 3 * i), __ldg(pts + 3 * i + 1), __ldg(pts + 3 * i + 2),
-                       1.0f / __ldg(pdf + i));
+  out[i] = make_float4(ld_global(pts + 3 * i), ld_global(pts + 3 * i + 1), ld_global(pts + 3 * i + 2),
+                       1.0f / ld_global(pdf + i));
 }
 
 // Where the weight of dimension d and basis function k lies in [K / hidden, D, hidden]: the
@@ -100,19 +100,19 @@ __device__ __forceinline__ int weight_at(int d, int k, int hidden) {
 // WIDE: rows are 32-byte aligned, 256-bit accesses are allowed.
 template <int D, int K, bool WIDE>
 __global__ void __launch_bounds__(kKbThreads)
-kernel_basis_kernel(int64_t M, const float* __restrict__ p_in, const float* __restrict__ p_out,
-                    const int2* __restrict__ neigh, const float* __restrict__ pdf,
-                    const float* __restrict__ w1, const float* __restrict__ b1, float inv_radius,
+kernel_basis_kernel(int64_t M, const float* p_in, const float* p_out,
+                    const int2* neigh, const float* pdf,
+                    const float* w1, const float* b1, float inv_radius,
                     int act, float alpha, float* __restrict__ basis,
                     __nv_bfloat16* __restrict__ pair, int pdf_by_nbr, int hidden) {
   chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   __shared__ float w_s[D * K + K];
   for (int i = threadIdx.x; i < D * K + K; i += kKbThreads)
-    w_s[i] = i < D * K ? __ldg(w1 + weight_at<D>(i / K, i % K, hidden)) : __ldg(b1 + i - D * K);
+    w_s[i] = i < D * K ? ld_global(w1 + weight_at<D>(i / K, i % K, hidden)) : ld_global(b1 + i - D * K);
   __syncthreads();
   for (int64_t m = (int64_t)blockIdx.x * kKbThreads + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * kKbThreads) {
-    const int2 nb = __ldg(neigh + m);
+    const int2 nb = ld_global(neigh + m);
     float diff[D];
     const float inv_pdf = pair_inputs<D>(p_in, p_out, pdf, nb, m, inv_radius, pdf_by_nbr, diff);
     float* dst = basis + m * K;
@@ -161,22 +161,22 @@ template <int D>
 struct PairLoads { float in[D], out[D], density; };
 
 template <int D>
-__device__ __forceinline__ PairLoads<D> load_pair(const float* __restrict__ p_in,
-                                                  const float* __restrict__ p_out,
-                                                  const float* __restrict__ pdf, int2 nb,
+__device__ __forceinline__ PairLoads<D> load_pair(const float* p_in,
+                                                  const float* p_out,
+                                                  const float* pdf, int2 nb,
                                                   int64_t m, int pdf_mode) {
   PairLoads<D> r;
   if (D == 3 && pdf_mode == 2) {
-    const float4 pp = __ldg(reinterpret_cast<const float4*>(p_in) + nb.x);
+    const float4 pp = ld_global(reinterpret_cast<const float4*>(p_in) + nb.x);
     r.in[0] = pp.x; r.in[1] = pp.y; r.in[D - 1] = pp.z;
     r.density = pp.w;
   } else {
 #pragma unroll
-    for (int d = 0; d < D; ++d) r.in[d] = __ldg(p_in + (int64_t)nb.x * D + d);
-    r.density = __ldg(pdf + (pdf_mode ? (int64_t)nb.x : m));
+    for (int d = 0; d < D; ++d) r.in[d] = ld_global(p_in + (int64_t)nb.x * D + d);
+    r.density = ld_global(pdf + (pdf_mode ? (int64_t)nb.x : m));
   }
 #pragma unroll
-  for (int d = 0; d < D; ++d) r.out[d] = __ldg(p_out + (int64_t)nb.y * D + d);
+  for (int d = 0; d < D; ++d) r.out[d] = ld_global(p_out + (int64_t)nb.y * D + d);
   return r;
 }
 
@@ -187,11 +187,11 @@ __device__ __forceinline__ PairLoads<D> load_pair(const float* __restrict__ p_in
 // 17.8 million pairs, K 16: 446 -> 313 us (1.43 GB: 4.6 TB/s); 250 000 pairs, K 32: 52 -> 24.
 template <int D, int K, bool WIDE>
 __global__ void __launch_bounds__(kKbThreads, 2)
-kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
-                          const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                          const float* __restrict__ pdf, const float* __restrict__ w1,
-                          const float* __restrict__ b1, float inv_radius, int act, float alpha,
-                          const float* __restrict__ dbasis, float* __restrict__ dw1,
+kernel_basis_grads_kernel(int64_t M, const float* p_in,
+                          const float* p_out, const int2* neigh,
+                          const float* pdf, const float* w1,
+                          const float* b1, float inv_radius, int act, float alpha,
+                          const float* dbasis, float* __restrict__ dw1,
                           float* __restrict__ db1, int pdf_by_nbr, int hidden) {
   chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   constexpr int KT = k_tile(D, K);
@@ -207,21 +207,21 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
       if (WIDE) {
         ld_global_256(src + 8 * q, g + 8 * q);
       } else {
-        const float4 g0 = __ldg(reinterpret_cast<const float4*>(src) + 2 * q);
-        const float4 g1 = __ldg(reinterpret_cast<const float4*>(src) + 2 * q + 1);
+        const float4 g0 = ld_global(reinterpret_cast<const float4*>(src) + 2 * q);
+        const float4 g1 = ld_global(reinterpret_cast<const float4*>(src) + 2 * q + 1);
         g[8 * q] = g0.x; g[8 * q + 1] = g0.y; g[8 * q + 2] = g0.z; g[8 * q + 3] = g0.w;
         g[8 * q + 4] = g1.x; g[8 * q + 5] = g1.y; g[8 * q + 6] = g1.z; g[8 * q + 7] = g1.w;
       }
     }
   };
   // (past the end the last pair is loaded again)
-  int2 nb = __ldg(neigh + min(m, M - 1));
-  int2 nb_next = __ldg(neigh + min(m + stride, M - 1));
+  int2 nb = ld_global(neigh + min(m, M - 1));
+  int2 nb_next = ld_global(neigh + min(m + stride, M - 1));
   float g[KT];
   load_row(min(m, M - 1), g);
   PairLoads<D> cur = load_pair<D>(p_in, p_out, pdf, nb, min(m, M - 1), pdf_by_nbr);
   for (int i = threadIdx.x; i < D * K + K; i += kKbThreads)
-    w_s[i] = i < D * K ? __ldg(w1 + weight_at<D>(i / K, i % K, hidden)) : __ldg(b1 + i - D * K);
+    w_s[i] = i < D * K ? ld_global(w1 + weight_at<D>(i / K, i % K, hidden)) : ld_global(b1 + i - D * K);
   for (int i = threadIdx.x; i < (D + 1) * KT; i += kKbThreads) red[i] = 0.0f;
   __syncthreads();
   constexpr int kValues = ((D + 1) * KT + 31) / 32 * 32;
@@ -233,7 +233,7 @@ kernel_basis_grads_kernel(int64_t M, const float* __restrict__ p_in,
     const PairLoads<D> ahead = load_pair<D>(p_in, p_out, pdf, nb_next, next, pdf_by_nbr);
     float g_next[KT];
     load_row(next, g_next);
-    nb_next = __ldg(neigh + min(m + 2 * stride, M - 1));
+    nb_next = ld_global(neigh + min(m + 2 * stride, M - 1));
     float diff[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) diff[d] = (cur.in[d] - cur.out[d]) * inv_radius;
@@ -292,18 +292,18 @@ constexpr int kMaxKernelPoints = 64;
 
 template <int D, int K, bool WIDE>
 __global__ void __launch_bounds__(kKbThreads)
-kp_basis_kernel(int64_t M, int num_kp, const float* __restrict__ p_in,
-                const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                const float* __restrict__ kernel_points, float inv_radius, float sigma,
+kp_basis_kernel(int64_t M, int num_kp, const float* p_in,
+                const float* p_out, const int2* neigh,
+                const float* kernel_points, float inv_radius, float sigma,
                 int interpolation, float* __restrict__ basis) {
   chain_enter(M, (int64_t)gridDim.x * kKbThreads);
   __shared__ float kp_s[kMaxKernelPoints * D];
-  for (int i = threadIdx.x; i < num_kp * D; i += kKbThreads) kp_s[i] = __ldg(kernel_points + i);
+  for (int i = threadIdx.x; i < num_kp * D; i += kKbThreads) kp_s[i] = ld_global(kernel_points + i);
   __syncthreads();
   const float gauss_sigma = sigma / 3.0f;
   for (int64_t m = (int64_t)blockIdx.x * kKbThreads + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * kKbThreads) {
-    const int2 nb = __ldg(neigh + m);
+    const int2 nb = ld_global(neigh + m);
     float diff[D];
     pair_diff<D>(p_in, p_out, nb, inv_radius, diff);
     float* dst = basis + m * K;
@@ -349,24 +349,24 @@ kp_basis_kernel(int64_t M, int num_kp, const float* __restrict__ p_in,
 constexpr int kPdfHidden = 16;
 
 __global__ void __launch_bounds__(kKbThreads)
-pointconv_pdf_kernel(int64_t ns, const int32_t* __restrict__ ranges,
-                     const int2* __restrict__ neigh, const float* __restrict__ pdf, const float* __restrict__ w1,
-                     const float* __restrict__ b1, const float* __restrict__ w2,
-                     const float* __restrict__ b2, float* __restrict__ out) {
+pointconv_pdf_kernel(int64_t ns, const int32_t* ranges,
+                     const int2* neigh, const float* pdf, const float* w1,
+                     const float* b1, const float* w2,
+                     const float* b2, float* __restrict__ out) {
   chain_enter(ns * 32, (int64_t)gridDim.x * kKbThreads);
   __shared__ float par[3 * kPdfHidden + 1];
   for (int i = threadIdx.x; i < 3 * kPdfHidden + 1; i += kKbThreads)
-    par[i] = i < kPdfHidden ? __ldg(w1 + i)
-             : i < 2 * kPdfHidden ? __ldg(b1 + i - kPdfHidden)
-             : i < 3 * kPdfHidden ? __ldg(w2 + i - 2 * kPdfHidden) : __ldg(b2);
+    par[i] = i < kPdfHidden ? ld_global(w1 + i)
+             : i < 2 * kPdfHidden ? ld_global(b1 + i - kPdfHidden)
+             : i < 3 * kPdfHidden ? ld_global(w2 + i - 2 * kPdfHidden) : ld_global(b2);
   __syncthreads();
   const int lane = lane_id();
   const int64_t warps = ((int64_t)gridDim.x * kKbThreads) >> 5;
   for (int64_t s = ((int64_t)blockIdx.x * kKbThreads + threadIdx.x) >> 5; s < ns; s += warps) {
-    const int a = s ? __ldg(ranges + s - 1) : 0;
-    const int e = __ldg(ranges + s);
+    const int a = s ? ld_global(ranges + s - 1) : 0;
+    const int e = ld_global(ranges + s);
     float mx = -INFINITY;
-    auto density = [&](int m) { return __ldg(pdf + (neigh ? __ldg(&neigh[m].x) : m)); };
+    auto density = [&](int m) { return ld_global(pdf + (neigh ? ld_global(&neigh[m].x) : m)); };
     for (int m = a + lane; m < e; m += 32) mx = fmaxf(mx, density(m));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));

@@ -67,11 +67,11 @@ __device__ __forceinline__ void load_params(const MlpShape& s, float* par) {
     const int ho = s.h[l + 1], hp = s.hp[l + 1];
     for (int i = threadIdx.x; i < s.G * s.h[l] * hp; i += blockDim.x) {
       const int r = i / hp, c = i - r * hp;
-      par[s.w_off[l] + i] = c < ho ? __ldg(s.w[l] + r * ho + c) : 0.0f;
+      par[s.w_off[l] + i] = c < ho ? ld_global(s.w[l] + r * ho + c) : 0.0f;
     }
     for (int i = threadIdx.x; i < s.G * hp; i += blockDim.x) {
       const int r = i / hp, c = i - r * hp;
-      par[s.b_off[l] + i] = c < ho ? __ldg(s.b[l] + r * ho + c) : 0.0f;
+      par[s.b_off[l] + i] = c < ho ? ld_global(s.b[l] + r * ho + c) : 0.0f;
     }
   }
 }
@@ -107,18 +107,18 @@ __device__ __forceinline__ void layer8(const MlpShape& s, const float* par, int 
   }
 }
 
-__device__ __forceinline__ void load_diff(const MlpShape& s, int2 nb, const float* __restrict__ p_in,
-                                          const float* __restrict__ p_out, float inv_radius,
+__device__ __forceinline__ void load_diff(const MlpShape& s, int2 nb, const float* p_in,
+                                          const float* p_out, float inv_radius,
                                           float* col, int stride) {
   for (int d = 0; d < s.D; ++d)
-    col[d * stride] = (__ldg(p_in + (int64_t)nb.x * s.D + d) - __ldg(p_out + (int64_t)nb.y * s.D + d)) *
+    col[d * stride] = (ld_global(p_in + (int64_t)nb.x * s.D + d) - ld_global(p_out + (int64_t)nb.y * s.D + d)) *
                       inv_radius;
 }
 
 __global__ void __launch_bounds__(128)
-kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
-                        const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                        const float* __restrict__ pdf, float inv_radius, int act, float alpha,
+kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
+                        const float* p_out, const int2* neigh,
+                        const float* pdf, float inv_radius, int act, float alpha,
                         int pdf_by_nbr, float* __restrict__ basis) {
   chain_enter(M, (int64_t)gridDim.x * blockDim.x);
   extern __shared__ __align__(16) float par[];
@@ -132,9 +132,9 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   const bool quads = hl % 4 == 0 && (uintptr_t)basis % 16 == 0;
   for (int64_t m = (int64_t)blockIdx.x * stride + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * stride) {
-    const int2 nb = __ldg(neigh + m);
+    const int2 nb = ld_global(neigh + m);
     load_diff(s, nb, p_in, p_out, inv_radius, diff, stride);
-    const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+    const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
     for (int g = 0; g < s.G; ++g) {
       const float* in = diff;
       for (int l = 0; l < s.L; ++l) {
@@ -171,10 +171,10 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
 }
 
 __global__ void __launch_bounds__(128)
-kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
-                        const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                        const float* __restrict__ pdf, float inv_radius, int act, float alpha,
-                        int pdf_by_nbr, const float* __restrict__ dbasis,
+kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
+                        const float* p_out, const int2* neigh,
+                        const float* pdf, float inv_radius, int act, float alpha,
+                        int pdf_by_nbr, const float* dbasis,
                         float* __restrict__ dweights, float* __restrict__ dbiases,
                         float* __restrict__ dp_in, float* __restrict__ dp_out,
                         float* __restrict__ dpdf) {
@@ -199,8 +199,8 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
 #pragma unroll
     for (int d = 0; d < TFGPC_MAX_DIMS; ++d) ddiff[d] = 0.0f;
     if (live) {
-      nb = __ldg(neigh + m);
-      inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+      nb = ld_global(neigh + m);
+      inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
       load_diff(s, nb, p_in, p_out, inv_radius, my_units, stride);
     } else {
       for (int d = 0; d < s.D; ++d) my_units[d * stride] = 0.0f;
@@ -229,7 +229,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               if (e < cnt) {
-                const float b = live ? __ldg(gb + e) : 0.0f;
+                const float b = live ? ld_global(gb + e) : 0.0f;
                 grads[(8 * q + e) * stride + threadIdx.x] = b * inv_pdf * act_slope(v[e], act, alpha);
                 if (dpdf) dpdf_m -= b * act_fwd(v[e], act, alpha) * inv_pdf * inv_pdf;
               }
@@ -361,8 +361,8 @@ struct SmallParams {
       const int rows = second ? kH1 : 3, in = s.h[l], out = s.h[l + 1];
       float v = 0.0f;
       if (c < out) {
-        if (r == rows) v = __ldg(s.b[l] + g * out + c);
-        else if (r < in) v = __ldg(s.w[l] + (g * in + r) * out + c);
+        if (r == rows) v = ld_global(s.b[l] + g * out + c);
+        else if (r < in) v = ld_global(s.w[l] + (g * in + r) * out + c);
       }
       p[i] = v;
     }
@@ -380,9 +380,9 @@ __device__ __forceinline__ void set4(float* acc, float4 b) {
 // One pair per thread.
 template <int H2>
 __global__ void __launch_bounds__(256)
-small_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
-                       const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                       const float* __restrict__ pdf, float inv_radius, int act, float alpha,
+small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
+                       const float* p_out, const int2* neigh,
+                       const float* pdf, float inv_radius, int act, float alpha,
                        int pdf_by_nbr, float* __restrict__ basis) {
   chain_enter(M, (int64_t)gridDim.x * 256);
   __shared__ SmallParams<H2> par;
@@ -393,14 +393,14 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
     par.load(s, g, 256);
     __syncthreads();
     for (int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x; m < M; m += (int64_t)gridDim.x * 256) {
-      const int2 nb = __ldg(neigh + m);
-      const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+      const int2 nb = ld_global(neigh + m);
+      const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
       float h[kH1];
 #pragma unroll
       for (int q = 0; q < kH1 / 4; ++q) set4(h + 4 * q, par.b1[q]);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
-        const float x = (__ldg(p_in + (int64_t)nb.x * 3 + d) - __ldg(p_out + (int64_t)nb.y * 3 + d)) *
+        const float x = (ld_global(p_in + (int64_t)nb.x * 3 + d) - ld_global(p_out + (int64_t)nb.y * 3 + d)) *
                         inv_radius;
 #pragma unroll
         for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, x, par.w1[d][q]);
@@ -434,10 +434,10 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
 // blockIdx.y: the MLP.
 template <int H2>
 __global__ void __launch_bounds__(128, 3)
-small_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
-                       const float* __restrict__ p_out, const int2* __restrict__ neigh,
-                       const float* __restrict__ pdf, float inv_radius, int act, float alpha,
-                       int pdf_by_nbr, const float* __restrict__ dbasis,
+small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
+                       const float* p_out, const int2* neigh,
+                       const float* pdf, float inv_radius, int act, float alpha,
+                       int pdf_by_nbr, const float* dbasis,
                        float* __restrict__ dweights, float* __restrict__ dbiases,
                        float* __restrict__ dp_in, float* __restrict__ dp_out,
                        float* __restrict__ dpdf) {
@@ -463,22 +463,22 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* __restrict__ p_in,
   for (int64_t m0 = (int64_t)blockIdx.x * 64 + (threadIdx.x >> 5) * 16; m0 < M; m0 += stride) {
     const int64_t m = m0 + (lane >> 1);
     const bool live = m < M;
-    const int2 nb = __ldg(neigh + (live ? m : M - 1));
+    const int2 nb = ld_global(neigh + (live ? m : M - 1));
     float diff[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      diff[d] = (__ldg(p_in + (int64_t)nb.x * 3 + d) - __ldg(p_out + (int64_t)nb.y * 3 + d)) * inv_radius;
-    const float inv_pdf = 1.0f / __ldg(pdf + (pdf_by_nbr ? (int64_t)nb.x : live ? m : M - 1));
+      diff[d] = (ld_global(p_in + (int64_t)nb.x * 3 + d) - ld_global(p_out + (int64_t)nb.y * 3 + d)) * inv_radius;
+    const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : live ? m : M - 1));
     float up[HJ];
     const float* gb = dbasis + m * k_total + g * hl + half * HJ;
 #pragma unroll
     for (int j = 0; j < HJ; j += 4) {
       if (quads) {
-        const float4 q = live ? __ldg(reinterpret_cast<const float4*>(gb + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 q = live ? ld_global(reinterpret_cast<const float4*>(gb + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
         set4(up + j, q);
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) up[j + e] = live && half * HJ + j + e < hl ? __ldg(gb + j + e) : 0.0f;
+        for (int e = 0; e < 4; ++e) up[j + e] = live && half * HJ + j + e < hl ? ld_global(gb + j + e) : 0.0f;
       }
     }
     // own hidden units, the partner's by a shuffle

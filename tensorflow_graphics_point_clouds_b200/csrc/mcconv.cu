@@ -125,12 +125,12 @@ struct Blocks {
 
 // out[(c * k_src + k), o] = padded[(c * k_dst + k), o]
 __global__ void crop_weights_kernel(int64_t n, int cols, int ld, int k_src, int k_dst,
-                                    const float* __restrict__ padded, float* __restrict__ out) {
+                                    const float* padded, float* __restrict__ out) {
   chain_enter();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t r = i / cols, c = r / k_src;
-  out[i] = __ldg(padded + (c * k_dst + (r - c * k_src)) * ld + (i - r * cols));
+  out[i] = ld_global(padded + (c * k_dst + (r - c * k_src)) * ld + (i - r * cols));
 }
 
 int check_blocks(const char* op, int K, int C, int Cout, const Blocks& b) {

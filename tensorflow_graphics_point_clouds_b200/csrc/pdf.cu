@@ -14,41 +14,41 @@ constexpr int kPdfThreads = 256;
 constexpr float kInvSqrt2Pi = 0.39894228f;  // compute_pdf_kernels.cu.cc:111
 
 template <int D>
-__device__ __forceinline__ void load_bandwidth(int mode, int64_t n, const float* __restrict__ inv_bw,
-                                               const float* __restrict__ inv_r, float* bw, float* ir) {
+__device__ __forceinline__ void load_bandwidth(int mode, int64_t n, const float* inv_bw,
+                                               const float* inv_r, float* bw, float* ir) {
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     // mode 1 uses sqrt(number of points) as the inverse bandwidth
     // (compute_pdf_kernels.cu.cc:47-56, applied with numSamples at :102).
-    bw[d] = mode == 1 ? sqrtf((float)n) : __ldg(inv_bw + d);
-    ir[d] = __ldg(inv_r + d);
+    bw[d] = mode == 1 ? sqrtf((float)n) : ld_global(inv_bw + d);
+    ir[d] = ld_global(inv_r + d);
   }
 }
 
 template <int D>
 __global__ void __launch_bounds__(kPdfThreads)
-compute_pdf_kernel(int mode, int64_t n, int64_t n_bw, const float* __restrict__ centers,
-                   const float* __restrict__ pts,
-                   const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
-                   const float* __restrict__ inv_bw, const float* __restrict__ inv_r,
+compute_pdf_kernel(int mode, int64_t n, int64_t n_bw, const float* centers,
+                   const float* pts,
+                   const int2* neigh, const int32_t* ranges,
+                   const float* inv_bw, const float* inv_r,
                    float* __restrict__ pdf_out) {
   float bw[D], ir[D];
   load_bandwidth<D>(mode, n_bw, inv_bw, inv_r, bw, ir);
   const int lane = lane_id();
   const int64_t warps = ((int64_t)gridDim.x * kPdfThreads) >> 5;
   for (int64_t i = ((int64_t)blockIdx.x * kPdfThreads + threadIdx.x) >> 5; i < n; i += warps) {
-    const int a = i ? __ldg(ranges + i - 1) : 0;
-    const int e = __ldg(ranges + i);
+    const int a = i ? ld_global(ranges + i - 1) : 0;
+    const int e = ld_global(ranges + i);
     float p[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = __ldg(centers + i * D + d);
+    for (int d = 0; d < D; ++d) p[d] = ld_global(centers + i * D + d);
     float acc = 0.0f;
     for (int m = a + lane; m < e; m += 32) {
-      const int j = __ldg(&neigh[m].x);
+      const int j = ld_global(&neigh[m].x);
       float local = 1.0f;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        float t = (__ldg(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
+        float t = (ld_global(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
         local *= bw[d] * expf(t * t * (-0.5f)) * kInvSqrt2Pi;
       }
       acc += local;
@@ -65,29 +65,29 @@ compute_pdf_kernel(int mode, int64_t n, int64_t n_bw, const float* __restrict__ 
 // scattered with fp32 atomics like the reference does.
 template <int D>
 __global__ void __launch_bounds__(kPdfThreads)
-compute_pdf_grads_kernel(int mode, int64_t n, const float* __restrict__ pts,
-                         const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
-                         const float* __restrict__ inv_bw, const float* __restrict__ inv_r,
-                         const float* __restrict__ pdf_grads, float* __restrict__ grads_out) {
+compute_pdf_grads_kernel(int mode, int64_t n, const float* pts,
+                         const int2* neigh, const int32_t* ranges,
+                         const float* inv_bw, const float* inv_r,
+                         const float* pdf_grads, float* __restrict__ grads_out) {
   chain_enter(n * 32, (int64_t)gridDim.x * kPdfThreads);
   float bw[D], ir[D];
   load_bandwidth<D>(mode, n, inv_bw, inv_r, bw, ir);
   const int lane = lane_id();
   const int64_t warps = ((int64_t)gridDim.x * kPdfThreads) >> 5;
   for (int64_t i = ((int64_t)blockIdx.x * kPdfThreads + threadIdx.x) >> 5; i < n; i += warps) {
-    const int a = i ? __ldg(ranges + i - 1) : 0;
-    const int e = __ldg(ranges + i);
-    const float g = __ldg(pdf_grads + i);
+    const int a = i ? ld_global(ranges + i - 1) : 0;
+    const int e = ld_global(ranges + i);
+    const float g = ld_global(pdf_grads + i);
     float p[D], own[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) { p[d] = __ldg(pts + i * D + d); own[d] = 0.0f; }
+    for (int d = 0; d < D; ++d) { p[d] = ld_global(pts + i * D + d); own[d] = 0.0f; }
     for (int m = a + lane; m < e; m += 32) {
-      const int j = __ldg(&neigh[m].x);
+      const int j = ld_global(&neigh[m].x);
       float t[D];
       float local = g;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        t[d] = (__ldg(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
+        t[d] = (ld_global(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
         local *= bw[d] * expf(t[d] * t[d] * (-0.5f)) * kInvSqrt2Pi;
       }
       if (j != i) {  // the self pair has t == 0: it adds +0 and -0
@@ -109,13 +109,13 @@ compute_pdf_grads_kernel(int mode, int64_t n, const float* __restrict__ pts,
 
 // out[neighbor of pair m] += values[m]
 __global__ void __launch_bounds__(kPdfThreads)
-add_by_neighbor_kernel(int64_t M, int64_t n, const int2* __restrict__ neigh,
-                       const float* __restrict__ values, float* __restrict__ out) {
+add_by_neighbor_kernel(int64_t M, int64_t n, const int2* neigh,
+                       const float* values, float* __restrict__ out) {
   chain_enter(M, (int64_t)gridDim.x * kPdfThreads);
   for (int64_t m = (int64_t)blockIdx.x * kPdfThreads + threadIdx.x; m < M;
        m += (int64_t)gridDim.x * kPdfThreads) {
-    const int j = __ldg(&neigh[m].x);
-    if (j >= 0 && j < n) atomicAdd(out + j, __ldg(values + m));
+    const int j = ld_global(&neigh[m].x);
+    if (j >= 0 && j < n) atomicAdd(out + j, ld_global(values + m));
   }
 }
 

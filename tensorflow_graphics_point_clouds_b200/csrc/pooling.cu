@@ -25,8 +25,8 @@ constexpr int kPoolThreads = 256;
 // loads, 22 now.
 template <int VEC>
 __global__ void __launch_bounds__(kPoolThreads)
-neighborhood_pool_kernel(int mode, int C, int64_t ns, const float* __restrict__ features,
-                         const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
+neighborhood_pool_kernel(int mode, int C, int64_t ns, const float* features,
+                         const int2* neigh, const int32_t* ranges,
                          float* __restrict__ out) {
   const int groups = C / VEC;
   const int64_t total = ns * groups;
@@ -35,20 +35,20 @@ neighborhood_pool_kernel(int mode, int C, int64_t ns, const float* __restrict__ 
        i += (int64_t)gridDim.x * kPoolThreads) {
     const int64_t s = i / groups;
     const int c = (int)(i - s * groups) * VEC;
-    const int a = s ? __ldg(ranges + s - 1) : 0;
-    const int e = __ldg(ranges + s);
+    const int a = s ? ld_global(ranges + s - 1) : 0;
+    const int e = ld_global(ranges + s);
     float acc[VEC];
 #pragma unroll
     for (int k = 0; k < VEC; ++k) acc[k] = mode == 0 ? -FLT_MAX : 0.0f;
 #pragma unroll 4
     for (int m = a; m < e; ++m) {
-      const float* row = features + (int64_t)__ldg(&neigh[m].x) * C + c;
+      const float* row = features + (int64_t)ld_global(&neigh[m].x) * C + c;
       float v[VEC];
       if (VEC == 4) {
-        const float4 f = __ldg(reinterpret_cast<const float4*>(row));
+        const float4 f = ld_global(reinterpret_cast<const float4*>(row));
         v[0] = f.x; v[VEC > 1] = f.y; v[VEC > 1 ? 2 : 0] = f.z; v[VEC - 1] = f.w;
       } else {
-        v[0] = __ldg(row);
+        v[0] = ld_global(row);
       }
 #pragma unroll
       for (int k = 0; k < VEC; ++k) acc[k] = mode == 0 ? fmaxf(acc[k], v[k]) : acc[k] + v[k];
@@ -89,7 +89,7 @@ constexpr int kPoolRun = 16;
 
 __global__ void __launch_bounds__(kPoolThreads)
 global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
-                   const float* __restrict__ features, const int32_t* __restrict__ batch_ids,
+                   const float* features, const int32_t* batch_ids,
                    float* out, float* counts) {
   const int64_t total = (n + kPoolRun - 1) / kPoolRun * C;
   chain_enter(total, (int64_t)gridDim.x * kPoolThreads);
@@ -102,8 +102,8 @@ global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
 #pragma unroll
     for (int k = 0; k < kPoolRun; ++k) {
       const int64_t p = run * kPoolRun + k;
-      b[k] = p < n ? __ldg(batch_ids + p) : -1;
-      v[k] = p < n ? __ldg(features + p * C + c) : 0.0f;
+      b[k] = p < n ? ld_global(batch_ids + p) : -1;
+      v[k] = p < n ? ld_global(features + p * C + c) : 0.0f;
     }
     unsigned top = 0u;
     float sum = 0.0f, count = 0.0f;
@@ -128,7 +128,7 @@ global_pool_kernel(int mode, int C, int64_t n, int64_t batch_size,
 }
 
 __global__ void pool_finish_kernel(int mode, int C, int64_t n, float* out,
-                                   const float* __restrict__ counts) {
+                                   const float* counts) {
   chain_enter();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -140,22 +140,22 @@ __global__ void pool_finish_kernel(int mode, int C, int64_t n, float* out,
   }
 }
 
-__global__ void add_bias_kernel(int64_t n, int C, float* x, const float* __restrict__ bias) {
+__global__ void add_bias_kernel(int64_t n, int C, float* x, const float* bias) {
   chain_enter();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n * C) x[i] += __ldg(bias + (i % C));
+  if (i < n * C) x[i] += ld_global(bias + (i % C));
 }
 
 // x = act(x * scale + bias): inference batch normalisation with stored
 // statistics folded into scale and bias, followed by the activation
 // (modelnet40_small.py:236-243).  act 0: none, 1: leaky ReLU with slope alpha.
 __global__ void scale_bias_act_kernel(int64_t total, int C, float* x, float scale,
-                                      const float* __restrict__ bias, int act, float alpha) {
+                                      const float* bias, int act, float alpha) {
   chain_enter(total, (int64_t)gridDim.x * blockDim.x);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
     float v = x[i] * scale;
-    if (bias) v += __ldg(bias + (i % C));
+    if (bias) v += ld_global(bias + (i % C));
     if (act == 1) v = v > 0.0f ? v : v * alpha;
     x[i] = v;
   }

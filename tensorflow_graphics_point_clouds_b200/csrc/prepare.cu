@@ -26,7 +26,7 @@ __device__ __forceinline__ void split_block(const SplitJob& j, unsigned block) {
   const int c = (int)(i - r * octets) * kSplitPer;
   int64_t src = r;
   if (j.order) {
-    src = __ldg(j.order + r);
+    src = ld_global(j.order + r);
   } else if (j.k_src != j.k_dst) {
     const unsigned ch = r / (unsigned)j.k_dst;
     const int k = (int)(r - ch * j.k_dst);
@@ -41,14 +41,14 @@ __device__ __forceinline__ void split_block(const SplitJob& j, unsigned block) {
 #pragma unroll
       for (int e = 0; e < kSplitPer; e += 4) {
         if (c + e < j.cols) {
-          const float4 q = __ldg(reinterpret_cast<const float4*>(p + e));
+          const float4 q = ld_global(reinterpret_cast<const float4*>(p + e));
           v[e] = q.x; v[e + 1] = q.y; v[e + 2] = q.z; v[e + 3] = q.w;
         }
       }
     } else {
 #pragma unroll
       for (int e = 0; e < kSplitPer; ++e)
-        if (c + e < j.cols) v[e] = __ldg(p + e);
+        if (c + e < j.cols) v[e] = ld_global(p + e);
     }
   }
   uint4 h, m;

@@ -35,12 +35,12 @@ __device__ __forceinline__ int64_t block_sum(int64_t v, int64_t* smem) {
 __device__ __forceinline__ int64_t elems_of(const ScanSize& s) {
   if (!s.num_cells) return s.n;
   int64_t t = s.batch_size;
-  for (int d = 0; d < s.dims; ++d) t *= __ldg(s.num_cells + d);
+  for (int d = 0; d < s.dims; ++d) t *= ld_global(s.num_cells + d);
   return t + 3;
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-scan_reduce_kernel(const int32_t* __restrict__ in, ScanSize size, int64_t* __restrict__ tile_sums) {
+scan_reduce_kernel(const int32_t* in, ScanSize size, int64_t* __restrict__ tile_sums) {
   chain_enter();
   __shared__ int64_t smem[32];
   const int64_t n = elems_of(size);
@@ -91,8 +91,8 @@ scan_sums_kernel(ScanSize size, int64_t* tile_sums) {
 // last tile's block also delivers the report.
 template <int THREADS, int ITEMS, bool EXCLUSIVE>
 __global__ void __launch_bounds__(THREADS)
-scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, ScanSize size,
-                  const int64_t* __restrict__ tile_sums, bool sums_scanned,
+scan_tiles_kernel(const int32_t* in, int32_t* __restrict__ out, ScanSize size,
+                  const int64_t* tile_sums, bool sums_scanned,
                   int64_t* __restrict__ total, ScanReport rep) {
   chain_enter();
   constexpr int kTile = THREADS * ITEMS;
@@ -103,9 +103,9 @@ scan_tiles_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, Sca
   if (tile0 >= n) return;
   int64_t before = 0;
   if (sums_scanned) {
-    before = __ldg(tile_sums + blockIdx.x);
+    before = ld_global(tile_sums + blockIdx.x);
   } else if (blockIdx.x > 0) {
-    for (int64_t t = threadIdx.x; t < blockIdx.x; t += THREADS) before += __ldg(tile_sums + t);
+    for (int64_t t = threadIdx.x; t < blockIdx.x; t += THREADS) before += ld_global(tile_sums + t);
     before = block_sum<THREADS>(before, smem);
   }
   // coalesced in, through shared memory to runs of ITEMS per thread and back
@@ -177,7 +177,7 @@ constexpr int kDirectThreads = 512;
 constexpr int kDirectTile = 4 * kDirectThreads;
 
 __global__ void __launch_bounds__(kDirectThreads)
-scan_direct_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n,
+scan_direct_kernel(const int32_t* in, int32_t* __restrict__ out, int64_t n,
                    int64_t* __restrict__ total, ScanReport rep) {
   chain_enter();
   constexpr int kWarps = kDirectThreads / 32;
@@ -187,17 +187,17 @@ scan_direct_kernel(const int32_t* __restrict__ in, int32_t* __restrict__ out, in
   int64_t before = 0;
 #pragma unroll 8
   for (int i = threadIdx.x; i < (int)(tile0 / 4); i += kDirectThreads) {
-    const int4 v = __ldg(in4 + i);
+    const int4 v = ld_global(in4 + i);
     before += ((int64_t)v.x + v.y) + ((int64_t)v.z + v.w);
   }
   const int64_t at = tile0 + 4 * threadIdx.x;
   int v[4];
   if (at + 4 <= n) {
-    const int4 q = __ldg(in4 + at / 4);
+    const int4 q = ld_global(in4 + at / 4);
     v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
   } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = at + e < n ? __ldg(in + at + e) : 0;
+    for (int e = 0; e < 4; ++e) v[e] = at + e < n ? ld_global(in + at + e) : 0;
   }
   const int64_t own = ((int64_t)v[0] + v[1]) + ((int64_t)v[2] + v[3]);
   const int lane = lane_id(), w = threadIdx.x >> 5;

@@ -74,7 +74,7 @@ constexpr size_t kPageBytes = 4096;
 struct Mailbox { void* host; void* dev; cudaEvent_t mark; };
 thread_local Mailbox g_mail[64] = {};
 
-__global__ void mailbox_kernel(const uint32_t* __restrict__ src, uint32_t* dst, int words) {
+__global__ void mailbox_kernel(const uint32_t* src, uint32_t* dst, int words) {
   chain_enter();
   for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
   __threadfence_system();
