@@ -11,6 +11,7 @@
 // Backward: dpre = dbasis / pdf * act'(pre); dw1[d, k] = sum_m diff_d * dpre_k,
 // db1[k] = sum_m dpre_k, accumulated in registers over a grid-stride loop,
 // reduced through shuffles and shared memory, one atomic per block and value.
+#include "activation.cuh"
 #include "basis_proj.cuh"
 #include "prepare.cuh"
 
@@ -21,16 +22,6 @@ constexpr int kKbThreads = 256;
 // Basis functions handled per thread in the backward pass: (D + 1) accumulators each.
 __host__ __device__ constexpr int k_tile(int D, int K) {
   return D <= 3 && K >= 16 ? 16 : 8;
-}
-
-__device__ __forceinline__ float act_fwd(float x, int act, float alpha) {
-  if (act == 1) return x > 0.0f ? x : expm1f(x);       // ELU
-  return x > 0.0f ? x : x * alpha;                      // leaky ReLU (alpha 0: ReLU)
-}
-
-__device__ __forceinline__ float act_bwd(float x, int act, float alpha) {
-  if (act == 1) return x > 0.0f ? 1.0f : expf(x);
-  return x > 0.0f ? 1.0f : alpha;
 }
 
 // 256-bit accesses to global memory (sm_100): a thread that owns a 64-byte row
@@ -126,8 +117,11 @@ kernel_basis_kernel(int64_t M, const float* p_in, const float* p_out,
         float pre = w_s[D * K + k];
 #pragma unroll
         for (int d = 0; d < D; ++d) pre = fmaf(diff[d], w_s[d * K + k], pre);
-        v[i] = act_fwd(pre, act, alpha) * inv_pdf;
+        v[i] = pre;
       }
+      activate<8>(v, act, alpha);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] *= inv_pdf;
       if (!basis) {
       } else if (WIDE) {
         st_global_256(dst + 8 * q, v);
@@ -239,14 +233,22 @@ kernel_basis_grads_kernel(int64_t M, const float* p_in,
     for (int d = 0; d < D; ++d) diff[d] = (cur.in[d] - cur.out[d]) * inv_radius;
     const float inv_pdf = D == 3 && pdf_by_nbr == 2 ? cur.density : 1.0f / cur.density;
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-      float pre = w_s[D * K + k0 + k];
+    for (int k = 0; k < KT; k += 4) {
+      float pre[4], slope[4];
 #pragma unroll
-      for (int d = 0; d < D; ++d) pre = fmaf(diff[d], w_s[d * K + k0 + k], pre);
-      const float dpre = g[k] * inv_pdf * act_bwd(pre, act, alpha);
-      acc[D * KT + k] += dpre;
+      for (int e = 0; e < 4; ++e) {
+        pre[e] = w_s[D * K + k0 + k + e];
 #pragma unroll
-      for (int d = 0; d < D; ++d) acc[d * KT + k] = fmaf(diff[d], dpre, acc[d * KT + k]);
+        for (int d = 0; d < D; ++d) pre[e] = fmaf(diff[d], w_s[d * K + k0 + k + e], pre[e]);
+      }
+      slopes<4>(pre, slope, act, alpha);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float dpre = g[k + e] * inv_pdf * slope[e];
+        acc[D * KT + k + e] += dpre;
+#pragma unroll
+        for (int d = 0; d < D; ++d) acc[d * KT + k + e] = fmaf(diff[d], dpre, acc[d * KT + k + e]);
+      }
     }
     cur = ahead;
 #pragma unroll

@@ -25,6 +25,7 @@
 //     points_out, by atomics;
 //   * the gradient of the density, d_pdf[m] = -sum_k dbasis[m,k] basis[m,k] / pdf[m],
 //     which the caller carries on through ComputePdfPtGrads.
+#include "activation.cuh"
 #include "prepare.cuh"
 
 namespace tfgpc {
@@ -49,18 +50,6 @@ struct MlpShape {
   const float* w[kMaxLayers];  // [G][h[l-1]][h[l]]
   const float* b[kMaxLayers];  // [G][h[l]]
 };
-
-__device__ __forceinline__ float act_fwd(float x, int act, float alpha) {
-  if (act == 1) return x > 0.0f ? x : expm1f(x);
-  return x > 0.0f ? x : x * alpha;
-}
-
-// Slope at x.  (From the activation's value it would be wrong for a negative alpha, whose
-// values below zero are positive, and value + 1 loses the digits of ELU's exp(x).)
-__device__ __forceinline__ float act_slope(float x, int act, float alpha) {
-  if (x > 0.0f) return 1.0f;
-  return act == 1 ? expf(x) : alpha;
-}
 
 __device__ __forceinline__ void load_params(const MlpShape& s, float* par) {
   for (int l = 0; l < s.L; ++l) {
@@ -145,8 +134,7 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
           float acc[8];
           layer8(s, par, l, g, q, in, stride, acc);
           const int cnt = min(8, s.h[l + 1] - 8 * q);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[e] = act_fwd(acc[e], act, alpha);
+          activate<8>(acc, act, alpha);
           if (!last) {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
@@ -215,12 +203,15 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
           float v[8];
           layer8(s, par, l, g, q, my_units + row * stride, stride, v);
           const int cnt = min(8, ho - 8 * q);
+          float slope[8];
+          slopes<8>(v, slope, act, alpha);
+          if (!last || dpdf) activate<8>(v, act, alpha);
           if (!last) {
 #pragma unroll
             for (int e = 0; e < 8; ++e)
               if (e < cnt) {
-                my_units[(next + 8 * q + e) * stride] = act_fwd(v[e], act, alpha);
-                my_units[(next + ho + 8 * q + e) * stride] = act_slope(v[e], act, alpha);
+                my_units[(next + 8 * q + e) * stride] = v[e];
+                my_units[(next + ho + 8 * q + e) * stride] = slope[e];
               }
           } else {
             // gradient of the last layer's pre-activations: dbasis / pdf * slope; the
@@ -230,8 +221,8 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
             for (int e = 0; e < 8; ++e)
               if (e < cnt) {
                 const float b = live ? ld_global(gb + e) : 0.0f;
-                grads[(8 * q + e) * stride + threadIdx.x] = b * inv_pdf * act_slope(v[e], act, alpha);
-                if (dpdf) dpdf_m -= b * act_fwd(v[e], act, alpha) * inv_pdf * inv_pdf;
+                grads[(8 * q + e) * stride + threadIdx.x] = b * inv_pdf * slope[e];
+                if (dpdf) dpdf_m -= b * v[e] * inv_pdf * inv_pdf;
               }
           }
         }
@@ -339,8 +330,8 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
 //
 // The layers' usual sizes fit registers: no activation passes through shared memory, which
 // bounded the general kernels (355 000 pairs, ELU, 8-16: forward 34 us and 78 warp
-// instructions per pair, gradients 131 and 224; now 25 and 95 us).  Units are padded to H1 = 8 and H2 = 8 or
-// 16 with zero weights: a padded unit is zero, and nothing comes back through it.
+// instructions per pair, gradients 131 and 224; now 24 and 81 us).  Units are padded to
+// H1 = 8 and H2 = 8 or 16 with zero weights: a padded unit is zero, and nothing comes back through it.
 constexpr int kH1 = 8;
 
 bool small_mlp(const MlpShape& s) {
@@ -379,7 +370,7 @@ __device__ __forceinline__ void set4(float* acc, float4 b) {
 
 // One pair per thread.
 template <int H2>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
                        const float* p_out, const int2* neigh,
                        const float* pdf, float inv_radius, int act, float alpha,
@@ -393,6 +384,9 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
     par.load(s, g, 256);
     __syncthreads();
     for (int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x; m < M; m += (int64_t)gridDim.x * 256) {
+      // the weights are read anew for each pair: kept over the loop they take 174 registers, and
+      // the few warps left wait out the gathers (355 000 pairs: 56 us)
+      asm volatile("" ::: "memory");
       const int2 nb = ld_global(neigh + m);
       const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
       float h[kH1];
@@ -405,8 +399,7 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
 #pragma unroll
         for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, x, par.w1[d][q]);
       }
-#pragma unroll
-      for (int i = 0; i < kH1; ++i) h[i] = act_fwd(h[i], act, alpha);
+      activate<kH1>(h, act, alpha);
       float* dst = basis + m * k_total + g * hl;
 #pragma unroll
       for (int q = 0; q < H2 / 4; ++q) {
@@ -414,8 +407,9 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
         set4(v, par.b2[q]);
 #pragma unroll
         for (int i = 0; i < kH1; ++i) fma4(v, h[i], par.w2[i][q]);
+        activate<4>(v, act, alpha);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = act_fwd(v[e], act, alpha) * inv_pdf;
+        for (int e = 0; e < 4; ++e) v[e] *= inv_pdf;
         if (quads) {
           if (4 * q < hl) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
         } else {
@@ -486,10 +480,10 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
     set4(own, par.b1[half]);
 #pragma unroll
     for (int d = 0; d < 3; ++d) fma4(own, diff[d], par.w1[d][half]);
+    slopes<HI>(own, slope1, act, alpha);
+    activate<HI>(own, act, alpha);
 #pragma unroll
     for (int i = 0; i < HI; ++i) {
-      slope1[i] = act_slope(own[i], act, alpha);
-      own[i] = act_fwd(own[i], act, alpha);
       const float other = __shfl_xor_sync(0xffffffffu, own[i], 1);
       a1[i] = half ? other : own[i];
       a1[HI + i] = half ? own[i] : other;
@@ -504,11 +498,14 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
 #pragma unroll
       for (int i = 0; i < kH1; ++i) fma4(v, a1[i], par.w2[i][half * (HJ / 4) + q]);
       // d/dpre of the last layer; the density's own gradient: basis = a / pdf -> -a / pdf^2
+      float slope[4];
+      slopes<4>(v, slope, act, alpha);
+      if (dpdf) activate<4>(v, act, alpha);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float b = up[4 * q + e];
-        if (dpdf) dpdf_m -= b * act_fwd(v[e], act, alpha) * inv_pdf * inv_pdf;
-        v[e] = b * inv_pdf * act_slope(v[e], act, alpha);
+        if (dpdf) dpdf_m -= b * v[e] * inv_pdf * inv_pdf;
+        v[e] = b * inv_pdf * slope[e];
         acc[kB2 + 4 * q + e] += v[e];
       }
 #pragma unroll
