@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 
 #include "cell_grid.cuh"
+#include "prepare.cuh"
 
 namespace tfgpc {
 namespace {
@@ -428,6 +429,7 @@ struct ClusterBuild {
   tfgpc_cell_grid g;
   int32_t *arrival, *members, *crowded, *page;
   bool place;
+  AlsoClear also;
 };
 
 template <int D>
@@ -445,6 +447,7 @@ grid_cluster_kernel(ClusterBuild a) {
   const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
   const int n = (int)a.n, boxes = a.batch_size * D;
   const int stride = ranks * kClusterThreads, first = rank * kClusterThreads + tid;
+  for (int64_t i = first; i < a.also.words; i += stride) a.also.p[i] = 0u;
   // ---- boxes of this block's points
   for (int i = tid; i < boxes; i += kClusterThreads) box[0][i] = box[1][i] = 0xffffffffu;
   if (tid < D) asked[tid] = 1;
@@ -716,7 +719,8 @@ CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch
 
 int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                     const int32_t* batch_ids, const float* cell_sizes,
-                    const int32_t* num_cells_in, const CellGridWs& w, int32_t* page) {
+                    const int32_t* num_cells_in, const CellGridWs& w, int32_t* page,
+                    AlsoClear also) {
   const int64_t n = g.n;
   const int D = g.D, B = (int)g.batch_size;
   const int64_t cells = table_cells(D, B, g.max_cells);
@@ -727,7 +731,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
       (int64_t)B * D <= kClusterBoxes) {
     ProfScope prof(st, "grid_cluster");
     const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.arrival, w.members,
-                         w.crowded, page, n <= kClusterPlacePoints};
+                         w.crowded, page, n <= kClusterPlacePoints, also};
     int rc = TFGPC_OK;
     TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a));
     if (rc) return rc;
@@ -749,7 +753,11 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   }
   {
     ProfScope prof(st, "compute_keys");
-    TFGPC_CUDA(cudaMemsetAsync(g.cell_start, 0, (size_t)(cells + 3) * 4, st));
+    Prepare jobs;
+    jobs.zero(g.cell_start, (size_t)(cells + 3) * 4);
+    jobs.zero(also.p, (size_t)also.words * 4);
+    int rc = prepare(st, jobs);
+    if (rc) return rc;
     TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0,
         keys_histogram_kernel<kD>, n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells,
         g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded, cells)));

@@ -26,10 +26,14 @@ struct CellGridWs {
 CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch_size,
                            int max_cells);
 
+// Words that a build clears along the way, for what follows it.
+struct AlsoClear { uint32_t* p = nullptr; int64_t words = 0; };
+
 // Enqueues the build; the cell counts go to words 0 .. kReportTotal of `page`.
 int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                     const int32_t* batch_ids, const float* cell_sizes,
-                    const int32_t* num_cells_in, const CellGridWs& w, int32_t* page);
+                    const int32_t* num_cells_in, const CellGridWs& w, int32_t* page,
+                    AlsoClear also = AlsoClear());
 
 // Argument check of every entry on a built grid (cell_search.cu).
 int check_cell_grid(const char* op, const tfgpc_cell_grid* g);

@@ -530,9 +530,15 @@ size_t sample_ws_bytes(int64_t n) {
   return align_up((size_t)n + kHeadBytes, 256) + align_up((size_t)kMaxBlocks * 4, 256);
 }
 
+// What has to be zero before the kernel starts: barrier words, and the points' states.
+size_t clear_bytes(int64_t n, int mode) {
+  return align_up(mode == 0 ? (size_t)n + kHeadBytes : kHeadBytes, 4);
+}
+
 // Enqueues the sampling; the number of samples goes to words kReportTotal .. of the page.
 int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const float* inv_radii,
-                 float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page) {
+                 float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page,
+                 bool cleared) {
   const size_t state = align_up((size_t)g.n + kHeadBytes, 256);
   SampleArgs a;
   a.c = view_of(g);
@@ -548,7 +554,7 @@ int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const floa
   a.page = page + kReportTotal;
   a.period_ns = barrier_period_ns(g.n);
   ProfScope prof(st, mode == 0 ? "sampling_poisson" : "sampling_cell_average");
-  TFGPC_CUDA(cudaMemsetAsync(ws, 0, mode == 0 ? (size_t)g.n + kHeadBytes : kHeadBytes, st));
+  if (!cleared) TFGPC_CUDA(cudaMemsetAsync(ws, 0, clear_bytes(g.n, mode), st));
   switch (g.D) {
     case 2: return launch_sample<2>(st, a);
     case 3: return launch_sample<3>(st, a);
@@ -608,7 +614,7 @@ extern "C" int tfgpc_cells_sample(void* stream, const tfgpc_cell_grid* grid, int
   rc = report_page(&page);
   if (rc) return rc;
   rc = sample_async(st, *grid, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
-                    sample_indices_out, ws, (int32_t*)page);
+                    sample_indices_out, ws, (int32_t*)page, false);
   if (rc) return rc;
   return finish_sample(st, *grid, nullptr, num_samples_out);
 }
@@ -639,10 +645,11 @@ extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
   void* page = nullptr;
   rc = report_page(&page);
   if (rc) return rc;
-  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page);
+  const AlsoClear also{(uint32_t*)sample_ws, (int64_t)(clear_bytes(g.n, mode) / 4)};
+  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, num_cells_in, w, (int32_t*)page, also);
   if (rc) return rc;
   rc = sample_async(st, g, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
-                    sample_indices_out, sample_ws, (int32_t*)page);
+                    sample_indices_out, sample_ws, (int32_t*)page, true);
   if (rc) return rc;
   return finish_sample(st, g, num_cells_host_out, num_samples_out);
 }
