@@ -153,9 +153,13 @@ py::tuple kernel_mlp_grads(const Tensor& p_in_, const Tensor& p_out_, const Tens
 
 // [n] sums of values [M] over the pairs of every point (first index)
 Tensor add_by_neighbor(const Tensor& neigh_, const Tensor& values_, int64_t n) {
-  Tensor neigh = i32(neigh_), values = f32(values_);
-  require(neigh.dim() == 2 && neigh.size(1) == 2 && values.numel() == neigh.size(0),
+  on_gpu(neigh_);
+  require(values_.device() == neigh_.device(),
+          "AddByNeighbor expects the values on the device of the neighbor list");
+  require(neigh_.dim() == 2 && neigh_.size(1) == 2 && values_.dim() == 1 &&
+              values_.size(0) == neigh_.size(0),
           "AddByNeighbor expects one value and two indices per pair");
+  Tensor neigh = i32(neigh_), values = f32(values_);
   Tensor out = empty({n}, at::kFloat, values);
   check(tfgpc_add_by_neighbor(stream(), neigh.size(0), ip(neigh), fp(values), n, fpm(out)));
   return out;

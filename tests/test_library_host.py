@@ -119,3 +119,15 @@ def test_list_parts_cover_the_list(part_end, begin, pairs, parts):
   for a, b in zip(ends, ends[1:]):
     assert begin <= a <= b <= end
     assert b == end or share * chunk <= b - a <= (share + 1) * chunk
+
+
+def test_sums_by_neighbor_refuse_host_memory():
+  """Pointers of another device never reach the kernel: raised before any launch."""
+  torch = pytest.importorskip("torch")
+  from tensorflow_graphics_point_clouds_b200 import _lib
+  add = _lib.host().add_by_neighbor
+  pairs, values = torch.zeros((3, 2), dtype=torch.int32), torch.ones(3)
+  with pytest.raises(ValueError, match="GPU only"):
+    add(pairs, values, 4)
+  with pytest.raises(ValueError, match="GPU only"):
+    add(pairs.to("meta"), values, 4)
