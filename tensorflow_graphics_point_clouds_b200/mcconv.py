@@ -203,6 +203,12 @@ def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
                                        bandwidth=bandwidth)
 
 
+def _gets_pdf_from_table(neighborhood):
+  """Whether get_pdf gathers from the table of pdf_by_neighbor_id."""
+  from . import pc
+  return getattr(type(neighborhood), 'get_pdf', None) is pc.Neighborhood.get_pdf
+
+
 class MCConv:
   """Monte-Carlo convolution layer (MCConv.py:36-278) with explicit backward.
 
@@ -461,14 +467,16 @@ class PointConv(_ProjectedConv):
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    neigh = neighborhood
-    if neigh is None:
+    if neighborhood is None and type(self)._neighborhood is _ProjectedConv._neighborhood:
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
-    pdf, table_ids = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0), None
-    if pdf is None:
-      pdf = neigh.get_pdf(bandwidth=bandwidth, mode=0)
     else:
-      table_ids = neigh._original_neigh_ids
+      neigh = self._neighborhood(point_cloud_in, point_cloud_out, radius, neighborhood)
+    # the densities as a table, unless get_pdf is not the library's own
+    pdf, table_ids = None, None
+    if _gets_pdf_from_table(neigh):
+      pdf, table_ids = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0), neigh._original_neigh_ids
+    if pdf is None:
+      pdf, table_ids = neigh.get_pdf(bandwidth=bandwidth, mode=0), None
     scale = pointconv_pdf(pdf, neigh._samples_neigh_ranges, self.pdf_weights[0],
                           self.pdf_biases[0], self.pdf_weights[1], self.pdf_biases[1], table_ids)
     # PointConv.py:272: the kernel input is the point difference itself (radius 1)

@@ -66,3 +66,29 @@ def test_density_transform_by_neighbor():
   ranges = neigh._samples_neigh_ranges
   assert torch.equal(mcconv.pointconv_pdf(table, ranges, *par, ids),
                      mcconv.pointconv_pdf(neigh.get_pdf(), ranges, *par))
+
+
+def test_pointconv_takes_overridden_neighborhoods_and_densities():
+  g = torch.Generator(device=DEV).manual_seed(5)
+  a = cloud(500, 2, 3, g)
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  args = (r(3, 16), r(16), r(16 * 4, 32), (r(1, 16), r(16, 1)), (r(1, 16), r(1, 1)), 4)
+  feat = r(500, 4)
+  seen = []
+
+  class Layer(mcconv.PointConv):
+    def _neighborhood(self, *b):
+      seen.append(b)
+      return super()._neighborhood(*b)
+
+  want = mcconv.PointConv(*args).forward(feat, a, a, 0.2)
+  assert torch.equal(Layer(*args).forward(feat, a, a, 0.2), want) and len(seen) == 1
+
+  class Other(pc.Neighborhood):
+    def get_pdf(self, **kw):
+      seen.append(kw)
+      return super().get_pdf(**kw)
+
+  neigh = Other(pc.Grid(a, 0.2), 0.2, a)
+  out = mcconv.PointConv(*args).forward(feat, a, a, 0.2, neighborhood=neigh)
+  assert torch.equal(out, want) and len(seen) == 2
