@@ -203,10 +203,11 @@ def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
                                        bandwidth=bandwidth)
 
 
-def _gets_pdf_from_table(neighborhood):
-  """Whether get_pdf gathers from the table of pdf_by_neighbor_id."""
-  from . import pc
-  return getattr(type(neighborhood), 'get_pdf', None) is pc.Neighborhood.get_pdf
+def _is_own(obj, name):
+  """Whether the method is the library's: not replaced in a subclass, on the class or on
+  the object."""
+  own = getattr(type(obj), '_library_' + name.lstrip('_'), None)
+  return own is not None and getattr(getattr(obj, name), '__func__', None) is own
 
 
 class MCConv:
@@ -247,13 +248,15 @@ class MCConv:
     from . import pc
     return pc.grid_neighborhood(point_cloud_in, radius, point_cloud_out)
 
+  _library_build_neighborhood = build_neighborhood
+
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
     neigh = neighborhood
     if neigh is None:
-      own = getattr(self.build_neighborhood, '__func__', None) is MCConv.build_neighborhood
-      neigh = (_neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth) if own
-               else self.build_neighborhood(point_cloud_in, point_cloud_out, radius))
+      neigh = (_neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
+               if _is_own(self, 'build_neighborhood') else
+               self.build_neighborhood(point_cloud_in, point_cloud_out, radius))
     # the densities as a per-point table where the neighborhood has them so (it
     # then never forms the per-pair array), else per pair
     pdf = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0)
@@ -397,6 +400,8 @@ class _ProjectedConv:
     from . import pc
     return pc.grid_neighborhood(point_cloud_in, radius, point_cloud_out)
 
+  _library_neighborhood = _neighborhood
+
   def _project(self, basis, features, neigh, weights, ns, keep_for_backward):
     if self._op is None or self._op.ns != ns or self._op.backward_ws != keep_for_backward:
       self._op = ProjectionGemm(self.k_pad, self.cin, self.cout_pad, ns, features.device,
@@ -467,13 +472,13 @@ class PointConv(_ProjectedConv):
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    if neighborhood is None and type(self)._neighborhood is _ProjectedConv._neighborhood:
+    if neighborhood is None and _is_own(self, '_neighborhood'):
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
     else:
       neigh = self._neighborhood(point_cloud_in, point_cloud_out, radius, neighborhood)
     # the densities as a table, unless get_pdf is not the library's own
     pdf, table_ids = None, None
-    if _gets_pdf_from_table(neigh):
+    if _is_own(neigh, 'get_pdf'):
       pdf, table_ids = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0), neigh._original_neigh_ids
     if pdf is None:
       pdf, table_ids = neigh.get_pdf(bandwidth=bandwidth, mode=0), None

@@ -427,6 +427,8 @@ class Neighborhood:
         self._pdf = self._point_pdf[self._neighbors[:, 0].to(torch.int64)]
     return self._pdf
 
+  _library_get_pdf = get_pdf
+
   def pdf_point_grads(self, pdf_grads, bandwidth=0.2, mode=0):
     """Gradient of a loss with respect to the grid's points [N, D] (in their
     original order) through the per-pair densities of get_pdf, given the loss's
