@@ -252,11 +252,12 @@ class MCConv:
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    neigh = neighborhood
-    if neigh is None:
-      neigh = (_neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
-               if _is_own(self, 'build_neighborhood') else
-               self.build_neighborhood(point_cloud_in, point_cloud_out, radius))
+    neigh, packed = neighborhood, None
+    if neigh is None and _is_own(self, 'build_neighborhood'):
+      neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
+      packed = neigh._packed      # (of these points: no other neighborhood's is asked for)
+    elif neigh is None:
+      neigh = self.build_neighborhood(point_cloud_in, point_cloud_out, radius)
     # the densities as a per-point table where the neighborhood has them so (it
     # then never forms the per-pair array), else per pair
     pdf = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0)
@@ -275,7 +276,6 @@ class MCConv:
     # (points, 1 / density) as one 16-byte row per point: one gather per pair
     kb_in, kb_pdf, kb_mode = p_in, pdf, int(by_nbr)
     if one_layer and by_nbr and self.dims == 3:
-      packed = neigh._packed
       kb_in, kb_pdf, kb_mode = pack_points_density(p_in, pdf) if packed is None else packed, None, 2
     if grouped:
       # the basis only as the bf16 pair the tensor-core kernels read

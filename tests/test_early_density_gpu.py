@@ -92,3 +92,17 @@ def test_pointconv_takes_overridden_neighborhoods_and_densities():
   neigh = Other(pc.Grid(a, 0.2), 0.2, a)
   out = mcconv.PointConv(*args).forward(feat, a, a, 0.2, neighborhood=neigh)
   assert torch.equal(out, want) and len(seen) == 2
+
+
+def test_a_neighborhood_given_by_the_caller_brings_no_points():
+  """Its pairs and densities count; the kernel inputs are the points of the clouds given."""
+  g = torch.Generator(device=DEV).manual_seed(6)
+  a = cloud(400, 2, 3, g)
+  moved = pc.PointCloud(a._points * 1.25 + 0.5, a._batch_ids, 2)
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  args, feat = (r(1, 3, 16), r(1, 1, 16), r(1, 64, 32), 4), r(400, 4)
+  outs = []
+  for build in (pc.grid_neighborhood_with_pdf, pc.grid_neighborhood):
+    layer = mcconv.MCConv(*args)
+    outs.append(layer.forward(feat, moved, moved, 0.2, neighborhood=build(a, 0.2, a)))
+  assert torch.equal(*outs)
