@@ -328,12 +328,20 @@ def cell_table_elems(dims, batch_size, max_cells):
 
 def build_cell_grid(points, batch_ids, batch_size, cell_sizes, max_cells, cells=None,
                     inv_radii=None, samples=None, samples_batch_ids=None, samples_are_points=-1,
-                    max_neighs=0, inv_bandwidth=None, pdf_mode=0):
-  """(grid, count of the neighborhood around the samples or None without samples,
-  densities, packed table); the last two, None without inv_bandwidth, as in
-  tfgpc_cell_grid_neighborhood_pdf: at every point in the points' own order.
+                    max_neighs=0):
+  """(grid, count of the neighborhood around the samples or None without samples).
   cells: as in grid_neighborhood_count; samples_are_points 0: samples and their batch
   ids, 1: the points in their own order, 2: the sorted points, -1: no samples."""
+  return _lib.host().build_grid(points, batch_ids, batch_size, cell_sizes, max_cells, cells,
+                                inv_radii, samples_are_points, samples, samples_batch_ids,
+                                max_neighs, None, 0)[:2]
+
+
+def build_cell_grid_with_pdf(points, batch_ids, batch_size, cell_sizes, max_cells, inv_bandwidth,
+                             cells=None, inv_radii=None, samples=None, samples_batch_ids=None,
+                             samples_are_points=-1, max_neighs=0, pdf_mode=0):
+  """The pair of build_cell_grid, the density at every point in the points' own order and,
+  in three dimensions, the packed table (tfgpc_cell_grid_neighborhood_pdf)."""
   return _lib.host().build_grid(points, batch_ids, batch_size, cell_sizes, max_cells, cells,
                                 inv_radii, samples_are_points, samples, samples_batch_ids,
                                 max_neighs, inv_bandwidth, pdf_mode)

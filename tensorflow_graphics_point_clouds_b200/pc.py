@@ -496,10 +496,12 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   samples = dict(samples=None if smp is None else smp._points,
                  samples_batch_ids=None if smp is None else smp._batch_ids,
                  samples_are_points=mode, max_neighs=max_neighbors)
-  inv_bw = _to_dims(bandwidth, d, dev, inverse=True) if with_pdf else None
-  built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells,
-                     inv_radii=_to_dims(radius, d, dev, inverse=True), inv_bandwidth=inv_bw,
-                     pdf_mode=pdf_mode, **samples)
+  build, density = ops.build_cell_grid, {}
+  if with_pdf:
+    build = ops.build_cell_grid_with_pdf
+    density = dict(inv_bandwidth=_to_dims(bandwidth, d, dev, inverse=True), pdf_mode=pdf_mode)
+  built = _cell_grid(pc, sizes, build, cells=cells,
+                     inv_radii=_to_dims(radius, d, dev, inverse=True), **density, **samples)
   grid = object.__new__(Grid)
   grid._cell_sizes = _to_dims(radius, d, dev)
   if built is not None:

@@ -131,3 +131,22 @@ def test_sums_by_neighbor_refuse_host_memory():
     add(pairs, values, 4)
   with pytest.raises(ValueError, match="GPU only"):
     add(pairs.to("meta"), values, 4)
+
+
+def test_build_cell_grid_returns_a_pair(monkeypatch):
+  """(grid, count); with densities there are four values, from an entry of its own."""
+  pytest.importorskip("torch")
+  from tensorflow_graphics_point_clouds_b200 import _lib, custom_ops
+  seen = []
+
+  class Host:
+    @staticmethod
+    def build_grid(*args):
+      seen.append(args)
+      return "grid", "count", "pdf", "packed"
+
+  monkeypatch.setattr(_lib, "host", lambda: Host)
+  grid, count = custom_ops.build_cell_grid("points", "ids", 2, [0.1] * 3, 64, max_neighs=5)
+  assert (grid, count) == ("grid", "count") and seen[0][-3:] == (5, None, 0)
+  both = custom_ops.build_cell_grid_with_pdf("points", "ids", 2, [0.1] * 3, 64, "inv", pdf_mode=1)
+  assert both == ("grid", "count", "pdf", "packed") and seen[1][-3:] == (0, "inv", 1)
