@@ -331,7 +331,9 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
 // The layers' usual sizes fit registers: no activation passes through shared memory, which
 // bounded the general kernels (355 000 pairs, ELU, 8-16: forward 34 us and 78 warp
 // instructions per pair, gradients 131 and 224; now 24 and 81 us).  Units are padded to
-// H1 = 8 and H2 = 8 or 16 with zero weights: a padded unit is zero, and nothing comes back through it.
+// H1 = 8 and H2 = 8 or 16 with zero weights.  A padded unit is zero, and nothing comes back
+// through it, only where its inputs and what reaches it are finite (infinity times its zero
+// weights is no number): it is set to zero.
 constexpr int kH1 = 8;
 
 bool small_mlp(const MlpShape& s) {
@@ -400,6 +402,10 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
         for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, x, par.w1[d][q]);
       }
       activate<kH1>(h, act, alpha);
+      if (s.h[1] < kH1) {
+#pragma unroll
+        for (int i = 0; i < kH1; ++i) h[i] = i < s.h[1] ? h[i] : 0.0f;
+      }
       float* dst = basis + m * k_total + g * hl;
 #pragma unroll
       for (int q = 0; q < H2 / 4; ++q) {
@@ -425,8 +431,11 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
 // Two lanes per pair, each with half of the last layer's units and, of what comes before
 // them, half of the hidden ones: the gradients of all parameters are sums over pairs in
 // (9 H2 + 32) / 2 registers per lane, 88 at H2 = 16, folded over the warp once at the end.
-// blockIdx.y: the MLP.
-template <int H2>
+// blockIdx.y: the MLP.  PADDED: 0 for 8 and H2 units, 1 for fewer in the first layer, 2 for fewer
+// in the last or in both; instances of their own, since what keeps the padding at zero costs a
+// tenth to a fifth (890 000 pairs, leaky ReLU, us without and with: 8-16 58 and 68; two MLPs of
+// 4-8 77 and 87).
+template <int H2, int PADDED>
 __global__ void __launch_bounds__(128, 3)
 small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
                        const float* p_out, const int2* neigh,
@@ -462,7 +471,11 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
 #pragma unroll
     for (int d = 0; d < 3; ++d)
       diff[d] = (ld_global(p_in + (int64_t)nb.x * 3 + d) - ld_global(p_out + (int64_t)nb.y * 3 + d)) * inv_radius;
-    const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : live ? m : M - 1));
+    float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : live ? m : M - 1));
+    if (!live) {      // (a lane without a pair adds zeros)
+      diff[0] = diff[1] = diff[2] = 0.0f;
+      inv_pdf = 0.0f;
+    }
     float up[HJ];
     const float* gb = dbasis + m * k_total + g * hl + half * HJ;
 #pragma unroll
@@ -482,6 +495,10 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
     for (int d = 0; d < 3; ++d) fma4(own, diff[d], par.w1[d][half]);
     slopes<HI>(own, slope1, act, alpha);
     activate<HI>(own, act, alpha);
+    if (PADDED && !(fabsf((diff[0] + diff[1]) + diff[2]) < INFINITY)) {
+#pragma unroll
+      for (int i = 0; i < HI; ++i) own[i] = half * HI + i < h1 ? own[i] : 0.0f;
+    }
 #pragma unroll
     for (int i = 0; i < HI; ++i) {
       const float other = __shfl_xor_sync(0xffffffffu, own[i], 1);
@@ -504,8 +521,9 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float b = up[4 * q + e];
-        if (dpdf) dpdf_m -= b * v[e] * inv_pdf * inv_pdf;
-        v[e] = b * inv_pdf * slope[e];
+        const bool used = PADDED < 2 || half * HJ + 4 * q + e < hl;
+        if (dpdf && used) dpdf_m -= b * v[e] * inv_pdf * inv_pdf;
+        v[e] = used ? b * inv_pdf * slope[e] : 0.0f;
         acc[kB2 + 4 * q + e] += v[e];
       }
 #pragma unroll
@@ -536,6 +554,8 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
       const int who = live ? nb.y : -1;
       const int prev = __shfl_up_sync(0xffffffffu, who, 2);
       const bool head = lane < 2 || prev != who;
+#pragma unroll
+      for (int i = 0; PADDED && i < HI; ++i) g1[i] = half * HI + i < h1 ? g1[i] : 0.0f;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         const float4 w = par.w1[d][half];
@@ -781,8 +801,14 @@ extern "C" int tfgpc_kernel_mlp_grads_layers(
     const unsigned most = max(3u * sm_count() / (unsigned)s.G, 1u);
     dim3 blocks(min(blocks_for(M, 64), most), (unsigned)s.G);
     ProfScope prof(st, "kernel_mlp_grads");
-    TFGPC_CUDA(launch_chained(st, blocks, 128, 0,
-        s.h[2] <= 8 ? small_mlp_grads_kernel<8> : small_mlp_grads_kernel<16>, s, M, points_in,
+    const int padded = s.h[2] % 8 != 0 ? 2 : s.h[1] < kH1 ? 1 : 0;
+    auto kernel = s.h[2] <= 8 ? small_mlp_grads_kernel<8, 0> : small_mlp_grads_kernel<16, 0>;
+    if (padded == 1)
+      kernel = s.h[2] <= 8 ? small_mlp_grads_kernel<8, 1> : small_mlp_grads_kernel<16, 1>;
+    if (padded == 2)
+      kernel = s.h[2] <= 8 ? small_mlp_grads_kernel<8, 2> : small_mlp_grads_kernel<16, 2>;
+    TFGPC_CUDA(launch_chained(st, blocks, 128, 0, kernel,
+        s, M, points_in,
         points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
         basis_grads, dweights_out, dbiases_out, dpoints_in_out, dpoints_out_out, dpdf_out));
     return TFGPC_OK;

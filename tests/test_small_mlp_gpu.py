@@ -51,3 +51,67 @@ def test_against_64_bits(mlps, h1, h2, m, act, points):
   for a, b in zip(flat(grads), want):
     assert a.shape == b.grad.shape
     assert (a.double() - b.grad).norm() <= 1e-4 * b.grad.norm() + 1e-9
+
+
+class Activation(torch.autograd.Function):
+  """ELU (1) or leaky ReLU (0), slopes from the pre-activations: no number stays none."""
+
+  @staticmethod
+  def forward(ctx, x, act):
+    ctx.save_for_backward(x)
+    ctx.act = act
+    return torch.where(x > 0, x, torch.expm1(x) if act else 0.2 * x)
+
+  @staticmethod
+  def backward(ctx, up):
+    x, = ctx.saved_tensors
+    return up * torch.where(x > 0, 1.0, torch.exp(x) if ctx.act else 0.2), None
+
+
+def kinds(t):
+  return torch.stack([t.isnan(), t.isposinf(), t.isneginf()])
+
+
+# what the padded units and the lanes without a pair must keep to themselves: densities of
+# zero, sums that overflow, a point at infinity; in float32, as the kernels work
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("special", ["pdf", "overflow", "point"])
+@pytest.mark.parametrize("mlps,h1,h2,m", [(1, 5, 13, 3), (1, 8, 16, 65), (1, 6, 7, 33), (2, 3, 8, 17)])
+def test_infinities_stay_where_they_arise(mlps, h1, h2, m, special, act):
+  g = torch.Generator(device=DEV).manual_seed(m + act)
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  # (back through a weight of 3e38 what is left depends on the order of the sums)
+  n, points = 20, mlps == 1 and special != "overflow"
+  p_in, p_out, pdf = r(n, 3), r(n, 3), 0.5 + torch.rand(m, generator=g, device=DEV)
+  ws, bs = [r(mlps, 3, h1), r(mlps, h1, h2)], [r(mlps, 1, h1), r(mlps, 1, h2)]
+  pairs = torch.stack([torch.randint(0, n - 1, (m,), generator=g, device=DEV),
+                       torch.sort(torch.randint(0, n, (m,), generator=g, device=DEV)).values], 1).int()
+  if special == "pdf":
+    pdf[-1] = pdf[m // 2] = 0.0
+  elif special == "overflow":
+    p_in[:, 0] = 10.0 * torch.sign(r(n))          # (no pair near the limit)
+    ws[0][0, 0, 0] = 3e38
+  else:
+    pairs[-1, 0] = n - 1
+    p_in[n - 1, 1] = float("inf")
+  up = r(m, mlps * h2)
+  leaf = lambda t: t.clone().requires_grad_(True)
+  i, o, q, w, b = leaf(p_in), leaf(p_out), leaf(pdf), [leaf(t) for t in ws], [leaf(t) for t in bs]
+  diff = (i[pairs[:, 0].long()] - o[pairs[:, 1].long()]) * 2.0
+  outs = []
+  for k in range(mlps):
+    a = diff
+    for x, y in zip(w, b):      # (products one by one: no zeros of a blocked product between them)
+      a = (a[:, :, None] * x[k][None]).sum(1) + y[k]
+      a = Activation.apply(a, act)
+    outs.append(a)
+  ref = torch.cat(outs, 1) / q[:, None]
+  ref.backward(up)
+  got = mcconv.kernel_mlp_basis(p_in, p_out, pairs, pdf, ws, bs, 0.5, act, 0.2)
+  flat = lambda x: [t for y in x for t in (flat(y) if isinstance(y, (list, tuple)) else [y])]
+  grads = flat(mcconv.kernel_mlp_grads(p_in, p_out, pairs, pdf, ws, bs, 0.5, up, act, 0.2,
+                                       point_grads=points))
+  want = [t.grad for t in flat([w, b] + ([i, o, q] if points else []))]
+  assert not ref.isfinite().all() or special != "pdf"
+  for x, y in zip([got] + grads, [ref.detach()] + want):
+    assert torch.equal(kinds(x), kinds(y))
