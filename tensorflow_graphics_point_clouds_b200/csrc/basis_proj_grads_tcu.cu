@@ -158,10 +158,10 @@ basis_proj_grads_tcu_kernel(int64_t ns, int64_t M, int64_t groups,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kMmaWarp) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
-  chain_enter(groups, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_enter(groups, gridDim.x);
   const uint32_t tmem_base = *(volatile uint32_t*)&bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
 

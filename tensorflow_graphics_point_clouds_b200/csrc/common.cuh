@@ -122,6 +122,10 @@ __device__ __forceinline__ T ld_global(const T* p) { return *p; }
 // lives with what is left of the L1 cache, and blocks take their places in another order:
 // 524 288 points, us, 1.3 ms kernels before them: kernel-MLP gradients 347 -> 578, dX product
 // 1560 -> 1752, projection gradients 2380 -> 2527.
+// A kernel with tensor memory calls it behind the barrier that follows its allocation: a
+// successor that may come while a block still waits for its columns could take them first and
+// then wait for that block.  (With the call before the barrier nothing but the size of these
+// kernels' shared memory, 169 KB or more, kept two of them off one SM.)
 __device__ __forceinline__ void chain_enter(int64_t items = 0, int64_t per_turn = 0) {
   if (items <= 8 * per_turn && gridDim.x <= 4096)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

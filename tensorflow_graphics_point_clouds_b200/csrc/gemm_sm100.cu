@@ -143,10 +143,10 @@ gemm_bf16x3_kernel(const __grid_constant__ CUtensorMap tm_a_hi,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) tmem_alloc(smem_u32(&bars->tmem_base), kTmemCols);
-  chain_enter((int64_t)total_tiles * 4, gridDim.x);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_enter((int64_t)total_tiles * 4, gridDim.x);
   const uint32_t tmem_base = *(volatile uint32_t*)&bars->tmem_base;
   volatile int* abort_flag = &bars->abort_flag;
 
