@@ -310,8 +310,8 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
     int per_sm = 1;
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
-        ranges, out, hi, mid, shift));
+    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, out, hi, mid, shift);
+    TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
   if (vec) {
@@ -366,8 +366,9 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M
     int per_sm = 1;
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
     unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
-        ranges, in_grads, dbasis, dfeat, shift));
+    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, in_grads, dbasis,
+                                            dfeat, shift);
+    TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
   if (vec)

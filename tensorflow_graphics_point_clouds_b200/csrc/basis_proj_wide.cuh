@@ -9,6 +9,13 @@
 //   - the feature rows, the only scattered traffic, are fetched U at a time
 //     before any of them is used, which keeps U independent 512-byte row reads
 //     in flight per warp.
+// Both kernels are launched after their predecessor's end and load on the read-only path,
+// like the narrow ones (basis_proj.cu): plain loads stay behind the writes of the sample
+// before and cost registers.  Chained with plain loads and as they are, us, lists of 30:
+// 15 000 samples, gradients, K = 64: C = 24 1035 / 840, C = 64 1932 / 1577, C = 128 3803 / 3070,
+// K = 8, C = 96 134 / 136; forward, K = 64, C = 72 364 / 329.  900 samples, forward, C = 256:
+// K = 8 12.6 / 11.0, K = 16 19.8 / 15.0, K = 64 94 / 68; gradients, K = 32, C = 256 88 / 63.
+// (Chained with plain loads and no early release of the successor: as slow.)
 #pragma once
 
 #include "basis_proj.cuh"
@@ -42,11 +49,11 @@ struct FeatVec<1> {
 // loop its first 32*K floats hold the staged basis rows; afterwards the whole
 // tile stages the warp's output for coalesced stores.
 template <int K>
-__device__ __forceinline__ void stage_basis_chunk(float* tile, const float* basis,
+__device__ __forceinline__ void stage_basis_chunk(float* tile, const float* __restrict__ basis,
                                                   int base, int cnt, int lane) {
   const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)base * K);
   float4* dst = reinterpret_cast<float4*>(tile);
-  for (int i = lane; i < cnt * (K / 4); i += 32) dst[i] = ld_global(src + i);
+  for (int i = lane; i < cnt * (K / 4); i += 32) dst[i] = __ldg(src + i);
 }
 
 // ---- small PTX helpers ---------------------------------------------------------
@@ -104,12 +111,11 @@ __host__ __device__ constexpr int bpw_warp_floats() {
 
 template <int K, int OUT>
 __global__ void __launch_bounds__(kBpwThreads, 2)
-basis_proj_wide_kernel(int C, int64_t ns, const float* basis,
-                       const float* feat, const int2* neigh,
-                       const int32_t* ranges, float* __restrict__ out,
+basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
+                       const float* __restrict__ feat, const int2* __restrict__ neigh,
+                       const int32_t* __restrict__ ranges, float* __restrict__ out,
                        __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
                        int shift) {
-  chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -123,8 +129,8 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* basis,
   float* wtile = tile + R * 32 * kCpl;          // [32 neighbors][K]
   const int64_t warps = ((int64_t)gridDim.x * kBpwThreads) >> 5;
   for (int64_t s = ((int64_t)blockIdx.x * kBpwThreads + threadIdx.x) >> 5; s < ns; s += warps) {
-    const int a = s ? ld_global(ranges + s - 1) : 0;
-    const int e = ld_global(ranges + s);
+    const int a = s ? __ldg(ranges + s - 1) : 0;
+    const int e = __ldg(ranges + s);
     for (int c0 = 0; c0 < C; c0 += kChunk) {
       const int cbase = c0 + lane * kCpl;
       const bool c_ok = cbase < C;  // C is a multiple of CPL on this path
@@ -136,7 +142,7 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* basis,
       for (int base = a; base < e; base += 32) {
         const int cnt = min(32, e - base);
         __syncwarp();
-        const int my_j = lane < cnt ? ld_global(&neigh[base + lane].x) : 0;
+        const int my_j = lane < cnt ? __ldg(&neigh[base + lane].x) : 0;
         stage_basis_chunk<K>(wtile, basis, base, cnt, lane);
         // fill the ring: rows 0 .. R-1 of the chunk (one commit group per row)
 #pragma unroll
@@ -222,12 +228,11 @@ __host__ __device__ constexpr int bpw_grads_warp_floats() {
 
 template <int K>
 __global__ void __launch_bounds__(kBpwThreads, 2)
-basis_proj_grads_wide_kernel(int C, int64_t ns, const float* basis,
-                             const float* feat, const int2* neigh,
-                             const int32_t* ranges,
-                             const float* in_grads, float* __restrict__ dbasis,
+basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
+                             const float* __restrict__ feat, const int2* __restrict__ neigh,
+                             const int32_t* __restrict__ ranges,
+                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
                              float* __restrict__ dfeat, int shift) {
-  chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kChunk = 32 * kCpl;
   constexpr int R = kBpwRing;
@@ -257,12 +262,12 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* basis,
     if (lane & (1 << t)) perm += K >> (t + 1);
   const int permq = perm >> 2;  // in units of 4 values (one 128-bit load)
   for (int64_t s = ((int64_t)blockIdx.x * kBpwThreads + threadIdx.x) >> 5; s < ns; s += warps) {
-    const int a = s ? ld_global(ranges + s - 1) : 0;
-    const int e = ld_global(ranges + s);
+    const int a = s ? __ldg(ranges + s - 1) : 0;
+    const int e = __ldg(ranges + s);
     for (int base = a; base < e; base += 32) {
       const int cnt = min(32, e - base);
       __syncwarp();
-      const int my_j = lane < cnt ? ld_global(&neigh[base + lane].x) : 0;
+      const int my_j = lane < cnt ? __ldg(&neigh[base + lane].x) : 0;
       stage_basis_chunk<K>(wtile, basis, base, cnt, lane);
       for (int i = lane; i < 32 * K; i += 32) dtile[i] = 0.0f;
       for (int c0 = 0; c0 < C; c0 += kChunk) {
@@ -283,7 +288,7 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* basis,
           for (int q = 0; q < K / 4; ++q) {
             const ulonglong2* src = reinterpret_cast<const ulonglong2*>(
                 in_grads + block_offset<K>(s, C, cbase + cc, 4 * (q ^ permq), shift));
-            const ulonglong2 v = c_ok ? ld_global(src) : make_ulonglong2(0ull, 0ull);
+            const ulonglong2 v = c_ok ? __ldg(src) : make_ulonglong2(0ull, 0ull);
             g[cc][2 * q] = v.x; g[cc][2 * q + 1] = v.y;
           }
         }
