@@ -370,37 +370,44 @@ __device__ __forceinline__ void set4(float* acc, float4 b) {
   acc[0] = b.x; acc[1] = b.y; acc[2] = b.z; acc[3] = b.w;
 }
 
-// One pair per thread.
+// One pair per thread, MLP after MLP: its gathers are made once, and its row of the basis is
+// written by one thread.  (With the pairs inside the loop over the MLPs, two of 4-8 on 890 000
+// pairs took 41 us, the general kernel 38; 31 so.)  Up to rows of 32 values: longer ones the
+// general kernel, whose smaller blocks have more of them under way, writes faster (four MLPs of
+// 8-16, leaky ReLU, 890 000 pairs: 164 us here and 133, though 23 and 28 on 160 000).
 template <int H2>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, 5)
 small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
                        const float* p_out, const int2* neigh,
                        const float* pdf, float inv_radius, int act, float alpha,
                        int pdf_by_nbr, float* __restrict__ basis) {
   chain_enter(M, (int64_t)gridDim.x * 256);
-  __shared__ SmallParams<H2> par;
+  extern __shared__ __align__(16) float par_s[];
+  SmallParams<H2>* const par = reinterpret_cast<SmallParams<H2>*>(par_s);
   const int hl = s.h[2], k_total = s.G * hl;
   const bool quads = hl % 4 == 0 && (uintptr_t)basis % 16 == 0;
-  for (int g = 0; g < s.G; ++g) {
-    if (g > 0) __syncthreads();
-    par.load(s, g, 256);
-    __syncthreads();
-    for (int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x; m < M; m += (int64_t)gridDim.x * 256) {
+  for (int g = 0; g < s.G; ++g) par[g].load(s, g, 256);
+  __syncthreads();
+  for (int64_t m = (int64_t)blockIdx.x * 256 + threadIdx.x; m < M; m += (int64_t)gridDim.x * 256) {
+    const int2 nb = ld_global(neigh + m);
+    const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+    float diff[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      diff[d] = (ld_global(p_in + (int64_t)nb.x * 3 + d) - ld_global(p_out + (int64_t)nb.y * 3 + d)) *
+                inv_radius;
+    for (int g = 0; g < s.G; ++g) {
       // the weights are read anew for each pair: kept over the loop they take 174 registers, and
       // the few warps left wait out the gathers (355 000 pairs: 56 us)
       asm volatile("" ::: "memory");
-      const int2 nb = ld_global(neigh + m);
-      const float inv_pdf = 1.0f / ld_global(pdf + (pdf_by_nbr ? (int64_t)nb.x : m));
+      const SmallParams<H2>& w = par[g];
       float h[kH1];
 #pragma unroll
-      for (int q = 0; q < kH1 / 4; ++q) set4(h + 4 * q, par.b1[q]);
+      for (int q = 0; q < kH1 / 4; ++q) set4(h + 4 * q, w.b1[q]);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float x = (ld_global(p_in + (int64_t)nb.x * 3 + d) - ld_global(p_out + (int64_t)nb.y * 3 + d)) *
-                        inv_radius;
+      for (int d = 0; d < 3; ++d)
 #pragma unroll
-        for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, x, par.w1[d][q]);
-      }
+        for (int q = 0; q < kH1 / 4; ++q) fma4(h + 4 * q, diff[d], w.w1[d][q]);
       activate<kH1>(h, act, alpha);
       if (s.h[1] < kH1) {
 #pragma unroll
@@ -410,9 +417,9 @@ small_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
 #pragma unroll
       for (int q = 0; q < H2 / 4; ++q) {
         float v[4];
-        set4(v, par.b2[q]);
+        set4(v, w.b2[q]);
 #pragma unroll
-        for (int i = 0; i < kH1; ++i) fma4(v, h[i], par.w2[i][q]);
+        for (int i = 0; i < kH1; ++i) fma4(v, h[i], w.w2[i][q]);
         activate<4>(v, act, alpha);
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] *= inv_pdf;
@@ -725,10 +732,11 @@ extern "C" int tfgpc_kernel_mlp_basis_layers(
   TFGPC_REQUIRE(points_in && points_out && neighbors && pdf && weights && biases && basis_out,
                 "KernelMlpBasis got a null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  if (small_mlp(s)) {
+  if (small_mlp(s) && s.G * s.h[2] <= 32) {
     const unsigned blocks = min(blocks_for(M, 256), (unsigned)(sm_count() * 8));
+    const size_t smem = s.G * (s.h[2] <= 8 ? sizeof(SmallParams<8>) : sizeof(SmallParams<16>));
     ProfScope prof(st, "kernel_mlp_basis");
-    TFGPC_CUDA(launch_chained(st, blocks, 256, 0,
+    TFGPC_CUDA(launch_chained(st, blocks, 256, smem,
         s.h[2] <= 8 ? small_mlp_basis_kernel<8> : small_mlp_basis_kernel<16>, s, M, points_in,
         points_out, (const int2*)neighbors, pdf, inv_radius, activation, alpha, pdf_by_neighbor,
         basis_out));

@@ -68,6 +68,13 @@ class Activation(torch.autograd.Function):
     return up * torch.where(x > 0, 1.0, torch.exp(x) if ctx.act else 0.2), None
 
 
+# rows of the basis around the 32 values up to which the register kernel takes several MLPs
+@pytest.mark.parametrize("mlps,h1,h2,m", [(2, 8, 16, 513), (4, 8, 8, 300), (3, 4, 11, 257),
+                                          (32, 2, 1, 100), (5, 7, 8, 65), (33, 1, 1, 9)])
+def test_several_mlps(mlps, h1, h2, m):
+  test_against_64_bits(mlps, h1, h2, m, 1, False)
+
+
 def kinds(t):
   return torch.stack([t.isnan(), t.isposinf(), t.isneginf()])
 
