@@ -39,4 +39,14 @@ __device__ __forceinline__ void slopes(const float* x, float* s, int act, float 
   }
 }
 
+// One unit: a branch on its sign in place of an exponential that nobody needs.
+__device__ __forceinline__ float activation_of(float x, int act, float alpha) {
+  if (act == 1) return x > 0.0f ? x : expm1f(x);
+  return x > 0.0f ? x : x * alpha;
+}
+__device__ __forceinline__ float slope_of(float x, int act, float alpha) {
+  if (x > 0.0f) return 1.0f;
+  return act == 1 ? expf(x) : alpha;
+}
+
 }  // namespace tfgpc

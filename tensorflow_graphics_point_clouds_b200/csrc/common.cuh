@@ -132,6 +132,12 @@ __device__ __forceinline__ void chain_enter(int64_t items = 0, int64_t per_turn 
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The wait alone: the next kernel comes as the blocks end.  For kernels of a few blocks per
+// SM that all run at once: a successor of the same kind that comes early finds the SMs
+// unevenly full and keeps its uneven places (general kernel MLP, four of 8-16 on 94 000 pairs of
+// two dimensions: 26 us behind itself with the early release, 19.4 without).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 inline unsigned blocks_for(int64_t work, int per_block) {
   int64_t b = (work + per_block - 1) / per_block;
   return (unsigned)(b < 1 ? 1 : b);

@@ -109,7 +109,7 @@ kernel_mlp_basis_kernel(MlpShape s, int64_t M, const float* p_in,
                         const float* p_out, const int2* neigh,
                         const float* pdf, float inv_radius, int act, float alpha,
                         int pdf_by_nbr, float* __restrict__ basis) {
-  chain_enter(M, (int64_t)gridDim.x * blockDim.x);
+  chain_wait();
   extern __shared__ __align__(16) float par[];
   const int stride = blockDim.x;
   float* diff = par + s.params + threadIdx.x;        // [D][pair]
@@ -166,7 +166,7 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
                         float* __restrict__ dweights, float* __restrict__ dbiases,
                         float* __restrict__ dp_in, float* __restrict__ dp_out,
                         float* __restrict__ dpdf) {
-  chain_enter(M, (int64_t)gridDim.x * blockDim.x);
+  chain_wait();
   extern __shared__ __align__(16) float par[];       // parameters
   const int tile = blockDim.x;
   const int stride = tile + 4;                       // rows of [unit][pair], banks shifted by 4
@@ -204,6 +204,26 @@ kernel_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
           layer8(s, par, l, g, q, my_units + row * stride, stride, v);
           const int cnt = min(8, ho - 8 * q);
           float slope[8];
+          if (cnt < 8) {      // unit by unit: eight exponentials for one or two units cost more
+            if (!last) {
+#pragma unroll
+              for (int e = 0; e < 7; ++e)
+                if (e < cnt) {
+                  my_units[(next + 8 * q + e) * stride] = activation_of(v[e], act, alpha);
+                  my_units[(next + ho + 8 * q + e) * stride] = slope_of(v[e], act, alpha);
+                }
+            } else {
+              const float* gb = dbasis + m * k_total + g * hl + 8 * q;
+#pragma unroll
+              for (int e = 0; e < 7; ++e)
+                if (e < cnt) {
+                  const float b = live ? ld_global(gb + e) : 0.0f;
+                  grads[(8 * q + e) * stride + threadIdx.x] = b * inv_pdf * slope_of(v[e], act, alpha);
+                  if (dpdf) dpdf_m -= b * activation_of(v[e], act, alpha) * inv_pdf * inv_pdf;
+                }
+            }
+            continue;
+          }
           slopes<8>(v, slope, act, alpha);
           if (!last || dpdf) activate<8>(v, act, alpha);
           if (!last) {

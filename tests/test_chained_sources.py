@@ -76,7 +76,8 @@ def test_chained_kernels(name):
   for kernel, (is_kernel, signature, body) in funcs.items():
     if not is_kernel:
       continue
-    chained = "chain_enter(" in body
+    enter = re.search(r"chain_(enter|wait)\(", body)
+    chained = enter is not None
     # launched one way or the other, by name or through a variable that holds the name
     for m in re.finditer(r"\b%s\b(?:<[^;<>()]*(?:\([^()]*\))?[^;<>()]*>)?" % kernel, text):
       line = text[text.rfind(";", 0, m.start()) + 1:m.start()]
@@ -102,7 +103,7 @@ def test_chained_kernels(name):
     for f in reached(kernel, funcs):
       assert not READ_ONLY.search(funcs[f][1] + funcs[f][2]), (kernel, f)
     # and nothing is read or written before
-    before = body[:body.index("chain_enter(")]
+    before = body[:enter.start()]
     assert not re.search(r"ld_global|__ldc|atomic|\bst_|mbar_wait|tma_|cp_async", before), kernel
     # tensor memory is held before the next kernel may come and ask for it
     if "tmem_alloc" in body:
