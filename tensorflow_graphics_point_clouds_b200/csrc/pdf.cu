@@ -27,28 +27,28 @@ __device__ __forceinline__ void load_bandwidth(int mode, int64_t n, const float*
 
 template <int D>
 __global__ void __launch_bounds__(kPdfThreads)
-compute_pdf_kernel(int mode, int64_t n, int64_t n_bw, const float* centers,
-                   const float* pts,
-                   const int2* neigh, const int32_t* ranges,
-                   const float* inv_bw, const float* inv_r,
+compute_pdf_kernel(int mode, int64_t n, int64_t n_bw, const float* __restrict__ centers,
+                   const float* __restrict__ pts,
+                   const int2* __restrict__ neigh, const int32_t* __restrict__ ranges,
+                   const float* __restrict__ inv_bw, const float* __restrict__ inv_r,
                    float* __restrict__ pdf_out) {
   float bw[D], ir[D];
   load_bandwidth<D>(mode, n_bw, inv_bw, inv_r, bw, ir);
   const int lane = lane_id();
   const int64_t warps = ((int64_t)gridDim.x * kPdfThreads) >> 5;
   for (int64_t i = ((int64_t)blockIdx.x * kPdfThreads + threadIdx.x) >> 5; i < n; i += warps) {
-    const int a = i ? ld_global(ranges + i - 1) : 0;
-    const int e = ld_global(ranges + i);
+    const int a = i ? __ldg(ranges + i - 1) : 0;
+    const int e = __ldg(ranges + i);
     float p[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = ld_global(centers + i * D + d);
+    for (int d = 0; d < D; ++d) p[d] = __ldg(centers + i * D + d);
     float acc = 0.0f;
     for (int m = a + lane; m < e; m += 32) {
-      const int j = ld_global(&neigh[m].x);
+      const int j = __ldg(&neigh[m].x);
       float local = 1.0f;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        float t = (ld_global(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
+        float t = (__ldg(pts + (int64_t)j * D + d) - p[d]) * bw[d] * ir[d];
         local *= bw[d] * expf(t * t * (-0.5f)) * kInvSqrt2Pi;
       }
       acc += local;
