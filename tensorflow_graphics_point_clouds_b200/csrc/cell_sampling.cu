@@ -66,12 +66,12 @@ struct Taken {
 template <int D>
 __device__ __forceinline__ void load_coords(const CellsView& c, int j, float* p) {
   if (D <= 3) {
-    const float4 v = ld_global(c.packed + j);
+    const float4 v = __ldg(c.packed + j);
     p[0] = v.x; p[1] = v.y;
     if (D == 3) p[D - 1] = v.z;
   } else {
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = ld_global(c.points + (int64_t)j * D + d);
+    for (int d = 0; d < D; ++d) p[d] = __ldg(c.points + (int64_t)j * D + d);
   }
 }
 
@@ -96,7 +96,7 @@ __device__ __forceinline__ bool within(const float* s, const float* p, const flo
 template <int D>
 __device__ __forceinline__ int2 later_points(int code, const int* cell, int batch, const int* nc,
                                              int total, bool own,
-                                             const int32_t* start) {
+                                             const int32_t* __restrict__ start) {
   int base = 0, scale = 1, rem = code >> 1, mine = 0, theirs = 0;
   bool ok = true;
 #pragma unroll
@@ -123,7 +123,7 @@ __device__ __forceinline__ int2 later_points(int code, const int* cell, int batc
   }
   if (!ok) return make_int2(0, 0);
   base = (batch * scale + base) * nc[D - 1];
-  return make_int2(ld_global(start + (total - (base + hi))), ld_global(start + (total - (base + lo)) + 1));
+  return make_int2(__ldg(start + (total - (base + hi))), __ldg(start + (total - (base + lo)) + 1));
 }
 
 // Marks the neighbors of the taken points: the candidates of the cell, kSteps per lane
@@ -270,8 +270,8 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int total) {
     const int b = b0 + lane;
     int share = 0;
     if (b < c.batch_size) {
-      const int points = ld_global(c.start + (total - b * cells) + 1) -
-                         ld_global(c.start + (total - (b + 1) * cells) + 1);
+      const int points = __ldg(c.start + (total - b * cells) + 1) -
+                         __ldg(c.start + (total - (b + 1) * cells) + 1);
       share = 1 + (int)(spare * points / c.n);
     }
     int upto = share;
@@ -295,14 +295,13 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int total) {
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 cells_sample_kernel(SampleArgs a) {
-  chain_enter();
   __shared__ int warp_total[kWarps];
   __shared__ int64_t before_s;
   __shared__ int crowded[kMaxCrowded], num_crowded[2];     // (counters of this pass and the next)
   const int lane = lane_id(), w = threadIdx.x >> 5;
   int nc[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) nc[d] = ld_global(a.c.num_cells + d);
+  for (int d = 0; d < D; ++d) nc[d] = __ldg(a.c.num_cells + d);
   const int total = total_cells<D>(nc, a.c.batch_size);
   if (total == 0) return;        // (a grid that got no cells: the call fails)
   const int64_t n = a.c.n;
@@ -311,9 +310,9 @@ cells_sample_kernel(SampleArgs a) {
   if (a.mode == 0) {
     float inv_r[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) inv_r[d] = ld_global(a.inv_radii + d);
+    for (int d = 0; d < D; ++d) inv_r[d] = __ldg(a.inv_radii + d);
     // points outside every cell have no neighbors: all of them are taken
-    const int lead = ld_global(a.c.start + 1), tail = ld_global(a.c.start + total + 1);
+    const int lead = __ldg(a.c.start + 1), tail = __ldg(a.c.start + total + 1);
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < lead + (n - tail);
          i += (int64_t)gridDim.x * kThreads)
       a.state[i < lead ? i : tail + (i - lead)] = 2;
@@ -344,8 +343,8 @@ cells_sample_kernel(SampleArgs a) {
         }
         *batch = team.cloud < 0 ? rem : team.cloud;
         key += *batch * scale;
-        *begin = ld_global(a.c.start + (total - key));
-        *end = ld_global(a.c.start + (total - key) + 1);
+        *begin = __ldg(a.c.start + (total - key));
+        *end = __ldg(a.c.start + (total - key) + 1);
       };
       // a lane looks at every `warps`-th cell: crowded regions spread over the warps
       for (int c0 = 0; c0 < cells; c0 += 32 * warps) {
@@ -396,7 +395,7 @@ cells_sample_kernel(SampleArgs a) {
   auto chosen = [&](int64_t i) {
     if (i >= last) return false;
     return a.mode == 0 ? __ldcg(a.state + i) == 2
-                       : i == 0 || ld_global(a.keys + i) != ld_global(a.keys + i - 1);
+                       : i == 0 || __ldg(a.keys + i) != __ldg(a.keys + i - 1);
   };
   int mine = 0;
   for (int64_t i = first + threadIdx.x; i < last; i += kThreads) mine += chosen(i);
@@ -453,24 +452,24 @@ cells_sample_kernel(SampleArgs a) {
       const int64_t o = out + ahead + __popc(m & ((1u << lane) - 1u));
       if (a.mode == 0) {
 #pragma unroll
-        for (int d = 0; d < D; ++d) a.pts_out[o * D + d] = ld_global(a.c.points + i * D + d);
-        a.batch_out[o] = ld_global(a.c.batch_ids + i);
-        a.index_out[o] = ld_global(a.c.indices + i);
+        for (int d = 0; d < D; ++d) a.pts_out[o * D + d] = __ldg(a.c.points + i * D + d);
+        a.batch_out[o] = __ldg(a.c.batch_ids + i);
+        a.index_out[o] = __ldg(a.c.indices + i);
       } else {
-        const int64_t key = ld_global(a.keys + i);
+        const int64_t key = __ldg(a.keys + i);
         float acc[D];
 #pragma unroll
         for (int d = 0; d < D; ++d) acc[d] = 0.0f;
         int64_t end = i;
         if (key >= 0 && key < total) {
-          end = ld_global(a.c.start + (total - (int)key) + 1);
+          end = __ldg(a.c.start + (total - (int)key) + 1);
         } else {
-          while (end < n && ld_global(a.keys + end) == key) ++end;
+          while (end < n && __ldg(a.keys + end) == key) ++end;
         }
 #pragma unroll 4
         for (int64_t q = i; q < end; ++q)
 #pragma unroll
-          for (int d = 0; d < D; ++d) acc[d] += ld_global(a.c.points + q * D + d);
+          for (int d = 0; d < D; ++d) acc[d] += __ldg(a.c.points + q * D + d);
         const float cnt = (float)(end - i);
 #pragma unroll
         for (int d = 0; d < D; ++d) a.pts_out[o * D + d] = acc[d] / cnt;

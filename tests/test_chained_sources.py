@@ -78,6 +78,7 @@ def test_chained_kernels(name):
       continue
     enter = re.search(r"chain_(enter|wait)\(", body)
     chained = enter is not None
+    launched = False
     # launched one way or the other, by name or through a variable that holds the name
     for m in re.finditer(r"\b%s\b(?:<[^;<>()]*(?:\([^()]*\))?[^;<>()]*>)?" % kernel, text):
       line = text[text.rfind(";", 0, m.start()) + 1:m.start()]
@@ -94,9 +95,11 @@ def test_chained_kernels(name):
         uses = [u for u in uses if "launch_chained" in u or "<<<" in u]
         assert uses, kernel
       for use in uses:
+        launched = launched or "launch_chained" in use or "cudaLaunchKernelEx" in use
         by_attribute = "launch_chained" in use or "cudaLaunchKernelEx" in use
         if by_attribute or "<<<" in use:
           assert by_attribute == chained, "%s: %s" % (kernel, use.strip()[:200])
+    assert launched == chained, kernel
     if not chained:
       continue
     # inputs are written until the wait ends: no read-only loads, here or in what it calls
