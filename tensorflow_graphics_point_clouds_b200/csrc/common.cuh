@@ -114,10 +114,12 @@ cudaError_t launch_chained(cudaStream_t st, dim3 grid, dim3 block, size_t smem, 
 template <typename T>
 __device__ __forceinline__ T ld_global(const T* p) { return *p; }
 
-// Waits for the kernel before this one and, in a short kernel, lets the next one be set up
-// at once (else that happens as the blocks end).  Nothing but the kernel's own parameters,
-// shared memory and tensor memory is touched before it.  Short: the grid makes at most
-// eight turns over `items`, per_turn at a time, and is not much more than a wave of blocks.
+// Waits for the kernel before this one and, unless the launch is a long one, lets the next
+// kernel be set up at once (else that happens as the blocks end).  Nothing but the kernel's own
+// parameters, shared memory and tensor memory is touched before it.  Long: more than 4096
+// blocks or, in a kernel that states its work, more than eight turns of the grid over `items`,
+// per_turn at a time.  (A kernel that states none, like the walks of the grid search, goes by
+// its blocks alone, however long each of them works: the kernels behind the walks are small.)
 // Set up early beside a long kernel that takes an SM's whole shared memory, the next one
 // lives with what is left of the L1 cache, and blocks take their places in another order:
 // 524 288 points, us, 1.3 ms kernels before them: kernel-MLP gradients 347 -> 578, dX product
@@ -127,7 +129,7 @@ __device__ __forceinline__ T ld_global(const T* p) { return *p; }
 // then wait for that block.  (With the call before the barrier nothing but the size of these
 // kernels' shared memory, 169 KB or more, kept two of them off one SM.)
 __device__ __forceinline__ void chain_enter(int64_t items = 0, int64_t per_turn = 0) {
-  if (items <= 8 * per_turn && gridDim.x <= 4096)
+  if (items <= 8 * per_turn && (uint64_t)gridDim.x * gridDim.y * gridDim.z <= 4096)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
