@@ -203,14 +203,13 @@ keys_histogram_kernel(int64_t n, const float* pts,
                       const int32_t* batch_ids, int batch_size,
                       const float* smin_all, const int32_t* num_cells,
                       const float* inv_cell, int64_t* __restrict__ keys_out,
-                      int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded,
-                      int64_t capacity) {
+                      int32_t* counts, int32_t* __restrict__ arrival, int32_t* crowded) {
   chain_enter();
   const Grid<D> g = load_grid<D>(num_cells, inv_cell);
   const int total = total_cells<D>(g.nc, batch_size);
   const int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   const unsigned live = __ballot_sync(0xffffffffu, i < n);
-  if (i >= n || total <= 0 || total > capacity) return;     // (what the table holds)
+  if (i >= n || total == 0) return;
   const int b = ld_global(batch_ids + i);
   const int bs = min(max(b, 0), batch_size - 1);   // (the key keeps the id that was passed in)
   float p[D], smin[D];
@@ -760,7 +759,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
     if (rc) return rc;
     TFGPC_DIM_SWITCH(D, TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0,
         keys_histogram_kernel<kD>, n, points, batch_ids, B, g.scaled_aabb_min, g.num_cells,
-        g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded, cells)));
+        g.inv_cell_sizes, g.keys, g.cell_start, w.arrival, w.crowded)));
   }
   int rc = exclusive_scan_cells(st, g.cell_start, g.num_cells, D, B, cells + 3, w.sums);
   if (rc) return rc;
