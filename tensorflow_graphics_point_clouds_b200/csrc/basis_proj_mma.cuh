@@ -78,14 +78,6 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// the three passes of the split product
-__device__ __forceinline__ void mma3(float* d, const uint32_t* a_hi, const uint32_t* a_mid,
-                                     uint32_t bh0, uint32_t bh1, uint32_t bm0, uint32_t bm1) {
-  mma16816(d, a_hi, bm0, bm1);
-  mma16816(d, a_mid, bh0, bh1);
-  mma16816(d, a_hi, bh0, bh1);
-}
-
 __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid) {
   split2_bf16(x, y, hi, mid);
 }
@@ -116,41 +108,30 @@ __device__ __forceinline__ void cp_wait() {
 // fetched while this one is processed) and handed out by shuffle, so moving from chunk
 // to chunk and sample to sample costs no memory access.  A job is one chunk of up to
 // 16 pairs; a sample without pairs still yields one empty job so that its (zero) result
-// gets written.  With parts > 1 (gradients, whose pairs are independent) every sample
-// is walked as `parts` items, each a run of its chunks.
+// gets written.
 struct Job {
-  int64_t s;     // item (sample * parts + part), -1 once the walk is over
+  int64_t s;     // sample, -1 once the walk is over
   int base;      // first pair of the chunk
   int cnt;       // pairs in the chunk (0 .. 16)
-  bool first, last;  // first / last chunk of the item
+  bool first, last;  // first / last chunk of the sample
   __device__ __forceinline__ bool valid() const { return s >= 0; }
 };
 
 struct Walker {
   const int32_t* ranges;
-  int64_t ns, blk, stride;     // ns: items
-  int lane, li, r_end, a0, nr_end, na0, base, e, bs, parts;
+  int64_t ns, blk, stride;
+  int lane, li, r_end, a0, nr_end, na0, base, e, bs;
   bool started;
-
-  // end of the pairs of item i
-  __device__ __forceinline__ int item_end(int64_t i) const {
-    if (parts == 1) return ld_global(ranges + i);
-    const int64_t s = i / parts;
-    const int p = (int)(i - s * parts) + 1;
-    const int end = ld_global(ranges + s);
-    const int begin = s > 0 ? ld_global(ranges + s - 1) : 0;
-    return part_end(begin, end, p, parts, kChunk);
-  }
 
   __device__ __forceinline__ void load_block(int64_t b, int& rend, int& first) const {
     const int64_t s0 = b * bs;
-    rend = (lane < bs && s0 + lane < ns) ? item_end(s0 + lane) : 0;
-    first = (s0 > 0 && s0 < ns) ? item_end(s0 - 1) : 0;
+    rend = (lane < bs && s0 + lane < ns) ? ld_global(ranges + s0 + lane) : 0;
+    first = (s0 > 0 && s0 < ns) ? ld_global(ranges + s0 - 1) : 0;
   }
 
-  __device__ __forceinline__ void init(const int32_t* r, int64_t items, int64_t warp,
-                                       int64_t warps, int ln, int block, int part_count) {
-    ranges = r; ns = items; blk = warp; stride = warps; lane = ln; bs = block; parts = part_count;
+  __device__ __forceinline__ void init(const int32_t* r, int64_t samples, int64_t warp,
+                                       int64_t warps, int ln, int block) {
+    ranges = r; ns = samples; blk = warp; stride = warps; lane = ln; bs = block;
     li = 0; base = 0; e = 0; started = false;
     load_block(blk, r_end, a0);
     load_block(blk + stride, nr_end, na0);
@@ -182,13 +163,6 @@ struct Walker {
     j.s = blk * bs + li; j.base = base; j.cnt = min(kChunk, e - base);
     j.first = true; j.last = base + kChunk >= e;
     return j;
-  }
-
-  // item that follows s in the walk of this warp (>= ns when there is none)
-  __device__ __forceinline__ int64_t after(int64_t s) const {
-    const int64_t b = s / bs;
-    if (s + 1 < (b + 1) * bs && s + 1 < ns) return s + 1;
-    return (b + stride) * bs;
   }
 };
 
@@ -301,7 +275,7 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
     const int w = min(cfg::kCC, C - c0);
     const int mt_cnt = w >> 4;
     Walker walk;
-    walk.init(ranges, ns, warp, warps, lane, bs, 1);
+    walk.init(ranges, ns, warp, warps, lane, bs);
     Job cur = walk.next(), n1 = walk.next(), n2 = walk.next();
     int idx1 = load_idx(n1, neigh, lane);
     __syncwarp();
@@ -494,6 +468,8 @@ __device__ __forceinline__ void red_add(float* dst, const float* v) {
 }
 
 // The chunks of a team, one after the other (see Walker; an item without pairs is left out).
+// Every sample is walked as `parts` items, each a run of its chunks: a sample's pairs are
+// independent here.
 struct Chunk {
   int item, base, end;     // item -1: no more
   bool first;
