@@ -1,5 +1,6 @@
-"""Kernels that are set up while their predecessor runs (launch_chained) read what it
-wrote: behind a slow producer of their inputs, and replayed from a captured graph."""
+"""Kernels that are set up while their predecessor runs (launch_chained) behind kernels of
+torch, which let nothing come early, and replayed from a captured graph.  (Behind a kernel
+that does let its successor come early: test_early_release_gpu.py.)"""
 import pytest
 import torch
 
