@@ -287,6 +287,18 @@ basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __rest
   }
 }
 
+// Blocks of one resident wave of a wide kernel.
+template <typename Kernel>
+static int wide_grid(Kernel kern, int64_t ns, size_t smem, unsigned* grid) {
+  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  cudaSharedmemCarveoutMaxShared));
+  int per_sm = 1;
+  TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, smem));
+  *grid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
+  return TFGPC_OK;
+}
+
 template <int K, int OUT>
 static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* basis,
                              const float* feat, const int2* neigh, const int32_t* ranges,
@@ -300,16 +312,24 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
   unsigned grid = min(blocks_for(ns, (int)samples_per_block), (unsigned)(sm_count() * 64));
   ProfScope prof(st, OUT == 0 ? "basis_proj" : "basis_proj_split");
   if (G == 32 && C % kCpl == 0 && ((uintptr_t)feat % 16 == 0) && (C * 4) % (kCpl * 4) == 0) {
-    auto kern = basis_proj_wide_kernel<K, OUT>;
     const size_t wsmem = (size_t)(kBpwThreads / 32) * bpw_warp_floats<K>() * sizeof(float);
-    TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem));
-    TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    cudaSharedmemCarveoutMaxShared));
     // exactly one resident wave: all warps then sweep the samples in lock step
     // and the feature rows they gather stay within a few clouds, i.e. in L2
-    int per_sm = 1;
-    TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
-    unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
+    if constexpr (wide_chained<K>(false, 1)) {
+      if (wide_chained<K>(false, C)) {
+        auto kern = basis_proj_wide_kernel<K, OUT, true>;
+        unsigned wgrid = 0;
+        int rc = wide_grid(kern, ns, wsmem, &wgrid);
+        if (rc) return rc;
+        TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
+            ranges, out, hi, mid, shift));
+        return TFGPC_OK;
+      }
+    }
+    auto kern = basis_proj_wide_kernel<K, OUT, false>;
+    unsigned wgrid = 0;
+    int rc = wide_grid(kern, ns, wsmem, &wgrid);
+    if (rc) return rc;
     kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, out, hi, mid, shift);
     TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
@@ -358,17 +378,22 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M
   ProfScope prof(st, "basis_proj_grads");
   if (G == 32 && C % kCpl == 0 && ((uintptr_t)feat % 16 == 0) && ((uintptr_t)dfeat % 16 == 0) &&
       ((uintptr_t)dbasis % 16 == 0)) {
-    auto kern = basis_proj_grads_wide_kernel<K>;
     const size_t wsmem = (size_t)(kBpwThreads / 32) * bpw_grads_warp_floats<K>() * sizeof(float);
-    TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem));
-    TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                    cudaSharedmemCarveoutMaxShared));
-    int per_sm = 1;
-    TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBpwThreads, wsmem));
-    unsigned wgrid = min(blocks_for(ns, kBpwThreads / 32), (unsigned)(sm_count() * max(per_sm, 1)));
-    kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, in_grads, dbasis,
-                                            dfeat, shift);
-    TFGPC_LAUNCH_CHECK();
+    unsigned wgrid = 0;
+    if constexpr (wide_chained<K>(true, 1)) {
+      auto kern = basis_proj_grads_wide_kernel<K, true>;
+      int rc = wide_grid(kern, ns, wsmem, &wgrid);
+      if (rc) return rc;
+      TFGPC_CUDA(launch_chained(st, wgrid, kBpwThreads, wsmem, kern, C, ns, basis, feat, neigh,
+          ranges, in_grads, dbasis, dfeat, shift));
+    } else {
+      auto kern = basis_proj_grads_wide_kernel<K, false>;
+      int rc = wide_grid(kern, ns, wsmem, &wgrid);
+      if (rc) return rc;
+      kern<<<wgrid, kBpwThreads, wsmem, st>>>(C, ns, basis, feat, neigh, ranges, in_grads, dbasis,
+                                              dfeat, shift);
+      TFGPC_LAUNCH_CHECK();
+    }
     return TFGPC_OK;
   }
   if (vec)

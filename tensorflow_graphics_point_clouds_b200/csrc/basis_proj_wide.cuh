@@ -9,13 +9,15 @@
 //   - the feature rows, the only scattered traffic, are fetched U at a time
 //     before any of them is used, which keeps U independent 512-byte row reads
 //     in flight per warp.
-// Both kernels are launched after their predecessor's end and load on the read-only path,
-// like the narrow ones (basis_proj.cu): plain loads stay behind the writes of the sample
-// before and cost registers.  Chained with plain loads and as they are, us, lists of 30:
-// 15 000 samples, gradients, K = 64: C = 24 1035 / 840, C = 64 1932 / 1577, C = 128 3803 / 3070,
-// K = 8, C = 96 134 / 136; forward, K = 64, C = 72 364 / 329.  900 samples, forward, C = 256:
-// K = 8 12.6 / 11.0, K = 16 19.8 / 15.0, K = 64 94 / 68; gradients, K = 32, C = 256 88 / 63.
-// (Chained with plain loads and no early release of the successor: as slow.)
+// Two instances of each kernel.  CHAINED false: launched after its predecessor's end, with loads
+// on the read-only path, like the narrow kernels (basis_proj.cu): plain loads stay behind the
+// writes of the sample before and cost registers.  CHAINED true: set up while the predecessor
+// runs, with plain loads; only for K = 8, whose few accumulators leave room (wide_chained).
+// Chained and not, us, lists of 30: 15 000 samples, gradients, K = 64: C = 24 1035 / 840, C = 64
+// 1932 / 1577, C = 128 3803 / 3070; forward, K = 64, C = 72 364 / 329.  900 samples, forward,
+// C = 256: K = 16 19.8 / 15.0, K = 64 94 / 68.  But K = 8, forward, one pass over the channels, C = 128:
+// 56.6 / 60.1 and 5.6 / 7.0 at 900 samples (two passes, C = 256: 110.4 / 111.3 and 12.5 / 11.0);
+// gradients, C = 128 136 / 140, C = 136 256 / 255 and 24.0 / 25.3.
 #pragma once
 
 #include "basis_proj.cuh"
@@ -23,6 +25,15 @@
 namespace tfgpc {
 
 constexpr int kBpwThreads = 256;
+
+// Which of the two instances (see above).
+template <int K>
+constexpr bool wide_chained(bool gradients, int C) {
+  return K == 8 && (gradients || C <= 32 * BpCfg<K>::kCpl);
+}
+
+template <bool CHAINED, typename T>
+__device__ __forceinline__ T ld_input(const T* p) { return CHAINED ? ld_global(p) : __ldg(p); }
 constexpr int kBpwUnroll = 4;
 
 template <int CPL>
@@ -48,12 +59,12 @@ struct FeatVec<1> {
 // Per-warp shared-memory tile: 32 rows of kRow floats.  During the neighbor
 // loop its first 32*K floats hold the staged basis rows; afterwards the whole
 // tile stages the warp's output for coalesced stores.
-template <int K>
-__device__ __forceinline__ void stage_basis_chunk(float* tile, const float* __restrict__ basis,
+template <int K, bool CHAINED>
+__device__ __forceinline__ void stage_basis_chunk(float* tile, const float* basis,
                                                   int base, int cnt, int lane) {
   const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)base * K);
   float4* dst = reinterpret_cast<float4*>(tile);
-  for (int i = lane; i < cnt * (K / 4); i += 32) dst[i] = __ldg(src + i);
+  for (int i = lane; i < cnt * (K / 4); i += 32) dst[i] = ld_input<CHAINED>(src + i);
 }
 
 // ---- small PTX helpers ---------------------------------------------------------
@@ -109,13 +120,14 @@ __host__ __device__ constexpr int bpw_warp_floats() {
              : kBpwRing * 32 * BpCfg<K>::kCpl + 32 * K;
 }
 
-template <int K, int OUT>
+template <int K, int OUT, bool CHAINED>
 __global__ void __launch_bounds__(kBpwThreads, 2)
-basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
-                       const float* __restrict__ feat, const int2* __restrict__ neigh,
-                       const int32_t* __restrict__ ranges, float* __restrict__ out,
+basis_proj_wide_kernel(int C, int64_t ns, const float* basis,
+                       const float* feat, const int2* neigh,
+                       const int32_t* ranges, float* __restrict__ out,
                        __nv_bfloat16* __restrict__ out_hi, __nv_bfloat16* __restrict__ out_mid,
                        int shift) {
+  if (CHAINED) chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kAcc = BpCfg<K>::kAcc;
   constexpr int kRow = BpCfg<K>::kRow;
@@ -129,8 +141,8 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
   float* wtile = tile + R * 32 * kCpl;          // [32 neighbors][K]
   const int64_t warps = ((int64_t)gridDim.x * kBpwThreads) >> 5;
   for (int64_t s = ((int64_t)blockIdx.x * kBpwThreads + threadIdx.x) >> 5; s < ns; s += warps) {
-    const int a = s ? __ldg(ranges + s - 1) : 0;
-    const int e = __ldg(ranges + s);
+    const int a = s ? ld_input<CHAINED>(ranges + s - 1) : 0;
+    const int e = ld_input<CHAINED>(ranges + s);
     for (int c0 = 0; c0 < C; c0 += kChunk) {
       const int cbase = c0 + lane * kCpl;
       const bool c_ok = cbase < C;  // C is a multiple of CPL on this path
@@ -142,8 +154,8 @@ basis_proj_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
       for (int base = a; base < e; base += 32) {
         const int cnt = min(32, e - base);
         __syncwarp();
-        const int my_j = lane < cnt ? __ldg(&neigh[base + lane].x) : 0;
-        stage_basis_chunk<K>(wtile, basis, base, cnt, lane);
+        const int my_j = lane < cnt ? ld_input<CHAINED>(&neigh[base + lane].x) : 0;
+        stage_basis_chunk<K, CHAINED>(wtile, basis, base, cnt, lane);
         // fill the ring: rows 0 .. R-1 of the chunk (one commit group per row)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -226,13 +238,14 @@ __host__ __device__ constexpr int bpw_grads_warp_floats() {
   return kBpwRing * 32 * BpCfg<K>::kCpl + 2 * 32 * K;
 }
 
-template <int K>
+template <int K, bool CHAINED>
 __global__ void __launch_bounds__(kBpwThreads, 2)
-basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
-                             const float* __restrict__ feat, const int2* __restrict__ neigh,
-                             const int32_t* __restrict__ ranges,
-                             const float* __restrict__ in_grads, float* __restrict__ dbasis,
+basis_proj_grads_wide_kernel(int C, int64_t ns, const float* basis,
+                             const float* feat, const int2* neigh,
+                             const int32_t* ranges,
+                             const float* in_grads, float* __restrict__ dbasis,
                              float* __restrict__ dfeat, int shift) {
+  if (CHAINED) chain_enter(ns * 32, (int64_t)gridDim.x * kBpwThreads);
   constexpr int kCpl = BpCfg<K>::kCpl;
   constexpr int kChunk = 32 * kCpl;
   constexpr int R = kBpwRing;
@@ -262,13 +275,13 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
     if (lane & (1 << t)) perm += K >> (t + 1);
   const int permq = perm >> 2;  // in units of 4 values (one 128-bit load)
   for (int64_t s = ((int64_t)blockIdx.x * kBpwThreads + threadIdx.x) >> 5; s < ns; s += warps) {
-    const int a = s ? __ldg(ranges + s - 1) : 0;
-    const int e = __ldg(ranges + s);
+    const int a = s ? ld_input<CHAINED>(ranges + s - 1) : 0;
+    const int e = ld_input<CHAINED>(ranges + s);
     for (int base = a; base < e; base += 32) {
       const int cnt = min(32, e - base);
       __syncwarp();
-      const int my_j = lane < cnt ? __ldg(&neigh[base + lane].x) : 0;
-      stage_basis_chunk<K>(wtile, basis, base, cnt, lane);
+      const int my_j = lane < cnt ? ld_input<CHAINED>(&neigh[base + lane].x) : 0;
+      stage_basis_chunk<K, CHAINED>(wtile, basis, base, cnt, lane);
       for (int i = lane; i < 32 * K; i += 32) dtile[i] = 0.0f;
       for (int c0 = 0; c0 < C; c0 += kChunk) {
         const int cbase = c0 + lane * kCpl;
@@ -288,7 +301,7 @@ basis_proj_grads_wide_kernel(int C, int64_t ns, const float* __restrict__ basis,
           for (int q = 0; q < K / 4; ++q) {
             const ulonglong2* src = reinterpret_cast<const ulonglong2*>(
                 in_grads + block_offset<K>(s, C, cbase + cc, 4 * (q ^ permq), shift));
-            const ulonglong2 v = c_ok ? __ldg(src) : make_ulonglong2(0ull, 0ull);
+            const ulonglong2 v = c_ok ? ld_input<CHAINED>(src) : make_ulonglong2(0ull, 0ull);
             g[cc][2 * q] = v.x; g[cc][2 * q + 1] = v.y;
           }
         }

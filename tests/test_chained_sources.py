@@ -78,11 +78,14 @@ def test_chained_kernels(name):
       continue
     enter = re.search(r"chain_(enter|wait)\(", body)
     chained = enter is not None
+    # a kernel with both kinds of instance: the last template argument says which
+    switched = "if (CHAINED) chain_enter(" in body
     launched = False
     # launched one way or the other, by name or through a variable that holds the name
     for m in re.finditer(r"\b%s\b(?:<[^;<>()]*(?:\([^()]*\))?[^;<>()]*>)?" % kernel, text):
       line = text[text.rfind(";", 0, m.start()) + 1:m.start()]
       after = text[m.end():].lstrip()
+      wanted = "true>" in m.group(0) if switched else chained
       if "__global__" in line:
         continue
       variable = re.search(r"auto\*? (\w+) =", line)
@@ -98,12 +101,14 @@ def test_chained_kernels(name):
         launched = launched or "launch_chained" in use or "cudaLaunchKernelEx" in use
         by_attribute = "launch_chained" in use or "cudaLaunchKernelEx" in use
         if by_attribute or "<<<" in use:
-          assert by_attribute == chained, "%s: %s" % (kernel, use.strip()[:200])
+          assert by_attribute == wanted, "%s: %s" % (kernel, use.strip()[:200])
     assert launched == chained, kernel
     if not chained:
       continue
     # inputs are written until the wait ends: no read-only loads, here or in what it calls
-    for f in reached(kernel, funcs):
+    # (ld_input<CHAINED> loads as the instance may)
+    for f in reached(kernel, funcs) - ({"ld_input"} if switched else set()):
+      assert not re.search(r"ld_input<(?!CHAINED>)", funcs[f][2]), (kernel, f)
       assert not READ_ONLY.search(funcs[f][1] + funcs[f][2]), (kernel, f)
     # and nothing is read or written before
     before = body[:enter.start()]
