@@ -166,10 +166,14 @@ basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __rest
   const int chunk = G * kCpl;
   const bool single_pass = C <= chunk;
   // pairs beyond the last range belong to no sample: their gradient is zero
-  if (single_pass)
+  auto clear_rest = [&]() {
     for (int64_t i = (int64_t)__ldg(ranges + ns - 1) * K + warp0 * 32 + lane; i < M * K;
          i += warps * 32)
       dbasis[i] = 0.0f;
+  };
+  // (first where registers are left, else last: 15 000 samples of 30 pairs, first and last, us:
+  // K = 32, C = 3 130 / 119, C = 16 189 / 175, C = 24 316 / 299; K = 16, C = 24 130 / 133)
+  if (K < 32 && single_pass) clear_rest();
   for (int64_t s0 = warp0 * groups_per_warp; s0 < ns; s0 += warps * groups_per_warp) {
     const int64_t s = s0 + lane / G;
     const bool active = s < ns;
@@ -285,6 +289,7 @@ basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __rest
       }
     }
   }
+  if (K >= 32 && single_pass) clear_rest();
 }
 
 // Blocks of one resident wave of a wide kernel.
