@@ -129,7 +129,8 @@ def pack_points_density(points, pdf):
 def kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, radius, activation=0,
                  alpha=0.2, pdf_by_neighbor=False):
   """basis[m, k] = act(diff_m . w1[:, k] + b1[k]) / pdf[m] (tfgpc_kernel_basis).
-  w1 [D, K] (or [G, D, K / G], G kernel MLPs), b1 [K]; neighbors hold (index into points_in, index into points_out).
+  w1 [D, K] (or [G, D, K / G], G kernel MLPs), b1 [K]; neighbors hold (index into points_in,
+  index into points_out).
   pdf_by_neighbor: pdf is a table with one density per point of points_in, read
   at the pair's neighbor index, instead of the per-pair array."""
   return _lib.host().kernel_basis(points_in, points_out, neighbors, pdf, w1, b1, float(radius),
@@ -197,17 +198,21 @@ def _grouped_supported(k, c):
   return _lib.lib().tfgpc_mcconv_grouped_supported(c_int(k), c_int(c)) != 0
 
 
+def _library_get_pdf():
+  from . import pc
+  return pc.LIBRARY_GET_PDF
+
+
 def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
   from . import pc
   return pc.grid_neighborhood_with_pdf(point_cloud_in, radius, point_cloud_out,
                                        bandwidth=bandwidth)
 
 
-def _is_own(obj, name):
-  """Whether the method is the library's: not replaced in a subclass, on the class or on
-  the object."""
-  own = getattr(type(obj), '_library_' + name.lstrip('_'), None)
-  return own is not None and getattr(getattr(obj, name), '__func__', None) is own
+def _is_own(method, own):
+  """Whether a bound method is the library's function `own`: not replaced in a subclass, on
+  the class or on the object."""
+  return getattr(method, '__func__', None) is own
 
 
 class MCConv:
@@ -248,12 +253,10 @@ class MCConv:
     from . import pc
     return pc.grid_neighborhood(point_cloud_in, radius, point_cloud_out)
 
-  _library_build_neighborhood = build_neighborhood
-
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
     neigh, packed = neighborhood, None
-    if neigh is None and _is_own(self, 'build_neighborhood'):
+    if neigh is None and _is_own(self.build_neighborhood, _LIBRARY_BUILD_NEIGHBORHOOD):
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
       packed = neigh._packed      # (of these points: no other neighborhood's is asked for)
     elif neigh is None:
@@ -356,6 +359,9 @@ class MCConv:
     return dfeat, dw1, db1, dwf
 
 
+_LIBRARY_BUILD_NEIGHBORHOOD = MCConv.build_neighborhood
+
+
 # ---- KPConv and PointConv: other bases on the same projection + weight product
 
 def _basis_count(k):
@@ -400,8 +406,6 @@ class _ProjectedConv:
     from . import pc
     return pc.grid_neighborhood(point_cloud_in, radius, point_cloud_out)
 
-  _library_neighborhood = _neighborhood
-
   def _project(self, basis, features, neigh, weights, ns, keep_for_backward):
     if self._op is None or self._op.ns != ns or self._op.backward_ws != keep_for_backward:
       self._op = ProjectionGemm(self.k_pad, self.cin, self.cout_pad, ns, features.device,
@@ -419,6 +423,9 @@ class _ProjectedConv:
     return self._op.backward(basis, features, neigh._original_neigh_ids,
                              neigh._samples_neigh_ranges, weights, out_grads,
                              blocks=(1, self.k, self.cout))
+
+
+_LIBRARY_NEIGHBORHOOD = _ProjectedConv._neighborhood
 
 
 class KPConv(_ProjectedConv):
@@ -472,14 +479,15 @@ class PointConv(_ProjectedConv):
 
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
-    if neighborhood is None and _is_own(self, '_neighborhood'):
+    if neighborhood is None and _is_own(self._neighborhood, _LIBRARY_NEIGHBORHOOD):
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
     else:
       neigh = self._neighborhood(point_cloud_in, point_cloud_out, radius, neighborhood)
     # the densities as a table, unless get_pdf is not the library's own
     pdf, table_ids = None, None
-    if _is_own(neigh, 'get_pdf'):
-      pdf, table_ids = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0), neigh._original_neigh_ids
+    if _is_own(neigh.get_pdf, _library_get_pdf()):
+      pdf = neigh.pdf_by_neighbor_id(bandwidth=bandwidth, mode=0)
+      table_ids = neigh._original_neigh_ids
     if pdf is None:
       pdf, table_ids = neigh.get_pdf(bandwidth=bandwidth, mode=0), None
     scale = pointconv_pdf(pdf, neigh._samples_neigh_ranges, self.pdf_weights[0],

@@ -427,8 +427,6 @@ class Neighborhood:
         self._pdf = self._point_pdf[self._neighbors[:, 0].to(torch.int64)]
     return self._pdf
 
-  _library_get_pdf = get_pdf
-
   def pdf_point_grads(self, pdf_grads, bandwidth=0.2, mode=0):
     """Gradient of a loss with respect to the grid's points [N, D] (in their
     original order) through the per-pair densities of get_pdf, given the loss's
@@ -457,6 +455,9 @@ class Neighborhood:
     out = torch.empty_like(grads_sorted)
     out[g._sorted_indices.to(torch.int64)] = grads_sorted
     return out
+
+
+LIBRARY_GET_PDF = Neighborhood.get_pdf     # (the class's own may be replaced: mcconv.PointConv)
 
 
 def grid_neighborhood(point_cloud, radius, point_cloud_sample=None, max_neighbors=0):
@@ -496,12 +497,13 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   samples = dict(samples=None if smp is None else smp._points,
                  samples_batch_ids=None if smp is None else smp._batch_ids,
                  samples_are_points=mode, max_neighs=max_neighbors)
-  build, density = ops.build_cell_grid, {}
+  inv_radii = _to_dims(radius, d, dev, inverse=True)
   if with_pdf:
-    build = ops.build_cell_grid_with_pdf
-    density = dict(inv_bandwidth=_to_dims(bandwidth, d, dev, inverse=True), pdf_mode=pdf_mode)
-  built = _cell_grid(pc, sizes, build, cells=cells,
-                     inv_radii=_to_dims(radius, d, dev, inverse=True), **density, **samples)
+    built = _cell_grid(pc, sizes, ops.build_cell_grid_with_pdf, cells=cells, inv_radii=inv_radii,
+                       inv_bandwidth=_to_dims(bandwidth, d, dev, inverse=True), pdf_mode=pdf_mode,
+                       **samples)
+  else:
+    built = _cell_grid(pc, sizes, ops.build_cell_grid, cells=cells, inv_radii=inv_radii, **samples)
   grid = object.__new__(Grid)
   grid._cell_sizes = _to_dims(radius, d, dev)
   if built is not None:
