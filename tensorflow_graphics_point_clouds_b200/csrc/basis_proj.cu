@@ -304,10 +304,22 @@ static int wide_grid(Kernel kern, int64_t ns, size_t smem, unsigned* grid) {
   return TFGPC_OK;
 }
 
+// basis_proj_tile.cu
+bool basis_proj_tile_takes(int K, int C, int64_t ns, const float* feat);
+bool basis_proj_grads_tile_takes(int K, int C, const float* feat);
+int basis_proj_tile(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
+                    const float* feat, const int2* neigh, const int32_t* ranges, float* out,
+                    __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
+int basis_proj_grads_tile(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
+                          const float* feat, const int2* neigh, const int32_t* ranges,
+                          const float* in_grads, float* dbasis, float* dfeat, int hidden);
+
 template <int K, int OUT>
 static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* basis,
                              const float* feat, const int2* neigh, const int32_t* ranges,
                              float* out, __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden = K) {
+  if (basis_proj_tile_takes(K, C, ns, feat))
+    return basis_proj_tile(st, K, C, ns, basis, feat, neigh, ranges, out, hi, mid, hidden);
   constexpr int kCpl = BpCfg<K>::kCpl;
   const int shift = hidden_shift(hidden);
   const int G = bp_group_lanes(C, kCpl);
@@ -373,6 +385,9 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M
                                    const float* feat, const int2* neigh, const int32_t* ranges,
                                    const float* in_grads, float* dbasis, float* dfeat,
                                    int hidden) {
+  if (basis_proj_grads_tile_takes(K, C, feat))
+    return basis_proj_grads_tile(st, K, C, ns, M, basis, feat, neigh, ranges, in_grads, dbasis,
+                                 dfeat, hidden);
   constexpr int kCpl = BpCfg<K>::kCpl;
   const int shift = hidden_shift(hidden);
   const int G = bp_group_lanes(C, kCpl);
@@ -455,9 +470,11 @@ extern "C" int tfgpc_basis_proj(void* stream, int K, int C, int64_t ns, int64_t 
 }
 
 namespace tfgpc {
-// Layers of fewer than 32 lanes write a pair's gradient row once; the others add into it.
-bool basis_proj_grads_adds_dbasis(int K, int C) {
-  return bp_group_lanes(C, K >= 64 ? 1 : K == 32 ? 2 : 4) == 32;
+// Layers of fewer than 32 lanes write a pair's gradient row once, and so do the tile kernels;
+// the others add into it.
+bool basis_proj_grads_adds_dbasis(int K, int C, const float* feat) {
+  return !basis_proj_grads_tile_takes(K, C, feat) &&
+         bp_group_lanes(C, K >= 64 ? 1 : K == 32 ? 2 : 4) == 32;
 }
 
 // The gradients on the SIMT kernels, in_grads with the columns of block_offset.
@@ -489,7 +506,7 @@ extern "C" int tfgpc_basis_proj_grads(void* stream, int K, int C, int64_t ns, in
   TFGPC_REQUIRE((M == 0 || dbasis_out) && (n_in == 0 || dfeat_out),
                 "BasisProjGradsOp got a null pointer");
   Prepare jobs;
-  if (ns == 0 || basis_proj_grads_adds_dbasis(K, C))
+  if (ns == 0 || basis_proj_grads_adds_dbasis(K, C, features))
     jobs.zero(dbasis_out, (size_t)M * K * sizeof(float));
   jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
   rc = prepare((cudaStream_t)stream, jobs);

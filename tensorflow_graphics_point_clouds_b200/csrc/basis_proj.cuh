@@ -59,4 +59,24 @@ __device__ __forceinline__ void split2_bf16(float x, float y, uint32_t& hi, uint
   mid = *reinterpret_cast<const uint32_t*>(&m);
 }
 
+// Two fp32 FMAs per instruction (sm_100 packed fp32): d = a * b + c on both
+// halves of 64-bit register pairs.  Halves the issue slots of the FMA-bound
+// inner loops of the projections.
+__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b,
+                                                    unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
 }  // namespace tfgpc

@@ -69,26 +69,6 @@ __device__ __forceinline__ void stage_basis_chunk(float* tile, const float* basi
 
 // ---- small PTX helpers ---------------------------------------------------------
 
-// Two fp32 FMAs per instruction (sm_100 packed fp32): d = a * b + c on both
-// halves of 64-bit register pairs.  Halves the issue slots of the FMA-bound
-// inner loops below.
-__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b,
-                                                    unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-
 // Asynchronous global -> shared copy of one lane's slice of a feature row.
 template <int BYTES>
 __device__ __forceinline__ void cp_async_row(float* dst_smem, const float* src) {

@@ -18,7 +18,7 @@ int basis_proj_split(cudaStream_t st, int K, int C, int64_t ns, const float* bas
                      __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden);
 // (adds into dfeat, and into dbasis where basis_proj_grads_adds_dbasis says so: the caller
 // clears them)
-bool basis_proj_grads_adds_dbasis(int K, int C);
+bool basis_proj_grads_adds_dbasis(int K, int C, const float* feat);
 int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t M,
                             const float* basis, const float* feat, const int32_t* neigh,
                             const int32_t* ranges, const float* in_grads, float* dbasis,
@@ -349,7 +349,7 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   pw.cleared = gemm_adds_slices(pw);
   if (pw.cleared) jobs.zero(pw.c, (size_t)ck * co * sizeof(float));
   jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
-  if (!fs_ok && basis_proj_grads_adds_dbasis(K, C))
+  if (!fs_ok && basis_proj_grads_adds_dbasis(K, C, features))
     jobs.zero(dbasis_out, (size_t)M * K * sizeof(float));
   rc = prepare(st, jobs);
   if (rc) return rc;
