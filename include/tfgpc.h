@@ -566,6 +566,20 @@ int tfgpc_mcconv_backward_blocks(void* stream, int K, int C, int Cout, int group
                                  float* dbasis_out, float* dfeat_out,
                                  float* dweights_out, void* ws, size_t ws_bytes);
 
+/* tfgpc_mcconv_backward_blocks without the gradient of the basis, for layers whose
+ * kernel is not trained (rigid KPConv, KPConv.py:171-230).
+ * tfgpc_mcconv_feature_grads_supported: layers and buffers it takes. */
+int tfgpc_mcconv_feature_grads_supported(int K, int C, const float* features,
+                                         const float* dfeat);
+int tfgpc_mcconv_backward_features(void* stream, int K, int C, int Cout, int groups,
+                                   int k_src, int cout_src, int64_t ns,
+                                   int64_t n_in, int64_t M, const float* basis,
+                                   const float* features, const int32_t* neighbors,
+                                   const int32_t* ranges, const float* weights,
+                                   const float* out_grads, int x_in_workspace,
+                                   float* dfeat_out, float* dweights_out, void* ws,
+                                   size_t ws_bytes);
+
 /* ---- MCConv forward and backward on a group plan -------------------------
  * No counterpart in the reference; same results as tfgpc_mcconv_forward /
  * _backward.  BasisProj and BasisProjGrads (basis_proj_kernels.cu.cc:30-127,

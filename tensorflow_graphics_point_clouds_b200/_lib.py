@@ -78,6 +78,8 @@ SYMBOLS = {
     "tfgpc_mcconv_blocks_supported": c_int,
     "tfgpc_mcconv_forward_blocks": c_int,
     "tfgpc_mcconv_backward_blocks": c_int,
+    "tfgpc_mcconv_feature_grads_supported": c_int,
+    "tfgpc_mcconv_backward_features": c_int,
     "tfgpc_linear_workspace_bytes": c_sz,
     "tfgpc_linear_f32": c_int,
     "tfgpc_mcconv_grouped_supported": c_int,

@@ -40,12 +40,12 @@ int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __n
   return TFGPC_OK;
 }
 
-template <int K, int CC>
+template <int K, int CC, bool BASIS>
 int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* basis,
                  const __nv_bfloat16* fs, const int2* neigh, const int32_t* ranges,
                  const float* in_grads, float* dbasis, float* dfeat, int hidden) {
-  typedef bpm::GradCfg<K, CC> cfg;
-  auto kern = bpm::basis_proj_grads_mma_kernel<K, CC>;
+  typedef bpm::GradCfg<K, CC, BASIS> cfg;
+  auto kern = bpm::basis_proj_grads_mma_kernel<K, CC, BASIS>;
   constexpr int smem = cfg::kTeams * cfg::kTeamBytes;
   TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   // few samples with long lists: several teams share a sample's chunks
@@ -55,7 +55,7 @@ int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* bas
   if (parts > most) parts = most;
   if (parts < 1) parts = 1;
   Shape s = walk_shape(ns * parts, cfg::kTeams);
-  ProfScope prof(st, "basis_proj_grads_mma");
+  ProfScope prof(st, BASIS ? "basis_proj_grads_mma" : "basis_proj_feature_grads_mma");
   TFGPC_CUDA(launch_chained(st, s.grid, cfg::kThreads, smem, kern, s.bs, (int)parts,
       hidden_shift(hidden), C, ns, M, basis, fs, neigh, ranges, in_grads, dbasis, dfeat));
   return TFGPC_OK;
@@ -99,13 +99,16 @@ int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* b
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
+// dbasis null: the gradient of the features alone.
 int basis_proj_grads_mma(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          const float* in_grads, float* dbasis, float* dfeat, int hidden) {
   // (at K = 16 wide layers take two passes: a team could not share their fragments)
-  TFGPC_CC_SWITCH(K, C, return launch_grads<kK, (kK * kCC > 1024 && kK == 16 ? 64 : kCC)>(
-                            st, C, ns, M, basis, fs, (const int2*)neigh, ranges, in_grads, dbasis,
-                            dfeat, hidden))
+  TFGPC_CC_SWITCH(K, C, constexpr int kPass = kK == 16 && kCC > 64 ? 64 : kCC;
+                  return dbasis ? launch_grads<kK, kPass, true>(st, C, ns, M, basis, fs, (const int2*)neigh,
+                                                                ranges, in_grads, dbasis, dfeat, hidden)
+                                : launch_grads<kK, kPass, false>(st, C, ns, M, basis, fs, (const int2*)neigh,
+                                                                 ranges, in_grads, nullptr, dfeat, hidden))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 

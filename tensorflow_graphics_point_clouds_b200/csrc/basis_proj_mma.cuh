@@ -424,7 +424,9 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
 // piece of dX twice through L1: 228 against 185 us on 33 000 samples.)
 // dbasis is written, not accumulated (every pair belongs to exactly one sample; layers
 // wider than a pass add to it pass by pass); dfeat must be zero on entry.
-template <int K, int CC>
+// BASIS false: dfeat alone, for layers whose basis is not trained: (1) is left out, and no
+// features are gathered.
+template <int K, int CC, bool BASIS>
 struct GradCfg {
   static_assert(K * CC <= 2048 && CC % 32 == 0 && (K * CC <= 1024 || K >= 32), "fragments");
   static constexpr int kTeam = K * CC > 1024 ? 2 : 1;       // warps per sample
@@ -435,12 +437,14 @@ struct GradCfg {
   static constexpr int kFeatStride = CC * 4 + 16;           // bytes: hi[CC] | mid[CC] | pad
   static constexpr int kKStride = K * 2 + 16;               // a bf16 row over k
   static constexpr int kRawStride = K + 4;                  // floats, a row of dX over k
-  static constexpr int kFeatBytes = kChunk * kFeatStride;
+  static constexpr int kFeatBytes = BASIS ? kChunk * kFeatStride : 0;
   static constexpr int kStageBytes = kFeatBytes + 2 * kChunk * kKStride;
   static constexpr int kRawBytes = CC * kRawStride * 4;
   static constexpr int kTeamBytes = kRawBytes + 2 * kStageBytes;
   static constexpr int kFit = 227 * 1024 / kTeamBytes * kTeam;      // warps: 16 of 128 registers
-  static constexpr int kTeams = (kFit >= 16 && kMt1 == 1 ? 16 : 12) / kTeam;     // or 12 of 168
+  static constexpr int kWarps = !BASIS && K * CC <= 512 ? 24                        // or 24 of 80
+                                : kFit >= 16 && (kMt1 == 1 || !BASIS) ? 16 : 12;    // or 12 of 168
+  static constexpr int kTeams = kWarps / kTeam;
   static constexpr int kThreads = kTeams * kTeam * 32;
   static constexpr int kBasisVecs = kChunk * K / 4 / (32 * kTeam);   // float4 per lane and chunk
   static_assert(kTeams * kTeamBytes <= 227 * 1024 && (kTeam == 1 || kTeams <= 15),
@@ -535,15 +539,15 @@ struct ChunkWalk {
   }
 };
 
-template <int K, int CC>
-__global__ void __launch_bounds__(GradCfg<K, CC>::kThreads, 1)
+template <int K, int CC, bool BASIS>
+__global__ void __launch_bounds__(GradCfg<K, CC, BASIS>::kThreads, 1)
 basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int64_t M,
                             const float* basis,
                             const __nv_bfloat16* fs, const int2* neigh,
                             const int32_t* ranges,
                             const float* in_grads, float* __restrict__ dbasis,
                             float* __restrict__ dfeat) {
-  typedef GradCfg<K, CC> cfg;
+  typedef GradCfg<K, CC, BASIS> cfg;
   constexpr int W = cfg::kTeam;
   chain_enter(ns * parts * 32 * W, (int64_t)gridDim.x * blockDim.x);
   extern __shared__ __align__(128) uint8_t bpm_smem[];
@@ -571,7 +575,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
   const int row1 = 16 * cfg::kMt1 * sub, row2 = 16 * cfg::kMt2 * sub;   // this warp's rows
 
   // pairs beyond the last range belong to no sample: their gradient is zero
-  if (blockIdx.x == 0 && threadIdx.x < 32) {
+  if (BASIS && blockIdx.x == 0 && threadIdx.x < 32) {
     const int64_t covered = ns > 0 ? ld_global(ranges + ns - 1) : 0;
     for (int64_t i = covered * K + lane; i < M * K; i += 32) dbasis[i] = 0.0f;
   }
@@ -649,7 +653,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
     if (w < CC) {
       // channels that do not exist, on either side of (1)
       for (int i = tid; i < (CC - w) * cfg::kRawStride; i += 32 * W) raw[w * cfg::kRawStride + i] = 0.0f;
-      for (int i = tid; i < 2 * kChunk * 2 * (CC - w) / 8; i += 32 * W) {
+      for (int i = tid; BASIS && i < 2 * kChunk * 2 * (CC - w) / 8; i += 32 * W) {
         const int r = i / (2 * (CC - w) / 8), e = i % (2 * (CC - w) / 8), h = e / ((CC - w) / 8);
         uint8_t* row = mem + cfg::kRawBytes + (r / kChunk) * cfg::kStageBytes + (r % kChunk) * cfg::kFeatStride;
         *reinterpret_cast<uint4*>(row + h * (CC * 2) + (w + e % ((CC - w) / 8) * 8) * 2) =
@@ -669,7 +673,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
     for (int t = 0; t < cfg::kBasisVecs; ++t) rows[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (cur.valid()) {
       issue_dx(cur.item);
-      issue_rows(0, cur, idx0);
+      if (BASIS) issue_rows(0, cur, idx0);
       load_rows(cur, rows);
       store_rows(0, rows);
     }
@@ -686,7 +690,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
       team_sync();
       if (cur.first) {
 #pragma unroll
-        for (int mt = 0; mt < cfg::kMt1; ++mt) {
+        for (int mt = 0; mt < (BASIS ? cfg::kMt1 : 0); ++mt) {
           const int k = row1 + out_row(mt, kVec1);
 #pragma unroll
           for (int ks = 0; ks < cfg::kKs1; ++ks) {
@@ -723,7 +727,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
         issue_dx(n2.item);
       }
       if (n1.valid()) {
-        issue_rows(st ^ 1, n1, idx1);
+        if (BASIS) issue_rows(st ^ 1, n1, idx1);
         load_rows(n1, rows);
       }
       cp_commit();
@@ -737,7 +741,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
         if (p >= cnt) break;
         float d1[cfg::kMt1][4], d2[cfg::kMt2][4];
 #pragma unroll
-        for (int ks = 0; ks < cfg::kKs1; ++ks) {
+        for (int ks = 0; ks < (BASIS ? cfg::kKs1 : 0); ++ks) {
           uint32_t b[4];
           ldsm_x4(tile + f_off + p * cfg::kFeatStride + ks * 32, b);
 #pragma unroll
@@ -777,7 +781,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
               if (w == CC || row2 + out_row(mt, kVec2) < w) red_add<kVec2>(df + c, v);
             }
 #pragma unroll
-            for (int mt = 0; mt < cfg::kMt1; mt += kVec1 / 2) {
+            for (int mt = 0; mt < (BASIS ? cfg::kMt1 : 0); mt += kVec1 / 2) {
               float v[kVec1];
 #pragma unroll
               for (int i = 0; i < kVec1; ++i) v[i] = d1[mt + i / 2][2 * (i % 2) + e];

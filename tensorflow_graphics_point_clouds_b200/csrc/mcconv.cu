@@ -23,6 +23,11 @@ int basis_proj_grads_blocks(cudaStream_t st, int K, int C, int64_t ns, int64_t M
                             const float* basis, const float* feat, const int32_t* neigh,
                             const int32_t* ranges, const float* in_grads, float* dbasis,
                             float* dfeat, int hidden);
+// basis_proj_tile.cu: the gradients of narrow layers (dbasis may be null)
+bool basis_proj_grads_tile_takes(int K, int C, const float* feat);
+int basis_proj_grads_tile(cudaStream_t st, int K, int C, int64_t ns, int64_t M, const float* basis,
+                          const float* feat, const int2* neigh, const int32_t* ranges,
+                          const float* in_grads, float* dbasis, float* dfeat, int hidden);
 // basis_proj_mma.cu: the projection on warp-level tensor-core MMAs
 bool basis_proj_mma_supported(int K, int C);
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
@@ -269,11 +274,13 @@ extern "C" int tfgpc_mcconv_backward(void* stream, int K, int C, int Cout, int64
                                       dbasis_out, dfeat_out, dweights_out, ws, ws_bytes);
 }
 
-extern "C" int tfgpc_mcconv_backward_blocks(
+// want_basis false: without the gradient of the basis (dbasis_out is null).
+static int backward_blocks(
     void* stream, int K, int C, int Cout, int groups, int k_src, int cout_src, int64_t ns,
     int64_t n_in, int64_t M, const float* basis, const float* features, const int32_t* neighbors,
     const int32_t* ranges, const float* weights, const float* out_grads, int x_in_workspace,
-    float* dbasis_out, float* dfeat_out, float* dweights_out, void* ws, size_t ws_bytes) {
+    bool want_basis, float* dbasis_out, float* dfeat_out, float* dweights_out, void* ws,
+    size_t ws_bytes) {
   int rc = check_mc_args("MCConvBackward", K, C, Cout, ns, n_in, M);
   if (rc) return rc;
   const Blocks blocks{groups, k_src, cout_src};
@@ -290,8 +297,8 @@ extern "C" int tfgpc_mcconv_backward_blocks(
     if (n_in > 0 && dfeat_out) TFGPC_CUDA(cudaMemsetAsync(dfeat_out, 0, sizeof(float) * (size_t)n_in * C, st));
     return TFGPC_OK;
   }
-  TFGPC_REQUIRE(basis && features && neighbors && ranges && out_grads && dbasis_out && dfeat_out && ws,
-                "MCConvBackward got a null pointer");
+  TFGPC_REQUIRE(basis && features && neighbors && ranges && out_grads &&
+                (dbasis_out || !want_basis) && dfeat_out && ws, "MCConvBackward got a null pointer");
   TFGPC_REQUIRE((uintptr_t)basis % 16 == 0 && (uintptr_t)out_grads % 16 == 0 &&
                 (uintptr_t)ws % 256 == 0,
                 "MCConvBackward expects 16-byte aligned buffers and a 256-byte aligned workspace");
@@ -302,7 +309,10 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   const int hidden = K / groups;
   const bool fs_ok = on_mma(w, features) && (uintptr_t)dbasis_out % 32 == 0 &&
                      (uintptr_t)dfeat_out % 16 == 0;
-  const bool image = fs_ok && groups == 1 && basis_proj_grads_tc_supported(K, C);
+  TFGPC_REQUIRE(want_basis || fs_ok || basis_proj_grads_tile_takes(K, C, features),
+                "MCConvBackwardFeatures expects 16-byte aligned features and feature gradients of a "
+                "supported layer");
+  const bool image = want_basis && fs_ok && groups == 1 && basis_proj_grads_tc_supported(K, C);
   // dX[ns, C*K] = dOut[ns, Cout] * W^T: B rows are W's rows, reduction over Cout
   GemmProblem px{};
   px.M = ns;
@@ -349,7 +359,7 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   pw.cleared = gemm_adds_slices(pw);
   if (pw.cleared) jobs.zero(pw.c, (size_t)ck * co * sizeof(float));
   jobs.zero(dfeat_out, (size_t)n_in * C * sizeof(float));
-  if (!fs_ok && basis_proj_grads_adds_dbasis(K, C, features))
+  if (want_basis && !fs_ok && basis_proj_grads_adds_dbasis(K, C, features))
     jobs.zero(dbasis_out, (size_t)M * K * sizeof(float));
   rc = prepare(st, jobs);
   if (rc) return rc;
@@ -382,9 +392,12 @@ extern "C" int tfgpc_mcconv_backward_blocks(
     if (fs_ok)
       rc = basis_proj_grads_mma(st, K, C, ns, M, basis, w.fs, neighbors, ranges, w.dx, dbasis_out,
                                 dfeat_out, hidden);
-    else
+    else if (want_basis)
       rc = basis_proj_grads_blocks(st, K, C, ns, M, basis, features, neighbors, ranges, w.dx,
                                    dbasis_out, dfeat_out, hidden);
+    else
+      rc = basis_proj_grads_tile(st, K, C, ns, M, basis, features, (const int2*)neighbors, ranges,
+                                 w.dx, nullptr, dfeat_out, hidden);
   }
   if (rc) return rc;
   rc = gemm_bf16x3(st, pw, w.err);
@@ -392,6 +405,35 @@ extern "C" int tfgpc_mcconv_backward_blocks(
   TFGPC_CUDA(launch_chained(st, blocks_for(weight_elems, 256), 256, 0, crop_weights_kernel,
       weight_elems, cout_src, Cout, k_src, K, w.dw_pad, dweights_out));
   return TFGPC_OK;
+}
+
+extern "C" int tfgpc_mcconv_backward_blocks(
+    void* stream, int K, int C, int Cout, int groups, int k_src, int cout_src, int64_t ns,
+    int64_t n_in, int64_t M, const float* basis, const float* features, const int32_t* neighbors,
+    const int32_t* ranges, const float* weights, const float* out_grads, int x_in_workspace,
+    float* dbasis_out, float* dfeat_out, float* dweights_out, void* ws, size_t ws_bytes) {
+  return backward_blocks(stream, K, C, Cout, groups, k_src, cout_src, ns, n_in, M, basis, features,
+                         neighbors, ranges, weights, out_grads, x_in_workspace, true, dbasis_out,
+                         dfeat_out, dweights_out, ws, ws_bytes);
+}
+
+// (the kernels that leave out the basis read and reduce 16-byte pieces beyond eight channels)
+extern "C" int tfgpc_mcconv_feature_grads_supported(int K, int C, const float* features,
+                                                    const float* dfeat) {
+  if (!valid_basis(K) || !valid_features(C)) return 0;
+  if (basis_proj_grads_tile_takes(K, C, features)) return 1;
+  return basis_proj_mma_supported(K, C) && (uintptr_t)features % 16 == 0 &&
+                 (uintptr_t)dfeat % 16 == 0 ? 1 : 0;
+}
+
+extern "C" int tfgpc_mcconv_backward_features(
+    void* stream, int K, int C, int Cout, int groups, int k_src, int cout_src, int64_t ns,
+    int64_t n_in, int64_t M, const float* basis, const float* features, const int32_t* neighbors,
+    const int32_t* ranges, const float* weights, const float* out_grads, int x_in_workspace,
+    float* dfeat_out, float* dweights_out, void* ws, size_t ws_bytes) {
+  return backward_blocks(stream, K, C, Cout, groups, k_src, cout_src, ns, n_in, M, basis, features,
+                         neighbors, ranges, weights, out_grads, x_in_workspace, false, nullptr,
+                         dfeat_out, dweights_out, ws, ws_bytes);
 }
 
 extern "C" int tfgpc_mcconv_grouped_supported(int K, int C) {

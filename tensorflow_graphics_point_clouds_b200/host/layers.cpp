@@ -254,7 +254,7 @@ Tensor project_forward(int k, int c, int cout, int groups, int k_src, int cout_s
 py::tuple project_backward(int k, int c, int cout, int groups, int k_src, int cout_src,
                            const Tensor& ws, const Tensor& basis_, const Tensor& features_,
                            const Tensor& neigh_, const Tensor& ranges_, const Tensor& weights_,
-                           const Tensor& out_grads_, bool reuse) {
+                           const Tensor& out_grads_, bool reuse, bool want_basis) {
   Tensor basis = f32(basis_), features = f32(features_), neigh = i32(neigh_), ranges = i32(ranges_),
          weights = f32(weights_), g = f32(out_grads_);
   check_pairs(k, basis, neigh);
@@ -262,8 +262,16 @@ py::tuple project_backward(int k, int c, int cout, int groups, int k_src, int co
                    weight_elems(k, c, cout, groups, k_src, cout_src), features);
   require(g.numel() == ranges.size(0) * (groups > 1 ? cout : cout_src),
           "MCConv expects one gradient per output feature of every sample");
-  Tensor dbasis = at::empty_like(basis), dfeat = at::empty_like(features),
-         dw = at::empty_like(weights);
+  Tensor dfeat = at::empty_like(features), dw = at::empty_like(weights);
+  if (!want_basis && tfgpc_mcconv_feature_grads_supported(k, c, fp(features), fp(dfeat))) {
+    check(tfgpc_mcconv_backward_features(stream(), k, c, cout, groups, k_src, cout_src,
+                                         ranges.size(0), features.size(0), basis.size(0), fp(basis),
+                                         fp(features), ip(neigh), ip(ranges), fp(weights), fp(g),
+                                         reuse, fpm(dfeat), fpm(dw), ws.data_ptr(),
+                                         (size_t)ws.numel()));
+    return py::make_tuple(py::none(), dfeat, dw);
+  }
+  Tensor dbasis = at::empty_like(basis);
   check(tfgpc_mcconv_backward_blocks(stream(), k, c, cout, groups, k_src, cout_src,
                                      ranges.size(0), features.size(0), basis.size(0), fp(basis),
                                      fp(features), ip(neigh), ip(ranges), fp(weights), fp(g), reuse,

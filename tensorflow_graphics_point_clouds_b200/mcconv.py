@@ -58,7 +58,8 @@ class ProjectionGemm:
     return out
 
   def backward(self, basis, features, neighbors, ranges, weights, out_grads, reuse_forward=True,
-               blocks=None):
+               blocks=None, want_basis=True):
+    """(dbasis, dfeat, dweights); want_basis=False: dbasis is not needed and may be None."""
     if not self.backward_ws:
       raise RuntimeError("this ProjectionGemm was created without backward workspace")
     self._ensure_workspace(features.shape[0])
@@ -66,7 +67,7 @@ class ProjectionGemm:
     groups, k_src, cout_src = blocks or (1, self.k, self.cout)
     return _lib.host().project_backward(self.k, self.c, self.cout, groups, k_src, cout_src, self.ws,
                                         basis, features, neighbors, ranges, weights, out_grads,
-                                        reuse)
+                                        reuse, bool(want_basis))
 
   def forward_grouped(self, basis_pair, features, weights, order, plan):
     """The forward pass through tfgpc_mcconv_forward_grouped: the projection runs
@@ -419,13 +420,17 @@ class _ProjectedConv:
     return out[:, :self.cout] if self.cout_pad != self.cout else out
 
   def _backward(self, out_grads):
+    return self._gradients(out_grads)
+
+  def _gradients(self, out_grads, **options):
     neigh, basis, features, weights = self._saved
     return self._op.backward(basis, features, neigh._original_neigh_ids,
                              neigh._samples_neigh_ranges, weights, out_grads,
-                             blocks=(1, self.k, self.cout))
+                             blocks=(1, self.k, self.cout), **options)
 
 
 _LIBRARY_NEIGHBORHOOD = _ProjectedConv._neighborhood
+_LIBRARY_BACKWARD = _ProjectedConv._backward
 
 
 class KPConv(_ProjectedConv):
@@ -452,7 +457,10 @@ class KPConv(_ProjectedConv):
   def backward(self, out_grads):
     """(d_features, d_weights) of the last forward call; the kernel points of the
     rigid layer are not trained."""
-    _, dfeat, dw = self._backward(out_grads)
+    if _is_own(self._backward, _LIBRARY_BACKWARD):
+      _, dfeat, dw = self._gradients(out_grads, want_basis=False)
+    else:
+      _, dfeat, dw = self._backward(out_grads)
     return dfeat, dw
 
 
