@@ -28,7 +28,7 @@ int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __n
   typedef bpm::Cfg<K, CC> cfg;
   auto kern = bpm::basis_proj_mma_kernel<K, CC, OUT>;
   constexpr int smem = cfg::kFwdWarps * cfg::kFwdWarpBytes;
-  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  TFGPC_CUDA((allow_shared<bpm::basis_proj_mma_kernel<K, CC, OUT>>(smem)));
   Shape s = walk_shape(ns, cfg::kFwdWarps);
   // few samples: the channel passes run side by side
   const int passes = (C + CC - 1) / CC;
@@ -47,7 +47,7 @@ int launch_grads(cudaStream_t st, int C, int64_t ns, int64_t M, const float* bas
   typedef bpm::GradCfg<K, CC, BASIS> cfg;
   auto kern = bpm::basis_proj_grads_mma_kernel<K, CC, BASIS>;
   constexpr int smem = cfg::kTeams * cfg::kTeamBytes;
-  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  TFGPC_CUDA((allow_shared<bpm::basis_proj_grads_mma_kernel<K, CC, BASIS>>(smem)));
   // few samples with long lists: several teams share a sample's chunks
   const int64_t teams = (int64_t)sm_count() * cfg::kTeams;
   int64_t parts = ns > 0 ? 2 * teams / ns : 1;

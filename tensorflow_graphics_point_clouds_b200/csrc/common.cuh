@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "tfgpc.h"
 
 namespace tfgpc {
@@ -65,6 +67,21 @@ struct ProfPause {
 
 // Number of SMs of the current device (cached per device).
 int sm_count();
+
+// Lets a kernel take `bytes` of dynamic shared memory: asked of the driver once per device
+// and size (every launch of a product or projection asked again, 0.6 us each).
+template <auto kKernel>
+cudaError_t allow_shared(int bytes) {
+  static std::atomic<int> allowed[64];      // (the most so far)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const bool known = dev >= 0 && dev < 64;
+  if (known && bytes <= allowed[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && known) allowed[dev].store(bytes, std::memory_order_relaxed);
+  return e;
+}
 
 // Blocking read of a few values (4 .. 4096 bytes, a multiple of 4) from device
 // memory, through mapped pinned host memory instead of a copy engine: it does

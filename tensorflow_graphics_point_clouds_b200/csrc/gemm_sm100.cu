@@ -498,7 +498,7 @@ int launch(cudaStream_t st, const CUtensorMap* maps, int64_t M, int64_t N, int b
   auto kern = gemm_bf16x3_kernel<A_MN, B_MN, OUT>;
   const int stages = stages_for(bn);
   const size_t smem = (size_t)stages * stage_bytes(bn) + kFixedBytes;
-  TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  TFGPC_CUDA((allow_shared<gemm_bf16x3_kernel<A_MN, B_MN, OUT>>((int)smem)));
   const int64_t tiles = (int64_t)sch.m_tiles * sch.n_tiles * sch.batches * sch.k_splits;
   const int grid = tiles < sm_count() ? (int)tiles : sm_count();
   ProfScope prof(st, OUT == 4 ? "gemm_bf16x3_mn_k_scatter" : OUT == 3 ? "gemm_bf16x3_mn_k_image"

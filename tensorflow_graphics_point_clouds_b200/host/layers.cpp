@@ -63,13 +63,12 @@ py::tuple kernel_basis_grads(const Tensor& p_in_, const Tensor& p_out_, const Te
   Tensor pdf_keep;
   const float* pdf = maybe(pdf_, &pdf_keep);
   const OneLayer mlp(w1);
-  Tensor both = empty({mlp.d + 1, mlp.k}, at::kFloat, p_in);
-  float* dw = fpm(both);
+  Tensor dw = empty(w1.sizes(), at::kFloat, p_in), db = empty({mlp.k}, at::kFloat, p_in);
   check(tfgpc_kernel_basis_mlps_grads(stream(), mlp.d, mlp.k, mlp.g, neigh.size(0), fp(p_in),
                                       fp(p_out), ip(neigh), pdf, fp(w1), fp(b1),
                                       (float)(1.0 / radius), act, (float)alpha, pdf_mode,
-                                      fp(dbasis), dw, dw + (int64_t)mlp.d * mlp.k));
-  return py::make_tuple(both.narrow(0, 0, mlp.d).view(w1.sizes()), both.select(0, mlp.d));
+                                      fp(dbasis), fpm(dw), fpm(db)));
+  return py::make_tuple(dw, db);
 }
 
 // Parameters of a kernel MLP, one tensor per layer: weights [G, H_{l-1}, H_l], biases

@@ -9,6 +9,8 @@ their gradients as another (tfgpc_mcconv_backward); the kernel MLP runs as one
 kernel per direction (tfgpc_kernel_basis*, or tfgpc_kernel_mlp_* for more hidden
 layers and point gradients).
 """
+import functools
+
 import torch
 
 from . import _lib
@@ -195,6 +197,7 @@ NON_LINEARITIES = {'relu': (0, 0.0), 'lrelu': (0, 0.2), 'leakyrelu': (0, 0.2),
                    'leaky_relu': (0, 0.2), 'elu': (1, 0.0)}
 
 
+@functools.lru_cache(maxsize=256)
 def _grouped_supported(k, c):
   return _lib.lib().tfgpc_mcconv_grouped_supported(c_int(k), c_int(c)) != 0
 

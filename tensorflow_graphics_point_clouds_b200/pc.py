@@ -30,6 +30,10 @@ _DIMS_CACHE = {}
 
 def _to_dims(value, dims, device, inverse=False):
   """value per dimension as a device tensor, or (inverse) its float32 reciprocal."""
+  if type(value) is float:
+    t = _DIMS_CACHE.get((value, dims, device, inverse))
+    if t is not None:
+      return t
   if not torch.is_tensor(value):
     flat = [float(v) for v in (value if hasattr(value, '__len__') else [value])]
     key = (tuple(flat), dims, device, inverse)
@@ -40,6 +44,8 @@ def _to_dims(value, dims, device, inverse=False):
       t = torch.tensor(flat * dims if len(flat) == 1 else flat, dtype=torch.float32)
       t = (torch.reciprocal(t) if inverse else t).to(device)
       _DIMS_CACHE[key] = t
+    if type(value) is float:
+      _DIMS_CACHE[value, dims, device, inverse] = t
     return t
   if inverse:
     return torch.reciprocal(_to_dims(value, dims, device))
@@ -51,9 +57,15 @@ def _to_dims(value, dims, device, inverse=False):
 
 def _host_dims(value, dims):
   """value per dimension as a list of floats (a device tensor costs a blocking read)."""
+  if type(value) is float:
+    return [value] * dims
   flat = (value.detach().reshape(-1).cpu().tolist() if torch.is_tensor(value) else
           [float(v) for v in (value if hasattr(value, '__len__') else [value])])
   return flat * dims if len(flat) == 1 else flat
+
+
+def _is_array(t, dtype):
+  return type(t) is torch.Tensor and t.dtype is dtype and t.is_contiguous()
 
 
 class PointCloud:
@@ -66,9 +78,12 @@ class PointCloud:
     # and returns the maximum over all shards (dist.allreduce_max_), so that every
     # rank builds the keys the unsharded batch would have.
     self._num_cells_reduce = num_cells_reduce
-    self._points = torch.as_tensor(points).to(torch.float32).contiguous()
-    self._batch_ids = torch.as_tensor(batch_ids, device=self._points.device).to(
-        torch.int32).contiguous()
+    # (arrays that are what the ops take already, as the output of one is, are looked at once)
+    if not _is_array(points, torch.float32):
+      points = torch.as_tensor(points).to(torch.float32).contiguous()
+    if not (_is_array(batch_ids, torch.int32) and batch_ids.device == points.device):
+      batch_ids = torch.as_tensor(batch_ids, device=points.device).to(torch.int32).contiguous()
+    self._points, self._batch_ids = points, batch_ids
     if batch_size is None:
       batch_size = int(ops.read_device(self._batch_ids.max().reshape(1))[0]) + 1
     self._batch_size = int(batch_size)
@@ -336,6 +351,9 @@ class Neighborhood:
       # a self neighborhood mostly feeds the density estimate and the sampling,
       # which read sorted ids only: the original-id list is built if asked for
       self._nbrs = ops.find_neighbors_fill(self._count)
+    elif self._grid._cells is not None:
+      # (the permutation is not needed as a tensor)
+      self._nbrs, self._orig_ids = ops._cells_fill(self._count, True, None, None)
     else:
       self._nbrs, self._orig_ids = ops.find_neighbors_fill(self._count,
                                                             self._grid._sorted_indices)
