@@ -21,14 +21,14 @@ Shape walk_shape(int64_t items, int warps) {
   return s;
 }
 
-template <int K, int CC, int OUT>
+template <int K, int CC, int OUT, bool BLOCKS>
 int launch_fwd(cudaStream_t st, int C, int64_t ns, const float* basis, const __nv_bfloat16* fs,
                const int2* neigh, const int32_t* ranges, float* out, __nv_bfloat16* hi,
                __nv_bfloat16* mid, int hidden) {
   typedef bpm::Cfg<K, CC> cfg;
-  auto kern = bpm::basis_proj_mma_kernel<K, CC, OUT>;
+  auto kern = bpm::basis_proj_mma_kernel<K, CC, OUT, BLOCKS>;
   constexpr int smem = cfg::kFwdWarps * cfg::kFwdWarpBytes;
-  TFGPC_CUDA((allow_shared<bpm::basis_proj_mma_kernel<K, CC, OUT>>(smem)));
+  TFGPC_CUDA((allow_shared<bpm::basis_proj_mma_kernel<K, CC, OUT, BLOCKS>>(smem)));
   Shape s = walk_shape(ns, cfg::kFwdWarps);
   // few samples: the channel passes run side by side
   const int passes = (C + CC - 1) / CC;
@@ -85,8 +85,11 @@ bool basis_proj_mma_supported(int K, int C) {
 int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                          const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                          __nv_bfloat16* hi, __nv_bfloat16* mid, int hidden) {
-  TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 1>(st, C, ns, basis, fs, (const int2*)neigh,
-                                                      ranges, nullptr, hi, mid, hidden))
+  TFGPC_CC_SWITCH(K, C, return hidden == kK
+      ? launch_fwd<kK, kCC, 1, false>(st, C, ns, basis, fs, (const int2*)neigh, ranges, nullptr, hi,
+                                      mid, hidden)
+      : launch_fwd<kK, kCC, 1, true>(st, C, ns, basis, fs, (const int2*)neigh, ranges, nullptr, hi,
+                                     mid, hidden))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }
 
@@ -94,7 +97,7 @@ int basis_proj_mma_split(cudaStream_t st, int K, int C, int64_t ns, const float*
 int basis_proj_mma_f32(cudaStream_t st, int K, int C, int64_t ns, const float* basis,
                        const __nv_bfloat16* fs, const int32_t* neigh, const int32_t* ranges,
                        float* out) {
-  TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 0>(st, C, ns, basis, fs, (const int2*)neigh,
+  TFGPC_CC_SWITCH(K, C, return launch_fwd<kK, kCC, 0, false>(st, C, ns, basis, fs, (const int2*)neigh,
                                                       ranges, out, nullptr, nullptr, kK))
   return fail(TFGPC_EINVAL, "tensor-core projection expects 16, 32 or 64 basis functions");
 }

@@ -93,6 +93,22 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
                : "memory");
 }
 
+// What is done under a condition here is predicated, not branched around: with a branch each,
+// and 64-bit products for the addresses, a copied row came to 28 instructions and a reduced one
+// to 58, of 390 to 610 per chunk.  65 536 samples of 33 pairs, us before -> now: forward K = 16,
+// C = 32 106 -> 84, C = 64 137 -> 122, K = 32, C = 64 218 -> 205; gradients 152 -> 140, 249 -> 237,
+// 392 -> 385.
+__device__ __forceinline__ void cp_async16_if(uint32_t dst, const void* src, bool ok) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n"
+               "@p cp.async.cg.shared.global [%0], [%1], 16;\n}" ::"r"(dst), "l"(src),
+               "r"((uint32_t)ok) : "memory");
+}
+
+// p + i * bytes, as one wide multiply-add
+__device__ __forceinline__ const uint8_t* row_at(const uint8_t* p, int i, uint32_t bytes) {
+  return p + (uint64_t)(uint32_t)i * bytes;
+}
+
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 template <int N>
@@ -184,15 +200,15 @@ __device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat1
   constexpr int kRpi = 32 / (2 * kLph);        // rows per warp instruction
   const int sub = lane % (2 * kLph), rsub = lane / (2 * kLph);
   const int half = sub / kLph, seg = sub % kLph;
-  const bool seg_ok = seg * 8 < w;
-  const uint32_t dst0 = tile + half * (cfg::kCC * 2) + seg * 16;
-  const int64_t src0 = (int64_t)half * C + c0 + seg * 8;
+  const int have = seg * 8 < w ? cnt : 0;      // (a lane without channels: zeros)
+  const uint32_t dst0 = tile + half * (cfg::kCC * 2) + seg * 16 + rsub * cfg::kFeatStride;
+  const uint8_t* const src0 = reinterpret_cast<const uint8_t*>(fs + (half * C + c0 + (seg * 8 < w ? seg * 8 : 0)));
+  const uint32_t stride = 4u * (uint32_t)C;
 #pragma unroll
   for (int it = 0; it < kChunk / kRpi; ++it) {
-    const int row = it * kRpi + rsub;
-    const int j = __shfl_sync(0xffffffffu, idx, row);
-    if (seg_ok)
-      cp_async16_zfill(dst0 + row * cfg::kFeatStride, fs + (int64_t)j * 2 * C + src0, row < cnt);
+    const int j = __shfl_sync(0xffffffffu, idx, it * kRpi + rsub);
+    cp_async16_zfill(dst0 + it * kRpi * cfg::kFeatStride, row_at(src0, j, stride),
+                     it * kRpi + rsub < have);
   }
 }
 
@@ -246,8 +262,8 @@ __device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float
 // into two bf16 arrays [ns, C*K] (left operand of the tensor-core GEMM).
 // The passes over the channels are dealt to gridDim.y.  The columns of a row lie in the
 // order of block_offset: 2^shift = K is the op's (c, k), less are the blocks of several
-// kernel MLPs, one after the other.
-template <int K, int CC, int OUT>
+// kernel MLPs, one after the other (BLOCKS: without them a row's places are constants).
+template <int K, int CC, int OUT, bool BLOCKS>
 __global__ void __launch_bounds__(Cfg<K, CC>::kFwdWarps * 32, 1)
 basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
                       const __nv_bfloat16* fs, const int2* neigh,
@@ -362,7 +378,8 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
       }
       if (cur.last) {
         // lane (g, q): channels c0 + 16*mt + g (+8), basis functions 16*j + 4*q .. +3
-        const int64_t obase = cur.s * C * K + ((c0 + g) << shift);
+        const int sh = BLOCKS ? shift : K == 16 ? 4 : K == 32 ? 5 : 6;
+        const int64_t obase = cur.s * C * K + ((c0 + g) << sh) + (BLOCKS ? 0 : 4 * q);
 #pragma unroll
         for (int mt = 0; mt < cfg::kMT; ++mt) {
           if (mt < mt_cnt) {
@@ -371,8 +388,9 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
 #pragma unroll
               for (int h = 0; h < 2; ++h) {   // rows g and g + 8
                 const int k = 16 * j + 4 * q;
-                const int64_t o = obase + (((k >> shift) * C + 16 * mt + 8 * h) << shift) +
-                                  (k & ((1 << shift) - 1));
+                const int64_t o = obase + (BLOCKS ? (((k >> sh) * C + 16 * mt + 8 * h) << sh) +
+                                                        (k & ((1 << sh) - 1))
+                                                  : ((16 * mt + 8 * h) << sh) + 16 * j);
                 if (OUT == 0) {
                   *reinterpret_cast<float4*>(out + o) =
                       make_float4(acc[mt][2 * j][2 * h], acc[mt][2 * j][2 * h + 1],
@@ -462,13 +480,27 @@ __device__ __forceinline__ void mma16816_first(float* d, const uint32_t* a, uint
 }
 
 template <int N>
-__device__ __forceinline__ void red_add(float* dst, const float* v) {
+__device__ __forceinline__ void red_add_if(float* dst, const float* v, bool ok) {
   if (N == 4)
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]), "f"(v[1]),
-                 "f"(v[2]), "f"(v[N - 1]) : "memory");
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n"
+                 "@p red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"l"(dst), "f"(v[0]),
+                 "f"(v[1]), "f"(v[N / 2]), "f"(v[N - 1]), "r"((uint32_t)ok) : "memory");
   else
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(v[0]), "f"(v[1])
-                 : "memory");
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n"
+                 "@p red.global.add.v2.f32 [%0], {%1, %2};\n}" ::"l"(dst), "f"(v[0]), "f"(v[1]),
+                 "r"((uint32_t)ok) : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void store_if(float* dst, const float* v, bool ok) {
+  if (N == 4)
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n"
+                 "@p st.global.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"l"(dst), "f"(v[0]), "f"(v[1]),
+                 "f"(v[N / 2]), "f"(v[N - 1]), "r"((uint32_t)ok) : "memory");
+  else
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n"
+                 "@p st.global.v2.f32 [%0], {%1, %2};\n}" ::"l"(dst), "f"(v[0]), "f"(v[1]),
+                 "r"((uint32_t)ok) : "memory");
 }
 
 // The chunks of a team, one after the other (see Walker; an item without pairs is left out).
@@ -615,7 +647,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
     const int seg = lane % kSeg, half_row = lane / kSeg % 2, row0 = sub * kRpi + lane / (2 * kSeg);
     const uint32_t f_dst = smem_addr(mem) + cfg::kRawBytes + row0 * cfg::kFeatStride +
                            half_row * (CC * 2) + seg * 16;
-    const __nv_bfloat16* const f_src = fs + (int64_t)half_row * C + c0 + seg * 8;
+    const uint8_t* const f_src = reinterpret_cast<const uint8_t*>(fs + ((int64_t)half_row * C + c0 + seg * 8));
     const int row_limit = seg * 8 < w ? row0 : kChunk;      // a lane without channels: no row
     auto issue_rows = [&](int st, const Chunk& j, int idx) {
       const uint32_t dst = f_dst + st * cfg::kStageBytes;
@@ -623,8 +655,8 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
 #pragma unroll
       for (int it = 0; it < kChunk / kRpi / W; ++it) {
         const int p = __shfl_sync(0xffffffffu, idx, it * W * kRpi + row0);
-        if (row_limit + it * W * kRpi < cnt)
-          cp_async16(dst + it * W * kRpi * cfg::kFeatStride, f_src + (int64_t)p * (2 * C));
+        cp_async16_if(dst + it * W * kRpi * cfg::kFeatStride, row_at(f_src, p, 4u * (uint32_t)C),
+                      row_limit + it * W * kRpi < cnt);
       }
     };
     // basis rows: float4 number tid + 32 W t of the chunk
@@ -682,6 +714,7 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
     uint32_t a2h[cfg::kMt2][cfg::kKs2][4], a2m[cfg::kMt2][cfg::kKs2][4];
     float* const db_lane = dbasis + row1 + out_row(0, kVec1) + 2 * q * K;
     float* const df_lane = dfeat + c0 + row2 + out_row(0, kVec2);
+    const int channels = w - (row2 + out_row(0, kVec2));      // from the lane's first one on
     int st = 0;
     while (cur.valid()) {
       // the rows of this chunk have landed, and dX if it is the item's first; the other
@@ -770,29 +803,26 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int pt = __shfl_sync(0xffffffffu, idx0, p + 2 * q + e);
-          if (p + 2 * q + e < cnt) {
-            float* const df = df_lane + (int64_t)pt * C;
+          const bool ok = p + 2 * q + e < cnt;
+          float* const df = (float*)row_at((const uint8_t*)df_lane, pt, 4u * (uint32_t)C);
 #pragma unroll
-            for (int mt = 0; mt < cfg::kMt2; mt += kVec2 / 2) {
-              float v[kVec2];
+          for (int mt = 0; mt < cfg::kMt2; mt += kVec2 / 2) {
+            float v[kVec2];
 #pragma unroll
-              for (int i = 0; i < kVec2; ++i) v[i] = d2[mt + i / 2][2 * (i % 2) + e];
-              const int c = out_row(mt, kVec2) - out_row(0, kVec2);
-              if (w == CC || row2 + out_row(mt, kVec2) < w) red_add<kVec2>(df + c, v);
-            }
+            for (int i = 0; i < kVec2; ++i) v[i] = d2[mt + i / 2][2 * (i % 2) + e];
+            const int c = out_row(mt, kVec2) - out_row(0, kVec2);
+            red_add_if<kVec2>(df + c, v, ok && c < channels);
+          }
 #pragma unroll
-            for (int mt = 0; mt < (BASIS ? cfg::kMt1 : 0); mt += kVec1 / 2) {
-              float v[kVec1];
+          for (int mt = 0; mt < (BASIS ? cfg::kMt1 : 0); mt += kVec1 / 2) {
+            float v[kVec1];
 #pragma unroll
-              for (int i = 0; i < kVec1; ++i) v[i] = d1[mt + i / 2][2 * (i % 2) + e];
-              float* dst = db + (p + e) * K + (out_row(mt, kVec1) - out_row(0, kVec1));
-              if (c0 > 0)      // (a load of the pass before's sum would stall the warp)
-                red_add<kVec1>(dst, v);
-              else if (kVec1 == 4)
-                *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[kVec1 - 1]);
-              else
-                *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
-            }
+            for (int i = 0; i < kVec1; ++i) v[i] = d1[mt + i / 2][2 * (i % 2) + e];
+            float* dst = db + (p + e) * K + (out_row(mt, kVec1) - out_row(0, kVec1));
+            if (c0 > 0)      // (a load of the pass before's sum would stall the warp)
+              red_add_if<kVec1>(dst, v, ok);
+            else
+              store_if<kVec1>(dst, v, ok);
           }
         }
       }
