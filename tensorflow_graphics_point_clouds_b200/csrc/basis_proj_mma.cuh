@@ -15,9 +15,8 @@
 // lane and handed to the MMAs by ldmatrix, never touching registers in between.
 //
 // Shared-memory rows are padded by 16 bytes so that the eight row reads of one
-// ldmatrix fall into distinct bank groups.  Basis functions are stored in a
-// permuted order inside every group of 16 (position 8*t + 2*a + b holds
-// k = 4*a + 2*t + b): the two accumulator tiles of a tile pair then give every
+// ldmatrix fall into distinct bank groups.  Column 2a + b of the tile t of a pair of basis
+// tiles stands for basis function 4a + 2t + b: the two accumulator tiles then give every
 // lane four consecutive k (or channels), i.e. 128-bit stores and reductions.
 #pragma once
 
@@ -41,11 +40,10 @@ struct Cfg {
   static constexpr int kNT = K / 8;      // 8-wide basis tiles
   static constexpr int kNTP = K / 16;    // tile pairs
   static constexpr int kFeatStride = kCC * 4 + 16;  // bytes: hi[kCC] | mid[kCC] | pad
-  static constexpr int kKStride = K * 2 + 16;       // bytes of one bf16 row over k (+ pad)
+  static constexpr int kBasisStride = K + 4;        // floats of a basis row (+ pad)
   static constexpr int kFeatBytes = kChunk * kFeatStride;
-  static constexpr int kBasisBytes = 2 * kChunk * kKStride;   // hi rows, then mid rows
+  static constexpr int kBasisBytes = kChunk * kBasisStride * 4;
   static constexpr int kFwdWarpBytes = 2 * kFeatBytes + 2 * kBasisBytes;
-  static constexpr int kBasisVecs = K / 8;   // float4 loads per lane for a 16-row basis chunk
   // warps per block (one block per SM): what 64 K registers and 227 KB allow
   static constexpr int kFwdRegWarps = CC * K >= 2048 ? 12 : CC * K >= 1024 ? 16 : 24;
   static constexpr int kMaxSmem = 227 * 1024;
@@ -212,52 +210,42 @@ __device__ __forceinline__ void issue_features(uint32_t tile, const __nv_bfloat1
   }
 }
 
-// Basis rows of a chunk, 16 x K floats contiguous in memory: each lane loads
-// K/8 float4 (zeros beyond the chunk) ...
+// Starts the copy of a chunk's basis rows, 16 x K floats contiguous in memory (zeros beyond
+// the chunk).
 template <int K>
-__device__ __forceinline__ void load_basis(const float* basis, int base, int cnt,
-                                           int lane, float4* v) {
-  const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)base * K);
+__device__ __forceinline__ void issue_basis(uint32_t tile, const float* basis, int base, int cnt,
+                                            int lane) {
+  const float* src = basis + (int64_t)base * K + lane * 4;
 #pragma unroll
   for (int t = 0; t < K / 8; ++t) {
-    const int i = lane + 32 * t;
-    v[t] = (i / (K / 4) < cnt) ? ld_global(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int row = (lane + 32 * t) / (K / 4), a4 = lane % (K / 4);
+    cp_async16_zfill(tile + (row * (K + 4) + a4 * 4) * 4, src + 128 * t, row < cnt);
   }
 }
 
-// Writes four consecutive k (4*a4 .. 4*a4+3) of one row, split into hi and mid,
-// at their permuted positions.
+// The right operand of tile pair j out of a chunk's basis rows: rows 2q, 2q + 1 and, eight
+// further on, of the column that the tiles' column g stands for, split.
 template <int K>
-__device__ __forceinline__ void store_split4(uint8_t* hi_row, uint8_t* mid_row, int a4,
-                                             const float4& v) {
-  uint32_t h01, m01, h23, m23;
-  split2(v.x, v.y, h01, m01);
-  split2(v.z, v.w, h23, m23);
-  const int off = (16 * (a4 >> 2) + 2 * (a4 & 3)) * 2;  // bytes
-  *reinterpret_cast<uint32_t*>(hi_row + off) = h01;
-  *reinterpret_cast<uint32_t*>(hi_row + off + 16) = h23;
-  *reinterpret_cast<uint32_t*>(mid_row + off) = m01;
-  *reinterpret_cast<uint32_t*>(mid_row + off + 16) = m23;
-}
-
-// ... and stores them split into the chunk's basis tile (hi rows, then mid rows).
-template <int K>
-__device__ __forceinline__ void store_basis(uint8_t* tile, int lane, const float4* v) {
-  constexpr int kKStride = K * 2 + 16;
+__device__ __forceinline__ void basis_operand(const float* tile, int j, int g, int q, uint32_t* hi,
+                                              uint32_t* mid) {
+  const float* p = tile + 2 * q * (K + 4) + 16 * j + 4 * (g >> 1) + (g & 1);
 #pragma unroll
-  for (int t = 0; t < K / 8; ++t) {
-    const int i = lane + 32 * t;
-    const int row = i / (K / 4), a4 = i % (K / 4);
-    store_split4<K>(tile + row * kKStride, tile + (kChunk + row) * kKStride, a4, v[t]);
-  }
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+      split2(p[8 * half * (K + 4) + 2 * t], p[(8 * half + 1) * (K + 4) + 2 * t], hi[2 * t + half],
+             mid[2 * t + half]);
 }
 
 // ---- forward ---------------------------------------------------------------------------
 //
 // X[s] as D[c, k] += A[c, pair] * B[pair, k] per chunk: A comes transposed out of
-// the gathered feature rows (ldmatrix.trans), B transposed out of the staged
-// basis rows.  Features of chunk i+1 are in flight, and its basis rows and the
-// indices of chunk i+2 are on their way to registers, while chunk i is multiplied.
+// the gathered feature rows (ldmatrix.trans), B out of the basis rows, split on the way to
+// registers.  Features and basis rows of chunk i+1 are in flight, and the indices of chunk
+// i+2 are on their way to registers, while chunk i is multiplied.  (The basis rows by
+// registers, split and stored for ldmatrix at the end of a chunk, had the warp wait for them
+// there.  65 536 samples of 33 pairs, us before -> now: forward K = 16, C = 32 84 -> 79, K = 32,
+// C = 32 134 -> 114, C = 64 205 -> 183 to 203; gradients 140 -> 133, 212 -> 192, 385 -> 342 to 383.)
 // OUT = 0: fp32 [ns, C, K] (the op's output).  OUT = 1: the same values split
 // into two bf16 arrays [ns, C*K] (left operand of the tensor-core GEMM).
 // The passes over the channels are dealt to gridDim.y.  The columns of a row lie in the
@@ -278,14 +266,15 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
   uint8_t* wsm = bpm_smem + (size_t)warp_in_block * cfg::kFwdWarpBytes;
   // two feature tiles, then two basis tiles
   auto feat_tile = [&](int b) { return wsm + b * cfg::kFeatBytes; };
-  auto basis_tile = [&](int b) { return wsm + 2 * cfg::kFeatBytes + b * cfg::kBasisBytes; };
+  auto basis_tile = [&](int b) {
+    return reinterpret_cast<float*>(wsm + 2 * cfg::kFeatBytes + b * cfg::kBasisBytes);
+  };
   const int64_t warp = (int64_t)blockIdx.x * warps_per_block + warp_in_block;
   const int64_t warps = (int64_t)gridDim.x * warps_per_block;
   const int g = lane >> 2, q = lane & 3;
   const int mi = lane >> 3, r = lane & 7;
   // ldmatrix row addresses (bytes inside a tile) of this lane
   const uint32_t a_off = (r + 8 * (mi >> 1)) * cfg::kFeatStride + 8 * (mi & 1) * 2;
-  const uint32_t b_off = (r + 8 * (mi & 1)) * cfg::kKStride + 8 * (mi >> 1) * 2;
 
   for (int c0 = blockIdx.y * cfg::kCC; c0 < C; c0 += gridDim.y * cfg::kCC) {
     const int w = min(cfg::kCC, C - c0);
@@ -298,22 +287,19 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
     if (cur.valid()) {
       const int idx0 = load_idx(cur, neigh, lane);
       issue_features<K, CC>(smem_addr(feat_tile(0)), fs, C, c0, w, idx0, cur.cnt, lane);
-      float4 bv[cfg::kBasisVecs];
-      load_basis<K>(basis, cur.base, cur.cnt, lane, bv);
-      store_basis<K>(basis_tile(0), lane, bv);
+      issue_basis<K>(smem_addr(basis_tile(0)), basis, cur.base, cur.cnt, lane);
     }
     cp_commit();
     float acc[cfg::kMT][cfg::kNT][4];
     int buf = 0;
     while (cur.valid()) {
       const int idx2 = load_idx(n2, neigh, lane);
-      float4 bv[cfg::kBasisVecs];
       if (n1.valid()) {
         issue_features<K, CC>(smem_addr(feat_tile(buf ^ 1)), fs, C, c0, w, idx1, n1.cnt, lane);
-        load_basis<K>(basis, n1.base, n1.cnt, lane, bv);
+        issue_basis<K>(smem_addr(basis_tile(buf ^ 1)), basis, n1.base, n1.cnt, lane);
       }
       cp_commit();
-      cp_wait<1>();   // the features of `cur` have landed
+      cp_wait<1>();   // the rows of `cur` have landed
       __syncwarp();
       if (cur.first) {
 #pragma unroll
@@ -325,7 +311,7 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
       }
       if (cur.cnt > 0) {
         const uint32_t ft = smem_addr(feat_tile(buf)) + a_off;
-        const uint32_t bt = smem_addr(basis_tile(buf)) + b_off;
+        const float* const bt = basis_tile(buf);
         // The basis operands, all at once where several channel tiles use them.  (Held for a
         // single pair of tiles, the 32 of K = 64 spilled: 241 us for 33 000 samples at C = 32,
         // 106 without.)
@@ -333,10 +319,8 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
         constexpr int kHeld = kHold ? cfg::kNTP : 1;
         uint32_t bh[kHeld][4], bm[kHeld][4];
 #pragma unroll
-        for (int j = 0; j < cfg::kNTP && kHold; ++j) {
-          ldsm_x4_t(bt + j * 32, bh[j % kHeld]);
-          ldsm_x4_t(bt + kChunk * cfg::kKStride + j * 32, bm[j % kHeld]);
-        }
+        for (int j = 0; j < cfg::kNTP && kHold; ++j)
+          basis_operand<K>(bt, j, g, q, bh[j % kHeld], bm[j % kHeld]);
         // Two 16-channel tiles at a time, and pass by pass over all their
         // accumulator tiles: consecutive MMAs never touch the same accumulator,
         // so none of them waits for the one before it.
@@ -353,10 +337,7 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
             }
 #pragma unroll
             for (int j0 = 0; j0 < cfg::kNTP; j0 += kHeld) {
-              if (!kHold) {
-                ldsm_x4_t(bt + j0 * 32, bh[0]);
-                ldsm_x4_t(bt + kChunk * cfg::kKStride + j0 * 32, bm[0]);
-              }
+              if (!kHold) basis_operand<K>(bt, j0, g, q, bh[0], bm[0]);
 #pragma unroll
               for (int pass = 0; pass < 3; ++pass) {
 #pragma unroll
@@ -407,7 +388,6 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
           }
         }
       }
-      if (n1.valid()) store_basis<K>(basis_tile(buf ^ 1), lane, bv);
       __syncwarp();
       cur = n1; n1 = n2; n2 = walk.next();
       idx1 = idx2;
@@ -429,9 +409,9 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
 // Both fragment sets together are C * K / 16 registers; where one warp cannot hold them a
 // team of two shares a sample: both warps see all pairs, (1) is split by basis functions and
 // (2) by channels, so that no sum crosses warps.
-// While a chunk is multiplied the next one's feature rows are on their way to the team's
-// other stage and its basis rows to registers, and dX of the next sample to the place that
-// this one's has left for registers.
+// While a chunk is multiplied the next one's feature and basis rows are on their way to the
+// team's other stage, and dX of the next sample to the place that this one's has left for
+// registers.
 // What bounds it: the SM's L1 data path (62 % of its wavefronts, 75 % on the busiest SM:
 // copies into shared memory, operand reads, reductions at ~24 B/clk) and the instructions
 // around the MMAs (issue 50 %).  65 536 samples of 28 pairs at C = 64, K = 32: 345 -> 290 us
@@ -453,10 +433,10 @@ struct GradCfg {
   static constexpr int kMt2 = CC / 16 / kTeam;              // tiles of (2)
   static constexpr int kKs2 = K / 16;
   static constexpr int kFeatStride = CC * 4 + 16;           // bytes: hi[CC] | mid[CC] | pad
-  static constexpr int kKStride = K * 2 + 16;               // a bf16 row over k
+  static constexpr int kBasisStride = K + 8;                // floats of a basis row (+ pad)
   static constexpr int kRawStride = K + 4;                  // floats, a row of dX over k
   static constexpr int kFeatBytes = BASIS ? kChunk * kFeatStride : 0;
-  static constexpr int kStageBytes = kFeatBytes + 2 * kChunk * kKStride;
+  static constexpr int kStageBytes = kFeatBytes + kChunk * kBasisStride * 4;
   static constexpr int kRawBytes = CC * kRawStride * 4;
   static constexpr int kTeamBytes = kRawBytes + 2 * kStageBytes;
   static constexpr int kFit = 227 * 1024 / kTeamBytes * kTeam;      // warps: 16 of 128 registers
@@ -596,8 +576,6 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
   // ldmatrix rows of this lane: pair lane % 8 of a group; matrices 0 and 1 are the hi terms of
   // columns 0-7 and 8-15 of a 16-column step, 2 and 3 the mid terms
   const uint32_t f_off = (lane & 7) * cfg::kFeatStride + ((lane >> 3) & 1) * 16 + (lane >> 4) * (CC * 2);
-  const uint32_t b_off = cfg::kFeatBytes + ((lane & 7) + (lane >> 4) * kChunk) * cfg::kKStride +
-                         ((lane >> 3) & 1) * 16;
   // The row order inside a tile gives a lane consecutive outputs: row g + 8h of a lone tile
   // is output 2g + h, of tile t of a pair output 4g + 2t + h of the pair's 32.
   constexpr int kVec1 = cfg::kMt1 % 2 == 0 ? 4 : 2, kVec2 = cfg::kMt2 % 2 == 0 ? 4 : 2;
@@ -659,26 +637,16 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
                       row_limit + it * W * kRpi < cnt);
       }
     };
-    // basis rows: float4 number tid + 32 W t of the chunk
-    auto load_rows = [&](const Chunk& j, float4* v) {
-      const float4* src = reinterpret_cast<const float4*>(basis + (int64_t)j.base * K) + tid;
+    // basis rows: 16 bytes number tid + 32 W t of the chunk
+    const uint32_t b_dst = smem_addr(mem) + cfg::kRawBytes + cfg::kFeatBytes +
+                           (tid / (K / 4) * cfg::kBasisStride + tid % (K / 4) * 4) * 4;
+    auto issue_basis = [&](int st, const Chunk& j) {
+      const float* src = basis + (int64_t)j.base * K + tid * 4;
       const int have = j.cnt() * (K / 4) - tid;
 #pragma unroll
       for (int t = 0; t < cfg::kBasisVecs; ++t)
-        if (32 * W * t < have) v[t] = ld_global(src + 32 * W * t);
-    };
-    uint8_t* const b_dst = mem + cfg::kRawBytes + cfg::kFeatBytes + tid / (K / 4) * cfg::kKStride +
-                           tid % (K / 4) * 8;
-    auto store_rows = [&](int st, const float4* v) {
-#pragma unroll
-      for (int t = 0; t < cfg::kBasisVecs; ++t) {
-        uint2 h, m;
-        split2(v[t].x, v[t].y, h.x, m.x);
-        split2(v[t].z, v[t].w, h.y, m.y);
-        uint8_t* dst = b_dst + st * cfg::kStageBytes + t * (32 * W / (K / 4)) * cfg::kKStride;
-        *reinterpret_cast<uint2*>(dst) = h;
-        *reinterpret_cast<uint2*>(dst + kChunk * cfg::kKStride) = m;
-      }
+        cp_async16_if(b_dst + st * cfg::kStageBytes + t * (32 * W / (K / 4)) * cfg::kBasisStride * 4,
+                      src + 128 * W * t, 32 * W * t < have);
     };
 
     if (c0 > 0) team_sync();       // (the pass before has read its stages and dX)
@@ -700,14 +668,10 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
       return j.valid() && lane < j.cnt() ? ld_global(&neigh[j.base + lane].x) : 0;
     };
     int idx0 = load_idx(cur), idx1 = load_idx(n1);
-    float4 rows[cfg::kBasisVecs];
-#pragma unroll
-    for (int t = 0; t < cfg::kBasisVecs; ++t) rows[t] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (cur.valid()) {
       issue_dx(cur.item);
       if (BASIS) issue_rows(0, cur, idx0);
-      load_rows(cur, rows);
-      store_rows(0, rows);
+      issue_basis(0, cur);
     }
     cp_commit();
     uint32_t a1h[cfg::kMt1][cfg::kKs1][4], a1m[cfg::kMt1][cfg::kKs1][4];
@@ -761,12 +725,15 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
       }
       if (n1.valid()) {
         if (BASIS) issue_rows(st ^ 1, n1, idx1);
-        load_rows(n1, rows);
+        issue_basis(st ^ 1, n1);
       }
       cp_commit();
       const int idx2 = load_idx(n2);
       // ---- the products, eight pairs at a time
       const uint32_t tile = smem_addr(mem) + cfg::kRawBytes + st * cfg::kStageBytes;
+      const float* const rows_of = reinterpret_cast<const float*>(mem + cfg::kRawBytes + st * cfg::kStageBytes +
+                                                                  cfg::kFeatBytes) +
+                                   g * cfg::kBasisStride + 2 * q;
       const int cnt = cur.cnt();
       float* const db = db_lane + (int64_t)cur.base * K;
 #pragma unroll
@@ -787,8 +754,13 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
         }
 #pragma unroll
         for (int ks = 0; ks < cfg::kKs2; ++ks) {
-          uint32_t b[4];
-          ldsm_x4(tile + b_off + p * cfg::kKStride + ks * 32, b);
+          uint32_t b[4];      // hi terms of columns 2q, 2q + 1 and, eight further on; mid terms
+          const float* row = rows_of + p * cfg::kBasisStride + 16 * ks;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const float2 x = *reinterpret_cast<const float2*>(row + 8 * half);
+            split2(x.x, x.y, b[half], b[2 + half]);
+          }
 #pragma unroll
           for (int pass = 0; pass < 3; ++pass)
 #pragma unroll
@@ -827,7 +799,6 @@ basis_proj_grads_mma_kernel(int bs, int parts, int shift, int C, int64_t ns, int
         }
       }
       st ^= 1;
-      if (n1.valid()) store_rows(st, rows);
       cur = n1; n1 = n2; n2 = walk.next(n1);
       idx0 = idx1; idx1 = idx2;
     }
