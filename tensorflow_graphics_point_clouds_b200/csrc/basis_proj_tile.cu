@@ -18,11 +18,11 @@
 //              K = 32, C = 1  27 -> 7, 47 -> 17, 114 -> 91    C = 8  15 -> 7, 44 -> 28, 247 -> 127
 //              K = 64, C = 1  48 -> 5, 103 -> 35, 228 -> 115  C = 8  21 -> 9, 201 -> 58, 729 -> 223
 //              K = 32, C = 24 21 -> 15, 191 -> 134, 765 -> 534
-//   gradients  K =  8, C = 1  42 -> 13, 74 -> 14, 158 -> 49   C = 8  29 -> 13, 46 -> 22, 148 -> 90
-//              K = 16, C = 3  81 -> 13, 154 -> 24, 311 -> 109 C = 8  41 -> 13, 67 -> 32, 225 -> 137
+//   gradients  K =  8, C = 1  42 -> 13, 74 -> 14, 158 -> 49   C = 8  29 -> 13, 46 -> 22, 148 -> 87
+//              K = 16, C = 3  81 -> 13, 154 -> 24, 311 -> 109 C = 8  41 -> 13, 67 -> 31, 225 -> 133
 //              K = 32, C = 1  153 -> 13, 308 -> 41, 624 -> 130   K = 64  294 -> 10, 577 -> 55, 1166 -> 214
-//              K =  8, C = 64 29 -> 21, 101 -> 84, 373 -> 337    C = 128 (27, 31, 128, 161, 494, 605)
-//              K = 16, C = 24 31 -> 20, 111 -> 94, 415 -> 367  K = 64  134 -> 51, 833 -> 258, 3385 -> 1024
+//              K =  8, C = 64 29 -> 21, 101 -> 82, 373 -> 334    C = 128 (27, 31, 128, 161, 494, 605)
+//              K = 16, C = 24 31 -> 20, 111 -> 90, 415 -> 350  K = 64  134 -> 51, 833 -> 246, 3385 -> 973
 // (bytes of K = 64, C = 1 at 6450 GB/s: 92 and 179 us).  Bound by HBM for one channel, else by
 // the latency of the gathers (13 to 20 warps an SM, issue 35 to 50 %) and the instructions
 // around the multiply-adds.
@@ -42,8 +42,6 @@ struct Tile {
   static constexpr int kKt = K == 64 ? 8 : 4;
   static constexpr int kKl = K / kKt;
   static constexpr int kSlots = 32 / (kKl * CL);      // pairs of a step
-  static constexpr int kBatch = kSlots <= 2 ? 2 : 1;  // steps whose loads are made together
-  static constexpr int kAhead = 2 * kBatch;           // steps whose loads are under way
   static_assert(kKl * CL <= 32, "a pair's tile fits a warp");
 };
 
@@ -198,7 +196,9 @@ basis_proj_tile_kernel(int C, int64_t ns, int per, const float* basis, const flo
                        int shift, bool vec) {
   chain_enter();
   typedef Tile<K, CT, CL> tile;
-  constexpr int kKt = tile::kKt, kSlots = tile::kSlots, kBatch = tile::kBatch, kAhead = tile::kAhead;
+  constexpr int kKt = tile::kKt, kSlots = tile::kSlots;
+  constexpr int kBatch = kSlots <= 2 ? 2 : 1;      // steps whose loads are made together
+  constexpr int kAhead = 2 * kBatch;               // and are under way
   const int lane = lane_id();
   const int k0 = lane % tile::kKl * kKt, c0 = lane / tile::kKl % CL * CT;
   const int slot = lane / (tile::kKl * CL);
@@ -279,20 +279,46 @@ basis_proj_tile_kernel(int C, int64_t ns, int per, const float* basis, const flo
   }
 }
 
+// dst[0 .. N) += v under a condition, without a branch; have: values that exist.
 template <int N>
-__device__ __forceinline__ void add_values(float* dst, const float* v, int have, bool vec) {
-  if (N == 4 && vec) {
-    if (have > 0)
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(v[0]),
-                   "f"(v[1 % N]), "f"(v[2 % N]), "f"(v[3 % N]) : "memory");
+__device__ __forceinline__ void add_values(float* dst, const float* v, int have, bool vec, bool ok) {
+  if (N >= 4 && vec) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n"
+                   "@p red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"l"(dst + i), "f"(v[i]),
+                   "f"(v[(i + 1) % N]), "f"(v[(i + 2) % N]), "f"(v[(i + 3) % N]),
+                   "r"((uint32_t)(ok && have > i)) : "memory");
   } else if (N == 2 && vec) {
-    if (have > 0)
-      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(v[0]), "f"(v[1 % N])
-                   : "memory");
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n"
+                 "@p red.global.add.v2.f32 [%0], {%1, %2};\n}" ::"l"(dst), "f"(v[0]), "f"(v[1 % N]),
+                 "r"((uint32_t)(ok && have > 0)) : "memory");
   } else {
 #pragma unroll
     for (int i = 0; i < N; ++i)
-      if (i < have) atomicAdd(dst + i, v[i]);
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n"
+                   "@p red.global.add.f32 [%0], %1;\n}" ::"l"(dst + i), "f"(v[i]),
+                   "r"((uint32_t)(ok && i < have)) : "memory");
+  }
+}
+
+template <int N>
+__device__ __forceinline__ void store_values(float* dst, const float* v, bool vec, bool ok) {
+  if (N % 4 == 0 && vec) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\n"
+                   "@p st.global.v4.f32 [%0], {%1, %2, %3, %4};\n}" ::"l"(dst + i), "f"(v[i]),
+                   "f"(v[(i + 1) % N]), "f"(v[(i + 2) % N]), "f"(v[(i + 3) % N]), "r"((uint32_t)ok)
+                   : "memory");
+  } else if (N == 2 && vec) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %3, 0;\n@p st.global.v2.f32 [%0], {%1, %2};\n}"
+                 ::"l"(dst), "f"(v[0]), "f"(v[1 % N]), "r"((uint32_t)ok) : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.global.f32 [%0], %1;\n}"
+                   ::"l"(dst + i), "f"(v[i]), "r"((uint32_t)ok) : "memory");
   }
 }
 
@@ -371,28 +397,19 @@ basis_proj_grads_tile_kernel(int C, int64_t ns, int64_t M, int per, const float*
         bool owner;
         constexpr int kStepsF = log2_of(tile::kKl);
         fold<CT, kStepsF, 1>(df, lane, 1, &at, &owner);
-        if (owner && live)
-          add_values<folded<CT, kStepsF, 1>()>(dfeat + (int64_t)j * C + c0 + at, df, C - c0 - at, vec);
+        // (by predicate; where few lanes of a small K have something, those lanes branch first.
+        // 65 536 samples, us, branch and predicate: K = 32, C = 8 256 / 214, K = 64, C = 24
+        // 1024 / 973, K = 8, C = 24 208 / 246, K = 16, C = 24 350 / 440)
+        constexpr bool kBranch = CL > 2 && K <= 16;
+        if (!kBranch || (owner && live))
+          add_values<folded<CT, kStepsF, 1>()>(dfeat + (int64_t)j * C + c0 + at, df, C - c0 - at, vec,
+                                               kBranch || (owner && live));
         if (BASIS) {
           constexpr int kStepsB = log2_of(CL);
-          constexpr int kLeft = folded<kKt, kStepsB, 1>();
           fold<kKt, kStepsB, 1>(db, lane, tile::kKl, &at, &owner);
-          if (owner && live) {
-            float* dst = dbasis + (int64_t)m * K + k0 + at;
-            if (kLeft > 1 && !vec_basis) {
-#pragma unroll
-              for (int q = 0; q < kLeft; ++q) dst[q] = db[q];
-            } else if (kLeft % 4 == 0) {
-#pragma unroll
-              for (int q = 0; q < kLeft; q += 4)
-                *reinterpret_cast<float4*>(dst + q) =
-                    make_float4(db[q], db[(q + 1) % kKt], db[(q + 2) % kKt], db[(q + 3) % kKt]);
-            } else if (kLeft == 2) {
-              *reinterpret_cast<float2*>(dst) = make_float2(db[0], db[1]);
-            } else {
-              *dst = db[0];
-            }
-          }
+          if (!kBranch || (owner && live))
+            store_values<folded<kKt, kStepsB, 1>()>(dbasis + (int64_t)m * K + k0 + at, db, vec_basis,
+                                                    kBranch || (owner && live));
         }
       }
     }
