@@ -166,12 +166,14 @@ cells_walk_kernel(WalkArgs a) {
   const Grid<D> g = load_grid<D>(c.num_cells, c.inv_cell);
   const int total = total_cells<D>(g.nc, c.batch_size);
   if (total == 0) return;        // (a grid that got no cells: the call fails)
+  float radius[D];       // its inverse
   f32x2 inv_r[D], scale[D], scale_lo[D];
   double norm_exact = 1.0;
   bool isotropic = true;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
     const float r = ld_global(a.inv_radii + d);
+    radius[d] = r;
     inv_r[d] = pack2(r, r);
     if (MODE == kDensity) {
       const float bw = a.bw_mode == 1 ? sqrtf((float)c.n) : ld_global(a.inv_bw + d);
@@ -242,11 +244,12 @@ cells_walk_kernel(WalkArgs a) {
         const int steps = (min(candidates - base, 32 * kSteps) + 31) >> 5;
         for (unsigned todo = members; todo; todo &= todo - 1u) {
           const int who = __ffs(todo) - 1;
+          float one[D];
           f32x2 sp[D];
 #pragma unroll
           for (int d = 0; d < D; ++d) {
-            const float x = __shfl_sync(0xffffffffu, s.p[d], who);
-            sp[d] = pack2(x, x);
+            one[d] = __shfl_sync(0xffffffffu, s.p[d], who);
+            sp[d] = pack2(one[d], one[d]);
           }
           int n_hit = 0, id = 0, begin = 0;
           float acc = 0.0f;
@@ -257,7 +260,25 @@ cells_walk_kernel(WalkArgs a) {
           }
 #pragma unroll
           for (int k = 0; k < kSteps; k += 2) {
-            if (k < steps) {
+            if (MODE == kCount && D <= 3 && k < steps) {
+              // One by one: where nothing follows the test the packed forms, which keep the
+              // multiply-add pipes busy longer, are the slower ones.  Surfaces 366 -> 331 us, 524 288
+              // uniform points with 34 neighbors 102 -> 96, with 16 105 and 105; four dimensions
+              // 179 and 186.  (Density and fill of surfaces so: 503 -> 532, 665 -> 685.)
+              float x[2][D];
+#pragma unroll
+              for (int d = 0; d < D; ++d) unpack2(np[d][k / 2], x[0][d], x[1][d]);
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                float d2 = 0.0f;
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                  const float t = __fmul_rn(__fadd_rn(one[d], x[u][d]), radius[d]);
+                  d2 = d == 0 ? __fmul_rn(t, t) : __fmaf_rn(t, t, d2);
+                }
+                n_hit += d2 < 1.0f;
+              }
+            } else if (k < steps) {
               f32x2 t2[D], d2;
 #pragma unroll
               for (int d = 0; d < D; ++d) {
