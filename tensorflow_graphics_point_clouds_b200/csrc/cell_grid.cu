@@ -414,7 +414,18 @@ constexpr int kClusterBoxes = 1024;        // batch size x D at most
 // them alone, so a large one goes to the whole GPU.  The sorted copies scatter 44 bytes
 // a point: from 8192 points on they are a launch of their own (41 000 points: 13 us of
 // the cluster's 33, 4.4 by themselves).
+// It is bound by its six barriers (about 1200 cycles each) and, between them, by single trips
+// to L2 and by instructions that are not in the cache yet: 11 us for 4096 points.  Hence each
+// trip is made once, for all points of a thread together: points are read for the boxes and
+// kept until the cell is known, bucket and number until the place is; a warp takes neighboring
+// points and folds their box in registers; the scan keeps what it summed up, without a barrier
+// of the block per 4096 cells; sums go to the other blocks before a barrier instead of being
+// fetched after it.  us before -> now, kernel: 42 000 points in 7300 cells 23 -> 19, 38 000 in
+// 226 000 28 -> 18; 3-level cell averages of 5 x 9000 points 171 -> 158, three-level classifier
+// 668 -> 639, layer step on 59 000 points 208 -> 203.  Left: the atomics of 16 SMs (7300 cycles
+// for 59 000 points, about two per atomic of an SM).
 constexpr int kMaxRanks = 16;
+constexpr int kHeld = 4;                   // points of a thread at most
 constexpr int64_t kClusterPoints = 65536;
 constexpr int64_t kClusterCells = int64_t(1) << 21;
 constexpr int64_t kClusterPlacePoints = 8192;
@@ -426,174 +437,296 @@ struct ClusterBuild {
   int batch_size, max_cells;
   DimValues cell_sizes;
   tfgpc_cell_grid g;
-  int32_t *arrival, *members, *crowded, *page;
+  int32_t *members, *crowded, *page;
   bool place;
   AlsoClear also;
 };
 
+// Loads and the atomic under predicates: those of a thread's points are under way together, and
+// what is not there costs an issue slot.
+__device__ __forceinline__ int load_if(const int32_t* p, bool ok, int otherwise) {
+  int v = otherwise;
+  asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.cg.s32 %0, [%1];}"
+               : "+r"(v) : "l"(p), "r"((unsigned)ok) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_if(const float* p, bool ok) {
+  float v = 0.0f;
+  asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.f32 %0, [%1];}"
+               : "+f"(v) : "l"(p), "r"((unsigned)ok) : "memory");
+  return v;
+}
+__device__ __forceinline__ int count_if(int32_t* p, bool ok) {
+  int v = 0;
+  asm volatile("{.reg .pred q; setp.ne.u32 q, %2, 0; @q atom.global.add.s32 %0, [%1], 1;}"
+               : "+r"(v) : "l"(p), "r"((unsigned)ok) : "memory");
+  return v;
+}
+// table[at .. at + 4), zeros from `end` on; wide: the table begins at a multiple of 16 bytes.
+__device__ __forceinline__ int4 load_four(const int32_t* table, int at, int end, bool wide) {
+  int4 v = make_int4(0, 0, 0, 0);
+  const bool all = wide && at + 4 <= end;
+  asm volatile("{.reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.cg.v4.s32 {%0, %1, %2, %3}, [%4];}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+               : "l"(table + at), "r"((unsigned)all) : "memory");
+  v.x = load_if(table + at, !all && at < end, v.x);
+  v.y = load_if(table + at + 1, !all && at + 1 < end, v.y);
+  v.z = load_if(table + at + 2, !all && at + 2 < end, v.z);
+  v.w = load_if(table + at + 3, !all && at + 3 < end, v.w);
+  return v;
+}
+__device__ __forceinline__ void store_four(int32_t* table, int at, int end, bool wide, int4 v) {
+  if (wide && at + 4 <= end) {
+    __stcg((int4*)(table + at), v);
+    return;
+  }
+  if (at < end) __stcg(table + at, v.x);
+  if (at + 1 < end) __stcg(table + at + 1, v.y);
+  if (at + 2 < end) __stcg(table + at + 2, v.z);
+  if (at + 3 < end) __stcg(table + at + 3, v.w);
+}
+
+// A thread holds its points (kHeld at most) from the boxes to their places: coordinates until
+// the cell is known, then bucket and number in it.
 template <int D>
 __global__ void __launch_bounds__(kClusterThreads, 1)
 grid_cluster_kernel(ClusterBuild a) {
   chain_enter();
   // [0] ordered keys of the lower corners, [1] complements of those of the upper ones
   __shared__ unsigned box[2][kClusterBoxes];
-  __shared__ float smin_s[kClusterBoxes];
-  __shared__ int asked[D], nc_s[D];
-  __shared__ int warp_sum_s[32], block_sum_s;
+  __shared__ float smin_s[kClusterBoxes], inv_s[D];
+  __shared__ int asked[D];
+  __shared__ int warp_sum_s[32], block_sum_s[kMaxRanks];     // (of every block)
   __shared__ RankScratch<kClusterThreads> scratch;
   cg::cluster_group cluster = cg::this_cluster();
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
   const int n = (int)a.n, boxes = a.batch_size * D;
   const int stride = ranks * kClusterThreads, first = rank * kClusterThreads + tid;
+  // A warp's points follow one another, as they mostly lie in one cloud.
+  const int steps = (n + stride - 1) / stride;
+  const int mine = (w * ranks + rank) * 32 * steps + lane;
+  const int here = (min(n - mine, 32 * steps) + 31) >> 5;    // this lane's points (or none: <= 0)
+  float p[kHeld][D];
+  int cloud[kHeld];
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) {
+    const bool live = k < here;
+    cloud[k] = load_if(a.batch_ids + (mine + 32 * k), live, -1);
+#pragma unroll
+    for (int d = 0; d < D; ++d) p[k][d] = load_if(a.pts + (int64_t)(mine + 32 * k) * D + d, live);
+  }
   for (int64_t i = first; i < a.also.words; i += stride) a.also.p[i] = 0u;
   // ---- boxes of this block's points
   for (int i = tid; i < boxes; i += kClusterThreads) box[0][i] = box[1][i] = 0xffffffffu;
   if (tid < D) asked[tid] = 1;
   __syncthreads();
-  for (int i0 = first - lane; i0 < n; i0 += stride) {
-    const int i = i0 + lane;
-    const bool live = i < n;
-    const int b = live ? ld_global(a.batch_ids + i) : -1;
-    float lo[D], hi[D];
+  // (the lanes' least keys; all of them of cloud b if `uniform`)
+  auto fold = [&](const float* lo, const float* hi, int b, bool live, bool uniform) {
+    unsigned kl[D], kh[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const float v = live ? ld_global(a.pts + (int64_t)i * D + d) : 0.0f;
-      // (a coordinate that is no number counts for no box)
-      lo[d] = live ? fminf(INFINITY, v) : INFINITY;
-      hi[d] = live ? fmaxf(-INFINITY, v) : -INFINITY;
-    }
-    const int b0 = __shfl_sync(0xffffffffu, b, 0);
-    const bool uniform = __all_sync(0xffffffffu, b == b0 || !live);
+    for (int d = 0; d < D; ++d) { kl[d] = ordered(lo[d]); kh[d] = ~ordered(hi[d]); }
     if (uniform) {
-#pragma unroll
-      for (int d = 0; d < D; ++d)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-          hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-        }
-    }
-    if (b >= 0 && b < a.batch_size && (!uniform || lane == 0)) {
+      unsigned least = 0xffffffffu;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        atomicMin(&box[0][b * D + d], ordered(lo[d]));
-        atomicMin(&box[1][b * D + d], ~ordered(hi[d]));
+        const unsigned l = __reduce_min_sync(0xffffffffu, kl[d]);
+        const unsigned h = __reduce_min_sync(0xffffffffu, kh[d]);
+        if (lane == d) least = l;
+        if (lane == D + d) least = h;
+      }
+      if (lane < 2 * D && b >= 0 && b < a.batch_size)
+        atomicMin(&box[lane >= D][b * D + lane - (lane >= D ? D : 0)], least);
+    } else if (live && b >= 0 && b < a.batch_size) {
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        atomicMin(&box[0][b * D + d], kl[d]);
+        atomicMin(&box[1][b * D + d], kh[d]);
+      }
+    }
+  };
+  {
+    const int b0 = __shfl_sync(0xffffffffu, cloud[0], 0);
+    bool same = true;
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) same = same && (k >= here || cloud[k] == b0);
+    if (__all_sync(0xffffffffu, same)) {
+      float lo[D], hi[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d) { lo[d] = INFINITY; hi[d] = -INFINITY; }
+#pragma unroll
+      for (int k = 0; k < kHeld; ++k)
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          // (a coordinate that is no number counts for no box)
+          lo[d] = k < here ? fminf(lo[d], p[k][d]) : lo[d];
+          hi[d] = k < here ? fmaxf(hi[d], p[k][d]) : hi[d];
+        }
+      fold(lo, hi, b0, false, true);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < steps; ++k) {
+        const bool live = k < here;
+        int b = cloud[0];
+        float lo[D], hi[D];
+#pragma unroll
+        for (int d = 0; d < D; ++d) lo[d] = p[0][d];
+#pragma unroll
+        for (int q = 1; q < kHeld; ++q) {
+          b = k == q ? cloud[q] : b;
+#pragma unroll
+          for (int d = 0; d < D; ++d) lo[d] = k == q ? p[q][d] : lo[d];
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          hi[d] = live ? fmaxf(-INFINITY, lo[d]) : -INFINITY;
+          lo[d] = live ? fminf(INFINITY, lo[d]) : INFINITY;
+        }
+        const int first_b = __shfl_sync(0xffffffffu, b, 0);
+        fold(lo, hi, b, live, __all_sync(0xffffffffu, b == first_b || !live));
       }
     }
   }
   cluster.sync();
   // ---- parameters, by every block for itself (see boxes_kernel)
-  for (int i = tid; i < boxes; i += kClusterThreads) {
-    unsigned kl = 0xffffffffu, kh = 0xffffffffu;
-#pragma unroll
-    for (int r = 0; r < kMaxRanks; ++r) {      // (all loads in flight together)
-      const unsigned* other = cluster.map_shared_rank(&box[0][0], min(r, ranks - 1));
-      kl = min(kl, other[i]);
-      kh = min(kh, other[kClusterBoxes + i]);
+  // (each of the `ranks` blocks, a power of two, is read by a warp or several; that others read
+  // this one's boxes meanwhile, some of them lowered already, changes no minimum)
+  if (w % ranks != rank) {
+    const unsigned* other = cluster.map_shared_rank(&box[0][0], w % ranks);
+    for (int i = w / ranks * 32 + lane; i < boxes; i += max(32 / ranks, 1) * 32) {
+      const unsigned kl = ld_global(other + i), kh = ld_global(other + kClusterBoxes + i);
+      atomicMin(&box[0][i], kl);
+      atomicMin(&box[1][i], kh);
     }
-    const int d = i % D;
-    const float cs = a.cell_sizes.v[d];
+  }
+  if (w == 31 && lane < D) {
+    inv_s[lane] = __fdiv_rn(1.0f, a.cell_sizes.v[lane]);
+    if (rank == 0) a.g.inv_cell_sizes[lane] = inv_s[lane];
+  }
+  __syncthreads();
+  // (two threads per box, so that their divisions are one piece of code: instructions that are
+  // not in the cache yet cost more here than the work)
+  for (int x = tid; x < 2 * boxes; x += kClusterThreads) {
+    const int i = x >> 1, d = i % D;
+    const unsigned kl = box[0][i], kh = box[1][i];
     const float mn = __fsub_rn(kl == 0xffffffffu ? INFINITY : unordered(kl), 1e-9f);
     const float mx = __fadd_rn(kh == 0xffffffffu ? -INFINITY : unordered(~kh), 1e-9f);
-    const float sm = __fdiv_rn(mn, cs);
-    smin_s[i] = sm;
-    if (rank == 0) {
-      a.g.aabb_min[i] = mn;
-      a.g.aabb_max[i] = mx;
-      a.g.scaled_aabb_min[i] = sm;
+    const float q = __fdiv_rn(x & 1 ? __fsub_rn(mx, mn) : mn, a.cell_sizes.v[d]);
+    if (x & 1) {
+      const float c = ceilf(q);
+      if (c > 0.0f && c < 2147483000.0f) atomicMax(&asked[d], (int)c);
+    } else {
+      smin_s[i] = q;
+      if (rank == 0) {
+        a.g.aabb_min[i] = mn;
+        a.g.aabb_max[i] = mx;
+        a.g.scaled_aabb_min[i] = q;
+      }
     }
-    const float c = ceilf(__fdiv_rn(__fsub_rn(mx, mn), cs));
-    if (c > 0.0f && c < 2147483000.0f) atomicMax(&asked[d], (int)c);
   }
   __syncthreads();
   bool over = false;
+  Grid<D> g;
 #pragma unroll
-  for (int d = 0; d < D; ++d) over = over || asked[d] > a.max_cells;
+  for (int d = 0; d < D; ++d) {
+    g.nc[d] = asked[d];
+    g.inv[d] = inv_s[d];
+    over = over || g.nc[d] > a.max_cells;
+  }
   if (over) {                // (the same in every block)
     if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
     cluster.sync();          // no block leaves while others read its shared memory
     return;
   }
-  if (tid < D) nc_s[tid] = asked[tid];
-  __syncthreads();
-  Grid<D> g;
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    g.nc[d] = nc_s[d];
-    g.inv[d] = __fdiv_rn(1.0f, a.cell_sizes.v[d]);
-    if (rank == 0 && tid == 0) a.g.inv_cell_sizes[d] = g.inv[d];
-  }
   const int total = total_cells<D>(g.nc, a.batch_size);
   int32_t* const table = a.g.cell_start;
-  for (int i = first; i < total + 3; i += stride) __stcg(table + i, 0);
+  const bool wide = ((uintptr_t)table & 15) == 0;
+  for (int i = 4 * first; i < total + 3; i += 4 * stride)
+    store_four(table, i, total + 3, wide, make_int4(0, 0, 0, 0));
   if (first == 0) __stcg(a.crowded, 0);
   cluster.sync();
-  // ---- keys and the number of points per bucket (see keys_histogram_kernel)
-  for (int i0 = first - lane; i0 < n; i0 += stride) {
-    const int i = i0 + lane;
-    const unsigned live = __ballot_sync(0xffffffffu, i < n);
-    if (i >= n) break;
-    const int b = ld_global(a.batch_ids + i);
-    const int bs = min(max(b, 0), a.batch_size - 1);
-    float p[D];
-    int cell[D];
+  // ---- keys and the number of points per bucket (see keys_histogram_kernel and arrive)
+  int bucket[kHeld], number[kHeld];
+  bool apart = true;
 #pragma unroll
-    for (int d = 0; d < D; ++d) p[d] = ld_global(a.pts + (int64_t)i * D + d);
-    cell_of<D>(p, smin_s + bs * D, g, cell);
-    const int64_t key = key_of<D>(cell, g, b);
-    __stcg((long long*)a.g.keys + i, (long long)key);
-    __stcg(a.arrival + i, arrive(table, bucket_of(key, total), live, a.crowded));
+  for (int k = 0; k < kHeld; ++k) {
+    bucket[k] = number[k] = 0;
+    if (k >= steps) continue;
+    const bool live = k < here;
+    if (live) {
+      int cell[D];
+      cell_of<D>(p[k], smin_s + min(max(cloud[k], 0), a.batch_size - 1) * D, g, cell);
+      const int64_t key = key_of<D>(cell, g, cloud[k]);
+      __stcg((long long*)a.g.keys + mine + 32 * k, (long long)key);
+      bucket[k] = bucket_of(key, total);
+    }
+    const int b0 = __shfl_sync(0xffffffffu, bucket[k], 0);
+    apart = apart && __popc(__ballot_sync(0xffffffffu, live && bucket[k] == b0)) <= 4;
+  }
+  if (apart) {
+    int most = 0;
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) number[k] = count_if(table + bucket[k], k < here);
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) most = max(most, number[k]);
+    if (most >= kCrowdedBucket) __stcg(a.crowded, 1);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) {
+      const unsigned live = __ballot_sync(0xffffffffu, k < here);
+      if (k < here) number[k] = arrive(table, bucket[k], live, a.crowded);
+    }
   }
   cluster.sync();
-  // ---- exclusive scan of the table: a stretch per block, its sum first
+  // ---- exclusive scan of the table: a stretch per block and of it one per warp, the sums first
   const int per = (((total + 3) + ranks - 1) / ranks + 3) / 4 * 4;
-  const int begin = min(rank * per, total + 3), end = min(begin + per, total + 3);
+  const int per_warp = ((per + 31) / 32 + 127) / 128 * 128;
+  const int block_end = min((rank + 1) * per, total + 3);
+  const int begin = rank * per + w * per_warp, end = min(begin + per_warp, block_end);
+  int4 v[kHeld];          // the warp's first pieces of 128
   int sum = 0;
-  for (int i = begin + tid; i < end; i += kClusterThreads) sum += __ldcg(table + i);
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) v[k] = load_four(table, begin + 128 * k + 4 * lane, end, wide);
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) sum += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+  for (int i = begin + 128 * kHeld + 4 * lane; i < end; i += 128) {
+    const int4 x = load_four(table, i, end, wide);
+    sum += (x.x + x.y) + (x.z + x.w);
+  }
   sum = __reduce_add_sync(0xffffffffu, sum);
   if (lane == 0) warp_sum_s[w] = sum;
   __syncthreads();
   if (w == 0) {
     sum = __reduce_add_sync(0xffffffffu, warp_sum_s[lane]);
-    if (lane == 0) block_sum_s = sum;
+    if (lane < ranks) *cluster.map_shared_rank(&block_sum_s[rank], lane) = sum;
   }
   cluster.sync();
-  int run = 0;
-  if (lane < rank) run = *cluster.map_shared_rank(&block_sum_s, lane);
-  run = __reduce_add_sync(0xffffffffu, run);
-  for (int t0 = begin; t0 < end; t0 += 4 * kClusterThreads) {
-    const int i = t0 + 4 * tid;
-    int v[4], x = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      v[k] = i + k < end ? __ldcg(table + i + k) : 0;
-      x += v[k];
-    }
-    const int own = x;
+  int run = __reduce_add_sync(0xffffffffu, (lane < rank ? block_sum_s[lane & (kMaxRanks - 1)] : 0) +
+                                               (lane < w ? warp_sum_s[lane] : 0));
+  auto scan_piece = [&](int at, int4 x) {
+    const int own = (x.x + x.y) + (x.z + x.w);
+    int y = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const int z = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) y += z;
     }
-    __syncthreads();
-    if (lane == 31) warp_sum_s[w] = x;
-    __syncthreads();
-    const int s = warp_sum_s[lane];
-    int at = run + x - own + __reduce_add_sync(0xffffffffu, lane < w ? s : 0);
-    run += __reduce_add_sync(0xffffffffu, s);
+    const int s = run + y - own;
+    store_four(table, at, end, wide, make_int4(s, s + x.x, s + x.x + x.y, s + x.x + x.y + x.z));
+    run += __shfl_sync(0xffffffffu, y, 31);
+  };
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (i + k < end) __stcg(table + i + k, at);
-      at += v[k];
-    }
-  }
+  for (int k = 0; k < kHeld; ++k)
+    if (begin + 128 * k < end) scan_piece(begin + 128 * k + 4 * lane, v[k]);
+  for (int i = begin + 128 * kHeld; i < end; i += 128)
+    scan_piece(i + 4 * lane, load_four(table, i + 4 * lane, end, wide));
   cluster.sync();
   // ---- members of the buckets, then every point's place (see place_kernel)
-  for (int i = first; i < n; i += stride) {
-    const int r = bucket_of(__ldcg((const long long*)a.g.keys + i), total);
-    __stcg(a.members + __ldcg(table + r) + __ldcg(a.arrival + i), i);
-  }
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k) number[k] += load_if(table + bucket[k], k < here, 0);
+#pragma unroll
+  for (int k = 0; k < kHeld; ++k)
+    if (k < here) __stcg(a.members + number[k], mine + 32 * k);
   cluster.sync();   // (also: no block leaves while others read its shared memory)
   if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
   if (!a.place) return;
@@ -638,22 +771,22 @@ grid_cluster_kernel(ClusterBuild a) {
   }
 }
 
+// Blocks of the largest cluster the device takes.
 template <int D>
-int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
+int cluster_ranks(int* most) {
   static int ranks_of[64] = {0};     // per device (the same value whoever computes it)
   int dev = 0;
   TFGPC_CUDA(cudaGetDevice(&dev));
   int ranks = dev < 64 ? ranks_of[dev] : 0;
-  cudaLaunchConfig_t cfg{};
-  cfg.blockDim = dim3(kClusterThreads);
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim = {kMaxRanks, 1, 1};
-  cfg.gridDim = dim3(kMaxRanks);
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
   if (ranks == 0) {
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.gridDim = dim3(kMaxRanks);
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {kMaxRanks, 1, 1};
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
     int fit = 0;
     if (cudaFuncSetAttribute(grid_cluster_kernel<D>,
                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
@@ -663,6 +796,18 @@ int launch_cluster(cudaStream_t st, const ClusterBuild& a) {
     ranks = fit > 0 ? kMaxRanks : 8;
     if (dev < 64) ranks_of[dev] = ranks;
   }
+  *most = ranks;
+  return TFGPC_OK;
+}
+
+template <int D>
+int launch_cluster(cudaStream_t st, const ClusterBuild& a, int ranks) {
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  cfg.attrs = at;
   // a thread per point, and per 16 cells the table has room for
   const int64_t room = table_cells(D, a.batch_size, a.max_cells) / 16;
   const int64_t threads = a.n > room ? a.n : room;
@@ -726,13 +871,19 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   DimValues cs{};
   for (int d = 0; d < D; ++d) cs.v[d] = cell_sizes[d];
   const unsigned blocks = blocks_for(n, kThreads);
+  int ranks = 0;
   if (!num_cells_in && n <= kClusterPoints && cells <= kClusterCells &&
       (int64_t)B * D <= kClusterBoxes) {
-    ProfScope prof(st, "grid_cluster");
-    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.arrival, w.members,
-                         w.crowded, page, n <= kClusterPlacePoints, also};
     int rc = TFGPC_OK;
-    TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a));
+    TFGPC_DIM_SWITCH(D, rc = cluster_ranks<kD>(&ranks));
+    if (rc) return rc;
+  }
+  if (ranks > 0 && n <= (int64_t)ranks * kClusterThreads * kHeld) {
+    ProfScope prof(st, "grid_cluster");
+    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.members, w.crowded,
+                         page, n <= kClusterPlacePoints, also};
+    int rc = TFGPC_OK;
+    TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a, ranks));
     if (rc) return rc;
     return a.place ? TFGPC_OK : place(st, g, points, batch_ids, w);
   }
