@@ -8,6 +8,8 @@
 // traffic and no barriers in the neighbor loop.  (The reference: one 64-thread
 // block per (sample, 8 channels), two __syncthreads per neighbor step,
 // basis_proj_kernels.cu.cc:30-127.)
+// Layers of few channels mostly take the warp tiles of basis_proj_tile.cu; to G < 32 come here
+// those whose rows are not 16-byte aligned and, of K <= 16, forward passes over many samples.
 #include "basis_proj.cuh"
 #include "basis_proj_wide.cuh"
 #include "prepare.cuh"

@@ -414,12 +414,14 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
 // registers.
 // What bounds it: the SM's L1 data path (62 % of its wavefronts, 75 % on the busiest SM:
 // copies into shared memory, operand reads, reductions at ~24 B/clk) and the instructions
-// around the MMAs (issue 50 %).  65 536 samples of 28 pairs at C = 64, K = 32: 345 -> 290 us
-// (1.07 GB: 3.7 TB/s); 41 000 at C = 64, K = 16: 166 -> 139.  (One warp per sample with dX as
-// bf16 rows in shared memory, read by ldmatrix again for every chunk, took 25 KB at C = 64,
-// K = 32 -- 8 warps per SM -- and a chunk of nine pairs cost as much as one of sixteen.
-// Everything straight from global memory to registers, without shared memory, read each
-// piece of dX twice through L1: 228 against 185 us on 33 000 samples.)
+// around the MMAs (issue 50 %).  What teams and fragments gave, 65 536 samples of 28 pairs at
+// C = 64, K = 32: 345 -> 290 us (now 54 500 of 32 pairs: 235, 0.9 GB: 3.8 TB/s); 41 000 at
+// C = 64, K = 16: 166 -> 139, without the gradient of the basis 86 (the reductions of 1.15
+// million rows: 60).  (One warp per sample with dX as bf16 rows in shared memory, read by
+// ldmatrix again for every chunk, took 25 KB at C = 64, K = 32 -- 8 warps per SM -- and a chunk
+// of nine pairs cost as much as one of sixteen.  Everything straight from global memory to
+// registers, without shared memory, read each piece of dX twice through L1: 228 against 185 us
+// on 33 000 samples.)
 // dbasis is written, not accumulated (every pair belongs to exactly one sample; layers
 // wider than a pass add to it pass by pass); dfeat must be zero on entry.
 // BASIS false: dfeat alone, for layers whose basis is not trained: (1) is left out, and no
