@@ -581,6 +581,14 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
       const int who = live ? nb.y : -1;
       const int prev = __shfl_up_sync(0xffffffffu, who, 2);
       const bool head = lane < 2 || prev != who;
+      // (found once for the three coordinates: ELU, 8-16, 8 clouds of up to 16 384 points with 24
+      // neighbors 340 -> 334 us)
+      bool joined[4];      // with the pair that many lanes on
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const int id = __shfl_down_sync(0xffffffffu, who, 2 << t);
+        joined[t] = lane + (2 << t) < 32 && id == who;
+      }
 #pragma unroll
       for (int i = 0; PADDED && i < HI; ++i) g1[i] = half * HI + i < h1 ? g1[i] : 0.0f;
 #pragma unroll
@@ -590,10 +598,9 @@ small_mlp_grads_kernel(MlpShape s, int64_t M, const float* p_in,
         float v = (mine + __shfl_xor_sync(0xffffffffu, mine, 1)) * inv_radius;
         if (live && half == 0 && dp_in) atomicAdd(dp_in + (int64_t)nb.x * 3 + d, v);
 #pragma unroll
-        for (int o = 2; o < 32; o <<= 1) {
-          const float y = __shfl_down_sync(0xffffffffu, v, o);
-          const int id = __shfl_down_sync(0xffffffffu, who, o);
-          if (lane + o < 32 && id == who) v += y;
+        for (int t = 0; t < 4; ++t) {
+          const float y = __shfl_down_sync(0xffffffffu, v, 2 << t);
+          if (joined[t]) v += y;
         }
         if (live && half == 1 && head && dp_out) atomicAdd(dp_out + (int64_t)nb.y * 3 + d, -v);
       }
