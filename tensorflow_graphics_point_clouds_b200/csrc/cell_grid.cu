@@ -521,7 +521,7 @@ grid_cluster_kernel(ClusterBuild a) {
   for (int i = tid; i < boxes; i += kClusterThreads) box[0][i] = box[1][i] = 0xffffffffu;
   if (tid < D) asked[tid] = 1;
   __syncthreads();
-  // (the lanes' least keys; all of them of cloud b if `uniform`)
+  // (the lanes' least keys; `uniform`: all of them of cloud b, the same in every lane)
   auto fold = [&](const float* lo, const float* hi, int b, bool live, bool uniform) {
     unsigned kl[D], kh[D];
 #pragma unroll
@@ -582,8 +582,10 @@ grid_cluster_kernel(ClusterBuild a) {
           hi[d] = live ? fmaxf(-INFINITY, lo[d]) : -INFINITY;
           lo[d] = live ? fminf(INFINITY, lo[d]) : INFINITY;
         }
+        // (a lane without a point writes a value too where all of them lie in one cloud)
         const int first_b = __shfl_sync(0xffffffffu, b, 0);
-        fold(lo, hi, b, live, __all_sync(0xffffffffu, b == first_b || !live));
+        const bool uniform = __all_sync(0xffffffffu, b == first_b || !live);
+        fold(lo, hi, uniform ? first_b : b, live, uniform);
       }
     }
   }

@@ -31,14 +31,20 @@ class CellGrid(ctypes.Structure):
     ([12288] * 4, 3, 0.06, 36, 0, "apart"), ([7001] * 7, 3, 0.0669, 32, 0, "mixed"),
     ([49153], 3, 0.0313, 64, 0, "apart"), ([65535], 3, 0.0157, 128, 1, "apart"),
     ([65536], 2, 0.00144, 1440, 0, "mixed"), ([30000, 30000], 3, 0.4, 6, 0, "crowded"),
-    ([40000], 3, 0.2, 12, 0, "strange")])
+    ([40000], 3, 0.2, 12, 0, "strange"),
+    # a warp of two clouds whose last 32 points are fewer than a box has corners' coordinates
+    ([32768, 1], 3, 0.1, 32, 0, "apart"), ([20000, 3], 3, 0.1, 32, 0, "apart"),
+    ([20511, 2], 2, 0.02, 128, 0, "apart"), ([16992, 7], 6, 0.4, 8, 0, "apart"),
+    ([16600, 16201], 3, 0.1, 32, 0, "last")])
 def test_grid_of_one_cluster(sizes, d, cell, most, shift, form):
   rng = np.random.default_rng(5)
   n, b = sum(sizes), len(sizes)
   bid = np.repeat(np.arange(b), sizes).astype(np.int32)
   pts = rng.uniform(-1, 1, (n, d)).astype(np.float32)
-  if form == "mixed":
+  if form in ("mixed", "last"):
     rng.shuffle(bid)
+  if form == "last":               # the corner of its cloud
+    pts[-1] = 1.0625
   if form == "crowded":            # a cell of thousands, in runs and single points
     pts[5000:29000] = 0.5 + 0.01 * pts[5000:29000]
     pts[30000::3] = -0.5
