@@ -5,8 +5,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
-#include <atomic>
-
+#include "granted.h"
 #include "tfgpc.h"
 
 namespace tfgpc {
@@ -69,18 +68,17 @@ struct ProfPause {
 int sm_count();
 
 // Lets a kernel take `bytes` of dynamic shared memory: asked of the driver once per device
-// and size (every launch of a product or projection asked again, 0.6 us each).
+// and larger size (every launch of a product or projection asked again, 0.6 us each).
 template <auto kKernel>
 cudaError_t allow_shared(int bytes) {
-  static std::atomic<int> allowed[64];      // (the most so far)
+  static Granted granted[64];
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  const cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const bool known = dev >= 0 && dev < 64;
-  if (known && bytes <= allowed[dev].load(std::memory_order_relaxed)) return cudaSuccess;
-  e = cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess && known) allowed[dev].store(bytes, std::memory_order_relaxed);
-  return e;
+  auto ask = [](int size) {
+    return (int)cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, size);
+  };
+  return (cudaError_t)(dev >= 0 && dev < 64 ? granted[dev].reach(bytes, ask) : ask(bytes));
 }
 
 // Blocking read of a few values (4 .. 4096 bytes, a multiple of 4) from device

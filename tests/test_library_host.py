@@ -121,6 +121,55 @@ def test_list_parts_cover_the_list(part_end, begin, pairs, parts):
     assert b == end or share * chunk <= b - a <= (share + 1) * chunk
 
 
+GRANTED_SRC = """
+#include <chrono>
+#include <thread>
+#include "granted.h"
+// Two threads ask for `first` and `second`, the second while the first one's request is on its
+// way; then `first` is asked for again.  What the driver holds at the end.
+extern "C" int held(int first, int second) {
+  tfgpc::Granted granted;
+  std::atomic<int> driver{0}, under_way{0}, second_done{0};
+  std::thread other([&] {
+    while (!under_way) std::this_thread::yield();
+    granted.reach(second, [&](int size) { driver = size; return 0; });
+    second_done = 1;
+  });
+  granted.reach(first, [&](int size) {
+    driver = size;
+    under_way = 1;
+    for (int i = 0; i < 200 && !second_done; ++i)
+      std::this_thread::sleep_for(std::chrono::milliseconds(1));
+    return 0;
+  });
+  other.join();
+  granted.reach(first, [&](int size) { driver = size; return 0; });
+  return driver;
+}
+// A request that is refused is made again.
+extern "C" int asked_after_refusal() {
+  tfgpc::Granted granted;
+  int asked = 0;
+  granted.reach(5, [&](int) { ++asked; return 1; });
+  granted.reach(5, [&](int) { ++asked; return 0; });
+  granted.reach(5, [&](int) { ++asked; return 0; });
+  return asked;
+}
+"""
+
+
+def test_shared_memory_of_two_threads(tmp_path):
+  """The shared memory that a kernel may take is not lowered under a thread that counts on it."""
+  src, so = tmp_path / "granted.cpp", tmp_path / "granted.so"
+  src.write_text(GRANTED_SRC)
+  subprocess.run(["g++", "-O1", "-std=c++17", "-pthread", "-shared", "-fPIC", "-I", build.CSRC,
+                  str(src), "-o", str(so)], check=True)
+  lib = ctypes.CDLL(str(so))
+  assert lib.held(230656, 197888) == 230656
+  assert lib.held(197888, 230656) == 230656
+  assert lib.asked_after_refusal() == 2
+
+
 def test_sums_by_neighbor_refuse_host_memory():
   """Pointers of another device never reach the kernel: raised before any launch."""
   torch = pytest.importorskip("torch")
