@@ -78,9 +78,11 @@ class PointCloud:
     # and returns the maximum over all shards (dist.allreduce_max_), so that every
     # rank builds the keys the unsharded batch would have.
     self._num_cells_reduce = num_cells_reduce
-    # (arrays that are what the ops take already, as the output of one is, are looked at once)
+    # (arrays that are what the ops take already, as the output of one is, are looked at once;
+    # as_tensor moves the points to a default device, where one is set)
+    points = torch.as_tensor(points)
     if not _is_array(points, torch.float32):
-      points = torch.as_tensor(points).to(torch.float32).contiguous()
+      points = points.to(torch.float32).contiguous()
     if not (_is_array(batch_ids, torch.int32) and batch_ids.device == points.device):
       batch_ids = torch.as_tensor(batch_ids, device=points.device).to(torch.int32).contiguous()
     self._points, self._batch_ids = points, batch_ids

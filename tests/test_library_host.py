@@ -199,3 +199,22 @@ def test_build_cell_grid_returns_a_pair(monkeypatch):
   assert (grid, count) == ("grid", "count") and seen[0][-3:] == (5, None, 0)
   both = custom_ops.build_cell_grid_with_pdf("points", "ids", 2, [0.1] * 3, 64, "inv", pdf_mode=1)
   assert both == ("grid", "count", "pdf", "packed") and seen[1][-3:] == (0, "inv", 1)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("ids", ["int32", "int64"])
+def test_clouds_follow_the_default_device(dtype, ids):
+  """Host arrays given to a cloud go to the default device, whatever their type is, and the
+  batch ids with the points; without one they stay where they are, uncopied if they can."""
+  torch = pytest.importorskip("torch")
+  from tensorflow_graphics_point_clouds_b200 import pc
+  points = torch.zeros((4, 3), dtype=getattr(torch, dtype))
+  batch_ids = torch.zeros(4, dtype=getattr(torch, ids))
+  cloud = pc.PointCloud(points, batch_ids, 1)
+  assert cloud._points.device.type == cloud._batch_ids.device.type == "cpu"
+  assert (cloud._points is points) == (dtype == "float32")
+  assert (cloud._batch_ids is batch_ids) == (ids == "int32")
+  with torch.device("meta"):
+    cloud = pc.PointCloud(points, batch_ids, 1)
+  assert cloud._points.device.type == cloud._batch_ids.device.type == "meta"
+  assert cloud._points.dtype == torch.float32 and cloud._batch_ids.dtype == torch.int32
