@@ -434,6 +434,7 @@ class _ProjectedConv:
 
 _LIBRARY_NEIGHBORHOOD = _ProjectedConv._neighborhood
 _LIBRARY_BACKWARD = _ProjectedConv._backward
+_LIBRARY_OP_BACKWARD = ProjectionGemm.backward
 
 
 class KPConv(_ProjectedConv):
@@ -460,7 +461,9 @@ class KPConv(_ProjectedConv):
   def backward(self, out_grads):
     """(d_features, d_weights) of the last forward call; the kernel points of the
     rigid layer are not trained."""
-    if _is_own(self._backward, _LIBRARY_BACKWARD):
+    # (without those of the basis, unless somebody else's function is called on the way)
+    if (_is_own(self._backward, _LIBRARY_BACKWARD) and
+        _is_own(getattr(self._op, 'backward', None), _LIBRARY_OP_BACKWARD)):
       _, dfeat, dw = self._gradients(out_grads, want_basis=False)
     else:
       _, dfeat, dw = self._backward(out_grads)

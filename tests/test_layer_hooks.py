@@ -11,6 +11,8 @@ from tensorflow_graphics_point_clouds_b200 import mcconv, pc
     (mcconv.MCConv, "build_neighborhood", mcconv._LIBRARY_BUILD_NEIGHBORHOOD),
     (mcconv.PointConv, "_neighborhood", mcconv._LIBRARY_NEIGHBORHOOD),
     (mcconv.KPConv, "_neighborhood", mcconv._LIBRARY_NEIGHBORHOOD),
+    (mcconv.KPConv, "_backward", mcconv._LIBRARY_BACKWARD),
+    (mcconv.ProjectionGemm, "backward", mcconv._LIBRARY_OP_BACKWARD),
     (pc.Neighborhood, "get_pdf", mcconv._library_get_pdf())])
 def test_replaced_hooks_are_seen(cls, name, own, monkeypatch):
   is_own = lambda c, obj=None: mcconv._is_own(getattr(obj or object.__new__(c), name), own)
@@ -33,3 +35,27 @@ def test_a_neighborhood_of_the_users_own_is_not_the_librarys():
     def get_pdf(self, **kw):
       return None
   assert not mcconv._is_own(Mine().get_pdf, mcconv._library_get_pdf())
+
+
+@pytest.mark.parametrize("where", ["layer", "op", "class"])
+def test_kernel_points_call_replaced_gradients_as_ever(where, monkeypatch):
+  """A replaced _backward, an own _op and a wrapped ProjectionGemm.backward know nothing of
+  gradients that leave out the basis."""
+  def backward(basis, features, neighbors, ranges, weights, out_grads, reuse_forward=True,
+               blocks=None):
+    assert (basis, features, neighbors, ranges, weights, out_grads) == ("b", "f", "n", "r", "w", "g")
+    assert blocks == (1, 15, 24)
+    return "db", "df", "dw"
+
+  neigh = types.SimpleNamespace(_original_neigh_ids="n", _samples_neigh_ranges="r")
+  layer = object.__new__(mcconv.KPConv)
+  layer.k, layer.cout, layer._saved = 15, 24, (neigh, "b", "f", "w")
+  layer._op = object.__new__(mcconv.ProjectionGemm)
+  if where == "layer":
+    layer._backward = lambda out_grads: ("db", "df", "dw")
+  elif where == "op":
+    layer._op = types.SimpleNamespace(backward=backward)
+  else:
+    monkeypatch.setattr(mcconv.ProjectionGemm, "backward",
+                        lambda self, *args, **kw: backward(*args, **kw))
+  assert layer.backward("g") == ("df", "dw")
