@@ -68,6 +68,9 @@ def _is_array(t, dtype):
   return type(t) is torch.Tensor and t.dtype is dtype and t.is_contiguous()
 
 
+_LIBRARY_FILL = ops.find_neighbors_fill
+
+
 class PointCloud:
   """Segmented point cloud: points [N, D] float32 and batch ids [N] int32."""
 
@@ -353,8 +356,8 @@ class Neighborhood:
       # a self neighborhood mostly feeds the density estimate and the sampling,
       # which read sorted ids only: the original-id list is built if asked for
       self._nbrs = ops.find_neighbors_fill(self._count)
-    elif self._grid._cells is not None:
-      # (the permutation is not needed as a tensor)
+    elif self._count.cells is not None and ops.find_neighbors_fill is _LIBRARY_FILL:
+      # (the library's own needs no permutation as a tensor)
       self._nbrs, self._orig_ids = ops._cells_fill(self._count, True, None, None)
     else:
       self._nbrs, self._orig_ids = ops.find_neighbors_fill(self._count,

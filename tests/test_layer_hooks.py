@@ -59,3 +59,36 @@ def test_kernel_points_call_replaced_gradients_as_ever(where, monkeypatch):
     monkeypatch.setattr(mcconv.ProjectionGemm, "backward",
                         lambda self, *args, **kw: backward(*args, **kw))
   assert layer.backward("g") == ("df", "dw")
+
+
+@pytest.mark.parametrize("replaced", [False, True])
+@pytest.mark.parametrize("own_cloud", [False, True])
+def test_a_replaced_fill_is_called(own_cloud, replaced, monkeypatch):
+  """Every neighborhood's list comes from ops.find_neighbors_fill where somebody replaced it;
+  the library's own is spared the permutation as a tensor."""
+  asked = []
+
+  class Grid:
+    _cells = "cells"
+
+    @property
+    def _sorted_indices(self):
+      asked.append("permutation")
+      return "permutation"
+
+  def fill(count, *rest):
+    assert count is neigh._counted and rest == (() if own_cloud else ("permutation",))
+    return "list" if own_cloud else ("list", "ids")
+
+  neigh = object.__new__(pc.Neighborhood)
+  neigh._nbrs = neigh._orig_ids = None
+  neigh._counted, neigh._grid = types.SimpleNamespace(cells="cells"), Grid()
+  neigh._equal_samples = own_cloud
+  if replaced:
+    monkeypatch.setattr(pc.ops, "find_neighbors_fill", fill)
+  else:
+    monkeypatch.setattr(pc.ops, "_cells_fill", lambda count, with_ids, inv_bw, mode:
+                        ("list", "ids") if with_ids else "list")
+  assert neigh._neighbors == "list"
+  assert own_cloud or neigh._original_neigh_ids == "ids"
+  assert bool(asked) == (replaced and not own_cloud)
