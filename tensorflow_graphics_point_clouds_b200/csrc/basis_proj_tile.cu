@@ -119,11 +119,11 @@ struct PairStream {
   __device__ __forceinline__ void init(unsigned begin, unsigned last) {
     idx_after = neighbor_of(begin + lane, last);
   }
-  // the sample of the pairs [begin, end), those of the sample before ended at begin; the
-  // warp's last one ends at `last`
+  // the sample of the pairs [begin, end), those of the sample before ended at begin; none of
+  // the warp's ends behind `last`.  (An end ahead of its begin is an empty list.)
   __device__ __forceinline__ void start(unsigned begin, unsigned end, unsigned last) {
     a = begin;
-    total = end - begin;
+    total = (int)end > (int)begin ? end - begin : 0;
     at = 0;
     idx = idx_after;
     idx_next = neighbor_of(begin + 32 + lane, end);
@@ -182,7 +182,7 @@ struct WarpSamples {
     *e = (unsigned)__shfl_sync(0xffffffffu, ends, i);
   }
   __device__ __forceinline__ unsigned last() const {
-    return (unsigned)__shfl_sync(0xffffffffu, ends, count > 0 ? count - 1 : 0);
+    return (unsigned)__reduce_max_sync(0xffffffffu, max(ends, 0));
   }
 };
 
@@ -364,7 +364,7 @@ basis_proj_grads_tile_kernel(int C, int64_t ns, int64_t M, int per, const float*
 #pragma unroll
       for (int q = 0; q < kKt; q += 4) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c < have && a < e)
+        if (c < have && pairs.total > 0)
           v = ld_global(reinterpret_cast<const float4*>(
               in_grads + block_offset<K>(mine.first + i, C, c0 + c, k0 + q, shift)));
         g[c][q] = v.x; g[c][q + 1] = v.y; g[c][q + 2] = v.z; g[c][q + 3] = v.w;

@@ -86,3 +86,32 @@ def test_columns_of_several_mlps(c, k, groups):
                    (dw, torch.einsum("scgh,sgo->gcho", x4, u3).reshape(w.shape)),
                    (db, ref_db), (df, ref_df)):
     assert (got.double() - ref).norm() <= 6 * 2.0 ** -17 * ref.norm()
+
+
+@pytest.mark.parametrize("c,k", [(1, 8), (1, 64), (3, 16), (8, 8), (8, 32), (7, 64), (24, 8), (40, 16)])
+@pytest.mark.parametrize("ns", [3, 6, 300, 10000])
+def test_ranges_that_step_back(c, k, ns):
+  """A range that ends before it begins is an empty list; what lies in several samples' ranges
+  belongs to each of them (and its basis gradient to any)."""
+  g = torch.Generator(device=DEV).manual_seed(ns)
+  steps = torch.randint(-9, 13, (ns,), generator=g, device=DEV)
+  steps[0], steps[-1] = 10, 40
+  ends = torch.cumsum(steps, 0).clamp(min=1)
+  ends[1], ends[-1] = 4, ends.max() + 3
+  begins = torch.cat([ends.new_zeros(1), ends[:-1]])
+  lengths = (ends - begins).clamp(min=0)
+  owner = torch.repeat_interleave(torch.arange(ns, device=DEV), lengths)
+  pair = begins[owner] + torch.arange(len(owner), device=DEV) - (torch.cumsum(lengths, 0) - lengths)[owner]
+  m, n = int(ends[-1]), 211
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  nbr = torch.randint(0, n, (m,), generator=g, device=DEV)
+  basis, feat, up = r(m, k), r(n, c), r(ns, c, k)
+  args = (basis, feat, torch.stack([nbr, nbr], 1).int(), ends.int())
+  out = ops.basis_proj(*args)
+  db, df = ops.basis_proj_grads(*args, up)
+  ref_out, ref_db, ref_df = reference(nbr[pair], owner, basis[pair], feat, up)
+  close(out, ref_out, int(lengths.max()))
+  close(df, ref_df, k * (len(owner) // n + 1))
+  alone = torch.bincount(pair, minlength=m)[pair] == 1
+  assert alone.any()
+  close(db[pair[alone]], ref_db[alone], c)
