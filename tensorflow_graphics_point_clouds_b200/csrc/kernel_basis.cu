@@ -293,11 +293,16 @@ kernel_basis_grads_kernel(int64_t M, const float* p_in,
 //
 // Instructions bound it (1.15 million pairs of 16 values: 74 MB written, 12 us), and a division
 // per value was most of them.  The divisor is known before the launch: dist times its inverse in
-// two floats, inv + rest, by one multiplication and one fma rounds like the division (Brisebarre,
-// Muller, Raina: Accelerating correctly rounded floating-point division when the divisor is known
-// in advance; 80 million values of dist / sigma: not one differs).
-// 1.15 million pairs, us before -> now: 15 points of 16, linear 28.1 -> 24.3, Gaussian 31.8 ->
-// 28.3; 60 of 64 114 -> 92.  (A point's coordinates by one 16-byte load: 25.8, 29.4 and 118.)
+// two floats, inv + rest, by one multiplication and one fma is within an ulp of the quotient
+// (Brisebarre, Muller, Raina: Accelerating correctly rounded floating-point division when the
+// divisor is known in advance).  For most divisors that is the rounded quotient already, not for
+// all (0.48: dist 0.426666617 came out an ulp high); one correction by the remainder rounds it
+// for every one (Markstein: Computation of elementary functions on the IBM RISC System/6000
+// processor, theorem on the last step of a division).  All 2^23 mantissas of dist over 600
+// divisors: none differs from the division, 16 did without the correction.
+// 1.15 million pairs, us, by division / now / without the correction: 15 points of 16, linear
+// 28.1 / 25.2 / 24.4, Gaussian 31.8 / 29.1 / 28.5; 60 of 64 114 / 97 / 92.  (A point's coordinates
+// by one 16-byte load, without the correction: 25.8, 29.4 and 118.)
 constexpr int kMaxKernelPoints = 64;
 
 struct Divisor {
@@ -341,7 +346,9 @@ kp_basis_kernel(int64_t M, int num_kp, const float* p_in,
             d2 = fmaf(t, t, d2);
           }
           const float dist = sqrtf(d2);
-          const float r = by.by_inverse ? fmaf(dist, by.inv, dist * by.rest) : dist / by.value;
+          const float near = fmaf(dist, by.inv, dist * by.rest);
+          const float r = by.by_inverse ? fmaf(fmaf(-near, by.value, dist), by.inv, near)
+                                        : dist / by.value;
           if (interpolation == 0) {
             w = fmaxf(1.0f - r, 0.0f);
           } else {

@@ -50,3 +50,26 @@ def test_weights(d, k, num, sigma, interpolation):
       bound = want * (np.minimum(r * r, 700.0) + 4) * 2.0 ** -24 + 1e-38
       near = np.abs(out[:, :num] - want) <= bound
       assert (near | (np.isnan(want) & np.isnan(out[:, :num]))).all()
+
+
+@pytest.mark.parametrize("sigma,tie", [(0.03, 0.426666617), (0.48, 0.426666617), (1.92, 0.426666617),
+                                       (0.916666687, 0.401041716), (0.6, 0.1), (0.75, 0.1)])
+def test_quotients_round_like_a_division(sigma, tie):
+  """tie / sigma lies next to the middle of two floats, where the inverse in two floats alone
+  rounds the other way.  One coordinate, so that dist is its size: the root of its rounded square."""
+  rng = np.random.default_rng(7)
+  m, sigma = 100000, F32(sigma)
+  points = np.zeros((m, 3), F32)
+  points[:, 0] = rng.uniform(0, 1.25 * sigma, m)
+  points[0, 0], points[1, 0], points[2, 0] = 0.0, tie, -F32(tie)
+  points[3:9, 0] = F32(tie) * F32(2) ** np.arange(-6, 0)
+  nb = np.stack([np.arange(m), np.zeros(m)], 1).astype(np.int32)
+  t = [torch.as_tensor(a).cuda() for a in (points, nb)]
+  kernel, out = torch.zeros((1, 3)).cuda(), torch.empty((m, 8), device="cuda")
+  rc = _lib.lib().tfgpc_kp_basis(
+      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), 3, 8, 1, _lib.c_i64(m),
+      _lib.ptr(t[0]), _lib.ptr(t[0]), _lib.ptr(t[1]), _lib.ptr(kernel), ctypes.c_float(1.0),
+      ctypes.c_float(sigma), 0, _lib.ptr(out))
+  assert rc == 0
+  want = np.fmax(F32(1) - np.abs(points[:, 0]) / sigma, F32(0))
+  assert np.array_equal(out.cpu().numpy()[:, 0], want)
