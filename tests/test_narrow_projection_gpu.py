@@ -52,10 +52,9 @@ def test_against_64_bits(c, offset, k, lengths):
   if lengths == "many" and c * k > 512:
     pytest.skip("the reference's [pairs, C, K] arrays")
   nbr, owner, pairs, ends, basis, feat, up = case(c, k, LENGTHS[lengths], 97 * c + k, offset)
-  if k > 8 and c % 16 == 0:
-    pytest.skip("on the tensor cores")
-  out = ops.basis_proj(basis, feat, pairs, ends)
-  db, df = ops.basis_proj_grads(basis, feat, pairs, ends, up)
+  # (without scratch no layer goes to the tensor cores)
+  out = ops.basis_proj(basis, feat, pairs, ends, scratch=False)
+  db, df = ops.basis_proj_grads(basis, feat, pairs, ends, up, scratch=False)
   m, most = len(owner), max(LENGTHS[lengths])
   ref_out, ref_db, ref_df = reference(nbr, owner, basis[:m], feat, up)
   close(out, ref_out, most)
