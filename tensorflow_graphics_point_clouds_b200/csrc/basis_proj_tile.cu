@@ -17,13 +17,21 @@
 //              K = 16, C = 8  13 -> 7, 19 -> 17, (71, 79)     C = 3  17 -> 7, 27 -> 15, (61, 69)
 //              K = 32, C = 1  27 -> 7, 47 -> 17, 114 -> 91    C = 8  15 -> 7, 44 -> 28, 247 -> 127
 //              K = 64, C = 1  48 -> 5, 103 -> 35, 228 -> 115  C = 8  21 -> 9, 201 -> 58, 729 -> 223
-//              K = 32, C = 24 21 -> 15, 191 -> 134, 765 -> 534
+//              K = 32, C = 16 15 -> 10, 99 -> 68, 433 -> 275     C = 24 21 -> 15, 191 -> 132, 764 -> 519
 //   gradients  K =  8, C = 1  42 -> 13, 74 -> 14, 158 -> 49   C = 8  29 -> 13, 46 -> 22, 148 -> 87
 //              K = 16, C = 3  81 -> 13, 154 -> 24, 311 -> 109 C = 8  41 -> 13, 67 -> 31, 225 -> 133
 //              K = 32, C = 1  153 -> 13, 308 -> 41, 624 -> 130   K = 64  294 -> 10, 577 -> 55, 1166 -> 214
 //              K =  8, C = 64 29 -> 21, 101 -> 82, 373 -> 334    C = 128 (27, 31, 128, 161, 494, 605)
 //              K = 16, C = 24 31 -> 20, 111 -> 90, 415 -> 350  K = 64  134 -> 51, 833 -> 246, 3385 -> 973
-// (bytes of K = 64, C = 1 at 6450 GB/s: 92 and 179 us).  Bound by HBM for one channel, else by
+//              K = 32, C = 16 34 -> 17, 143 -> 98, 486 -> 366  C = 24 44 -> 28, 238 -> 228, 877 -> 858
+// (bytes of K = 64, C = 1 at 6450 GB/s: 92 and 179 us.)
+// Above eight channels the forward tiles are taken at K = 32 alone; elsewhere (us, the lanes of
+// basis_proj.cu or the wide kernel, tiles in brackets, the same samples) they lose on many:
+//              K =  8, C = 24 12, 29, 117 (7, 23, 140)         C = 64 13, 42, 190 (10, 44, 243)
+//              K = 16, C = 24 12, 35, 158 (10, 44, 265)        C = 56 15, 65, 286 (15, 112, 461)
+//              K = 64, C = 24 23, 119, 455 (23, 198, 778)
+// (K = 64, C = 16, which only calls without scratch bring here: 34, 321, 1287 (15, 114, 443).)
+// Bound by HBM for one channel, else by
 // the latency of the gathers (13 to 20 warps an SM, issue 35 to 50 %) and the instructions
 // around the multiply-adds.
 #include "basis_proj.cuh"
@@ -398,8 +406,10 @@ basis_proj_grads_tile_kernel(int C, int64_t ns, int64_t M, int per, const float*
         constexpr int kStepsF = log2_of(tile::kKl);
         fold<CT, kStepsF, 1>(df, lane, 1, &at, &owner);
         // (by predicate; where few lanes of a small K have something, those lanes branch first.
-        // 65 536 samples, us, branch and predicate: K = 32, C = 8 256 / 214, K = 64, C = 24
-        // 1024 / 973, K = 8, C = 24 208 / 246, K = 16, C = 24 350 / 440)
+        // 65 536 samples, us, branch and predicate: one channel block K = 32, C = 8 256 / 214;
+        // two K = 8, C = 16 136 / 129, K = 16 212 / 212, K = 32 376 / 366, K = 64 540 / 540; four
+        // K = 8, C = 24 208 / 246, K = 16 350 / 440, K = 64 980 / 975.  K = 32 with four, 652 / 858,
+        // would gain from the branch too, and is left as it is)
         constexpr bool kBranch = CL > 2 && K <= 16;
         if (!kBranch || (owner && live))
           add_values<folded<CT, kStepsF, 1>()>(dfeat + (int64_t)j * C + c0 + at, df, C - c0 - at, vec,
@@ -512,7 +522,9 @@ int with_basis(int K, const Call& call) {
 
 // Whether these kernels take a layer: where they were the faster ones (figures above).  Up to
 // eight channels anything goes; more are read as 16-byte pieces.  Many samples fill the GPU
-// with a few lanes each, and at K <= 16 those then spend fewer instructions on a pair.
+// with a few lanes each, and at K <= 16 those then spend fewer instructions on a pair (8 channels
+// of 65 536 samples: lanes 57 and 70 us at K = 8 and 16, tiles 51 and 78; 3 channels 37 and 61, 43
+// and 68).
 bool basis_proj_tile_takes(int K, int C, int64_t ns, const float* feat) {
   if (C > 8) return C <= FwdCall::most_channels(K) && (uintptr_t)feat % 16 == 0;
   return K >= 32 || C == 1 || ns <= 32768;
