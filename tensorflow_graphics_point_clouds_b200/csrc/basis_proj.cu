@@ -8,8 +8,10 @@
 // traffic and no barriers in the neighbor loop.  (The reference: one 64-thread
 // block per (sample, 8 channels), two __syncthreads per neighbor step,
 // basis_proj_kernels.cu.cc:30-127.)
-// Layers of few channels mostly take the warp tiles of basis_proj_tile.cu; to G < 32 come here
-// those whose rows are not 16-byte aligned and, of K <= 16, forward passes over many samples.
+// Layers of few channels mostly take the warp tiles of basis_proj_tile.cu.  Here come, forward,
+// those of more than eight channels (at K = 32 with features off 16 bytes) and, of K <= 16, those
+// over many samples; gradients of more than eight channels whose features are off 16 bytes or,
+// beyond the tiles' channels, whose dbasis or dfeat is (with VEC: dbasis alone).
 #include "basis_proj.cuh"
 #include "basis_proj_wide.cuh"
 #include "prepare.cuh"
@@ -150,9 +152,9 @@ basis_proj_kernel(int C, int64_t ns, int G, const float* __restrict__ basis,
 // fit one pass, else accumulated with atomics.
 // Launched after its predecessor's end, unlike most kernels here, as is basis_proj_kernel:
 // its loads are then read-only ones, which the compiler takes ahead of the writes of the
-// pair before.  14 892 samples with 32 pairs, 32 basis functions, us, chained and not:
-// gradients 490 / 253 at one channel, 178 / 107 at three, 104 / 89 at eight; forward 53 / 43,
-// 31 / 30, 42 / 38.
+// pair before.  65 536 samples of 33 pairs, us, so and chained: gradients with features off 16
+// bytes K = 8, C = 24 285 / 295, K = 16, C = 24 448 / 449, K = 32, C = 24 877 / 949; forward K = 8,
+// C = 24 119 / 135, C = 64 190 / 211, K = 16, C = 24 158 / 155.
 template <int K, bool VEC>
 __global__ void __launch_bounds__(kBpThreads)
 basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __restrict__ basis,
@@ -173,8 +175,9 @@ basis_proj_grads_kernel(int C, int64_t ns, int64_t M, int G, const float* __rest
          i += warps * 32)
       dbasis[i] = 0.0f;
   };
-  // (first where registers are left, else last: 15 000 samples of 30 pairs, first and last, us:
-  // K = 32, C = 3 130 / 119, C = 16 189 / 175, C = 24 316 / 299; K = 16, C = 24 130 / 133)
+  // (first where registers are left, else last: the same samples, features off 16 bytes, first
+  // and last, us: K = 8, C = 24 285 / 288, K = 16, C = 24 448 / 450, K = 32, C = 16 526 / 487,
+  // C = 24 931 / 877, K = 64, C = 16 2122 / 2017)
   if (K < 32 && single_pass) clear_rest();
   for (int64_t s0 = warp0 * groups_per_warp; s0 < ns; s0 += warps * groups_per_warp) {
     const int64_t s = s0 + lane / G;
@@ -353,19 +356,13 @@ static int launch_basis_proj(cudaStream_t st, int C, int64_t ns, const float* ba
     TFGPC_LAUNCH_CHECK();
     return TFGPC_OK;
   }
-  if (vec) {
-    auto kern = basis_proj_kernel<K, true, OUT>;
-    if (smem > 48 * 1024)
-      TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
-    TFGPC_LAUNCH_CHECK();
-  } else {
-    auto kern = basis_proj_kernel<K, false, OUT>;
-    if (smem > 48 * 1024)
-      TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
-    TFGPC_LAUNCH_CHECK();
-  }
+  auto kern = basis_proj_kernel<K, false, OUT>;
+  if constexpr (kCpl == 4)
+    if (vec) kern = basis_proj_kernel<K, true, OUT>;
+  if (smem > 48 * 1024)
+    TFGPC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<grid, kBpThreads, smem, st>>>(C, ns, G, basis, feat, neigh, ranges, out, hi, mid, shift);
+  TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }
 
@@ -418,12 +415,11 @@ static int launch_basis_proj_grads(cudaStream_t st, int C, int64_t ns, int64_t M
     }
     return TFGPC_OK;
   }
-  if (vec)
-    basis_proj_grads_kernel<K, true><<<grid, kBpThreads, 0, st>>>(
-        C, ns, M, G, basis, feat, neigh, ranges, in_grads, dbasis, dfeat, shift);
-  else
-    basis_proj_grads_kernel<K, false><<<grid, kBpThreads, 0, st>>>(
-        C, ns, M, G, basis, feat, neigh, ranges, in_grads, dbasis, dfeat, shift);
+  auto kern = basis_proj_grads_kernel<K, false>;
+  if constexpr (kCpl == 4)
+    if (vec) kern = basis_proj_grads_kernel<K, true>;
+  kern<<<grid, kBpThreads, 0, st>>>(C, ns, M, G, basis, feat, neigh, ranges, in_grads, dbasis, dfeat,
+                                    shift);
   TFGPC_LAUNCH_CHECK();
   return TFGPC_OK;
 }

@@ -13,8 +13,8 @@
 // on the read-only path, like the narrow kernels (basis_proj.cu): plain loads stay behind the
 // writes of the sample before and cost registers.  CHAINED true: set up while the predecessor
 // runs, with plain loads; only for K = 8, whose few accumulators leave room (wide_chained).
-// Chained and not, us, lists of 30: 15 000 samples, gradients, K = 64: C = 24 1035 / 840, C = 64
-// 1932 / 1577, C = 128 3803 / 3070; forward, K = 64, C = 72 364 / 329.  900 samples, forward,
+// Chained and not, us, lists of 30: 15 000 samples, gradients, K = 64: C = 64 1932 / 1577,
+// C = 128 3803 / 3070; forward, K = 64, C = 72 364 / 329.  900 samples, forward,
 // C = 256: K = 16 19.8 / 15.0, K = 64 94 / 68.  But K = 8, forward, one pass over the channels, C = 128:
 // 56.6 / 60.1 and 5.6 / 7.0 at 900 samples (two passes, C = 256: 110.4 / 111.3 and 12.5 / 11.0);
 // gradients, C = 128 136 / 140, C = 136 256 / 255 and 24.0 / 25.3.
