@@ -412,9 +412,9 @@ basis_proj_mma_kernel(int bs, int shift, int C, int64_t ns, const float* basis,
 // While a chunk is multiplied the next one's feature and basis rows are on their way to the
 // team's other stage, and dX of the next sample to the place that this one's has left for
 // registers.
-// What bounds it: the SM's L1 data path (62 % of its wavefronts, 75 % on the busiest SM:
+// What bounds it: the SM's L1 data path (62 % of its wavefronts, 69 % on the busiest SM:
 // copies into shared memory, operand reads, reductions at ~24 B/clk) and the instructions
-// around the MMAs (issue 50 %).  What teams and fragments gave, 65 536 samples of 28 pairs at
+// around the MMAs (issue 51 %).  What teams and fragments gave, 65 536 samples of 28 pairs at
 // C = 64, K = 32: 345 -> 290 us (now 54 500 of 32 pairs: 235, 0.9 GB: 3.8 TB/s); 41 000 at
 // C = 64, K = 16: 166 -> 139, without the gradient of the basis 86 (the reductions of 1.15
 // million rows: 60).  (One warp per sample with dX as bf16 rows in shared memory, read by

@@ -32,7 +32,7 @@
 //              K = 64, C = 24 23, 119, 455 (23, 198, 778)
 // (K = 64, C = 16, which only calls without scratch bring here: 34, 321, 1287 (15, 114, 443).)
 // Bound by HBM for one channel, else by
-// the latency of the gathers (13 to 20 warps an SM, issue 35 to 50 %) and the instructions
+// the latency of the gathers (10 to 17 warps an SM, issue 28 to 52 %) and the instructions
 // around the multiply-adds.
 #include "basis_proj.cuh"
 

@@ -414,7 +414,7 @@ constexpr int kClusterBoxes = 1024;        // batch size x D at most
 // them alone, so a large one goes to the whole GPU.  The sorted copies scatter 44 bytes
 // a point: from 8192 points on they are a launch of their own (41 000 points: 13 us of
 // the cluster's 33, 4.4 by themselves).
-// It is bound by its six barriers (about 1200 cycles each) and, between them, by single trips
+// It is bound by its barriers (900 to 1900 cycles each) and, between them, by single trips
 // to L2 and by instructions that are not in the cache yet: 11 us for 4096 points.  Hence each
 // trip is made once, for all points of a thread together: points are read for the boxes and
 // kept until the cell is known, bucket and number until the place is; a warp takes neighboring
@@ -422,7 +422,7 @@ constexpr int kClusterBoxes = 1024;        // batch size x D at most
 // of the block per 4096 cells; sums go to the other blocks before a barrier instead of being
 // fetched after it.  us before -> now, kernel: 42 000 points in 7300 cells 23 -> 19, 38 000 in
 // 226 000 28 -> 18; 3-level cell averages of 5 x 9000 points 171 -> 158, three-level classifier
-// 668 -> 639, layer step on 59 000 points 208 -> 203.  Left: the atomics of 16 SMs (7300 cycles
+// 668 -> 639 (its runs differ by up to 15 %), layer step on 59 000 points 208 -> 203.  Left: the atomics of 16 SMs (7300 cycles
 // for 59 000 points, about two per atomic of an SM).
 constexpr int kMaxRanks = 16;
 constexpr int kHeld = 4;                   // points of a thread at most

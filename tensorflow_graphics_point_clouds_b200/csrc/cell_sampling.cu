@@ -37,8 +37,8 @@ constexpr size_t kHeadBytes = (size_t)(kMaxTeams + 4) * 4;   // barrier words be
 // left for it: spills, 1 % of a hierarchy); one over all points of a call takes some 30 ns
 // a point, which the period of the barriers allows for.
 constexpr int kProgressMarks = 65536;
-// Points of a cell whose average its warp works out together, 32 points' loads at a time, and
-// adds up in the same order.  (By one thread, four loads at a time, the cells of several
+// A cell of more points than that has its average worked out by its warp together, 32 points'
+// loads at a time, added up in the same order.  (By one thread, four loads at a time, the cells of several
 // hundred points decided: 5 x 9001 points, cells of 0.04, 22 -> 13 us in this kernel.)
 constexpr int kLongCell = 64;
 inline unsigned long long barrier_period_ns(int64_t n) { return 500000000ull + 100ull * n; }
