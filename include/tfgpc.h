@@ -303,6 +303,18 @@ int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
                         const int32_t* samples_batch_ids, int samples_are_points,
                         float* pdf_out);
 
+/* The same for the grid's own points (samples_are_points 1 or 2) by half the distance
+ * tests, with a workspace of 8 bytes a point, 8-byte aligned (NULL: as without).
+ * tfgpc_cells_density_workspace_bytes: those bytes where that is faster on a grid of n
+ * points with `pairs` neighbor pairs, else 0. */
+size_t tfgpc_cells_density_workspace_bytes(int D, int64_t n, int64_t pairs);
+int tfgpc_cells_density_ws(void* stream, const tfgpc_cell_grid* grid,
+                           const float* inv_radii, const float* inv_bandwidth,
+                           int mode, int64_t ns, const float* samples,
+                           const int32_t* samples_batch_ids,
+                           int samples_are_points, void* ws, size_t ws_bytes,
+                           float* pdf_out);
+
 /* Sampling (tfgpc_sampling_count + _store) on a built grid without a neighbor list:
  * mode 0 Poisson disk with the neighbors of a self neighborhood without limit
  * (inv_radii [D]), mode 1 cell average.  The outputs hold n rows, the first

@@ -51,6 +51,8 @@ SYMBOLS = {
     "tfgpc_cells_count": c_int,
     "tfgpc_cells_fill": c_int,
     "tfgpc_cells_density": c_int,
+    "tfgpc_cells_density_workspace_bytes": c_sz,
+    "tfgpc_cells_density_ws": c_int,
     "tfgpc_cells_sample_workspace_bytes": c_sz,
     "tfgpc_cells_sample": c_int,
     "tfgpc_cell_grid_sample": c_int,

@@ -218,10 +218,15 @@ cells_walk_kernel(WalkArgs a) {
       const int candidates = __shfl_sync(0xffffffffu, before, 31);
       const int offset = r.y - before;   // sorted index of candidate i of this tube: i + offset
       for (int base = 0; base < candidates; base += 32 * kSteps) {
+        const int steps = (min(candidates - base, 32 * kSteps) + 31) >> 5;
         f32x2 np[D][kSteps / 2];         // negated coordinates of the lane's candidates
         int at[kSteps], index[kSteps];
 #pragma unroll
         for (int k = 0; k < kSteps; k += 2) {
+          // (few candidates: half the places stay empty.  524 288 points with 12 neighbors, density
+          // 131 -> 108 us in three dimensions, 76 -> 65 in two; a branch per pair of steps costs
+          // small clouds more than it saves, 10.6 -> 11.6 us, and four dimensions 3 % here too)
+          if (MODE == kDensity && D <= 3 && k >= kSteps / 2 && steps <= kSteps / 2) continue;
           float p[2][D];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
@@ -241,7 +246,6 @@ cells_walk_kernel(WalkArgs a) {
 #pragma unroll
           for (int d = 0; d < D; ++d) np[d][k / 2] = pack2(-p[0][d], -p[1][d]);
         }
-        const int steps = (min(candidates - base, 32 * kSteps) + 31) >> 5;
         for (unsigned todo = members; todo; todo &= todo - 1u) {
           const int who = __ffs(todo) - 1;
           float one[D];
@@ -337,6 +341,218 @@ cells_walk_kernel(WalkArgs a) {
     if (D == 3 && a.packed)
       a.packed[s.id] = make_float4(s.p[0], s.p[1], s.p[D - 1], 1.0f / density);
   }
+}
+
+// ---- densities of the grid's own points by half the tests ---------------------------
+//
+// The relation is symmetric, and so are the rounded differences: a pair is worked out once,
+// at the point that comes first in the sorted order, and counts for both.
+
+// A sum of exponentials as a whole number: sums of such numbers come out the same in any order.
+// (A density of a point is at least the one of itself, the sum of a density 1: 2^-32 of that is
+// 1/256 of the float's last place.)
+constexpr float kDensityUnit = 4294967296.0f;
+__device__ __forceinline__ void add_density(unsigned long long* sums, int j, float v) {
+  atomicAdd(sums + j, __float2ull_rn(v * kDensityUnit));
+}
+
+struct DensityScale {
+  float hi, lo;
+};
+__device__ __forceinline__ float density_bandwidth(const WalkArgs& a, int d) {
+  return a.bw_mode == 1 ? sqrtf((float)a.c.n) : ld_global(a.inv_bw + d);
+}
+__device__ __forceinline__ DensityScale density_scale(float bw) {
+  const double factor = (double)bw * bw * (-0.5 * 1.4426950408889634);
+  const float hi = (float)factor;
+  return DensityScale{hi, (float)(factor - (double)hi)};
+}
+
+// The walk of cells_walk_kernel over the sorted points, with the candidates behind a cell's first
+// sample only: a lane keeps the sums of its candidates over the cell's samples beside theirs.
+// Two tests in some 19 instructions count for four, where two of kDensity take 17.  530 366 points
+// of surfaces (260 neighbors): 529 -> 320 us; the rule and more figures are at
+// tfgpc_cells_density_workspace_bytes.  Error against 64 bits, rms over 2 to 4 dimensions and
+// bandwidths of 0.05 to 1: 2.0e-8 to 5.3e-8, where kDensity has 1.8e-8 to 7.4e-8 (it rounds every
+// term onto one sum; here half of them come in sums of at most 16, as whole numbers).  Bound by issue
+// slots like the other walks; 16 more pairs of sums and places per lane, 78 registers.
+template <int D>
+__global__ void __launch_bounds__(kThreads)
+cells_density_half_kernel(WalkArgs a, unsigned long long* sums) {
+  chain_enter();
+  constexpr int kSteps = D <= 3 ? 8 : 4;
+  constexpr int kTubes = num_tubes<D>();
+  constexpr int kTop = kTubes > 16 ? 16 : kTubes > 8 ? 8 : kTubes > 4 ? 4 : 2;
+  const CellsView& c = a.c;
+  const int lane = lane_id();
+  const int64_t v0 = (((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5) * a.span;
+  if (v0 >= a.ns) return;
+  const Grid<D> g = load_grid<D>(c.num_cells, c.inv_cell);
+  const int total = total_cells<D>(g.nc, c.batch_size);
+  if (total == 0) return;
+  f32x2 inv_r[D], scale[D], scale_lo[D];
+  bool isotropic = true;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float r = ld_global(a.inv_radii + d);
+    inv_r[d] = pack2(r, r);
+    const DensityScale f = density_scale(density_bandwidth(a, d));
+    scale[d] = pack2(f.hi, f.hi);
+    scale_lo[d] = pack2(f.lo, f.lo);
+    isotropic = isotropic && scale[d] == scale[0] && scale_lo[d] == scale_lo[0];
+  }
+  const bool live = lane < a.span && v0 + lane < a.ns;
+  const Sample<D> s = load_sample<D>(c, SampleSource{2, nullptr, nullptr}, v0 + lane, live, g);
+  float my_density = 0.0f;
+  if (s.key >= 0) {          // the point itself, unless it is no neighbor of itself (no number)
+    bool finite = true;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      float r, unused;
+      unpack2(inv_r[d], r, unused);
+      finite = finite && (s.p[d] - s.p[d]) * r == 0.0f;
+    }
+    my_density = finite ? 1.0f : 0.0f;
+  }
+  unsigned open = __ballot_sync(0xffffffffu, s.key >= 0);
+  while (open) {
+    const int leader = __ffs(open) - 1;
+    const int leader_key = __shfl_sync(0xffffffffu, s.key, leader);
+    const unsigned members = __ballot_sync(0xffffffffu, s.key == leader_key);
+    open &= ~members;
+    int cell[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) cell[d] = __shfl_sync(0xffffffffu, s.cell[d], leader);
+    const int batch = __shfl_sync(0xffffffffu, s.batch, leader);
+    const int after = (int)v0 + leader + 1;
+    for (int tube0 = 0; tube0 < kTubes; tube0 += 32) {
+      int2 r = make_int2(0, 0);
+      if (tube0 + lane < kTubes)
+        r = tube_points<D>(kTubes - 1 - (tube0 + lane), cell, batch, g.nc, total, c.start);
+      r.x = min(max(r.x, after), r.y);       // (behind the cell's first sample only)
+      int before = r.y - r.x;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += y;
+      }
+      const int candidates = __shfl_sync(0xffffffffu, before, 31);
+      const int offset = r.y - before;
+      for (int base = 0; base < candidates; base += 32 * kSteps) {
+        const int steps = (min(candidates - base, 32 * kSteps) + 31) >> 5;
+        f32x2 np[D][kSteps / 2], sum2[kSteps / 2];
+        int at[kSteps];
+#pragma unroll
+        for (int k = 0; k < kSteps; k += 2) {
+          if (k >= steps) continue;
+          float p[2][D];
+          sum2[k / 2] = 0ull;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int i = base + 32 * (k + u) + lane;
+            int t = 0;
+#pragma unroll
+            for (int o = kTop; o > 0; o >>= 1) {
+              const int y = __shfl_sync(0xffffffffu, before, t + o - 1);
+              if (y <= i) t += o;
+            }
+            at[k + u] = i + __shfl_sync(0xffffffffu, offset, t & 31);
+            int unused;
+#pragma unroll
+            for (int d = 0; d < D; ++d) p[u][d] = INFINITY;
+            if (i < candidates) load_point<D>(c, at[k + u], p[u], &unused);
+          }
+#pragma unroll
+          for (int d = 0; d < D; ++d) np[d][k / 2] = pack2(-p[0][d], -p[1][d]);
+        }
+        for (unsigned todo = members; todo; todo &= todo - 1u) {
+          const int who = __ffs(todo) - 1;
+          const int self = (int)v0 + who;
+          f32x2 sp[D], acc2 = 0ull;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            const float x = __shfl_sync(0xffffffffu, s.p[d], who);
+            sp[d] = pack2(x, x);
+          }
+#pragma unroll
+          for (int k = 0; k < kSteps; k += 2) {
+            if (k < steps) {
+              f32x2 t2[D], d2, e2;
+#pragma unroll
+              for (int d = 0; d < D; ++d) {
+                t2[d] = mul2(add2(sp[d], np[d][k / 2]), inv_r[d]);
+                d2 = d == 0 ? mul2(t2[d], t2[d]) : fma2(t2[d], t2[d], d2);
+              }
+              if (isotropic) {
+                e2 = fma2(d2, scale[0], mul2(d2, scale_lo[0]));
+              } else {
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                  const f32x2 sq = mul2(t2[d], t2[d]);
+                  const f32x2 low = d == 0 ? mul2(sq, scale_lo[d]) : fma2(sq, scale_lo[d], e2);
+                  e2 = fma2(sq, scale[d], low);
+                }
+              }
+              float dist[2], e[2];
+              unpack2(d2, dist[0], dist[1]);
+              unpack2(e2, e[0], e[1]);
+#pragma unroll
+              for (int u = 0; u < 2; ++u) {
+                bool hit = dist[u] < 1.0f;
+                // (the sample's own cell begins the candidates: fewer than 16 of its warp's)
+                if (k + u == 0) hit = hit && at[0] > self;
+                e[u] = hit ? exp2_approx(e[u]) : 0.0f;
+              }
+              const f32x2 both = pack2(e[0], e[1]);
+              acc2 = add2(acc2, both);
+              sum2[k / 2] = add2(sum2[k / 2], both);
+            }
+          }
+          float x, y;
+          unpack2(acc2, x, y);
+          x = warp_sum(x + y);
+          if (lane == who) my_density += x;
+        }
+#pragma unroll
+        for (int k = 0; k < kSteps; k += 2) {
+          if (k < steps) {
+            float x, y;
+            unpack2(sum2[k / 2], x, y);
+            if (x > 0.0f) add_density(sums, at[k], x);
+            if (y > 0.0f) add_density(sums, at[k + 1], y);
+          }
+        }
+      }
+    }
+  }
+  if (my_density > 0.0f) add_density(sums, (int)v0 + lane, my_density);
+}
+
+// The densities from the sums: of sorted point v to its original place (mode 1) or to v (2).
+template <int D>
+__global__ void __launch_bounds__(256)
+density_of_sums_kernel(WalkArgs a, const unsigned long long* sums) {
+  chain_enter();
+  const int64_t v = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (v >= a.ns) return;
+  if (total_cells<D>(load_grid<D>(a.c.num_cells, a.c.inv_cell).nc, a.c.batch_size) == 0)
+    return;                  // (a grid that got no cells: its sorted arrays hold nothing)
+  double norm = 1.0 / (double)kDensityUnit;
+  float worst = 0.0f;        // (no number where an exponent's factor is none)
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float bw = density_bandwidth(a, d);
+    const DensityScale f = density_scale(bw);
+    worst += f.hi * 0.0f + f.lo * 0.0f;
+    norm *= bw * 0.3989422804014327;
+  }
+  float p[D];
+  int index;
+  load_point<D>(a.c, v, p, &index);
+  const float density = (float)((double)ld_global(sums + v) * norm) + worst;
+  const int64_t row = a.src.mode == 1 ? index : v;
+  a.density[row] = density;
+  if (D == 3 && a.packed) a.packed[row] = make_float4(p[0], p[1], p[D - 1], 1.0f / density);
 }
 
 // Samples per warp: more of them share the candidates of a cell (a cell of a uniform
@@ -447,13 +663,24 @@ struct DensityRequest {
   float4* packed;
 };
 
+// sums: [n] zeros, for the densities of the grid's own points, or null.
 int enqueue_density(cudaStream_t st, const tfgpc_cell_grid& g, const SampleSource& src, int64_t ns,
-                    const float* inv_radii, const DensityRequest& d) {
+                    const float* inv_radii, const DensityRequest& d, unsigned long long* sums) {
   WalkArgs a = walk_args(g, src, ns, inv_radii, 0);
   a.inv_bw = d.inv_bandwidth;
   a.bw_mode = d.mode;
   a.density = d.pdf;
   a.packed = d.packed;
+  if (sums) {
+    a.span = samples_per_warp(ns);
+    const unsigned blocks = blocks_for((ns + a.span - 1) / a.span, kThreads / 32);
+    ProfScope prof(st, "compute_pdf");
+    TFGPC_DIM_SWITCH(g.D,
+        TFGPC_CUDA(launch_chained(st, blocks, kThreads, 0, cells_density_half_kernel<kD>, a, sums));
+        TFGPC_CUDA(launch_chained(st, blocks_for(ns, 256), 256, 0, density_of_sums_kernel<kD>, a,
+                                  sums)));
+    return TFGPC_OK;
+  }
   return launch_walk<kDensity>(st, "compute_pdf", g.D, a);
 }
 
@@ -499,7 +726,8 @@ int grid_neighborhood(cudaStream_t st, const tfgpc_cell_grid* grid, const float*
   }
   if (density) {
     rc = mark_report(st);
-    if (!rc) rc = enqueue_density(st, g, SampleSource{1, nullptr, nullptr}, g.n, inv_radii, *density);
+    if (!rc) rc = enqueue_density(st, g, SampleSource{1, nullptr, nullptr}, g.n, inv_radii, *density,
+                                  nullptr);
     if (rc) return rc;
   }
   return finish_report(st, g.D, g.max_cells, ns > 0, num_cells_host_out, total_out, density != nullptr);
@@ -600,11 +828,12 @@ extern "C" int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid, const
   return launch_walk<kFill>((cudaStream_t)stream, "find_neighbors_fill", grid->D, a);
 }
 
-extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
-                                   const float* inv_radii, const float* inv_bandwidth, int mode,
-                                   int64_t ns, const float* samples,
-                                   const int32_t* samples_batch_ids, int samples_are_points,
-                                   float* pdf_out) {
+namespace {
+
+int cells_density(cudaStream_t st, const tfgpc_cell_grid* grid, const float* inv_radii,
+                  const float* inv_bandwidth, int mode, int64_t ns, const float* samples,
+                  const int32_t* samples_batch_ids, int samples_are_points, void* ws,
+                  size_t ws_bytes, float* pdf_out) {
   int rc = check_cell_grid("ComputePdf", grid);
   if (rc) return rc;
   rc = check_samples("ComputePdf", grid, ns, samples, samples_batch_ids, samples_are_points, 0);
@@ -612,7 +841,49 @@ extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
   TFGPC_REQUIRE(mode == 0 || mode == 1, "ComputePdf expects mode 0 or 1 (got %d)", mode);
   if (ns == 0) return TFGPC_OK;
   TFGPC_REQUIRE(inv_radii && pdf_out && (mode == 1 || inv_bandwidth), "ComputePdf got a null pointer");
-  return enqueue_density((cudaStream_t)stream, *grid,
-                         SampleSource{samples_are_points, samples, samples_batch_ids}, ns,
-                         inv_radii, DensityRequest{inv_bandwidth, mode, pdf_out, nullptr});
+  unsigned long long* sums = nullptr;
+  if (ws && samples_are_points != 0) {
+    if (ws_bytes < (size_t)ns * 8) return fail(TFGPC_ENOMEM, "ComputePdf workspace too small");
+    TFGPC_REQUIRE((uintptr_t)ws % 8 == 0, "ComputePdf expects an 8-byte aligned workspace");
+    sums = (unsigned long long*)ws;
+    TFGPC_CUDA(cudaMemsetAsync(sums, 0, (size_t)ns * 8, st));
+  }
+  return enqueue_density(st, *grid, SampleSource{samples_are_points, samples, samples_batch_ids},
+                         ns, inv_radii, DensityRequest{inv_bandwidth, mode, pdf_out, nullptr}, sums);
+}
+
+}  // namespace
+
+extern "C" int tfgpc_cells_density(void* stream, const tfgpc_cell_grid* grid,
+                                   const float* inv_radii, const float* inv_bandwidth, int mode,
+                                   int64_t ns, const float* samples,
+                                   const int32_t* samples_batch_ids, int samples_are_points,
+                                   float* pdf_out) {
+  return cells_density((cudaStream_t)stream, grid, inv_radii, inv_bandwidth, mode, ns, samples,
+                       samples_batch_ids, samples_are_points, nullptr, 0, pdf_out);
+}
+
+// Half the tests pay where a cell's samples have many candidates: what a cell costs before its
+// first test stays, each candidate's sum takes an atomic, and there are a launch and a memset
+// more.  us, all tests / half of them: surfaces of 130 to 260 neighbors, 65 536 points 97 / 76,
+// 524 288 471 / 315; four dimensions with 34 (560 candidates) 65 536 points 52 / 47, 524 288
+// 307 / 241, with 12 (200) 37 / 35 and 229 / 183; three with 34 (220) 23 / 27 and 131 / 125, with
+// 12 (77) 24 / 27 and 131 / 123; two with 34 (97) 15 / 20 and 73 / 79.  The candidates are
+// estimated as those of a uniform cloud with `pairs` neighbors in all.
+extern "C" size_t tfgpc_cells_density_workspace_bytes(int D, int64_t n, int64_t pairs) {
+  constexpr int64_t kPoints = 65536;
+  constexpr double kCandidates = 256.0;
+  // 3^D cells over the unit ball's volume
+  constexpr double kPerNeighbor[] = {2.86, 6.45, 16.4, 46.2, 141.0};
+  if (!valid_dims(D) || n < kPoints || n >= (int64_t)INT32_MAX) return 0;
+  return (double)pairs * kPerNeighbor[D - TFGPC_MIN_DIMS] >= kCandidates * (double)n ? (size_t)n * 8 : 0;
+}
+
+extern "C" int tfgpc_cells_density_ws(void* stream, const tfgpc_cell_grid* grid,
+                                      const float* inv_radii, const float* inv_bandwidth, int mode,
+                                      int64_t ns, const float* samples,
+                                      const int32_t* samples_batch_ids, int samples_are_points,
+                                      void* ws, size_t ws_bytes, float* pdf_out) {
+  return cells_density((cudaStream_t)stream, grid, inv_radii, inv_bandwidth, mode, ns, samples,
+                       samples_batch_ids, samples_are_points, ws, ws_bytes, pdf_out);
 }

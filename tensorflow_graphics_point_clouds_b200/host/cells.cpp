@@ -233,13 +233,17 @@ static py::tuple fill_neighbors(const CountPtr& c, bool with_ids) {
                         with_ids ? py::cast(both.select(0, 1)) : py::object(py::none()));
 }
 
-// Density at every point of the grid, in the unsorted (mode 1) or sorted (2) order.
+// Density at every point of the grid, in the unsorted (mode 1) or sorted (2) order.  pairs:
+// neighbors of all points within these radii, as far as known.
 static Tensor density(const GridPtr& grid, const Tensor& inv_radii, const Tensor& inv_bandwidth,
-                      int pdf_mode, int mode) {
+                      int pdf_mode, int mode, double pairs) {
   Tensor r = f32(inv_radii), bw = f32(inv_bandwidth);
   Tensor out = empty({grid->g.n}, at::kFloat, grid->points);
-  check(tfgpc_cells_density(stream(), &grid->g, fp(r), fp(bw), pdf_mode, grid->g.n, nullptr,
-                            nullptr, mode, fpm(out)));
+  const size_t need = tfgpc_cells_density_workspace_bytes(grid->g.D, grid->g.n, (int64_t)pairs);
+  Tensor ws;
+  if (need) ws = bytes(need, grid->points);
+  check(tfgpc_cells_density_ws(stream(), &grid->g, fp(r), fp(bw), pdf_mode, grid->g.n, nullptr,
+                               nullptr, mode, need ? ws.data_ptr() : nullptr, need, fpm(out)));
   return out;
 }
 
@@ -324,7 +328,8 @@ void bind_cells(py::module_& m) {
   m.def("build_grid", &build_grid);
   m.def("count_neighbors", &count_neighbors);
   m.def("fill_neighbors", &fill_neighbors);
-  m.def("density", &density);
+  m.def("density", &density, py::arg("grid"), py::arg("inv_radii"), py::arg("inv_bandwidth"),
+        py::arg("pdf_mode"), py::arg("mode"), py::arg("pairs") = 0.0);
   m.def("sample", &sample);
   m.def("build_and_sample", &build_and_sample);
 }

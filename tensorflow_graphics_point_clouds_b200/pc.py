@@ -375,6 +375,13 @@ class Neighborhood:
       self._orig_ids, _ = ops.original_neighbor_ids(self._nbrs, self._grid._sorted_indices)
     return self._orig_ids
 
+  def _pairs_of_all_points(self):
+    """About how many neighbors the grid's points have in all, 0 if nothing is counted yet."""
+    count = self._counted
+    if count is None or count.ranges.shape[0] == 0:
+      return 0.0
+    return float(count.total) * self._grid._point_cloud._points.shape[0] / count.ranges.shape[0]
+
   def _samples_are_grid_points(self):
     return self._equal_samples or (self._sample_mode == 1 and self.max_neighbors == 0)
 
@@ -391,10 +398,11 @@ class Neighborhood:
     if g._cells is not None and not (self._equal_samples and self.max_neighbors > 0):
       # straight from the grid, without the list of a self neighborhood; by original
       # index, which the layers read the densities by, unless the samples are sorted
+      pairs = self._pairs_of_all_points()
       if self._equal_samples:
-        self._point_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 2)
+        self._point_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 2, pairs)
       else:
-        self._sample_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 1)
+        self._sample_pdf = ops._lib.host().density(g._cells, inv_r, inv_bw, mode, 1, pairs)
     elif self._equal_samples:
       self._point_pdf = ops.compute_pdf_with_pt_grads(
           g._sorted_points, self._neighbors, self._samples_neigh_ranges, inv_bw, inv_r, mode)
