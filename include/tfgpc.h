@@ -294,6 +294,18 @@ int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid,
                      int max_neighs, const int32_t* ranges, int64_t total,
                      int32_t* neigh_out, int32_t* ids_out);
 
+/* tfgpc_cells_count with the densities of tfgpc_cell_grid_neighborhood_pdf (workspace of its
+ * own size, 16-byte aligned): for a grid that is there already. */
+size_t tfgpc_cells_count_pdf_workspace_bytes(int64_t ns);
+int tfgpc_cells_count_pdf(void* stream, const tfgpc_cell_grid* grid,
+                          const float* inv_radii, int64_t ns,
+                          const float* samples,
+                          const int32_t* samples_batch_ids,
+                          int samples_are_points, int max_neighs,
+                          int32_t* ranges_out, const float* inv_bandwidth,
+                          int pdf_mode, float* pdf_out, float* packed_out,
+                          void* ws, size_t ws_bytes, int64_t* total_out);
+
 /* ComputePdf at the samples over the grid's points within the radius, without a
  * neighbor list: what tfgpc_compute_pdf_at_samples gives for the list of a
  * neighborhood without limit. */
@@ -338,6 +350,28 @@ int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
                            size_t ws_bytes, void* sample_ws,
                            size_t sample_ws_bytes, int32_t* num_cells_host_out,
                            int64_t* num_samples_out);
+
+/* tfgpc_cell_grid_sample of several levels, each on the samples of the one before, with one
+ * blocking read: tfgpc_cell_grid_sample_level enqueues level 0, 1, .. and does not block,
+ * tfgpc_cell_grid_sample_report waits for all of them (same host thread).  A level leaves the number
+ * of its samples in *num_samples_dev_out; the next one takes that pointer as n_dev (NULL: it has
+ * grid->n points) and holds grid->n points at most, few enough for one cluster (65 536, a table of
+ * 2^21 cells, batch_size * D <= 1024).  Workspaces may be shared by the levels of a stream.
+ * num_cells_host_out [levels,D], num_samples_out [levels]; *levels_done_out: levels that were
+ * built (none from a level on that got more than its grid->n points or asked for more than its
+ * max_cells; the first: TFGPC_ENOMEM). */
+#define TFGPC_MAX_CHAINED_LEVELS 16
+int tfgpc_cell_grid_sample_level(
+    void* stream, int level, const tfgpc_cell_grid* grid, const float* points,
+    const int32_t* batch_ids, const int64_t* n_dev, const float* cell_sizes,
+    int mode, const float* inv_radii, float* sample_pts_out,
+    int32_t* sample_batch_ids_out, int32_t* sample_indices_out,
+    int64_t* num_samples_dev_out, void* ws, size_t ws_bytes, void* sample_ws,
+    size_t sample_ws_bytes);
+int tfgpc_cell_grid_sample_report(void* stream, int levels, int D, int max_cells,
+                                  int32_t* num_cells_host_out,
+                                  int64_t* num_samples_out,
+                                  int* levels_done_out);
 
 /* ---- FindNeighbors fill pass with original ids and densities --------------
  * tfgpc_find_neighbors_fill_ordered (sample_order may be NULL) that, in the same

@@ -49,6 +49,8 @@ SYMBOLS = {
     "tfgpc_cell_grid_neighborhood": c_int,
     "tfgpc_cell_grid_neighborhood_pdf": c_int,
     "tfgpc_cells_count": c_int,
+    "tfgpc_cells_count_pdf_workspace_bytes": c_sz,
+    "tfgpc_cells_count_pdf": c_int,
     "tfgpc_cells_fill": c_int,
     "tfgpc_cells_density": c_int,
     "tfgpc_cells_density_workspace_bytes": c_sz,
@@ -56,6 +58,8 @@ SYMBOLS = {
     "tfgpc_cells_sample_workspace_bytes": c_sz,
     "tfgpc_cells_sample": c_int,
     "tfgpc_cell_grid_sample": c_int,
+    "tfgpc_cell_grid_sample_level": c_int,
+    "tfgpc_cell_grid_sample_report": c_int,
     "tfgpc_pack_points_density": c_int,
     "tfgpc_find_neighbors_fill_fused": c_int,
     "tfgpc_original_neighbor_ids": c_int,

@@ -55,7 +55,10 @@ class SmallClassifier:
     status = mcconv.product_status(x.device)
     last = len(self.convs) - 1
     for i, conv in enumerate(self.convs):
-      x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], keep_for_backward=False)
+      # (the hierarchy's grid of this cloud has the layer's cells)
+      grid = mcconv.layer_on_grid(conv, hier._neighborhoods[i]._grid)
+      x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], neighborhood=grid,
+                       keep_for_backward=False)
       if i < last:
         x = self._bn_act(x)
         x = mcconv.conv1x1(x, *self.conv1x1[i], status=status)

@@ -347,11 +347,14 @@ __device__ __forceinline__ int rank_in_tile(RankScratch<THREADS>& s, const int32
   return rank;
 }
 
+// Points up to which the cluster writes the sorted copies itself (see ClusterBuild).
+constexpr int64_t kClusterPlacePoints = 8192;
+
 // One thread per slot of `members`: the rank of its point inside the bucket, and the
 // point's row of every sorted array; then the tube ranges, read off the table.
 template <int D, int THREADS>
 __global__ void __launch_bounds__(THREADS)
-place_kernel(int64_t n, const int32_t* members, const int64_t* keys,
+place_kernel(int64_t n, const int64_t* n_dev, const int32_t* members, const int64_t* keys,
              const int32_t* num_cells, int batch_size,
              const int32_t* start, const float* pts,
              const int32_t* batch_ids, int32_t* __restrict__ perm,
@@ -359,6 +362,11 @@ place_kernel(int64_t n, const int32_t* members, const int64_t* keys,
              float4* __restrict__ packed, int2* __restrict__ ds,
              const int32_t* crowded) {
   chain_enter();
+  if (n_dev) {
+    const int64_t most = n;
+    n = ld_global(n_dev);
+    if (n <= kClusterPlacePoints || n > most) return;     // (placed by the cluster, or no grid)
+  }
   int nc[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = ld_global(num_cells + d);
@@ -428,10 +436,10 @@ constexpr int kMaxRanks = 16;
 constexpr int kHeld = 4;                   // points of a thread at most
 constexpr int64_t kClusterPoints = 65536;
 constexpr int64_t kClusterCells = int64_t(1) << 21;
-constexpr int64_t kClusterPlacePoints = 8192;
 
 struct ClusterBuild {
-  int64_t n;
+  int64_t n;                   // points, or (n_dev) at most so many
+  const int64_t* n_dev;        // their number where the host does not know it; 0, or more: no grid
   const float* pts;
   const int32_t* batch_ids;
   int batch_size, max_cells;
@@ -501,7 +509,8 @@ grid_cluster_kernel(ClusterBuild a) {
   cg::cluster_group cluster = cg::this_cluster();
   const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
-  const int n = (int)a.n, boxes = a.batch_size * D;
+  const int64_t points = a.n_dev ? ld_global(a.n_dev) : a.n;
+  const int n = points <= a.n ? (int)points : 0, boxes = a.batch_size * D;
   const int stride = ranks * kClusterThreads, first = rank * kClusterThreads + tid;
   // A warp's points follow one another, as they mostly lie in one cloud.
   const int steps = (n + stride - 1) / stride;
@@ -627,7 +636,9 @@ grid_cluster_kernel(ClusterBuild a) {
     }
   }
   __syncthreads();
-  bool over = false;
+  bool over = n == 0;          // (what it would be a grid of has failed, or does not fit)
+  if (over && tid < D) asked[tid] = a.max_cells + 1;
+  __syncthreads();
   Grid<D> g;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -731,7 +742,7 @@ grid_cluster_kernel(ClusterBuild a) {
     if (k < here) __stcg(a.members + number[k], mine + 32 * k);
   cluster.sync();   // (also: no block leaves while others read its shared memory)
   if (rank == 0 && tid == 0) clip_and_report(D, a.max_cells, asked, a.g.num_cells, a.page);
-  if (!a.place) return;
+  if (a.n_dev ? n > kClusterPlacePoints : !a.place) return;
   const bool any = __ldcg(a.crowded) != 0;
   for (int tile0 = rank * kClusterThreads; tile0 < n; tile0 += stride) {
     const int i = tile0 + tid;
@@ -829,21 +840,40 @@ constexpr int64_t kLargeTilePoints = 131072;
 
 template <int THREADS>
 int launch_place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
-                  const int32_t* batch_ids, const CellGridWs& w) {
+                  const int32_t* batch_ids, const CellGridWs& w, const int64_t* n_dev) {
   TFGPC_DIM_SWITCH(g.D, TFGPC_CUDA(launch_chained(st, blocks_for(g.n, THREADS), THREADS, 0,
-      place_kernel<kD, THREADS>, g.n, w.members, g.keys, g.num_cells, (int)g.batch_size,
+      place_kernel<kD, THREADS>, g.n, n_dev, w.members, g.keys, g.num_cells, (int)g.batch_size,
       g.cell_start, points, batch_ids, g.sorted_indices, g.sorted_keys, g.sorted_points,
       g.sorted_batch_ids, (float4*)g.packed, (int2*)g.ds, w.crowded)));
   return TFGPC_OK;
 }
 
 int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const int32_t* batch_ids,
-          const CellGridWs& w) {
-  return g.n >= kLargeTilePoints ? launch_place<512>(st, g, points, batch_ids, w)
-                                 : launch_place<256>(st, g, points, batch_ids, w);
+          const CellGridWs& w, const int64_t* n_dev = nullptr) {
+  return g.n >= kLargeTilePoints ? launch_place<512>(st, g, points, batch_ids, w, n_dev)
+                                 : launch_place<256>(st, g, points, batch_ids, w, n_dev);
+}
+
+// Blocks of the cluster that a grid can be built by, 0: it is too large for one.
+int cluster_for(const tfgpc_cell_grid& g, int* ranks) {
+  *ranks = 0;
+  if (g.n > kClusterPoints || table_cells(g.D, g.batch_size, g.max_cells) > kClusterCells ||
+      g.batch_size * g.D > kClusterBoxes)
+    return TFGPC_OK;
+  int rc = TFGPC_OK;
+  TFGPC_DIM_SWITCH(g.D, rc = cluster_ranks<kD>(ranks));
+  if (!rc && g.n > (int64_t)*ranks * kClusterThreads * kHeld) *ranks = 0;
+  return rc;
 }
 
 }  // namespace
+
+int cell_grid_takes_cluster(const tfgpc_cell_grid& g, bool* takes) {
+  int ranks = 0;
+  const int rc = cluster_for(g, &ranks);
+  *takes = ranks > 0;
+  return rc;
+}
 
 CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch_size,
                            int max_cells) {
@@ -866,7 +896,7 @@ CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch
 int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                     const int32_t* batch_ids, const float* cell_sizes,
                     const int32_t* num_cells_in, const CellGridWs& w, int32_t* page,
-                    AlsoClear also) {
+                    AlsoClear also, const int64_t* n_dev) {
   const int64_t n = g.n;
   const int D = g.D, B = (int)g.batch_size;
   const int64_t cells = table_cells(D, B, g.max_cells);
@@ -874,20 +904,19 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   for (int d = 0; d < D; ++d) cs.v[d] = cell_sizes[d];
   const unsigned blocks = blocks_for(n, kThreads);
   int ranks = 0;
-  if (!num_cells_in && n <= kClusterPoints && cells <= kClusterCells &&
-      (int64_t)B * D <= kClusterBoxes) {
-    int rc = TFGPC_OK;
-    TFGPC_DIM_SWITCH(D, rc = cluster_ranks<kD>(&ranks));
+  if (!num_cells_in) {
+    int rc = cluster_for(g, &ranks);
     if (rc) return rc;
   }
-  if (ranks > 0 && n <= (int64_t)ranks * kClusterThreads * kHeld) {
+  TFGPC_REQUIRE(!n_dev || ranks > 0, "a grid of points not counted yet is too large for a cluster");
+  if (ranks > 0) {
     ProfScope prof(st, "grid_cluster");
-    const ClusterBuild a{n, points, batch_ids, B, g.max_cells, cs, g, w.members, w.crowded,
+    const ClusterBuild a{n, n_dev, points, batch_ids, B, g.max_cells, cs, g, w.members, w.crowded,
                          page, n <= kClusterPlacePoints, also};
     int rc = TFGPC_OK;
     TFGPC_DIM_SWITCH(D, rc = launch_cluster<kD>(st, a, ranks));
     if (rc) return rc;
-    return a.place ? TFGPC_OK : place(st, g, points, batch_ids, w);
+    return a.place ? TFGPC_OK : place(st, g, points, batch_ids, w, n_dev);
   }
   if (num_cells_in) {
     ProfScope prof(st, "grid_params");

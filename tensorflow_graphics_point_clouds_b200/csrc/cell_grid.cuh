@@ -29,11 +29,14 @@ CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch
 // Words that a build clears along the way, for what follows it.
 struct AlsoClear { uint32_t* p = nullptr; int64_t words = 0; };
 
-// Enqueues the build; the cell counts go to words 0 .. kReportTotal of `page`.
+// Enqueues the build; the cell counts go to words 0 .. kReportTotal of `page`.  n_dev: the number
+// of points where an earlier kernel of the stream works it out (0, or more than g.n: no grid, as if
+// it had too many cells); only where cell_grid_takes_cluster.
+int cell_grid_takes_cluster(const tfgpc_cell_grid& g, bool* takes);
 int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                     const int32_t* batch_ids, const float* cell_sizes,
                     const int32_t* num_cells_in, const CellGridWs& w, int32_t* page,
-                    AlsoClear also = AlsoClear());
+                    AlsoClear also = AlsoClear(), const int64_t* n_dev = nullptr);
 
 // Argument check of every entry on a built grid (cell_search.cu).
 int check_cell_grid(const char* op, const tfgpc_cell_grid* g);

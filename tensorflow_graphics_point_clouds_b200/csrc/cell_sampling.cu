@@ -43,6 +43,11 @@ constexpr int kProgressMarks = 65536;
 constexpr int kLongCell = 64;
 inline unsigned long long barrier_period_ns(int64_t n) { return 500000000ull + 100ull * n; }
 
+// A warp per 8 points (16: 158 against 140 us in the three-level classifier).
+__host__ __device__ __forceinline__ int64_t blocks_wanted(int64_t n) {
+  return (n + 8 * kWarps - 1) / (8 * kWarps);
+}
+
 struct SampleArgs {
   CellsView c;
   const int64_t* keys;         // sorted
@@ -56,6 +61,8 @@ struct SampleArgs {
   int32_t* batch_out;
   int32_t* index_out;          // original indices (Poisson)
   int32_t* page;               // number of samples (64 bits), then the error word
+  const int64_t* n_dev;        // number of points (c.n: at most), or null
+  int64_t* samples_dev;        // number of samples, 0 if anything failed, or null
   unsigned long long period_ns;
 };
 
@@ -264,12 +271,11 @@ __device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cel
 struct Team { int cloud, begin, size; };
 
 // One block per cloud and the others in proportion to the clouds' points.
-__device__ __forceinline__ Team team_of(const CellsView& c, int total) {
+__device__ __forceinline__ Team team_of(const CellsView& c, int64_t n, int blocks, int total) {
   const int lane = lane_id();
-  if (c.batch_size > kMaxTeams || c.batch_size * 2 > (int)gridDim.x)
-    return Team{-1, 0, (int)gridDim.x};
+  if (c.batch_size > kMaxTeams || c.batch_size * 2 > blocks) return Team{-1, 0, blocks};
   const int cells = total / c.batch_size;
-  const long long spare = (int)gridDim.x - c.batch_size;
+  const long long spare = blocks - c.batch_size;
   int before = 0;
   for (int b0 = 0; b0 < c.batch_size; b0 += 32) {
     const int b = b0 + lane;
@@ -277,7 +283,7 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int total) {
     if (b < c.batch_size) {
       const int points = __ldg(c.start + (total - b * cells) + 1) -
                          __ldg(c.start + (total - (b + 1) * cells) + 1);
-      share = 1 + (int)(spare * points / c.n);
+      share = 1 + (int)(spare * points / n);
     }
     int upto = share;
 #pragma unroll
@@ -308,8 +314,13 @@ cells_sample_kernel(SampleArgs a) {
 #pragma unroll
   for (int d = 0; d < D; ++d) nc[d] = __ldg(a.c.num_cells + d);
   const int total = total_cells<D>(nc, a.c.batch_size);
-  if (total == 0) return;        // (a grid that got no cells: the call fails)
-  const int64_t n = a.c.n;
+  if (total == 0) {              // (a grid that got no cells: the call fails)
+    if (a.samples_dev && blockIdx.x == 0 && threadIdx.x == 0) *a.samples_dev = 0;
+    return;
+  }
+  const int64_t n = a.n_dev ? __ldg(a.n_dev) : a.c.n;
+  const int blocks = a.n_dev ? (int)min((int64_t)gridDim.x, blocks_wanted(n)) : (int)gridDim.x;
+  if ((int)blockIdx.x >= blocks) return;      // (nobody waits for them)
   unsigned barriers = 0;
   bool ok = true;
   if (a.mode == 0) {
@@ -319,11 +330,11 @@ cells_sample_kernel(SampleArgs a) {
     // points outside every cell have no neighbors: all of them are taken
     const int lead = __ldg(a.c.start + 1), tail = __ldg(a.c.start + total + 1);
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < lead + (n - tail);
-         i += (int64_t)gridDim.x * kThreads)
+         i += (int64_t)blocks * kThreads)
       a.state[i < lead ? i : tail + (i - lead)] = 2;
     if (threadIdx.x == 0) num_crowded[0] = 0;
     __syncthreads();
-    const Team team = team_of(a.c, total);
+    const Team team = team_of(a.c, n, blocks, total);
     const int warps = team.size * kWarps;
     // neighboring cells go to different blocks: crowded ones come side by side
     const int warp = w * team.size + (int)blockIdx.x - team.begin;
@@ -391,11 +402,11 @@ cells_sample_kernel(SampleArgs a) {
                         a.period_ns) && ok;
     }
     if (team.cloud < 0) barriers = (1 << D) - 1;
-    ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, a.arrived + 2,
+    ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
                       a.period_ns) && ok;
   }
   // ---- compaction: every block counts, then writes, its stretch of the points
-  const int64_t per = (n + gridDim.x - 1) / gridDim.x;
+  const int64_t per = (n + blocks - 1) / blocks;
   const int64_t first = min((int64_t)blockIdx.x * per, n), last = min(first + per, n);
   auto chosen = [&](int64_t i) {
     if (i >= last) return false;
@@ -413,12 +424,12 @@ cells_sample_kernel(SampleArgs a) {
     for (int i = 0; i < kWarps; ++i) t += warp_total[i];
     __stcg(a.block_total + blockIdx.x, t);
   }
-  ok = grid_barrier(a.arrived, ++barriers * gridDim.x, a.arrived + 1, a.arrived + 2,
+  ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
                     a.period_ns) && ok;
   ok = ok && !any_gave_up(a.arrived + 1);
   if (w == 0) {
     int64_t t = 0, all = 0;
-    for (int i = lane; i < gridDim.x; i += 32) {
+    for (int i = lane; i < blocks; i += 32) {
       const int v = __ldcg(a.block_total + i);
       all += v;
       if (i < (int)blockIdx.x) t += v;
@@ -434,6 +445,7 @@ cells_sample_kernel(SampleArgs a) {
         a.page[0] = (int32_t)(uint32_t)all;
         a.page[1] = (int32_t)(all >> 32);
         a.page[2] = ok ? 0 : 1;
+        if (a.samples_dev) *a.samples_dev = ok ? all : 0;
       }
     }
   }
@@ -533,8 +545,8 @@ int launch_sample(cudaStream_t st, SampleArgs a) {
     TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
     per_sm = v < 1 ? 1 : v;
   }
-  // a warp per 8 points (16: 158 against 140 us in the three-level classifier), at most 4 blocks per SM and what is resident at once
-  int64_t blocks = (a.c.n + 8 * kWarps - 1) / (8 * kWarps);
+  // at most 4 blocks per SM and what is resident at once
+  int64_t blocks = blocks_wanted(a.c.n);
   const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
   if (blocks > most) blocks = most;
   if (blocks > kMaxBlocks) blocks = kMaxBlocks;
@@ -582,7 +594,7 @@ size_t clear_bytes(int64_t n, int mode) {
 // Enqueues the sampling; the number of samples goes to words kReportTotal .. of the page.
 int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const float* inv_radii,
                  float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page,
-                 bool cleared) {
+                 bool cleared, const int64_t* n_dev = nullptr, int64_t* samples_dev = nullptr) {
   const size_t state = align_up((size_t)g.n + kHeadBytes, 256);
   SampleArgs a;
   a.c = view_of(g);
@@ -596,6 +608,8 @@ int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const floa
   a.batch_out = batch_out;
   a.index_out = index_out;
   a.page = page + kReportTotal;
+  a.n_dev = n_dev;
+  a.samples_dev = samples_dev;
   a.period_ns = barrier_period_ns(g.n);
   ProfScope prof(st, mode == 0 ? "sampling_poisson" : "sampling_cell_average");
   if (!cleared) TFGPC_CUDA(cudaMemsetAsync(ws, 0, clear_bytes(g.n, mode), st));
@@ -620,11 +634,9 @@ int check_sample(const tfgpc_cell_grid* g, int mode, const float* inv_radii, con
   return TFGPC_OK;
 }
 
-int finish_sample(cudaStream_t st, const tfgpc_cell_grid& g, int32_t* num_cells_host_out,
-                  int64_t* num_samples_out) {
-  int32_t host[kReportWords + 1];
-  int rc = read_report(st, sizeof(host), host);
-  if (rc) return rc;
+// The outputs of a blocking entry from the words that a level has left in the report page.
+int level_report(const int32_t* host, const tfgpc_cell_grid& g, int32_t* num_cells_host_out,
+                 int64_t* num_samples_out) {
   for (int d = 0; num_cells_host_out && d < g.D; ++d) num_cells_host_out[d] = host[d];
   if (num_cells_host_out && host[TFGPC_MAX_DIMS])
     return fail(TFGPC_ENOMEM, "SamplingOp: the grid needs more than max_cells = %d cells in a "
@@ -635,6 +647,17 @@ int finish_sample(cudaStream_t st, const tfgpc_cell_grid& g, int32_t* num_cells_
                      ((int64_t)host[kReportTotal + 1] << 32);
   return TFGPC_OK;
 }
+
+int finish_sample(cudaStream_t st, const tfgpc_cell_grid& g, int32_t* num_cells_host_out,
+                  int64_t* num_samples_out) {
+  int32_t host[kReportWords + 1];
+  int rc = read_report(st, sizeof(host), host);
+  return rc ? rc : level_report(host, g, num_cells_host_out, num_samples_out);
+}
+
+constexpr int kMaxLevels = TFGPC_MAX_CHAINED_LEVELS;
+constexpr int kLevelWords = 16;          // of the report page, one level
+static_assert(kReportWords + 1 <= kLevelWords && kMaxLevels * kLevelWords * 4 <= 4096, "page");
 
 }  // namespace
 }  // namespace tfgpc
@@ -696,6 +719,70 @@ extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
                     sample_indices_out, sample_ws, (int32_t*)page, true);
   if (rc) return rc;
   return finish_sample(st, g, num_cells_host_out, num_samples_out);
+}
+
+// With a blocking read per level the GPU waited 31 to 44 us between two levels of 10 to 80: for
+// the host to see the number of points, to make the next level's arrays and for its first launch
+// to arrive.
+extern "C" int tfgpc_cell_grid_sample_level(
+    void* stream, int level, const tfgpc_cell_grid* grid, const float* points,
+    const int32_t* batch_ids, const int64_t* n_dev, const float* cell_sizes, int mode,
+    const float* inv_radii, float* sample_pts_out, int32_t* sample_batch_ids_out,
+    int32_t* sample_indices_out, int64_t* num_samples_dev_out, void* ws, size_t ws_bytes,
+    void* sample_ws, size_t sample_ws_bytes_given) {
+  TFGPC_REQUIRE(level >= 0 && level < kMaxLevels, "SamplingOp expects a level below %d", kMaxLevels);
+  int64_t unused = 0;
+  int rc = check_sample(grid, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                        sample_indices_out, sample_ws, sample_ws_bytes_given, &unused);
+  if (rc) return rc;
+  const tfgpc_cell_grid& g = *grid;
+  TFGPC_REQUIRE(points && batch_ids && cell_sizes && ws && num_samples_dev_out,
+                "SamplingOp got a null pointer");
+  TFGPC_REQUIRE(n_dev != num_samples_dev_out, "SamplingOp expects two counts, not one");
+  for (int d = 0; d < g.D; ++d)
+    TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "SamplingOp expects positive cell sizes");
+  if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, 0, g.batch_size, g.max_cells))
+    return fail(TFGPC_ENOMEM, "SamplingOp workspace too small");
+  if (n_dev) {
+    bool takes = false;
+    rc = cell_grid_takes_cluster(g, &takes);
+    if (rc) return rc;
+    TFGPC_REQUIRE(takes, "SamplingOp: too large a level for points not counted yet");
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  int32_t* words = (int32_t*)page + level * kLevelWords;
+  const CellGridWs w = carve_cell_grid(ws, g.n, 0, g.D, g.batch_size, g.max_cells);
+  const AlsoClear also{(uint32_t*)sample_ws, (int64_t)(clear_bytes(g.n, mode) / 4)};
+  rc = cell_grid_build(st, g, points, batch_ids, cell_sizes, nullptr, w, words, also, n_dev);
+  if (rc) return rc;
+  return sample_async(st, g, mode, inv_radii, sample_pts_out, sample_batch_ids_out,
+                      sample_indices_out, sample_ws, words, true, n_dev, num_samples_dev_out);
+}
+
+extern "C" int tfgpc_cell_grid_sample_report(void* stream, int levels, int D, int max_cells,
+                                             int32_t* num_cells_host_out, int64_t* num_samples_out,
+                                             int* levels_done_out) {
+  TFGPC_REQUIRE(levels >= 1 && levels <= kMaxLevels && valid_dims(D),
+                "SamplingOp expects 1 to %d levels and a valid dimension", kMaxLevels);
+  TFGPC_REQUIRE(num_cells_host_out && num_samples_out && levels_done_out,
+                "SamplingOp got a null pointer");
+  int32_t host[kMaxLevels * kLevelWords];
+  int rc = read_report((cudaStream_t)stream, (size_t)levels * kLevelWords * 4, host);
+  if (rc) return rc;
+  tfgpc_cell_grid g{};
+  g.D = D;
+  g.max_cells = max_cells;
+  *levels_done_out = 0;
+  for (int l = 0; l < levels; ++l) {
+    rc = level_report(host + l * kLevelWords, g, num_cells_host_out + l * D, num_samples_out + l);
+    if (rc == TFGPC_ENOMEM && l > 0) break;       // (the levels before it stand)
+    if (rc) return rc;
+    *levels_done_out = l + 1;
+  }
+  return TFGPC_OK;
 }
 
 extern "C" int tfgpc_debug_sampling_barrier(void* stream, void* ws, size_t ws_bytes,

@@ -805,6 +805,51 @@ extern "C" int tfgpc_cells_count(void* stream, const tfgpc_cell_grid* grid, cons
   return finish_report(st, grid->D, grid->max_cells, true, nullptr, total_out);
 }
 
+extern "C" size_t tfgpc_cells_count_pdf_workspace_bytes(int64_t ns) {
+  return ns < 0 ? 0 : align_up(tfgpc_find_neighbors_workspace_bytes(ns), 256) + (size_t)ns * 4;
+}
+
+extern "C" int tfgpc_cells_count_pdf(void* stream, const tfgpc_cell_grid* grid,
+                                     const float* inv_radii, int64_t ns, const float* samples,
+                                     const int32_t* samples_batch_ids, int samples_are_points,
+                                     int max_neighs, int32_t* ranges_out,
+                                     const float* inv_bandwidth, int pdf_mode, float* pdf_out,
+                                     float* packed_out, void* ws, size_t ws_bytes,
+                                     int64_t* total_out) {
+  int rc = check_cell_grid("FindNeighbors", grid);
+  if (rc) return rc;
+  rc = check_samples("FindNeighbors", grid, ns, samples, samples_batch_ids, samples_are_points,
+                     max_neighs);
+  if (rc) return rc;
+  TFGPC_REQUIRE(total_out && inv_radii && pdf_out && ws && (uintptr_t)ws % 16 == 0 &&
+                (ns == 0 || ranges_out), "FindNeighbors got a null pointer");
+  TFGPC_REQUIRE((pdf_mode == 0 || pdf_mode == 1) && (pdf_mode == 1 || inv_bandwidth) &&
+                (!packed_out || (grid->D == 3 && (uintptr_t)packed_out % 16 == 0)),
+                "FindNeighbors: densities need mode 0 or 1, a bandwidth and an output (packed: "
+                "16-byte aligned, three dimensions)");
+  if (ws_bytes < tfgpc_cells_count_pdf_workspace_bytes(ns))
+    return fail(TFGPC_ENOMEM, "FindNeighbors workspace too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  void* page = nullptr;
+  rc = report_page(&page);
+  if (rc) return rc;
+  *total_out = 0;
+  if (ns > 0) {
+    int64_t* sums = (int64_t*)ws;
+    rc = count_and_scan(st, *grid, inv_radii, ns,
+                        SampleSource{samples_are_points, samples, samples_batch_ids}, max_neighs,
+                        ranges_out, sums, sums + scan_block_sums_elems(ns), (int32_t*)page,
+                        (int32_t*)((char*)ws + align_up(tfgpc_find_neighbors_workspace_bytes(ns), 256)));
+    if (rc) return rc;
+  }
+  rc = mark_report(st);
+  if (!rc)
+    rc = enqueue_density(st, *grid, SampleSource{1, nullptr, nullptr}, grid->n, inv_radii,
+                         DensityRequest{inv_bandwidth, pdf_mode, pdf_out, (float4*)packed_out}, nullptr);
+  if (rc) return rc;
+  return finish_report(st, grid->D, grid->max_cells, ns > 0, nullptr, total_out, true);
+}
+
 extern "C" int tfgpc_cells_fill(void* stream, const tfgpc_cell_grid* grid, const float* inv_radii,
                                 int64_t ns, const float* samples,
                                 const int32_t* samples_batch_ids, int samples_are_points,

@@ -1,4 +1,6 @@
 // Grids with a cell table, neighborhoods, densities and sampling.
+#include <algorithm>
+
 #include "host.h"
 
 namespace tfgpc_host {
@@ -33,8 +35,31 @@ class CellGrid {
     batch_ids = i32(bids);
     on_gpu(points);
     on_gpu(batch_ids);
-    const int64_t n = points.size(0), d = points.size(1), b = batch_size;
-    require(batch_ids.size(0) == n, "ComputeKeysOp expects the same number of points as batch ids");
+    require(batch_ids.size(0) == points.size(0),
+            "ComputeKeysOp expects the same number of points as batch ids");
+    allocate(points.size(0), points.size(1), batch_size, max_cells, points);
+    if (!cells.is_none()) {
+      void** slot = (void**)&g.aabb_min;
+      for (int i : {0, 1, 3, 4}) {
+        given.push_back(f32(cells[py::str(kFields[i].name)].cast<Tensor>()));
+        slot[i] = given.back().data_ptr();
+      }
+      given.push_back(i32(cells[py::str("num_cells")].cast<Tensor>()));
+    }
+  }
+
+  // A grid of at most n points that come later (set_points).
+  CellGrid(int64_t n, int64_t d, int64_t batch_size, int max_cells, const Tensor& like) {
+    allocate(n, d, batch_size, max_cells, like);
+  }
+
+  void set_points(const Tensor& pts, const Tensor& bids) {
+    points = pts;
+    batch_ids = bids;
+    g.n = pts.size(0);
+  }
+
+  void allocate(int64_t n, int64_t d, int64_t b, int max_cells, const Tensor& like) {
     g.D = (int)d;
     g.max_cells = max_cells;
     g.n = n;
@@ -48,17 +73,10 @@ class CellGrid {
       offset[i] = total;
       total += align256((size_t)elems[i] * (kFields[i].type == at::kLong ? 8 : 4));
     }
-    arena = bytes(total, points);
+    arena = bytes(total, like);
     char* base = (char*)arena.data_ptr();
     void** slot = (void**)&g.aabb_min;
     for (int i = 0; i < kNumFields; ++i) slot[i] = elems[i] > 0 ? base + offset[i] : nullptr;
-    if (!cells.is_none()) {
-      for (int i : {0, 1, 3, 4}) {
-        given.push_back(f32(cells[py::str(kFields[i].name)].cast<Tensor>()));
-        slot[i] = given.back().data_ptr();
-      }
-      given.push_back(i32(cells[py::str("num_cells")].cast<Tensor>()));
-    }
   }
 
   const int32_t* cells_in() const { return given.empty() ? nullptr : ip(given.back()); }
@@ -220,6 +238,35 @@ static CountPtr count_neighbors(const GridPtr& grid, const Tensor& inv_radii, in
   return c;
 }
 
+// (count, density at the points in their own order, table of tfgpc_pack_points_density or None)
+static py::tuple count_neighbors_with_pdf(const GridPtr& grid, const Tensor& inv_radii, int mode,
+                                          const OptTensor& samples, const OptTensor& sample_ids,
+                                          int max_neighs, const Tensor& inv_bandwidth,
+                                          int pdf_mode) {
+  CountPtr c = std::make_shared<Count>();
+  c->grid = grid;
+  c->samples = make_samples(*grid, mode, samples, sample_ids);
+  c->inv_radii = f32(inv_radii);
+  c->max_neighs = max_neighs;
+  const int64_t ns = c->samples.ns;
+  c->ranges = empty({ns}, at::kInt, grid->points);
+  Tensor inv_bw = f32(inv_bandwidth), pdf = empty({grid->g.n}, at::kFloat, grid->points);
+  OptTensor packed;
+  if (grid->g.D == 3) packed = empty({grid->g.n, 4}, at::kFloat, grid->points);
+  const size_t need = tfgpc_cells_count_pdf_workspace_bytes(ns);
+  Tensor ws = bytes(need, grid->points);
+  void* st = stream();
+  int rc;
+  {
+    py::gil_scoped_release release;
+    rc = tfgpc_cells_count_pdf(st, &grid->g, fp(c->inv_radii), ns, c->samples.p(), c->samples.b(),
+                               mode, max_neighs, ipm(c->ranges), fp(inv_bw), pdf_mode, fpm(pdf),
+                               packed ? fpm(*packed) : nullptr, ws.data_ptr(), need, &c->total);
+  }
+  check(rc);
+  return py::make_tuple(c, pdf, packed);
+}
+
 // (pairs with sorted indices, pairs with original indices or None)
 static py::tuple fill_neighbors(const CountPtr& c, bool with_ids) {
   const int64_t m = c->total;
@@ -310,6 +357,103 @@ static py::tuple build_and_sample(const Tensor& points, const Tensor& batch_ids,
   return py::make_tuple(grid, cut[0], cut[1], cut[2]);
 }
 
+// The levels of a hierarchy one after the other: a level is under way from its add on, so that the
+// host makes the next one's arrays meanwhile; finish blocks.
+class SampleLevels {
+ public:
+  SampleLevels(const Tensor& points, const Tensor& batch_ids, int64_t batch_size,
+               const std::vector<double>& cell_sizes, int max_cells, int mode,
+               const Tensor& inv_radii)
+      : mode_(mode), stream_(stream()) {
+    Level level;
+    level.grid = std::make_shared<CellGrid>(points, batch_ids, batch_size, max_cells, py::none());
+    require(level.grid->g.n > 0, "SamplingOp expects points");
+    like_ = level.grid->points;
+    counts_ = bytes(TFGPC_MAX_CHAINED_LEVELS * 8, like_);
+    enqueue(std::move(level), cell_sizes, inv_radii);
+  }
+
+  // A level of at most `room` points.
+  void add(const std::vector<double>& cell_sizes, int max_cells, const Tensor& inv_radii,
+           int64_t room) {
+    require(levels_.size() < TFGPC_MAX_CHAINED_LEVELS, "SamplingOp: too many levels");
+    const tfgpc_cell_grid& first = levels_[0].grid->g;
+    Level level;
+    level.grid = std::make_shared<CellGrid>(std::min(room, first.n), first.D, first.batch_size,
+                                            max_cells, like_);
+    enqueue(std::move(level), cell_sizes, inv_radii);
+  }
+
+  GridPtr grid(int level) const { return levels_.at(level).grid; }
+
+  // [(points, batch ids, original indices or None, cells per dimension at most)] of the levels
+  // that could be built
+  py::list finish() {
+    const int n = (int)levels_.size(), d = levels_[0].grid->g.D;
+    std::vector<int32_t> nc((size_t)n * d);
+    std::vector<int64_t> counts(n);
+    int done = 0, rc;
+    {
+      py::gil_scoped_release release;
+      rc = tfgpc_cell_grid_sample_report(stream_, n, d, levels_[0].grid->g.max_cells, nc.data(),
+                                         counts.data(), &done);
+    }
+    if (rc) {
+      const std::vector<int32_t> first(nc.begin(), nc.begin() + d);
+      raise_error(rc, tfgpc_last_error(), &first);
+    }
+    py::list out;
+    for (int l = 0; l < done; ++l) {
+      Level& level = levels_[l];
+      level.grid->num_cells_host.assign(nc.begin() + l * d, nc.begin() + (l + 1) * d);
+      const Tensor pts = level.pts.narrow(0, 0, counts[l]), ids = level.ids.narrow(0, 0, counts[l]);
+      if (l + 1 < done) levels_[l + 1].grid->set_points(pts, ids);
+      out.append(py::make_tuple(pts, ids,
+                                level.idx ? py::cast(level.idx->narrow(0, 0, counts[l]))
+                                          : py::object(py::none()),
+                                *std::max_element(nc.begin() + l * d, nc.begin() + (l + 1) * d)));
+    }
+    return out;
+  }
+
+ private:
+  struct Level {
+    GridPtr grid;
+    Tensor radii, pts, ids;
+    OptTensor idx;
+  };
+
+  void enqueue(Level&& level, const std::vector<double>& cell_sizes, const Tensor& inv_radii) {
+    const CellGrid& grid = *level.grid;
+    const int64_t n = grid.g.n;
+    const int l = (int)levels_.size();
+    require((int)cell_sizes.size() == grid.g.D, "SamplingOp expects one cell size per dimension");
+    const std::vector<float> sizes = to_floats(cell_sizes);
+    level.radii = f32(inv_radii);
+    level.pts = empty({n, grid.g.D}, at::kFloat, like_);
+    level.ids = empty({n}, at::kInt, like_);
+    if (mode_ == 0) level.idx = empty({n}, at::kInt, like_);
+    const size_t need = tfgpc_cell_grid_workspace_bytes(grid.g.D, n, 0, grid.g.batch_size, grid.g.max_cells);
+    const size_t need_s = tfgpc_cells_sample_workspace_bytes(n);
+    if (!ws_.defined() || (size_t)ws_.numel() < align256(need) + need_s)
+      ws_ = bytes(align256(need) + need_s, like_);
+    char* p = (char*)ws_.data_ptr();
+    int64_t* counts = (int64_t*)counts_.data_ptr();
+    const Level* before = l > 0 ? &levels_[l - 1] : nullptr;
+    check(tfgpc_cell_grid_sample_level(
+        stream_, l, &grid.g, before ? fp(before->pts) : fp(grid.points),
+        before ? ip(before->ids) : ip(grid.batch_ids), before ? counts + l - 1 : nullptr,
+        sizes.data(), mode_, fp(level.radii), fpm(level.pts), ipm(level.ids),
+        level.idx ? ipm(*level.idx) : nullptr, counts + l, p, need, p + align256(need), need_s));
+    levels_.push_back(std::move(level));
+  }
+
+  int mode_;
+  void* stream_;
+  Tensor like_, counts_, ws_;
+  std::vector<Level> levels_;
+};
+
 void bind_cells(py::module_& m) {
   py::class_<CellGrid, GridPtr>(m, "CellGrid")
       .def("__getattr__", [](const CellGrid& g, const std::string& name) { return g.get(name); })
@@ -327,11 +471,18 @@ void bind_cells(py::module_& m) {
   m.def("cell_table_elems", &tfgpc_cell_table_elems);
   m.def("build_grid", &build_grid);
   m.def("count_neighbors", &count_neighbors);
+  m.def("count_neighbors_with_pdf", &count_neighbors_with_pdf);
   m.def("fill_neighbors", &fill_neighbors);
   m.def("density", &density, py::arg("grid"), py::arg("inv_radii"), py::arg("inv_bandwidth"),
         py::arg("pdf_mode"), py::arg("mode"), py::arg("pairs") = 0.0);
   m.def("sample", &sample);
   m.def("build_and_sample", &build_and_sample);
+  py::class_<SampleLevels>(m, "SampleLevels")
+      .def(py::init<const Tensor&, const Tensor&, int64_t, const std::vector<double>&, int, int,
+                    const Tensor&>())
+      .def("add", &SampleLevels::add)
+      .def("grid", &SampleLevels::grid)
+      .def("finish", &SampleLevels::finish);
 }
 
 }  // namespace tfgpc_host

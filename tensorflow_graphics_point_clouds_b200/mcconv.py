@@ -213,6 +213,28 @@ def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
                                        bandwidth=bandwidth)
 
 
+class _GridOfInput:
+  """In the place of a layer's neighborhood: a grid of its input cloud with cells of its
+  radius, as a hierarchy over the cloud has built it in the same pass."""
+
+  def __init__(self, grid):
+    self.grid = grid
+
+
+def _neighborhood_on(grid, radius, point_cloud_out, bandwidth):
+  from . import pc
+  return pc.grid_neighborhood_on(grid, radius, point_cloud_out, bandwidth=bandwidth)
+
+
+def layer_on_grid(layer, grid):
+  """What to give a layer as its neighborhood for it to work on `grid` (see _GridOfInput):
+  None, its own, where its forward or build_neighborhood is not the library's."""
+  if (_is_own(layer.forward, _LIBRARY_FORWARD) and
+      _is_own(layer.build_neighborhood, _LIBRARY_BUILD_NEIGHBORHOOD)):
+    return _GridOfInput(grid)
+  return None
+
+
 def _is_own(method, own):
   """Whether a bound method is the library's function `own`: not replaced in a subclass, on
   the class or on the object."""
@@ -260,7 +282,10 @@ class MCConv:
   def forward(self, features, point_cloud_in, point_cloud_out, radius, neighborhood=None,
               bandwidth=0.2, keep_for_backward=True):
     neigh, packed = neighborhood, None
-    if neigh is None and _is_own(self.build_neighborhood, _LIBRARY_BUILD_NEIGHBORHOOD):
+    if isinstance(neigh, _GridOfInput):
+      neigh = _neighborhood_on(neigh.grid, radius, point_cloud_out, bandwidth)
+      packed = neigh._packed
+    elif neigh is None and _is_own(self.build_neighborhood, _LIBRARY_BUILD_NEIGHBORHOOD):
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
       packed = neigh._packed      # (of these points: no other neighborhood's is asked for)
     elif neigh is None:
@@ -363,7 +388,7 @@ class MCConv:
     return dfeat, dw1, db1, dwf
 
 
-_LIBRARY_BUILD_NEIGHBORHOOD = MCConv.build_neighborhood
+_LIBRARY_BUILD_NEIGHBORHOOD, _LIBRARY_FORWARD = MCConv.build_neighborhood, MCConv.forward
 
 
 # ---- KPConv and PointConv: other bases on the same projection + weight product

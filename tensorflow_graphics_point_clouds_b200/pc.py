@@ -568,6 +568,22 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   return neigh
 
 
+def grid_neighborhood_on(grid, radius, point_cloud_sample, bandwidth=0.2, mode=0):
+  """grid_neighborhood_with_pdf on a grid of cells of `radius` that is there already, the
+  samples another cloud's."""
+  if grid._cells is None or point_cloud_sample is grid._point_cloud:
+    neigh = Neighborhood(grid, radius, point_cloud_sample)
+    neigh.compute_pdf(bandwidth=bandwidth, mode=mode)
+    return neigh
+  neigh = object.__new__(Neighborhood)._attach(grid, radius, point_cloud_sample, 0)
+  inv_bw = _to_dims(bandwidth, grid._point_cloud._dimension, neigh._radii.device, inverse=True)
+  neigh._counted, neigh._sample_pdf, neigh._packed = ops._lib.host().count_neighbors_with_pdf(
+      grid._cells, neigh._inv_radii, 0, point_cloud_sample._points, point_cloud_sample._batch_ids,
+      0, inv_bw, mode)
+  neigh._pdf_ready = True
+  return neigh
+
+
 # Cells up to this many radii wide are sampled from the grid, wider ones from a neighbor
 # list: a cell's taken points are marked around by one block, (taken) x (candidates) tests,
 # and a wide cell holds many of both.  From the grid / by lists, us, at 1, 3, 4, 6 and 8 radii:
@@ -602,21 +618,84 @@ def sample(neighborhood, sample_mode='poisson'):
   return PointCloud(pts, bids, g._batch_size), idx
 
 
+# Points and cells up to which the grid of a level can be built for a number of points that the
+# host does not know yet, and levels of one call (tfgpc_cell_grid_sample_levels).
+_LEVELS_POINTS, _LEVELS_CELLS, _LEVELS_BOXES, _LEVELS_MOST = 65536, 1 << 21, 1024, 16
+_LIBRARY_BUILD_AND_SAMPLE = ops.build_cell_grid_and_sample
+
+
 class PointHierarchy:
   """PointHierarchy.py:40-98: per level Grid -> self Neighborhood -> sample.  Grid and
-  sampling of a level are one library call with one blocking read; the neighborhoods
-  count and write their lists when they are used (the sampling needs none)."""
+  sampling of a level are one library call; the levels after one follow it without a
+  blocking read of their own, as long as they have 65 536 points at most.  The
+  neighborhoods count and write their lists when they are used (the sampling needs none)."""
 
   def __init__(self, point_cloud, cell_sizes, sample_mode='poisson'):
     self._point_clouds = [point_cloud]
     self._neighborhoods = []
     self._sample_indices = []
-    cur = point_cloud
-    for cs in cell_sizes:
-      neigh, cur, idx = self._level(cur, cs, sample_mode)
-      self._neighborhoods.append(neigh)
-      self._point_clouds.append(cur)
-      self._sample_indices.append(idx)
+    cur, done, cell_sizes = point_cloud, 0, list(cell_sizes)
+    while done < len(cell_sizes):
+      levels = self._levels(cur, cell_sizes[done:], sample_mode)
+      for neigh, cur, idx in levels or [self._level(cur, cell_sizes[done], sample_mode)]:
+        self._neighborhoods.append(neigh)
+        self._point_clouds.append(cur)
+        self._sample_indices.append(idx)
+        done += 1
+
+  def _levels(self, pc, cell_sizes, sample_mode):
+    """Several levels in one call, or None where that is not for these."""
+    n, d, b = pc._points.shape[0], pc._dimension, pc._batch_size
+    if (len(cell_sizes) < 2 or n == 0 or b * d > _LEVELS_BOXES or
+        pc._num_cells_reduce is not None or
+        getattr(self._level, '__func__', self._level) is not _LIBRARY_LEVEL or
+        ops.build_cell_grid_and_sample is not _LIBRARY_BUILD_AND_SAMPLE):
+      return None
+    dev = pc._points.device
+    mode = SAMPLE_MODES[sample_mode.lower()]
+
+    def build(points, batch_ids, batch_size, sizes, max_cells):
+      run = ops._lib.host().SampleLevels(points, batch_ids, batch_size, sizes, max_cells, mode,
+                                         _to_dims(cell_sizes[0], d, dev, inverse=True))
+      all_sizes = [sizes]
+      for cs in cell_sizes[1:_LEVELS_MOST]:
+        # the box of a level lies in the one before: its cells are known to be no more than these
+        level = _host_dims(cs, d)
+        bound = math.ceil(max_cells * max(a / c for a, c in zip(sizes, level)) + 1.0)
+        bound = 1 << (max(1, bound) - 1).bit_length()
+        if b * float(bound) ** d > _LEVELS_CELLS:
+          break
+        run.add(level, bound, _to_dims(cs, d, dev, inverse=True), _LEVELS_POINTS)
+        all_sizes.append(level)
+      # what does not take the numbers of samples is made while they are worked out
+      cloud, levels = pc, []
+      for l, level in enumerate(all_sizes):
+        grid = object.__new__(Grid)
+        grid._cell_sizes = _to_dims(cell_sizes[l], d, dev)
+        grid._adopt(cloud, run.grid(l), level)
+        neigh = object.__new__(Neighborhood)._attach(grid, cell_sizes[l], None, 0)
+        cloud = object.__new__(PointCloud)
+        cloud._points = cloud._batch_ids = points      # (its own once they are known)
+        cloud._num_cells_reduce = cloud._aabb = None
+        cloud._batch_size, cloud._dimension = b, d
+        levels.append((neigh, cloud))
+      built = run.finish()
+      return levels[0][0]._grid._cells, levels, built
+
+    built = _cell_grid(pc, _host_dims(cell_sizes[0], d), build)
+    if built is None:
+      return None
+    done = []
+    for (neigh, cloud), (points, batch_ids, idx, cells) in zip(built[1], built[2]):
+      if done:              # (what a grid of this cloud asks for, as _cell_grid keeps it)
+        bound = max(_FIRST_BOUND, 1 << (cells - 1).bit_length())
+        key = _bound_key(neigh._grid._point_cloud, neigh._grid._sizes)
+        for known in (key, key[:3]):
+          if _MAX_CELLS.get(known) != bound:
+            _remember(_MAX_CELLS, known, bound)
+      cloud._points, cloud._batch_ids = points, batch_ids
+      done.append((neigh, cloud, idx))
+    return done
 
   @staticmethod
   def _level(pc, radius, sample_mode):
@@ -637,3 +716,6 @@ class PointHierarchy:
     grid._adopt(pc, built[0], sizes)
     neigh = object.__new__(Neighborhood)._attach(grid, radius, None, 0)
     return neigh, PointCloud(built[1], built[2], pc._batch_size), built[3]
+
+
+_LIBRARY_LEVEL = PointHierarchy._level

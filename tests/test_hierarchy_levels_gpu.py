@@ -1,0 +1,90 @@
+"""Levels of a hierarchy that follow one another without a blocking read, against one call per
+level: bit for bit, at the edges of what a level may hold.  And neighborhoods with densities on a
+grid that is there already."""
+import pytest
+import torch
+
+from tensorflow_graphics_point_clouds_b200 import mcconv, pc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def cloud(n, b, d, seed, outside=0):
+  g = torch.Generator(device=DEV).manual_seed(seed)
+  ids = torch.sort(torch.randint(0, b, (n,), generator=g, device=DEV)).values.int()
+  if outside:
+    ids[-outside:] = b + 3
+  return pc.PointCloud(torch.rand((n, d), generator=g, device=DEV), ids, b)
+
+
+def one_by_one(start, radii, mode):
+  cur, out = start, []
+  for r in radii:
+    neigh, cur, idx = pc.PointHierarchy._level(cur, r, mode)
+    out.append((neigh, cur, idx))
+  return out
+
+
+# level 1 with 1 to 8192 points (sorted copies in the cluster) and more, with more than the 65 536
+# that can follow, a radius that shrinks (a table too large to follow), per dimension, many clouds
+@pytest.mark.parametrize("n,b,d,radii,outside", [
+    (1, 1, 3, [0.1, 0.2], 0), (3000, 3, 3, [0.05, 0.1, 0.2], 5), (60000, 2, 3, [0.02, 0.04], 0),
+    (60000, 1, 2, [0.004, 0.3, 0.4], 0), (100000, 4, 3, [0.05, 0.1, 0.2, 0.4], 0),
+    (90000, 1, 2, [0.002, 0.004, 0.01], 0), (5000, 2, 3, [0.2, 0.01, 0.3], 0),
+    (5000, 2, 3, [[0.1, 0.2, 0.05], [0.2, 0.1, 0.1]], 0), (4000, 400, 3, [0.3, 0.6], 0),
+    (5000, 2, 4, [0.2, 0.4, 0.8], 0)])
+@pytest.mark.parametrize("mode", ["poisson", "average"])
+def test_same_as_one_level_at_a_time(n, b, d, radii, outside, mode):
+  if mode == "average" and outside:
+    outside = 0
+  a = cloud(n, b, d, n + d, outside)
+  ref = one_by_one(a, radii, mode)
+  for _ in range(2):                    # (with bounds of cells not known yet, and known)
+    hier = pc.PointHierarchy(a, radii, mode)
+    assert len(hier._point_clouds) == len(radii) + 1
+    before = a
+    for l, (neigh, points, idx) in enumerate(ref):
+      got, grid = hier._point_clouds[l + 1], hier._neighborhoods[l]._grid
+      assert torch.equal(got._points, points._points)
+      assert torch.equal(got._batch_ids, points._batch_ids)
+      assert (idx is None) == (hier._sample_indices[l] is None)
+      assert idx is None or torch.equal(hier._sample_indices[l], idx)
+      assert grid._point_cloud is before and got._batch_size == b and got._dimension == d
+      for name in ("_sorted_points", "_sorted_indices", "_cur_keys", "_num_cells"):
+        assert torch.equal(getattr(grid, name), getattr(neigh._grid, name)), name
+      assert torch.equal(hier._neighborhoods[l]._neighbors, neigh._neighbors)
+      before = got
+
+
+def test_a_replaced_level_is_called(monkeypatch):
+  seen, library = [], pc.PointHierarchy._level
+  monkeypatch.setattr(pc.PointHierarchy, "_level",
+                      staticmethod(lambda *a: seen.append(1) or library(*a)))
+  pc.PointHierarchy(cloud(500, 2, 3, 1), [0.1, 0.2])
+  assert len(seen) == 2
+
+
+@pytest.mark.parametrize("n,ns,d", [(1, 1, 3), (5000, 700, 3), (5000, 20000, 2), (90000, 70000, 3)])
+def test_neighborhood_on_a_grid(n, ns, d):
+  a, out = cloud(n, 2, d, n), cloud(ns, 2, d, n + 1)
+  grid = pc.Grid(a, 0.1)
+  got = pc.grid_neighborhood_on(grid, 0.1, out, bandwidth=0.3)
+  ref = pc.grid_neighborhood_with_pdf(a, 0.1, out, bandwidth=0.3)
+  assert torch.equal(got._samples_neigh_ranges, ref._samples_neigh_ranges)
+  assert torch.equal(got._original_neigh_ids, ref._original_neigh_ids)
+  assert torch.equal(got.pdf_by_neighbor_id(), ref.pdf_by_neighbor_id())
+  assert d != 3 or torch.equal(got._packed, ref._packed)
+
+
+def test_a_layer_on_a_grid():
+  a, out = cloud(3000, 2, 3, 5), cloud(900, 2, 3, 6)
+  g = torch.Generator(device=DEV).manual_seed(7)
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  layer = mcconv.MCConv(r(1, 3, 16), r(1, 1, 16), r(1, 128, 32), 8)
+  x = r(3000, 8)
+  ref = layer.forward(x, a, out, 0.1)
+  given = mcconv.layer_on_grid(layer, pc.Grid(a, 0.1))
+  assert torch.equal(layer.forward(x, a, out, 0.1, neighborhood=given), ref)
+  layer.build_neighborhood = lambda *args: None
+  assert mcconv.layer_on_grid(layer, pc.Grid(a, 0.1)) is None
