@@ -7,10 +7,10 @@
 // so no neighbor list is needed: on 8 clouds of 100 000 Gaussian-mixture points
 // searching and writing the lists of four levels took 3.2 ms, the passes over them 0.6.
 // The passes and the compaction of the taken points in ascending index are one
-// cooperative launch; what bounds it is the chain of passes on small levels and the
-// marking on crowded ones.  Only cells of later passes are marked (13 of 26 neighbors
-// on average).  Clouds do not meet, so each has a team of blocks, in proportion to its
-// points, with barriers of its own.
+// cooperative launch; what bounds it is the marking of crowded cells.  Levels of up to 65 536
+// points are first tried without passes, whose chain bounds them (settle_kernel).  Only cells of
+// later passes are marked (13 of 26 neighbors on average).  Clouds do not meet, so each has a team
+// of blocks, in proportion to its points, with barriers of its own.
 //
 // Cell average (sampling_avg_kernels.cu.cc:43-88): one thread per occupied cell,
 // sequential fp32 sum of its points / count, cells in ascending first index (a warp per cell
@@ -31,7 +31,14 @@ constexpr int kMaxTeams = kMaxBlocks / 2;
 // 427 -> 385 us in this kernel).
 constexpr int kCrowded = 96;
 constexpr int kMaxCrowded = 128;
-constexpr size_t kHeadBytes = (size_t)(kMaxTeams + 4) * 4;   // barrier words before the states
+constexpr int kHeadWords = 8;             // before the teams' counters
+constexpr size_t kHeadBytes = (size_t)(kMaxTeams + kHeadWords) * 4;   // before the states
+// Levels of up to this many points are first tried without passes (settle_kernel).
+constexpr int64_t kFlowPoints = 65536;
+constexpr int kFlowPer = 128;             // points of a block
+constexpr int kFlowLists = 32;            // words of neighbors of a point
+constexpr int kFlowCell = 256;            // points of a cell
+constexpr int kFlowWork = 448;            // candidates of a point x points of eight lanes
 // Candidates of a mark loop between two signs of progress: well under a millisecond, and
 // none at all in cells of ordinary size.  A selection shows none (its loop has no register
 // left for it: spills, 1 % of a hierarchy); one over all points of a call takes some 30 ns
@@ -43,9 +50,16 @@ constexpr int kProgressMarks = 65536;
 constexpr int kLongCell = 64;
 inline unsigned long long barrier_period_ns(int64_t n) { return 500000000ull + 100ull * n; }
 
-// A warp per 8 points (16: 158 against 140 us in the three-level classifier).
+// Blocks of the two kernels for n points: a warp per 8 points (16: 158 against 140 us in the
+// three-level classifier), 8 lanes per point.
 __host__ __device__ __forceinline__ int64_t blocks_wanted(int64_t n) {
   return (n + 8 * kWarps - 1) / (8 * kWarps);
+}
+__host__ __device__ __forceinline__ int64_t settle_blocks(int64_t n) {
+  return (n + kThreads / 8 - 1) / (kThreads / 8);
+}
+__device__ __forceinline__ int sample_blocks(int64_t n, int grid) {
+  return (int)min((int64_t)grid, blocks_wanted(n));
 }
 
 struct SampleArgs {
@@ -55,8 +69,12 @@ struct SampleArgs {
   const float* inv_radii;
   uint8_t* state;              // [n] 0 open, 1 blocked, 2 taken (zero on entry)
   unsigned* arrived;           // barrier counter of the grid, error word, progress, a word unused,
-                               // then the teams' counters; all zero on entry
-  int32_t* block_total;        // [gridDim.x]
+                               // whether settle_kernel has failed, from kHeadWords on the teams'
+                               // counters; all zero on entry
+  unsigned long long* settled; // [n / 32] taken points below, settled ones above, zero on entry; null:
+                               // settle_kernel does not run
+  int write_blocks;            // gridDim.x of cells_sample_kernel
+  int32_t* block_total;        // [gridDim.x], zero on entry where `settled` is
   float* pts_out;
   int32_t* batch_out;
   int32_t* index_out;          // original indices (Poisson)
@@ -266,6 +284,39 @@ __device__ __forceinline__ void poisson_cell(const SampleArgs& a, const int* cel
     mark_neighbors<D>(a, taken, cell, batch, nc, total, inv_r, false, part, parts);
 }
 
+// Sorted points [x, y) of earlier passes in one half of a tube around `cell` (see later_points):
+// both ends from an odd last coordinate, the middle if the leading coordinates' bits are lower.
+template <int D>
+__device__ __forceinline__ int2 earlier_points(int code, const int* cell, int batch, const int* nc,
+                                               int total, const int32_t* __restrict__ start) {
+  int base = 0, scale = 1, rem = code >> 1, mine = 0, theirs = 0;
+  bool ok = true;
+#pragma unroll
+  for (int d = D - 2; d >= 0; --d) {
+    const int c = cell[d] + rem % 3 - 1;
+    rem /= 3;
+    ok = ok && c >= 0 && c < nc[d];
+    base += c * scale;
+    scale *= nc[d];
+    mine |= (cell[d] & 1) << d;
+    theirs |= (c & 1) << d;
+  }
+  const int z = cell[D - 1];
+  const bool second = code & 1, odd = z & 1;
+  int lo, hi;
+  if (theirs < mine) {
+    lo = odd ? z - 1 : z;
+    hi = odd ? min(z + 1, nc[D - 1] - 1) : z;
+    ok = ok && !second;
+  } else {
+    lo = hi = second ? z + 1 : z - 1;
+    ok = ok && odd && lo < nc[D - 1];
+  }
+  if (!ok) return make_int2(0, 0);
+  base = (batch * scale + base) * nc[D - 1];
+  return make_int2(__ldg(start + (total - (base + hi))), __ldg(start + (total - (base + lo)) + 1));
+}
+
 // The team of a block: blocks [begin, begin + size) work on `cloud`; with too many clouds
 // for teams, all blocks on all of them (cloud -1).  size 0: a block left over.
 struct Team { int cloud, begin, size; };
@@ -303,11 +354,191 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int64_t n, int block
   return Team{0, 0, 0};
 }
 
+// The selection without passes: a point is settled as soon as its earlier neighbors (of earlier
+// passes, or before it in its cell) are, not when all cells of their passes are.  Eight lanes find
+// those neighbors, as words of 32 points and masks; then they look at the words until one of the
+// neighbors is taken, or all are settled and none is.  All blocks are resident (a cooperative
+// launch), and a point waits for earlier ones only.  What is taken is counted for the block that
+// will write it (cells_sample_kernel, which follows and has nothing to wait for).  The chain of a level is a
+// search and some twenty trips to L2, where the passes have ten barriers and a walk per cell between
+// them: levels of 54 000, 10 600 and 2000 points take 81, 57 and 48 us by passes, 46, 23 and 21 so.
+// Where cells are crowded the passes, which test around taken points only, are the faster ones.  A
+// block finds that out from its first points' cells, before it tests any of them, or from a list or
+// a cell that is too full; then nothing of this counts (three levels from 60 000 points with 282
+// earlier candidates each: 1110 us without that, 265 with it, 330 by passes and a read per level).
+template <int D>
+__global__ void __launch_bounds__(kThreads, 4)
+settle_kernel(SampleArgs a) {
+  constexpr int kGroups = kThreads / 8, kTurns = kFlowPer / kGroups, kPer = kFlowLists / 8;
+  constexpr int kHalves = 2 * num_tubes<D>();
+  constexpr int kMine = D <= 3 ? (kHalves + 7) / 8 : 1;       // halves of a lane looked up at once
+  __shared__ uint2 lists[kFlowPer][kFlowLists];
+  __shared__ int listed[kFlowPer], candidates_s;
+  const int lane = lane_id(), eighth = lane & 7, group = threadIdx.x >> 3;
+  int nc[D];
+  float inv_r[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    nc[d] = __ldg(a.c.num_cells + d);
+    inv_r[d] = __ldg(a.inv_radii + d);
+  }
+  const int total = total_cells<D>(nc, a.c.batch_size);
+  if (total == 0) return;        // (a grid that got no cells: the call fails)
+  const int64_t n = a.n_dev ? __ldg(a.n_dev) : a.c.n;
+  volatile unsigned* const failed = a.arrived + 4;
+  // (as few blocks as have a point for every eight lanes)
+  const int blocks = (int)min((int64_t)gridDim.x, settle_blocks(n));
+  if ((int)blockIdx.x >= blocks) return;
+  if ((n + 3) / 4 > (int64_t)blocks * (kFlowPer / 4)) {       // (too few blocks are resident)
+    *failed = 1u;
+    return;
+  }
+  const int write_blocks = sample_blocks(n, a.write_blocks);
+  const int per = (int)((n + write_blocks - 1) / write_blocks);    // points that a block writes
+  const int turns = (int)((n + (int64_t)blocks * kGroups - 1) / ((int64_t)blocks * kGroups));
+  // Point q of this block: four neighboring ones to a warp at a time (mostly of one cell), and
+  // every blocks-th such four to a block: neighboring ones cost the same, and the slowest block
+  // decides.
+  auto point = [&](int q) { return ((int)blockIdx.x + (q >> 2) * blocks) * 4 + (q & 3); };
+  for (int i = threadIdx.x; i < kFlowPer; i += kThreads) listed[i] = 0;
+  if (threadIdx.x == 0) candidates_s = 0;
+  __syncthreads();
+  for (int turn = 0; turn < turns; ++turn) {
+    const int q = group + turn * kGroups;
+    const int j = point(q);
+    const int64_t key = j < n ? __ldg(a.keys + j) : -1;
+    const bool live = key >= 0 && key < total;         // (else in no cell: without neighbors)
+    int cell[D], rem = live ? (int)key : 0;
+#pragma unroll
+    for (int d = D - 1; d >= 0; --d) {
+      cell[d] = rem % nc[d];
+      rem /= nc[d];
+    }
+    int begin = 0, end = 0;
+    int2 r[kMine];
+#pragma unroll
+    for (int k = 0; k < kMine; ++k) r[k] = make_int2(0, 0);
+    if (live) {
+      begin = __ldg(a.c.start + (total - (int)key));
+      end = __ldg(a.c.start + (total - (int)key) + 1);
+#pragma unroll
+      for (int k = 0; k < kMine; ++k)
+        if (8 * k + eighth < kHalves)
+          r[k] = earlier_points<D>(8 * k + eighth, cell, rem, nc, total, a.c.start);
+    }
+    if (turn == 0) {
+      int mine = 0;
+#pragma unroll
+      for (int k = 0; k < kMine; ++k) mine += r[k].y - r[k].x;
+      if (kMine * 8 < kHalves && live)
+        for (int t = 8 * kMine + eighth; t < kHalves; t += 8) {
+          const int2 x = earlier_points<D>(t, cell, rem, nc, total, a.c.start);
+          mine += x.y - x.x;
+        }
+      mine = __reduce_add_sync(0xffffffffu, mine);
+      if (lane == 0) atomicAdd(&candidates_s, mine);
+      __syncthreads();
+      if (candidates_s > kFlowWork * kGroups / turns) {
+        if (threadIdx.x == 0) *failed = 1u;
+        return;
+      }
+    }
+    if (*failed) return;
+    if (!live) continue;
+    if (end - begin > kFlowCell) *failed = 1u;
+    float p[D];
+    load_coords<D>(a.c, j, p);
+    // the neighbors among the points [x, y), words w, w + step, ..
+    auto search = [&](int2 r, int w, int step) {
+      for (; r.x < r.y && w * 32 < r.y; w += step) {
+        unsigned mask = 0;
+        const int to = min(r.y, w * 32 + 32);
+        // (four loads under way together, also of the last few)
+        for (int i = max(r.x, w * 32); i < to; i += 4) {
+          float o[4][D];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) load_coords<D>(a.c, min(i + u, to - 1), o[u]);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (within<D>(p, o[u], inv_r)) mask |= 1u << (min(i + u, to - 1) & 31);
+        }
+        if (mask) {
+          const int slot = atomicAdd(&listed[q], 1);
+          if (slot < kFlowLists) lists[q][slot] = make_uint2((unsigned)w, mask);
+          else *failed = 1u;
+        }
+      }
+    };
+#pragma unroll 1
+    for (int k = 0; k < kMine; ++k) {
+      int2 x = r[0];
+#pragma unroll
+      for (int u = 1; u < kMine; ++u) x = k == u ? r[u] : x;
+      search(x, x.x >> 5, 1);
+    }
+    for (int t = 8 * kMine + eighth; t < kHalves; t += 8) {
+      const int2 x = earlier_points<D>(t, cell, rem, nc, total, a.c.start);
+      search(x, x.x >> 5, 1);
+    }
+    search(make_int2(begin, j), (begin >> 5) + eighth, 8);
+  }
+  __syncwarp();
+  unsigned left = 0;          // turns whose point is not settled yet
+#pragma unroll
+  for (int k = 0; k < kTurns; ++k) left |= (k < turns && point(group + k * kGroups) < n) << k;
+  unsigned long long t0 = 0;
+  for (unsigned look = 1; __any_sync(0xffffffffu, left); ++look) {
+    if ((look & 7u) == 0 && __any_sync(0xffffffffu, *failed != 0u)) return;
+    if ((look & 255u) == 0) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (__any_sync(0xffffffffu, t - t0 > 2 * a.period_ns)) {
+        *(volatile unsigned*)(a.arrived + 1) = 1u;     // (no other block waits for long either)
+        *failed = 1u;
+        return;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kTurns; ++k) {
+      if (!__any_sync(0xffffffffu, left >> k & 1u)) continue;
+      const int q = group + k * kGroups;
+      const bool open = left >> k & 1u;
+      const int count = open ? min(listed[q], kFlowLists) : 0;
+      bool blocked = false, waits = false;
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) {
+        const int slot = eighth + 8 * e;
+        if (slot < count) {
+          const uint2 l = lists[q][slot];
+          const unsigned long long v =
+              *(const volatile unsigned long long*)(a.settled + l.x);
+          blocked = blocked || ((unsigned)v & l.y) != 0u;
+          waits = waits || (l.y & ~(unsigned)(v >> 32)) != 0u;
+        }
+      }
+      const unsigned any_blocked = __ballot_sync(0xffffffffu, blocked) >> (lane & 24) & 0xffu;
+      const unsigned any_waits = __ballot_sync(0xffffffffu, waits) >> (lane & 24) & 0xffu;
+      if (open && (any_blocked || !any_waits)) {
+        left &= ~(1u << k);
+        if (eighth == 0) {
+          const int j = point(q);
+          const unsigned long long bit = 1ull << (j & 31);
+          atomicOr(a.settled + (j >> 5), any_blocked ? bit << 32 : bit << 32 | bit);
+          if (!any_blocked) {
+            __stcg(a.state + j, (uint8_t)2);
+            atomicAdd(a.block_total + j / per, 1);
+          }
+        }
+      }
+    }
+  }
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 cells_sample_kernel(SampleArgs a) {
-  __shared__ int warp_total[kWarps];
-  __shared__ int64_t before_s;
+  __shared__ int warp_total[kWarps], warp_all[kWarps], before_s;
   __shared__ int crowded[kMaxCrowded], num_crowded[2];     // (counters of this pass and the next)
   const int lane = lane_id(), w = threadIdx.x >> 5;
   int nc[D];
@@ -319,10 +550,10 @@ cells_sample_kernel(SampleArgs a) {
     return;
   }
   const int64_t n = a.n_dev ? __ldg(a.n_dev) : a.c.n;
-  const int blocks = a.n_dev ? (int)min((int64_t)gridDim.x, blocks_wanted(n)) : (int)gridDim.x;
+  const int blocks = sample_blocks(n, (int)gridDim.x);
   if ((int)blockIdx.x >= blocks) return;      // (nobody waits for them)
   unsigned barriers = 0;
-  bool ok = true;
+  bool ok = true, settled = false;
   if (a.mode == 0) {
     float inv_r[D];
 #pragma unroll
@@ -334,11 +565,21 @@ cells_sample_kernel(SampleArgs a) {
       a.state[i < lead ? i : tail + (i - lead)] = 2;
     if (threadIdx.x == 0) num_crowded[0] = 0;
     __syncthreads();
-    const Team team = team_of(a.c, n, blocks, total);
+    if (a.settled) {
+      settled = a.arrived[4] == 0u;
+      if (!settled) {          // all states as before that kernel
+        for (int64_t i = lead + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < tail;
+             i += (int64_t)blocks * kThreads)
+          a.state[i] = 0;
+        ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
+                          a.period_ns) && ok;
+      }
+    }
+    const Team team = settled ? Team{0, 0, 0} : team_of(a.c, n, blocks, total);
     const int warps = team.size * kWarps;
     // neighboring cells go to different blocks: crowded ones come side by side
     const int warp = w * team.size + (int)blockIdx.x - team.begin;
-    unsigned* const counter = team.cloud < 0 ? a.arrived : a.arrived + 4 + team.cloud;
+    unsigned* const counter = team.cloud < 0 ? a.arrived : a.arrived + kHeadWords + team.cloud;
     for (int pass = 0; pass < (1 << D) && team.size > 0; ++pass) {
       int half[D], cells = team.cloud < 0 ? a.c.batch_size : 1;
 #pragma unroll
@@ -398,12 +639,13 @@ cells_sample_kernel(SampleArgs a) {
         poisson_cell<D>(a, cell, batch, begin, end, nc, total, inv_r, w, kWarps);
       }
       if (pass + 1 == (1 << D)) break;     // (the compaction begins with a barrier)
-      ok = grid_barrier(counter, (pass + 1) * team.size, a.arrived + 1, a.arrived + 2,
+      ok = grid_barrier(counter, (pass + 1 + (team.cloud < 0 ? barriers : 0)) * team.size, a.arrived + 1, a.arrived + 2,
                         a.period_ns) && ok;
     }
-    if (team.cloud < 0) barriers = (1 << D) - 1;
-    ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
-                      a.period_ns) && ok;
+    if (team.cloud < 0) barriers += (1 << D) - 1;
+    if (!settled)
+      ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
+                        a.period_ns) && ok;
   }
   // ---- compaction: every block counts, then writes, its stretch of the points
   const int64_t per = (n + blocks - 1) / blocks;
@@ -413,37 +655,50 @@ cells_sample_kernel(SampleArgs a) {
     return a.mode == 0 ? __ldcg(a.state + i) == 2
                        : i == 0 || __ldg(a.keys + i) != __ldg(a.keys + i - 1);
   };
-  int mine = 0;
-  for (int64_t i = first + threadIdx.x; i < last; i += kThreads) mine += chosen(i);
+  if (!settled) {
+    int mine = 0;
+    for (int64_t i = first + threadIdx.x; i < last; i += kThreads) mine += chosen(i);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if (lane == 0) warp_total[w] = mine;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int i = 0; i < kWarps; ++i) t += warp_total[i];
-    __stcg(a.block_total + blockIdx.x, t);
+    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+    if (lane == 0) warp_total[w] = mine;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int t = 0;
+      for (int i = 0; i < kWarps; ++i) t += warp_total[i];
+      __stcg(a.block_total + blockIdx.x, t);
+    }
+    ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
+                      a.period_ns) && ok;
   }
-  ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
-                    a.period_ns) && ok;
   ok = ok && !any_gave_up(a.arrived + 1);
-  if (w == 0) {
-    int64_t t = 0, all = 0;
-    for (int i = lane; i < blocks; i += 32) {
-      const int v = __ldcg(a.block_total + i);
-      all += v;
-      if (i < (int)blockIdx.x) t += v;
-    }
+  {
+    // samples of the blocks before this one, and all
+    int t = 0, all = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      t += __shfl_xor_sync(0xffffffffu, t, o);
-      all += __shfl_xor_sync(0xffffffffu, all, o);
+    for (int k = 0; k < kMaxBlocks / kThreads; ++k) {
+      const int i = (int)threadIdx.x + k * kThreads;
+      const int v = i < blocks ? __ldcg(a.block_total + i) : 0;
+      all += v;
+      t += i < (int)blockIdx.x ? v : 0;
     }
+    t = __reduce_add_sync(0xffffffffu, t);
+    all = __reduce_add_sync(0xffffffffu, all);
+    __syncthreads();
     if (lane == 0) {
+      warp_total[w] = t;
+      warp_all[w] = all;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      t = all = 0;
+      for (int i = 0; i < kWarps; ++i) {
+        t += warp_total[i];
+        all += warp_all[i];
+      }
       before_s = t;
       if (blockIdx.x == 0) {
-        a.page[0] = (int32_t)(uint32_t)all;
-        a.page[1] = (int32_t)(all >> 32);
+        a.page[0] = all;
+        a.page[1] = 0;
         a.page[2] = ok ? 0 : 1;
         if (a.samples_dev) *a.samples_dev = ok ? all : 0;
       }
@@ -537,22 +792,36 @@ cells_sample_kernel(SampleArgs a) {
   }
 }
 
-template <int D>
-int launch_sample(cudaStream_t st, SampleArgs a) {
+// Blocks of a cooperative launch that are resident at once, at most 4 per SM.
+template <auto kKernel>
+int resident_blocks(int64_t wanted, unsigned* blocks) {
   static int per_sm = 0;     // (the same value whoever computes it)
   if (per_sm == 0) {
     int v = 0;
-    TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, cells_sample_kernel<D>, kThreads, 0));
+    TFGPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kKernel, kThreads, 0));
     per_sm = v < 1 ? 1 : v;
   }
-  // at most 4 blocks per SM and what is resident at once
-  int64_t blocks = blocks_wanted(a.c.n);
   const int64_t most = (int64_t)sm_count() * (per_sm < 4 ? per_sm : 4);
-  if (blocks > most) blocks = most;
-  if (blocks > kMaxBlocks) blocks = kMaxBlocks;
+  if (wanted > most) wanted = most;
+  *blocks = (unsigned)(wanted > kMaxBlocks ? kMaxBlocks : wanted);
+  return TFGPC_OK;
+}
+
+template <int D>
+int launch_sample(cudaStream_t st, SampleArgs a) {
+  unsigned blocks = 0;
+  int rc = resident_blocks<cells_sample_kernel<D>>(blocks_wanted(a.c.n), &blocks);
+  if (rc) return rc;
+  a.write_blocks = (int)blocks;
   void* args[] = {&a};
-  TFGPC_CUDA(cudaLaunchCooperativeKernel(cells_sample_kernel<D>, dim3((unsigned)blocks),
-                                         dim3(kThreads), args, 0, st));
+  if (a.settled) {
+    unsigned first = 0;
+    rc = resident_blocks<settle_kernel<D>>(settle_blocks(a.c.n), &first);
+    if (rc) return rc;
+    TFGPC_CUDA(cudaLaunchCooperativeKernel(settle_kernel<D>, dim3(first), dim3(kThreads), args, 0, st));
+  }
+  TFGPC_CUDA(cudaLaunchCooperativeKernel(cells_sample_kernel<D>, dim3(blocks), dim3(kThreads), args,
+                                         0, st));
   return TFGPC_OK;
 }
 
@@ -582,20 +851,24 @@ __global__ void barrier_probe_kernel(unsigned* words, int late_block, int late_a
   if (!ok) atomicAdd(words + 5, 1u);
 }
 
-size_t sample_ws_bytes(int64_t n) {
-  return align_up((size_t)n + kHeadBytes, 256) + align_up((size_t)kMaxBlocks * 4, 256);
+// Barrier words, a byte of state per point, of a level that settle_points is tried on two bits, and
+// the blocks' totals.
+size_t settled_at(int64_t n) { return align_up((size_t)n + kHeadBytes, 8); }
+size_t totals_at(int64_t n) {
+  return settled_at(n) + (n <= kFlowPoints ? (size_t)((n + 31) / 32) * 8 : 0);
 }
 
-// What has to be zero before the kernel starts: barrier words, and the points' states.
+size_t sample_ws_bytes(int64_t n) { return align_up(totals_at(n) + (size_t)kMaxBlocks * 4, 256); }
+
+// What has to be zero before the kernel starts.
 size_t clear_bytes(int64_t n, int mode) {
-  return align_up(mode == 0 ? (size_t)n + kHeadBytes : kHeadBytes, 4);
+  return mode != 0 ? kHeadBytes : totals_at(n) + (n <= kFlowPoints ? (size_t)kMaxBlocks * 4 : 0);
 }
 
 // Enqueues the sampling; the number of samples goes to words kReportTotal .. of the page.
 int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const float* inv_radii,
                  float* pts_out, int32_t* batch_out, int32_t* index_out, void* ws, int32_t* page,
                  bool cleared, const int64_t* n_dev = nullptr, int64_t* samples_dev = nullptr) {
-  const size_t state = align_up((size_t)g.n + kHeadBytes, 256);
   SampleArgs a;
   a.c = view_of(g);
   a.keys = g.sorted_keys;
@@ -603,7 +876,9 @@ int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const floa
   a.inv_radii = inv_radii;
   a.arrived = (unsigned*)ws;
   a.state = (uint8_t*)ws + kHeadBytes;
-  a.block_total = (int32_t*)((char*)ws + state);
+  a.settled = mode == 0 && g.n <= kFlowPoints ? (unsigned long long*)((char*)ws + settled_at(g.n))
+                                              : nullptr;
+  a.block_total = (int32_t*)((char*)ws + totals_at(g.n));
   a.pts_out = pts_out;
   a.batch_out = batch_out;
   a.index_out = index_out;
