@@ -223,10 +223,13 @@ cells_walk_kernel(WalkArgs a) {
         int at[kSteps], index[kSteps];
 #pragma unroll
         for (int k = 0; k < kSteps; k += 2) {
-          // (few candidates: half the places stay empty.  524 288 points with 12 neighbors, density
-          // 131 -> 108 us in three dimensions, 76 -> 65 in two; a branch per pair of steps costs
-          // small clouds more than it saves, 10.6 -> 11.6 us, and four dimensions 3 % here too)
-          if (MODE == kDensity && D <= 3 && k >= kSteps / 2 && steps <= kSteps / 2) continue;
+          // (few candidates: half the places stay empty.  524 288 points with 12 neighbors, three
+          // dimensions: density 131 -> 108 us, list 144 -> 121; surfaces list 411 -> 400.  Count and
+          // two lists gain as much there and lose 2 to 5 % with 34 neighbors and on surfaces; a branch
+          // per pair of steps costs small clouds more than it saves, 10.6 -> 11.6 us, and four
+          // dimensions 3 % here too)
+          if ((MODE == kDensity || MODE == kFill) && D <= 3 && k >= kSteps / 2 && steps <= kSteps / 2)
+            continue;
           float p[2][D];
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
