@@ -457,6 +457,17 @@ int tfgpc_compute_pdf_pt_grads(void* stream, int D, int mode, int64_t n,
                                const float* inv_radii, const float* pdf_grads,
                                float* pt_grads_out);
 
+/* The same for lists that hold (j, i) with every (i, j), as those of a self neighborhood
+ * without limit do: without atomics, in a fixed order. */
+int tfgpc_compute_pdf_pt_grads_symmetric(void* stream, int D, int mode,
+                                         int64_t n, const float* points,
+                                         const int32_t* neighbors, int64_t M,
+                                         const int32_t* ranges,
+                                         const float* inv_bandwidth,
+                                         const float* inv_radii,
+                                         const float* pdf_grads,
+                                         float* pt_grads_out);
+
 /* Density at arbitrary sample positions: the same sum as tfgpc_compute_pdf but
  * centred on samples [ns,D] whose neighbor lists (neighbors [M,2], ranges
  * [ns]) index points [n,D]; mode 1 uses sqrt(n).  When the samples are the

@@ -67,6 +67,7 @@ SYMBOLS = {
     "tfgpc_find_neighbors_count_static": c_int,
     "tfgpc_compute_pdf": c_int,
     "tfgpc_compute_pdf_pt_grads": c_int,
+    "tfgpc_compute_pdf_pt_grads_symmetric": c_int,
     "tfgpc_add_by_neighbor": c_int,
     "tfgpc_basis_proj": c_int,
     "tfgpc_basis_proj_grads": c_int,

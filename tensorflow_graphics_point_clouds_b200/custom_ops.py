@@ -439,13 +439,27 @@ def compute_pdf_at_samples(samples, points, neighbors, sample_neigh_indices, inv
 def compute_pdf_pt_grads(points, neighbors, sample_neigh_indices, inv_bandwidth, inv_radii,
                          pdf_grads, mode):
   """ComputePdfPtGrads (compute_pdf/cc/ops/compute_pdf_ops.cpp:58-74)."""
+  return _pdf_pt_grads(_lib.lib().tfgpc_compute_pdf_pt_grads, points, neighbors,
+                       sample_neigh_indices, inv_bandwidth, inv_radii, pdf_grads, mode)
+
+
+def compute_pdf_pt_grads_symmetric(points, neighbors, sample_neigh_indices, inv_bandwidth,
+                                   inv_radii, pdf_grads, mode):
+  """compute_pdf_pt_grads for lists that hold (j, i) with every (i, j)
+  (tfgpc_compute_pdf_pt_grads_symmetric)."""
+  return _pdf_pt_grads(_lib.lib().tfgpc_compute_pdf_pt_grads_symmetric, points, neighbors,
+                       sample_neigh_indices, inv_bandwidth, inv_radii, pdf_grads, mode)
+
+
+def _pdf_pt_grads(entry, points, neighbors, sample_neigh_indices, inv_bandwidth, inv_radii,
+                  pdf_grads, mode):
   points, neighbors, ranges, inv_bw, inv_r, n, d, mode = _pdf_args(
       points, neighbors, sample_neigh_indices, inv_bandwidth, inv_radii, mode)
   pdf_grads = _f32(pdf_grads)
   if pdf_grads.shape[0] != n:
     raise _lib.TfgpcError(1, "ComputePDFPtGradsOp expects one pdf gradient per point")
   out = torch.empty((n, d), dtype=torch.float32, device=points.device)
-  _lib.check(_lib.lib().tfgpc_compute_pdf_pt_grads(
+  _lib.check(entry(
       _stream(), c_int(d), c_int(mode), c_i64(n), ptr(points), ptr(neighbors),
       c_i64(neighbors.shape[0]), ptr(ranges), ptr(inv_bw), ptr(inv_r), ptr(pdf_grads), ptr(out)))
   return out

@@ -69,6 +69,7 @@ def _is_array(t, dtype):
 
 
 _LIBRARY_FILL = ops.find_neighbors_fill
+_LIBRARY_PT_GRADS = ops.compute_pdf_pt_grads
 
 
 class PointCloud:
@@ -471,18 +472,21 @@ class Neighborhood:
     inv_bw = _to_dims(bandwidth, d, self._radii.device, inverse=True)
     n = g._point_cloud._points.shape[0]
     pdf_grads = torch.as_tensor(pdf_grads, dtype=torch.float32)
+    # the lists of a self neighborhood without limit are symmetric
+    pt_grads = ops.compute_pdf_pt_grads
+    if pt_grads is _LIBRARY_PT_GRADS and not (self._equal_samples and self.max_neighbors > 0):
+      pt_grads = ops.compute_pdf_pt_grads_symmetric
     if not self._equal_samples and self._samples_are_grid_points():
       # the grid's own cloud as samples: these lists are the self neighborhood's, in the
       # points' own order
       ids = self._original_neigh_ids
       per_point = ops._lib.host().add_by_neighbor(ids, pdf_grads, n)
-      return ops.compute_pdf_pt_grads(g._point_cloud._points, ids, self._samples_neigh_ranges,
-                                      inv_bw, self._inv_radii, per_point, mode)
+      return pt_grads(g._point_cloud._points, ids, self._samples_neigh_ranges, inv_bw,
+                      self._inv_radii, per_point, mode)
     per_point = ops._lib.host().add_by_neighbor(self._neighbors, pdf_grads, n)
     nb = self if self._equal_samples else Neighborhood(g, self._radius)
-    grads_sorted = ops.compute_pdf_pt_grads(
-        g._sorted_points, nb._neighbors, nb._samples_neigh_ranges, inv_bw, self._inv_radii,
-        per_point, mode)
+    grads_sorted = pt_grads(g._sorted_points, nb._neighbors, nb._samples_neigh_ranges, inv_bw,
+                            self._inv_radii, per_point, mode)
     out = torch.empty_like(grads_sorted)
     out[g._sorted_indices.to(torch.int64)] = grads_sorted
     return out
