@@ -653,7 +653,12 @@ class PointHierarchy:
     if (len(cell_sizes) < 2 or n == 0 or b * d > _LEVELS_BOXES or
         pc._num_cells_reduce is not None or
         getattr(self._level, '__func__', self._level) is not _LIBRARY_LEVEL or
-        ops.build_cell_grid_and_sample is not _LIBRARY_BUILD_AND_SAMPLE):
+        ops.build_cell_grid_and_sample is not _LIBRARY_BUILD_AND_SAMPLE or
+        PointCloud is not _LIBRARY_CLOUD or PointCloud.__init__ is not _LIBRARY_CLOUD_INIT or
+        torch.as_tensor(pc._points) is not pc._points):       # (a default device moves them)
+      return None
+    all_sizes = [_host_dims(cs, d) for cs in cell_sizes[:_LEVELS_MOST]]
+    if not all(0.0 < c < math.inf for size in all_sizes for c in size):
       return None
     dev = pc._points.device
     mode = SAMPLE_MODES[sample_mode.lower()]
@@ -661,32 +666,31 @@ class PointHierarchy:
     def build(points, batch_ids, batch_size, sizes, max_cells):
       run = ops._lib.host().SampleLevels(points, batch_ids, batch_size, sizes, max_cells, mode,
                                          _to_dims(cell_sizes[0], d, dev, inverse=True))
-      all_sizes = [sizes]
-      for cs in cell_sizes[1:_LEVELS_MOST]:
+      taken = 1
+      for cs, level in zip(cell_sizes[1:], all_sizes[1:]):
         # the box of a level lies in the one before: its cells are known to be no more than these
-        level = _host_dims(cs, d)
         bound = math.ceil(max_cells * max(a / c for a, c in zip(sizes, level)) + 1.0)
         bound = 1 << (max(1, bound) - 1).bit_length()
         if b * float(bound) ** d > _LEVELS_CELLS:
           break
         run.add(level, bound, _to_dims(cs, d, dev, inverse=True), _LEVELS_POINTS)
-        all_sizes.append(level)
+        taken += 1
       # what does not take the numbers of samples is made while they are worked out
       cloud, levels = pc, []
-      for l, level in enumerate(all_sizes):
+      for l in range(taken):
         grid = object.__new__(Grid)
         grid._cell_sizes = _to_dims(cell_sizes[l], d, dev)
-        grid._adopt(cloud, run.grid(l), level)
+        grid._adopt(cloud, run.grid(l), all_sizes[l])
         neigh = object.__new__(Neighborhood)._attach(grid, cell_sizes[l], None, 0)
         cloud = object.__new__(PointCloud)
-        cloud._points = cloud._batch_ids = points      # (its own once they are known)
+        # (what its constructor sets, its own points once they are known)
+        cloud._points, cloud._batch_size, cloud._dimension = points, b, d
         cloud._num_cells_reduce = cloud._aabb = None
-        cloud._batch_size, cloud._dimension = b, d
         levels.append((neigh, cloud))
       built = run.finish()
       return levels[0][0]._grid._cells, levels, built
 
-    built = _cell_grid(pc, _host_dims(cell_sizes[0], d), build)
+    built = _cell_grid(pc, all_sizes[0], build)
     if built is None:
       return None
     done = []
@@ -723,3 +727,4 @@ class PointHierarchy:
 
 
 _LIBRARY_LEVEL = PointHierarchy._level
+_LIBRARY_CLOUD, _LIBRARY_CLOUD_INIT = PointCloud, PointCloud.__init__

@@ -4,7 +4,7 @@ grid that is there already."""
 import pytest
 import torch
 
-from tensorflow_graphics_point_clouds_b200 import mcconv, pc
+from tensorflow_graphics_point_clouds_b200 import _lib, mcconv, pc
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -63,6 +63,25 @@ def test_a_replaced_level_is_called(monkeypatch):
                       staticmethod(lambda *a: seen.append(1) or library(*a)))
   pc.PointHierarchy(cloud(500, 2, 3, 1), [0.1, 0.2])
   assert len(seen) == 2
+
+
+def test_a_replaced_cloud_is_called(monkeypatch):
+  class Cloud(pc.PointCloud):
+    pass
+
+  a = cloud(500, 2, 3, 2)
+  monkeypatch.setattr(pc, "PointCloud", Cloud)
+  hier = pc.PointHierarchy(a, [0.1, 0.2])
+  assert [type(c) for c in hier._point_clouds[1:]] == [Cloud, Cloud]
+
+
+@pytest.mark.parametrize("radii", [[0.1, 0.0], [0.1, -0.2]])
+def test_levels_are_refused_as_before(radii):
+  a = cloud(500, 2, 3, 3)
+  with pytest.raises(_lib.TfgpcError):
+    one_by_one(a, radii, "poisson")
+  with pytest.raises(_lib.TfgpcError):
+    pc.PointHierarchy(a, radii)
 
 
 @pytest.mark.parametrize("n,ns,d", [(1, 1, 3), (5000, 700, 3), (5000, 20000, 2), (90000, 70000, 3)])
