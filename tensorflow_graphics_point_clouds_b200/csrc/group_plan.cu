@@ -48,6 +48,13 @@ namespace {
 
 constexpr int kPlanThreads = 256;
 constexpr int kPlanWarps = kPlanThreads / 32;
+constexpr int kHeldPairs = 192;               // pairs of a group in the registers of its warp
+constexpr int kStagedRows = kMaxMerge / 4;    // rows of a group in its warp's shared memory
+static_assert(kHeldPairs % 32 == 0, "whole turns of a warp");
+static_assert(kStagedRows * sizeof(int4) <= kMaxMerge * sizeof(int32_t) &&
+              kStagedRows * sizeof(int32_t) <= (kMaxMerge + 2) * sizeof(int16_t) &&
+              (kMaxMerge + 2) * sizeof(int16_t) % sizeof(int32_t) == 0,
+              "staged rows and ids lie where the other way of merging keeps its values");
 
 // Pairs of sample s: [a, a + n).
 __device__ __forceinline__ void sample_range(const int32_t* ranges, int64_t s, int& a,
@@ -95,17 +102,29 @@ __device__ __forceinline__ int lower_bound(const int32_t* l, int n, int x) {
 // is "first" if no list of a lower slot holds the same id; the row of an id is
 // the number of first elements with a smaller id, counted list by list with one
 // binary search each and a running count of the first flags.
-__global__ void __launch_bounds__(kPlanThreads)
+//
+// A group is a chain of loads (order, ranges, pairs) around some 800 instructions of its
+// warp, so warps in flight and instructions count, not bytes (20 % of the memory's rate).
+// Through the bit set: the pairs of up to kHeldPairs are read at once and stay in registers
+// for both passes over them, the words of the set are counted four to a lane, up to
+// kStagedRows rows are put together in shared memory and stored in order (a store per
+// pair is a sector each), and every group has its own warp, since a grid of eight blocks per
+// SM is not resident at once and its second turn left SMs idle.  16.7 M pairs in 131 072
+// groups, us: 303; pairs in registers and a warp per group 215; words four to a lane
+// as well 212, with the registers of four blocks per SM in place of spills 185; rows
+// staged too 189, and with 192 pairs instead of 256, at five blocks per SM, 168 to 178 (the
+// same without staging 193 to 201).
+__global__ void __launch_bounds__(kPlanThreads, 5)
 group_merge_kernel(int64_t ns, int64_t groups, const int32_t* order,
                    const int32_t* ranges, const int2* nb_sorted,
                    const int2* nb_ids, const int32_t* group_begin,
                    int32_t* __restrict__ group_rows, int32_t* __restrict__ rows_id,
                    int4* __restrict__ rows_pair) {
   chain_enter(groups, (int64_t)gridDim.x * kPlanWarps);
-  __shared__ int32_t s_val[kPlanWarps][kMaxMerge];
-  __shared__ int16_t s_pre[kPlanWarps][kMaxMerge + 2];
-  __shared__ uint32_t s_bits[kPlanWarps][kBitmapBits / 32];
-  __shared__ uint16_t s_wpre[kPlanWarps][kBitmapBits / 32];
+  __shared__ __align__(16) int32_t s_val[kPlanWarps][kMaxMerge];
+  __shared__ __align__(16) int16_t s_pre[kPlanWarps][kMaxMerge + 2];
+  __shared__ __align__(16) uint32_t s_bits[kPlanWarps][kBitmapBits / 32];
+  __shared__ __align__(16) uint16_t s_wpre[kPlanWarps][kBitmapBits / 32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int32_t* val = s_val[w];
   int16_t* pre = s_pre[w];
@@ -129,7 +148,23 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* order,
       i = e - off;
       m = a + i;
     };
+    const int d1 = a1 - o1, d2 = a2 - o2, d3 = a3 - o3;
+    auto pair_of = [&](int e) { return e + (e >= o3 ? d3 : e >= o2 ? d2 : e >= o1 ? d1 : a0); };
     // ---- groups whose ids span few values: one bit per value, rank = bits below
+    const bool held = total <= kHeldPairs;
+    int held_x[kHeldPairs / 32], held_id[kHeldPairs / 32];
+    if (held) {
+#pragma unroll
+      for (int k = 0; k < kHeldPairs / 32; ++k) {
+        if (k * 32 >= total) break;
+        const int e = k * 32 + lane;
+        if (e < total) {
+          const int m = pair_of(e);
+          held_x[k] = ld_global(&nb_sorted[m].x);
+          held_id[k] = ld_global(&nb_ids[m].x);
+        }
+      }
+    }
     int lo = INT32_MAX, hi = -1;
     if (lane < 8 && total > 0) {
       // lists ascend: the smallest id is a list's first, the largest its last element
@@ -151,41 +186,80 @@ group_merge_kernel(int64_t ns, int64_t groups, const int32_t* order,
     if (total > 0 && hi - lo < kBitmapBits) {
       uint32_t* bits = s_bits[w];
       uint16_t* wpre = s_wpre[w];
+      // four words to a lane, 128 words at a time
       const int words = ((hi - lo) >> 5) + 1;
-      for (int i = lane; i < words; i += 32) bits[i] = 0u;
+      for (int i = lane * 4; i < words; i += 128)
+        *reinterpret_cast<uint4*>(bits + i) = make_uint4(0u, 0u, 0u, 0u);
       __syncwarp();
-      for (int e = lane; e < total; e += 32) {
-        int q, i, m;
-        locate(e, q, i, m);
-        const int x = ld_global(&nb_sorted[m].x) - lo;
+      auto mark = [&](int id) {
+        const int x = id - lo;
         atomicOr(&bits[x >> 5], 1u << (x & 31));
+      };
+      if (held) {
+#pragma unroll
+        for (int k = 0; k < kHeldPairs / 32; ++k) {
+          if (k * 32 >= total) break;
+          if (k * 32 + lane < total) mark(held_x[k]);
+        }
+      } else {
+        for (int e = lane; e < total; e += 32) mark(ld_global(&nb_sorted[pair_of(e)].x));
       }
       __syncwarp();
       // exclusive running count of the set bits, word by word
-      const int per = (words + 31) >> 5;
-      int mine = 0;
-      for (int i = lane * per; i < min(words, (lane + 1) * per); ++i) mine += __popc(bits[i]);
-      int run = mine;
+      int rows = 0;
+      for (int i0 = 0; i0 < words; i0 += 128) {
+        const int i = i0 + lane * 4;
+        uint4 b = make_uint4(0u, 0u, 0u, 0u);
+        if (i < words) b = *reinterpret_cast<const uint4*>(bits + i);
+        const int c1 = __popc(b.x), c2 = c1 + __popc(b.y), c3 = c2 + __popc(b.z);
+        const int mine = c3 + __popc(b.w);
+        int run = mine;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, run, o);
+          if (lane >= o) run += v;
+        }
+        const int below = rows + run - mine;
+        if (i < words)
+          *reinterpret_cast<ushort4*>(wpre + i) =
+              make_ushort4((unsigned short)below, (unsigned short)(below + c1),
+                           (unsigned short)(below + c2), (unsigned short)(below + c3));
+        rows += __shfl_sync(0xffffffffu, run, 31);
       }
-      const int rows = __shfl_sync(0xffffffffu, run, 31);
-      run -= mine;
-      for (int i = lane * per; i < min(words, (lane + 1) * per); ++i) {
-        wpre[i] = (uint16_t)run;
-        run += __popc(bits[i]);
-      }
-      for (int r = lane; r < rows; r += 32) rows_pair[base + r] = make_int4(-1, -1, -1, -1);
-      __syncwarp();
-      for (int e = lane; e < total; e += 32) {
-        int q, i, m;
-        locate(e, q, i, m);
-        const int x = ld_global(&nb_sorted[m].x) - lo;
-        const int rank = wpre[x >> 5] + __popc(bits[x >> 5] & ((1u << (x & 31)) - 1u));
-        rows_id[base + rank] = ld_global(&nb_ids[m].x);   // every pair of a row holds the same id
-        reinterpret_cast<int32_t*>(rows_pair + base + rank)[q] = m;
+      auto fill = [&](int4* row, int32_t* row_id) {
+        for (int r = lane; r < rows; r += 32) row[r] = make_int4(-1, -1, -1, -1);
+        __syncwarp();
+        auto put = [&](int e, int id, int neighbor) {
+          const int x = id - lo;
+          const int rank = wpre[x >> 5] + __popc(bits[x >> 5] & ((1u << (x & 31)) - 1u));
+          const int q = (e >= o1) + (e >= o2) + (e >= o3);
+          row_id[rank] = neighbor;   // every pair of a row holds the same id
+          reinterpret_cast<int32_t*>(row + rank)[q] = pair_of(e);
+        };
+        if (held) {
+#pragma unroll
+          for (int k = 0; k < kHeldPairs / 32; ++k) {
+            if (k * 32 >= total) break;
+            if (k * 32 + lane < total) put(k * 32 + lane, held_x[k], held_id[k]);
+          }
+        } else {
+          for (int e = lane; e < total; e += 32) {
+            const int m = pair_of(e);
+            put(e, ld_global(&nb_sorted[m].x), ld_global(&nb_ids[m].x));
+          }
+        }
+      };
+      if (rows <= kStagedRows) {
+        int4* const row = reinterpret_cast<int4*>(val);
+        int32_t* const row_id = reinterpret_cast<int32_t*>(pre);
+        fill(row, row_id);
+        __syncwarp();
+        for (int r = lane; r < rows; r += 32) {
+          rows_pair[base + r] = row[r];
+          rows_id[base + r] = row_id[r];
+        }
+      } else {
+        fill(rows_pair + base, rows_id + base);
       }
       if (lane == 0) group_rows[g] = rows;
       __syncwarp();
@@ -283,7 +357,7 @@ extern "C" int tfgpc_mcconv_group_plan(void* stream, int64_t ns, int64_t M, cons
   int rc = inclusive_scan_i32(st, v.group_begin + 1, v.group_begin + 1, v.groups, v.scan_sums,
                               v.scan_sums + scan_block_sums_elems(v.groups));
   if (rc) return rc;
-  unsigned grid = min(blocks_for(v.groups, gp::kPlanWarps), (unsigned)(sm_count() * 8));
+  unsigned grid = blocks_for(v.groups, gp::kPlanWarps);
   TFGPC_CUDA(launch_chained(st, grid, gp::kPlanThreads, 0, gp::group_merge_kernel, ns, v.groups,
       order, ranges, (const int2*)neighbors_sorted, (const int2*)neighbor_ids, v.group_begin,
       v.group_rows, v.rows_id, v.rows_pair));

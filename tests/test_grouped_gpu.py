@@ -88,6 +88,42 @@ def test_group_plan_matches_numpy(n_pts, n_smp, radius, own):
   check_plan(nb, order, plan)
 
 
+class Lists:
+  """Neighbor lists as a neighborhood holds them, ascending ids each."""
+
+  def __init__(self, lists):
+    sizes = np.array([len(l) for l in lists])
+    srt = np.stack([np.concatenate(lists), np.repeat(np.arange(len(lists)), sizes)], 1)
+    self._samples_neigh_ranges = t(np.cumsum(sizes).astype(np.int32))
+    self._neighbors = t(srt.astype(np.int32))
+    self._original_neigh_ids = t(np.stack([srt[:, 0] * 7 + 3, srt[:, 1]], 1).astype(np.int32))
+
+
+@pytest.mark.parametrize("pairs,rows", [(1, 1), (31, 9), (33, 32), (128, 127), (191, 128),
+                                        (192, 128), (193, 129), (192, 129), (193, 128), (600, 300)])
+@pytest.mark.parametrize("span", [1, 4096, 4097, 8192, 8193])
+def test_group_plan_at_the_edges_of_registers_staging_and_words(pairs, rows, span):
+  # `rows` distinct ids spread over `span` values (their own count at least), dealt to four
+  # lists that hold `pairs` ids in all, where as many fit; several groups, the last of three samples
+  rng = np.random.default_rng(pairs * 31 + rows)
+  lists = []
+  for group in range(9):
+    width = max(span, rows)
+    inner = rng.permutation(np.arange(1, max(width - 1, 1)))[:max(rows - 2, 0)]
+    ids = np.unique(np.concatenate([[0, width - 1][:rows], inner])).astype(np.int64) + 17 * group
+    slots = 4 if group < 8 else 3
+    hit = np.zeros((slots, len(ids)), bool)
+    hit[rng.integers(0, slots, len(ids)), np.arange(len(ids))] = True   # every id once
+    free = np.flatnonzero(~hit.reshape(-1))
+    more = max(min(pairs - len(ids), len(free)), 0)
+    hit.reshape(-1)[rng.permutation(free)[:more]] = True
+    lists += [ids[h] for h in hit]
+  nb = Lists(lists)
+  order, plan = mcconv.group_plan(nb)
+  torch.cuda.synchronize()
+  check_plan(nb, order, plan)
+
+
 @pytest.mark.parametrize("n_pts,radius,own", [(3001, 0.12, True), (2500, 0.3, True),
                                               (1500, 0.55, True), (3000, 0.1, False),
                                               (602, 0.05, True)])
