@@ -331,7 +331,8 @@ int tfgpc_cells_density_ws(void* stream, const tfgpc_cell_grid* grid,
  * mode 0 Poisson disk with the neighbors of a self neighborhood without limit
  * (inv_radii [D]), mode 1 cell average.  The outputs hold n rows, the first
  * *num_samples_out [host] are written; sample_indices_out (mode 0) are indices into
- * the UNSORTED points.  Blocks once.  tfgpc_cell_grid_sample builds the grid in the
+ * the UNSORTED points.  The workspace is aligned to 4 bytes (to 8 for levels of up to
+ * 65 536 points to take their fastest way).  Blocks once.  tfgpc_cell_grid_sample builds the grid in the
  * same call (`ws` of tfgpc_cell_grid_workspace_bytes with ns = 0), with the one
  * blocking read and the status of tfgpc_cell_grid_neighborhood. */
 size_t tfgpc_cells_sample_workspace_bytes(int64_t n);

@@ -966,8 +966,9 @@ int sample_async(cudaStream_t st, const tfgpc_cell_grid& g, int mode, const floa
   a.inv_radii = inv_radii;
   a.arrived = (unsigned*)ws;
   a.state = (uint8_t*)ws + kHeadBytes;
-  a.settled = mode == 0 && g.n <= kFlowPoints ? (unsigned long long*)((char*)ws + settled_at(g.n))
-                                              : nullptr;
+  // (by passes where a caller's workspace is not aligned for words of 64 bits)
+  const bool flow = mode == 0 && g.n <= kFlowPoints && (uintptr_t)ws % 8 == 0;
+  a.settled = flow ? (unsigned long long*)((char*)ws + settled_at(g.n)) : nullptr;
   a.block_total = (int32_t*)((char*)ws + totals_at(g.n));
   a.pts_out = pts_out;
   a.batch_out = batch_out;
@@ -995,6 +996,7 @@ int check_sample(const tfgpc_cell_grid* g, int mode, const float* inv_radii, con
   TFGPC_REQUIRE(mode == 0 || mode == 1, "SamplingOp expects mode 0 (poisson) or 1 (average)");
   TFGPC_REQUIRE(pts_out && batch_out && ws && num_samples_out &&
                 (mode == 1 || (index_out && inv_radii)), "SamplingOp got a null pointer");
+  TFGPC_REQUIRE((uintptr_t)ws % 4 == 0, "SamplingOp expects a workspace aligned to 4 bytes");
   if (ws_bytes < sample_ws_bytes(g->n)) return fail(TFGPC_ENOMEM, "SamplingOp workspace too small");
   return TFGPC_OK;
 }

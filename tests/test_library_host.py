@@ -94,6 +94,23 @@ def test_layer_entries_reject_bad_arguments(lib):
   assert lib.tfgpc_global_pool_workspace_bytes(i64(32)) >= 128
 
 
+class CellGrid(ctypes.Structure):
+  """tfgpc_cell_grid: for calls that are refused before anything is read."""
+  _fields_ = [("D", ctypes.c_int), ("max_cells", ctypes.c_int), ("n", ctypes.c_int64),
+              ("batch_size", ctypes.c_int64), ("arrays", ctypes.c_void_p * 13)]
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("offset", [1, 2, 6])
+def test_sampling_refuses_misaligned_workspaces(lib, mode, offset):
+  grid = CellGrid(3, 16, 100, 1, (ctypes.c_void_p * 13)(*[4096] * 13))
+  some, i64 = ctypes.c_void_p(4096), ctypes.c_int64(0)
+  need = ctypes.c_size_t(lib.tfgpc_cells_sample_workspace_bytes(ctypes.c_int64(100)))
+  rc = lib.tfgpc_cells_sample(None, ctypes.byref(grid), mode, some, some, some, some,
+                              ctypes.c_void_p(4096 + offset), need, ctypes.byref(i64))
+  assert rc == 1 and b"aligned to 4 bytes" in lib.tfgpc_last_error()
+
+
 @pytest.fixture(scope="module")
 def part_end(tmp_path_factory):
   """part_end of csrc/list_parts.h, compiled for the host."""

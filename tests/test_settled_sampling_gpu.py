@@ -1,12 +1,16 @@
 """Poisson disks settled point by point (levels of up to 65 536 points) against the CPU oracle:
 one to several points per eight lanes, chains through a cell, lists and cells that are too full (the
 passes do those), points outside the batch, two to five dimensions."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
+from test_cell_table_gpu import CellGridArrays
 
 from oracle import pylib_ref as pr
-from tensorflow_graphics_point_clouds_b200 import pc
+from tensorflow_graphics_point_clouds_b200 import _lib, pc
+from tensorflow_graphics_point_clouds_b200._lib import c_i64, c_sz, ptr
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -50,3 +54,35 @@ def test_points_outside_the_batch_are_taken():
   got = set(idx.tolist())
   assert set(range(10)) | set(range(680, 700)) <= got
   assert got - set(range(10)) - set(range(680, 700)) == {i + 10 for i in ref.tolist()}
+
+
+@pytest.mark.parametrize("n", [1, 2000, 65536])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_workspaces_aligned_to_words(n, mode):
+  """A workspace that is not aligned for 64-bit words is sampled with as ever: by passes."""
+  gen = torch.Generator(device=DEV).manual_seed(n)
+  points = torch.rand((n, 3), generator=gen, device=DEV)
+  ids = torch.zeros(n, dtype=torch.int32, device=DEV)
+  lib, g = _lib.lib(), CellGridArrays(3, 32, n, 1)
+  need = lib.tfgpc_cell_grid_workspace_bytes(3, c_i64(n), c_i64(0), c_i64(1), 32)
+  need_s = lib.tfgpc_cells_sample_workspace_bytes(c_i64(n))
+  ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+  room = torch.empty(need_s + 8, dtype=torch.uint8, device=DEV)
+  inv = torch.full((3,), 20.0, device=DEV)
+  stream, got = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), []
+  for offset in (0, 4, 2):
+    out = [torch.empty((n, 3), device=DEV)] + [torch.empty_like(ids) for _ in range(2)]
+    tail = (mode, ptr(inv), *map(ptr, out))
+    at = ctypes.c_void_p(room.data_ptr() + offset)
+    asked, first, second = (ctypes.c_int32 * 3)(), c_i64(0), c_i64(0)
+    rc = [lib.tfgpc_cell_grid_sample(
+        stream, ctypes.byref(g), ptr(points), ptr(ids), (ctypes.c_float * 3)(*[0.05] * 3), None,
+        *tail, ptr(ws), c_sz(need), at, c_sz(need_s), asked, ctypes.byref(first))]
+    rc.append(lib.tfgpc_cells_sample(stream, ctypes.byref(g), *tail, at, c_sz(need_s),
+                                     ctypes.byref(second)))
+    if offset == 2:
+      assert rc == [1, 1]
+      continue
+    assert rc == [0, 0] and first.value == second.value
+    got.append([x[:first.value].cpu() for x in (out if mode == 0 else out[:2])])
+  assert all(torch.equal(a, b) for a, b in zip(*got)) and len(got) == 2
