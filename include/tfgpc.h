@@ -354,7 +354,8 @@ int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
 
 /* tfgpc_cell_grid_sample of several levels, each on the samples of the one before, with one
  * blocking read: tfgpc_cell_grid_sample_level enqueues level 0, 1, .. and does not block,
- * tfgpc_cell_grid_sample_report waits for all of them (same host thread).  A level leaves the number
+ * tfgpc_cell_grid_sample_report waits for all of them (same host thread, and no other entry
+ * that blocks in between: it would report in the same place).  A level leaves the number
  * of its samples in *num_samples_dev_out; the next one takes that pointer as n_dev (NULL: it has
  * grid->n points) and holds grid->n points at most, few enough for one cluster (65 536, a table of
  * 2^21 cells, batch_size * D <= 1024).  Workspaces may be shared by the levels of a stream.

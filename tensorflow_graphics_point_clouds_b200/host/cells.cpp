@@ -358,9 +358,15 @@ static py::tuple build_and_sample(const Tensor& points, const Tensor& batch_ids,
 }
 
 // The levels of a hierarchy one after the other: a level is under way from its add on, so that the
-// host makes the next one's arrays meanwhile; finish blocks.
+// host makes the next one's arrays meanwhile; finish blocks.  The levels under way write to the
+// report page of this thread, as every reporting call of it does: where finish is not reached,
+// they are waited for.
 class SampleLevels {
  public:
+  SampleLevels(const SampleLevels&) = delete;
+  SampleLevels& operator=(const SampleLevels&) = delete;
+  ~SampleLevels() { wait(); }
+
   SampleLevels(const Tensor& points, const Tensor& batch_ids, int64_t batch_size,
                const std::vector<double>& cell_sizes, int max_cells, int mode,
                const Tensor& inv_radii)
@@ -386,6 +392,16 @@ class SampleLevels {
 
   GridPtr grid(int level) const { return levels_.at(level).grid; }
 
+  // Until nothing of it is under way; what the levels have reported is dropped.
+  void wait() {
+    if (!under_way_) return;
+    under_way_ = false;
+    int32_t nc[TFGPC_MAX_DIMS];
+    int64_t count = 0;
+    int done = 0;
+    tfgpc_cell_grid_sample_report(stream_, 1, levels_[0].grid->g.D, 1, nc, &count, &done);
+  }
+
   // [(points, batch ids, original indices or None, cells per dimension at most)] of the levels
   // that could be built
   py::list finish() {
@@ -393,6 +409,7 @@ class SampleLevels {
     std::vector<int32_t> nc((size_t)n * d);
     std::vector<int64_t> counts(n);
     int done = 0, rc;
+    under_way_ = false;
     {
       py::gil_scoped_release release;
       rc = tfgpc_cell_grid_sample_report(stream_, n, d, levels_[0].grid->g.max_cells, nc.data(),
@@ -446,9 +463,11 @@ class SampleLevels {
         sizes.data(), mode_, fp(level.radii), fpm(level.pts), ipm(level.ids),
         level.idx ? ipm(*level.idx) : nullptr, counts + l, p, need, p + align256(need), need_s));
     levels_.push_back(std::move(level));
+    under_way_ = true;
   }
 
   int mode_;
+  bool under_way_ = false;
   void* stream_;
   Tensor like_, counts_, ws_;
   std::vector<Level> levels_;
@@ -482,6 +501,7 @@ void bind_cells(py::module_& m) {
                     const Tensor&>())
       .def("add", &SampleLevels::add)
       .def("grid", &SampleLevels::grid)
+      .def("wait", &SampleLevels::wait)
       .def("finish", &SampleLevels::finish);
 }
 

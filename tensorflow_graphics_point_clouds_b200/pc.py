@@ -666,6 +666,13 @@ class PointHierarchy:
     def build(points, batch_ids, batch_size, sizes, max_cells):
       run = ops._lib.host().SampleLevels(points, batch_ids, batch_size, sizes, max_cells, mode,
                                          _to_dims(cell_sizes[0], d, dev, inverse=True))
+      try:
+        return further_levels(run, points, sizes, max_cells)
+      except BaseException:
+        run.wait()          # (its kernels write where the next call of this thread reads)
+        raise
+
+    def further_levels(run, points, sizes, max_cells):
       taken = 1
       for cs, level in zip(cell_sizes[1:], all_sizes[1:]):
         # the box of a level lies in the one before: its cells are known to be no more than these

@@ -84,6 +84,32 @@ def test_levels_are_refused_as_before(radii):
     pc.PointHierarchy(a, radii)
 
 
+@pytest.mark.parametrize("where", ["_to_dims", "_attach"])
+def test_levels_under_way_are_waited_for(where, monkeypatch):
+  """Where anything fails between the first level and the report, no kernel is left that would
+  write to what the thread's next call reads."""
+  a = cloud(5000, 2, 3, 4)
+  pc.PointHierarchy(a, [0.1, 0.2])
+  holder, calls = (pc, 1) if where == "_to_dims" else (pc.Neighborhood, 0)
+  library, seen = getattr(holder, where), []
+
+  def failing(*args, **kwargs):
+    seen.append(1)
+    if len(seen) > calls:
+      raise KeyboardInterrupt
+    return library(*args, **kwargs)
+
+  stream = torch.cuda.Stream()
+  with torch.cuda.stream(stream):
+    torch.cuda._sleep(100_000_000)              # (tens of ms: the levels wait behind it)
+    monkeypatch.setattr(holder, where, failing)
+    with pytest.raises(KeyboardInterrupt):
+      pc.PointHierarchy(a, [0.1, 0.2])
+    assert stream.query()
+  monkeypatch.undo()
+  assert len(pc.PointHierarchy(a, [0.1, 0.2])._point_clouds) == 3
+
+
 @pytest.mark.parametrize("n,ns,d", [(1, 1, 3), (5000, 700, 3), (5000, 20000, 2), (90000, 70000, 3)])
 def test_neighborhood_on_a_grid(n, ns, d):
   a, out = cloud(n, 2, d, n), cloud(ns, 2, d, n + 1)
