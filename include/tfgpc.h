@@ -357,12 +357,15 @@ int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
  * tfgpc_cell_grid_sample_report waits for all of them (same host thread, and no other entry
  * that blocks in between: it would report in the same place).  A level leaves the number
  * of its samples in *num_samples_dev_out; the next one takes that pointer as n_dev (NULL: it has
- * grid->n points) and holds grid->n points at most, few enough for one cluster (65 536, a table of
- * 2^21 cells, batch_size * D <= 1024).  Workspaces may be shared by the levels of a stream.
+ * grid->n points) and holds grid->n points at most: no more than tfgpc_cell_grid_level_points, those
+ * of the largest grid that one cluster of the current device builds (65 536 where clusters of 16
+ * blocks are granted; 0: none, as for tables of more than 2^21 cells and batch_size * D > 1024).
+ * Workspaces may be shared by the levels of a stream.
  * num_cells_host_out [levels,D], num_samples_out [levels]; *levels_done_out: levels that were
  * built (none from a level on that got more than its grid->n points or asked for more than its
  * max_cells; the first: TFGPC_ENOMEM). */
 #define TFGPC_MAX_CHAINED_LEVELS 16
+int64_t tfgpc_cell_grid_level_points(int D, int64_t batch_size, int max_cells);
 int tfgpc_cell_grid_sample_level(
     void* stream, int level, const tfgpc_cell_grid* grid, const float* points,
     const int32_t* batch_ids, const int64_t* n_dev, const float* cell_sizes,

@@ -895,25 +895,25 @@ int place(cudaStream_t st, const tfgpc_cell_grid& g, const float* points, const 
                                  : launch_place<256>(st, g, points, batch_ids, w, n_dev);
 }
 
-// Blocks of the cluster that a grid can be built by, 0: it is too large for one.
-int cluster_for(const tfgpc_cell_grid& g, int* ranks) {
+// Blocks of the cluster that a grid of so many points can be built by, 0: it is too large for one.
+int cluster_for(int D, int64_t n, int64_t batch_size, int max_cells, int* ranks) {
   *ranks = 0;
-  if (g.n > kClusterPoints || table_cells(g.D, g.batch_size, g.max_cells) > kClusterCells ||
-      g.batch_size * g.D > kClusterBoxes)
+  const int64_t cells = table_cells(D, batch_size, max_cells);
+  if (n > kClusterPoints || cells <= 0 || cells > kClusterCells || batch_size * D > kClusterBoxes)
     return TFGPC_OK;
   int rc = TFGPC_OK;
-  TFGPC_DIM_SWITCH(g.D, rc = cluster_ranks<kD>(ranks));
-  if (!rc && g.n > (int64_t)*ranks * kClusterThreads * kHeld) *ranks = 0;
+  TFGPC_DIM_SWITCH(D, rc = cluster_ranks<kD>(ranks));
+  if (!rc && n > (int64_t)*ranks * kClusterThreads * kHeld) *ranks = 0;
   return rc;
 }
 
 }  // namespace
 
-int cell_grid_takes_cluster(const tfgpc_cell_grid& g, bool* takes) {
+int64_t cell_grid_cluster_points(int D, int64_t batch_size, int max_cells) {
   int ranks = 0;
-  const int rc = cluster_for(g, &ranks);
-  *takes = ranks > 0;
-  return rc;
+  if (cluster_for(D, 1, batch_size, max_cells, &ranks)) return 0;
+  const int64_t held = (int64_t)ranks * kClusterThreads * kHeld;
+  return held < kClusterPoints ? held : kClusterPoints;
 }
 
 CellGridWs carve_cell_grid(void* ws, int64_t n, int64_t ns, int D, int64_t batch_size,
@@ -946,7 +946,7 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
   const unsigned blocks = blocks_for(n, kThreads);
   int ranks = 0;
   if (!num_cells_in) {
-    int rc = cluster_for(g, &ranks);
+    int rc = cluster_for(D, n, B, g.max_cells, &ranks);
     if (rc) return rc;
   }
   TFGPC_REQUIRE(!n_dev || ranks > 0, "a grid of points not counted yet is too large for a cluster");

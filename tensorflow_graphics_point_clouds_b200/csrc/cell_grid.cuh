@@ -31,8 +31,9 @@ struct AlsoClear { uint32_t* p = nullptr; int64_t words = 0; };
 
 // Enqueues the build; the cell counts go to words 0 .. kReportTotal of `page`.  n_dev: the number
 // of points where an earlier kernel of the stream works it out (0, or more than g.n: no grid, as if
-// it had too many cells); only where cell_grid_takes_cluster.
-int cell_grid_takes_cluster(const tfgpc_cell_grid& g, bool* takes);
+// it had too many cells); only where g.n is cell_grid_cluster_points at most: the points of the
+// largest such grid that a cluster of this device builds, 0: none.
+int64_t cell_grid_cluster_points(int D, int64_t batch_size, int max_cells);
 int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* points,
                     const int32_t* batch_ids, const float* cell_sizes,
                     const int32_t* num_cells_in, const CellGridWs& w, int32_t* page,

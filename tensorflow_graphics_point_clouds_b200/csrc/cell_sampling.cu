@@ -1088,6 +1088,11 @@ extern "C" int tfgpc_cell_grid_sample(void* stream, const tfgpc_cell_grid* grid,
   return finish_sample(st, g, num_cells_host_out, num_samples_out);
 }
 
+extern "C" int64_t tfgpc_cell_grid_level_points(int D, int64_t batch_size, int max_cells) {
+  if (!valid_dims(D) || batch_size < 1 || batch_size >= (int64_t)INT32_MAX || max_cells < 1) return 0;
+  return cell_grid_cluster_points(D, batch_size, max_cells);
+}
+
 // With a blocking read per level the GPU waited 31 to 44 us between two levels of 10 to 80: for
 // the host to see the number of points, to make the next level's arrays and for its first launch
 // to arrive.
@@ -1110,12 +1115,8 @@ extern "C" int tfgpc_cell_grid_sample_level(
     TFGPC_REQUIRE(cell_sizes[d] > 0.0f, "SamplingOp expects positive cell sizes");
   if (ws_bytes < tfgpc_cell_grid_workspace_bytes(g.D, g.n, 0, g.batch_size, g.max_cells))
     return fail(TFGPC_ENOMEM, "SamplingOp workspace too small");
-  if (n_dev) {
-    bool takes = false;
-    rc = cell_grid_takes_cluster(g, &takes);
-    if (rc) return rc;
-    TFGPC_REQUIRE(takes, "SamplingOp: too large a level for points not counted yet");
-  }
+  TFGPC_REQUIRE(!n_dev || g.n <= cell_grid_cluster_points(g.D, g.batch_size, g.max_cells),
+                "SamplingOp: too large a level for points not counted yet");
   cudaStream_t st = (cudaStream_t)stream;
   void* page = nullptr;
   rc = report_page(&page);

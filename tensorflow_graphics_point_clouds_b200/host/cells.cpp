@@ -494,6 +494,7 @@ void bind_cells(py::module_& m) {
   m.def("fill_neighbors", &fill_neighbors);
   m.def("density", &density, py::arg("grid"), py::arg("inv_radii"), py::arg("inv_bandwidth"),
         py::arg("pdf_mode"), py::arg("mode"), py::arg("pairs") = 0.0);
+  m.def("level_points", &tfgpc_cell_grid_level_points);
   m.def("sample", &sample);
   m.def("build_and_sample", &build_and_sample);
   py::class_<SampleLevels>(m, "SampleLevels")

@@ -622,17 +622,17 @@ def sample(neighborhood, sample_mode='poisson'):
   return PointCloud(pts, bids, g._batch_size), idx
 
 
-# Points and cells up to which the grid of a level can be built for a number of points that the
-# host does not know yet, and levels of one call (tfgpc_cell_grid_sample_levels).
-_LEVELS_POINTS, _LEVELS_CELLS, _LEVELS_BOXES, _LEVELS_MOST = 65536, 1 << 21, 1024, 16
+# Levels of one call (tfgpc_cell_grid_sample_level).
+_LEVELS_MOST = 16
 _LIBRARY_BUILD_AND_SAMPLE = ops.build_cell_grid_and_sample
 
 
 class PointHierarchy:
   """PointHierarchy.py:40-98: per level Grid -> self Neighborhood -> sample.  Grid and
   sampling of a level are one library call; the levels after one follow it without a
-  blocking read of their own, as long as they have 65 536 points at most.  The
-  neighborhoods count and write their lists when they are used (the sampling needs none)."""
+  blocking read of their own, as long as one cluster can build their grids (65 536 points
+  at most).  The neighborhoods count and write their lists when they are used (the sampling
+  needs none)."""
 
   def __init__(self, point_cloud, cell_sizes, sample_mode='poisson'):
     self._point_clouds = [point_cloud]
@@ -650,12 +650,12 @@ class PointHierarchy:
   def _levels(self, pc, cell_sizes, sample_mode):
     """Several levels in one call, or None where that is not for these."""
     n, d, b = pc._points.shape[0], pc._dimension, pc._batch_size
-    if (len(cell_sizes) < 2 or n == 0 or b * d > _LEVELS_BOXES or
-        pc._num_cells_reduce is not None or
+    if (len(cell_sizes) < 2 or n == 0 or pc._num_cells_reduce is not None or
         getattr(self._level, '__func__', self._level) is not _LIBRARY_LEVEL or
         ops.build_cell_grid_and_sample is not _LIBRARY_BUILD_AND_SAMPLE or
         PointCloud is not _LIBRARY_CLOUD or PointCloud.__init__ is not _LIBRARY_CLOUD_INIT or
-        torch.as_tensor(pc._points) is not pc._points):       # (a default device moves them)
+        torch.as_tensor(pc._points) is not pc._points or      # (a default device moves them)
+        ops._lib.host().level_points(d, b, 1) == 0):
       return None
     all_sizes = [_host_dims(cs, d) for cs in cell_sizes[:_LEVELS_MOST]]
     if not all(0.0 < c < math.inf for size in all_sizes for c in size):
@@ -676,11 +676,15 @@ class PointHierarchy:
       taken = 1
       for cs, level in zip(cell_sizes[1:], all_sizes[1:]):
         # the box of a level lies in the one before: its cells are known to be no more than these
-        bound = math.ceil(max_cells * max(a / c for a, c in zip(sizes, level)) + 1.0)
-        bound = 1 << (max(1, bound) - 1).bit_length()
-        if b * float(bound) ** d > _LEVELS_CELLS:
+        bound = max_cells * max(a / c for a, c in zip(sizes, level)) + 1.0
+        if bound > _ONE_CALL_CELLS_LIMIT:
           break
-        run.add(level, bound, _to_dims(cs, d, dev, inverse=True), _LEVELS_POINTS)
+        bound = 1 << (math.ceil(bound) - 1).bit_length()
+        # (what a cluster holds depends on the device)
+        room = ops._lib.host().level_points(d, b, bound)
+        if room == 0:
+          break
+        run.add(level, bound, _to_dims(cs, d, dev, inverse=True), room)
         taken += 1
       # what does not take the numbers of samples is made while they are worked out
       cloud, levels = pc, []

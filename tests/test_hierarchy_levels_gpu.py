@@ -57,6 +57,50 @@ def test_same_as_one_level_at_a_time(n, b, d, radii, outside, mode):
       before = got
 
 
+@pytest.mark.parametrize("held", [32768, 0])
+@pytest.mark.parametrize("n", [40000, 32768, 70000])
+def test_devices_whose_clusters_hold_less(n, held, monkeypatch):
+  """A partition of a device may grant smaller clusters, or none: levels of more points than
+  they hold are refused by the entry, and such hierarchies are built as ever."""
+  host = _lib.host()
+
+  class Levels:
+    def __init__(self, *args):
+      self.run, self.n = host.SampleLevels(*args), args[0].shape[0]
+
+    def __getattr__(self, name):
+      return getattr(self.run, name)
+
+    def add(self, sizes, max_cells, inv_radii, room):
+      if min(room, self.n) > held:
+        raise _lib.TfgpcError(1, "too large a level for points not counted yet")
+      self.run.add(sizes, max_cells, inv_radii, room)
+
+  class Host:
+    SampleLevels = Levels
+
+    def __getattr__(self, name):
+      return getattr(host, name)
+
+    def level_points(self, *args):
+      return min(host.level_points(*args), held)
+
+  a = cloud(n, 2, 3, 6)
+  ref = one_by_one(a, [0.02, 0.04, 0.1], "poisson")
+  monkeypatch.setattr(_lib, "host", Host)
+  hier = pc.PointHierarchy(a, [0.02, 0.04, 0.1])
+  for got, (_, points, _) in zip(hier._point_clouds[1:], ref):
+    assert torch.equal(got._points, points._points)
+
+
+def test_points_of_a_level():
+  points = _lib.lib().tfgpc_cell_grid_level_points
+  assert points(3, _lib.c_i64(1), 128) in (32768, 65536)
+  assert points(3, _lib.c_i64(1), 129) == 0 and points(2, _lib.c_i64(1), 1 << 30) == 0
+  assert points(3, _lib.c_i64(342), 2) == 0 and points(3, _lib.c_i64(341), 2) > 0
+  assert points(7, _lib.c_i64(1), 2) == points(3, _lib.c_i64(0), 2) == points(3, _lib.c_i64(1), 0) == 0
+
+
 def test_a_replaced_level_is_called(monkeypatch):
   seen, library = [], pc.PointHierarchy._level
   monkeypatch.setattr(pc.PointHierarchy, "_level",
