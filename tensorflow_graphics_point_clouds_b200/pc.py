@@ -68,7 +68,7 @@ def _is_array(t, dtype):
   return type(t) is torch.Tensor and t.dtype is dtype and t.is_contiguous()
 
 
-_LIBRARY_FILL = ops.find_neighbors_fill
+_LIBRARY_FILL, _LIBRARY_COUNT = ops.find_neighbors_fill, ops.find_neighbors_count
 _LIBRARY_PT_GRADS = ops.compute_pdf_pt_grads
 
 
@@ -472,9 +472,11 @@ class Neighborhood:
     inv_bw = _to_dims(bandwidth, d, self._radii.device, inverse=True)
     n = g._point_cloud._points.shape[0]
     pdf_grads = torch.as_tensor(pdf_grads, dtype=torch.float32)
-    # the lists of a self neighborhood without limit are symmetric
+    # the library's lists of a self neighborhood without limit are symmetric
     pt_grads = ops.compute_pdf_pt_grads
-    if pt_grads is _LIBRARY_PT_GRADS and not (self._equal_samples and self.max_neighbors > 0):
+    if (pt_grads is _LIBRARY_PT_GRADS and not (self._equal_samples and self.max_neighbors > 0) and
+        ops.find_neighbors_fill is _LIBRARY_FILL and ops.find_neighbors_count is _LIBRARY_COUNT and
+        type(self) is Neighborhood is _LIBRARY_NEIGHBORHOOD):
       pt_grads = ops.compute_pdf_pt_grads_symmetric
     if not self._equal_samples and self._samples_are_grid_points():
       # the grid's own cloud as samples: these lists are the self neighborhood's, in the
@@ -492,6 +494,7 @@ class Neighborhood:
     return out
 
 
+_LIBRARY_NEIGHBORHOOD = Neighborhood
 LIBRARY_GET_PDF = Neighborhood.get_pdf     # (the class's own may be replaced: mcconv.PointConv)
 
 

@@ -50,3 +50,43 @@ def test_limited_lists_are_not_symmetric(monkeypatch):
   monkeypatch.setattr(ops, "compute_pdf_pt_grads", lambda *a: torch.zeros((500, 3), device=DEV))
   nb = pc.Neighborhood(grid, 0.3)
   assert not nb.pdf_point_grads(torch.rand(nb.num_pairs, device=DEV)).any() and len(seen) == 2
+
+
+@pytest.mark.parametrize("own", [True, False])
+@pytest.mark.parametrize("where", ["fill", "class"])
+def test_lists_of_ones_own_need_not_be_symmetric(where, own, monkeypatch):
+  """Lists of a replaced fill, or of a class derived from Neighborhood, are taken as they are:
+  here every pair but the ones of a point with itself leads to the first point."""
+  g = torch.Generator(device=DEV).manual_seed(11)
+  cloud = pc.PointCloud(torch.rand((300, 3), generator=g, device=DEV),
+                        torch.zeros(300, dtype=torch.int32, device=DEV), 1)
+
+  def one_way(pairs):
+    pairs = pairs.clone()
+    pairs[:, 0] = torch.where(pairs[:, 0] == pairs[:, 1], pairs[:, 0], 0)
+    return pairs
+
+  library = ops.find_neighbors_fill
+  if where == "fill":
+    def fill(*args):
+      lists = library(*args)
+      return tuple(map(one_way, lists)) if isinstance(lists, tuple) else one_way(lists)
+    monkeypatch.setattr(ops, "find_neighbors_fill", fill)
+    nb = pc.Neighborhood(pc.Grid(cloud, 0.3), 0.3, cloud if own else None)
+  else:
+    class Mine(pc.Neighborhood):
+      _neighbors = property(lambda self: one_way(pc.Neighborhood._neighbors.fget(self)))
+      _original_neigh_ids = property(
+          lambda self: one_way(pc.Neighborhood._original_neigh_ids.fget(self)))
+    nb = Mine(pc.Grid(cloud, 0.3), 0.3, cloud if own else None)
+  grads, grid = torch.randn(nb.num_pairs, generator=g, device=DEV), nb._grid
+  lists = nb._original_neigh_ids if own else nb._neighbors
+  per_point = torch.zeros(300, device=DEV).index_add_(0, lists[:, 0].long(), grads)
+  ref = ops.compute_pdf_pt_grads(cloud._points if own else grid._sorted_points, lists,
+                                 nb._samples_neigh_ranges, torch.full((3,), 5.0, device=DEV),
+                                 nb._inv_radii, per_point, 0)
+  if not own:
+    ref = torch.empty_like(ref).index_copy_(0, grid._sorted_indices.long(), ref)
+  # (float32 sums of up to 300 terms by atomics, in any order)
+  scale = ref.abs().max()
+  assert ((nb.pdf_point_grads(grads) - ref).abs() <= 300 * 6e-8 * scale).all()
