@@ -57,8 +57,8 @@ class SmallClassifier:
     for i, conv in enumerate(self.convs):
       # (the hierarchy's grid of this cloud has the layer's cells)
       grid = mcconv.layer_on_grid(conv, hier._neighborhoods[i]._grid)
-      x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], neighborhood=grid,
-                       keep_for_backward=False)
+      on = {} if grid is None else dict(neighborhood=grid)    # (a replaced forward may not know it)
+      x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], keep_for_backward=False, **on)
       if i < last:
         x = self._bn_act(x)
         x = mcconv.conv1x1(x, *self.conv1x1[i], status=status)

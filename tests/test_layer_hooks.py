@@ -4,7 +4,7 @@ import types
 
 import pytest
 
-from tensorflow_graphics_point_clouds_b200 import mcconv, pc
+from tensorflow_graphics_point_clouds_b200 import classifier, mcconv, pc
 
 
 @pytest.mark.parametrize("cls,name,own", [
@@ -92,3 +92,43 @@ def test_a_replaced_fill_is_called(own_cloud, replaced, monkeypatch):
   assert neigh._neighbors == "list"
   assert own_cloud or neigh._original_neigh_ids == "ids"
   assert bool(asked) == (replaced and not own_cloud)
+
+
+def bare_classifier(monkeypatch, layers, hierarchy):
+  """A classifier of these layers alone: everything around them passes its input on."""
+  net = object.__new__(classifier.SmallClassifier)
+  net.pool_before_head, net.bn_scale = True, 1.0
+  net.radii, net.convs = [0.1 * (i + 1) for i in range(len(layers))], layers
+  net.conv1x1, net.dense = [("w", "b")] * len(layers), [("w", "b")]
+  net._bn_act = lambda x: x
+  monkeypatch.setattr(classifier.pc, "PointCloud", lambda *args: "cloud 0")
+  monkeypatch.setattr(classifier.pc, "PointHierarchy", lambda *args: hierarchy)
+  for name in ("product_status", "check_product_status"):
+    monkeypatch.setattr(mcconv, name, lambda *args: None)
+  for name in ("conv1x1", "global_pool"):
+    monkeypatch.setattr(mcconv, name, lambda x, *args, **kw: x)
+  return net
+
+
+@pytest.mark.parametrize("where", ["object", "class"])
+def test_a_classifier_calls_replaced_layers_as_ever(where, monkeypatch):
+  """A forward of one's own need not know the parameter `neighborhood`."""
+  seen = []
+
+  def forward(features, point_cloud_in, point_cloud_out, radius, keep_for_backward=True):
+    seen.append((point_cloud_in, point_cloud_out, radius, keep_for_backward))
+    return features
+
+  layers = [object.__new__(mcconv.MCConv) for _ in range(2)]
+  if where == "object":
+    for layer in layers:
+      layer.forward = forward
+  else:
+    monkeypatch.setattr(mcconv.MCConv, "forward", lambda self, *args, **kw: forward(*args, **kw))
+  grids = [types.SimpleNamespace(_grid="grid")] * 2
+  hierarchy = types.SimpleNamespace(_point_clouds=["cloud %d" % i for i in range(3)],
+                                    _neighborhoods=grids)
+  features = types.SimpleNamespace(device="cpu")
+  net = bare_classifier(monkeypatch, layers, hierarchy)
+  assert net.forward("points", "ids", 1, features) is features
+  assert seen == [("cloud 0", "cloud 1", 0.1, False), ("cloud 1", "cloud 2", 0.2, False)]
