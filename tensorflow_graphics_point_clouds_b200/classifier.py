@@ -51,12 +51,13 @@ class SmallClassifier:
     cloud = pc.PointCloud(points, batch_ids, batch_size)
     hier = pc.PointHierarchy(cloud, self.radii, 'poisson')
     clouds = hier._point_clouds
+    grids = [neigh._grid for neigh in getattr(hier, '_neighborhoods', ())]
     x = features
     status = mcconv.product_status(x.device)
     last = len(self.convs) - 1
     for i, conv in enumerate(self.convs):
       # (the hierarchy's grid of this cloud has the layer's cells)
-      grid = mcconv.layer_on_grid(conv, hier._neighborhoods[i]._grid)
+      grid = mcconv.layer_on_grid(conv, grids[i]) if grids else None
       on = {} if grid is None else dict(neighborhood=grid)    # (a replaced forward may not know it)
       x = conv.forward(x, clouds[i], clouds[i + 1], self.radii[i], keep_for_backward=False, **on)
       if i < last:

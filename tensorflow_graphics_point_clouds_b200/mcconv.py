@@ -215,15 +215,18 @@ def _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth):
 
 class _GridOfInput:
   """In the place of a layer's neighborhood: a grid of its input cloud with cells of its
-  radius, as a hierarchy over the cloud has built it in the same pass."""
+  radius, as a hierarchy over the cloud has built it in the same pass (of another cloud or
+  with other cells it is not used)."""
 
   def __init__(self, grid):
     self.grid = grid
 
 
-def _neighborhood_on(grid, radius, point_cloud_out, bandwidth):
+def _neighborhood_on(grid, point_cloud_in, radius, point_cloud_out, bandwidth):
   from . import pc
-  return pc.grid_neighborhood_on(grid, radius, point_cloud_out, bandwidth=bandwidth)
+  if pc.is_grid_of(grid, point_cloud_in, radius):
+    return pc.grid_neighborhood_on(grid, radius, point_cloud_out, bandwidth=bandwidth)
+  return _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)
 
 
 def layer_on_grid(layer, grid):
@@ -283,7 +286,7 @@ class MCConv:
               bandwidth=0.2, keep_for_backward=True):
     neigh, packed = neighborhood, None
     if isinstance(neigh, _GridOfInput):
-      neigh = _neighborhood_on(neigh.grid, radius, point_cloud_out, bandwidth)
+      neigh = _neighborhood_on(neigh.grid, point_cloud_in, radius, point_cloud_out, bandwidth)
       packed = neigh._packed
     elif neigh is None and _is_own(self.build_neighborhood, _LIBRARY_BUILD_NEIGHBORHOOD):
       neigh = _neighborhood_with_pdf(point_cloud_in, point_cloud_out, radius, bandwidth)

@@ -575,6 +575,20 @@ def _grid_neighborhood(pc, radius, sizes, point_cloud_sample, max_neighbors, cel
   return neigh
 
 
+_LIBRARY_WITH_PDF, _LIBRARY_BUILD_WITH_PDF = grid_neighborhood_with_pdf, ops.build_cell_grid_with_pdf
+
+
+def is_grid_of(grid, point_cloud, radius):
+  """Whether grid_neighborhood_on(grid, radius, ..) is what grid_neighborhood_with_pdf gives
+  for this cloud: a grid over it with cells of this radius (wider ones would list the same
+  neighbors from more candidates, narrower ones would miss some), and nobody has replaced what
+  would be called else."""
+  return (type(grid) is Grid and grid._point_cloud is point_cloud and
+          grid._cell_sizes is _to_dims(radius, point_cloud._dimension, point_cloud._points.device) and
+          grid_neighborhood_with_pdf is _LIBRARY_WITH_PDF and
+          ops.build_cell_grid_with_pdf is _LIBRARY_BUILD_WITH_PDF)
+
+
 def grid_neighborhood_on(grid, radius, point_cloud_sample, bandwidth=0.2, mode=0):
   """grid_neighborhood_with_pdf on a grid of cells of `radius` that is there already, the
   samples another cloud's."""

@@ -177,3 +177,33 @@ def test_a_layer_on_a_grid():
   assert torch.equal(layer.forward(x, a, out, 0.1, neighborhood=given), ref)
   layer.build_neighborhood = lambda *args: None
   assert mcconv.layer_on_grid(layer, pc.Grid(a, 0.1)) is None
+
+
+@pytest.mark.parametrize("what", ["narrow cells", "wide cells", "cells per dimension",
+                                  "another cloud", "replaced"])
+def test_a_layer_is_given_a_grid_of_something_else(what, monkeypatch):
+  """A grid with other cells than the layer's radius, or of another cloud than its input, or where
+  the call that it stands for is somebody else's: the layer finds its neighbors as usual."""
+  a, b, out = cloud(2000, 2, 3, 5), cloud(2000, 2, 3, 8), cloud(600, 2, 3, 6)
+  g = torch.Generator(device=DEV).manual_seed(7)
+  r = lambda *s: torch.randn(s, generator=g, device=DEV)
+  layer = mcconv.MCConv(r(1, 3, 16), r(1, 1, 16), r(1, 128, 32), 8)
+  x = r(2000, 8)
+  ref = layer.forward(x, a, out, 0.2)
+  cells = {"narrow cells": 0.05, "wide cells": 0.4, "cells per dimension": [0.2, 0.2, 0.1]}
+  grid, seen = pc.Grid(b if what == "another cloud" else a, cells.get(what, 0.2)), []
+  library = pc.grid_neighborhood_with_pdf
+  if what == "replaced":
+    monkeypatch.setattr(pc, "grid_neighborhood_with_pdf",
+                        lambda *args, **kw: seen.append(1) or library(*args, **kw))
+  given = mcconv.layer_on_grid(layer, grid)
+  assert torch.equal(layer.forward(x, a, out, 0.2, neighborhood=given), ref)
+  assert len(seen) == (what == "replaced")
+
+
+def test_layers_of_a_classifier_work_on_its_grids(monkeypatch):
+  a = cloud(3000, 2, 3, 9)
+  hier = pc.PointHierarchy(a, [0.1, 0.2])
+  for i, radius in enumerate([0.1, 0.2]):
+    assert pc.is_grid_of(hier._neighborhoods[i]._grid, hier._point_clouds[i], radius)
+    assert not pc.is_grid_of(hier._neighborhoods[i]._grid, hier._point_clouds[i], 0.15)

@@ -111,8 +111,10 @@ def bare_classifier(monkeypatch, layers, hierarchy):
 
 
 @pytest.mark.parametrize("where", ["object", "class"])
-def test_a_classifier_calls_replaced_layers_as_ever(where, monkeypatch):
-  """A forward of one's own need not know the parameter `neighborhood`."""
+@pytest.mark.parametrize("grids", [True, False])
+def test_a_classifier_calls_replaced_layers_as_ever(grids, where, monkeypatch):
+  """A forward of one's own need not know the parameter `neighborhood`, a hierarchy of one's own
+  may have clouds alone."""
   seen = []
 
   def forward(features, point_cloud_in, point_cloud_out, radius, keep_for_backward=True):
@@ -125,9 +127,9 @@ def test_a_classifier_calls_replaced_layers_as_ever(where, monkeypatch):
       layer.forward = forward
   else:
     monkeypatch.setattr(mcconv.MCConv, "forward", lambda self, *args, **kw: forward(*args, **kw))
-  grids = [types.SimpleNamespace(_grid="grid")] * 2
-  hierarchy = types.SimpleNamespace(_point_clouds=["cloud %d" % i for i in range(3)],
-                                    _neighborhoods=grids)
+  hierarchy = types.SimpleNamespace(_point_clouds=["cloud %d" % i for i in range(3)])
+  if grids:
+    hierarchy._neighborhoods = [types.SimpleNamespace(_grid="grid")] * 2
   features = types.SimpleNamespace(device="cpu")
   net = bare_classifier(monkeypatch, layers, hierarchy)
   assert net.forward("points", "ids", 1, features) is features
