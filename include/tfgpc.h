@@ -378,6 +378,11 @@ int tfgpc_cell_grid_sample_report(void* stream, int levels, int D, int max_cells
                                   int64_t* num_samples_out,
                                   int* levels_done_out);
 
+/* The arrays of a built grid into those of another one of the same points, whose max_cells is no
+ * larger, nor smaller than the grid's cells in any dimension. */
+int tfgpc_cell_grid_copy(void* stream, const tfgpc_cell_grid* from,
+                         const tfgpc_cell_grid* to);
+
 /* ---- FindNeighbors fill pass with original ids and densities --------------
  * tfgpc_find_neighbors_fill_ordered (sample_order may be NULL) that, in the same
  * pass, also writes what pylib computes from the neighbor list afterwards:

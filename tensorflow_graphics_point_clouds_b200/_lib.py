@@ -58,6 +58,7 @@ SYMBOLS = {
     "tfgpc_cells_sample_workspace_bytes": c_sz,
     "tfgpc_cells_sample": c_int,
     "tfgpc_cell_grid_sample": c_int,
+    "tfgpc_cell_grid_copy": c_int,
     "tfgpc_cell_grid_level_points": c_i64,
     "tfgpc_cell_grid_sample_level": c_int,
     "tfgpc_cell_grid_sample_report": c_int,

@@ -907,6 +907,25 @@ int cluster_for(int D, int64_t n, int64_t batch_size, int max_cells, int* ranks)
   return rc;
 }
 
+// Arrays of words, one after the other, kCopyWords to a thread.
+constexpr int kCopies = 13, kCopyWords = 8;
+struct Copies {
+  const uint32_t* from[kCopies];
+  uint32_t* to[kCopies];
+  int64_t words[kCopies];
+  int first_block[kCopies + 1];
+};
+__global__ void __launch_bounds__(kThreads) copy_kernel(const __grid_constant__ Copies a) {
+  int i = 0;
+  while ((int)blockIdx.x >= a.first_block[i + 1]) ++i;
+  const int64_t w0 = (int64_t)((int)blockIdx.x - a.first_block[i]) * (kThreads * kCopyWords);
+#pragma unroll
+  for (int u = 0; u < kCopyWords; ++u) {
+    const int64_t w = w0 + u * kThreads + (int)threadIdx.x;
+    if (w < a.words[i]) a.to[i][w] = a.from[i][w];
+  }
+}
+
 }  // namespace
 
 int64_t cell_grid_cluster_points(int D, int64_t batch_size, int max_cells) {
@@ -993,3 +1012,37 @@ int cell_grid_build(cudaStream_t st, const tfgpc_cell_grid& g, const float* poin
 }
 
 }  // namespace tfgpc
+
+// Arrays that were made for more points than came are held for as long as the grid: a level of a
+// hierarchy whose number of points nobody knew kept up to 13 MB.  One launch of 4 to 8 us.
+extern "C" int tfgpc_cell_grid_copy(void* stream, const tfgpc_cell_grid* from,
+                                    const tfgpc_cell_grid* to) {
+  using namespace tfgpc;
+  int rc = check_cell_grid("CellGridCopy", from);
+  if (!rc) rc = check_cell_grid("CellGridCopy", to);
+  if (rc) return rc;
+  TFGPC_REQUIRE(from->D == to->D && from->n == to->n && from->batch_size == to->batch_size &&
+                to->max_cells <= from->max_cells,
+                "CellGridCopy expects grids of as many points and clouds, into no larger a table");
+  const int64_t n = to->n, D = to->D, b = to->batch_size;
+  const int64_t words[kCopies] = {b * D, b * D, D, b * D, D, 2 * n, n, 2 * n, n * D, n,
+                                  D <= 3 ? 4 * n : 0,
+                                  (int64_t)tfgpc_cell_table_elems(to->D, b, to->max_cells),
+                                  2 * b * (int64_t)to->max_cells * to->max_cells};
+  const void* const* src = (const void* const*)&from->aabb_min;
+  void* const* dst = (void* const*)&to->aabb_min;
+  Copies a;
+  int64_t blocks = 0;
+  for (int i = 0; i < kCopies; ++i) {
+    a.from[i] = (const uint32_t*)src[i];
+    a.to[i] = (uint32_t*)dst[i];
+    a.words[i] = words[i];
+    a.first_block[i] = (int)blocks;
+    blocks += (words[i] + kThreads * kCopyWords - 1) / (kThreads * kCopyWords);
+  }
+  a.first_block[kCopies] = (int)blocks;
+  ProfScope prof((cudaStream_t)stream, "grid_copy");
+  copy_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(a);
+  TFGPC_CUDA(cudaGetLastError());
+  return TFGPC_OK;
+}

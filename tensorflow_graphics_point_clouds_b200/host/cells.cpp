@@ -59,24 +59,43 @@ class CellGrid {
     g.n = pts.size(0);
   }
 
+  // Bytes of every array of a grid, in the order of the struct, and of all of them.
+  struct Bytes { size_t of[kNumFields], total; };
+  static Bytes sizes(int64_t n, int64_t d, int64_t b, int max_cells) {
+    const int64_t table = (int64_t)tfgpc_cell_table_elems((int)d, b, max_cells);
+    const int64_t elems[kNumFields] = {b * d, b * d, d, b * d, d, n, n, n, n * d, n,
+                                       d <= 3 ? 4 * n : 0, table,
+                                       2 * b * (int64_t)max_cells * max_cells};
+    Bytes s{};
+    for (int i = 0; i < kNumFields; ++i) {
+      s.of[i] = (size_t)elems[i] * (kFields[i].type == at::kLong ? 8 : 4);
+      s.total += align256(s.of[i]);
+    }
+    return s;
+  }
+
   void allocate(int64_t n, int64_t d, int64_t b, int max_cells, const Tensor& like) {
     g.D = (int)d;
     g.max_cells = max_cells;
     g.n = n;
     g.batch_size = b;
-    const int64_t table = (int64_t)tfgpc_cell_table_elems((int)d, b, max_cells);
-    const int64_t elems[kNumFields] = {b * d, b * d, d, b * d, d, n, n, n, n * d, n,
-                                       d <= 3 ? 4 * n : 0, table,
-                                       2 * b * (int64_t)max_cells * max_cells};
-    size_t offset[kNumFields], total = 0;
-    for (int i = 0; i < kNumFields; ++i) {
-      offset[i] = total;
-      total += align256((size_t)elems[i] * (kFields[i].type == at::kLong ? 8 : 4));
-    }
-    arena = bytes(total, like);
-    char* base = (char*)arena.data_ptr();
+    const Bytes s = sizes(n, d, b, max_cells);
+    arena = bytes(s.total, like);
+    char* p = (char*)arena.data_ptr();
     void** slot = (void**)&g.aabb_min;
-    for (int i = 0; i < kNumFields; ++i) slot[i] = elems[i] > 0 ? base + offset[i] : nullptr;
+    for (int i = 0; i < kNumFields; ++i) {
+      slot[i] = s.of[i] > 0 ? p : nullptr;
+      p += align256(s.of[i]);
+    }
+  }
+
+  // Moves a built grid's arrays to an allocation for no more than its points and (of `max_cells`
+  // in a dimension at most) its cells.
+  void fit(int max_cells) {
+    CellGrid own(g.n, g.D, g.batch_size, max_cells, arena);
+    check(tfgpc_cell_grid_copy(stream(), &g, &own.g));
+    g = own.g;
+    arena = own.arena;
   }
 
   const int32_t* cells_in() const { return given.empty() ? nullptr : ip(given.back()); }
@@ -379,15 +398,20 @@ class SampleLevels {
     enqueue(std::move(level), cell_sizes, inv_radii);
   }
 
-  // A level of at most `room` points.
-  void add(const std::vector<double>& cell_sizes, int max_cells, const Tensor& inv_radii,
+  // A level of at most `room` points; false if there is no memory for so many.
+  bool add(const std::vector<double>& cell_sizes, int max_cells, const Tensor& inv_radii,
            int64_t room) {
     require(levels_.size() < TFGPC_MAX_CHAINED_LEVELS, "SamplingOp: too many levels");
     const tfgpc_cell_grid& first = levels_[0].grid->g;
-    Level level;
-    level.grid = std::make_shared<CellGrid>(std::min(room, first.n), first.D, first.batch_size,
-                                            max_cells, like_);
-    enqueue(std::move(level), cell_sizes, inv_radii);
+    try {
+      Level level;
+      level.grid = std::make_shared<CellGrid>(std::min(room, first.n), first.D, first.batch_size,
+                                              max_cells, like_);
+      enqueue(std::move(level), cell_sizes, inv_radii);
+    } catch (const c10::OutOfMemoryError&) {
+      return false;
+    }
+    return true;
   }
 
   GridPtr grid(int level) const { return levels_.at(level).grid; }
@@ -402,9 +426,9 @@ class SampleLevels {
     tfgpc_cell_grid_sample_report(stream_, 1, levels_[0].grid->g.D, 1, nc, &count, &done);
   }
 
-  // [(points, batch ids, original indices or None, cells per dimension at most)] of the levels
-  // that could be built
-  py::list finish() {
+  // ([(points, batch ids, original indices or None, cells per dimension at most)] of the levels
+  // that could be built, such cells that the next one has asked for)
+  py::tuple finish() {
     const int n = (int)levels_.size(), d = levels_[0].grid->g.D;
     std::vector<int32_t> nc((size_t)n * d);
     std::vector<int64_t> counts(n);
@@ -422,15 +446,25 @@ class SampleLevels {
     py::list out;
     for (int l = 0; l < done; ++l) {
       Level& level = levels_[l];
-      level.grid->num_cells_host.assign(nc.begin() + l * d, nc.begin() + (l + 1) * d);
+      CellGrid& grid = *level.grid;
+      grid.num_cells_host.assign(nc.begin() + l * d, nc.begin() + (l + 1) * d);
+      const int cells = *std::max_element(nc.begin() + l * d, nc.begin() + (l + 1) * d);
       const Tensor pts = level.pts.narrow(0, 0, counts[l]), ids = level.ids.narrow(0, 0, counts[l]);
+      const size_t own = CellGrid::sizes(grid.g.n, d, grid.g.batch_size, cells).total;
+      if (l > 0 && (size_t)grid.arena.numel() > 2 * own + kSpareBytes) {
+        try {
+          grid.fit(cells);
+        } catch (const c10::OutOfMemoryError&) {      // (it stays where it is)
+        }
+      }
       if (l + 1 < done) levels_[l + 1].grid->set_points(pts, ids);
       out.append(py::make_tuple(pts, ids,
                                 level.idx ? py::cast(level.idx->narrow(0, 0, counts[l]))
                                           : py::object(py::none()),
-                                *std::max_element(nc.begin() + l * d, nc.begin() + (l + 1) * d)));
+                                cells));
     }
-    return out;
+    const auto next = nc.begin() + done * d;
+    return py::make_tuple(out, done < n ? *std::max_element(next, next + d) : 0);
   }
 
  private:
@@ -439,6 +473,9 @@ class SampleLevels {
     Tensor radii, pts, ids;
     OptTensor idx;
   };
+
+  // A grid whose arrays are larger than twice its size and this gets ones of its size.
+  static constexpr size_t kSpareBytes = 1 << 20;
 
   void enqueue(Level&& level, const std::vector<double>& cell_sizes, const Tensor& inv_radii) {
     const CellGrid& grid = *level.grid;

@@ -11,7 +11,9 @@ arithmetic around the ops is float32 torch code that follows the TensorFlow
 expressions of the reference one to one, and the ops themselves run through
 `custom_ops` (the C ABI).
 """
+import itertools
 import math
+import operator
 
 import torch
 
@@ -641,7 +643,31 @@ def sample(neighborhood, sample_mode='poisson'):
 
 # Levels of one call (tfgpc_cell_grid_sample_level).
 _LEVELS_MOST = 16
+# Per kind of hierarchy (device, dimension, batch size, bits of the number of points, mode, cell
+# sizes): [the most points and the most cells in a dimension (0: not known) that its levels behind
+# the first have had, one after the other; the first one's bound of cells; (bound of cells, points)
+# that the next such levels are made for].  Without, for as many points as a cluster holds.
+_LEVEL_SIZES = {}
 _LIBRARY_BUILD_AND_SAMPLE = ops.build_cell_grid_and_sample
+
+
+def _level_rooms(host, batch_size, all_sizes, max_cells, seen):
+  """[(bound of cells, points)] that the levels behind the first are made for, as far as they can
+  follow it.  max_cells: the first one's bound; seen: see _LEVEL_SIZES."""
+  rooms, first, d = [], all_sizes[0], len(all_sizes[0])
+  seen = list(seen) + [0, 0] * len(all_sizes)
+  for level, points, cells in zip(all_sizes[1:], seen[::2], seen[1::2]):
+    # the box of a level lies in the one before: its cells are known to be no more than these
+    bound = max_cells * max(a / c for a, c in zip(first, level)) + 1.0
+    if bound > _ONE_CALL_CELLS_LIMIT:
+      break
+    bound = 1 << ((min(math.ceil(bound), cells) if cells else math.ceil(bound)) - 1).bit_length()
+    room = host.level_points(d, batch_size, bound)      # (what a cluster holds: by the device)
+    if room == 0 or points > room:
+      break
+    # (some more than there have been: they vary)
+    rooms.append((bound, min(room, 1 << (points + points // 4).bit_length()) if points else room))
+  return rooms
 
 
 class PointHierarchy:
@@ -671,18 +697,21 @@ class PointHierarchy:
         getattr(self._level, '__func__', self._level) is not _LIBRARY_LEVEL or
         ops.build_cell_grid_and_sample is not _LIBRARY_BUILD_AND_SAMPLE or
         PointCloud is not _LIBRARY_CLOUD or PointCloud.__init__ is not _LIBRARY_CLOUD_INIT or
-        torch.as_tensor(pc._points) is not pc._points or      # (a default device moves them)
-        ops._lib.host().level_points(d, b, 1) == 0):
+        torch.as_tensor(pc._points) is not pc._points):       # (a default device moves them)
       return None
     all_sizes = [_host_dims(cs, d) for cs in cell_sizes[:_LEVELS_MOST]]
-    if not all(0.0 < c < math.inf for size in all_sizes for c in size):
-      return None
-    dev = pc._points.device
+    dev, host = pc._points.device, ops._lib.host()
     mode = SAMPLE_MODES[sample_mode.lower()]
+    kind = dev, d, b, n.bit_length(), mode, tuple(map(tuple, all_sizes))
+    known = _LEVEL_SIZES.get(kind)
+    if known is None and (host.level_points(d, b, 1) == 0 or
+                          not all(0.0 < c < math.inf for size in all_sizes for c in size)):
+      return None
+    seen, first, rooms = known or ((), 0, ())
 
     def build(points, batch_ids, batch_size, sizes, max_cells):
-      run = ops._lib.host().SampleLevels(points, batch_ids, batch_size, sizes, max_cells, mode,
-                                         _to_dims(cell_sizes[0], d, dev, inverse=True))
+      run = host.SampleLevels(points, batch_ids, batch_size, sizes, max_cells, mode,
+                              _to_dims(cell_sizes[0], d, dev, inverse=True))
       try:
         return further_levels(run, points, sizes, max_cells)
       except BaseException:
@@ -690,18 +719,12 @@ class PointHierarchy:
         raise
 
     def further_levels(run, points, sizes, max_cells):
+      made = rooms if max_cells == first else _level_rooms(host, b, all_sizes, max_cells, seen)
       taken = 1
-      for cs, level in zip(cell_sizes[1:], all_sizes[1:]):
-        # the box of a level lies in the one before: its cells are known to be no more than these
-        bound = max_cells * max(a / c for a, c in zip(sizes, level)) + 1.0
-        if bound > _ONE_CALL_CELLS_LIMIT:
+      for bound, room in made:
+        if not run.add(all_sizes[taken], bound, _to_dims(cell_sizes[taken], d, dev, inverse=True),
+                       room):
           break
-        bound = 1 << (math.ceil(bound) - 1).bit_length()
-        # (what a cluster holds depends on the device)
-        room = ops._lib.host().level_points(d, b, bound)
-        if room == 0:
-          break
-        run.add(level, bound, _to_dims(cs, d, dev, inverse=True), room)
         taken += 1
       # what does not take the numbers of samples is made while they are worked out
       cloud, levels = pc, []
@@ -715,22 +738,36 @@ class PointHierarchy:
         cloud._points, cloud._batch_size, cloud._dimension = points, b, d
         cloud._num_cells_reduce = cloud._aabb = None
         levels.append((neigh, cloud))
-      built = run.finish()
-      return levels[0][0]._grid._cells, levels, built
+      built, asked = run.finish()
+      return levels[0][0]._grid._cells, levels, built, asked, max_cells, made[:taken - 1]
 
     built = _cell_grid(pc, all_sizes[0], build)
     if built is None:
       return None
-    done = []
-    for (neigh, cloud), (points, batch_ids, idx, cells) in zip(built[1], built[2]):
+    _, levels, built, asked, max_cells, made = built
+    done, now = [], []
+    for (neigh, cloud), (points, batch_ids, idx, cells) in zip(levels, built):
       if done:              # (what a grid of this cloud asks for, as _cell_grid keeps it)
         bound = max(_FIRST_BOUND, 1 << (cells - 1).bit_length())
         key = _bound_key(neigh._grid._point_cloud, neigh._grid._sizes)
         for known in (key, key[:3]):
           if _MAX_CELLS.get(known) != bound:
             _remember(_MAX_CELLS, known, bound)
+        now += held, cells
       cloud._points, cloud._batch_ids = points, batch_ids
+      held = points.shape[0]
       done.append((neigh, cloud, idx))
+    missed = len(done) <= len(made)
+    if missed:
+      # the next level got more points or cells than there was room for, those behind it may too
+      now += held, asked if held <= made[len(done) - 1][1] else 0
+      seen = seen[:len(now) - 1]
+    else:
+      now += held, 0
+    if missed or max_cells != first or len(now) > len(seen) or any(map(operator.gt, now, seen)):
+      seen = [max(x) for x in itertools.zip_longest(seen, now, fillvalue=0)]
+      _remember(_LEVEL_SIZES, kind, [seen, max_cells,
+                                     _level_rooms(host, b, all_sizes, max_cells, seen)])
     return done
 
   @staticmethod

@@ -74,7 +74,7 @@ def test_devices_whose_clusters_hold_less(n, held, monkeypatch):
     def add(self, sizes, max_cells, inv_radii, room):
       if min(room, self.n) > held:
         raise _lib.TfgpcError(1, "too large a level for points not counted yet")
-      self.run.add(sizes, max_cells, inv_radii, room)
+      return self.run.add(sizes, max_cells, inv_radii, room)
 
   class Host:
     SampleLevels = Levels
@@ -88,9 +88,104 @@ def test_devices_whose_clusters_hold_less(n, held, monkeypatch):
   a = cloud(n, 2, 3, 6)
   ref = one_by_one(a, [0.02, 0.04, 0.1], "poisson")
   monkeypatch.setattr(_lib, "host", Host)
+  monkeypatch.setattr(pc, "_LEVEL_SIZES", {})
   hier = pc.PointHierarchy(a, [0.02, 0.04, 0.1])
   for got, (_, points, _) in zip(hier._point_clouds[1:], ref):
     assert torch.equal(got._points, points._points)
+
+
+def host_with(add):
+  """The host layer with add(run, ..) in the place of SampleLevels.add."""
+  host = _lib.host()
+
+  class Levels:
+    def __init__(self, *args):
+      self.run = host.SampleLevels(*args)
+
+    def __getattr__(self, name):
+      return getattr(self.run, name)
+
+    def add(self, *args):
+      return add(self.run, *args)
+
+  class Host:
+    SampleLevels = Levels
+
+    def __getattr__(self, name):
+      return getattr(host, name)
+
+  return Host
+
+
+def same_levels(hier, ref):
+  assert len(hier._point_clouds) == len(ref) + 1
+  for got, neigh, (n, points, _) in zip(hier._point_clouds[1:], hier._neighborhoods, ref):
+    assert torch.equal(got._points, points._points)
+    for name in ("_sorted_indices", "_sorted_points", "_cur_keys"):
+      assert torch.equal(getattr(neigh._grid, name), getattr(n._grid, name))
+    assert torch.equal(neigh._neighbors, n._neighbors)
+
+
+@pytest.mark.parametrize("n,b,d,radii", [(65000, 4, 3, [0.05, 0.1, 0.2, 0.4]),
+                                         (100000, 8, 3, [0.03, 0.06, 0.12, 0.24]),
+                                         (60000, 1, 2, [0.004, 0.3, 0.4])])
+@pytest.mark.parametrize("mode", ["poisson", "average"])
+def test_memory_that_a_hierarchy_keeps(n, b, d, radii, mode, monkeypatch):
+  """Arrays of levels whose size was not known when they were made are as large as their content,
+  and no larger than twice that once such levels have been seen."""
+  a = cloud(n, b, d, 12)
+  pc.PointHierarchy(a, radii, mode)
+  monkeypatch.setattr(pc, "_LEVEL_SIZES", {})
+
+  def kept(build):
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    held = build()
+    return torch.cuda.memory_allocated() - before, held
+
+  one_by_one(a, radii, mode)
+  own, ref = kept(lambda: one_by_one(a, radii, mode))
+  for call in range(3):
+    used, hier = kept(lambda: pc.PointHierarchy(a, radii, mode))
+    assert used <= 1.3 * own + 3 * (1 << 20)
+    same_levels(hier, ref)
+
+
+@pytest.mark.parametrize("mode", ["poisson", "average"])
+def test_levels_known_to_be_too_large_are_not_asked_for(mode, monkeypatch):
+  a, radii, asked = cloud(100000, 1, 3, 13), [0.008, 0.01, 0.03], []
+  ref = one_by_one(a, radii, mode)
+  monkeypatch.setattr(_lib, "host", host_with(lambda run, *args: asked.append(1) or run.add(*args)))
+  monkeypatch.setattr(pc, "_LEVEL_SIZES", {})
+  same_levels(pc.PointHierarchy(a, radii, mode), ref)
+  assert asked
+  del asked[:]
+  same_levels(pc.PointHierarchy(a, radii, mode), ref)
+  assert not asked
+
+
+def test_levels_larger_than_the_ones_before(monkeypatch):
+  """Levels that do not fit what their kind has needed so far are built all the same, and the next
+  one's fit; so are those that there is no memory for."""
+  small, large = cloud(40000, 2, 3, 14), cloud(40000, 2, 3, 14)
+  small._points *= 0.2
+  radii = [0.02, 0.04, 0.08]
+  ref = one_by_one(large, radii, "poisson")
+  monkeypatch.setattr(pc, "_LEVEL_SIZES", {})
+  pc.PointHierarchy(small, radii)
+  (kind, (seen, _, _)), = pc._LEVEL_SIZES.items()
+  for _ in range(2):
+    same_levels(pc.PointHierarchy(large, radii), ref)
+  now, first, rooms = pc._LEVEL_SIZES[kind]
+  assert len(now) == len(seen) == 6 and all(x > y for x, y in zip(now[::2], seen[::2]))
+  assert all(x >= y > 0 for x, y in zip(now[1:4:2], seen[1::2])) and len(rooms) == 2
+  pc._LEVEL_SIZES[kind] = [[points * (i % 2 == 0) + 2 * (i % 2) for i, points in enumerate(now)],
+                           first, [(2, room) for _, room in rooms]]                # too few cells
+  for _ in range(2):
+    same_levels(pc.PointHierarchy(large, radii), ref)
+  assert pc._LEVEL_SIZES[kind] == [now, first, rooms]
+  monkeypatch.setattr(_lib, "host", host_with(lambda run, *args: False))           # no memory
+  same_levels(pc.PointHierarchy(large, radii), ref)
 
 
 def test_points_of_a_level():
