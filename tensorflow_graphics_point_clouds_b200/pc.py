@@ -742,7 +742,10 @@ class PointHierarchy:
       return levels[0][0]._grid._cells, levels, built, asked, max_cells, made[:taken - 1]
 
     built = _cell_grid(pc, all_sizes[0], build)
-    if built is None:
+    if built is None:       # (_level looks at the same grid again: one try between them)
+      fine = _TOO_FINE.get(_bound_key(pc, all_sizes[0]))
+      if fine is not None:
+        fine[0] += 1
       return None
     _, levels, built, asked, max_cells, made = built
     done, now = [], []

@@ -188,6 +188,33 @@ def test_levels_larger_than_the_ones_before(monkeypatch):
   same_levels(pc.PointHierarchy(large, radii), ref)
 
 
+def test_grids_that_are_too_fine_are_tried_as_often(monkeypatch):
+  """A grid whose table would be too large is tried once in 17 hierarchies, by whichever way the
+  level is built."""
+  a, tried = cloud(3000, 64, 3, 15), []
+  host = _lib.host()
+
+  def levels(*args):
+    tried.append(args[4])
+    return host.SampleLevels(*args)
+
+  class Host:
+    SampleLevels = staticmethod(levels)
+
+    def __getattr__(self, name):
+      return getattr(host, name)
+
+  monkeypatch.setattr(_lib, "host", Host)
+  for name in ("_TOO_FINE", "_MAX_CELLS", "_LEVEL_SIZES"):
+    monkeypatch.setattr(pc, name, {}, raising=False)
+  for call in range(18):
+    del tried[:]
+    hier = pc.PointHierarchy(a, [0.002, 0.2])
+    assert len(hier._point_clouds) == 3 and hier._neighborhoods[0]._grid._cells is None
+    # (the second level is one of its own: no SampleLevels for it)
+    assert bool(tried) == (call in (0, 17)), call
+
+
 def test_points_of_a_level():
   points = _lib.lib().tfgpc_cell_grid_level_points
   assert points(3, _lib.c_i64(1), 128) in (32768, 65536)
