@@ -617,10 +617,7 @@ settle_kernel(SampleArgs a) {
           const int j = point(q);
           const unsigned long long bit = 1ull << (j & 31);
           atomicOr(a.settled + (j >> 5), any_blocked ? bit << 32 : bit << 32 | bit);
-          if (!any_blocked) {
-            __stcg(a.state + j, (uint8_t)2);
-            atomicAdd(a.block_total + j / per, 1);
-          }
+          if (!any_blocked) atomicAdd(a.block_total + j / per, 1);
         }
       }
     }
@@ -658,16 +655,7 @@ cells_sample_kernel(SampleArgs a) {
       a.state[i < lead ? i : tail + (i - lead)] = 2;
     if (threadIdx.x == 0) num_crowded[0] = 0;
     __syncthreads();
-    if (a.settled) {
-      settled = a.arrived[4] == 0u;
-      if (!settled) {          // all states as before that kernel
-        for (int64_t i = lead + (int64_t)blockIdx.x * kThreads + threadIdx.x; i < tail;
-             i += (int64_t)blocks * kThreads)
-          a.state[i] = 0;
-        ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
-                          a.period_ns) && ok;
-      }
-    }
+    settled = a.settled != nullptr && a.arrived[4] == 0u;
     const Team team = settled ? Team{0, 0, 0} : team_of(a.c, n, blocks, total);
     const int warps = team.size * kWarps;
     // neighboring cells go to different blocks: crowded ones come side by side
@@ -732,10 +720,10 @@ cells_sample_kernel(SampleArgs a) {
         poisson_crowded_cell<D>(a, block_cell, cell, batch, begin, end, nc, total, inv_r);
       }
       if (pass + 1 == (1 << D)) break;     // (the compaction begins with a barrier)
-      ok = grid_barrier(counter, (pass + 1 + (team.cloud < 0 ? barriers : 0)) * team.size, a.arrived + 1, a.arrived + 2,
+      ok = grid_barrier(counter, (pass + 1) * team.size, a.arrived + 1, a.arrived + 2,
                         a.period_ns) && ok;
     }
-    if (team.cloud < 0) barriers += (1 << D) - 1;
+    if (team.cloud < 0) barriers = (1 << D) - 1;
     if (!settled)
       ok = grid_barrier(a.arrived, ++barriers * blocks, a.arrived + 1, a.arrived + 2,
                         a.period_ns) && ok;
@@ -745,6 +733,7 @@ cells_sample_kernel(SampleArgs a) {
   const int64_t first = min((int64_t)blockIdx.x * per, n), last = min(first + per, n);
   auto chosen = [&](int64_t i) {
     if (i >= last) return false;
+    if (settled) return (__ldcg((const unsigned*)(a.settled + (i >> 5))) >> (i & 31) & 1u) != 0u;
     return a.mode == 0 ? __ldcg(a.state + i) == 2
                        : i == 0 || __ldg(a.keys + i) != __ldg(a.keys + i - 1);
   };
