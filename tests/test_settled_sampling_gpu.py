@@ -134,3 +134,24 @@ def test_cells_too_full_are_left_to_the_passes_at_once(n, b):
     return sorted(times)[4]
   # (a search through such cells took 1.7 to 3 times as long as the passes, but at 300 points)
   assert us(0) <= 1.3 * us(4) + 20.0
+
+
+# cells of up to three radii: more than 96 points (a block works on them), more than 32 of them taken
+# (marked in between), more than 1024 (several rounds of the block's registers)
+@pytest.mark.parametrize("n,b,d,cell,radius", [
+    (6000, 1, 4, 0.6, 0.2), (9000, 2, 4, 0.5, 0.17), (5000, 1, 5, 0.75, 0.3),
+    (20000, 1, 3, 0.5, 0.167), (5000, 1, 3, 0.5, 0.167), (4000, 1, 2, 0.45, 0.151)])
+def test_crowded_cells_of_many_samples(n, b, d, cell, radius):
+  rng = np.random.default_rng(n + d)
+  pts = rng.uniform(0, 1, (n, d)).astype(np.float32)
+  ids = np.sort(rng.integers(0, b, n)).astype(np.int32)
+  grid = pr.Grid(pts, ids, b, cell)
+  _, _, ref = pr.sample(pr.Neighborhood(grid, radius), 0)
+  keys, held = np.unique(grid.keys, return_counts=True)
+  taken = np.array([(grid.keys[ref] == k).sum() for k in keys])
+  assert d < 4 or (taken[held > 96] > 32).any()
+  neigh = pc.Neighborhood(pc.Grid(pc.PointCloud(torch.from_numpy(pts).to(DEV),
+                                                torch.from_numpy(ids).to(DEV), b), cell), radius)
+  for _ in range(2):
+    cloud, idx = pc.sample(neigh, "poisson")
+    assert np.array_equal(idx.cpu().numpy(), ref)
