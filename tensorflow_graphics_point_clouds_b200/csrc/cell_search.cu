@@ -549,13 +549,8 @@ density_of_sums_kernel(WalkArgs a, const unsigned long long* sums) {
     worst += f.hi * 0.0f + f.lo * 0.0f;
     norm *= bw * 0.3989422804014327;
   }
-  float p[D];
-  int index;
-  load_point<D>(a.c, v, p, &index);
-  const float density = (float)((double)ld_global(sums + v) * norm) + worst;
-  const int64_t row = a.src.mode == 1 ? index : v;
-  a.density[row] = density;
-  if (D == 3 && a.packed) a.packed[row] = make_float4(p[0], p[1], p[D - 1], 1.0f / density);
+  const int64_t row = a.src.mode == 1 ? ld_global(a.c.indices + v) : v;
+  a.density[row] = (float)((double)ld_global(sums + v) * norm) + worst;
 }
 
 // Samples per warp: more of them share the candidates of a cell (a cell of a uniform
@@ -666,7 +661,7 @@ struct DensityRequest {
   float4* packed;
 };
 
-// sums: [n] zeros, for the densities of the grid's own points, or null.
+// sums: [n] zeros, for the densities of the grid's own points (without a packed table), or null.
 int enqueue_density(cudaStream_t st, const tfgpc_cell_grid& g, const SampleSource& src, int64_t ns,
                     const float* inv_radii, const DensityRequest& d, unsigned long long* sums) {
   WalkArgs a = walk_args(g, src, ns, inv_radii, 0);
