@@ -27,8 +27,9 @@ constexpr int kMaxBlocks = 1024;
 constexpr int kMaxTeams = kMaxBlocks / 2;
 // Cells of more points than this are left to the end of a block's pass, for all its
 // warps together: one warp with a cell of a thousand points, and a few thousand to
-// mark, keeps its whole team waiting (8 x 100 000 Gaussian-mixture points, four levels:
-// 427 -> 385 us in this kernel).
+// mark, keeps its whole team waiting.  us of this kernel at 48, 96, 160, 256 and 512: first of four
+// levels of 8 x 100 000 Gaussian-mixture points 201, 203, 209, 210, 251; 70 000 points in 400
+// clumps 73, 63, 61, 61, 61; 400 000 in 40 clumps 182, 229, 238, 254, 336; no cell that full: the same.
 constexpr int kCrowded = 96;
 constexpr int kMaxCrowded = 128;
 constexpr int kHeadWords = 8;             // before the teams' counters
@@ -290,8 +291,9 @@ struct BlockCell {
 // The selection in a crowded cell by a whole block: its points stand in registers, kHeld per thread
 // at a time, and a turn takes the first that is open and closes its neighbors, all at once.  A cell
 // is then as many turns of one barrier as it has points to take, a dozen mostly, where a warp went
-// through its points 32 at a time (and the block's others with it, to share the marks): first of four levels of
-// 8 x 100 000 Gaussian-mixture points 217 -> 207 us, first of three of 60 000 102 -> 98.
+// through its points 32 at a time (and the block's others with it, to share the marks): first of
+// four levels of 8 x 100 000 Gaussian-mixture points 217 -> 207 us, first of three of 60 000
+// 102 -> 98; cells of three radii, with dozens to take, 363 -> 376.
 template <int D>
 __device__ __forceinline__ void poisson_crowded_cell(const SampleArgs& a, BlockCell<D>& s,
                                                      const int* cell, int batch, int begin,
@@ -448,16 +450,19 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int64_t n, int block
 // those neighbors, as words of 32 points and masks; then they look at the words until one of the
 // neighbors is taken, or all are settled and none is.  All blocks are resident (a cooperative
 // launch), and a point waits for earlier ones only.  What is taken is counted for the block that
-// will write it (cells_sample_kernel, which follows and has nothing to wait for).  The chain of a level is a
-// search and some twenty trips to L2, where the passes have ten barriers and a walk per cell between
-// them: levels of 54 000, 10 600 and 2000 points take 81, 57 and 48 us by passes, 46, 23 and 21 so.
+// will write it (cells_sample_kernel, which follows and has nothing to wait for).  The chain of a
+// level is a search and some twenty trips to L2, where the passes have ten barriers and a walk per
+// cell between them: levels of 54 000, 10 600 and 2000 points take 81, 57 and 48 us by passes, 46,
+// 23 and 21 so.
 // Where cells are crowded the passes, which test around taken points only, are the faster ones.  A
 // block finds that out from its first points' cells and their own, before it tests any of them, or
 // from a list that is too full; a point of too full a cell is not searched for either.  Then nothing
 // of this counts (three levels from 60 000 points with 282 earlier candidates each: 1110 us without
 // that, 265 with it, 330 by passes and a read per level.  20 000 points in one cell, this kernel and
 // the passes, without a look at a point's own cell 408 + 43 us, with it 4 + 43; in eight clouds of
-// a cell each 190 + 31 and 4 + 31).
+// a cell each 190 + 31 and 4 + 31).  What a trial in vain costs the passes: 5 us where every block
+// sees it at once, 15 to 27 where few do or a list runs over (20 000 points in 40 clumps 21 + 61 us,
+// by passes alone 60).
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 settle_kernel(SampleArgs a) {
@@ -933,7 +938,7 @@ __global__ void barrier_probe_kernel(unsigned* words, int late_block, int late_a
   if (!ok) atomicAdd(words + 5, 1u);
 }
 
-// Barrier words, a byte of state per point, of a level that settle_points is tried on two bits, and
+// Barrier words, a byte of state per point, of a level that settle_kernel is tried on two bits, and
 // the blocks' totals.
 size_t settled_at(int64_t n) { return align_up((size_t)n + kHeadBytes, 8); }
 size_t totals_at(int64_t n) {

@@ -609,10 +609,10 @@ def grid_neighborhood_on(grid, radius, point_cloud_sample, bandwidth=0.2, mode=0
 
 # Cells up to this many radii wide are sampled from the grid, wider ones from a neighbor
 # list: a cell's taken points are marked around by one block, (taken) x (candidates) tests,
-# and a wide cell holds many of both.  From the grid / by lists, us, at 1, 3, 4, 6 and 8 radii:
-# 100 000 points 89/247, 363/1121, 1295/2134, 6364/5647, 16914/9854 (40 neighbors a point),
-# 106/286, 228/403, 717/622, 1453/1489, 5846/2980 (6); 20 000 points 79/204, 211/251,
-# 640/346, 1107/705, 2397/1340 (6).
+# and a wide cell holds many of both (and is a turn of the block per taken point).  From the grid /
+# by lists, us, at 1, 3, 4, 6 and 8 radii: 100 000 points 96/260, 376/1141, 1251/2158, 6240/5650,
+# 17115/10160 (40 neighbors a point), 106/279, 230/386, 723/630, 1803/1507, 6490/3040 (6);
+# 20 000 points 54/202, 234/260, 680/367, 1244/748, 2633/1375 (6).
 _SAMPLED_CELLS = 3.0
 
 
