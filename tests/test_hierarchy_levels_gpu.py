@@ -188,6 +188,36 @@ def test_levels_larger_than_the_ones_before(monkeypatch):
   same_levels(pc.PointHierarchy(large, radii), ref)
 
 
+@pytest.mark.parametrize("unit", [0.25, 3.0, 1.0 / 128])
+@pytest.mark.parametrize("mode", ["poisson", "average"])
+def test_the_same_scene_in_another_unit(mode, unit, monkeypatch):
+  """Levels of a scene that has been seen in another unit of length are made for what it needed
+  there (and cell sizes that are no numbers are like no others)."""
+  a, rooms = cloud(40000, 2, 3, 16), []
+  radii = [0.02, 0.04, 0.08]
+  small = cloud(40000, 2, 3, 16)
+  small._points *= unit
+  ref = one_by_one(small, [r * unit for r in radii], mode)
+
+  def add(run, sizes, max_cells, inv_radii, room):
+    rooms.append((max_cells, room))
+    return run.add(sizes, max_cells, inv_radii, room)
+
+  monkeypatch.setattr(_lib, "host", host_with(add))
+  monkeypatch.setattr(pc, "_LEVEL_SIZES", {})
+  for _ in range(2):
+    del rooms[:]
+    pc.PointHierarchy(a, radii, mode)
+  first = list(rooms)
+  del rooms[:]
+  same_levels(pc.PointHierarchy(small, [r * unit for r in radii], mode), ref)
+  assert rooms == first and len(pc._LEVEL_SIZES) == 2
+  (kind, _), _ = pc._LEVEL_SIZES.items()
+  for no_number in (0.0, float("nan"), float("inf"), -1.0):
+    sizes = tuple(tuple(c * no_number for c in size) for size in kind[-1])
+    assert pc._same_in_another_unit(kind[:-1] + (sizes,)) is None
+
+
 def test_grids_that_are_too_fine_are_tried_as_often(monkeypatch):
   """A grid whose table would be too large is tried once in 17 hierarchies, by whichever way the
   level is built."""
