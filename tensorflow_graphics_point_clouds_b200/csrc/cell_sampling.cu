@@ -39,7 +39,20 @@ constexpr int64_t kFlowPoints = 65536;
 constexpr int kFlowPer = 128;             // points of a block
 constexpr int kFlowLists = 32;            // words of neighbors of a point
 constexpr int kFlowCell = 256;            // points of a cell
-constexpr int kFlowWork = 448;            // candidates of a point x points of eight lanes
+// Candidates (points of earlier passes in the cells around a point, and before it in its own) that a
+// level has on average, times the points of eight lanes, above which its passes are the faster
+// ones.  Settling takes as long as its tests, the passes about as long with few candidates as with
+// many.  us of a hierarchy of one level of four clouds, settled / by passes: 30 000 points in all (two
+// per eight lanes) with 101, 188 and 268 candidates 93/95, 106/103 and 116/110, 60 000 (four) with 55,
+// 106 and 202 107/106, 131/107 and 155/111; in two dimensions 15 000 with 149 and 296 71/69 and 80/75,
+// 60 000 with 28 and 55 90/95 and 98/86; in four 30 000 with 184 129/175, 60 000 with 203 189/190.
+// With more than kFlowMost candidates some lists run over: 15 000 points with 332 and 467 100/105
+// and 199/123.  Not so in levels of kFlowFew points, whose blocks each decide: 2000 points with 249
+// 80/103.
+constexpr int kFlowMost = 256, kFlowFew = 2048;
+__host__ __device__ constexpr int flow_work(int D) {
+  return D == 2 ? 160 : D == 3 ? 320 : 768 << (D - 4);
+}
 // Candidates of a mark loop between two signs of progress: well under a millisecond, and
 // none at all in cells of ordinary size.  A selection shows none (its loop has no register
 // left for it: spills, 1 % of a hierarchy); one over all points of a call takes some 30 ns
@@ -445,6 +458,28 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int64_t n, int block
   return Team{0, 0, 0};
 }
 
+// Candidates of point i by sample: those before it in its cell, and as many times as there are halves
+// those of one of them; very many where its cell is too full.  Over a block's threads, with points
+// from all over the level, the mean is 12 % off (rms over 200 levels; at most 36 %).  (A call: as a
+// part of settle_kernel it slows the search down by a third.)
+template <int D>
+__device__ __noinline__ int sampled_candidates(int i, const int64_t* keys, const int32_t* start,
+                                               const int32_t* num_cells, int total) {
+  constexpr int kHalves = 2 * num_tubes<D>();
+  const int64_t key = __ldg(keys + i);
+  if (key < 0 || key >= total) return 0;
+  int cell[D], nc[D], rem = (int)key;
+#pragma unroll
+  for (int d = D - 1; d >= 0; --d) {
+    nc[d] = __ldg(num_cells + d);
+    cell[d] = rem % nc[d];
+    rem /= nc[d];
+  }
+  const int2 x = earlier_points<D>(threadIdx.x * 37 % kHalves, cell, rem, nc, total, start);
+  const int begin = __ldg(start + (total - (int)key)), end = __ldg(start + (total - (int)key) + 1);
+  return end - begin > kFlowCell ? 1 << 20 : min(i - begin + kHalves * (x.y - x.x), 1 << 20);
+}
+
 // The selection without passes: a point is settled as soon as its earlier neighbors (of earlier
 // passes, or before it in its cell) are, not when all cells of their passes are.  Eight lanes find
 // those neighbors, as words of 32 points and masks; then they look at the words until one of the
@@ -454,15 +489,15 @@ __device__ __forceinline__ Team team_of(const CellsView& c, int64_t n, int block
 // level is a search and some twenty trips to L2, where the passes have ten barriers and a walk per
 // cell between them: levels of 54 000, 10 600 and 2000 points take 81, 57 and 48 us by passes, 46,
 // 23 and 21 so.
-// Where cells are crowded the passes, which test around taken points only, are the faster ones.  A
-// block finds that out from its first points' cells and their own, before it tests any of them, or
-// from a list that is too full; a point of too full a cell is not searched for either.  Then nothing
-// of this counts (three levels from 60 000 points with 282 earlier candidates each: 1110 us without
-// that, 265 with it, 330 by passes and a read per level.  20 000 points in one cell, this kernel and
-// the passes, without a look at a point's own cell 408 + 43 us, with it 4 + 43; in eight clouds of
-// a cell each 190 + 31 and 4 + 31).  What a trial in vain costs the passes: 5 us where every block
-// sees it at once, 15 to 27 where few do or a list runs over (20 000 points in 40 clumps 21 + 61 us,
-// by passes alone 60).
+// Where cells are crowded the passes, which test around taken points only, are the faster ones.  All
+// blocks of a level of more than kFlowFew points find that out from the same points, before they
+// test any: 1.2 us of a settled level, 6 in all of one that is left.  (When each went by its own points,
+// and few found it out, the others tested in vain for 16 to 43 us: levels of 30 000 and 60 000 points
+// with 100 to 270 candidates took 130 to 157 us, now 114 to 121, by passes alone 103 to 111.)  A block
+// with far more candidates than that, a list that runs over and a cell that is too full leave the
+// level to the passes as well, and a point of too full a cell is not searched for.  Then nothing of
+// this counts (20 000 points in one cell, this kernel and the passes, without a look at a point's
+// own cell 408 + 43 us, with it 4 + 43; in eight clouds of a cell each 190 + 31 and 4 + 31).
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 settle_kernel(SampleArgs a) {
@@ -470,7 +505,7 @@ settle_kernel(SampleArgs a) {
   constexpr int kHalves = 2 * num_tubes<D>();
   constexpr int kMine = D <= 3 ? (kHalves + 7) / 8 : 1;       // halves of a lane looked up at once
   __shared__ uint2 lists[kFlowPer][kFlowLists];
-  __shared__ int listed[kFlowPer], candidates_s;
+  __shared__ int listed[kFlowPer], candidates_s, sampled_s;
   const int lane = lane_id(), eighth = lane & 7, group = threadIdx.x >> 3;
   int nc[D];
   float inv_r[D];
@@ -498,8 +533,14 @@ settle_kernel(SampleArgs a) {
   // decides.
   auto point = [&](int q) { return ((int)blockIdx.x + (q >> 2) * blocks) * 4 + (q & 3); };
   for (int i = threadIdx.x; i < kFlowPer; i += kThreads) listed[i] = 0;
-  if (threadIdx.x == 0) candidates_s = 0;
+  if (threadIdx.x == 0) candidates_s = sampled_s = 0;
   __syncthreads();
+  if (n > kFlowFew) {
+    const int i = (int)((threadIdx.x >> 2) * n / (kThreads / 4));      // (the same in all blocks)
+    const int some = __reduce_add_sync(
+        0xffffffffu, sampled_candidates<D>(i, a.keys, a.c.start, a.c.num_cells, total));
+    if (lane == 0) atomicAdd(&sampled_s, some);
+  }
   for (int turn = 0; turn < turns; ++turn) {
     const int q = group + turn * kGroups;
     const int j = point(q);
@@ -535,12 +576,17 @@ settle_kernel(SampleArgs a) {
       mine = __reduce_add_sync(0xffffffffu, mine);
       if (lane == 0) atomicAdd(&candidates_s, mine);
       __syncthreads();
-      if (candidates_s > kFlowWork * kGroups / turns) {
+      const int limit = min(flow_work(D) / turns, kFlowMost);
+      if (sampled_s > limit * kThreads ||
+          candidates_s > (n > kFlowFew ? 4 * limit : 448) * kGroups) {
         if (threadIdx.x == 0) *failed = 1u;
         return;
       }
     }
-    if (end - begin > kFlowCell) *failed = 1u;
+    if (end - begin > kFlowCell) {
+      *failed = 1u;
+      return;
+    }
     if (*failed) return;
     if (!live) continue;
     float p[D];
