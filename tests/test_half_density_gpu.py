@@ -78,3 +78,19 @@ def test_neighborhoods_of_many_neighbors_take_half():
   late.compute_pdf(bandwidth=0.2)
   assert late._pairs_of_all_points() > 66000 * 100
   assert torch.allclose(early.point_pdf(), late.point_pdf(), rtol=1e-6, atol=0.0)
+
+
+@pytest.mark.parametrize("b,half", [(700, False), (100, True)])
+def test_clouds_of_few_points_take_all_tests(b, half):
+  """Many neighbors are few candidates where a cloud has no more points (the workspace shows which
+  way was taken)."""
+  n = 80000
+  gen = torch.Generator(device=DEV).manual_seed(b)
+  ids = torch.sort(torch.randint(0, b, (n,), generator=gen, device=DEV)).values.int()
+  neigh = pc.grid_neighborhood(pc.PointCloud(torch.rand((n, 3), generator=gen, device=DEV), ids, b), 0.57)
+  assert neigh._pairs_of_all_points() > 40 * n
+  torch.cuda.synchronize()
+  torch.cuda.reset_peak_memory_stats()
+  before = torch.cuda.memory_allocated()
+  neigh.compute_pdf(bandwidth=0.2)
+  assert (torch.cuda.max_memory_allocated() - before >= 12 * n) == half
