@@ -491,8 +491,9 @@ __device__ __noinline__ int sampled_candidates(int i, const int64_t* keys, const
 // 23 and 21 so.
 // Where cells are crowded the passes, which test around taken points only, are the faster ones.  All
 // blocks of a level of more than kFlowFew points find that out from the same points, before they
-// test any: 1.2 us of a settled level, 6 in all of one that is left.  (When each went by its own points,
-// and few found it out, the others tested in vain for 16 to 43 us: levels of 30 000 and 60 000 points
+// test any: 1.2 us of a settled level, 6 in all of one that is left.  (Blocks whose own points have
+// less than an eighth of that need not ask: a quarter would make some test in vain, 7000 points
+// with 260 neighbors 106 -> 124 us.  When each went by its own points, and few found it out, the others tested in vain for 16 to 43 us: levels of 30 000 and 60 000 points
 // with 100 to 270 candidates took 130 to 157 us, now 114 to 121, by passes alone 103 to 111.)  A block
 // with far more candidates than that, a list that runs over and a cell that is too full leave the
 // level to the passes as well, and a point of too full a cell is not searched for.  Then nothing of
@@ -535,12 +536,6 @@ settle_kernel(SampleArgs a) {
   for (int i = threadIdx.x; i < kFlowPer; i += kThreads) listed[i] = 0;
   if (threadIdx.x == 0) candidates_s = sampled_s = 0;
   __syncthreads();
-  if (n > kFlowFew) {
-    const int i = (int)((threadIdx.x >> 2) * n / (kThreads / 4));      // (the same in all blocks)
-    const int some = __reduce_add_sync(
-        0xffffffffu, sampled_candidates<D>(i, a.keys, a.c.start, a.c.num_cells, total));
-    if (lane == 0) atomicAdd(&sampled_s, some);
-  }
   for (int turn = 0; turn < turns; ++turn) {
     const int q = group + turn * kGroups;
     const int j = point(q);
@@ -577,6 +572,13 @@ settle_kernel(SampleArgs a) {
       if (lane == 0) atomicAdd(&candidates_s, mine);
       __syncthreads();
       const int limit = min(flow_work(D) / turns, kFlowMost);
+      if (n > kFlowFew && candidates_s > limit * kGroups / 8) {
+        const int i = (int)((threadIdx.x >> 2) * n / (kThreads / 4));      // (the same in all blocks)
+        const int some = __reduce_add_sync(
+            0xffffffffu, sampled_candidates<D>(i, a.keys, a.c.start, a.c.num_cells, total));
+        if (lane == 0) atomicAdd(&sampled_s, some);
+        __syncthreads();
+      }
       if (sampled_s > limit * kThreads ||
           candidates_s > (n > kFlowFew ? 4 * limit : 448) * kGroups) {
         if (threadIdx.x == 0) *failed = 1u;
