@@ -493,12 +493,13 @@ __device__ __noinline__ int sampled_candidates(int i, const int64_t* keys, const
 // blocks of a level of more than kFlowFew points find that out from the same points, before they
 // test any: 1.2 us of a settled level, 6 in all of one that is left.  (Blocks whose own points have
 // less than an eighth of that need not ask: a quarter would make some test in vain, 7000 points
-// with 260 neighbors 106 -> 124 us.  When each went by its own points, and few found it out, the others tested in vain for 16 to 43 us: levels of 30 000 and 60 000 points
-// with 100 to 270 candidates took 130 to 157 us, now 114 to 121, by passes alone 103 to 111.)  A block
-// with far more candidates than that, a list that runs over and a cell that is too full leave the
-// level to the passes as well, and a point of too full a cell is not searched for.  Then nothing of
-// this counts (20 000 points in one cell, this kernel and the passes, without a look at a point's
-// own cell 408 + 43 us, with it 4 + 43; in eight clouds of a cell each 190 + 31 and 4 + 31).
+// with 260 neighbors 106 -> 124 us.  When each went by its own points, and few found it out, the
+// others tested in vain for 16 to 43 us: levels of 30 000 and 60 000 points with 100 to 270
+// candidates took 130 to 157 us, now 114 to 121, by passes alone 103 to 111.)  A block with far more
+// candidates than that, a list that runs over and a cell that is too full leave the level to the
+// passes as well, and a point of too full a cell is not searched for.  Then nothing of this counts
+// (20 000 points in one cell, this kernel and the passes, without a look at a point's own cell
+// 408 + 43 us, with it 4 + 43; in eight clouds of a cell each 190 + 31 and 4 + 31).
 template <int D>
 __global__ void __launch_bounds__(kThreads, 4)
 settle_kernel(SampleArgs a) {
